@@ -1,13 +1,13 @@
 // Flash attention for sm_100a: tcgen05 MMAs with S / O accumulators in TMEM, TMA-fed K/V ring,
-// two 128-row query tiles per CTA processed ping-pong by two softmax warpgroups.
+// two 128-row query tiles per CTA processed ping-pong by two pairs of softmax warpgroups.
 //
 // Forward  (attn_fwd_kernel):  S = Q K^T -> online softmax (exp2 domain, lazy rescale) ->
-//                              P (bf16, swizzled smem) -> O += P V (O stays in TMEM).
+//                              P (16-bit, over S in TMEM) -> O += P V (O stays in TMEM).
 // Backward (two kernels, deterministic, no atomics):
-//   attn_bwd_dkdv_kernel : CTA per 128-key block, loops over 64-query blocks
-//                          S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q
-//   attn_bwd_dq_kernel   : CTA per 128-query block, loops over 64-key blocks
-//                          S = Q K^T, dP = dO V^T, dQ += dS K
+//   attn_bwd_kernel<dK, dV> : CTA per 128-key block, loops over 64-query blocks
+//                             S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q
+//   attn_bwd_kernel<dQ>     : CTA per 128-query block, loops over 64-key blocks
+//                             S = Q K^T, dP = dO V^T, dQ += dS K
 // Operands are strided [b, h, s, d] views (last dim contiguous) so the Megatron [s, b, h, d]
 // activations are consumed in place (4-D tensor maps); outputs are written in [s, b, h, d].
 //
@@ -16,7 +16,6 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-#include <cstdlib>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -46,14 +45,79 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ uint32_t pack16(float lo, float hi, bool bf16) {
-  if (bf16) return pack_bf16x2(lo, hi);
+template <bool kBf16>
+__device__ __forceinline__ uint32_t pack16(float lo, float hi) {
+  if constexpr (kBf16) return pack_bf16x2(lo, hi);
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// byte offset of 16-byte unit `u16` (0..7) of row `r` inside a [rows x 128 B] SWIZZLE_128B tile
-__device__ __forceinline__ uint32_t sw128_off(int r, int u16) {
-  return static_cast<uint32_t>(r) * 128u + (static_cast<uint32_t>(u16 ^ (r & 7)) << 4);
+// two fp32 lanes of one 64-bit register: the packed forms round like the scalar ones at half the issue slots
+__device__ __forceinline__ uint64_t f2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void un2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// tcgen05.mma takes its descriptors from uniform registers.  A loop run by one lane of a diverged warp moves each of them over before
+// every instruction (70 cycles an MMA measured, more than the 32 to 64 that these tiles take to execute); the issuing warp therefore runs
+// its loop converged, on descriptors that advance by constants, and one elected lane issues.
+__device__ __forceinline__ uint64_t desc_at(uint64_t base, uint32_t bytes) { return base + (bytes >> 4); }
+
+constexpr int kWaitLimit = 1 << 20;
+__device__ int g_attn_error = 0;
+// false: the wait ran out here, or another thread of the CTA gave up
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* failed) {
+  for (int i = 0; i < kWaitLimit; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255) == 255 && *failed) return false;
+  }
+  *failed = 1;
+  return false;
+}
+// the same for a whole warp, which leaves the wait converged
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* failed) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, failed));
+}
+
+// One warpgroup copies and issues, four do the softmax arithmetic.  A CTA of 640 threads starts with 96 registers each; the math
+// warpgroups take 104 and leave 64 to the first.
+constexpr int kThreads = 640, kMathRegs = 104, kIssueRegs = 64;
+static_assert(512 * kMathRegs + 128 * kIssueRegs <= kThreads * 96, "the shares come out of what the CTA was launched with");
+template <int N> __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// 32 accumulator columns of this thread's row, scaled, as 64 bytes of 16-bit results
+template <bool kBf16>
+__device__ __forceinline__ void store_row32(uint8_t* dst, const uint32_t (&v)[32], float mul) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    uint4 w;
+    w.x = pack16<kBf16>(__uint_as_float(v[u * 8 + 0]) * mul, __uint_as_float(v[u * 8 + 1]) * mul);
+    w.y = pack16<kBf16>(__uint_as_float(v[u * 8 + 2]) * mul, __uint_as_float(v[u * 8 + 3]) * mul);
+    w.z = pack16<kBf16>(__uint_as_float(v[u * 8 + 4]) * mul, __uint_as_float(v[u * 8 + 5]) * mul);
+    w.w = pack16<kBf16>(__uint_as_float(v[u * 8 + 6]) * mul, __uint_as_float(v[u * 8 + 7]) * mul);
+    *reinterpret_cast<uint4*>(dst + u * 16) = w;
+  }
+}
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 
 struct FwdParams {
@@ -63,55 +127,57 @@ struct FwdParams {
   int b, hq, hkv, sq, sk;
   float scale_log2;      // softmax scale * log2(e)
   int causal;
-  int is_bf16;
 };
 
-// kPTmem: P (bf16) overwrites the S columns in TMEM and feeds the PV product as the TMEM A operand
-// (halves the shared-memory traffic of a key block and frees room for a second V stage);
-// otherwise P goes through swizzled shared memory.
-template <int D, bool kPTmem>
+template <int D>
 struct FwdSmem {
   static constexpr int kDC = D / 64;                    // 64-element (128 B) chunks along d
   static constexpr int kTile = kBlockQ * 128 * kDC;     // bytes of a [128 x D] 16-bit tile
-  static constexpr int kKStages = 2;
-  static constexpr int kVStages = (D == 64 || kPTmem) ? 2 : 1;
-  static constexpr int kP = kPTmem ? 0 : kBlockQ * kBlockKV * 2;     // 32 KB
+  static constexpr int kStages = 2;
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + 2 * kTile;
-  static constexpr int kVOff = kKOff + kKStages * kTile;
-  static constexpr int kPOff = kVOff + kVStages * kTile;
-  static constexpr int kBarOff = kPOff + 2 * kP;
+  static constexpr int kVOff = kKOff + kStages * kTile;
+  static constexpr int kExOff = kVOff + kStages * kTile;          // [parity][tile][half][row] partial maxima, then sums
+  static constexpr int kBarOff = kExOff + 2 * 2 * 2 * kBlockQ * 4;
   static constexpr int kTotal = kBarOff + 256 + 1024;   // + barriers + alignment slack
 };
 
 // ------------------------------------------------------------------------------------ forward
-template <int D, bool kPTmem>
-__global__ void __launch_bounds__(384, 1)
+// P (16-bit) overwrites S columns in TMEM and feeds the PV product as the TMEM A operand.  Two query tiles alternate between the tensor
+// core (1024 cycles a key block at D = 128) and the softmax (1024 cycles of exponentials at one block's rate), so what counts is the time
+// from S to P of one tile.  Two warpgroups share it, 64 columns of each row apiece: S is read once into registers, the halves
+// exchange their row maxima through shared memory, and each packs its P into its own half of the S columns.
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
-  using L = FwdSmem<D, kPTmem>;
+  using L = FwdSmem<D>;
+  constexpr int kS = L::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::kQOff;
   uint8_t* sK = smem + L::kKOff;
   uint8_t* sV = smem + L::kVOff;
-  uint8_t* sP = smem + L::kPOff;
+  float* sEx = reinterpret_cast<float*>(smem + L::kExOff);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
   uint64_t* q_full = bars;            // 1
   uint64_t* k_full = bars + 1;        // 2
   uint64_t* k_empty = bars + 3;       // 2
   uint64_t* v_full = bars + 5;        // 2
   uint64_t* v_empty = bars + 7;       // 2
-  uint64_t* s_full = bars + 9;        // 2 (per q tile)
+  uint64_t* s_full = bars + 9;        // 2 (per q tile); S(j + 1) complete says that PV(j), issued before it, is too
   uint64_t* p_ready = bars + 11;      // 2
-  uint64_t* pv_done = bars + 13;      // 2
+  uint64_t* o_done = bars + 13;       // 2
+  uint64_t* drained = bars + 15;      // 1, failure path only
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  volatile int* failed = reinterpret_cast<volatile int*>(bars + 17);
 
-  const int warp_idx = threadIdx.x >> 5;
+  const int warp_idx = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // known to be uniform: see desc_at
   const int lane = threadIdx.x & 31;
-  // heaviest (largest q index) CTAs first for causal load balance
-  const int qblk2 = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
-  const int h = blockIdx.y, bi = blockIdx.z;
+  // (query block, head, batch) from one grid dimension, the longest rows of every head before any shorter ones
+  const int n_hb = p.hq * p.b, hb = static_cast<int>(blockIdx.x) % n_hb;
+  const int qblk2 = static_cast<int>(gridDim.x) / n_hb - 1 - static_cast<int>(blockIdx.x) / n_hb;
+  const int h = hb % p.hq, bi = hb / p.hq;
   const int hk = h / (p.hq / p.hkv);
   const int q0_0 = qblk2 * 2 * kBlockQ, q0_1 = q0_0 + kBlockQ;
   const int nkv_all = (p.sk + kBlockKV - 1) / kBlockKV;
@@ -127,8 +193,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 128); mbar_init(&pv_done[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 256); mbar_init(&o_done[i], 1);
     }
+    mbar_init(drained, 1);
+    *failed = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
   }
@@ -140,188 +208,180 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const uint32_t tmem_S = tmem_base;          // S[t] at col t*128
   const uint32_t tmem_O = tmem_base + 256;    // O[t] at col 256 + t*D
 
-  if (warp_idx == 0) {
-    // ============================================================ TMA producer
-    if (lane == 0) {
+  if (warp_idx < 4) {
+    regs_give<kIssueRegs>();
+    if (warp_idx == 0 && lane == 0) {
+      // ============================================================ TMA producer
       const int ntiles = (nkv_1 > 0) ? 2 : 1;
       mbar_arrive_expect_tx(q_full, ntiles * L::kTile);
       for (int t = 0; t < ntiles; ++t)
         for (int c = 0; c < L::kDC; ++c)
           tma_load_4d(&tmap_q, q_full, sQ + t * L::kTile + c * (kBlockQ * 128), c * 64, h, bi, t == 0 ? q0_0 : q0_1);
-      for (int j = 0; j < nmax; ++j) {
-        const int ks = j % L::kKStages, vs = j % L::kVStages;
-        mbar_wait(&k_empty[ks], ((j / L::kKStages) & 1) ^ 1);
-        mbar_arrive_expect_tx(&k_full[ks], L::kTile);
+      int nk = 0, nv = 0;
+      while (nk < nmax) {
+        const int st = nk % kS;
+        const uint32_t ph = ((nk / kS) & 1) ^ 1;
+        if (!wait_bar(&k_empty[st], ph, failed)) break;
+        mbar_arrive_expect_tx(&k_full[st], L::kTile);
         for (int c = 0; c < L::kDC; ++c)
-          tma_load_4d(&tmap_k, &k_full[ks], sK + ks * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, j * kBlockKV);
-        mbar_wait(&v_empty[vs], ((j / L::kVStages) & 1) ^ 1);
-        mbar_arrive_expect_tx(&v_full[vs], L::kTile);
+          tma_load_4d(&tmap_k, &k_full[st], sK + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, nk * kBlockKV);
+        ++nk;
+        if (!wait_bar(&v_empty[st], ph, failed)) break;
+        mbar_arrive_expect_tx(&v_full[st], L::kTile);
         for (int c = 0; c < L::kDC; ++c)
-          tma_load_4d(&tmap_v, &v_full[vs], sV + vs * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, j * kBlockKV);
+          tma_load_4d(&tmap_v, &v_full[st], sV + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, nv * kBlockKV);
+        ++nv;
       }
-    }
-  } else if (warp_idx == 1) {
-    // ============================================================ MMA issuer
-    if (lane == 0 && nmax > 0) {
-      const uint32_t idesc_s = make_idesc_f16(p.is_bf16 != 0, kBlockQ, kBlockKV, false, false);
-      const uint32_t idesc_o = make_idesc_f16(p.is_bf16 != 0, kBlockQ, D, false, true);
+      if (*failed) {                                        // let the copies in flight land before the CTA ends
+        volatile int never = 0;
+        wait_bar(q_full, 0, &never);
+        for (int i = max(0, nk - kS); i < nk; ++i) wait_bar(&k_full[i % kS], (i / kS) & 1, &never);
+        for (int i = max(0, nv - kS); i < nv; ++i) wait_bar(&v_full[i % kS], (i / kS) & 1, &never);
+      }
+    } else if (warp_idx == 1 && nmax > 0) {
+      // ============================================================ MMA issuer
+      constexpr uint32_t idesc_s = make_idesc_f16(kBf16, kBlockQ, kBlockKV, false, false);
+      constexpr uint32_t idesc_o = make_idesc_f16(kBf16, kBlockQ, D, false, true);
+      const uint64_t q_desc = make_smem_desc_sw128(smem_u32(sQ), 1024, 0), k_desc = make_smem_desc_sw128(smem_u32(sK), 1024, 0);
+      // V is MN-major for its product (N = d contiguous): 16 key rows per k-step, LBO = next 64-wide d chunk
+      const uint64_t v_desc = make_smem_desc_sw128(smem_u32(sV), 1024, kBlockKV * 128);
       auto issue_S = [&](int t, int j) {
-        const int ks = j % L::kKStages;
-        const uint32_t a0 = smem_u32(sQ + t * L::kTile), b0 = smem_u32(sK + ks * L::kTile);
+        const uint64_t a0 = desc_at(q_desc, t * L::kTile), b0 = desc_at(k_desc, (j % kS) * L::kTile);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * (kBlockQ * 128) + (k & 3) * 32;
-          umma_f16_ss(tmem_S + t * 128, make_smem_desc_sw128(a0 + off, 1024, 0),
-                      make_smem_desc_sw128(b0 + off, 1024, 0), idesc_s, k != 0 ? 1u : 0u);
+          for (int k = 0; k < D / 16; ++k) {
+            const uint32_t off = (k >> 2) * (kBlockQ * 128) + (k & 3) * 32;
+            umma_f16_ss(tmem_S + t * 128, desc_at(a0, off), desc_at(b0, off), idesc_s, k != 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[t]);
         }
-        umma_commit(&s_full[t]);
       };
       auto issue_PV = [&](int t, int j) {
-        const int vs = j % L::kVStages;
-        const uint32_t a0 = smem_u32(sP + t * L::kP), b0 = smem_u32(sV + vs * L::kTile);
+        const uint64_t b0 = desc_at(v_desc, (j % kS) * L::kTile);
+        const uint32_t first = j != 0 ? 1u : 0u;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < kBlockKV / 16; ++k) {
-          // V is MN-major for this product (N = d contiguous): 16 key rows per k-step,
-          // LBO = next 64-wide d chunk
-          const uint64_t bdesc = make_smem_desc_sw128(b0 + k * 16 * 128, 1024, kBlockKV * 128);
-          if constexpr (kPTmem) {
-            // A = P from TMEM: row = lane, 16 keys = 8 packed 32-bit columns per k-step
-            umma_f16_ts(tmem_O + t * D, tmem_S + t * 128 + k * 8, bdesc, idesc_o, (j | k) != 0 ? 1u : 0u);
-          } else {
-            const uint32_t aoff = (k >> 2) * (kBlockQ * 128) + (k & 3) * 32;
-            umma_f16_ss(tmem_O + t * D, make_smem_desc_sw128(a0 + aoff, 1024, 0), bdesc, idesc_o,
-                        (j | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < kBlockKV / 16; ++k)
+            // A = P from TMEM: row = lane, 16 keys = 8 packed 32-bit columns per k-step, 64 keys per half of the S columns
+            umma_f16_ts(tmem_O + t * D, tmem_S + t * 128 + (k >> 2) * 64 + (k & 3) * 8, desc_at(b0, k * 16 * 128), idesc_o, k != 0 ? 1u : first);
         }
-        umma_commit(&pv_done[t]);
       };
-      mbar_wait(q_full, 0);
-      mbar_wait(&k_full[0], 0);
-      tc_fence_after();
-      if (nkv_0 > 0) issue_S(0, 0);
-      if (nkv_1 > 0) issue_S(1, 0);
-      umma_commit(&k_empty[0]);
-      for (int j = 0; j < nmax; ++j) {
-        const int vs = j % L::kVStages;
-        mbar_wait(&v_full[vs], (j / L::kVStages) & 1);
-        if (j + 1 < nmax) mbar_wait(&k_full[(j + 1) % L::kKStages], ((j + 1) / L::kKStages) & 1);
+      auto commit = [&](uint64_t* bar) { if (elect_one()) umma_commit(bar); };
+      bool ok = wait_bar_warp(q_full, 0, failed) && wait_bar_warp(&k_full[0], 0, failed);
+      if (ok) {
+        tc_fence_after();
+        if (nkv_0 > 0) issue_S(0, 0);
+        if (nkv_1 > 0) issue_S(1, 0);
+        commit(&k_empty[0]);
+      }
+      for (int j = 0; j < nmax && ok; ++j) {
+        const int nx = (j + 1) % kS;
+        ok = wait_bar_warp(&v_full[j % kS], (j / kS) & 1, failed) && (j + 1 >= nmax || wait_bar_warp(&k_full[nx], ((j + 1) / kS) & 1, failed));
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           const int nt = t == 0 ? nkv_0 : nkv_1;
-          if (j >= nt) continue;
-          mbar_wait(&p_ready[t], j & 1);
+          if (j >= nt || !ok) continue;
+          ok = wait_bar_warp(&p_ready[t], j & 1, failed);
+          if (!ok) continue;
           tc_fence_after();
           issue_PV(t, j);
           if (j + 1 < nt) issue_S(t, j + 1);
+          else commit(&o_done[t]);
         }
-        umma_commit(&v_empty[vs]);
-        if (j + 1 < nmax) umma_commit(&k_empty[(j + 1) % L::kKStages]);
+        if (!ok) break;
+        commit(&v_empty[j % kS]);
+        if (j + 1 < nmax) commit(&k_empty[nx]);
+      }
+      if (!ok) {                                            // the MMAs in flight finish before TMEM is freed
+        volatile int never = 0;
+        commit(drained);
+        wait_bar_warp(drained, 0, &never);
       }
     }
-  } else if (warp_idx >= 4) {
+  } else {
     // ============================================================ softmax / correction / epilogue
-    const int t = (warp_idx - 4) >> 2;            // q tile of this warpgroup
+    regs_take<kMathRegs>();
+    const int t = (warp_idx - 4) >> 3;            // q tile of this warpgroup
+    const int half = ((warp_idx - 4) >> 2) & 1;   // its columns of S: 64 half .. 64 half + 63, and of O: D / 2 likewise
     const int quad = warp_idx & 3;                // TMEM lane quadrant
     const int r = quad * 32 + lane;               // row inside the tile
     const int q0 = t == 0 ? q0_0 : q0_1;
     const int qrow = q0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tS = tmem_S + t * 128 + lane_addr;
-    const uint32_t tO = tmem_O + t * D + lane_addr;
-    uint8_t* sPt = sP + t * L::kP;
-    float m = -INFINITY, l = 0.f;   // running max (exp2 domain, already scaled) and row sum
+    const uint32_t tS = tmem_S + t * 128 + half * 64 + lane_addr;
+    const uint32_t tO = tmem_O + t * D + half * (D / 2) + lane_addr;
+    float* ex = sEx + t * (2 * kBlockQ);          // + parity * 4 kBlockQ + half * kBlockQ + row
+    float m = -INFINITY;                          // running max (exp2 domain, already scaled)
+    uint64_t l2 = 0;                              // running sum of this half's even and odd columns
     const int n = t == 0 ? nkv_0 : nkv_1;
     const float sc = p.scale_log2;
-    const bool bf = p.is_bf16 != 0;
+    const uint64_t sc2 = f2(sc, sc);
 
-    // one key block: two sweeps over the S tile in TMEM (row max, then exp2 / pack / store P)
     auto block = [&](int j, auto masked_tag) {
       constexpr bool kMasked = decltype(masked_tag)::value;
-      const int kbase = j * kBlockKV;
-      const int limit = (kMasked ? min(p.sk, p.causal ? qrow + 1 : p.sk) : 0) - kbase;   // valid: col < limit
-      float mx = -INFINITY;
-      {
-        uint32_t v[2][32];
-        tmem_ld_32x32(tS, v[0]);
+      const int limit = (kMasked ? min(p.sk, p.causal ? qrow + 1 : p.sk) : 0) - j * kBlockKV - half * 64;   // valid: col < limit
+      uint32_t v[2][32];
+      tmem_ld_32x32(tS, v[0]);
+      tmem_ld_32x32(tS + 32, v[1]);
+      tmem_ld_wait();
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          tmem_ld_wait();
-          if (c < 3) tmem_ld_32x32(tS + (c + 1) * 32, v[(c + 1) & 1]);
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float x = __uint_as_float(v[c & 1][i]);
-            if (kMasked && c * 32 + i >= limit) x = -INFINITY;
-            mx = fmaxf(mx, x);
-          }
+        for (int i = 0; i < 32; ++i) {
+          if (kMasked && c * 32 + i >= limit) v[c][i] = 0xff800000u;   // -inf
+          mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[c][i]));
         }
-      }
-      float m_new = fmaxf(m, mx * sc);             // softmax scale is positive
+      const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      float* slot = ex + (j & 1) * (4 * kBlockQ);
+      slot[half * kBlockQ + r] = mine;
+      named_bar_sync(1 + t, 256);
+      float m_new = fmaxf(m, fmaxf(mine, slot[(half ^ 1) * kBlockQ + r]) * sc);   // softmax scale is positive
       if (m_new == -INFINITY) m_new = 0.f;         // fully masked so far: keep everything finite
       const bool grow = (m_new - m) > kRescaleThreshold;   // also true on the first block (m = -inf)
-      const float m_cur = grow ? m_new : m;
-      const float alpha = grow ? fast_exp2(m - m_cur) : 1.f;
-      if (j > 0) {
-        mbar_wait(&pv_done[t], (j - 1) & 1);
-        tc_fence_after();
-        if (__any_sync(0xffffffffu, grow)) {
+      if (__any_sync(0xffffffffu, grow)) {
+        const float m_cur = grow ? m_new : m;
+        const float alpha = grow ? fast_exp2(m - m_cur) : 1.f;
+        m = m_cur;
+        l2 = mul2(l2, f2(alpha, alpha));
+        if (j > 0) {
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t v[32];
-            tmem_ld_32x32(tO + c * 32, v);
+          for (int c = 0; c < D / 32; ++c) {     // in small pieces: the scores are in registers
+            uint32_t o[16];
+            tmem_ld_32x16(tO + c * 16, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st_32x32(tO + c * 32, v);
-          }
-          tmem_st_wait();
-        }
-      }
-      l *= alpha;
-      float rs0 = 0.f, rs1 = 0.f;
-      {
-        uint32_t v[2][32];
-        tmem_ld_32x32(tS, v[0]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          tmem_ld_wait();
-          if (c < 3) tmem_ld_32x32(tS + (c + 1) * 32, v[(c + 1) & 1]);
-          uint32_t pk[16];
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float p0 = fast_exp2(fmaf(__uint_as_float(v[c & 1][i]), sc, -m_cur));
-            float p1 = fast_exp2(fmaf(__uint_as_float(v[c & 1][i + 1]), sc, -m_cur));
-            if (kMasked) {
-              if (c * 32 + i >= limit) p0 = 0.f;
-              if (c * 32 + i + 1 >= limit) p1 = 0.f;
-            }
-            rs0 += p0;
-            rs1 += p1;
-            pk[i >> 1] = pack16(p0, p1, bf);
-          }
-          if constexpr (kPTmem) {
-            // packed P chunk c -> TMEM columns [16c, 16c+16) of this tile's S region; the fp32 S
-            // columns it overwrites ([32c', ...) with c' < c, or chunk 0 itself) are already consumed
-            tmem_st_32x16(tS + c * 16, pk);
-          } else {
-            // keys c*32 .. c*32+31 -> chunk (c>>1), 16-byte units (c&1)*4 .. +3 of row r
-            uint8_t* chunk = sPt + (c >> 1) * (kBlockQ * 128);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              *reinterpret_cast<uint4*>(chunk + sw128_off(r, (c & 1) * 4 + u)) =
-                  make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x16(tO + c * 16, o);
           }
         }
       }
-      l += rs0 + rs1;
-      m = m_cur;
-      if constexpr (kPTmem) tmem_st_wait();
+      const uint64_t nm2 = f2(-m, -m);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float p0, p1;
+          un2(fma2(f2(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), sc2, nm2), p0, p1);
+          p0 = fast_exp2(p0);
+          p1 = fast_exp2(p1);
+          l2 = add2(l2, f2(p0, p1));
+          pk[i >> 1] = pack16<kBf16>(p0, p1);
+        }
+        // packed chunk c -> columns [16c, 16c+16) of this half, whose scores are in registers
+        tmem_st_32x16(tS + c * 16, pk);
+      }
+      tmem_st_wait();
       tc_fence_before();
-      if constexpr (!kPTmem) fence_proxy_async_smem();
       mbar_arrive(&p_ready[t]);
     };
 
+    // a wait that runs out is noted, not acted on: the halves' warpgroups go on to their exchanges together, and every later wait ends at once
+    bool ok = true;
     for (int j = 0; j < n; ++j) {
-      mbar_wait(&s_full[t], j & 1);
+      wait_bar(&s_full[t], j & 1, failed);
+      __syncwarp();
       tc_fence_after();
       const int kbase = j * kBlockKV;
       // diagonal block of a causal tile, or the ragged tail of the key sequence
@@ -330,78 +390,94 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       else block(j, std::false_type{});
     }
     if (n > 0) {
-      mbar_wait(&pv_done[t], (n - 1) & 1);
+      ok = wait_bar_warp(&o_done[t], 0, failed);
       tc_fence_after();
+      float la, lb;
+      un2(l2, la, lb);
+      float* slot = ex + (n & 1) * (4 * kBlockQ);
+      slot[half * kBlockQ + r] = la + lb;
+      named_bar_sync(1 + t, 256);
+      const float l = slot[r] + slot[kBlockQ + r];
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      const bool valid = qrow < p.sq;
+      const bool valid = qrow < p.sq && ok;
       uint8_t* orow = reinterpret_cast<uint8_t*>(p.o) +
                       (static_cast<int64_t>(qrow) * p.o_ss + static_cast<int64_t>(bi) * p.o_sb +
-                       static_cast<int64_t>(h) * p.o_sh) * 2;
+                       static_cast<int64_t>(h) * p.o_sh + half * (D / 2)) * 2;
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
+      for (int c = 0; c < D / 64; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(tO + c * 32, v);
         tmem_ld_wait();
-        if (valid) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 w;
-            w.x = pack16(__uint_as_float(v[u * 8 + 0]) * inv_l, __uint_as_float(v[u * 8 + 1]) * inv_l, bf);
-            w.y = pack16(__uint_as_float(v[u * 8 + 2]) * inv_l, __uint_as_float(v[u * 8 + 3]) * inv_l, bf);
-            w.z = pack16(__uint_as_float(v[u * 8 + 4]) * inv_l, __uint_as_float(v[u * 8 + 5]) * inv_l, bf);
-            w.w = pack16(__uint_as_float(v[u * 8 + 6]) * inv_l, __uint_as_float(v[u * 8 + 7]) * inv_l, bf);
-            *reinterpret_cast<uint4*>(orow + c * 64 + u * 16) = w;
-          }
-        }
+        if (valid) store_row32<kBf16>(orow + c * 64, v, inv_l);
       }
-      if (valid)
+      if (valid && half == 0)
         p.lse[(static_cast<int64_t>(bi) * p.hq + h) * p.sq + qrow] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
     }
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *failed) atomicExch(&g_attn_error, 1);
   if (warp_idx == 2) tmem_dealloc<512>(tmem_base);
 }
 
 
 // ------------------------------------------------------------------------------------ backward
-// delta[b, h, s] = sum_d O * dO   (one warp per row)
-__global__ void attn_delta_kernel(const void* __restrict__ o, const void* __restrict__ d_o, float* __restrict__ delta,
-                                  const float* __restrict__ lse, float* __restrict__ lse2, int b, int h, int s, int d, int64_t o_sb, int64_t o_sh, int64_t o_ss,
-                                  int64_t do_sb, int64_t do_sh, int64_t do_ss, int is_bf16) {
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int64_t total = static_cast<int64_t>(b) * h * s;
-  if (row >= total) return;
-  const int si = static_cast<int>(row % s);
-  const int hi = static_cast<int>((row / s) % h);
-  const int bi = static_cast<int>(row / (static_cast<int64_t>(s) * h));
-  const uint32_t* po = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(o) + bi * o_sb + hi * o_sh + si * o_ss);
-  const uint32_t* pd = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(d_o) + bi * do_sb + hi * do_sh + si * do_ss);
-  float acc = 0.f;
-  for (int i = lane_id(); i < d / 2; i += 32) {
-    const uint32_t a = po[i], c = pd[i];
-    float2 fa, fc;
-    if (is_bf16) { fa = unpack_bf16x2(a); fc = unpack_bf16x2(c); }
-    else { fa = __half22float2(*reinterpret_cast<const __half2*>(&a)); fc = __half22float2(*reinterpret_cast<const __half2*>(&c)); }
-    acc += fa.x * fc.x + fa.y * fc.y;
+// -delta[b, h, s] = -sum_d O * dO and -lse * log2e, the addends of the backward kernels' packed multiply-adds.  D / 8 lanes share a row
+// (16 bytes each), a warp takes four groups of rows with all its loads in flight: 12.5 us for 32 heads x 4096 x 128 (a warp per row and
+// 4 bytes a lane took 35).
+template <int D>
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ d_o, float* __restrict__ ndelta, const float* __restrict__ lse,
+                  float* __restrict__ nlse2, int h, int s, int64_t o_sb, int64_t o_sh, int64_t o_ss, int64_t do_sb, int64_t do_sh, int64_t do_ss,
+                  int is_bf16) {
+  constexpr int kLanes = D / 8, kRows = 32 / kLanes, kSteps = 4;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = (lane % kLanes) * 8;
+  const int hi = blockIdx.y, bi = blockIdx.z;
+  const int s0 = (blockIdx.x * 8 + warp) * (kRows * kSteps) + lane / kLanes;
+  const uint16_t* po = o + bi * o_sb + hi * o_sh + col;
+  const uint16_t* pd = d_o + bi * do_sb + hi * do_sh + col;
+  uint4 a[kSteps], c[kSteps];
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int si = s0 + i * kRows;
+    a[i] = c[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (si < s) {
+      a[i] = *reinterpret_cast<const uint4*>(po + si * o_ss);
+      c[i] = *reinterpret_cast<const uint4*>(pd + si * do_ss);
+    }
   }
-  acc = warp_sum(acc);
-  if (lane_id() == 0) {
-    delta[row] = acc;
-    const float lv = lse[row];
-    lse2[row] = (lv == -INFINITY) ? INFINITY : lv * kLog2e;   // exp2-domain LSE; fully masked rows give P = 0
+#pragma unroll
+  for (int i = 0; i < kSteps; ++i) {
+    const int si = s0 + i * kRows;
+    const uint32_t wa[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, wc[4] = {c[i].x, c[i].y, c[i].z, c[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 fa, fc;
+      if (is_bf16) { fa = unpack_bf16x2(wa[k]); fc = unpack_bf16x2(wc[k]); }
+      else { fa = __half22float2(*reinterpret_cast<const __half2*>(&wa[k])); fc = __half22float2(*reinterpret_cast<const __half2*>(&wc[k])); }
+      acc += fa.x * fc.x + fa.y * fc.y;
+    }
+#pragma unroll
+    for (int k = kLanes / 2; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
+    if (si < s && lane % kLanes == 0) {
+      const int64_t row = (static_cast<int64_t>(bi) * h + hi) * s + si;
+      ndelta[row] = -acc;
+      const float lv = lse[row];
+      nlse2[row] = lv == -INFINITY ? -INFINITY : -lv * kLog2e;   // fully masked rows give P = 0
+    }
   }
 }
 
 struct BwdParams {
-  const float* lse;     // [b, hq, sq] LSE in the exp2 domain (lse * log2e)
-  const float* delta;   // [b, hq, sq]
+  const float* nlse;    // [b, hq, sq] -LSE in the exp2 domain (-lse * log2e)
+  const float* ndelta;  // [b, hq, sq] -delta
   void* out1;           // dq (kDQ) or dv
   void* out2;           // unused (kDQ) or dk
   int64_t o1_sb, o1_sh, o1_ss, o2_sb, o2_sh, o2_ss;
   int b, hq, hkv, sq, sk;
   float scale_log2, scale;
-  int causal, is_bf16;
+  int causal;
 };
 
 constexpr int kBwdRows = 128;   // resident rows per CTA (keys for dK/dV, queries for dQ)
@@ -425,8 +501,12 @@ struct BwdSmem {
 // kDQ = true : rows are queries (X1 = Q, X2 = dO, Y1 = K_j, Y2 = V_j): acc1 = dQ
 // P / dS (16-bit) overwrite the T1 / T2 accumulator columns in TMEM and feed the accumulate MMAs as
 // the TMEM A operand, so the only shared-memory traffic is the operand tiles themselves.
-template <int D, bool kDQ>
-__global__ void __launch_bounds__(256, 1)
+// A block's MMAs take about 1300 cycles (T at N = 64 is bound by its shared-memory reads), its exponentials and products about 2500
+// in one warpgroup: a warp per scheduler that waits on its own results.  So the blocks alternate between two T buffers, the
+// tensor core working on one while the other's P / dS are made, and two warpgroups share a buffer, 32 columns each.
+// CTAs start with the longest rows of a causal problem.  32 / 8 heads x 4096 x 128: dK / dV 405 -> 281 us, dQ 278 -> 231 us.
+template <int D, bool kDQ, bool kBf16>
+__global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_constant__ CUtensorMap tmap_x2,
                 const __grid_constant__ CUtensorMap tmap_y1, const __grid_constant__ CUtensorMap tmap_y2,
                 const BwdParams p) {
@@ -437,7 +517,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   uint8_t* sX1 = smem + L::kX1Off;
   uint8_t* sX2 = smem + L::kX2Off;
   uint8_t* sY = smem + L::kStageOff;
-  float* sStat = reinterpret_cast<float*>(smem + L::kStatOff);   // stage s: lse2 at s*128, delta at s*128+64
+  float* sStat = reinterpret_cast<float*>(smem + L::kStatOff);   // stage s: -lse2 at s*128, -delta at s*128+64
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
   uint64_t* x_full = bars;               // 1
   uint64_t* y_full = bars + 1;           // kS
@@ -445,22 +525,28 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   uint64_t* t_full = bars + 1 + 2 * kS;  // 2
   uint64_t* pds_ready = t_full + 2;      // 2
   uint64_t* acc_done = pds_ready + 2;    // 1
+  uint64_t* drained = acc_done + 1;      // 1, failure path only
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+  volatile int* failed = reinterpret_cast<volatile int*>(bars + 25);
 
-  const int warp_idx = threadIdx.x >> 5;
+  const int warp_idx = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // known to be uniform: see desc_at
   const int lane = threadIdx.x & 31;
-  const int bi = blockIdx.z;
   const int G = p.hq / p.hkv;
-  const int r0 = blockIdx.x * kBwdRows;
+  // (row block, head, batch) from one grid dimension: every head's longest row block comes before any shorter one
+  const int n_out = kDQ ? p.hq : p.hkv;
+  const int blk = static_cast<int>(blockIdx.x) / (n_out * p.b), hb = static_cast<int>(blockIdx.x) % (n_out * p.b);
+  const int out_head = hb % n_out, bi = hb / n_out;
+  const int n_blk = static_cast<int>(gridDim.x) / (n_out * p.b);
+  const int r0 = (kDQ ? n_blk - 1 - blk : blk) * kBwdRows;
   // iteration space
   int col_blk0, n_col, n_heads, head0;
   if (kDQ) {
-    head0 = blockIdx.y; n_heads = 1;
+    head0 = out_head; n_heads = 1;
     col_blk0 = 0;
     const int kmax = p.causal ? min(p.sk, r0 + kBwdRows) : p.sk;
     n_col = (kmax + kBwdCols - 1) / kBwdCols;
   } else {
-    head0 = blockIdx.y * G; n_heads = G;
+    head0 = out_head * G; n_heads = G;
     col_blk0 = p.causal ? r0 / kBwdCols : 0;
     n_col = (p.sq + kBwdCols - 1) / kBwdCols - col_blk0;
     if (n_col < 0) n_col = 0;
@@ -470,8 +556,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   if (threadIdx.x == 0) {
     mbar_init(x_full, 1);
     for (int i = 0; i < kS; ++i) { mbar_init(&y_full[i], 1); mbar_init(&y_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&pds_ready[i], 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&pds_ready[i], 256); }
     mbar_init(acc_done, 1);
+    mbar_init(drained, 1);
+    *failed = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_x1); tma_prefetch_desc(&tmap_x2); tma_prefetch_desc(&tmap_y1); tma_prefetch_desc(&tmap_y2);
   }
@@ -480,25 +568,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_T1 = tmem_base;          // T1[buf] at col buf*64  (P overwrites its first 32 cols)
-  const uint32_t tmem_T2 = tmem_base + 128;    // T2[buf] at col 128 + buf*64 (dS overwrites its first 32 cols)
+  const uint32_t tmem_T1 = tmem_base;          // T1[buf] at col buf*64: P overwrites the first half of each 32 cols
+  const uint32_t tmem_T2 = tmem_base + 128;    // T2[buf] at col 128 + buf*64: so does dS
   const uint32_t tmem_A1 = tmem_base + 256;    // dV or dQ
   const uint32_t tmem_A2 = tmem_base + 256 + D;  // dK
 
-  if (warp_idx == 0) {
-    // ============================================================ TMA producer
-    if (lane == 0 && n_iter > 0) {
-      const int hx = blockIdx.y;   // head of the resident tiles (kv head for dK/dV, q head for dQ)
+  if (warp_idx < 4) {
+    regs_give<kIssueRegs>();
+    if (warp_idx == 0 && lane == 0 && n_iter > 0) {
+      // ============================================================ TMA producer
       mbar_arrive_expect_tx(x_full, 2 * L::kX);
       for (int c = 0; c < L::kDC; ++c) {
-        tma_load_4d(&tmap_x1, x_full, sX1 + c * (kBwdRows * 128), c * 64, hx, bi, r0);
-        tma_load_4d(&tmap_x2, x_full, sX2 + c * (kBwdRows * 128), c * 64, hx, bi, r0);
+        tma_load_4d(&tmap_x1, x_full, sX1 + c * (kBwdRows * 128), c * 64, out_head, bi, r0);
+        tma_load_4d(&tmap_x2, x_full, sX2 + c * (kBwdRows * 128), c * 64, out_head, bi, r0);
       }
-      for (int it = 0; it < n_iter; ++it) {
+      int it = 0;
+      for (; it < n_iter; ++it) {
         const int ys = it % kS;
-        const int head = kDQ ? blockIdx.y / G : head0 + it / n_col;   // head of the streamed tiles
+        const int head = kDQ ? out_head / G : head0 + it / n_col;   // head of the streamed tiles
         const int c0 = (col_blk0 + it % n_col) * kBwdCols;
-        mbar_wait(&y_empty[ys], ((it / kS) & 1) ^ 1);
+        if (!wait_bar(&y_empty[ys], ((it / kS) & 1) ^ 1, failed)) break;
         mbar_arrive_expect_tx(&y_full[ys], 2 * L::kY + (kDQ ? 0 : 512));
         uint8_t* y1 = sY + ys * 2 * L::kY;
         uint8_t* y2 = y1 + L::kY;
@@ -508,193 +597,185 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
         }
         if (!kDQ) {
           const int64_t base = (static_cast<int64_t>(bi) * p.hq + head) * p.sq + c0;
-          bulk_load_1d(sStat + ys * 128, p.lse + base, 256, &y_full[ys]);
-          bulk_load_1d(sStat + ys * 128 + 64, p.delta + base, 256, &y_full[ys]);
+          bulk_load_1d(sStat + ys * 128, p.nlse + base, 256, &y_full[ys]);
+          bulk_load_1d(sStat + ys * 128 + 64, p.ndelta + base, 256, &y_full[ys]);
         }
       }
-    }
-  } else if (warp_idx == 1) {
-    // ============================================================ MMA issuer
-    if (lane == 0 && n_iter > 0) {
-      const uint32_t idesc_t = make_idesc_f16(p.is_bf16 != 0, kBwdRows, kBwdCols, false, false);
-      const uint32_t idesc_a = make_idesc_f16(p.is_bf16 != 0, kBwdRows, D, false, true);
+      if (*failed) {                                        // let the copies in flight land before the CTA ends
+        volatile int never = 0;
+        wait_bar(x_full, 0, &never);
+        for (int i = max(0, it - kS); i < it; ++i) wait_bar(&y_full[i % kS], (i / kS) & 1, &never);
+      }
+    } else if (warp_idx == 1 && n_iter > 0) {
+      // ============================================================ MMA issuer
+      constexpr uint32_t idesc_t = make_idesc_f16(kBf16, kBwdRows, kBwdCols, false, false);
+      constexpr uint32_t idesc_a = make_idesc_f16(kBf16, kBwdRows, D, false, true);
+      const uint64_t x_desc = make_smem_desc_sw128(smem_u32(sX1), 1024, 0), y_desc = make_smem_desc_sw128(smem_u32(sY), 1024, 0);
+      // streamed tile as MN-major B (N = d contiguous, K = its 64 rows)
+      const uint64_t yn_desc = make_smem_desc_sw128(smem_u32(sY), 1024, kBwdCols * 128);
+      auto commit = [&](uint64_t* bar) { if (elect_one()) umma_commit(bar); };
       auto issue_T = [&](int it) {
-        const int ys = it % kS, tb = it & 1;
-        const uint32_t x1 = smem_u32(sX1), x2 = smem_u32(sX2);
-        const uint32_t y1 = smem_u32(sY + ys * 2 * L::kY), y2 = y1 + L::kY;
+        const uint32_t tb = (it & 1) * 64;
+        const uint64_t y1 = desc_at(y_desc, (it % kS) * 2 * L::kY);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t xo = (k >> 2) * (kBwdRows * 128) + (k & 3) * 32;
-          const uint32_t yo = (k >> 2) * (kBwdCols * 128) + (k & 3) * 32;
-          umma_f16_ss(tmem_T1 + tb * 64, make_smem_desc_sw128(x1 + xo, 1024, 0), make_smem_desc_sw128(y1 + yo, 1024, 0),
-                      idesc_t, k != 0 ? 1u : 0u);
-        }
+          for (int x = 0; x < 2; ++x)
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t xo = (k >> 2) * (kBwdRows * 128) + (k & 3) * 32;
-          const uint32_t yo = (k >> 2) * (kBwdCols * 128) + (k & 3) * 32;
-          umma_f16_ss(tmem_T2 + tb * 64, make_smem_desc_sw128(x2 + xo, 1024, 0), make_smem_desc_sw128(y2 + yo, 1024, 0),
-                      idesc_t, k != 0 ? 1u : 0u);
+            for (int k = 0; k < D / 16; ++k) {
+              const uint32_t xo = x * (L::kX2Off - L::kX1Off) + (k >> 2) * (kBwdRows * 128) + (k & 3) * 32;
+              const uint32_t yo = x * L::kY + (k >> 2) * (kBwdCols * 128) + (k & 3) * 32;
+              umma_f16_ss((x == 0 ? tmem_T1 : tmem_T2) + tb, desc_at(x_desc, xo), desc_at(y1, yo), idesc_t, k != 0 ? 1u : 0u);
+            }
+          umma_commit(&t_full[it & 1]);
         }
-        umma_commit(&t_full[tb]);
       };
-      mbar_wait(x_full, 0);
-      mbar_wait(&y_full[0], 0);
-      tc_fence_after();
-      issue_T(0);
-      for (int it = 0; it < n_iter; ++it) {
+      bool ok = wait_bar_warp(x_full, 0, failed) && wait_bar_warp(&y_full[0], 0, failed);
+      if (ok) {
+        tc_fence_after();
+        issue_T(0);
+      }
+      for (int it = 0; it < n_iter && ok; ++it) {
         const int ys = it % kS, tb = it & 1;
         if (it + 1 < n_iter) {
-          mbar_wait(&y_full[(it + 1) % kS], ((it + 1) / kS) & 1);
+          ok = wait_bar_warp(&y_full[(it + 1) % kS], ((it + 1) / kS) & 1, failed);
+          if (!ok) break;
           tc_fence_after();
           issue_T(it + 1);     // overwrites T[(it+1)&1]: its P/dS were consumed by the accumulate MMAs of it-1
         }
-        mbar_wait(&pds_ready[tb], (it >> 1) & 1);
+        ok = wait_bar_warp(&pds_ready[tb], (it >> 1) & 1, failed);
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t y1 = smem_u32(sY + ys * 2 * L::kY), y2 = y1 + L::kY;
+        const uint64_t y1 = desc_at(yn_desc, ys * 2 * L::kY);
+        const uint32_t first = it != 0 ? 1u : 0u;
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < kBwdCols / 16; ++k) {
-          // streamed tile as MN-major B (N = d contiguous, K = its 64 rows); A = P / dS from TMEM
-          // (row = lane, 16 k-values = 8 packed 32-bit columns per step)
-          const uint64_t bdesc1 = make_smem_desc_sw128(y1 + k * 16 * 128, 1024, kBwdCols * 128);
-          if (kDQ) {
-            umma_f16_ts(tmem_A1, tmem_T2 + tb * 64 + k * 8, bdesc1, idesc_a, (it | k) != 0 ? 1u : 0u);
-          } else {
-            const uint64_t bdesc2 = make_smem_desc_sw128(y2 + k * 16 * 128, 1024, kBwdCols * 128);
-            umma_f16_ts(tmem_A1, tmem_T1 + tb * 64 + k * 8, bdesc2, idesc_a, (it | k) != 0 ? 1u : 0u);
-            umma_f16_ts(tmem_A2, tmem_T2 + tb * 64 + k * 8, bdesc1, idesc_a, (it | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < kBwdCols / 16; ++k) {
+            // A = P / dS from TMEM (row = lane, 16 k-values = 8 packed 32-bit columns per step)
+            const uint32_t acol = tb * 64 + (k >> 1) * 32 + (k & 1) * 8, acc = k != 0 ? 1u : first;
+            if (kDQ) {
+              umma_f16_ts(tmem_A1, tmem_T2 + acol, desc_at(y1, k * 16 * 128), idesc_a, acc);
+            } else {
+              umma_f16_ts(tmem_A1, tmem_T1 + acol, desc_at(y1, L::kY + k * 16 * 128), idesc_a, acc);
+              umma_f16_ts(tmem_A2, tmem_T2 + acol, desc_at(y1, k * 16 * 128), idesc_a, acc);
+            }
           }
+          umma_commit(&y_empty[ys]);
         }
-        umma_commit(&y_empty[ys]);
       }
-      umma_commit(acc_done);
+      if (ok) {
+        commit(acc_done);
+      } else {                                              // the MMAs in flight finish before TMEM is freed
+        volatile int never = 0;
+        commit(drained);
+        wait_bar_warp(drained, 0, &never);
+      }
     }
-  } else if (warp_idx >= 4) {
+  } else {
     // ============================================================ P / dS math + epilogue
+    regs_take<kMathRegs>();
+    const int wg = (warp_idx - 4) >> 2;
+    const int tb = wg >> 1, half = wg & 1;         // this warpgroup's blocks: it = tb, tb + 2, ...; its columns: 32 half .. 32 half + 31
     const int quad = warp_idx & 3;
     const int r = quad * 32 + lane;
     const int grow = r0 + r;                       // global row (key for dK/dV, query for dQ)
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const bool bf = p.is_bf16 != 0;
-    const float sc = p.scale_log2;
-    float row_lse2 = 0.f, row_delta = 0.f;         // dQ mode: statistics of this thread's query row
+    const uint64_t sc2 = f2(p.scale_log2, p.scale_log2);
+    uint64_t row_nlse = 0, row_ndelta = 0;         // dQ mode: statistics of this thread's query row
     if (kDQ) {
-      const int64_t idx = (static_cast<int64_t>(bi) * p.hq + blockIdx.y) * p.sq + min(grow, p.sq - 1);
-      row_lse2 = p.lse[idx];                       // already in the exp2 domain (-inf mapped to +inf)
-      row_delta = p.delta[idx];
+      const int64_t idx = (static_cast<int64_t>(bi) * p.hq + out_head) * p.sq + min(grow, p.sq - 1);
+      row_nlse = f2(p.nlse[idx], p.nlse[idx]);     // already in the exp2 domain (-inf for fully masked rows)
+      row_ndelta = f2(p.ndelta[idx], p.ndelta[idx]);
     }
+    const uint32_t a1 = tmem_T1 + tb * 64 + half * 32 + lane_addr, a2 = tmem_T2 + tb * 64 + half * 32 + lane_addr;
     // one streamed block: P = exp2(T1 * scale - lse2), dS = P * (T2 - delta), written back to TMEM
-    auto block = [&](int it, auto masked_tag) {
+    auto block = [&](int it, int c0, auto masked_tag) {
       constexpr bool kMasked = decltype(masked_tag)::value;
-      const int tb = it & 1, ys = it % kS;
-      const int c0 = (col_blk0 + it % n_col) * kBwdCols;
-      const float4* s_lse4 = reinterpret_cast<const float4*>(sStat + ys * 128);
-      const float4* s_delta4 = s_lse4 + 16;
-      const uint32_t a1 = tmem_T1 + tb * 64 + lane_addr, a2 = tmem_T2 + tb * 64 + lane_addr;
-      uint32_t t1[2][32], t2[2][32];
-      tmem_ld_32x32(a1, t1[0]);
-      tmem_ld_32x32(a2, t2[0]);
+      const ulonglong2* s_nlse = reinterpret_cast<const ulonglong2*>(sStat + (it % kS) * 128 + half * 32);
+      const ulonglong2* s_ndelta = s_nlse + 16;
+      uint32_t t1[2][16], t2[2][16];
+      tmem_ld_32x16(a1, t1[0]);
+      tmem_ld_32x16(a2, t2[0]);
+      tmem_ld_32x16(a1 + 16, t1[1]);
+      tmem_ld_32x16(a2 + 16, t2[1]);
+      tmem_ld_wait();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        tmem_ld_wait();
-        if (c == 0) {
-          tmem_ld_32x32(a1 + 32, t1[1]);
-          tmem_ld_32x32(a2 + 32, t2[1]);
-        }
-        uint32_t pk[16], dk[16];
+        uint32_t pk[8], dk[8];
 #pragma unroll
-        for (int i4 = 0; i4 < 8; ++i4) {
-          float l2[4], dl[4];
-          if (kDQ) {
+        for (int i4 = 0; i4 < 4; ++i4) {
+          ulonglong2 nl = make_ulonglong2(row_nlse, row_nlse), nd = make_ulonglong2(row_ndelta, row_ndelta);
+          if (!kDQ) { nl = s_nlse[c * 4 + i4]; nd = s_ndelta[c * 4 + i4]; }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { l2[e] = row_lse2; dl[e] = row_delta; }
-          } else {
-            const float4 a = s_lse4[c * 8 + i4], d4 = s_delta4[c * 8 + i4];
-            l2[0] = a.x; l2[1] = a.y; l2[2] = a.z; l2[3] = a.w;
-            dl[0] = d4.x; dl[1] = d4.y; dl[2] = d4.z; dl[3] = d4.w;
-          }
-          float pv[4], dv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = i4 * 4 + e;
-            float pe = fast_exp2(fmaf(__uint_as_float(t1[c][i]), sc, -l2[e]));
+          for (int e = 0; e < 2; ++e) {
+            const int i = i4 * 4 + e * 2;
+            float p0, p1, d0, d1;
+            un2(fma2(f2(__uint_as_float(t1[c][i]), __uint_as_float(t1[c][i + 1])), sc2, e == 0 ? nl.x : nl.y), p0, p1);
+            p0 = fast_exp2(p0);
+            p1 = fast_exp2(p1);
             if (kMasked) {
-              const int col = c0 + c * 32 + i;     // global column (query for dK/dV, key for dQ)
-              const int key = kDQ ? col : grow;
-              const int qry = kDQ ? grow : col;
-              if ((p.causal && key > qry) || key >= p.sk || qry >= p.sq) pe = 0.f;
+              const int col = c0 + half * 32 + c * 16 + i;     // global column (query for dK/dV, key for dQ)
+              auto hidden = [&](int cc) {
+                const int key = kDQ ? cc : grow, qry = kDQ ? grow : cc;
+                return (p.causal && key > qry) || key >= p.sk || qry >= p.sq;
+              };
+              if (hidden(col)) p0 = 0.f;
+              if (hidden(col + 1)) p1 = 0.f;
             }
-            pv[e] = pe;
-            dv[e] = pe * (__uint_as_float(t2[c][i]) - dl[e]);
+            un2(mul2(f2(p0, p1), add2(f2(__uint_as_float(t2[c][i]), __uint_as_float(t2[c][i + 1])), e == 0 ? nd.x : nd.y)), d0, d1);
+            if (!kDQ) pk[i >> 1] = pack16<kBf16>(p0, p1);
+            dk[i >> 1] = pack16<kBf16>(d0, d1);
           }
-          pk[i4 * 2] = pack16(pv[0], pv[1], bf);
-          pk[i4 * 2 + 1] = pack16(pv[2], pv[3], bf);
-          dk[i4 * 2] = pack16(dv[0], dv[1], bf);
-          dk[i4 * 2 + 1] = pack16(dv[2], dv[3], bf);
         }
-        // packed chunk c -> columns [16c, 16c+16) of the same accumulator buffer; only fp32 columns that
-        // are already in registers are overwritten (chunk 1 was loaded before chunk 0 is stored)
-        tmem_st_32x16(a2 + c * 16, dk);
-        if (!kDQ) tmem_st_32x16(a1 + c * 16, pk);
+        // packed chunk c -> columns [8c, 8c+8) of this half, whose fp32 values are in registers
+        tmem_st_32x8(a2 + c * 8, dk);
+        if (!kDQ) tmem_st_32x8(a1 + c * 8, pk);
       }
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&pds_ready[tb]);
     };
-    for (int it = 0; it < n_iter; ++it) {
-      const int tb = it & 1;
+    bool ok = true;
+    for (int it = tb; it < n_iter; it += 2) {
       const int c0 = (col_blk0 + it % n_col) * kBwdCols;
-      mbar_wait(&t_full[tb], (it >> 1) & 1);
+      ok = wait_bar_warp(&t_full[tb], (it >> 1) & 1, failed);
+      if (!ok) break;
       tc_fence_after();
       // masking: key index > query index is masked (causal); also ragged tails
       bool need_mask;
       if (kDQ) need_mask = (p.causal && c0 + kBwdCols - 1 > r0) || (c0 + kBwdCols > p.sk) || (r0 + kBwdRows > p.sq);
       else need_mask = (p.causal && c0 < r0 + kBwdRows - 1) || (c0 + kBwdCols > p.sq) || (r0 + kBwdRows > p.sk);
-      if (need_mask) block(it, std::true_type{});
-      else block(it, std::false_type{});
+      if (need_mask) block(it, c0, std::true_type{});
+      else block(it, c0, std::false_type{});
     }
-    if (n_iter > 0) {
-      mbar_wait(acc_done, 0);
+    if (n_iter > 0 && ok) ok = wait_bar_warp(acc_done, 0, failed);
+    if (ok) {
       tc_fence_after();
-    }
-    const int limit = kDQ ? p.sq : p.sk;
-    const bool valid = grow < limit;
-    const int oh = blockIdx.y;
-    auto store_acc = [&](uint32_t tacc, void* out, int64_t sb, int64_t sh, int64_t ss, float mul) {
-      uint8_t* orow = reinterpret_cast<uint8_t*>(out) +
-                      (static_cast<int64_t>(grow) * ss + static_cast<int64_t>(bi) * sb + static_cast<int64_t>(oh) * sh) * 2;
+      const int limit = kDQ ? p.sq : p.sk;
+      const bool valid = grow < limit;
+      auto store_acc = [&](uint32_t tacc, void* out, int64_t sb, int64_t sh, int64_t ss, float mul, int ch0, int ch1) {
+        uint8_t* orow = reinterpret_cast<uint8_t*>(out) +
+                        (static_cast<int64_t>(grow) * ss + static_cast<int64_t>(bi) * sb + static_cast<int64_t>(out_head) * sh) * 2;
+        for (int c = ch0; c < ch1; ++c) {
+          uint32_t v[32];
+          if (n_iter > 0) {
+            tmem_ld_32x32(tacc + c * 32 + lane_addr, v);
+            tmem_ld_wait();
+          } else {
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t v[32];
-        if (n_iter > 0) {
-          tmem_ld_32x32(tacc + c * 32 + lane_addr, v);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = 0u;
-        }
-        if (valid) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 w;
-            w.x = pack16(__uint_as_float(v[u * 8 + 0]) * mul, __uint_as_float(v[u * 8 + 1]) * mul, bf);
-            w.y = pack16(__uint_as_float(v[u * 8 + 2]) * mul, __uint_as_float(v[u * 8 + 3]) * mul, bf);
-            w.z = pack16(__uint_as_float(v[u * 8 + 4]) * mul, __uint_as_float(v[u * 8 + 5]) * mul, bf);
-            w.w = pack16(__uint_as_float(v[u * 8 + 6]) * mul, __uint_as_float(v[u * 8 + 7]) * mul, bf);
-            *reinterpret_cast<uint4*>(orow + c * 64 + u * 16) = w;
+            for (int i = 0; i < 32; ++i) v[i] = 0u;
           }
+          if (valid) store_row32<kBf16>(orow + c * 64, v, mul);
         }
-      }
-    };
-    if (kDQ) {
-      store_acc(tmem_A1, p.out1, p.o1_sb, p.o1_sh, p.o1_ss, p.scale);
-    } else {
-      store_acc(tmem_A1, p.out1, p.o1_sb, p.o1_sh, p.o1_ss, 1.f);
-      store_acc(tmem_A2, p.out2, p.o2_sb, p.o2_sh, p.o2_ss, p.scale);
+      };
+      // the warpgroups share the epilogue: 32 columns of dQ each, or half of dV's or dK's
+      if (kDQ) store_acc(tmem_A1, p.out1, p.o1_sb, p.o1_sh, p.o1_ss, p.scale, min(wg, D / 32), min(wg + 1, D / 32));
+      else if (tb == 0) store_acc(tmem_A1, p.out1, p.o1_sb, p.o1_sh, p.o1_ss, 1.f, half * (D / 64), (half + 1) * (D / 64));
+      else store_acc(tmem_A2, p.out2, p.o2_sb, p.o2_sh, p.o2_ss, p.scale, half * (D / 64), (half + 1) * (D / 64));
     }
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *failed) atomicExch(&g_attn_error, 1);
   if (warp_idx == 2) tmem_dealloc<512>(tmem_base);
 }
 
@@ -714,14 +795,14 @@ EncodeFn encode_fn() {
   });
   return fn;
 }
-thread_local std::string g_attn_error;
+thread_local std::string g_attn_err;
 
 // 4-D map over a strided [b, h, s, d] view: dims (d, h, b, s); box (64, 1, 1, rows)
 bool make_tmap_bhsd(CUtensorMap* map, const void* base, bool is_bf16, int d, int h, int b, int s, int64_t sh,
                     int64_t sb, int64_t ss, int rows) {
   ensure_cuda_context();
   EncodeFn fn = encode_fn();
-  if (!fn) { g_attn_error = "cuTensorMapEncodeTiled unavailable"; return false; }
+  if (!fn) { g_attn_err = "cuTensorMapEncodeTiled unavailable"; return false; }
   cuuint64_t dims[4] = {static_cast<cuuint64_t>(d), static_cast<cuuint64_t>(h), static_cast<cuuint64_t>(b),
                         static_cast<cuuint64_t>(s)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(sh) * 2, static_cast<cuuint64_t>(sb) * 2,
@@ -732,7 +813,20 @@ bool make_tmap_bhsd(CUtensorMap* map, const void* base, bool is_bf16, int d, int
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    g_attn_error = "cuTensorMapEncodeTiled(4d) failed: code " + std::to_string(static_cast<int>(r));
+    g_attn_err = "cuTensorMapEncodeTiled(4d) failed: code " + std::to_string(static_cast<int>(r));
+    return false;
+  }
+  return true;
+}
+
+// once per kernel: its shared memory, and that its register shares (regs_take / regs_give) fit what it is launched with
+template <typename K>
+bool prepare_kernel(K kern, int smem, const char* name) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) { g_attn_err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return false; }
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs * kThreads < 512 * kMathRegs + 128 * kIssueRegs) {
+    g_attn_err = std::string(name) + ": built with too few registers for its warpgroups' shares";
     return false;
   }
   return true;
@@ -742,33 +836,30 @@ bool strides_ok(int64_t sb, int64_t sh, int64_t ss, const void* ptr) {
   return (sb % 8 == 0) && (sh % 8 == 0) && (ss % 8 == 0) && (reinterpret_cast<uintptr_t>(ptr) % 16 == 0);
 }
 
-template <int D, bool kPTmem>
+template <int D, bool kBf16>
 int launch_fwd(const AttnArgs& a, cudaStream_t s) {
-  using L = FwdSmem<D, kPTmem>;
+  using L = FwdSmem<D>;
   CUtensorMap tq{}, tk{}, tv{};
   if (!make_tmap_bhsd(&tq, a.q, a.is_bf16, D, a.hq, a.b, a.sq, a.q_sh, a.q_sb, a.q_ss, kBlockQ)) return -5;
   if (!make_tmap_bhsd(&tk, a.k, a.is_bf16, D, a.hkv, a.b, a.sk, a.k_sh, a.k_sb, a.k_ss, kBlockKV)) return -5;
   if (!make_tmap_bhsd(&tv, a.v, a.is_bf16, D, a.hkv, a.b, a.sk, a.v_sh, a.v_sb, a.v_ss, kBlockKV)) return -5;
-  auto kern = attn_fwd_kernel<D, kPTmem>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
-    if (e != cudaSuccess) { g_attn_error = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return -10; }
-    attr_set = true;
-  }
+  auto kern = attn_fwd_kernel<D, kBf16>;
+  static const bool ready = prepare_kernel(kern, L::kTotal, "attn_fwd");
+  if (!ready) return -10;
   FwdParams p{};
   p.lse = a.lse; p.o = a.o; p.o_sb = a.o_sb; p.o_sh = a.o_sh; p.o_ss = a.o_ss;
   p.b = a.b; p.hq = a.hq; p.hkv = a.hkv; p.sq = a.sq; p.sk = a.sk;
-  p.scale_log2 = a.scale * kLog2e; p.causal = a.causal ? 1 : 0; p.is_bf16 = a.is_bf16 ? 1 : 0;
-  dim3 grid((a.sq + 2 * kBlockQ - 1) / (2 * kBlockQ), a.hq, a.b);
-  kern<<<grid, 384, L::kTotal, s>>>(tq, tk, tv, p);
+  p.scale_log2 = a.scale * kLog2e; p.causal = a.causal ? 1 : 0;
+  const int64_t ctas = static_cast<int64_t>((a.sq + 2 * kBlockQ - 1) / (2 * kBlockQ)) * a.hq * a.b;
+  if (ctas > 0x7fffffff) { g_attn_err = "too many query blocks"; return -12; }
+  kern<<<static_cast<unsigned>(ctas), kThreads, L::kTotal, s>>>(tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { g_attn_error = std::string("attn_fwd launch: ") + cudaGetErrorString(e); return -11; }
+  if (e != cudaSuccess) { g_attn_err = std::string("attn_fwd launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
 }
 
 
-template <int D, bool kDQ>
+template <int D, bool kDQ, bool kBf16>
 int launch_bwd_one(const AttnArgs& a, cudaStream_t s) {
   using L = BwdSmem<D, kDQ>;
   CUtensorMap x1{}, x2{}, y1{}, y2{};
@@ -785,72 +876,68 @@ int launch_bwd_one(const AttnArgs& a, cudaStream_t s) {
     ok = ok && make_tmap_bhsd(&y2, a.d_o, a.is_bf16, D, a.hq, a.b, a.sq, a.do_sh, a.do_sb, a.do_ss, kBwdCols);
   }
   if (!ok) return -5;
-  auto kern = attn_bwd_kernel<D, kDQ>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
-    if (e != cudaSuccess) { g_attn_error = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return -10; }
-    attr_set = true;
-  }
+  auto kern = attn_bwd_kernel<D, kDQ, kBf16>;
+  static const bool ready = prepare_kernel(kern, L::kTotal, "attn_bwd");
+  if (!ready) return -10;
   BwdParams p{};
-  p.lse = a.delta + static_cast<int64_t>(a.b) * a.hq * a.sq;   // exp2-domain LSE written by attn_delta_kernel
-  p.delta = a.delta;
+  p.nlse = a.delta + static_cast<int64_t>(a.b) * a.hq * a.sq;   // written by attn_delta_kernel
+  p.ndelta = a.delta;
   if (kDQ) { p.out1 = a.dq; p.o1_sb = a.dq_sb; p.o1_sh = a.dq_sh; p.o1_ss = a.dq_ss; }
   else {
     p.out1 = a.dv; p.o1_sb = a.dv_sb; p.o1_sh = a.dv_sh; p.o1_ss = a.dv_ss;
     p.out2 = a.dk; p.o2_sb = a.dk_sb; p.o2_sh = a.dk_sh; p.o2_ss = a.dk_ss;
   }
   p.b = a.b; p.hq = a.hq; p.hkv = a.hkv; p.sq = a.sq; p.sk = a.sk;
-  p.scale_log2 = a.scale * kLog2e; p.scale = a.scale; p.causal = a.causal ? 1 : 0; p.is_bf16 = a.is_bf16 ? 1 : 0;
-  dim3 grid(kDQ ? (a.sq + kBwdRows - 1) / kBwdRows : (a.sk + kBwdRows - 1) / kBwdRows, kDQ ? a.hq : a.hkv, a.b);
-  kern<<<grid, 256, L::kTotal, s>>>(x1, x2, y1, y2, p);
+  p.scale_log2 = a.scale * kLog2e; p.scale = a.scale; p.causal = a.causal ? 1 : 0;
+  const int64_t ctas = static_cast<int64_t>(((kDQ ? a.sq : a.sk) + kBwdRows - 1) / kBwdRows) * (kDQ ? a.hq : a.hkv) * a.b;
+  if (ctas > 0x7fffffff) { g_attn_err = "too many row blocks"; return -12; }
+  kern<<<static_cast<unsigned>(ctas), kThreads, L::kTotal, s>>>(x1, x2, y1, y2, p);
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { g_attn_error = std::string("attn_bwd launch: ") + cudaGetErrorString(e); return -11; }
+  if (e != cudaSuccess) { g_attn_err = std::string("attn_bwd launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
 }
 
 template <int D>
 int launch_bwd(const AttnArgs& a, cudaStream_t s) {
   const int64_t rows = static_cast<int64_t>(a.b) * a.hq * a.sq;
-  attn_delta_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, s>>>(
-      a.o, a.d_o, a.delta, a.lse, a.delta + rows, a.b, a.hq, a.sq, D, a.o_sb, a.o_sh, a.o_ss, a.do_sb, a.do_sh, a.do_ss, a.is_bf16 ? 1 : 0);
-  int rc = launch_bwd_one<D, false>(a, s);
+  constexpr int kPerBlock = 8 * 4 * (256 / D);   // warps x row groups x rows
+  if (a.hq > 65535 || a.b > 65535) { g_attn_err = "too many heads or sequences"; return -12; }
+  attn_delta_kernel<D><<<dim3((a.sq + kPerBlock - 1) / kPerBlock, a.hq, a.b), 256, 0, s>>>(
+      static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.d_o), a.delta, a.lse, a.delta + rows, a.hq, a.sq, a.o_sb, a.o_sh, a.o_ss,
+      a.do_sb, a.do_sh, a.do_ss, a.is_bf16 ? 1 : 0);
+  int rc = a.is_bf16 ? launch_bwd_one<D, false, true>(a, s) : launch_bwd_one<D, false, false>(a, s);
   if (rc != 0) return rc;
-  return launch_bwd_one<D, true>(a, s);
+  return a.is_bf16 ? launch_bwd_one<D, true, true>(a, s) : launch_bwd_one<D, true, false>(a, s);
 }
 
 }  // namespace
 
-const char* attn_last_error() { return g_attn_error.c_str(); }
+const char* attn_last_error() { return g_attn_err.c_str(); }
 
 int attn_fwd(const AttnArgs& a, cudaStream_t s) {
-  if (a.d != 64 && a.d != 128) { g_attn_error = "head dim must be 64 or 128"; return -1; }
-  if (a.hq % a.hkv != 0) { g_attn_error = "hq must be a multiple of hkv"; return -1; }
-  if (a.causal && a.sq != a.sk) { g_attn_error = "causal attention needs sq == sk"; return -2; }
-  if (a.probs_out) { g_attn_error = "probability export uses the materialising path"; return -3; }
+  if (a.d != 64 && a.d != 128) { g_attn_err = "head dim must be 64 or 128"; return -1; }
+  if (a.hq % a.hkv != 0) { g_attn_err = "hq must be a multiple of hkv"; return -1; }
+  if (a.causal && a.sq != a.sk) { g_attn_err = "causal attention needs sq == sk"; return -2; }
+  if (a.probs_out) { g_attn_err = "probability export uses the materialising path"; return -3; }
   if (!strides_ok(a.q_sb, a.q_sh, a.q_ss, a.q) || !strides_ok(a.k_sb, a.k_sh, a.k_ss, a.k) ||
       !strides_ok(a.v_sb, a.v_sh, a.v_ss, a.v) || !strides_ok(a.o_sb, a.o_sh, a.o_ss, a.o)) {
-    g_attn_error = "q/k/v/o need 16-byte aligned base and strides";
+    g_attn_err = "q/k/v/o need 16-byte aligned base and strides";
     return -4;
   }
-  static const bool p_tmem = [] {
-    const char* e = getenv("B200_ATTN_P_TMEM");
-    return e == nullptr || e[0] != '0';
-  }();
-  if (p_tmem) return a.d == 128 ? launch_fwd<128, true>(a, s) : launch_fwd<64, true>(a, s);
+  if (a.is_bf16) return a.d == 128 ? launch_fwd<128, true>(a, s) : launch_fwd<64, true>(a, s);
   return a.d == 128 ? launch_fwd<128, false>(a, s) : launch_fwd<64, false>(a, s);
 }
 
 int attn_bwd(const AttnArgs& a, cudaStream_t s) {
-  if (a.d != 64 && a.d != 128) { g_attn_error = "head dim must be 64 or 128"; return -1; }
-  if (a.hq % a.hkv != 0) { g_attn_error = "hq must be a multiple of hkv"; return -1; }
-  if (a.causal && a.sq != a.sk) { g_attn_error = "causal attention needs sq == sk"; return -2; }
-  if (a.sq % kBwdCols != 0 || a.sk % kBwdCols != 0) { g_attn_error = "backward needs sq, sk multiples of 64"; return -3; }
+  if (a.d != 64 && a.d != 128) { g_attn_err = "head dim must be 64 or 128"; return -1; }
+  if (a.hq % a.hkv != 0) { g_attn_err = "hq must be a multiple of hkv"; return -1; }
+  if (a.causal && a.sq != a.sk) { g_attn_err = "causal attention needs sq == sk"; return -2; }
+  if (a.sq % kBwdCols != 0 || a.sk % kBwdCols != 0) { g_attn_err = "backward needs sq, sk multiples of 64"; return -3; }
   if (!strides_ok(a.q_sb, a.q_sh, a.q_ss, a.q) || !strides_ok(a.k_sb, a.k_sh, a.k_ss, a.k) ||
       !strides_ok(a.v_sb, a.v_sh, a.v_ss, a.v) || !strides_ok(a.o_sb, a.o_sh, a.o_ss, a.o) ||
       !strides_ok(a.do_sb, a.do_sh, a.do_ss, a.d_o) || !strides_ok(a.dq_sb, a.dq_sh, a.dq_ss, a.dq) ||
       !strides_ok(a.dk_sb, a.dk_sh, a.dk_ss, a.dk) || !strides_ok(a.dv_sb, a.dv_sh, a.dv_ss, a.dv)) {
-    g_attn_error = "attention operands need 16-byte aligned base and strides";
+    g_attn_err = "attention operands need 16-byte aligned base and strides";
     return -4;
   }
   return a.d == 128 ? launch_bwd<128>(a, s) : launch_bwd<64>(a, s);
