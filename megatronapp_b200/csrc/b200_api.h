@@ -293,14 +293,24 @@ struct PagedAttnArgs {
   const int32_t* block_table;  // [R, max_blocks]
   const int32_t* tok_req;   // [T] row of block_table
   const int32_t* tok_len;   // [T] keys visible to the token (its position + 1)
-  float* ws_o;              // [T * heads * splits, d]   (splits > 1)
-  float* ws_ml;             // [T * heads * splits, 2]
+  const int32_t* cu;        // [n_seqs + 1] tokens of one request lie side by side (nullptr: each token by itself)
+  int n_seqs;
   int n_tokens, ng, group, head_dim, block_size, max_blocks;
   float scale_log2;
   bool is_bf16;
 };
+struct PagedWriteArgs {
+  const void *k, *v;        // [T, ng, d], strides below in elements, multiples of 8; last dim contiguous
+  void *k_cache, *v_cache;  // [n_slots, ng, d]
+  const int64_t* slots;     // [T]
+  int64_t k_st, k_sh, v_st, v_sh;
+  int n_tokens, ng, head_dim;
+};
 bool paged_attention_supported(int head_dim, int group);
-void paged_attention(const PagedAttnArgs& a, int splits, cudaStream_t s);
+void paged_write(const PagedWriteArgs& w, cudaStream_t s);
+int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
+int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s);
+const char* paged_attention_last_error();
 
 // ---------------------------------------------------------------- MoE (moe.cu)
 void moe_router_topk_fwd(const float* logits, float* probs, uint8_t* map, int32_t* tokens_per_expert, int n, int E, int k,

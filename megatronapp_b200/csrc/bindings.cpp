@@ -870,16 +870,36 @@ void embed_scatter(const Tensor& tokens, const Tensor& weight, std::vector<int64
   b200::embed_scatter(a, cur_stream());
   count();
 }
+// k_new / v_new [T, ng, d] are written to their cache rows `slots` first.  With cu (int32 [R + 1]) the tokens of a request share its
+// keys: chunk_tiles is the number of tiles of 64 / group tokens over the requests with more than 16 / group new tokens, cut into
+// chunk_splits key ranges each; splits <= 0 then says that there are no other requests (how theirs are cut up is the kernel's own business).
 Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& block_table,
-                       const Tensor& tok_req, const Tensor& tok_len, int64_t block_size, double scale, int64_t splits) {
+                       const Tensor& tok_req, const Tensor& tok_len, int64_t block_size, double scale, int64_t splits,
+                       const c10::optional<Tensor>& k_new, const c10::optional<Tensor>& v_new, const c10::optional<Tensor>& slots,
+                       const c10::optional<Tensor>& cu, int64_t chunk_tiles, int64_t chunk_splits) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && k_cache.dim() == 3 && k_cache.is_contiguous() && v_cache.is_contiguous());
   TORCH_CHECK(q.scalar_type() == k_cache.scalar_type() && (is_bf16(q) || q.scalar_type() == at::kHalf));
   TORCH_CHECK(block_table.scalar_type() == at::kInt && tok_req.scalar_type() == at::kInt && tok_len.scalar_type() == at::kInt);
   TORCH_CHECK(block_table.dim() == 2 && block_table.is_contiguous() && v_cache.sizes() == k_cache.sizes());
+  TORCH_CHECK(v_cache.scalar_type() == q.scalar_type() && tok_req.is_contiguous() && tok_len.is_contiguous() && block_size > 0);
   const int T = static_cast<int>(q.size(0)), np = static_cast<int>(q.size(1)), d = static_cast<int>(q.size(2));
   const int ng = static_cast<int>(k_cache.size(1));
+  TORCH_CHECK(tok_req.numel() >= T && tok_len.numel() >= T, "tok_req / tok_len must cover every token");
   TORCH_CHECK(np % ng == 0 && k_cache.size(2) == d && b200::paged_attention_supported(d, np / ng), "unsupported paged attention shape");
+  for (const Tensor* t : {&q, &k_cache, &v_cache}) TORCH_CHECK(reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "operands must be 16-byte aligned");
+  if (k_new.has_value() && T > 0) {
+    TORCH_CHECK(v_new.has_value() && slots.has_value() && slots->scalar_type() == at::kLong && slots->is_contiguous() && slots->numel() == T);
+    b200::PagedWriteArgs w{};
+    for (const Tensor* t : {&*k_new, &*v_new})
+      TORCH_CHECK(t->dim() == 3 && t->size(0) == T && t->size(1) == ng && t->size(2) == d && t->scalar_type() == q.scalar_type() && t->stride(2) == 1 &&
+                  t->stride(0) % 8 == 0 && t->stride(1) % 8 == 0 && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "bad new keys or values");
+    w.k = k_new->data_ptr(); w.v = v_new->data_ptr(); w.k_cache = k_cache.data_ptr(); w.v_cache = v_cache.data_ptr();
+    w.slots = slots->data_ptr<int64_t>(); w.k_st = k_new->stride(0); w.k_sh = k_new->stride(1); w.v_st = v_new->stride(0); w.v_sh = v_new->stride(1);
+    w.n_tokens = T; w.ng = ng; w.head_dim = d;
+    b200::paged_write(w, cur_stream());
+    count();
+  }
   auto out = at::empty_like(q);
   b200::PagedAttnArgs a{};
   a.q = q.data_ptr(); a.k_cache = k_cache.data_ptr(); a.v_cache = v_cache.data_ptr(); a.out = out.data_ptr();
@@ -887,14 +907,18 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
   a.n_tokens = T; a.ng = ng; a.group = np / ng; a.head_dim = d; a.block_size = static_cast<int>(block_size);
   a.max_blocks = static_cast<int>(block_table.size(1)); a.scale_log2 = static_cast<float>(scale * 1.4426950408889634);
   a.is_bf16 = is_bf16(q);
-  Tensor ws_o, ws_ml;
-  if (splits > 1) {
-    ws_o = at::empty({static_cast<int64_t>(T) * np * splits, d}, q.options().dtype(at::kFloat));
-    ws_ml = at::empty({static_cast<int64_t>(T) * np * splits, 2}, q.options().dtype(at::kFloat));
-    a.ws_o = ws_o.data_ptr<float>(); a.ws_ml = ws_ml.data_ptr<float>();
+  if (cu.has_value()) {
+    TORCH_CHECK(cu->scalar_type() == at::kInt && cu->is_contiguous() && cu->numel() >= 1, "cu must be int32");
+    a.cu = cu->data_ptr<int32_t>(); a.n_seqs = static_cast<int>(cu->numel()) - 1;
   }
-  if (T > 0) b200::paged_attention(a, static_cast<int>(splits), cur_stream());
-  count();
+  if (T == 0) return out;
+  const bool decode = !cu.has_value() || splits > 0;
+  Tensor ws;
+  if (decode) ws = at::empty({b200::paged_decode_workspace(a)}, q.options().dtype(at::kFloat));
+  const int rc = b200::paged_attention(a, decode, static_cast<int>(chunk_tiles), static_cast<int>(chunk_splits), decode ? ws.data_ptr<float>() : nullptr,
+                                       cur_stream());
+  TORCH_CHECK(rc == 0, "b200 paged_attention failed: ", rc, " ", b200::paged_attention_last_error());
+  count((decode ? 2 : 0) + (cu.has_value() && chunk_tiles > 0 ? 1 : 0));
   return out;
 }
 bool paged_attention_supported(int64_t head_dim, int64_t group) { return b200::paged_attention_supported(static_cast<int>(head_dim), static_cast<int>(group)); }
@@ -1085,7 +1109,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("shard_all_gather_cast", &shard_all_gather_cast);
   m.def("a2a_scatter_rows", &a2a_scatter_rows);
   m.def("embed_scatter", &embed_scatter);
-  m.def("paged_attention", &paged_attention);
+  m.def("paged_attention", &paged_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"), py::arg("tok_req"),
+        py::arg("tok_len"), py::arg("block_size"), py::arg("scale"), py::arg("splits"), py::arg("k_new") = py::none(), py::arg("v_new") = py::none(),
+        py::arg("slots") = py::none(), py::arg("cu") = py::none(), py::arg("chunk_tiles") = 0, py::arg("chunk_splits") = 1);
   m.def("paged_attention_supported", &paged_attention_supported);
   m.def("spin", &spin);
   m.def("write_flag", &write_flag);

@@ -3,188 +3,684 @@
 // One step of the engine carries a ragged mix of queries: single decode tokens of running requests and chunks of prompt
 // tokens of requests being prefilled.  Every query token t belongs to request r = tok_req[t] and sees the first
 // tok_len[t] keys of that request; keys live in fixed-size pages of a shared pool, found through the request's block
-// table.  A CTA owns one (query token, KV head) pair -- all G query heads of the group, so each key/value row is read
-// from HBM once per group -- and, for long contexts, one of `splits` key ranges; partial (max, sum, accumulator)
-// triples are merged by a second tiny kernel (flash-decoding).  Decode attention moves 2 * len * d * 2 bytes per
-// (token, KV head) and does O(G) flops per byte: it is HBM bound, so the kernel is built around 16-byte loads with
-// several keys in flight per warp, not around the tensor cores.
+// table.
+//
+// A tile is up to 16 or 64 rows, a row being one (token, query head) of one request and one KV head: all query heads of a group share
+// every key/value row that is read, and so do the tokens of a chunk.  Keys come in stages of 64, gathered page by page into a ring of
+// shared-memory buffers by 16-byte asynchronous copies (32 KB each at d = 128), and are
+// multiplied by m16n8k16 tensor instructions from there.  The weights stay exact to about 16 bits: each enters the value product as a 16-bit
+// part and the rest of it, so the result carries fp32 sums of fp32 weights as far as its 16-bit output can show.
+//   rows = 16 (decode, short chunks): the four warps take 16 keys of a stage each, bound by HBM.  The stages of all (request, KV head)
+//     pairs stand in one line that is cut evenly over three CTAs per SM, whatever the contexts' lengths; an item that a cut falls into
+//     leaves partial (max, sum, accumulator) triples, which a small second kernel merges.  64 contexts of 1k to 4k, 32 / 8 heads of 128:
+//     117 us, 5.7 TB/s, the rest latency of one stage's dependent steps (138 with three stages and two CTAs per SM; 456 with a key per 16
+//     lanes and no load in flight behind it).
+//   rows = 64 (chunks): a warp takes 16 rows and all keys of a stage, longest tiles first, bound by the tensor instructions.  Where the
+//     tiles are few and the context is long, the CTAs of a cluster take key ranges and merge through distributed shared memory.  Two
+//     chunks of 500 tokens beside 24 decoding requests: 865 us before, every token reading all its keys, 57 + 39 us now.
 //
 // Replaces the reference's dynamic-context attention (core/inference/contexts/dynamic_context.py + flash_attn_with_kvcache
 // in attention.py:590-603) and this repo's earlier gather + einsum path (inference/dynamic.py).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <string>
 
 #include "b200_api.h"
 #include "common.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace b200 {
 namespace {
 
-template <bool kBf16>
-__device__ __forceinline__ void unpack8(const int4& r, float (&f)[8]) {
-  const uint32_t w[4] = {static_cast<uint32_t>(r.x), static_cast<uint32_t>(r.y), static_cast<uint32_t>(r.z), static_cast<uint32_t>(r.w)};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    if constexpr (kBf16) {
-      f[2 * i] = __uint_as_float(w[i] << 16);
-      f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    } else {
-      const __half2 h = *reinterpret_cast<const __half2*>(&w[i]);
-      const float2 v = __half22float2(h);
-      f[2 * i] = v.x;
-      f[2 * i + 1] = v.y;
-    }
-  }
-}
+thread_local std::string g_paged_err;
+
+constexpr int kStageKeys = 64;
+constexpr int kDecodeCtas = 3 * 148;
 
 template <bool kBf16>
-__device__ __forceinline__ void store_out(void* base, int64_t idx, float v) {
-  if constexpr (kBf16) reinterpret_cast<__nv_bfloat16*>(base)[idx] = __float2bfloat16(v);
-  else reinterpret_cast<__half*>(base)[idx] = __float2half(v);
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  if constexpr (kBf16) return pack_bf16x2(lo, hi);
+  __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&h);
 }
+template <bool kBf16>
+__device__ __forceinline__ float2 unpack2(uint32_t v) {
+  if constexpr (kBf16) return unpack_bf16x2(v);
+  return __half22float2(*reinterpret_cast<const __half2*>(&v));
+}
+// c[16 x 8] += a[16 x 16] b[16 x 8]
+template <bool kBf16>
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (kBf16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// 16 bytes, zeros when !valid (the source is not read then)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int D, int G, bool kBf16>
-__global__ void __launch_bounds__(128) paged_attn_kernel(PagedAttnArgs a) {
-  constexpr int kLPK = D / 8;        // lanes that share one key row (16 B each)
-  constexpr int kKPW = 32 / kLPK;    // keys per warp per iteration
-  constexpr int kGroups = 4 * kKPW;  // key groups per CTA
-  const int t = blockIdx.x, hk = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z;
-  const int r = a.tok_req[t];
-  const int len = a.tok_len[t];
-  const int per = ((len + nsplit - 1) / nsplit + kGroups - 1) / kGroups * kGroups;
-  const int k0 = split * per, k1 = min(len, k0 + per);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int lk = lane % kLPK, grp = warp * kKPW + lane / kLPK;
-  // the key groups of a warp run different trip counts at the tail of a context: shuffles name only the group's lanes
-  const unsigned gmask = (kLPK == 32) ? 0xffffffffu : (((1u << kLPK) - 1u) << (lane / kLPK * kLPK));
-  const int np = a.ng * G;
+template <int D>
+struct Smem {
+  static constexpr int kPitch = D * 2 + 16;                          // bytes of a padded row: conflict-free ldmatrix
+  static constexpr int kStage = 2 * kStageKeys * kPitch;             // K rows, then V rows
+  static constexpr int kStages = D == 128 ? 2 : 3;
+  static constexpr int kStatOff = kStages * kStage;                  // max and sum of [4 warps][16] or 64 rows
+  static constexpr int kTotal = kStatOff + 2 * 64 * 4;
+  static_assert(64 * D * 4 <= kStatOff, "after the last stage, partial accumulators reuse the ring");
+};
 
-  __shared__ float s_m[kGroups][G], s_l[kGroups][G];
-  __shared__ float s_acc[kGroups][G][D];
+struct PagedParams {
+  PagedAttnArgs a;
+  int group_shift, bs_shift;   // log2 of the group; of the block size, or -1
+  int n_tiles;                 // chunks: tiles of this launch (its grid is n_tiles * ng * splits); decode: requests
+  int splits;                  // chunks: key ranges of a tile; decode: CTAs
+  float* ws;                   // decode: two partials of 16 rows x (d + 2) per CTA
+};
 
-  // this lane's 8 dims of every query head of the group, pre-scaled into the exp2 domain
-  float q[G][8];
-  {
-    const uint16_t* qp = reinterpret_cast<const uint16_t*>(a.q) + (static_cast<int64_t>(t) * np + hk * G) * D + lk * 8;
+// One tile's keys k0 .. k1 - 1 (stages aligned to k0): running maximum, sum and accumulator of this warp's rows g and g + 8.  RW row
+// tiles of 16 share the CTA's four warps, the others split the keys of a stage.
+template <int D, bool kBf16, int RW>
+struct Tile {
+  static constexpr int kWarpKeys = kStageKeys / (4 / RW), kNT = kWarpKeys / 8, kChunks = D / 8;
+  using L = Smem<D>;
+  float m[2], l[2], o[D / 8][4];
+
+  __device__ __forceinline__ void run(const PagedParams& p, uint8_t* smem, const int32_t* bt, int hk, int t0, int n, int min_vis, int k0, int k1) {
+    const PagedAttnArgs& a = p.a;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tg = lane & 3;
+    const int G = 1 << p.group_shift, np = a.ng << p.group_shift, n_rows = n << p.group_shift;
+    const int n_stages = k1 > k0 ? (k1 - k0 + kStageKeys - 1) / kStageKeys : 0;
+    // ---- gather of one stage into its ring buffer
+    const uint32_t ring = smem_u32(smem);
+    auto load = [&](int st) {
+      const uint32_t dst = ring + (st % L::kStages) * L::kStage + (tid % kChunks) * 16;
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      const int4 raw = *reinterpret_cast<const int4*>(qp + g * D);
-      unpack8<kBf16>(raw, q[g]);
+      for (int i = 0; i < kStageKeys * kChunks / 128; ++i) {
+        const int row = i * (128 / kChunks) + tid / kChunks, key = k0 + st * kStageKeys + row;
+        const bool valid = key < k1;
+        const int kk = valid ? key : k0;
+        const int blk = p.bs_shift >= 0 ? kk >> p.bs_shift : kk / a.block_size;
+        const int64_t slot = static_cast<int64_t>(bt[blk]) * a.block_size + (kk - blk * a.block_size);
+        const int64_t off = (slot * a.ng + hk) * D + (tid % kChunks) * 8;
+        cp_async16(dst + row * L::kPitch, static_cast<const uint16_t*>(a.k_cache) + off, valid);
+        cp_async16(dst + (kStageKeys + row) * L::kPitch, static_cast<const uint16_t*>(a.v_cache) + off, valid);
+      }
+    };
 #pragma unroll
-      for (int j = 0; j < 8; ++j) q[g][j] *= a.scale_log2;
+    for (int st = 0; st < L::kStages - 1; ++st) {
+      if (st < n_stages) load(st);
+      cp_async_commit();
+    }
+
+    // ---- queries of this warp's rows g and g + 8, as A fragments
+    const int wrow = RW == 1 ? 0 : warp * 16, wkey = RW == 1 ? warp * kWarpKeys : 0;
+    uint32_t qf[D / 16][4];
+    int vis[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = wrow + g + i * 8;
+      const bool valid = row < n_rows;
+      const int t = t0 + (valid ? row >> p.group_shift : 0);
+      vis[i] = valid ? a.tok_len[t] : 0;
+      const uint32_t* qp = reinterpret_cast<const uint32_t*>(static_cast<const uint16_t*>(a.q) +
+                                                             (static_cast<int64_t>(t) * np + hk * G + (valid ? row & (G - 1) : 0)) * D) + tg;
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        qf[k][i] = valid ? qp[k * 8] : 0u;
+        qf[k][i + 2] = valid ? qp[k * 8 + 4] : 0u;
+      }
+    }
+    m[0] = m[1] = -INFINITY;
+    l[0] = l[1] = 0.f;
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+    const float sc = a.scale_log2;
+    // ldmatrix row addresses: K in pairs of 8-key groups and 8-column groups, V in pairs of 8-column groups (transposed)
+    const uint32_t k_off = (wkey + (lane & 7) + ((lane >> 4) << 3)) * L::kPitch + ((lane >> 3) & 1) * 16;
+    const uint32_t v_off = (kStageKeys + wkey + (lane & 15)) * L::kPitch + (lane >> 4) * 16;
+
+    for (int st = 0; st < n_stages; ++st) {
+      cp_async_wait<L::kStages - 2>();
+      __syncthreads();                                               // stage st has landed; the buffer of st - 1 is free
+      if (st + L::kStages - 1 < n_stages) load(st + L::kStages - 1);
+      cp_async_commit();
+      const uint32_t buf = ring + (st % L::kStages) * L::kStage;
+      const int kb = k0 + st * kStageKeys;
+      const bool masked = kb + kStageKeys > min_vis || kb + kStageKeys > k1;
+      bool plain = true;
+      if (masked && n > 1) {
+        // a value that only some rows see must not reach the others, not even as zero times infinity
+        bool odd = false;
+        const int from = max(0, min_vis - kb);
+        for (int c = from * kChunks + tid; c < kStageKeys * kChunks; c += 128) {
+          const uint4 w = *reinterpret_cast<const uint4*>(smem + (st % L::kStages) * L::kStage + (kStageKeys + c / kChunks) * L::kPitch + (c % kChunks) * 16);
+          const uint32_t e = kBf16 ? 0x7f80u : 0x7c00u, ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) odd |= (ws[j] & e) == e || ((ws[j] >> 16) & e) == e;
+        }
+        plain = !__syncthreads_or(odd);
+      }
+
+      float s[kNT][4];
+#pragma unroll
+      for (int j = 0; j < kNT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+        for (int j = 0; j < kNT; j += 2) {
+          uint32_t b[4];
+          ldsm4(buf + k_off + j * 8 * L::kPitch + k * 32, b);
+          mma16816<kBf16>(s[j], qf[k], b[0], b[1]);
+          mma16816<kBf16>(s[j + 1], qf[k], b[2], b[3]);
+        }
+      if (masked) {
+#pragma unroll
+        for (int j = 0; j < kNT; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (kb + wkey + j * 8 + tg * 2 + (e & 1) >= min(vis[e >> 1], k1)) s[j][e] = -INFINITY;
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < kNT; ++j) mx = fmaxf(mx, fmaxf(s[j][2 * i], s[j][2 * i + 1]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float mn = fmaxf(m[i], mx * sc);
+        const float use = mn == -INFINITY ? 0.f : mn;                // nothing visible yet: keep the arithmetic finite
+        const float corr = exp2f(m[i] - use);
+        m[i] = mn;
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < kNT; ++j) {
+          s[j][2 * i] = exp2f(fmaf(s[j][2 * i], sc, -use));
+          s[j][2 * i + 1] = exp2f(fmaf(s[j][2 * i + 1], sc, -use));
+          sum += s[j][2 * i] + s[j][2 * i + 1];
+        }
+        l[i] = l[i] * corr + sum;                                    // this thread's columns; the quad's are added at the end
+        if (__any_sync(0xffffffffu, corr != 1.f)) {                  // seldom after the first stages
+#pragma unroll
+          for (int j = 0; j < D / 8; ++j) {
+            o[j][2 * i] *= corr;
+            o[j][2 * i + 1] *= corr;
+          }
+        }
+      }
+      if (plain) {
+#pragma unroll
+        for (int k = 0; k < kWarpKeys / 16; ++k) {
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x = s[2 * k + (e >> 1)][(e & 1) * 2], y = s[2 * k + (e >> 1)][(e & 1) * 2 + 1];
+            hi[e] = pack2<kBf16>(x, y);
+            const float2 h = unpack2<kBf16>(hi[e]);
+            lo[e] = pack2<kBf16>(x - h.x, y - h.y);
+          }
+#pragma unroll
+          for (int j = 0; j < D / 8; j += 2) {
+            uint32_t b[4];
+            ldsm4_t(buf + v_off + k * 16 * L::kPitch + j * 16, b);
+            mma16816<kBf16>(o[j], hi, b[0], b[1]);
+            mma16816<kBf16>(o[j], lo, b[0], b[1]);
+            mma16816<kBf16>(o[j + 1], hi, b[2], b[3]);
+            mma16816<kBf16>(o[j + 1], lo, b[2], b[3]);
+          }
+        }
+      } else {
+        const uint8_t* vrow = smem + (st % L::kStages) * L::kStage + (kStageKeys + wkey) * L::kPitch + tg * 4;
+#pragma unroll
+        for (int j = 0; j < kNT; ++j)
+          for (int c = 0; c < 8; ++c) {                              // key kb + wkey + 8 j + c, whose weights lane c / 2 of the quad holds
+            const float mine0 = (c & 1) ? s[j][1] : s[j][0], mine1 = (c & 1) ? s[j][3] : s[j][2];
+            const float p0 = __shfl_sync(0xffffffffu, mine0, (lane & ~3) | (c >> 1)), p1 = __shfl_sync(0xffffffffu, mine1, (lane & ~3) | (c >> 1));
+            const int key = kb + wkey + j * 8 + c;
+            const bool see0 = key < vis[0], see1 = key < vis[1];
+#pragma unroll
+            for (int d = 0; d < D / 8; ++d) {
+              const float2 v = unpack2<kBf16>(*reinterpret_cast<const uint32_t*>(vrow + (j * 8 + c) * L::kPitch + d * 16));
+              if (see0) { o[d][0] = fmaf(p0, v.x, o[d][0]); o[d][1] = fmaf(p0, v.y, o[d][1]); }
+              if (see1) { o[d][2] = fmaf(p1, v.x, o[d][2]); o[d][3] = fmaf(p1, v.y, o[d][3]); }
+            }
+          }
+      }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+      l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
     }
   }
-  float m[G], l[G], acc[G][8];
+
+  // this warp's accumulator as rows of a [64][D] fp32 buffer, with their maxima and sums
+  __device__ __forceinline__ void spill(float* part, float* s_m, float* s_l) const {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m[g] = -INFINITY;
-    l[g] = 0.f;
+    for (int i = 0; i < 2; ++i) {
+      const int row = warp * 16 + g + i * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[g][j] = 0.f;
-  }
-  const int32_t* bt = a.block_table + static_cast<int64_t>(r) * a.max_blocks;
-  const uint16_t* kc = reinterpret_cast<const uint16_t*>(a.k_cache);
-  const uint16_t* vc = reinterpret_cast<const uint16_t*>(a.v_cache);
-  for (int k = k0 + grp; k < k1; k += kGroups) {
-    const int64_t slot = static_cast<int64_t>(bt[k / a.block_size]) * a.block_size + k % a.block_size;
-    const int64_t off = (slot * a.ng + hk) * D + lk * 8;
-    const int4 kraw = ld_nc_v4(reinterpret_cast<const int4*>(kc + off));
-    const int4 vraw = ld_nc_v4(reinterpret_cast<const int4*>(vc + off));
-    float kf[8], vf[8];
-    unpack8<kBf16>(kraw, kf);
-    unpack8<kBf16>(vraw, vf);
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float s = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s = fmaf(q[g][j], kf[j], s);
-#pragma unroll
-      for (int o = kLPK / 2; o > 0; o >>= 1) s += __shfl_xor_sync(gmask, s, o, kLPK);
-      const float mn = fmaxf(m[g], s);
-      const float corr = exp2f(m[g] - mn), p = exp2f(s - mn);
-      l[g] = l[g] * corr + p;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[g][j] = fmaf(acc[g][j], corr, p * vf[j]);
-      m[g] = mn;
+      for (int j = 0; j < D / 8; ++j) *reinterpret_cast<float2*>(part + row * D + j * 8 + tg * 2) = make_float2(o[j][2 * i], o[j][2 * i + 1]);
+      if (tg == 0) {
+        s_m[row] = m[i];
+        s_l[row] = l[i];
+      }
     }
   }
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    if (lk == 0) {
-      s_m[grp][g] = m[g];
-      s_l[grp][g] = l[g];
+};
+
+// running sum of weighted partials; no keys: zeros
+struct Merge {
+  float M = -INFINITY, L = 0.f;
+  float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+  __device__ __forceinline__ void add(float m, float l, const float4& v) {
+    const float f = exp2f(m - M);
+    L = fmaf(l, f, L);
+    if (l > 0.f) {
+      O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
     }
+  }
+  template <bool kBf16> __device__ __forceinline__ uint2 result() const {
+    const float inv = L > 0.f ? 1.f / L : L;                         // 0 without keys; NaN stays NaN
+    return make_uint2(pack2<kBf16>(O.x * inv, O.y * inv), pack2<kBf16>(O.z * inv, O.w * inv));
+  }
+};
+
+// ---- decode: the stages of every (request, KV head), in one line
+// request r (or token, without cu) as this launch sees it: its tokens and its stages, 0 for requests that are chunks
+struct Item { int t0, n, stages, max_vis, min_vis; };
+__device__ __forceinline__ Item decode_item(const PagedParams& p, int r) {
+  Item it{0, 0, 0, 0, 0x7fffffff};
+  if (r >= p.n_tiles) return it;
+  it.t0 = p.a.cu == nullptr ? r : p.a.cu[r];
+  it.n = p.a.cu == nullptr ? 1 : p.a.cu[r + 1] - it.t0;
+  if ((it.n << p.group_shift) > 16) it.n = 0;
+  for (int i = 0; i < it.n; ++i) {
+    const int v = p.a.tok_len[it.t0 + i];
+    it.max_vis = max(it.max_vis, v);
+    it.min_vis = min(it.min_vis, v);
+  }
+  it.stages = it.n > 0 ? max(1, (it.max_vis + kStageKeys - 1) / kStageKeys) : 0;      // a request without keys still gets its zeros written
+  return it;
+}
+// one warp: the stages of all requests, and of those before request `upto`
+__device__ __forceinline__ void count_stages(const PagedParams& p, int upto, int& total, int& before) {
+  const int lane = threadIdx.x & 31;
+  total = before = 0;
+  for (int r = lane; r < p.n_tiles; r += 32) {
+    const int s = decode_item(p, r).stages;
+    total += s;
+    if (r < upto) before += s;
+  }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s_acc[grp][g][lk * 8 + j] = acc[g][j];
+  for (int o = 16; o > 0; o >>= 1) {
+    total += __shfl_xor_sync(0xffffffffu, total, o);
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+  }
+}
+// where the line is cut: its first `rem` parts have q + 1 stages, the others q
+struct Cuts {
+  int q, rem;
+  __device__ __forceinline__ Cuts(int line, int parts) : q(line / parts), rem(line % parts) {}
+  __device__ __forceinline__ int at(int i) const { return q * i + min(i, rem); }
+  __device__ __forceinline__ int part_of(int x) const { return x < rem * (q + 1) ? x / (q + 1) : rem + (x - rem * (q + 1)) / max(q, 1); }
+};
+
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams p) {
+  using L = Smem<D>;
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ int s_find[2];
+  const PagedAttnArgs& a = p.a;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
+  int total, before;
+  count_stages(p, 0, total, before);
+  const Cuts cuts(total * a.ng, p.splits);
+  int at = cuts.at(blockIdx.x);
+  const int end = cuts.at(blockIdx.x + 1);
+  if (at >= end) return;
+  // the request that this CTA's part of the line starts in
+  if (tid < 32) {
+    int seen = 0;
+    for (int r0 = 0; r0 < p.n_tiles; r0 += 32) {
+      const int s = decode_item(p, r0 + lane).stages;
+      int incl = s;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int first = (seen + incl - s) * a.ng;
+      if (s > 0 && at >= first && at < first + s * a.ng) {
+        s_find[0] = r0 + lane;
+        s_find[1] = at - first;
+      }
+      seen += __shfl_sync(0xffffffffu, incl, 31);
+      if (seen * a.ng > at) break;
+    }
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
-    const int g = idx / D, d = idx % D;
-    float M = -INFINITY;
+  int r = s_find[0], inside = s_find[1];
+  Item it = decode_item(p, r);
+  float* part = reinterpret_cast<float*>(smem);                      // [4 warps][16][D] over the ring
+  float* s_m = reinterpret_cast<float*>(smem + L::kStatOff);
+  float* s_l = s_m + 64;
+  Tile<D, kBf16, 1> tile;
+  while (true) {
+    const int hk = inside / it.stages, st0 = inside % it.stages;
+    const int n_st = min(it.stages - st0, end - at);
+    tile.run(p, smem, a.block_table + static_cast<int64_t>(a.tok_req[it.t0]) * a.max_blocks, hk, it.t0, it.n, it.min_vis, st0 * kStageKeys,
+             min(it.max_vis, (st0 + n_st) * kStageKeys));
+    __syncthreads();                                                 // the ring is not read any more
+    tile.spill(part, s_m, s_l);
+    __syncthreads();
+    const bool whole = n_st == it.stages;
+    // slot 0: a part that starts inside its item; slot 1: one that starts with it
+    float* ws = p.ws + (static_cast<int64_t>(blockIdx.x) * 2 + (st0 == 0 ? 1 : 0)) * (16 * (D + 2));
+    for (int idx = tid; idx < (it.n << p.group_shift) * (D / 4); idx += 128) {
+      const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+      Merge x;
 #pragma unroll
-    for (int c = 0; c < kGroups; ++c) M = fmaxf(M, s_m[c][g]);
-    float L = 0.f, O = 0.f;
-    if (M > -INFINITY) {
+      for (int w = 0; w < 4; ++w) x.M = fmaxf(x.M, s_m[w * 16 + row]);
+      if (x.M > -INFINITY) {
 #pragma unroll
-      for (int c = 0; c < kGroups; ++c) {
-        const float w = exp2f(s_m[c][g] - M);
-        L = fmaf(s_l[c][g], w, L);
-        O = fmaf(s_acc[c][g][d], w, O);
+        for (int w = 0; w < 4; ++w) x.add(s_m[w * 16 + row], s_l[w * 16 + row], *reinterpret_cast<const float4*>(part + (w * 16 + row) * D + col));
+      }
+      if (whole) {
+        uint16_t* out = static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
+        *reinterpret_cast<uint2*>(out + col) = x.result<kBf16>();
+      } else {
+        *reinterpret_cast<float4*>(ws + row * D + col) = x.O;
+        if (col == 0) {
+          ws[16 * D + row] = x.M;
+          ws[16 * D + 16 + row] = x.L;
+        }
       }
     }
-    const int64_t head = static_cast<int64_t>(t) * np + hk * G + g;
-    if (nsplit == 1) {
-      store_out<kBf16>(a.out, head * D + d, L > 0.f ? O / L : 0.f);
-    } else {
-      a.ws_o[(head * nsplit + split) * D + d] = O;
-      if (d == 0) {
-        a.ws_ml[(head * nsplit + split) * 2] = M;
-        a.ws_ml[(head * nsplit + split) * 2 + 1] = L;
-      }
+    at += n_st;
+    inside += n_st;
+    if (at >= end) return;
+    if (inside == it.stages * a.ng) {                                // on to the next request that is not a chunk
+      inside = 0;
+      do it = decode_item(p, ++r); while (it.stages == 0 && r < p.n_tiles);
+      if (it.stages == 0) return;
     }
+    __syncthreads();                                                 // the partials have been read; the ring fills again
   }
+}
+
+// items that a cut fell into: their CTAs' partials, one CTA per (request, KV head)
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(128) paged_merge_kernel(const PagedParams p) {
+  const PagedAttnArgs& a = p.a;
+  const int r = blockIdx.x / a.ng, hk = blockIdx.x % a.ng, G = 1 << p.group_shift, np = a.ng << p.group_shift;
+  const Item it = decode_item(p, r);
+  if (it.stages == 0) return;
+  int total, before;
+  count_stages(p, r, total, before);
+  const Cuts cuts(total * a.ng, p.splits);
+  const int first = before * a.ng + hk * it.stages, i0 = cuts.part_of(first), i1 = cuts.part_of(first + it.stages - 1);
+  if (i0 == i1) return;                                              // one CTA had all of it
+  auto slot = [&](int i) { return p.ws + (static_cast<int64_t>(i) * 2 + (i > i0 || cuts.at(i) > first ? 0 : 1)) * (16 * (D + 2)); };
+  // the parts' weights first, then the accumulators: every load of a pass stands by itself
+  __shared__ float s_f[16][kDecodeCtas + 1], s_inv[16];
+  const int rows = it.n << p.group_shift, parts = i1 - i0 + 1, lane = threadIdx.x & 31;
+  for (int row = threadIdx.x >> 5; row < rows; row += 4) {
+    float M = -INFINITY, L = 0.f;
+    for (int i = lane; i < parts; i += 32) {
+      s_f[row][i] = slot(i0 + i)[16 * D + row];
+      M = fmaxf(M, s_f[row][i]);
+    }
+    M = warp_max(M);
+    const float use = M == -INFINITY ? 0.f : M;
+    for (int i = lane; i < parts; i += 32) {
+      const float f = exp2f(s_f[row][i] - use), l = slot(i0 + i)[16 * D + 16 + row];
+      s_f[row][i] = l > 0.f ? f : 0.f;
+      L = fmaf(l, f, L);
+    }
+    L = warp_sum(L);
+    if (lane == 0) s_inv[row] = L > 0.f ? 1.f / L : L;               // 0 without keys; NaN stays NaN
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < rows * (D / 4); idx += 128) {
+    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int i = 0; i < parts; ++i) {
+      const float f = s_f[row][i];
+      const float4 v = *reinterpret_cast<const float4*>(slot(i0 + i) + row * D + col);
+      O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
+    }
+    const float inv = s_inv[row];
+    uint16_t* out = static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
+    *reinterpret_cast<uint2*>(out + col) = make_uint2(pack2<kBf16>(O.x * inv, O.y * inv), pack2<kBf16>(O.z * inv, O.w * inv));
+  }
+}
+
+// ---- chunks
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p) {
+  using L = Smem<D>;
+  constexpr int kRows = 64;
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ int s_tile[2];
+  const PagedAttnArgs& a = p.a;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tg = lane & 3;
+  const int rank = static_cast<int>(blockIdx.x) % p.splits, item = static_cast<int>(blockIdx.x) / p.splits;
+  const int hk = item % a.ng, tile_at = p.n_tiles - 1 - item / a.ng; // later tiles of a chunk see more keys: they go first
+  const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
+  // that run of 64 / G tokens among the requests with more than 16 rows
+  const int per_tile = kRows >> p.group_shift;
+  if (warp == 0) {
+    int before = 0;
+    for (int r0 = 0; r0 < a.n_seqs; r0 += 32) {
+      const int r = r0 + lane;
+      const int c0 = r < a.n_seqs ? a.cu[r] : 0, c1 = r < a.n_seqs ? a.cu[r + 1] : 0, len = c1 - c0;
+      const int tiles = (len << p.group_shift) > 16 ? (len + per_tile - 1) / per_tile : 0;
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int first = before + incl - tiles;
+      if (tiles > 0 && tile_at >= first && tile_at < first + tiles) {
+        const int off = (tile_at - first) * per_tile;
+        s_tile[0] = c0 + off;
+        s_tile[1] = min(per_tile, len - off);
+      }
+      before += __shfl_sync(0xffffffffu, incl, 31);
+      if (before > tile_at) break;
+    }
+    if (lane == 0 && before <= tile_at) s_tile[1] = 0;               // more tiles launched than there are
+  }
+  __syncthreads();
+  const int t0 = s_tile[0], n = s_tile[1];
+  if (n == 0) return;
+  const int n_rows = n << p.group_shift;
+  // keys that the tile's tokens see: all of them below min_vis, some up to max_vis
+  int max_vis = 0, min_vis = 0x7fffffff;
+  for (int i = lane; i < n; i += 32) {
+    const int v = a.tok_len[t0 + i];
+    max_vis = max(max_vis, v);
+    min_vis = min(min_vis, v);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    max_vis = max(max_vis, __shfl_xor_sync(0xffffffffu, max_vis, o));
+    min_vis = min(min_vis, __shfl_xor_sync(0xffffffffu, min_vis, o));
+  }
+  const int per = ((max_vis + p.splits - 1) / p.splits + kStageKeys - 1) / kStageKeys * kStageKeys;
+  const int k0 = rank * per, k1 = min(max_vis, k0 + per);
+  Tile<D, kBf16, 4> tile;
+  tile.run(p, smem, a.block_table + static_cast<int64_t>(a.tok_req[t0]) * a.max_blocks, hk, t0, n, min_vis, k0, k1);
+  auto out_row = [&](int row) {
+    return static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
+  };
+  if (p.splits == 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = warp * 16 + g + i * 8;
+      if (row >= n_rows) continue;
+      const float inv = tile.l[i] > 0.f ? 1.f / tile.l[i] : tile.l[i];
+      uint32_t* dst = reinterpret_cast<uint32_t*>(out_row(row)) + tg;
+#pragma unroll
+      for (int j = 0; j < D / 8; ++j) dst[j * 4] = pack2<kBf16>(tile.o[j][2 * i] * inv, tile.o[j][2 * i + 1] * inv);
+    }
+    return;
+  }
+  // ---- the cluster's partials
+  __syncthreads();                                                   // the ring is not read any more
+  float* part = reinterpret_cast<float*>(smem);                      // [64][D]
+  float* s_m = reinterpret_cast<float*>(smem + L::kStatOff);
+  float* s_l = s_m + 64;
+  tile.spill(part, s_m, s_l);
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  for (int idx = rank * 128 + tid; idx < n_rows * (D / 4); idx += p.splits * 128) {
+    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+    Merge x;
+    for (int c = 0; c < p.splits; ++c) x.M = fmaxf(x.M, *cluster.map_shared_rank(s_m + row, c));
+    if (x.M > -INFINITY) {
+      for (int c = 0; c < p.splits; ++c)
+        x.add(*cluster.map_shared_rank(s_m + row, c), *cluster.map_shared_rank(s_l + row, c),
+              *cluster.map_shared_rank(reinterpret_cast<const float4*>(part + row * D + col), c));
+    }
+    *reinterpret_cast<uint2*>(out_row(row) + col) = x.result<kBf16>();
+  }
+  cluster.sync();                                                    // no CTA leaves while another reads its partials
+}
+
+// new keys and values [T, ng, d] (any token and head strides) into their cache rows, 16 bytes per thread
+__global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* __restrict__ kc,
+                                                          uint4* __restrict__ vc, const int64_t* __restrict__ slots, int n_tok, int ng, int chunks,
+                                                          int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh) {
+  const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, row = static_cast<int64_t>(ng) * chunks;
+  if (idx >= n_tok * row) return;
+  const int64_t t = idx / row;
+  const int c = static_cast<int>(idx % row), h = c / chunks, u = c % chunks;
+  const int64_t dst = slots[t] * row + c;
+  kc[dst] = k[t * k_st + h * k_sh + u];
+  vc[dst] = v[t * v_st + h * v_sh + u];
 }
 
 template <int D, bool kBf16>
-__global__ void __launch_bounds__(D) paged_attn_combine_kernel(PagedAttnArgs a, int nsplit) {
-  const int64_t head = blockIdx.x;
-  const int d = threadIdx.x;
-  float M = -INFINITY;
-  for (int s = 0; s < nsplit; ++s) M = fmaxf(M, a.ws_ml[(head * nsplit + s) * 2]);
-  float L = 0.f, O = 0.f;
-  if (M > -INFINITY) {
-    for (int s = 0; s < nsplit; ++s) {
-      const float w = exp2f(a.ws_ml[(head * nsplit + s) * 2] - M);
-      L = fmaf(a.ws_ml[(head * nsplit + s) * 2 + 1], w, L);
-      O = fmaf(a.ws_o[(head * nsplit + s) * D + d], w, O);
-    }
-  }
-  store_out<kBf16>(a.out, head * D + d, L > 0.f ? O / L : 0.f);
+int launch_chunks(const PagedParams& p, cudaStream_t s) {
+  auto kern = paged_chunk_kernel<D, kBf16>;
+  static const cudaError_t ready = [&] {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }();
+  if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
+  const int64_t ctas = static_cast<int64_t>(p.n_tiles) * p.a.ng * p.splits;
+  if (ctas > 0x7fffffff) { g_paged_err = "paged attention: too many tiles"; return -12; }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = Smem<D>::kTotal;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(p.splits);
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = p.splits > 1 ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+  if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
+  return 0;
 }
 
-template <int D, int G>
-void launch(const PagedAttnArgs& a, int splits, cudaStream_t s) {
-  const dim3 grid(a.n_tokens, a.ng, splits);
-  if (a.is_bf16) paged_attn_kernel<D, G, true><<<grid, 128, 0, s>>>(a);
-  else paged_attn_kernel<D, G, false><<<grid, 128, 0, s>>>(a);
-  if (splits > 1) {
-    const int heads = a.n_tokens * a.ng * G;
-    if (a.is_bf16) paged_attn_combine_kernel<D, true><<<heads, D, 0, s>>>(a, splits);
-    else paged_attn_combine_kernel<D, false><<<heads, D, 0, s>>>(a, splits);
+template <int D, bool kBf16>
+int launch_decode(const PagedParams& p, cudaStream_t s) {
+  auto kern = paged_decode_kernel<D, kBf16>;
+  static const cudaError_t ready = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
+  if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
+  // the line of stages is counted in 32 bits
+  if (static_cast<int64_t>(p.n_tiles) * p.a.ng * ((static_cast<int64_t>(p.a.max_blocks) * p.a.block_size + kStageKeys - 1) / kStageKeys + 1) > 0x7fffffff) {
+    g_paged_err = "paged attention: too many requests";
+    return -12;
   }
+  kern<<<p.splits, 128, Smem<D>::kTotal, s>>>(p);
+  paged_merge_kernel<D, kBf16><<<p.n_tiles * p.a.ng, 128, 0, s>>>(p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
+  return 0;
+}
+
+int log2_exact(int v) {
+  for (int i = 0; i < 31; ++i)
+    if (v == 1 << i) return i;
+  return -1;
+}
+
+// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages
+int decode_ctas(const PagedAttnArgs& a) {
+  const int64_t items = static_cast<int64_t>(a.cu != nullptr ? a.n_seqs : a.n_tokens) * a.ng;
+  const int64_t longest = (static_cast<int64_t>(a.max_blocks) * a.block_size + kStageKeys - 1) / kStageKeys;
+  const int64_t n = items * longest / 2;
+  return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
 }
 
 }  // namespace
+
+const char* paged_attention_last_error() { return g_paged_err.c_str(); }
 
 bool paged_attention_supported(int head_dim, int group) {
   return (head_dim == 64 || head_dim == 128) && (group == 1 || group == 2 || group == 4 || group == 8);
 }
 
-void paged_attention(const PagedAttnArgs& a, int splits, cudaStream_t s) {
-#define B200_PA(D, G) if (a.head_dim == D && a.group == G) return launch<D, G>(a, splits, s);
-  B200_PA(128, 1) B200_PA(128, 2) B200_PA(128, 4) B200_PA(128, 8)
-  B200_PA(64, 1) B200_PA(64, 2) B200_PA(64, 4) B200_PA(64, 8)
-#undef B200_PA
+int64_t paged_decode_workspace(const PagedAttnArgs& a) { return static_cast<int64_t>(decode_ctas(a)) * 2 * 16 * (a.head_dim + 2); }
+
+void paged_write(const PagedWriteArgs& w, cudaStream_t s) {
+  const int chunks = w.head_dim / 8;
+  const int64_t n = static_cast<int64_t>(w.n_tokens) * w.ng * chunks;
+  if (n == 0) return;
+  paged_write_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
+      static_cast<const uint4*>(w.k), static_cast<const uint4*>(w.v), static_cast<uint4*>(w.k_cache), static_cast<uint4*>(w.v_cache), w.slots,
+      w.n_tokens, w.ng, chunks, w.k_st / 8, w.k_sh / 8, w.v_st / 8, w.v_sh / 8);
+}
+
+// with cu: chunk_tiles tiles of 64 rows over the requests with more than 16, in chunk_splits key ranges; decode: whether there are others
+int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s) {
+  PagedParams p{};
+  p.a = a;
+  p.group_shift = log2_exact(a.group);
+  p.bs_shift = log2_exact(a.block_size);
+  if (a.cu != nullptr && chunk_tiles > 0) {
+    p.n_tiles = chunk_tiles;
+    p.splits = 1;
+    while (2 * p.splits <= chunk_splits && p.splits < 16) p.splits *= 2;
+    const int rc = a.head_dim == 128 ? (a.is_bf16 ? launch_chunks<128, true>(p, s) : launch_chunks<128, false>(p, s))
+                                     : (a.is_bf16 ? launch_chunks<64, true>(p, s) : launch_chunks<64, false>(p, s));
+    if (rc != 0) return rc;
+  }
+  if (a.cu != nullptr && !decode) return 0;                          // every request is a chunk
+  p.n_tiles = a.cu != nullptr ? a.n_seqs : a.n_tokens;
+  p.splits = decode_ctas(a);
+  p.ws = ws;
+  return a.head_dim == 128 ? (a.is_bf16 ? launch_decode<128, true>(p, s) : launch_decode<128, false>(p, s))
+                           : (a.is_bf16 ? launch_decode<64, true>(p, s) : launch_decode<64, false>(p, s));
 }
 
 }  // namespace b200

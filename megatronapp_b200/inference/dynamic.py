@@ -61,6 +61,19 @@ class _Seq:
     state_row: int = -1        # row of this request in the recurrent-state tensors
 
 
+def key_ranges(tiles: int, max_len: int) -> int:
+    """Into how many key ranges (CTAs of a cluster) a (64-row tile, KV head) of a prompt portion is cut: only where the tiles leave
+    most of the 296 CTA places empty and the context is long enough to pay for the merge."""
+    n = 1
+    while n < 16 and tiles * n <= 148 and max_len >= 512 * n:
+        n *= 2
+    return n
+
+
+def _rows_of_16_bytes(t: torch.Tensor) -> bool:
+    return t.stride(2) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
 class DynamicInferenceContext:
     def __init__(self, max_sequence_length: int, num_blocks: int, block_size: int = 16,
                  max_tokens_per_step: int = 256, max_requests: int = 64):
@@ -162,6 +175,7 @@ class DynamicInferenceContext:
         self._tok_req = torch.tensor(tok_req, dtype=torch.int32).to(device)
         self._tok_len = torch.tensor(tok_len, dtype=torch.int32).to(device)
         self._max_len = l_max
+        self._paged_plans = {}
         self.positions = torch.cat(pos_all).to(device)
         self._write_slots = torch.cat(slots_all).to(device)
         self._q_index = self._q_valid = self._kv_slots = self._mask = None      # gather path: built on first use
@@ -299,6 +313,16 @@ class DynamicInferenceContext:
         return seqmix.sigmoid_attention_paged(q, kc, vc, self._block_table, self._tok_req, self._tok_len, self.block_size, scale, softcap,
                                               head_bias, turns_back, interleaved, self._max_len)
 
+    def _paged_plan(self, group: int, ng: int) -> tuple:
+        """How this step's paged attention is cut up: (requests with at most 16 rows, 64-row tiles of the others, key ranges of
+        those).  The same for all layers of one head layout, made once a step."""
+        plan = self._paged_plans.get((group, ng))
+        if plan is None:
+            new = [p[2] for p in self._plan]
+            chunks = [-(-n * group // 64) for n in new if n * group > 16]
+            plan = self._paged_plans[(group, ng)] = (len(new) - len(chunks), sum(chunks), key_ranges(sum(chunks) * ng, self._max_len))
+        return plan
+
     # -- attention over the paged cache --------------------------------------------
     def attend(self, layer: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
         """``q [T, np, hn]``, new ``k / v [T, ng, hn(v)]`` -> ``[T, np, hn_v]``; writes k / v into their pages first."""
@@ -307,20 +331,24 @@ class DynamicInferenceContext:
             self.kv[layer] = (torch.zeros(n_slots, *k.shape[1:], dtype=k.dtype, device=k.device),
                               torch.zeros(n_slots, *v.shape[1:], dtype=v.dtype, device=v.device))
         kc, vc = self.kv[layer]
-        kc[self._write_slots] = k
-        vc[self._write_slots] = v
         np_, ng = q.shape[1], k.shape[1]
         if q.is_cuda and self.use_paged_kernel and k.shape[-1] == v.shape[-1] == q.shape[-1] and q.dtype in (torch.bfloat16, torch.float16):
             from .. import ops
 
             ext = ops.ext()
             if ext.paged_attention_supported(q.shape[-1], np_ // ng):
-                # flash-decoding split of long contexts when the (token, KV head) grid alone cannot fill the GPU
-                ctas = q.shape[0] * ng
-                splits = 1 if ctas >= 296 else max(1, min(16, self._max_len // 512, 296 // max(1, ctas)))
+                decode, chunk_tiles, chunk_splits = self._paged_plan(np_ // ng, ng)
                 self.kernel_calls += 1
+                if k.dtype == v.dtype == q.dtype == kc.dtype and _rows_of_16_bytes(k) and _rows_of_16_bytes(v):
+                    new = (k, v, self._write_slots)                    # written by the same call
+                else:
+                    kc[self._write_slots] = k
+                    vc[self._write_slots] = v
+                    new = (None, None, None)
                 return ext.paged_attention(q.contiguous(), kc, vc, self._block_table, self._tok_req, self._tok_len,
-                                           self.block_size, float(scale), splits)
+                                           self.block_size, float(scale), decode, *new, self.packed.cu, chunk_tiles, chunk_splits)
+        kc[self._write_slots] = k
+        vc[self._write_slots] = v
         self._ensure_gather(q.device)
         qp = q[self._q_index]                                        # [R, n, np, hn]
         kp, vp = kc[self._kv_slots], vc[self._kv_slots]               # [R, L, ng, hn]

@@ -1,0 +1,89 @@
+"""Paged attention of the continuous-batching engine at the edges of its tiles, stages and key ranges, against 64 bits."""
+import pytest
+import torch
+
+
+def _step(reqs, hq, hkv, d, block, dtype, seed=0):
+    """A context holding ``reqs = [(tokens in the cache, new tokens)]`` and the new queries, keys and values (as strided views)."""
+    from megatronapp_b200.inference.dynamic import DynamicInferenceContext
+
+    g = torch.Generator("cuda").manual_seed(seed)
+    cx = DynamicInferenceContext(max(a + n for a, n in reqs) + 1, sum(-(-(a + n) // block) for a, n in reqs) + 1, block, 1 << 16, len(reqs))
+    for i in range(len(reqs)):
+        cx.add_request(str(i))
+    old = [(str(i), a) for i, (a, _) in enumerate(reqs) if a]
+    if old:
+        cx.begin_step(old[::-1], "cuda")
+        cx.end_step()
+    cx.begin_step([(str(i), n) for i, (_, n) in enumerate(reqs)], "cuda")
+    for t in cx.kv_pages(1, (hkv, d), (hkv, d), dtype):
+        t.normal_(generator=g)
+    T = sum(n for _, n in reqs)
+    q = torch.randn(T, hq, d, generator=g, device="cuda").to(dtype)
+    kv = torch.randn(T, hkv, 2, d, generator=g, device="cuda").to(dtype)
+    return cx, q, kv[:, :, 0], kv[:, :, 1]
+
+
+def _oracle(cx, reqs, q, k, v, scale, block):
+    kc, vc = (t.clone() for t in cx.kv[1])
+    kc[cx.write_slots], vc[cx.write_slots] = k, v
+    rep, t0, out = q.shape[1] // k.shape[1], 0, []
+    for i, (a, n) in enumerate(reqs):
+        slots = (torch.tensor(cx.seqs[str(i)].blocks).unsqueeze(1) * block + torch.arange(block)).view(-1)[:a + n].cuda()
+        kk, vv = (t[slots].double().repeat_interleave(rep, 1) for t in (kc, vc))
+        for j in range(n):
+            L = a + j + 1                                     # no masked key enters the sum
+            w = torch.softmax(torch.einsum("hd,lhd->hl", q[t0 + j].double(), kk[:L]) * scale, -1)
+            out.append(torch.einsum("hl,lhd->hd", w, vv[:L]))
+        t0 += n
+    return torch.stack(out), kc, vc
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reqs,hq,hkv,d,block,dtype", [
+    ([(0, 1)], 4, 4, 64, 16, torch.bfloat16),                                    # one key
+    ([(63, 1), (64, 1), (127, 1), (500, 1)], 8, 1, 128, 16, torch.bfloat16),     # around a stage
+    ([(5000, 1)], 8, 2, 128, 16, torch.float16),                                 # one item over many CTAs
+    ([(16383, 1), (3, 1)], 4, 4, 64, 32, torch.bfloat16),                        # cuts inside one item and around the other
+    ([(3000, 1)] * 7 + [(1, 1)] * 50 + [(5000, 1)], 4, 1, 64, 16, torch.bfloat16),
+    ([(9000, 30)], 8, 2, 128, 16, torch.bfloat16),                               # few tiles, long context: key ranges in a cluster
+    ([(1100, 40), (0, 20)], 4, 1, 64, 16, torch.float16),                        # a tile whose later ranges are empty
+    ([(10, 4), (0, 5), (100, 16), (7, 17)], 4, 1, 128, 16, torch.bfloat16),      # 16 rows and just more
+    ([(0, 64), (130, 1), (1000, 65)], 16, 2, 64, 16, torch.float16),             # whole row tiles and one token more
+    ([(40, 9), (900, 200), (0, 1), (77, 300)], 12, 12, 128, 24, torch.bfloat16),  # a block size that is no power of two
+    ([(0, 3)] * 40 + [(20, 70)] + [(5, 1)] * 30, 8, 8, 64, 16, torch.bfloat16)])  # more requests than a warp searches at once
+def test_tiles(reqs, hq, hkv, d, block, dtype):
+    cx, q, k, v = _step(reqs, hq, hkv, d, block, dtype)
+    want, kc, vc = _oracle(cx, reqs, q, k, v, d ** -0.5, block)
+    got = cx.attend(1, q, k, v, d ** -0.5)
+    assert cx.kernel_calls == 1
+    assert torch.equal(cx.kv[1][0], kc) and torch.equal(cx.kv[1][1], vc)
+    # fp32 sums of exact products: what is left is the result's own rounding, half a unit in the last place
+    unit = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+    assert float((got.double() - want).abs().max()) <= unit * max(1.0, float(want.abs().max()))
+    assert float((got.double() - want).norm()) <= 0.5 * unit * float(want.norm())
+
+
+@pytest.mark.gpu
+def test_values_of_later_tokens_stay_out():
+    """An infinite value of a chunk's token reaches the tokens that see it and no others."""
+    reqs = [(70, 100)]
+    cx, q, k, v = _step(reqs, 4, 2, 64, 16, torch.bfloat16)
+    v[60, 0, 5], v[60, 1, 3] = float("inf"), float("nan")
+    want, _, _ = _oracle(cx, reqs, q, k, v, 0.125, 16)
+    got = cx.attend(1, q, k, v, 0.125).double()
+    assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+    ok = torch.isfinite(want)
+    assert ok[:60].all() and not ok[60:, :2, 5].any() and not ok[60:, 2:, 3].any()
+    assert float((got[ok] - want[ok]).abs().max()) <= 2.0 ** -7
+
+
+def test_key_ranges():
+    from megatronapp_b200.inference.dynamic import key_ranges
+
+    assert key_ranges(8, 100) == 1                                 # too short to cut
+    assert key_ranges(8, 1 << 20) == 16 and key_ranges(149, 1 << 20) == 1
+    for tiles in (1, 7, 64, 500):
+        for n in (1, 255, 512, 1000, 4096, 100000):
+            r = key_ranges(tiles, n)
+            assert r in (1, 2, 4, 8, 16) and (r == 1 or n >= 256 * r)
