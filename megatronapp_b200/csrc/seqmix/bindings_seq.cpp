@@ -889,6 +889,79 @@ void selective_scan(const Tensor& x, c10::optional<Tensor> z, const Tensor& B, c
               " states per channel exceed the largest kernel instance (128)");
   count(); check_last_error("selective_scan");
 }
+// [b, l, heads, dim] whose steps are rows of contiguous heads, 16-byte aligned
+void check_steps(const Tensor& t, const char* name, at::ScalarType dtype) {
+  TORCH_CHECK(t.is_cuda() && t.dim() == 4 && t.scalar_type() == dtype && t.stride(3) == 1 && t.stride(2) == t.size(3) && t.stride(1) % 8 == 0 &&
+              t.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, name, " must be [b, l, heads, dim] with contiguous aligned heads");
+}
+b200seq::SsdArgs ssd_args(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& D) {
+  act_is_bf16(x, "x");
+  check_steps(x, "x", x.scalar_type());
+  check_steps(B, "B", x.scalar_type());
+  check_steps(C, "C", x.scalar_type());
+  check_f32(dt, "dt"); check_f32(A, "A"); check_f32(D, "D");
+  b200seq::SsdArgs p{};
+  p.b = static_cast<int>(x.size(0)); p.l = static_cast<int>(x.size(1)); p.h = static_cast<int>(x.size(2)); p.g = static_cast<int>(B.size(2));
+  TORCH_CHECK(b200seq::ssd_supported(static_cast<int>(x.size(3)), static_cast<int>(B.size(3))), "unsupported head or state size");
+  TORCH_CHECK(p.b > 0 && p.l > 0 && p.g > 0 && p.h % p.g == 0 && static_cast<int64_t>(p.b) * p.h <= 65535, "bad batch, length or head counts");
+  TORCH_CHECK(B.sizes() == C.sizes() && B.size(0) == p.b && B.size(1) == p.l && dt.dim() == 3 && dt.size(0) == p.b && dt.size(1) == p.l &&
+              dt.size(2) == p.h && A.numel() == p.h && D.numel() == p.h, "operands do not fit together");
+  p.x = x.data_ptr(); p.B = B.data_ptr(); p.C = C.data_ptr();
+  p.x_sb = x.stride(0); p.x_sl = x.stride(1); p.b_sb = B.stride(0); p.b_sl = B.stride(1); p.c_sb = C.stride(0); p.c_sl = C.stride(1);
+  p.dt = dt.data_ptr<float>(); p.A = A.data_ptr<float>(); p.D = D.data_ptr<float>();
+  p.n_chunks = (p.l + b200seq::ssd_block() - 1) / b200seq::ssd_block();
+  return p;
+}
+// -> y [b, l, h, 64], final state [b, h, 64, n], and what the backward needs: scores, states at the blocks' starts, the blocks' decays
+std::vector<Tensor> ssd_forward(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& D,
+                                c10::optional<Tensor> init) {
+  c10::cuda::CUDAGuard g(x.device());
+  b200seq::SsdArgs p = ssd_args(x, dt, A, B, C, D);
+  const int64_t n = B.size(3);
+  auto f32 = dt.options();
+  Tensor y = torch::empty({p.b, p.l, p.h, x.size(3)}, x.options()), last = torch::empty({p.b, p.h, x.size(3), n}, f32);
+  Tensor scores = torch::empty({p.b, p.n_chunks, p.g, b200seq::ssd_block(), b200seq::ssd_block()}, f32);
+  Tensor states = torch::empty({p.b, p.h, p.n_chunks, x.size(3), n}, f32), decay = torch::empty({p.b, p.h, p.n_chunks}, f32);
+  if (init.has_value() && init->defined()) {
+    check_f32(*init, "initial state");
+    TORCH_CHECK(init->sizes() == last.sizes(), "initial state must be [b, h, dim, n]");
+    p.first = init->data_ptr<float>();
+  }
+  p.y = y.data_ptr(); p.last = last.data_ptr<float>(); p.scores = scores.data_ptr<float>(); p.states = states.data_ptr<float>(); p.decay = decay.data_ptr<float>();
+  TORCH_CHECK(b200seq::ssd_forward(p, static_cast<int>(n), x.scalar_type() == at::kBFloat16, cur_stream()), "ssd_forward: shared memory");
+  count(4); check_last_error("ssd_forward");
+  return {y, last, scores, states, decay};
+}
+// -> dx, ddt, dA, dB, dC, dD, d(initial state)
+std::vector<Tensor> ssd_backward(const Tensor& dy, c10::optional<Tensor> dlast, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B,
+                                 const Tensor& C, const Tensor& D, const Tensor& scores, const Tensor& states, const Tensor& decay, bool want_first) {
+  c10::cuda::CUDAGuard g(x.device());
+  b200seq::SsdArgs p = ssd_args(x, dt, A, B, C, D);
+  const int64_t n = B.size(3);
+  const int sub = p.n_sub = b200seq::ssd_subgroups(p.n_chunks, p.g, p.b, p.h / p.g);
+  TORCH_CHECK(dy.is_contiguous() && dy.scalar_type() == x.scalar_type() && dy.sizes() == x.sizes() && reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0, "bad dy");
+  check_f32(scores, "scores"); check_f32(states, "states"); check_f32(decay, "decay");
+  TORCH_CHECK(static_cast<int64_t>(p.g) * sub <= 65535, "too many groups");
+  auto f32 = dt.options();
+  Tensor dx = torch::empty({p.b, p.l, p.h, x.size(3)}, x.options()), dB = torch::empty(B.sizes(), x.options()), dC = torch::empty(C.sizes(), x.options());
+  Tensor ddt = torch::empty_like(dt), dA = torch::empty({p.b, p.n_chunks, p.h}, f32), dD = torch::empty({p.b, p.n_chunks, p.h}, f32);
+  Tensor dstates = torch::empty_like(states), partial, dfirst;
+  if (sub > 1) partial = torch::empty({sub, 2, p.b, p.l, p.g, n}, f32);
+  if (want_first) dfirst = torch::empty({p.b, p.h, x.size(3), n}, f32);
+  if (dlast.has_value() && dlast->defined()) {
+    check_f32(*dlast, "final state's gradient");
+    TORCH_CHECK(dlast->numel() == static_cast<int64_t>(p.b) * p.h * x.size(3) * n);
+    p.dlast = dlast->data_ptr<float>();
+  }
+  p.scores = scores.data_ptr<float>(); p.states = states.data_ptr<float>(); p.decay = decay.data_ptr<float>();
+  p.dy = dy.data_ptr(); p.dstates = dstates.data_ptr<float>(); p.dfirst = want_first ? dfirst.data_ptr<float>() : nullptr;
+  p.dx = dx.data_ptr(); p.dB = dB.data_ptr(); p.dC = dC.data_ptr(); p.ddt = ddt.data_ptr<float>(); p.dA = dA.data_ptr<float>(); p.dD = dD.data_ptr<float>();
+  p.partial = sub > 1 ? partial.data_ptr<float>() : nullptr;
+  TORCH_CHECK(b200seq::ssd_backward(p, static_cast<int>(n), x.scalar_type() == at::kBFloat16, cur_stream()), "ssd_backward: shared memory");
+  count(sub > 1 ? 4 : 3); check_last_error("ssd_backward");
+  return {dx, ddt, dA.sum(at::IntArrayRef{0, 1}), dB, dC, dD.sum(at::IntArrayRef{0, 1}), dfirst};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -922,6 +995,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gen_delta_scan", &gen_delta_scan);
   m.def("mingru_scan", &mingru_scan);
   m.def("clamped_glu", &clamped_glu);
+  m.def("ssd_forward", &ssd_forward);
+  m.def("ssd_backward", &ssd_backward);
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("reset_launch_count", []() { g_launches.store(0); });
 }

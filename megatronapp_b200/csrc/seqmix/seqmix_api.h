@@ -300,4 +300,30 @@ bool rglru_chunked_supported(const LruArgs& p, int max_len);
 bool rglru_scan_chunked(const LruArgs& p, int R, cudaStream_t s);
 int rglru_chunked_status();       // 1: a kernel of this process gave up on a wait
 
+// Mamba-2 scan in blocks of ssd_block() steps.  x [b, l, h, 64], B / C [b, l, g, n] with strides over the batch and the steps (elements,
+// multiples of 4), the rest contiguous fp32: dt [b, l, h], A / D [h], scores [b, blocks, g, 64, 64], states / dstates [b, h, blocks, 64, n],
+// decay [b, h, blocks], first / last / dfirst / dlast [b, h, 64, n] (nullptr: zeros, or not wanted)
+struct SsdArgs {
+  const void *x, *B, *C;
+  int64_t x_sb, x_sl, b_sb, b_sl, c_sb, c_sl;
+  const float *dt, *A, *D;
+  int b, l, h, g, n_chunks, n_sub;
+  float *scores, *states, *decay;
+  const float* first;
+  float* last;
+  void* y;                        // [b, l, h, 64]
+  const void* dy;                 // [b, l, h, 64]
+  float* dstates;
+  const float* dlast;
+  float* dfirst;
+  void *dx, *dB, *dC;             // [b, l, h, 64], [b, l, g, n]
+  float *ddt, *dA, *dD;           // [b, l, h], [b, blocks, h] per block
+  float* partial;                 // [n_sub, 2, b, l, g, n] when n_sub > 1
+};
+int ssd_block();
+int ssd_subgroups(int n_chunks, int groups, int batch, int heads_per_group);
+bool ssd_supported(int head_dim, int state_dim);
+bool ssd_forward(const SsdArgs& p, int state_dim, bool bf16, cudaStream_t s);
+bool ssd_backward(const SsdArgs& p, int state_dim, bool bf16, cudaStream_t s);
+
 }  // namespace b200seq

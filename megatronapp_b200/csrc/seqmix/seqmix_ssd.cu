@@ -1,0 +1,571 @@
+// Mamba-2 state-space scan in blocks of 64 steps, forward and backward, everything in fp32:
+//
+//   S_t = exp(dt_t A) S_{t-1} + dt_t x_t B_t^T,   y_t = S_t C_t + D x_t          (per head; B and C per group of heads)
+//
+// Within a block (cum_t: running sum of dt A)
+//   y_t = sum_{u <= t} exp(cum_t - cum_u) (C_t . B_u) dt_u x_u + exp(cum_t) S C_t + D x_t
+// so the work is small products of 64-row tiles.  Forward: the scores C B^T once per group, what every block adds to the state, a pass over
+// the blocks that turns this into the state each block starts from, and the outputs.  Backward: the same two state kernels for the
+// gradient that enters each block's starting state, walked in reverse, then one kernel for all gradients of a block, whose CTA walks the
+// heads of a group so that the gradients of B and C add up in registers.  Exponents above the diagonal are never taken (they can overflow).
+//
+// Tiles are fp32 in shared memory, 4 x 4 or 4 x 8 results per thread: bound by fp32 multiply-adds (2.1 M per head and block backward,
+// 1.3 M forward) and the shared-memory reads that feed them.  The block-by-block PyTorch form took some 2900 launches and 14 ms of
+// device time for 64 heads x 2048 steps.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include "seq_common.cuh"
+#include "seqmix_api.h"
+
+namespace b200seq {
+namespace {
+
+constexpr int kT = 64;          // steps of a block
+constexpr int kP = 64;          // head width
+constexpr int kPitchT = kT + 4;  // padded rows: 16-byte aligned, conflict-free when 8 threads read 8 rows
+constexpr int kThreads = 256;
+
+template <typename T> __device__ __forceinline__ float4 ld4(const T* p);
+template <> __device__ __forceinline__ float4 ld4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <> __device__ __forceinline__ float4 ld4<__nv_bfloat16>(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+template <typename T> __device__ __forceinline__ void st4(T* p, float4 v);
+template <> __device__ __forceinline__ void st4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+template <> __device__ __forceinline__ void st4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
+  __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+
+// acc[i][j] += sum_k A(m_i, k) B(n_j, k).  An operand lies with k contiguous (X[m][k]; the thread's rows are t, t + 16, ...) or with
+// its own index contiguous (X[k][m]; groups of four: 4 t .. 4 t + 3, then 64 further on)
+template <int MI, int NI, bool AK, bool BK>
+__device__ __forceinline__ void mm(float (&acc)[MI][NI], const float* A, int pa, const float* B, int pb, int K, int ty, int tx) {
+#pragma unroll 2
+  for (int k = 0; k < K; k += 4) {
+    float a[MI][4], b[NI][4];
+    if constexpr (AK) {
+#pragma unroll
+      for (int i = 0; i < MI; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(A + (ty + 16 * i) * pa + k);
+        a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < MI / 4; ++q)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const float4 v = *reinterpret_cast<const float4*>(A + (k + kk) * pa + q * 64 + ty * 4);
+          a[q * 4][kk] = v.x; a[q * 4 + 1][kk] = v.y; a[q * 4 + 2][kk] = v.z; a[q * 4 + 3][kk] = v.w;
+        }
+    }
+    if constexpr (BK) {
+#pragma unroll
+      for (int j = 0; j < NI; ++j) {
+        const float4 v = *reinterpret_cast<const float4*>(B + (tx + 16 * j) * pb + k);
+        b[j][0] = v.x; b[j][1] = v.y; b[j][2] = v.z; b[j][3] = v.w;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < NI / 4; ++q)
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const float4 v = *reinterpret_cast<const float4*>(B + (k + kk) * pb + q * 64 + tx * 4);
+          b[q * 4][kk] = v.x; b[q * 4 + 1][kk] = v.y; b[q * 4 + 2][kk] = v.z; b[q * 4 + 3][kk] = v.w;
+        }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j) acc[i][j] = fmaf(a[i][kk], b[j][kk], acc[i][j]);
+  }
+}
+template <int MI, int NI>
+__device__ __forceinline__ void zero(float (&a)[MI][NI]) {
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j) a[i][j] = 0.f;
+}
+__device__ __forceinline__ float half_warp_sum(float v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// column of result j of a thread whose operand has its own index contiguous
+__device__ __forceinline__ int col4(int t, int j) { return (j >> 2) * 64 + t * 4 + (j & 3); }
+
+// 64 rows of W columns into padded fp32 rows; rows from `rows` on are zeros.  f(row): factor of the row
+template <int W, typename T, typename F>
+__device__ __forceinline__ void load_rows(float* dst, int pitch, const T* src, int64_t stride, int rows, F f) {
+  for (int i = threadIdx.x; i < kT * (W / 4); i += kThreads) {
+    const int r = i / (W / 4), c = (i % (W / 4)) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < rows) {
+      v = ld4(src + r * stride + c);
+      const float s = f(r);
+      v.x *= s; v.y *= s; v.z *= s; v.w *= s;
+    }
+    *reinterpret_cast<float4*>(dst + r * pitch + c) = v;
+  }
+}
+struct One { __device__ float operator()(int) const { return 1.f; } };
+
+// dt and the running sum of dt * A of one block (dt = 0 from `rows` on); all threads call it
+__device__ __forceinline__ void block_decay(float* s_dt, float* s_cum, const float* dt, int64_t stride, int rows, float a) {
+  if (threadIdx.x < 32) {
+    const int l = threadIdx.x;
+    const float d0 = 2 * l < rows ? dt[2 * l * stride] : 0.f, d1 = 2 * l + 1 < rows ? dt[(2 * l + 1) * stride] : 0.f;
+    const float v0 = d0 * a, pair = v0 + d1 * a;
+    float incl = pair;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (l >= o) incl += v;
+    }
+    s_dt[2 * l] = d0;
+    s_dt[2 * l + 1] = d1;
+    s_cum[2 * l] = (incl - pair) + v0;
+    s_cum[2 * l + 1] = incl;
+  }
+  __syncthreads();
+}
+
+// scores of a group's block: G[t][u] = C_t . B_u
+template <int N, typename T>
+__global__ void __launch_bounds__(kThreads) ssd_scores_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int kPitchN = N + 4;
+  float *sC = sm, *sB = sm + kT * kPitchN;
+  const int c = blockIdx.x, g = blockIdx.y, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  load_rows<N>(sC, kPitchN, static_cast<const T*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows, One{});
+  load_rows<N>(sB, kPitchN, static_cast<const T*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows, One{});
+  __syncthreads();
+  float acc[4][4];
+  zero(acc);
+  mm<4, 4, true, true>(acc, sC, kPitchN, sB, kPitchN, N, ty, tx);
+  float* out = p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[(ty + 16 * i) * kT + tx + 16 * j] = acc[i][j];
+}
+
+// kGrad = false: what a block adds to the state, sum_u exp(cum_end - cum_u) dt_u x_u B_u^T
+// kGrad = true : what its outputs' gradients put on its starting state, sum_t exp(cum_t) dy_t C_t^T
+template <int N, typename T, bool kGrad>
+__global__ void __launch_bounds__(kThreads) ssd_state_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int kPitchN = N + 4;
+  float *sX = sm, *sB = sX + kT * kPitchT, *s_dt = sB + kT * kPitchN, *s_cum = s_dt + kT;
+  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), g = h / (p.h / p.g);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  block_decay(s_dt, s_cum, p.dt + (static_cast<int64_t>(b) * p.l + t0) * p.h + h, p.h, rows, p.A[h]);
+  const float end = s_cum[kT - 1];
+  if constexpr (kGrad) {
+    load_rows<kP>(sX, kPitchT, static_cast<const T*>(p.dy) + ((static_cast<int64_t>(b) * p.l + t0) * p.h + h) * kP, static_cast<int64_t>(p.h) * kP, rows,
+                  [&](int r) { return expf(s_cum[r]); });
+    load_rows<N>(sB, kPitchN, static_cast<const T*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows, One{});
+  } else {
+    load_rows<kP>(sX, kPitchT, static_cast<const T*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP, p.x_sl, rows,
+                  [&](int r) { return expf(end - s_cum[r]) * s_dt[r]; });
+    load_rows<N>(sB, kPitchN, static_cast<const T*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows, One{});
+    if (threadIdx.x == 0) p.decay[(static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c] = expf(end);
+  }
+  __syncthreads();
+  float acc[4][N / 16];
+  zero(acc);
+  mm<4, N / 16, false, false>(acc, sX, kPitchT, sB, kPitchN, kT, ty, tx);
+  float* out = (kGrad ? p.dstates : p.states) + ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < N / 64; ++q)
+      *reinterpret_cast<float4*>(out + (ty * 4 + i) * N + q * 64 + tx * 4) = make_float4(acc[i][q * 4], acc[i][q * 4 + 1], acc[i][q * 4 + 2], acc[i][q * 4 + 3]);
+}
+
+// along the blocks, in place.  Forward: each block's contribution becomes the state it starts from.  Reverse: the gradient of each block's
+// starting state (its own outputs' part) becomes the gradient of the state it ends with.
+template <bool kReverse>
+__global__ void __launch_bounds__(kThreads) ssd_pass_kernel(float4* __restrict__ s, const float* __restrict__ decay, const float4* __restrict__ first,
+                                                            float4* __restrict__ last, int n_chunks, int per_head) {
+  const int64_t bh = blockIdx.y;
+  const int e = blockIdx.x * kThreads + threadIdx.x;
+  if (e >= per_head) return;
+  float4 run = first != nullptr ? first[bh * per_head + e] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4* base = s + bh * n_chunks * per_head + e;
+  const float* d = decay + bh * n_chunks;
+#pragma unroll 4
+  for (int i = 0; i < n_chunks; ++i) {
+    const int c = kReverse ? n_chunks - 1 - i : i;
+    const float4 v = base[static_cast<int64_t>(c) * per_head];
+    const float f = d[c];
+    base[static_cast<int64_t>(c) * per_head] = run;
+    run.x = fmaf(run.x, f, v.x); run.y = fmaf(run.y, f, v.y); run.z = fmaf(run.z, f, v.z); run.w = fmaf(run.w, f, v.w);
+  }
+  if (last != nullptr) last[bh * per_head + e] = run;
+}
+
+template <int N, typename T>
+__global__ void __launch_bounds__(kThreads) ssd_out_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int kPitchN = N + 4;
+  float *sM = sm, *sXT = sM + kT * kPitchT, *sC = sXT + kP * kPitchT, *sS = sC + kT * kPitchN, *s_dt = sS + kP * kPitchN, *s_cum = s_dt + kT;
+  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), g = h / (p.h / p.g);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  block_decay(s_dt, s_cum, p.dt + (static_cast<int64_t>(b) * p.l + t0) * p.h + h, p.h, rows, p.A[h]);
+  const float* G = p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT);
+  for (int i = threadIdx.x; i < kT * kT / 4; i += kThreads) {
+    const int t = i / (kT / 4), u = (i % (kT / 4)) * 4;
+    float4 v = *reinterpret_cast<const float4*>(G + t * kT + u);
+    float* e = reinterpret_cast<float*>(&v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = u + q <= t ? e[q] * expf(s_cum[t] - s_cum[u + q]) * s_dt[u + q] : 0.f;
+    *reinterpret_cast<float4*>(sM + t * kPitchT + u) = v;
+  }
+  const T* x = static_cast<const T*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP;
+  for (int i = threadIdx.x; i < kT * (kP / 4); i += kThreads) {
+    const int u = i % kT, q = (i / kT) * 4;
+    const float4 v = u < rows ? ld4(x + u * p.x_sl + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    sXT[q * kPitchT + u] = v.x;
+    sXT[(q + 1) * kPitchT + u] = v.y;
+    sXT[(q + 2) * kPitchT + u] = v.z;
+    sXT[(q + 3) * kPitchT + u] = v.w;
+  }
+  load_rows<N>(sC, kPitchN, static_cast<const T*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows, [&](int r) { return expf(s_cum[r]); });
+  load_rows<N>(sS, kPitchN, p.states + ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N), static_cast<int64_t>(N), kP, One{});
+  __syncthreads();
+  float acc[4][4];
+  zero(acc);
+  mm<4, 4, true, true>(acc, sM, kPitchT, sXT, kPitchT, kT, ty, tx);
+  mm<4, 4, true, true>(acc, sC, kPitchN, sS, kPitchN, N, ty, tx);
+  const float d = p.D[h];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sM[(ty + 16 * i) * kPitchT + tx + 16 * j] = fmaf(d, sXT[(tx + 16 * j) * kPitchT + ty + 16 * i], acc[i][j]);
+  __syncthreads();
+  T* y = static_cast<T*>(p.y) + ((static_cast<int64_t>(b) * p.l + t0) * p.h + h) * kP;
+  for (int i = threadIdx.x; i < rows * (kP / 4); i += kThreads) {
+    const int t = i / (kP / 4), q = (i % (kP / 4)) * 4;
+    st4(y + static_cast<int64_t>(t) * p.h * kP + q, *reinterpret_cast<const float4*>(sM + t * kPitchT + q));
+  }
+}
+
+// all gradients of one block for `per` heads of one group
+template <int N, typename T>
+__global__ void __launch_bounds__(kThreads, 1) ssd_grad_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int kPitchN = N + 4, NI = N / 16;
+  float* sC = sm;                              // [t][n]
+  float* sB = sC + kT * kPitchN;               // [u][n]
+  float* sS = sB + kT * kPitchN;               // [p][n] state at the block's start
+  float* sR = sS + kP * kPitchN;               // [p][n] gradient of the state at its end
+  float* sG = sR + kP * kPitchN;               // [t][u]
+  float* sX = sG + kT * kPitchT;               // [u][p]
+  float* sY = sX + kT * kPitchT;               // [t][p] dy
+  float* sM = sY + kT * kPitchT;               // [t][u] decayed scores, then the group's score gradients
+  float* sQ = sM + kT * kPitchT;               // [u][p] the end state's part of dx, then the score gradients transposed
+  float* s_dt = sQ + kT * kPitchT;
+  float *s_cum = s_dt + kT, *s_row = s_cum + kT, *s_end = s_row + kT, *s_dir = s_end + kT, *s_col = s_dir + kT, *s_red = s_col + 8 * kT;
+  const int c = blockIdx.x, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), hpg = p.h / p.g;
+  const int g = blockIdx.y / p.n_sub, sub = blockIdx.y % p.n_sub, per = hpg / p.n_sub;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, warp = tid >> 5, lane = tid & 31;
+  load_rows<N>(sC, kPitchN, static_cast<const T*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows, One{});
+  load_rows<N>(sB, kPitchN, static_cast<const T*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows, One{});
+  load_rows<kT>(sG, kPitchT, p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT), static_cast<int64_t>(kT), kT, One{});
+  float dC[4][NI], dB[4][NI], dG[4][4];
+  zero(dC);
+  zero(dB);
+  zero(dG);
+  for (int hi = 0; hi < per; ++hi) {
+    const int h = g * hpg + sub * per + hi;
+    const float a = p.A[h];
+    const int64_t row0 = (static_cast<int64_t>(b) * p.l + t0) * p.h + h, st0 = ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N);
+    __syncthreads();                           // the head before is done with its tiles
+    block_decay(s_dt, s_cum, p.dt + row0, p.h, rows, a);
+    load_rows<kP>(sX, kPitchT, static_cast<const T*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP, p.x_sl, rows, One{});
+    load_rows<kP>(sY, kPitchT, static_cast<const T*>(p.dy) + row0 * kP, static_cast<int64_t>(p.h) * kP, rows, One{});
+    load_rows<N>(sS, kPitchN, p.states + st0, static_cast<int64_t>(N), kP, One{});
+    load_rows<N>(sR, kPitchN, p.dstates + st0, static_cast<int64_t>(N), kP, One{});
+    __syncthreads();
+    const float end = s_cum[kT - 1];
+
+    // gradient of the scores, and through their decays of cum
+    {
+      float v[4][4], col[4] = {0.f, 0.f, 0.f, 0.f};
+      zero(v);
+      mm<4, 4, true, true>(v, sY, kPitchT, sX, kPitchT, kP, ty, tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = ty + 16 * i;
+        float row = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int u = tx + 16 * j;
+          const float w = u <= t ? expf(s_cum[t] - s_cum[u]) : 0.f, wg = w * sG[t * kPitchT + u];
+          sM[t * kPitchT + u] = wg;
+          const float d = v[i][j] * s_dt[u];
+          dG[i][j] = fmaf(d, w, dG[i][j]);
+          const float q = u < t ? d * wg : 0.f;           // on the diagonal the two ends cancel
+          row += q;
+          col[j] += q;
+        }
+        row = half_warp_sum(row);
+        if (tx == 0) s_row[t] = row;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        col[j] += __shfl_xor_sync(0xffffffffu, col[j], 16);
+        if (lane < 16) s_col[warp * kT + tx + 16 * j] = col[j];
+      }
+    }
+    // the end state's part of dx
+    {
+      float v[4][4];
+      zero(v);
+      mm<4, 4, true, true>(v, sB, kPitchN, sR, kPitchN, N, ty, tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float e = expf(end - s_cum[ty + 16 * i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sQ[(ty + 16 * i) * kPitchT + tx + 16 * j] = e * v[i][j];
+      }
+    }
+    // C through the starting state, B through the end state
+    {
+      float v[4][NI];
+      zero(v);
+      mm<4, NI, true, false>(v, sY, kPitchT, sS, kPitchN, kP, ty, tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int t = ty + 16 * i;
+        const float e = expf(s_cum[t]);
+        float row = 0.f;
+#pragma unroll
+        for (int j = 0; j < NI; ++j) {
+          const float w = e * v[i][j];
+          dC[i][j] += w;
+          row = fmaf(w, sC[t * kPitchN + col4(tx, j)], row);
+        }
+        row = half_warp_sum(row);
+        if (tx == 0) s_row[t] += row;
+      }
+    }
+    {
+      float v[4][NI];
+      zero(v);
+      mm<4, NI, true, false>(v, sX, kPitchT, sR, kPitchN, kP, ty, tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int u = ty + 16 * i;
+        const float e = expf(end - s_cum[u]) * s_dt[u];
+        float z = 0.f;
+#pragma unroll
+        for (int j = 0; j < NI; ++j) {
+          const float w = e * v[i][j];
+          dB[i][j] += w;
+          z = fmaf(w, sB[u * kPitchN + col4(tx, j)], z);
+        }
+        z = half_warp_sum(z);
+        if (tx == 0) s_end[u] = z;
+      }
+    }
+    __syncthreads();
+    // dx, dt through x, D, and the end state's gradient times the starting state
+    float dd = 0.f, rs = 0.f;
+    {
+      float v[4][4];
+      zero(v);
+      mm<4, 4, false, false>(v, sM, kPitchT, sY, kPitchT, kT, ty, tx);
+      const float d = p.D[h];
+      T* dx = static_cast<T*>(p.dx) + row0 * kP;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int u = ty * 4 + i;
+        float dir = 0.f, o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int q = tx * 4 + j;
+          const float pre = v[i][j] + sQ[u * kPitchT + q], xv = sX[u * kPitchT + q], yv = sY[u * kPitchT + q];
+          dir = fmaf(xv, pre, dir);
+          dd = fmaf(xv, yv, dd);
+          o[j] = fmaf(s_dt[u], pre, d * yv);
+        }
+        if (u < rows) st4(dx + static_cast<int64_t>(u) * p.h * kP + tx * 4, make_float4(o[0], o[1], o[2], o[3]));
+        dir = half_warp_sum(dir);
+        if (tx == 0) s_dir[u] = dir;
+      }
+      for (int i = tid; i < kP * (N / 4); i += kThreads) {
+        const int r = i / (N / 4), q = (i % (N / 4)) * 4;
+        const float4 s = *reinterpret_cast<const float4*>(sS + r * kPitchN + q), e = *reinterpret_cast<const float4*>(sR + r * kPitchN + q);
+        rs += s.x * e.x + s.y * e.y + s.z * e.z + s.w * e.w;
+      }
+      dd = dev::warp_sum(dd);
+      rs = dev::warp_sum(rs);
+      if (lane == 0) {
+        s_red[warp] = dd;
+        s_red[8 + warp] = rs;
+      }
+    }
+    __syncthreads();
+    // cum's gradient summed from the block's end, for dt and A
+    if (warp == 0) {
+      float g0[2], z = 0.f, acc_d = 0.f, acc_r = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        acc_d += s_red[w];
+        acc_r += s_red[8 + w];
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = 2 * lane + e;
+        float v = s_row[t] - s_end[t];
+        z += s_end[t];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v -= s_col[w * kT + t];
+        g0[e] = v;
+      }
+      z = dev::warp_sum(z);
+      if (lane == 31) g0[1] += z + expf(end) * acc_r;
+      float incl = g0[0] + g0[1];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float v = __shfl_down_sync(0xffffffffu, incl, o);
+        if (lane + o < 32) incl += v;
+      }
+      const float dda0 = incl, dda1 = incl - g0[0];
+      const int t = 2 * lane;
+      if (t < rows) p.ddt[row0 + static_cast<int64_t>(t) * p.h] = fmaf(a, dda0, s_dir[t]);
+      if (t + 1 < rows) p.ddt[row0 + static_cast<int64_t>(t + 1) * p.h] = fmaf(a, dda1, s_dir[t + 1]);
+      const float da = dev::warp_sum(s_dt[t] * dda0 + s_dt[t + 1] * dda1);
+      if (lane == 0) {
+        const int64_t at = (static_cast<int64_t>(b) * p.n_chunks + c) * p.h + h;
+        p.dA[at] = da;
+        p.dD[at] = acc_d;
+      }
+    }
+  }
+  // the scores' gradients into B and C
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sM[(ty + 16 * i) * kPitchT + tx + 16 * j] = dG[i][j];
+      sQ[(tx + 16 * j) * kPitchT + ty + 16 * i] = dG[i][j];
+    }
+  __syncthreads();
+  mm<4, NI, true, false>(dC, sM, kPitchT, sB, kPitchN, kT, ty, tx);
+  mm<4, NI, true, false>(dB, sQ, kPitchT, sC, kPitchN, kT, ty, tx);
+  const int64_t plane = static_cast<int64_t>(p.b) * p.l * p.g * N;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = ty + 16 * i;
+    if (t >= rows) continue;
+    const int64_t at = ((static_cast<int64_t>(b) * p.l + t0 + t) * p.g + g) * N + tx * 4;
+#pragma unroll
+    for (int q = 0; q < N / 64; ++q) {
+      const float4 vb = make_float4(dB[i][q * 4], dB[i][q * 4 + 1], dB[i][q * 4 + 2], dB[i][q * 4 + 3]);
+      const float4 vc = make_float4(dC[i][q * 4], dC[i][q * 4 + 1], dC[i][q * 4 + 2], dC[i][q * 4 + 3]);
+      if (p.n_sub == 1) {
+        st4(static_cast<T*>(p.dB) + at + q * 64, vb);
+        st4(static_cast<T*>(p.dC) + at + q * 64, vc);
+      } else {
+        st4(p.partial + sub * 2 * plane + at + q * 64, vb);
+        st4(p.partial + (sub * 2 + 1) * plane + at + q * 64, vc);
+      }
+    }
+  }
+}
+
+// dB and dC from the partial sums of n_sub CTAs
+template <typename T>
+__global__ void __launch_bounds__(kThreads) ssd_merge_kernel(const float4* __restrict__ part, T* __restrict__ dB, T* __restrict__ dC, int64_t plane4, int n_sub) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  if (i >= 2 * plane4) return;
+  const int64_t at = i % plane4;
+  float4 s = part[i];
+  for (int k = 1; k < n_sub; ++k) {
+    const float4 v = part[k * 2 * plane4 + i];
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  st4((i < plane4 ? dB : dC) + at * 4, s);
+}
+
+template <int N> constexpr int scores_smem() { return 2 * kT * (N + 4) * 4; }
+template <int N> constexpr int state_smem() { return (kT * kPitchT + kT * (N + 4) + 2 * kT) * 4; }
+template <int N> constexpr int out_smem() { return (2 * kT * kPitchT + 2 * kT * (N + 4) + 2 * kT) * 4; }
+template <int N> constexpr int grad_smem() { return (4 * kT * (N + 4) + 5 * kT * kPitchT + 13 * kT + 16) * 4; }
+static_assert(grad_smem<128>() <= 232448, "one CTA's shared memory");
+
+template <typename K>
+bool with_smem(K kern, int bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+
+template <int N, typename T>
+bool forward(const SsdArgs& p, cudaStream_t s) {
+  static const bool ok = with_smem(ssd_scores_kernel<N, T>, scores_smem<N>()) && with_smem(ssd_state_kernel<N, T, false>, state_smem<N>()) &&
+                         with_smem(ssd_out_kernel<N, T>, out_smem<N>());
+  if (!ok) return false;
+  ssd_scores_kernel<N, T><<<dim3(p.n_chunks, p.g, p.b), kThreads, scores_smem<N>(), s>>>(p);
+  ssd_state_kernel<N, T, false><<<dim3(p.n_chunks, p.h, p.b), kThreads, state_smem<N>(), s>>>(p);
+  constexpr int per = kP * N / 4;
+  ssd_pass_kernel<false><<<dim3(per / kThreads, p.b * p.h), kThreads, 0, s>>>(reinterpret_cast<float4*>(p.states), p.decay,
+                                                                              reinterpret_cast<const float4*>(p.first), reinterpret_cast<float4*>(p.last),
+                                                                              p.n_chunks, per);
+  ssd_out_kernel<N, T><<<dim3(p.n_chunks, p.h, p.b), kThreads, out_smem<N>(), s>>>(p);
+  return true;
+}
+
+template <int N, typename T>
+bool backward(const SsdArgs& p, cudaStream_t s) {
+  static const bool ok = with_smem(ssd_state_kernel<N, T, true>, state_smem<N>()) && with_smem(ssd_grad_kernel<N, T>, grad_smem<N>());
+  if (!ok) return false;
+  ssd_state_kernel<N, T, true><<<dim3(p.n_chunks, p.h, p.b), kThreads, state_smem<N>(), s>>>(p);
+  constexpr int per = kP * N / 4;
+  ssd_pass_kernel<true><<<dim3(per / kThreads, p.b * p.h), kThreads, 0, s>>>(reinterpret_cast<float4*>(p.dstates), p.decay,
+                                                                             reinterpret_cast<const float4*>(p.dlast), reinterpret_cast<float4*>(p.dfirst),
+                                                                             p.n_chunks, per);
+  ssd_grad_kernel<N, T><<<dim3(p.n_chunks, p.g * p.n_sub, p.b), kThreads, grad_smem<N>(), s>>>(p);
+  if (p.n_sub > 1) {
+    const int64_t plane4 = static_cast<int64_t>(p.b) * p.l * p.g * N / 4;
+    ssd_merge_kernel<T><<<static_cast<unsigned>((2 * plane4 + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+        reinterpret_cast<const float4*>(p.partial), static_cast<T*>(p.dB), static_cast<T*>(p.dC), plane4, p.n_sub);
+  }
+  return true;
+}
+
+}  // namespace
+
+int ssd_block() { return kT; }
+
+// a group's heads are shared among so many CTAs (a divisor of their number) that the grid fills the SMs three times over
+int ssd_subgroups(int n_chunks, int groups, int batch, int heads_per_group) {
+  int n = 1;
+  while (n < heads_per_group && static_cast<int64_t>(n_chunks) * groups * batch * n < 3 * 148) {
+    ++n;
+    while (heads_per_group % n != 0) ++n;
+  }
+  return n;
+}
+
+bool ssd_supported(int head_dim, int state_dim) { return head_dim == kP && (state_dim == 64 || state_dim == 128); }
+
+bool ssd_forward(const SsdArgs& p, int state_dim, bool bf16, cudaStream_t s) {
+  if (state_dim == 128) return bf16 ? forward<128, __nv_bfloat16>(p, s) : forward<128, float>(p, s);
+  return bf16 ? forward<64, __nv_bfloat16>(p, s) : forward<64, float>(p, s);
+}
+bool ssd_backward(const SsdArgs& p, int state_dim, bool bf16, cudaStream_t s) {
+  if (state_dim == 128) return bf16 ? backward<128, __nv_bfloat16>(p, s) : backward<128, float>(p, s);
+  return bf16 ? backward<64, __nv_bfloat16>(p, s) : backward<64, float>(p, s);
+}
+
+}  // namespace b200seq

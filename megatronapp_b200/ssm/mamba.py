@@ -3,9 +3,8 @@
 Parity: reference ``core/ssm/`` -- ``MambaMixer`` (in_proj -> causal depthwise conv1d -> selective
 state-space scan with scalar-per-head A, grouped B/C, D skip, gated RMSNorm -> out_proj),
 ``mamba_hybrid_layer_allocation.py`` (``Symbols``: ``M`` mamba, ``*`` attention, ``-`` MLP; ratio
-based allocation and explicit override patterns) and ``MambaStack``.  The scan is a chunked
-(block-parallel) PyTorch implementation of the SSD recurrence; the reference calls
-``mamba_ssm`` Triton kernels (SURVEY K23 marks the hand-written kernel a stretch goal).
+based allocation and explicit override patterns) and ``MambaStack``.  The scan is block-parallel: hand-written kernels for the usual
+head and state sizes on the GPU, the same blocks in PyTorch elsewhere; the reference calls ``mamba_ssm`` Triton kernels.
 """
 from __future__ import annotations
 
@@ -52,7 +51,7 @@ def allocate_layers(total_layers: int, attention_ratio: float, mlp_ratio: float,
     return layers
 
 
-def ssd_scan(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
+def ssd_scan_torch(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
     """x [b, l, h, p], dt [b, l, h] (>0), A [h] (<0), B/C [b, l, g, n], D [h] -> y [b, l, h, p], final state.
     Recurrence per head: S_t = exp(dt_t A) S_{t-1} + dt_t x_t B_t^T ;  y_t = S_t C_t + D x_t."""
     b, l, h, p = x.shape
@@ -71,10 +70,10 @@ def ssd_scan(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
         xb = xf[:, s:e] * dtf[:, s:e].unsqueeze(-1)                   # dt * x
         Bc, Cc = Bh[:, s:e], Ch[:, s:e]
         # intra-chunk: y_t += sum_{u<=t} exp(cum_t - cum_u) (C_t . B_u) dt_u x_u
-        L = torch.exp(cum.unsqueeze(2) - cum.unsqueeze(1))            # [b, t, u, h]
         c_len = e - s
-        mask = torch.tril(torch.ones(c_len, c_len, device=x.device, dtype=torch.bool))
-        L = L.masked_fill(~mask.view(1, c_len, c_len, 1), 0.0)
+        mask = torch.tril(torch.ones(c_len, c_len, device=x.device, dtype=torch.bool)).view(1, c_len, c_len, 1)
+        # [b, t, u, h]; masked before the exponential, which overflows above the diagonal and would turn the gradient into NaN
+        L = torch.exp((cum.unsqueeze(2) - cum.unsqueeze(1)).masked_fill(~mask, float("-inf")))
         G = torch.einsum("bthn,buhn->btuh", Cc, Bc) * L
         y = torch.einsum("btuh,buhp->bthp", G, xb)
         # contribution of the carried state: y_t += exp(cum_t) C_t . S_prev
@@ -85,6 +84,59 @@ def ssd_scan(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
         ys.append(y)
     y = torch.cat(ys, dim=1) + xf * D.float().view(1, 1, h, 1)
     return y.to(x.dtype), state
+
+
+class _SSDFn(torch.autograd.Function):
+    """The scan through csrc/seqmix/seqmix_ssd.cu.  A gradient that is to be differentiated again goes through the PyTorch form."""
+
+    @staticmethod
+    def forward(ctx, x, dt, A, B, C, D, init):
+        from ..ops import seqmix
+
+        y, last, scores, states, decay = seqmix.ext().ssd_forward(x, dt, A, B, C, D, init)
+        ctx.set_materialize_grads(False)
+        ctx.has_init = init is not None
+        ctx.save_for_backward(x, dt, A, B, C, D, scores, states, decay, *([init] if ctx.has_init else []))
+        return y, last
+
+    @staticmethod
+    def backward(ctx, dy, dlast):
+        x, dt, A, B, C, D, scores, states, decay, *init = ctx.saved_tensors
+        if dy is None and dlast is None:
+            return (None,) * 7
+        if torch.is_grad_enabled():
+            ins = [x, dt, A, B, C, D, *init]
+            y, last = ssd_scan_torch(x, dt, A, B, C, D, initial_state=init[0] if init else None)
+            outs = [(o, g) for o, g in ((y, dy), (last, dlast)) if g is not None]
+            want = [t for t, n in zip(ins, ctx.needs_input_grad) if n]
+            got = iter(torch.autograd.grad([o for o, _ in outs], want, [g for _, g in outs], create_graph=True, allow_unused=True))
+            return tuple(next(got) if n else None for n in ctx.needs_input_grad[:len(ins)]) + ((None,) * (7 - len(ins)))
+        from ..ops import seqmix
+
+        dy = torch.zeros_like(x, memory_format=torch.contiguous_format) if dy is None else dy.contiguous()
+        dlast = None if dlast is None else dlast.contiguous()
+        dx, ddt, dA, dB, dC, dD, dfirst = seqmix.ext().ssd_backward(dy, dlast, x, dt, A, B, C, D, scores, states, decay,
+                                                                    bool(ctx.has_init and ctx.needs_input_grad[6]))
+        return dx, ddt, dA, dB, dC, dD, dfirst
+
+
+def _steps(t: torch.Tensor) -> torch.Tensor:
+    """``[b, l, heads, dim]`` as the kernels take it: aligned rows of contiguous heads, any step and batch strides."""
+    ok = t.stride(3) == 1 and t.stride(2) == t.shape[3] and t.stride(1) % 8 == 0 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    return t if ok else t.clone(memory_format=torch.contiguous_format)
+
+
+def ssd_scan(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
+    """x [b, l, h, p], dt [b, l, h] (>0), A [h] (<0), B/C [b, l, g, n], D [h] -> y [b, l, h, p], final state (fp32).
+    Recurrence per head: S_t = exp(dt_t A) S_{t-1} + dt_t x_t B_t^T ;  y_t = S_t C_t + D x_t.  bf16 / fp32 CUDA tensors with 64-wide heads and
+    64 or 128 states run on the block kernels (64 steps a block, whatever ``chunk`` says), others, and tensors under forward-mode or
+    functorch transforms, in the PyTorch form."""
+    if (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and B.dtype == C.dtype == x.dtype and x.shape[3] == 64 and B.shape[3] in (64, 128)
+            and x.shape[2] % B.shape[2] == 0 and x.numel() > 0 and x.shape[0] * x.shape[2] <= 65535
+            and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()):
+        f32 = lambda t: t.float().contiguous()  # noqa: E731
+        return _SSDFn.apply(_steps(x), f32(dt), f32(A), _steps(B), _steps(C), f32(D), None if initial_state is None else f32(initial_state))
+    return ssd_scan_torch(x, dt, A, B, C, D, chunk, initial_state)
 
 
 @dataclass

@@ -1,0 +1,75 @@
+"""The Mamba-2 scan's block kernels against the step-by-step recurrence in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _oracle(x, dt, A, B, C, D, init):
+    b, l, h, p = x.shape
+    rep = h // B.shape[2]
+    B, C = (t.repeat_interleave(rep, dim=2) for t in (B, C))
+    S = init if init is not None else x.new_zeros(b, h, p, B.shape[3])
+    ys = []
+    for t in range(l):
+        S = S * torch.exp(dt[:, t] * A)[..., None, None] + (dt[:, t, :, None] * x[:, t]).unsqueeze(-1) * B[:, t].unsqueeze(-2)
+        ys.append((S * C[:, t].unsqueeze(-2)).sum(-1) + D.view(1, h, 1) * x[:, t])
+    return torch.stack(ys, 1), S
+
+
+def _case(b, l, h, g, n, dtype, init, steep=1.0, seed=0):
+    q = torch.Generator("cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=q, device="cuda")  # noqa: E731
+    # x, B and C as columns of one tensor, as the convolution leaves them
+    xbc = rnd(b, l, h * 64 + 2 * g * n).to(dtype)
+    x, B, C = xbc.split([h * 64, g * n, g * n], -1)
+    ins = [x.reshape(b, l, h, 64), torch.rand(b, l, h, generator=q, device="cuda") * 0.2 * steep, -torch.rand(h, generator=q, device="cuda") * 8 - 0.1,
+           B.reshape(b, l, g, n), C.reshape(b, l, g, n), rnd(h)]
+    return [t.requires_grad_() for t in ins] + [rnd(b, h, 64, n).requires_grad_() if init else None]
+
+
+@pytest.mark.parametrize("b,l,h,g,n,dtype,init,steep", [
+    (1, 1, 1, 1, 64, torch.float32, True, 1.0),               # one step from a state
+    (2, 63, 2, 1, 64, torch.float32, False, 1.0),
+    (1, 65, 4, 2, 128, torch.float32, True, 1.0),             # a second block of one step
+    (1, 200, 6, 1, 64, torch.float32, False, 1.0),            # six heads of one group over several CTAs
+    (2, 130, 8, 8, 128, torch.bfloat16, False, 1.0),          # a group per head
+    (1, 192, 3, 1, 128, torch.float32, True, 100.0)])         # decays that vanish: exponentials above the diagonal would overflow
+def test_against_the_recurrence(b, l, h, g, n, dtype, init, steep):
+    from megatronapp_b200.ops import seqmix
+    from megatronapp_b200.ssm.mamba import ssd_scan
+
+    ins = _case(b, l, h, g, n, dtype, init, steep)
+    before = seqmix.ext().launch_count()
+    y, last = ssd_scan(*ins[:6], initial_state=ins[6])
+    assert seqmix.ext().launch_count() == before + 4 and y.dtype == dtype and last.dtype == torch.float32
+    wide = [None if t is None else t.detach().double().requires_grad_() for t in ins]
+    want_y, want_last = _oracle(*wide)
+    dy, dl = torch.randn_like(y), torch.randn_like(last)
+    got = torch.autograd.grad((y, last), [t for t in ins if t is not None], (dy, dl))
+    want = torch.autograd.grad((want_y, want_last), [t for t in wide if t is not None], (dy.double(), dl.double()))
+    # decays inside a block are exponentials of differences of running sums: sums as large as `c` in fp32 leave 2^-23 c in the exponent
+    c = float((wide[1] * -wide[2]).detach().sum(1).max()) * min(1.0, 64 / l)
+    for i, (a, w) in enumerate(zip([y, last, *got], [want_y, want_last, *want])):
+        # fp32 sums over at most 200 steps and 128 columns of terms of either sign; results in x's type carry its rounding
+        tol = 2e-5 + 2.0 ** -23 * c if a.dtype == torch.float32 else 2.0 ** -8
+        assert torch.isfinite(a).all()
+        assert float((a.detach().double() - w.detach()).norm()) <= tol * max(float(w.norm()), 1e-6), i
+
+
+def test_other_ways_to_differentiate():
+    """Only the final state's gradient, a second derivative, and forward-mode take the routes that they need."""
+    from megatronapp_b200.ssm.mamba import ssd_scan, ssd_scan_torch
+
+    ins = _case(1, 70, 2, 1, 64, torch.float32, True)
+    outs = [torch.autograd.grad(f(*ins[:6], initial_state=ins[6])[1].square().sum(), ins[1]) for f in (ssd_scan, ssd_scan_torch)]
+    assert torch.allclose(outs[0][0], outs[1][0], rtol=1e-3, atol=1e-3 * float(outs[1][0].abs().max()))
+    twice = []
+    for f in (ssd_scan, ssd_scan_torch):
+        g, = torch.autograd.grad(f(*ins[:6], initial_state=ins[6])[0].square().sum(), ins[1], create_graph=True)
+        twice.append(torch.autograd.grad(g.square().sum(), ins[0])[0])
+    assert torch.allclose(twice[0], twice[1], rtol=1e-3, atol=1e-3 * float(twice[1].abs().max()))
+    with torch.autograd.forward_ad.dual_level():
+        x = torch.autograd.forward_ad.make_dual(ins[0].detach(), torch.ones_like(ins[0]))
+        y, _ = ssd_scan(x, *[t.detach() for t in ins[1:6]])
+        assert torch.autograd.forward_ad.unpack_dual(y).tangent is not None
