@@ -962,6 +962,79 @@ std::vector<Tensor> ssd_backward(const Tensor& dy, c10::optional<Tensor> dlast, 
   return {dx, ddt, dA.sum(at::IntArrayRef{0, 1}), dB, dC, dD.sum(at::IntArrayRef{0, 1}), dfirst};
 }
 
+// zx [s, b, 2 di + 2 gn + heads] contiguous, everything of its type but dt_bias and eps
+b200seq::MambaArgs mamba_args(const Tensor& zx, const Tensor& conv_w, const Tensor& conv_b, const Tensor& dt_bias, const Tensor& norm_w, int64_t groups,
+                              double eps) {
+  act_is_bf16(zx, "zx");
+  auto fits = [&](const Tensor& t, int64_t n) {
+    return t.is_cuda() && t.scalar_type() == zx.scalar_type() && t.is_contiguous() && t.numel() == n && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  check_f32(dt_bias, "dt_bias");
+  b200seq::MambaArgs p{};
+  TORCH_CHECK(zx.dim() == 3 && zx.numel() < (int64_t{1} << 40), "zx must be [s, b, width]");
+  p.s = static_cast<int>(zx.size(0)); p.b = static_cast<int>(zx.size(1)); p.width = static_cast<int>(zx.size(2));
+  p.di = static_cast<int>(norm_w.numel()); p.conv = static_cast<int>(conv_b.numel()); p.heads = static_cast<int>(dt_bias.numel());
+  p.groups = static_cast<int>(groups); p.eps = static_cast<float>(eps);
+  TORCH_CHECK(fits(zx, zx.numel()) && fits(conv_w, int64_t{4} * p.conv) && fits(conv_b, p.conv) && fits(norm_w, p.di), "operands of zx's type, contiguous, 16-byte aligned");
+  TORCH_CHECK(p.s > 0 && p.b > 0 && p.b <= 65535 && p.width == p.di + p.conv + p.heads && p.width % 4 == 0 && p.di % 4 == 0 && p.conv % 8 == 0 && p.conv > p.di &&
+              (p.conv - p.di) % 8 == 0 && p.groups > 0 && p.groups <= 65535 && p.di % p.groups == 0 && (p.di / p.groups) % 4 == 0 && p.di / p.groups <= 4096 &&
+              (p.s + 15) / 16 <= 65535, "unsupported mixer sizes");
+  p.zx = zx.data_ptr(); p.conv_w = conv_w.data_ptr(); p.conv_b = conv_b.data_ptr(); p.dt_bias = dt_bias.data_ptr<float>(); p.norm_w = norm_w.data_ptr();
+  return p;
+}
+// -> convolved x B C [b, s, conv], dt [b, s, heads]
+std::vector<Tensor> mamba_before_scan(const Tensor& zx, const Tensor& conv_w, const Tensor& conv_b, const Tensor& dt_bias, const Tensor& norm_w, int64_t groups) {
+  c10::cuda::CUDAGuard g(zx.device());
+  b200seq::MambaArgs p = mamba_args(zx, conv_w, conv_b, dt_bias, norm_w, groups, 0.0);
+  Tensor xbc = torch::empty({p.b, p.s, p.conv}, zx.options()), dt = torch::empty({p.b, p.s, p.heads}, dt_bias.options());
+  p.xbc = xbc.data_ptr(); p.dt = dt.data_ptr<float>();
+  b200seq::mamba_before_scan(p, zx.scalar_type() == at::kBFloat16, cur_stream());
+  count(2); check_last_error("mamba_before_scan");
+  return {xbc, dt};
+}
+// -> out [s, b, di], rstd [s, b, groups]
+std::vector<Tensor> mamba_gated_norm(const Tensor& y, const Tensor& zx, const Tensor& conv_w, const Tensor& conv_b, const Tensor& dt_bias, const Tensor& norm_w,
+                                     int64_t groups, double eps) {
+  c10::cuda::CUDAGuard g(zx.device());
+  b200seq::MambaArgs p = mamba_args(zx, conv_w, conv_b, dt_bias, norm_w, groups, eps);
+  TORCH_CHECK(y.is_contiguous() && y.scalar_type() == zx.scalar_type() && y.numel() == static_cast<int64_t>(p.s) * p.b * p.di, "bad y");
+  Tensor out = torch::empty({p.s, p.b, p.di}, zx.options()), rstd = torch::empty({p.s, p.b, p.groups}, dt_bias.options());
+  p.y = y.data_ptr(); p.out = out.data_ptr(); p.rstd = rstd.data_ptr<float>();
+  b200seq::mamba_gated_norm(p, zx.scalar_type() == at::kBFloat16, cur_stream());
+  count(); check_last_error("mamba_gated_norm");
+  return {out, rstd};
+}
+// the norm's half of the backward -> dy [b, s, di], dzx [s, b, width] with its z columns filled, d(norm weight) fp32 [di]
+std::vector<Tensor> mamba_gated_norm_grad(const Tensor& dout, const Tensor& rstd, const Tensor& y, const Tensor& zx, const Tensor& conv_w, const Tensor& conv_b,
+                                          const Tensor& dt_bias, const Tensor& norm_w, int64_t groups) {
+  c10::cuda::CUDAGuard g(zx.device());
+  b200seq::MambaArgs p = mamba_args(zx, conv_w, conv_b, dt_bias, norm_w, groups, 0.0);
+  TORCH_CHECK(y.is_contiguous() && y.scalar_type() == zx.scalar_type() && y.numel() == static_cast<int64_t>(p.s) * p.b * p.di, "bad y");
+  TORCH_CHECK(dout.is_contiguous() && dout.scalar_type() == zx.scalar_type() && dout.numel() == y.numel() && reinterpret_cast<uintptr_t>(dout.data_ptr()) % 16 == 0, "bad dout");
+  check_f32(rstd, "rstd");
+  Tensor dy = torch::empty_like(y), dzx = torch::empty_like(zx), part = torch::empty({b200seq::mamba_norm_parts(p.s, p.b), p.di}, dt_bias.options());
+  p.y = y.data_ptr(); p.dout = dout.data_ptr(); p.rstd = rstd.data_ptr<float>(); p.dy = dy.data_ptr(); p.dzx = dzx.data_ptr(); p.norm_part = part.data_ptr<float>();
+  b200seq::mamba_gated_norm_grad(p, zx.scalar_type() == at::kBFloat16, cur_stream());
+  count(); check_last_error("mamba_gated_norm_grad");
+  return {dy, dzx, part.sum(0)};
+}
+// the other half: fills dzx's columns x B C and dt -> d(taps and bias) fp32 [5, conv], d(dt_bias) fp32 [heads].  ddt is overwritten.
+std::vector<Tensor> mamba_before_scan_grad(const Tensor& dxs, const Tensor& dB, const Tensor& dC, Tensor ddt, Tensor dzx, const Tensor& zx, const Tensor& conv_w,
+                                           const Tensor& conv_b, const Tensor& dt_bias, const Tensor& norm_w, int64_t groups) {
+  c10::cuda::CUDAGuard g(zx.device());
+  b200seq::MambaArgs p = mamba_args(zx, conv_w, conv_b, dt_bias, norm_w, groups, 0.0);
+  const int64_t rows = static_cast<int64_t>(p.s) * p.b, gn = (p.conv - p.di) / 2;
+  for (const Tensor* t : {&dxs, &dB, &dC}) TORCH_CHECK(t->is_contiguous() && t->scalar_type() == zx.scalar_type() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "bad gradients");
+  TORCH_CHECK(dxs.numel() == rows * p.di && dB.numel() == rows * gn && dC.numel() == rows * gn && ddt.numel() == rows * p.heads && dzx.is_contiguous() &&
+              dzx.sizes() == zx.sizes() && dzx.scalar_type() == zx.scalar_type(), "bad gradients");
+  check_f32(ddt, "ddt");
+  Tensor part = torch::empty({static_cast<int64_t>(p.b) * b200seq::mamba_conv_parts(p.s), 5, p.conv}, dt_bias.options());
+  p.dxs = dxs.data_ptr(); p.dB = dB.data_ptr(); p.dC = dC.data_ptr(); p.ddt = ddt.data_ptr<float>(); p.dzx = dzx.data_ptr(); p.conv_part = part.data_ptr<float>();
+  b200seq::mamba_before_scan_grad(p, zx.scalar_type() == at::kBFloat16, cur_stream());
+  count(2); check_last_error("mamba_before_scan_grad");
+  return {part.sum(0), ddt.view({rows, p.heads}).sum(0)};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -995,6 +1068,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gen_delta_scan", &gen_delta_scan);
   m.def("mingru_scan", &mingru_scan);
   m.def("clamped_glu", &clamped_glu);
+  m.def("mamba_before_scan", &mamba_before_scan);
+  m.def("mamba_gated_norm", &mamba_gated_norm);
+  m.def("mamba_gated_norm_grad", &mamba_gated_norm_grad);
+  m.def("mamba_before_scan_grad", &mamba_before_scan_grad);
   m.def("ssd_forward", &ssd_forward);
   m.def("ssd_backward", &ssd_backward);
   m.def("launch_count", []() { return g_launches.load(); });

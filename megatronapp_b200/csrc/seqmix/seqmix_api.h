@@ -326,4 +326,33 @@ bool ssd_supported(int head_dim, int state_dim);
 bool ssd_forward(const SsdArgs& p, int state_dim, bool bf16, cudaStream_t s);
 bool ssd_backward(const SsdArgs& p, int state_dim, bool bf16, cudaStream_t s);
 
+// the parts of a Mamba-2 mixer around its scan; T = fp32 or bf16
+struct MambaArgs {
+  const void* zx;                 // [s, b, width]: z [di], x B C [conv], dt [heads]
+  const void *conv_w, *conv_b;    // [conv, 4], [conv]
+  const float* dt_bias;           // [heads]
+  void* xbc;                      // [b, s, conv]
+  float* dt;                      // [b, s, heads]
+  const void* y;                  // [b, s, di] the scan's result
+  const void* norm_w;             // [di]
+  void* out;                      // [s, b, di]
+  float* rstd;                    // [s, b, groups]
+  // gradients
+  const void* dout;               // [s, b, di]
+  void* dy;                       // [b, s, di]
+  const void *dxs, *dB, *dC;      // [b, s, di], [b, s, gn]
+  float* ddt;                     // [b, s, heads]: in d dt, out d(columns)
+  void* dzx;                      // [s, b, width]
+  float* conv_part;               // [b * mamba_conv_parts, 5, conv]: four taps, bias
+  float* norm_part;               // [mamba_norm_parts, di]
+  int s, b, width, di, conv, heads, groups;
+  float eps;
+};
+int mamba_conv_parts(int steps);
+int mamba_norm_parts(int steps, int batch);
+void mamba_before_scan(const MambaArgs& p, bool bf16, cudaStream_t s);
+void mamba_before_scan_grad(const MambaArgs& p, bool bf16, cudaStream_t s);
+void mamba_gated_norm(const MambaArgs& p, bool bf16, cudaStream_t s);
+void mamba_gated_norm_grad(const MambaArgs& p, bool bf16, cudaStream_t s);
+
 }  // namespace b200seq

@@ -139,6 +139,67 @@ def ssd_scan(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
     return ssd_scan_torch(x, dt, A, B, C, D, chunk, initial_state)
 
 
+def mixer_core_torch(zx, conv_w, conv_b, dt_bias, A, D, norm_w, groups: int, headdim: int, chunk: int = 64, scan=None):
+    """Between a mixer's two projections: ``zx [s, b, z | x B C | dt]`` -> gated, normed ``[s, b, d_inner]`` (fp32)."""
+    s, b, _ = zx.shape
+    zx = zx.transpose(0, 1)
+    di, c, nh = norm_w.numel(), conv_b.numel(), dt_bias.numel()
+    gn = (c - di) // 2
+    z, xBC, dt = torch.split(zx, [di, c, nh], dim=-1)
+    xBC = F.silu(F.conv1d(xBC.transpose(1, 2), conv_w, conv_b, padding=conv_w.shape[-1] - 1, groups=c)[..., :s].transpose(1, 2))
+    x, B, C = torch.split(xBC, [di, gn, gn], dim=-1)
+    dt = F.softplus(dt.float() + dt_bias)
+    y, _ = (scan or ssd_scan)(x.reshape(b, s, nh, headdim), dt, A, B.reshape(b, s, groups, gn // groups), C.reshape(b, s, groups, gn // groups), D, chunk)
+    y = (y.reshape(b, s, di) * F.silu(z)).float().view(b, s, groups, di // groups)     # gated RMSNorm, one statistic per B/C group
+    return ((y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5)).view(b, s, di) * norm_w.float()).transpose(0, 1)
+
+
+class _MixerCoreFn(torch.autograd.Function):
+    """``mixer_core_torch`` through csrc/seqmix/seqmix_mamba.cu and seqmix_ssd.cu."""
+
+    @staticmethod
+    def forward(ctx, zx, conv_w, conv_b, dt_bias, A, D, norm_w, groups, headdim):
+        from ..ops import seqmix
+
+        ext = seqmix.ext()
+        s, b, _ = zx.shape
+        di, nh = norm_w.numel(), dt_bias.numel()
+        gn = (conv_b.numel() - di) // 2
+        xbc, dt = ext.mamba_before_scan(zx, conv_w, conv_b, dt_bias, norm_w, groups)
+        x, B, C = _scan_views(xbc, di, gn, nh, headdim, groups)
+        y, _, scores, states, decay = ext.ssd_forward(x, dt, A, B, C, D, None)
+        out, rstd = ext.mamba_gated_norm(y, zx, conv_w, conv_b, dt_bias, norm_w, groups, 1e-5)
+        ctx.save_for_backward(zx, conv_w, conv_b, dt_bias, A, D, norm_w, xbc, dt, y, rstd, scores, states, decay)
+        ctx.groups, ctx.headdim = groups, headdim
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        zx, conv_w, conv_b, dt_bias, A, D, norm_w, xbc, dt, y, rstd, scores, states, decay = ctx.saved_tensors
+        groups = ctx.groups
+        if torch.is_grad_enabled():                     # to be differentiated again
+            ins = [zx, conv_w, conv_b, dt_bias, A, D, norm_w]
+            o = mixer_core_torch(*ins, groups, ctx.headdim, scan=ssd_scan_torch).to(dout.dtype)
+            got = iter(torch.autograd.grad(o, [t for t, n in zip(ins, ctx.needs_input_grad) if n], dout, create_graph=True, allow_unused=True))
+            return tuple(next(got) if n else None for n in ctx.needs_input_grad[:7]) + (None, None)
+        from ..ops import seqmix
+
+        ext = seqmix.ext()
+        di, nh = norm_w.numel(), dt_bias.numel()
+        gn = (conv_b.numel() - di) // 2
+        x, B, C = _scan_views(xbc, di, gn, nh, ctx.headdim, groups)
+        dy, dzx, dnorm = ext.mamba_gated_norm_grad(dout.contiguous(), rstd, y, zx, conv_w, conv_b, dt_bias, norm_w, groups)
+        dx, ddt, dA, dB, dC, dD, _ = ext.ssd_backward(dy, None, x, dt, A, B, C, D, scores, states, decay, False)
+        dconv, dbias = ext.mamba_before_scan_grad(dx, dB, dC, ddt, dzx, zx, conv_w, conv_b, dt_bias, norm_w, groups)
+        return (dzx, dconv[:4].t().reshape(conv_w.shape).to(conv_w.dtype), dconv[4].to(conv_b.dtype), dbias, dA, dD, dnorm.to(norm_w.dtype), None, None)
+
+
+def _scan_views(xbc, di, gn, nh, headdim, groups):
+    b, s, _ = xbc.shape
+    x, B, C = torch.split(xbc, [di, gn, gn], dim=-1)
+    return x.view(b, s, nh, headdim), B.view(b, s, groups, gn // groups), C.view(b, s, groups, gn // groups)
+
+
 @dataclass
 class MambaMixerSubmodules:
     in_proj: Union[ModuleSpec, type] = ColumnParallelLinear
@@ -197,9 +258,24 @@ class MambaMixer(MegatronModule):
         return ([("z", self.d_inner_local), ("x", self.d_inner_local), ("B", gn), ("C", gn), ("dt", self.nheads_local)],
                 [("x", self.d_inner_local), ("B", gn), ("C", gn)])
 
+    def _fused_core_ok(self, zx) -> bool:
+        """Sizes, types and ways of differentiating that the kernels between the projections take; the rest runs in PyTorch, around the
+        scan's own kernels where those fit."""
+        conv, di, ng = self.conv1d, self.d_inner_local, self.ngroups_local
+        return (zx.is_cuda and zx.dtype in (torch.bfloat16, torch.float32) and zx.is_contiguous() and zx.numel() > 0 and zx.data_ptr() % 16 == 0
+                and conv.weight.dtype == conv.bias.dtype == self.norm_weight.dtype == zx.dtype and self.d_conv == 4 and self.headdim == 64
+                and self.d_state in (64, 128) and zx.shape[2] % 8 == 0 and (di // ng) % 4 == 0 and di // ng <= 4096
+                and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (conv.weight, conv.bias, self.norm_weight))
+                and zx.shape[1] * self.nheads_local <= 65535 and zx.shape[0] <= 1 << 19 and not conv._forward_hooks and not conv._forward_pre_hooks
+                and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active())
+
     def forward(self, hidden_states, inference_context=None):
         zxbcdt, _ = self.in_proj(hidden_states)                         # [s, b, local]  (s is the full sequence)
         s, b, _ = zxbcdt.shape
+        if inference_context is None and self._fused_core_ok(zxbcdt):
+            y = _MixerCoreFn.apply(zxbcdt, self.conv1d.weight, self.conv1d.bias, self.dt_bias.float(), -torch.exp(self.A_log.float()), self.D.float(),
+                                   self.norm_weight, self.ngroups_local, self.headdim)
+            return self.out_proj(y)
         zxbcdt = zxbcdt.transpose(0, 1)                                # [b, s, ...]
         di, gn, nh, ng = self.d_inner_local, self.ngroups_local * self.d_state, self.nheads_local, self.ngroups_local
         z, xBC, dt = torch.split(zxbcdt, [di, di + 2 * gn, nh], dim=-1)

@@ -73,3 +73,40 @@ def test_other_ways_to_differentiate():
         x = torch.autograd.forward_ad.make_dual(ins[0].detach(), torch.ones_like(ins[0]))
         y, _ = ssd_scan(x, *[t.detach() for t in ins[1:6]])
         assert torch.autograd.forward_ad.unpack_dual(y).tangent is not None
+
+
+@pytest.mark.parametrize("s,b,hidden,g,n,dtype", [
+    (1, 1, 128, 1, 64, torch.float32),                        # one step; the convolution sees only padding before it
+    (35, 3, 128, 2, 64, torch.float32),                       # one step more than a run and its halo, batch inside the rows
+    (130, 2, 256, 8, 128, torch.bfloat16),                    # groups of 64 channels: a norm of half a warp
+    (66, 1, 2048, 1, 64, torch.bfloat16)])                    # one group of 4096 channels
+def test_mixer_core(s, b, hidden, g, n, dtype):
+    """Everything between the two projections, against the same in 64 bits."""
+    from megatronapp_b200.ssm.mamba import _MixerCoreFn, mixer_core_torch, ssd_scan_torch
+
+    q = torch.Generator("cuda").manual_seed(3)
+    rnd = lambda *sh: torch.randn(*sh, generator=q, device="cuda")  # noqa: E731
+    di = 2 * hidden
+    nh, c = di // 64, di + 2 * g * n
+    ins = [rnd(s, b, di + c + nh).to(dtype), (0.3 * rnd(c, 1, 4)).to(dtype), (0.1 * rnd(c)).to(dtype),
+           rnd(nh) - 4, -torch.rand(nh, generator=q, device="cuda") * 8 - 0.1, rnd(nh), (1 + 0.1 * rnd(di)).to(dtype)]
+    ins = [t.requires_grad_() for t in ins]
+    out = _MixerCoreFn.apply(*ins, g, 64)
+    wide = [t.detach().double().requires_grad_() for t in ins]
+
+    z, xbc, dt = wide[0].transpose(0, 1).split([di, c, nh], -1)
+    xbc = torch.nn.functional.silu(torch.nn.functional.conv1d(xbc.transpose(1, 2), wide[1], wide[2], padding=3, groups=c)[..., :s].transpose(1, 2))
+    x, B, C = xbc.split([di, g * n, g * n], -1)
+    y, _ = _oracle(x.reshape(b, s, nh, 64), torch.nn.functional.softplus(dt + wide[3]), wide[4], B.reshape(b, s, g, n), C.reshape(b, s, g, n), wide[5], None)
+    u = (y.reshape(b, s, di) * torch.nn.functional.silu(z)).view(b, s, g, di // g)
+    want = ((u * torch.rsqrt(u.pow(2).mean(-1, keepdim=True) + 1e-5)).view(b, s, di) * wide[6]).transpose(0, 1)
+    plain = mixer_core_torch(*ins, g, 64, scan=ssd_scan_torch).to(dtype)
+    do = torch.randn_like(out)
+    off = lambda a, w: float((a.detach().double() - w.detach()).norm())  # noqa: E731
+    got, ref, other = torch.autograd.grad(out, ins, do), torch.autograd.grad(want, wide, do.double()), torch.autograd.grad(plain, ins, do)
+    for i, (a, w, o) in enumerate(zip([out, *got], [want, *ref], [plain, *other])):
+        # fp32: rounding of the sums; bf16: the stored x B C, y and the gradients between the kernels each carry half a unit of 2^-8, and their
+        # results' own; independent, four of them.  In sums that cancel (over all steps, for A and the steps' bias) those roundings stand against
+        # the terms and not the sum, as they do in the PyTorch form, which rounds at more places
+        limit = (5e-5 if dtype == torch.float32 else 2.0 ** -7) * max(float(w.detach().norm()), 1e-6)
+        assert off(a, w) <= (limit if dtype == torch.float32 else max(limit, off(o, w))), i
