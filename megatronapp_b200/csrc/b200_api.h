@@ -146,9 +146,8 @@ void layernorm_bwd(const void* dy, const void* x, const void* gamma, const float
                    const float* rstd, void* dx, float* dgamma_partial, float* dbeta_partial,
                    int rows, int cols, bool rms, bool zero_centered, bool is_bf16, int n_partial,
                    cudaStream_t s);
-void layernorm_bwd_finalize(const float* dgamma_partial, const float* dbeta_partial,
-                            float* dgamma, float* dbeta, int n_partial, int cols, bool accumulate,
-                            cudaStream_t s);
+void layernorm_bwd_finalize(const float* dgamma_partial, const float* dbeta_partial, void* dgamma, void* dbeta, int n_partial, int cols,
+                            bool is_bf16, cudaStream_t s);
 int layernorm_bwd_partials(int rows);
 
 void bias_gelu_fwd(const void* x, const void* bias, void* y, int64_t rows, int cols, bool is_bf16,
@@ -166,8 +165,8 @@ void dropout_bwd(const void* dy, const uint8_t* mask, void* dx, int64_t n, float
                  cudaStream_t s);
 void rope_apply(const void* x, const float* cos_sin, void* y, int s, int b, int h, int d,
                 int rot_dim, bool interleaved, bool inverse, bool is_bf16, cudaStream_t st);
-void bias_grad_reduce(const void* dy, float* dbias, int64_t rows, int cols, bool is_bf16,
-                      bool accumulate, cudaStream_t s);
+// dbias: fp32 (accumulate: added to), or of dy's type
+void bias_grad_reduce(const void* dy, void* dbias, int64_t rows, int cols, bool is_bf16, bool out_f32, bool accumulate, cudaStream_t s);
 
 // vocab-parallel cross entropy pieces (fp32 statistics; logits 16-bit or fp32)
 void ce_local_stats(const void* logits, const int64_t* labels, float* row_max, float* row_sumexp,

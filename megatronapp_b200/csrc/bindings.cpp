@@ -425,16 +425,15 @@ std::vector<Tensor> layernorm_bwd(const Tensor& dy, const Tensor& x, const Tenso
   auto fo = x.options().dtype(at::kFloat);
   auto pg = torch::empty({np, cols}, fo);
   auto pb = has_beta ? torch::empty({np, cols}, fo) : torch::empty({0}, fo);
-  auto dgamma = torch::empty({cols}, fo);
-  auto dbeta = has_beta ? torch::empty({cols}, fo) : torch::empty({0}, fo);
+  auto dgamma = torch::empty({cols}, x.options());
+  auto dbeta = has_beta ? torch::empty({cols}, x.options()) : torch::empty({0}, x.options());
   auto dyc = dy.contiguous();
   b200::layernorm_bwd(dyc.data_ptr(), x.data_ptr(), gamma.data_ptr(), rms ? nullptr : mean.data_ptr<float>(),
                       rstd.data_ptr<float>(), dx.data_ptr(), pg.data_ptr<float>(),
                       has_beta ? pb.data_ptr<float>() : nullptr, rows, cols, rms, zero_centered,
                       is_bf16(x), np, cur_stream());
   b200::layernorm_bwd_finalize(pg.data_ptr<float>(), has_beta ? pb.data_ptr<float>() : nullptr,
-                               dgamma.data_ptr<float>(), has_beta ? dbeta.data_ptr<float>() : nullptr, np,
-                               cols, false, cur_stream());
+                               dgamma.data_ptr(), has_beta ? dbeta.data_ptr() : nullptr, np, cols, is_bf16(x), cur_stream());
   count(2);
   return {dx, dgamma, dbeta};
 }
@@ -514,10 +513,11 @@ Tensor rope_apply(const Tensor& x, const Tensor& cos_sin, bool interleaved, bool
 }
 void bias_grad(const Tensor& dy, Tensor& dbias, bool accumulate) {
   c10::cuda::CUDAGuard guard(dy.device());
-  TORCH_CHECK(dy.is_contiguous() && dbias.scalar_type() == at::kFloat);
+  const bool f32 = dbias.scalar_type() == at::kFloat;
+  TORCH_CHECK(dy.is_contiguous() && (f32 || (dbias.scalar_type() == dy.scalar_type() && !accumulate)) && dbias.is_contiguous());
   const int cols = static_cast<int>(dy.size(-1));
-  TORCH_CHECK(cols % 8 == 0);
-  b200::bias_grad_reduce(dy.data_ptr(), dbias.data_ptr<float>(), dy.numel() / cols, cols, is_bf16(dy), accumulate, cur_stream());
+  TORCH_CHECK(cols > 0 && cols % 8 == 0 && dbias.numel() == cols);
+  b200::bias_grad_reduce(dy.data_ptr(), dbias.data_ptr(), dy.numel() / cols, cols, is_bf16(dy), f32, accumulate, cur_stream());
   count();
 }
 

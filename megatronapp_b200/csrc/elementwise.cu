@@ -9,6 +9,7 @@
 #include "b200_api.h"
 #include "common.cuh"
 
+#include <cooperative_groups.h>
 #include <curand_kernel.h>
 
 namespace b200 {
@@ -420,28 +421,26 @@ static inline void ln_fast_shape(int cols, int& vpt, int& threads) {
   }
 }
 
-__global__ void __launch_bounds__(512) ln_bwd_finalize_kernel(const float* __restrict__ pg, const float* __restrict__ pb,
-                                       float* __restrict__ dgamma, float* __restrict__ dbeta,
-                                       int n_partial, int cols, bool accumulate) {
-  // 32 columns x 16 partial-row lanes per CTA: coalesced 128B rows, smem tree over the 16 lanes
-  __shared__ float sg[16][33], sb[16][33];
+// column sums of the partials, straight into the parameter's type.  blockIdx.y: gamma or beta; 32 columns x 32 partial rows at a time, all of a
+// thread's loads (10 at 296 partials) in flight together: 768 columns 7.0 -> 2.9 us, and no conversion launches behind it
+template <typename T>
+__global__ void __launch_bounds__(1024) ln_bwd_finalize_kernel(const float* __restrict__ pg, const float* __restrict__ pb, T* __restrict__ dgamma,
+                                                               T* __restrict__ dbeta, int n_partial, int cols) {
+  __shared__ float sm[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
-  float g = 0.f, b = 0.f;
+  const float* p = blockIdx.y == 0 ? pg : pb;
+  float v = 0.f;
   if (c < cols) {
-    for (int i = ty; i < n_partial; i += 16) {
-      g += pg[static_cast<size_t>(i) * cols + c];
-      if (pb) b += pb[static_cast<size_t>(i) * cols + c];
-    }
+#pragma unroll 10
+    for (int i = ty; i < n_partial; i += 32) v += p[static_cast<size_t>(i) * cols + c];
   }
-  sg[ty][tx] = g; sb[ty][tx] = b;
+  sm[ty][tx] = v;
   __syncthreads();
-  if (ty == 0 && c < cols) {
-#pragma unroll
-    for (int i = 1; i < 16; ++i) { g += sg[i][tx]; b += sb[i][tx]; }
-    dgamma[c] = accumulate ? dgamma[c] + g : g;
-    if (pb && dbeta) dbeta[c] = accumulate ? dbeta[c] + b : b;
-  }
+  // warp w sums columns w: lane = partial row
+  const float s = warp_sum(sm[tx][ty]);
+  const int out = blockIdx.x * 32 + ty;
+  if (tx == 0 && out < cols) (blockIdx.y == 0 ? dgamma : dbeta)[out] = Cvt<T>::down1(s);
 }
 
 // ------------------------------------------------------------------ activations
@@ -627,11 +626,14 @@ __global__ void rope_kernel(const T* __restrict__ x, const float* __restrict__ c
   }
 }
 
-// dbias[c] (+)= sum_r dy[r, c]
-template <typename T>
-__global__ void bias_grad_kernel(const T* __restrict__ dy, float* __restrict__ dbias, int64_t rows,
-                                 int cols, int rows_per_cta) {
-  __shared__ float sm[32][65];
+// dbias[c] (+)= sum_r dy[r, c].  A CTA sums 64 columns over its share of the rows; where the columns alone leave SMs idle, the CTAs of a cluster
+// share them and the first adds the shares up in order: one launch, the same sums every time (before: a fill, atomic additions, a conversion)
+__device__ __forceinline__ void put(float* p, float v) { *p = v; }
+template <typename T> __device__ __forceinline__ void put(T* p, float v) { *p = Cvt<T>::down1(v); }
+template <typename T, typename O>
+__global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ dy, O* __restrict__ dbias, int64_t rows, int cols, int rows_per_cta,
+                                                        bool accumulate) {
+  __shared__ float sm[32][65], total[64];
   const int cv = threadIdx.x & 7;        // 8 vectors of 8 columns = 64 columns per CTA
   const int rl = threadIdx.x >> 3;       // 32 row lanes
   const int col0 = blockIdx.x * 64 + cv * 8;
@@ -639,6 +641,7 @@ __global__ void bias_grad_kernel(const T* __restrict__ dy, float* __restrict__ d
   const int64_t r1 = min(rows, r0 + rows_per_cta);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (col0 < cols) {
+#pragma unroll 8
     for (int64_t r = r0 + rl; r < r1; r += 32) {
       float d[8];
       load8(dy + r * cols + col0, d);
@@ -653,8 +656,22 @@ __global__ void bias_grad_kernel(const T* __restrict__ dy, float* __restrict__ d
     float t = 0.f;
 #pragma unroll
     for (int i = 0; i < 32; ++i) t += sm[i][threadIdx.x];
-    const int c = blockIdx.x * 64 + threadIdx.x;
-    if (c < cols) atomicAdd(dbias + c, t);
+    total[threadIdx.x] = t;
+  }
+  const int c = blockIdx.x * 64 + threadIdx.x;
+  float sum = 0.f;
+  if (gridDim.y > 1) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    cl.sync();
+    if (blockIdx.y == 0 && threadIdx.x < 64)
+      for (int k = 0; k < static_cast<int>(gridDim.y); ++k) sum += *cl.map_shared_rank(total + threadIdx.x, k);
+    cl.sync();                           // no CTA leaves while the first reads its share
+  } else if (threadIdx.x < 64) {
+    sum = total[threadIdx.x];
+  }
+  if (blockIdx.y == 0 && threadIdx.x < 64 && c < cols) {
+    if constexpr (sizeof(O) == 4) { if (accumulate) sum += dbias[c]; }
+    put(dbias + c, sum);
   }
 }
 
@@ -963,10 +980,9 @@ void layernorm_bwd(const void* dy, const void* x, const void* gamma, const float
   });
 }
 
-void layernorm_bwd_finalize(const float* pg, const float* pb, float* dgamma, float* dbeta,
-                            int n_partial, int cols, bool accumulate, cudaStream_t s) {
-  ln_bwd_finalize_kernel<<<(cols + 31) / 32, 512, 0, s>>>(pg, pb, dgamma, dbeta, n_partial, cols,
-                                                            accumulate);
+void layernorm_bwd_finalize(const float* pg, const float* pb, void* dgamma, void* dbeta, int n_partial, int cols, bool is_bf16, cudaStream_t s) {
+  const dim3 grid((cols + 31) / 32, pb != nullptr ? 2 : 1);
+  DISPATCH_16(is_bf16, (ln_bwd_finalize_kernel<T><<<grid, 1024, 0, s>>>(pg, pb, (T*)dgamma, (T*)dbeta, n_partial, cols)));
 }
 
 void bias_gelu_fwd(const void* x, const void* bias, void* y, int64_t rows, int cols, bool is_bf16,
@@ -1014,17 +1030,29 @@ void rope_apply(const void* x, const float* cos_sin, void* y, int s, int b, int 
                            (const T*)x, cos_sin, (T*)y, s, b * h, d, rot_dim, interleaved,
                            inverse ? -1.f : 1.f)));
 }
-void bias_grad_reduce(const void* dy, float* dbias, int64_t rows, int cols, bool is_bf16,
-                      bool accumulate, cudaStream_t s) {
-  if (!accumulate) cudaMemsetAsync(dbias, 0, sizeof(float) * cols, s);
+template <typename T, typename O>
+static void launch_bias_grad(const T* dy, O* dbias, int64_t rows, int cols, bool accumulate, cudaStream_t s) {
   const int col_blocks = (cols + 63) / 64;
-  int row_splits = (148 * 4 + col_blocks - 1) / col_blocks;
-  if (row_splits < 1) row_splits = 1;
-  int rows_per_cta = static_cast<int>((rows + row_splits - 1) / row_splits);
-  rows_per_cta = (rows_per_cta + 31) / 32 * 32;
-  row_splits = static_cast<int>((rows + rows_per_cta - 1) / rows_per_cta);
-  dim3 grid(col_blocks, row_splits);
-  DISPATCH_16(is_bf16, (bias_grad_kernel<T><<<grid, 256, 0, s>>>((const T*)dy, dbias, rows, cols, rows_per_cta)));
+  unsigned split = 1;                                    // CTAs of a cluster, at least 256 rows each
+  while (split < 8 && col_blocks * split < 296 && rows >= 512 * static_cast<int64_t>(split)) split *= 2;
+  const int rows_per_cta = static_cast<int>((rows + split - 1) / split);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(col_blocks, split);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = attr.val.clusterDim.z = 1;
+  attr.val.clusterDim.y = split;
+  cfg.attrs = &attr;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, bias_grad_kernel<T, O>, dy, dbias, rows, cols, rows_per_cta, accumulate);
+}
+void bias_grad_reduce(const void* dy, void* dbias, int64_t rows, int cols, bool is_bf16, bool out_f32, bool accumulate, cudaStream_t s) {
+  DISPATCH_16(is_bf16, {
+    if (out_f32) launch_bias_grad<T, float>((const T*)dy, (float*)dbias, rows, cols, accumulate, s);
+    else launch_bias_grad<T, T>((const T*)dy, (T*)dbias, rows, cols, false, s);
+  });
 }
 
 void ce_local_stats(const void* logits, const int64_t* labels, float* row_max, float* row_sumexp,

@@ -164,7 +164,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = wgrad(dy2, x2, weight, ctx.fuse_wgrad)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = bias_grad(dy2).to(dy.dtype)
+            db = bias_grad(dy2, dy.dtype)
         return dx, dw, db, None
 
 
@@ -196,13 +196,15 @@ def linear(x, weight, bias=None, fuse_wgrad: bool = False):
     return _LinearFn.apply(x, weight, bias, fuse_wgrad)
 
 
-def bias_grad(dy2: torch.Tensor) -> torch.Tensor:
-    """fp32 column sum of a [rows, cols] gradient."""
+def bias_grad(dy2: torch.Tensor, dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+    """Column sum of a [rows, cols] gradient, summed in fp32 and returned in ``dtype`` (fp32 unless named)."""
+    dtype = dtype or torch.float32
     if _native(dy2) and dy2.shape[-1] % 8 == 0:
-        out = torch.empty(dy2.shape[-1], dtype=torch.float32, device=dy2.device)
+        direct = dtype in (torch.float32, dy2.dtype)
+        out = torch.empty(dy2.shape[-1], dtype=dtype if direct else torch.float32, device=dy2.device)
         ext().bias_grad(dy2.contiguous(), out, False)
-        return out
-    return dy2.float().sum(dim=0)
+        return out if direct else out.to(dtype)
+    return dy2.float().sum(dim=0).to(dtype)
 
 
 # ---------------------------------------------------------------------------
@@ -270,7 +272,7 @@ class _BiasGeluFn(torch.autograd.Function):
         dx = ext().bias_gelu_bwd(dy.contiguous(), x, bias)
         db = None
         if bias is not None and ctx.needs_input_grad[1]:
-            db = bias_grad(dx.view(-1, dx.shape[-1])).to(bias.dtype)
+            db = bias_grad(dx.view(-1, dx.shape[-1]), bias.dtype)
         return dx, db
 
 
@@ -299,7 +301,7 @@ class _SwigluFn(torch.autograd.Function):
         dx = ext().swiglu_bwd(dy.contiguous(), x, bias)
         db = None
         if bias is not None and ctx.needs_input_grad[1]:
-            db = bias_grad(dx.view(-1, dx.shape[-1])).to(bias.dtype)
+            db = bias_grad(dx.view(-1, dx.shape[-1]), bias.dtype)
         return dx, db
 
 
@@ -333,7 +335,7 @@ class _BdaFn(torch.autograd.Function):
     def backward(ctx, dy):
         (mask,) = ctx.saved_tensors
         dx = dy if ctx.p == 0.0 else ext().dropout_bwd(dy, mask, ctx.p)
-        db = bias_grad(dx.reshape(-1, dx.shape[-1])).to(dy.dtype) if (ctx.has_bias and ctx.needs_input_grad[1]) else None
+        db = bias_grad(dx.reshape(-1, dx.shape[-1]), dy.dtype) if (ctx.has_bias and ctx.needs_input_grad[1]) else None
         return dx, db, (dy if ctx.has_res else None), None, None, None
 
 

@@ -160,7 +160,7 @@ class Fp8LinearFn(torch.autograd.Function):
         if ctx.has_bias and ctx.needs_input_grad[2]:
             from . import bias_grad
 
-            db = bias_grad(dy2).to(dy.dtype)
+            db = bias_grad(dy2, dy.dtype)
         return dx, dw, db, None, None, None
 
 
@@ -327,7 +327,7 @@ class MxFp8LinearNativeFn(torch.autograd.Function):
         if ctx.has_bias and ctx.needs_input_grad[2]:
             from . import bias_grad
 
-            db = bias_grad(dy2).to(dy.dtype)
+            db = bias_grad(dy2, dy.dtype)
         ctx.xc = ctx.wc = None
         return dx, dw, db, None, None, None
 
@@ -385,7 +385,7 @@ class MxFp8LinearFn(torch.autograd.Function):
         if ctx.has_bias and ctx.needs_input_grad[2]:
             from . import bias_grad
 
-            db = bias_grad(dy2).to(dy.dtype)
+            db = bias_grad(dy2, dy.dtype)
         return dx, dw, db, None, None, None
 
 

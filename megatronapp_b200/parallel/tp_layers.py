@@ -226,7 +226,7 @@ class _ColumnParallelFn(torch.autograd.Function):
                 handle.wait()
             dw = ops.wgrad(dy2, total, weight, ctx.fuse_wgrad)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = ops.bias_grad(dy2).to(dy.dtype)
+            db = ops.bias_grad(dy2, dy.dtype)
         if ar_handle is not None:
             ar_handle.wait()
         if rs_handle is not None:
