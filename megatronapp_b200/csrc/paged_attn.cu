@@ -71,6 +71,12 @@ __device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t (&r)[4]) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
+// Launches of a step overlap: every kernel lets the next one start once all its own CTAs run, and waits for the one before where it reads
+// what that wrote: the write kernel's rows (the first of the others), the decode parts (merge).  The decode kernel beside chunks reads
+// nothing of theirs, and what both read was complete before the first began: it waits before its end, which keeps the stream's order
+// for what follows.
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -88,7 +94,8 @@ struct PagedParams {
   PagedAttnArgs a;
   int group_shift, bs_shift;   // log2 of the group; of the block size, or -1
   int n_tiles;                 // chunks: tiles of this launch (its grid is n_tiles * ng * splits); decode: requests
-  int splits;                  // chunks: key ranges of a tile; decode: CTAs
+  int splits;                  // chunks: key ranges of a tile; decode: CTAs, or 0 for one per (request, KV head)
+  bool beside_chunks;          // decode: the launch before is the chunks'
   float* ws;                   // decode: two partials of 16 rows x (d + 2) per CTA
 };
 
@@ -354,14 +361,30 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
   const PagedAttnArgs& a = p.a;
   const int tid = threadIdx.x, lane = tid & 31;
   const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
-  int total, before;
-  count_stages(p, 0, total, before);
-  const Cuts cuts(total * a.ng, p.splits);
-  int at = cuts.at(blockIdx.x);
-  const int end = cuts.at(blockIdx.x + 1);
-  if (at >= end) return;
+  allow_next();
+  if (!p.beside_chunks) await_previous();
+  int at, end;
+  if (p.splits == 0) {                                               // one item, whole
+    const int stages = decode_item(p, blockIdx.x / a.ng).stages;
+    at = 0;
+    end = stages;
+    if (tid == 0) {
+      s_find[0] = blockIdx.x / a.ng;
+      s_find[1] = static_cast<int>(blockIdx.x % a.ng) * stages;
+    }
+  } else {
+    int total, before;
+    count_stages(p, 0, total, before);
+    const Cuts cuts(total * a.ng, p.splits);
+    at = cuts.at(blockIdx.x);
+    end = cuts.at(blockIdx.x + 1);
+  }
+  if (at >= end) {
+    if (p.beside_chunks) await_previous();
+    return;
+  }
   // the request that this CTA's part of the line starts in
-  if (tid < 32) {
+  if (p.splits != 0 && tid < 32) {
     int seen = 0;
     for (int r0 = 0; r0 < p.n_tiles; r0 += 32) {
       const int s = decode_item(p, r0 + lane).stages;
@@ -420,19 +443,21 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     }
     at += n_st;
     inside += n_st;
-    if (at >= end) return;
+    if (at >= end) break;
     if (inside == it.stages * a.ng) {                                // on to the next request that is not a chunk
       inside = 0;
       do it = decode_item(p, ++r); while (it.stages == 0 && r < p.n_tiles);
-      if (it.stages == 0) return;
+      if (it.stages == 0) break;
     }
     __syncthreads();                                                 // the partials have been read; the ring fills again
   }
+  if (p.beside_chunks) await_previous();
 }
 
 // items that a cut fell into: their CTAs' partials, one CTA per (request, KV head)
 template <int D, bool kBf16>
-__global__ void __launch_bounds__(128) paged_merge_kernel(const PagedParams p) {
+__global__ void __launch_bounds__(512) paged_merge_kernel(const PagedParams p) {
+  await_previous();
   const PagedAttnArgs& a = p.a;
   const int r = blockIdx.x / a.ng, hk = blockIdx.x % a.ng, G = 1 << p.group_shift, np = a.ng << p.group_shift;
   const Item it = decode_item(p, r);
@@ -446,7 +471,7 @@ __global__ void __launch_bounds__(128) paged_merge_kernel(const PagedParams p) {
   // the parts' weights first, then the accumulators: every load of a pass stands by itself
   __shared__ float s_f[16][kDecodeCtas + 1], s_inv[16];
   const int rows = it.n << p.group_shift, parts = i1 - i0 + 1, lane = threadIdx.x & 31;
-  for (int row = threadIdx.x >> 5; row < rows; row += 4) {
+  for (int row = threadIdx.x >> 5; row < rows; row += 16) {
     float M = -INFINITY, L = 0.f;
     for (int i = lane; i < parts; i += 32) {
       s_f[row][i] = slot(i0 + i)[16 * D + row];
@@ -463,18 +488,34 @@ __global__ void __launch_bounds__(128) paged_merge_kernel(const PagedParams p) {
     if (lane == 0) s_inv[row] = L > 0.f ? 1.f / L : L;               // 0 without keys; NaN stays NaN
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < rows * (D / 4); idx += 128) {
-    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+  // four groups of threads take every fourth part of 128 column quads at a time
+  __shared__ float4 s_o[3][128];
+  const int group = threadIdx.x >> 7, thread = threadIdx.x & 127;
+  for (int idx0 = 0; idx0 < rows * (D / 4); idx0 += 128) {
+    const int idx = idx0 + thread, row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+    const bool valid = idx < rows * (D / 4);
     float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid) {
 #pragma unroll 8
-    for (int i = 0; i < parts; ++i) {
-      const float f = s_f[row][i];
-      const float4 v = *reinterpret_cast<const float4*>(slot(i0 + i) + row * D + col);
-      O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
+      for (int i = group; i < parts; i += 4) {
+        const float f = s_f[row][i];
+        const float4 v = *reinterpret_cast<const float4*>(slot(i0 + i) + row * D + col);
+        O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
+      }
     }
-    const float inv = s_inv[row];
-    uint16_t* out = static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
-    *reinterpret_cast<uint2*>(out + col) = make_uint2(pack2<kBf16>(O.x * inv, O.y * inv), pack2<kBf16>(O.z * inv, O.w * inv));
+    if (group > 0) s_o[group - 1][thread] = O;
+    __syncthreads();
+    if (group == 0 && valid) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float4 v = s_o[k][thread];
+        O.x += v.x; O.y += v.y; O.z += v.z; O.w += v.w;
+      }
+      const float inv = s_inv[row];
+      uint16_t* out = static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
+      *reinterpret_cast<uint2*>(out + col) = make_uint2(pack2<kBf16>(O.x * inv, O.y * inv), pack2<kBf16>(O.z * inv, O.w * inv));
+    }
+    __syncthreads();
   }
 }
 
@@ -490,6 +531,8 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
   const int rank = static_cast<int>(blockIdx.x) % p.splits, item = static_cast<int>(blockIdx.x) / p.splits;
   const int hk = item % a.ng, tile_at = p.n_tiles - 1 - item / a.ng; // later tiles of a chunk see more keys: they go first
   const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
+  await_previous();
+  allow_next();
   // that run of 64 / G tokens among the requests with more than 16 rows
   const int per_tile = kRows >> p.group_shift;
   if (warp == 0) {
@@ -576,6 +619,7 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
 __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* __restrict__ kc,
                                                           uint4* __restrict__ vc, const int64_t* __restrict__ slots, int n_tok, int ng, int chunks,
                                                           int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh) {
+  allow_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, row = static_cast<int64_t>(ng) * chunks;
   if (idx >= n_tok * row) return;
   const int64_t t = idx / row;
@@ -583,6 +627,27 @@ __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restric
   const int64_t dst = slots[t] * row + c;
   kc[dst] = k[t * k_st + h * k_sh + u];
   vc[dst] = v[t * v_st + h * v_sh + u];
+}
+
+// in the stream's order, but for what the kernels' own waits leave open (await_previous)
+template <typename K>
+int launch(K kern, unsigned ctas, int threads, int smem, int cluster, const PagedParams& p, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+  if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
+  return 0;
 }
 
 template <int D, bool kBf16>
@@ -595,20 +660,7 @@ int launch_chunks(const PagedParams& p, cudaStream_t s) {
   if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
   const int64_t ctas = static_cast<int64_t>(p.n_tiles) * p.a.ng * p.splits;
   if (ctas > 0x7fffffff) { g_paged_err = "paged attention: too many tiles"; return -12; }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = Smem<D>::kTotal;
-  cfg.stream = s;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(p.splits);
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = p.splits > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
-  if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
-  return 0;
+  return launch(kern, static_cast<unsigned>(ctas), 128, Smem<D>::kTotal, p.splits, p, s);
 }
 
 template <int D, bool kBf16>
@@ -621,11 +673,9 @@ int launch_decode(const PagedParams& p, cudaStream_t s) {
     g_paged_err = "paged attention: too many requests";
     return -12;
   }
-  kern<<<p.splits, 128, Smem<D>::kTotal, s>>>(p);
-  paged_merge_kernel<D, kBf16><<<p.n_tiles * p.a.ng, 128, 0, s>>>(p);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
-  return 0;
+  const unsigned items = static_cast<unsigned>(p.n_tiles * p.a.ng);
+  const int rc = launch(kern, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, p, s);
+  return rc != 0 || p.splits == 0 ? rc : launch(paged_merge_kernel<D, kBf16>, items, 512, 0, 1, p, s);
 }
 
 int log2_exact(int v) {
@@ -634,10 +684,14 @@ int log2_exact(int v) {
   return -1;
 }
 
-// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages
+// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Contexts of up to 8 stages (512
+// keys), or 16 where all items run at once, are not cut at all (0): the merge kernel then costs as much as the imbalance that it
+// removes (a step of 34 requests of 64 to 153 keys x 12 heads beside two chunks of 37: 44.7 us cut, 23.2 whole; 5 requests of up to
+// 600 keys x 8 heads: 29.1 and 16.3)
 int decode_ctas(const PagedAttnArgs& a) {
   const int64_t items = static_cast<int64_t>(a.cu != nullptr ? a.n_seqs : a.n_tokens) * a.ng;
   const int64_t longest = (static_cast<int64_t>(a.max_blocks) * a.block_size + kStageKeys - 1) / kStageKeys;
+  if (longest <= 8 || (longest <= 16 && items <= kDecodeCtas)) return 0;
   const int64_t n = items * longest / 2;
   return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
 }
@@ -679,6 +733,7 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
   p.n_tiles = a.cu != nullptr ? a.n_seqs : a.n_tokens;
   p.splits = decode_ctas(a);
   p.ws = ws;
+  p.beside_chunks = a.cu != nullptr && chunk_tiles > 0;
   return a.head_dim == 128 ? (a.is_bf16 ? launch_decode<128, true>(p, s) : launch_decode<128, false>(p, s))
                            : (a.is_bf16 ? launch_decode<64, true>(p, s) : launch_decode<64, false>(p, s));
 }
