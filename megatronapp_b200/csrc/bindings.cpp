@@ -97,7 +97,9 @@ void gemm_grouped(const Tensor& A, const Tensor& B, Tensor& D, const Tensor& off
     TORCH_CHECK(b_mn ? (group_stride == g.K && B.size(1) == g.N) : (group_stride == g.N && B.size(1) == g.K),
                 "GroupM: weight shape does not match A/D");
   } else {
-    g.group_mode = b200::kGroupK; g.epilogue = b200::kEpiAccumF32;
+    // 2: added to D, 3: stored (groups without rows as zeros)
+    TORCH_CHECK(mode == 2 || mode == 3, "grouped gemm: unknown mode");
+    g.group_mode = b200::kGroupK; g.epilogue = mode == 3 ? b200::kEpiStoreF32 : b200::kEpiAccumF32;
     g.a_mn_major = true; g.b_mn_major = true;
     g.M = static_cast<int>(A.size(1)); g.K = static_cast<int>(A.size(0)); g.N = static_cast<int>(B.size(1));
     TORCH_CHECK(A.size(0) == B.size(0), "GroupK: A and B must have the same row capacity");

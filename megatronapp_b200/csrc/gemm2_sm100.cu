@@ -32,7 +32,7 @@
 //   kModeGroupM   grouped GEMM over a 256-row-padded ragged row layout (MoE experts, forward + dgrad): m-block ->
 //                 group through a device-side offsets array (no host sync), B/bias selected per group, optional
 //                 per-row scale (router probability) in the epilogue.  (reference moe/experts.py:90-265 gmm)
-//   kModeGroupK   grouped wgrad: per group D_g[M,N] += A_g^T B_g with the K range of group g taken from the same
+//   kModeGroupK   grouped wgrad: per group D_g[M,N] (+)= A_g^T B_g with the K range of group g taken from the same
 //                 offsets array; fp32 TMA reduce-add into main_grad.
 #include "b200_api.h"
 #include "common.cuh"
@@ -499,7 +499,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     uint32_t* pending_flag = nullptr;   // RS: flag of the previous pushed tile, not yet published
     for (int tile = cluster_id; tile < num_tiles; tile += n_clusters) {
       const Tile2 t = tile_info<kMode>(p, tile);
-      if (!t.valid) continue;
+      // a group without rows has no product, but where D is stored and not added to, its tiles are zeros
+      const bool empty = kMode == kModeGroupK && kEpi == kEpiStoreF32 && !t.valid;
+      if (!t.valid && !empty) continue;
       const int m_blk = t.m_blk, n_blk = t.n_blk;
       const int m0 = m_blk * 256 + cta_rank * BM;
       // RS bookkeeping: who owns these rows, and where they sit inside the owner's shard
@@ -528,8 +530,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           named_bar_sync(3, kEpiThreads);
         }
       }
-      mbar_wait(&tmem_full_bar[acc], acc_phase);
-      tc_fence_after();
+      if (!empty) {
+        mbar_wait(&tmem_full_bar[acc], acc_phase);
+        tc_fence_after();
+      }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + acc * BN;
       float rscale = 1.f;
       if constexpr (kMode == kModeGroupM) {
@@ -542,10 +546,15 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 #pragma unroll 1
       for (int c = 0; c < BN / 64; ++c) {
         uint32_t v0[32], v1[32];
-        tmem_ld_32x32(taddr + c * 64, v0);
-        tmem_ld_32x32(taddr + c * 64 + 32, v1);
-        tmem_ld_wait();
-        if (c == BN / 64 - 1) {
+        if (!empty) {
+          tmem_ld_32x32(taddr + c * 64, v0);
+          tmem_ld_32x32(taddr + c * 64 + 32, v1);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v0[i] = v1[i] = 0u;
+        }
+        if (c == BN / 64 - 1 && !empty) {
           tc_fence_before();
           __syncwarp();
           if (lane == 0) {
@@ -675,7 +684,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           }
         }
       }
-      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      if (!empty && ++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
     if (epi_tid == 0) {
       tma_store_wait_all<0>();
@@ -795,8 +804,8 @@ int gemm2_bf16(const GemmArgs& a) {
   } else if (a.group_mode == kGroupK) {
     mode = kModeGroupK;
     if (a.group_offsets == nullptr || a.n_groups < 1) { g_err2 = "grouped GEMM needs group_offsets"; return -4; }
-    if (!a.a_mn_major || !a.b_mn_major || a.epilogue != kEpiAccumF32) {
-      g_err2 = "GroupK: MN-major A and B, fp32 accumulate epilogue"; return -4;
+    if (!a.a_mn_major || !a.b_mn_major || (a.epilogue != kEpiAccumF32 && a.epilogue != kEpiStoreF32)) {
+      g_err2 = "GroupK: MN-major A and B, fp32 epilogue"; return -4;
     }
     if (a.M % 256 != 0) { g_err2 = "GroupK: M (output features) must be a multiple of 256"; return -4; }
   } else if (a.comm == kCommAllGatherK) {
@@ -914,6 +923,7 @@ int gemm2_bf16(const GemmArgs& a) {
   G2_CASE(false, false, kEpiStore16, kModeGroupM)
   G2_CASE(false, true, kEpiStore16, kModeGroupM)
   G2_CASE(true, true, kEpiAccumF32, kModeGroupK)
+  G2_CASE(true, true, kEpiStoreF32, kModeGroupK)
 #undef G2_CASE
   g_err2 = "unsupported combination for the 2-CTA kernel";
   return -3;

@@ -14,6 +14,7 @@ from ..parallel import state as ps
 from ..transformer.mlp import MLP
 from ..transformer.module import MegatronModule
 from ..transformer.spec_utils import ModuleSpec, build_module
+from .experts import GroupedMLP
 from .router import TopKRouter
 from .token_dispatcher import (MoEAllGatherTokenDispatcher, MoEAlltoAllTokenDispatcher, MoEArenaDispatcher, MoEFusedDispatcher,
                                MoEPeerScatterDispatcher)
@@ -50,6 +51,10 @@ class MoELayer(MegatronModule):
         else:
             raise ValueError(f"unsupported token dispatcher type {kind}")
         self.experts = build_module(submodules.experts, self.num_local_experts, config)
+        if isinstance(self.token_dispatcher, (MoEFusedDispatcher, MoEArenaDispatcher)) and isinstance(self.experts, GroupedMLP) \
+                and config.gradient_accumulation_fusion:
+            # every backward pass runs one grouped wgrad per matrix over all experts, with or without tokens
+            self.experts.weight1.b200_wgrad_store_first = self.experts.weight2.b200_wgrad_store_first = True
         self.shared_experts = None
         if config.moe_shared_expert_intermediate_size:
             from .shared_experts import SharedExpertMLP

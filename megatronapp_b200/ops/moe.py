@@ -142,25 +142,29 @@ def grouped_wgrad(dy, x, weight, lay: RaggedLayout, stride: int, fuse: bool):
     main_grad = getattr(weight, "main_grad", None)
     native = _native(dy) and dy.dtype == x.dtype and stride % 256 == 0 and x.shape[1] % 8 == 0
 
-    def run(dst32):
+    def run(dst32, store: bool):
         if native:
-            ext().gemm_grouped(dy, x, dst32, lay.offsets, 2, True, None, 0, None, None, lay.E_local, stride)
+            ext().gemm_grouped(dy, x, dst32, lay.offsets, 3 if store else 2, True, None, 0, None, None, lay.E_local, stride)
         else:
+            if store:
+                dst32.zero_()
             offs = lay.offsets.tolist()
             for g in range(lay.E_local):
                 r0, r1 = offs[g], offs[g + 1]
                 if r1 > r0:
                     dst32[g * stride:(g + 1) * stride] += dy[r0:r1].float().t() @ x[r0:r1].float()
 
+    owned = getattr(weight, "b200_wgrad_store_first", False)
     if fuse and main_grad is not None and main_grad.dtype == torch.float32:
-        run(main_grad)
+        # the first micro-batch of a step stores (the buffer then is not zeroed for it), the later ones add
+        run(main_grad, owned and not getattr(weight, "grad_added_to_main_grad", False))
         weight.grad_added_to_main_grad = True
         hook = getattr(weight, "grad_ready_hook", None)
-        if hook is not None and getattr(weight, "b200_wgrad_store_first", False):
+        if hook is not None and owned:
             hook()
         return None
-    dw = torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
-    run(dw)
+    dw = torch.empty(weight.shape, dtype=torch.float32, device=weight.device)
+    run(dw, True)
     return dw.to(weight.dtype)
 
 

@@ -322,7 +322,9 @@ class DistributedDataParallel(nn.Module):
             if param.grad is not None:
                 # the fused wgrad path returns None (never a dummy), so whatever arrives here is a
                 # real contribution (e.g. the embedding lookup of a tied weight) and is always added
-                if param.main_grad.dtype == torch.float32 and param.grad.is_cuda and param.grad.is_contiguous():
+                if getattr(param, "b200_wgrad_store_first", False) and not param.grad_added_to_main_grad:
+                    param.main_grad.copy_(param.grad)      # not zeroed: see ParamAndGradBuffer.zero
+                elif param.main_grad.dtype == torch.float32 and param.grad.is_cuda and param.grad.is_contiguous():
                     ops.ext().add_into_f32(param.main_grad, param.grad)
                 else:
                     param.main_grad.add_(param.grad.to(param.main_grad.dtype))
