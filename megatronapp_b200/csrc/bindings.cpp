@@ -74,7 +74,7 @@ void gemm(const Tensor& A, const Tensor& B, Tensor& D, bool a_mn, bool b_mn, int
 
 // Grouped GEMM over the 256-row-padded ragged layout written by moe_permute (MoE experts).
 //   mode 1 (GroupM): D[cap, N] = A[cap, K] . W_g^T, W stacked [G * stride, .]; b_mn selects dgrad (W stored [K-rows, N]).
-//   mode 2 (GroupK): D32[G * stride, N] += A[cap, M]^T . B[cap, N] restricted to the rows of each group.
+//   mode 2 (GroupK): D32[G * stride, N] += A[cap, M]^T . B[cap, N] restricted to the rows of each group; mode 3 stores instead.
 void gemm_grouped(const Tensor& A, const Tensor& B, Tensor& D, const Tensor& offsets, int mode, bool b_mn,
                   const c10::optional<Tensor>& bias, int act, const c10::optional<Tensor>& D_pre,
                   const c10::optional<Tensor>& row_scale, int n_groups, int group_stride) {
