@@ -45,10 +45,9 @@ namespace b200 {
 namespace {
 
 constexpr int BM = 128;         // rows per CTA (256 per pair)
-constexpr int BN = 256;         // tile N (128 rows of B per CTA)
+constexpr int kWide = 256, kNarrow = 128;   // tile N (half of it rows of B per CTA)
 constexpr int BK = 64;
 constexpr int UK = 16;
-constexpr int kStagesDefault = 6;
 enum : int { kModePlain = 0, kModeAG = 1, kModeRS = 2, kModeGroupM = 3, kModeGroupK = 4, kModeAGK = 5 };
 constexpr int kThreads = 256;
 constexpr int kEpiThreads = 128;
@@ -88,13 +87,13 @@ struct PeerMaps2 {
   CUtensorMap m[kMaxPeers];
 };
 
-// Shared-memory plan: six 32 KB operand stages + two 16 KB epilogue staging buffers.  (Measured at TP4: giving the
+// Shared-memory plan: six 32 KB operand stages (eight of 24 KB at N = 128) + two 16 KB epilogue staging buffers.  (Measured at TP4: giving the
 // reduce-scatter mode 6 staging buffers / 4 stages does NOT speed up the peer pushes -- 50 MB of 128-byte row segments
 // leave a GPU at ~400 GB/s whatever the bytes in flight per SM, NCCL's ring moves the same bytes at ~470 GB/s -- so the
 // link-bound attention-projection case stays transfer-bound and the plan is the same for every mode.)
-template <int kMode>
+template <int BN>
 struct Smem2T {
-  static constexpr int kStages = kStagesDefault;
+  static constexpr int kStages = BN == kWide ? 6 : 8;
   static constexpr int kCBufs = 2;
   static constexpr int kA = BM * BK * 2;          // 16 KB
   static constexpr int kB = (BN / 2) * BK * 2;    // 16 KB (this CTA's half of the B tile)
@@ -213,12 +212,12 @@ __device__ __forceinline__ Tile2 tile_info(const P2& p, int tile) {
   return t;
 }
 
-template <bool kAMn, bool kBMn, int kEpi, int kMode>
+template <bool kAMn, bool kBMn, int kEpi, int kMode, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a_local,
              const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_d,
              const __grid_constant__ CUtensorMap tmap_d_pre, const __grid_constant__ PeerMaps2 peer_maps, const P2 p) {
-  using L = Smem2T<kMode>;
+  using L = Smem2T<BN>;
   constexpr int kStages = L::kStages;
   constexpr int kCBufs = L::kCBufs;
   extern __shared__ uint8_t smem_raw[];
@@ -748,18 +747,18 @@ bool tmap2(CUtensorMap* map, const void* base, int dtype /*0 bf16 1 f16 2 f32*/,
   return true;
 }
 
-template <bool AM, bool BMj, int EPI, int MODE>
+template <bool AM, bool BMj, int EPI, int MODE, int BN>
 int launch2(const GemmArgs& a, const P2& p, const CUtensorMap& ta, const CUtensorMap& tal, const CUtensorMap& tb,
             const CUtensorMap& td, const CUtensorMap& tdp, const PeerMaps2& pm, int grid) {
-  auto kern = gemm2_kernel<AM, BMj, EPI, MODE>;
+  auto kern = gemm2_kernel<AM, BMj, EPI, MODE, BN>;
   static bool set = false;
   if (!set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem2T<MODE>::kTotal) != cudaSuccess) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem2T<BN>::kTotal) != cudaSuccess) {
       g_err2 = "cudaFuncSetAttribute failed"; return -10;
     }
     set = true;
   }
-  kern<<<grid, kThreads, Smem2T<MODE>::kTotal, a.stream>>>(ta, tal, tb, td, tdp, pm, p);
+  kern<<<grid, kThreads, Smem2T<BN>::kTotal, a.stream>>>(ta, tal, tb, td, tdp, pm, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_err2 = std::string("launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
@@ -786,12 +785,20 @@ bool gemm2_supported(const GemmArgs& a) {
   return a.M >= 256 && a.N >= 128;
 }
 
+// Tiles of 128 columns where all of them still run at once: twice the pairs work.  Such a tile takes about 0.8 of a wide one's time, its
+// operands' shared-memory reads and writes being the bound (64 k-blocks of 768 x 768: 22.7 us against 26.8; 1024^3: 12.4 against 16.0;
+// 512 x 2048 x 2048: 16 against 20.6; 1024 x 1536 x 6144: 31 against 39), so a second wave of them is never worth it (2048 x 4096 x 4096:
+// 68 against 52; 1280 x 5120 x 8192: 106 against 89).
+static int tile_width(const GemmArgs& a, int clusters) {
+  const int64_t m = (a.M + 255) / 256;
+  return m * ((a.N + kNarrow - 1) / kNarrow) <= clusters ? kNarrow : kWide;
+}
+
 int gemm2_bf16(const GemmArgs& a) {
   P2 p{};
   p.M = a.M; p.N = a.N; p.K = a.K; p.ldd = a.ldd; p.D = a.D; p.D_pre = a.D_pre; p.bias = a.bias; p.act = a.act;
   p.is_bf16 = a.is_bf16 ? 1 : 0;
   p.num_m_blocks = (a.M + 255) / 256;
-  p.num_n_blocks = (a.N + BN - 1) / BN;
   p.num_k_blocks = (a.K + BK - 1) / BK;
   p.n_chunks = 1; p.m_blocks_per_chunk = p.num_m_blocks; p.chunk_base = 0; p.chunk_dir = 1;
   p.tp_rank = a.tp_rank; p.tp_size = a.tp_size; p.epoch = a.epoch; p.col_splits = 1;
@@ -852,6 +859,8 @@ int gemm2_bf16(const GemmArgs& a) {
       p.chunk_base = (a.tp_rank + 1) % a.tp_size; p.chunk_dir = 1;  // own rows last
     }
   }
+  const int BN = mode == kModePlain ? tile_width(a, clusters) : kWide;
+  p.num_n_blocks = (a.N + BN - 1) / BN;
   if (mode == kModePlain || mode == kModeGroupM) {
     // L2 banding: tiles walk n-groups (8 x 256 columns) inside a band of m-blocks.  Without bands the whole A operand is
     // re-streamed from HBM once per n-group as soon as it no longer fits L2; with bands B is re-read once per band.
@@ -906,9 +915,13 @@ int gemm2_bf16(const GemmArgs& a) {
     }
   }
   const int grid = clusters * 2;
-#define G2_CASE(AM, BMJ, EPI, MODE) \
-  if (a.a_mn_major == AM && a.b_mn_major == BMJ && a.epilogue == EPI && mode == MODE) \
-    return launch2<AM, BMJ, EPI, MODE>(a, p, ta, tal, tb, td, tdp, pm, grid);
+#define G2_CASE(AM, BMJ, EPI, MODE)                                                                                      \
+  if (a.a_mn_major == AM && a.b_mn_major == BMJ && a.epilogue == EPI && mode == MODE) {                                  \
+    if constexpr (MODE == kModePlain) {                                                                                  \
+      if (BN == kNarrow) return launch2<AM, BMJ, EPI, MODE, kNarrow>(a, p, ta, tal, tb, td, tdp, pm, grid);               \
+    }                                                                                                                    \
+    return launch2<AM, BMJ, EPI, MODE, kWide>(a, p, ta, tal, tb, td, tdp, pm, grid);                                      \
+  }
   G2_CASE(false, false, kEpiStore16, kModePlain)
   G2_CASE(false, true, kEpiStore16, kModePlain)
   G2_CASE(true, true, kEpiStore16, kModePlain)
