@@ -100,9 +100,10 @@ __device__ __forceinline__ float half_warp_sum(float v) {
 __device__ __forceinline__ int col4(int t, int j) { return (j >> 2) * 64 + t * 4 + (j & 3); }
 
 // 64 rows of W columns into padded fp32 rows; rows from `rows` on are zeros.  f(row): factor of the row
-template <int W, typename T, typename F>
+template <int W, int kBy = kThreads, typename T, typename F>
 __device__ __forceinline__ void load_rows(float* dst, int pitch, const T* src, int64_t stride, int rows, F f) {
-  for (int i = threadIdx.x; i < kT * (W / 4); i += kThreads) {
+#pragma unroll 8
+  for (int i = threadIdx.x & (kBy - 1); i < kT * (W / 4); i += kBy) {
     const int r = i / (W / 4), c = (i % (W / 4)) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) {
@@ -269,9 +270,12 @@ __global__ void __launch_bounds__(kThreads) ssd_out_kernel(const SsdArgs p) {
   }
 }
 
-// all gradients of one block for `per` heads of one group
+// all gradients of one block for `per` heads of one group.  The first half of the threads takes the scores, C and x, the second half what
+// goes through the state at the block's end, B among it: half of the multiply-adds each, and four warps per scheduler instead of two.
+// While the first half finishes dx the second fetches the next head's states.  64 heads x 2048 steps x 64 x 128: 485 us with 256 threads that
+// took one product after the other, 375 now.
 template <int N, typename T>
-__global__ void __launch_bounds__(kThreads, 1) ssd_grad_kernel(const SsdArgs p) {
+__global__ void __launch_bounds__(2 * kThreads, 1) ssd_grad_kernel(const SsdArgs p) {
   extern __shared__ __align__(16) float sm[];
   constexpr int kPitchN = N + 4, NI = N / 16;
   float* sC = sm;                              // [t][n]
@@ -287,110 +291,133 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_grad_kernel(const SsdArgs p) 
   float *s_cum = s_dt + kT, *s_row = s_cum + kT, *s_end = s_row + kT, *s_dir = s_end + kT, *s_col = s_dir + kT, *s_red = s_col + 8 * kT;
   const int c = blockIdx.x, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), hpg = p.h / p.g;
   const int g = blockIdx.y / p.n_sub, sub = blockIdx.y % p.n_sub, per = hpg / p.n_sub;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, warp = tid >> 5, lane = tid & 31;
-  load_rows<N>(sC, kPitchN, static_cast<const T*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows, One{});
-  load_rows<N>(sB, kPitchN, static_cast<const T*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows, One{});
-  load_rows<kT>(sG, kPitchT, p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT), static_cast<int64_t>(kT), kT, One{});
-  float dC[4][NI], dB[4][NI], dG[4][4];
-  zero(dC);
-  zero(dB);
+  const bool second = threadIdx.x >= kThreads;
+  const int tid = threadIdx.x & (kThreads - 1), tx = tid & 15, ty = tid >> 4, warp = tid >> 5, lane = tid & 31;
+  load_rows<N, 2 * kThreads>(sC, kPitchN, static_cast<const T*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows, One{});
+  load_rows<N, 2 * kThreads>(sB, kPitchN, static_cast<const T*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows, One{});
+  load_rows<kT, 2 * kThreads>(sG, kPitchT, p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT), static_cast<int64_t>(kT), kT, One{});
+  const int h0 = g * hpg + sub * per;
+  auto state_at = [&](int h) { return ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N); };
+  load_rows<N, 2 * kThreads>(sS, kPitchN, p.states + state_at(h0), static_cast<int64_t>(N), kP, One{});
+  load_rows<N, 2 * kThreads>(sR, kPitchN, p.dstates + state_at(h0), static_cast<int64_t>(N), kP, One{});
+  float acc[4][NI], dG[4][4];                  // dC in the first half, dB in the second
+  zero(acc);
   zero(dG);
   for (int hi = 0; hi < per; ++hi) {
-    const int h = g * hpg + sub * per + hi;
+    const int h = h0 + hi;
     const float a = p.A[h];
-    const int64_t row0 = (static_cast<int64_t>(b) * p.l + t0) * p.h + h, st0 = ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N);
+    const int64_t row0 = (static_cast<int64_t>(b) * p.l + t0) * p.h + h;
     __syncthreads();                           // the head before is done with its tiles
-    block_decay(s_dt, s_cum, p.dt + row0, p.h, rows, a);
-    load_rows<kP>(sX, kPitchT, static_cast<const T*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP, p.x_sl, rows, One{});
-    load_rows<kP>(sY, kPitchT, static_cast<const T*>(p.dy) + row0 * kP, static_cast<int64_t>(p.h) * kP, rows, One{});
-    load_rows<N>(sS, kPitchN, p.states + st0, static_cast<int64_t>(N), kP, One{});
-    load_rows<N>(sR, kPitchN, p.dstates + st0, static_cast<int64_t>(N), kP, One{});
-    __syncthreads();
+    load_rows<kP, 2 * kThreads>(sX, kPitchT, static_cast<const T*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP, p.x_sl, rows, One{});
+    load_rows<kP, 2 * kThreads>(sY, kPitchT, static_cast<const T*>(p.dy) + row0 * kP, static_cast<int64_t>(p.h) * kP, rows, One{});
+    block_decay(s_dt, s_cum, p.dt + row0, p.h, rows, a);  // and all tiles are there
     const float end = s_cum[kT - 1];
 
-    // gradient of the scores, and through their decays of cum
-    {
-      float v[4][4], col[4] = {0.f, 0.f, 0.f, 0.f};
-      zero(v);
-      mm<4, 4, true, true>(v, sY, kPitchT, sX, kPitchT, kP, ty, tx);
+    if (!second) {
+      // gradient of the scores, and through their decays of cum
+      {
+        float v[4][4], col[4] = {0.f, 0.f, 0.f, 0.f};
+        zero(v);
+        mm<4, 4, true, true>(v, sY, kPitchT, sX, kPitchT, kP, ty, tx);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = ty + 16 * i;
-        float row = 0.f;
+        for (int i = 0; i < 4; ++i) {
+          const int t = ty + 16 * i;
+          float row = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int u = tx + 16 * j;
+            const float w = u <= t ? expf(s_cum[t] - s_cum[u]) : 0.f, wg = w * sG[t * kPitchT + u];
+            sM[t * kPitchT + u] = wg;
+            const float d = v[i][j] * s_dt[u];
+            dG[i][j] = fmaf(d, w, dG[i][j]);
+            const float q = u < t ? d * wg : 0.f;           // on the diagonal the two ends cancel
+            row += q;
+            col[j] += q;
+          }
+          row = half_warp_sum(row);
+          if (tx == 0) s_row[t] = row;
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int u = tx + 16 * j;
-          const float w = u <= t ? expf(s_cum[t] - s_cum[u]) : 0.f, wg = w * sG[t * kPitchT + u];
-          sM[t * kPitchT + u] = wg;
-          const float d = v[i][j] * s_dt[u];
-          dG[i][j] = fmaf(d, w, dG[i][j]);
-          const float q = u < t ? d * wg : 0.f;           // on the diagonal the two ends cancel
-          row += q;
-          col[j] += q;
+          col[j] += __shfl_xor_sync(0xffffffffu, col[j], 16);
+          if (lane < 16) s_col[warp * kT + tx + 16 * j] = col[j];
         }
-        row = half_warp_sum(row);
-        if (tx == 0) s_row[t] = row;
       }
+      // C through the starting state
+      {
+        float v[4][NI];
+        zero(v);
+        mm<4, NI, true, false>(v, sY, kPitchT, sS, kPitchN, kP, ty, tx);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        col[j] += __shfl_xor_sync(0xffffffffu, col[j], 16);
-        if (lane < 16) s_col[warp * kT + tx + 16 * j] = col[j];
-      }
-    }
-    // the end state's part of dx
-    {
-      float v[4][4];
-      zero(v);
-      mm<4, 4, true, true>(v, sB, kPitchN, sR, kPitchN, N, ty, tx);
+        for (int i = 0; i < 4; ++i) {
+          const int t = ty + 16 * i;
+          const float e = expf(s_cum[t]);
+          float row = 0.f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float e = expf(end - s_cum[ty + 16 * i]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) sQ[(ty + 16 * i) * kPitchT + tx + 16 * j] = e * v[i][j];
-      }
-    }
-    // C through the starting state, B through the end state
-    {
-      float v[4][NI];
-      zero(v);
-      mm<4, NI, true, false>(v, sY, kPitchT, sS, kPitchN, kP, ty, tx);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = ty + 16 * i;
-        const float e = expf(s_cum[t]);
-        float row = 0.f;
-#pragma unroll
-        for (int j = 0; j < NI; ++j) {
-          const float w = e * v[i][j];
-          dC[i][j] += w;
-          row = fmaf(w, sC[t * kPitchN + col4(tx, j)], row);
+          for (int j = 0; j < NI; ++j) {
+            const float w = e * v[i][j];
+            acc[i][j] += w;
+            row = fmaf(w, sC[t * kPitchN + col4(tx, j)], row);
+          }
+          row = half_warp_sum(row);
+          if (tx == 0) s_row[t] += row;
         }
-        row = half_warp_sum(row);
-        if (tx == 0) s_row[t] += row;
       }
-    }
-    {
-      float v[4][NI];
-      zero(v);
-      mm<4, NI, true, false>(v, sX, kPitchT, sR, kPitchN, kP, ty, tx);
+    } else {
+      // the end state's part of dx
+      {
+        float v[4][4];
+        zero(v);
+        mm<4, 4, true, true>(v, sB, kPitchN, sR, kPitchN, N, ty, tx);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int u = ty + 16 * i;
-        const float e = expf(end - s_cum[u]) * s_dt[u];
-        float z = 0.f;
+        for (int i = 0; i < 4; ++i) {
+          const float e = expf(end - s_cum[ty + 16 * i]);
 #pragma unroll
-        for (int j = 0; j < NI; ++j) {
-          const float w = e * v[i][j];
-          dB[i][j] += w;
-          z = fmaf(w, sB[u * kPitchN + col4(tx, j)], z);
+          for (int j = 0; j < 4; ++j) sQ[(ty + 16 * i) * kPitchT + tx + 16 * j] = e * v[i][j];
         }
-        z = half_warp_sum(z);
-        if (tx == 0) s_end[u] = z;
+      }
+      // B through the end state
+      {
+        float v[4][NI];
+        zero(v);
+        mm<4, NI, true, false>(v, sX, kPitchT, sR, kPitchN, kP, ty, tx);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int u = ty + 16 * i;
+          const float e = expf(end - s_cum[u]) * s_dt[u];
+          float z = 0.f;
+#pragma unroll
+          for (int j = 0; j < NI; ++j) {
+            const float w = e * v[i][j];
+            acc[i][j] += w;
+            z = fmaf(w, sB[u * kPitchN + col4(tx, j)], z);
+          }
+          z = half_warp_sum(z);
+          if (tx == 0) s_end[u] = z;
+        }
+      }
+      // the end state's gradient times the starting state
+      {
+        float rs = 0.f;
+        for (int i = tid; i < kP * (N / 4); i += kThreads) {
+          const int r = i / (N / 4), q = (i % (N / 4)) * 4;
+          const float4 s = *reinterpret_cast<const float4*>(sS + r * kPitchN + q), e = *reinterpret_cast<const float4*>(sR + r * kPitchN + q);
+          rs += s.x * e.x + s.y * e.y + s.z * e.z + s.w * e.w;
+        }
+        rs = dev::warp_sum(rs);
+        if (lane == 0) s_red[8 + warp] = rs;
       }
     }
     __syncthreads();
-    // dx, dt through x, D, and the end state's gradient times the starting state
-    float dd = 0.f, rs = 0.f;
+    if (second) {
+      if (hi + 1 < per) {
+        load_rows<N>(sS, kPitchN, p.states + state_at(h + 1), static_cast<int64_t>(N), kP, One{});
+        load_rows<N>(sR, kPitchN, p.dstates + state_at(h + 1), static_cast<int64_t>(N), kP, One{});
+      }
+      continue;
+    }
+    // dx, dt through x, and D
+    float dd = 0.f;
     {
       float v[4][4];
       zero(v);
@@ -413,19 +440,10 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_grad_kernel(const SsdArgs p) 
         dir = half_warp_sum(dir);
         if (tx == 0) s_dir[u] = dir;
       }
-      for (int i = tid; i < kP * (N / 4); i += kThreads) {
-        const int r = i / (N / 4), q = (i % (N / 4)) * 4;
-        const float4 s = *reinterpret_cast<const float4*>(sS + r * kPitchN + q), e = *reinterpret_cast<const float4*>(sR + r * kPitchN + q);
-        rs += s.x * e.x + s.y * e.y + s.z * e.z + s.w * e.w;
-      }
       dd = dev::warp_sum(dd);
-      rs = dev::warp_sum(rs);
-      if (lane == 0) {
-        s_red[warp] = dd;
-        s_red[8 + warp] = rs;
-      }
+      if (lane == 0) s_red[warp] = dd;
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");                  // the first half alone
     // cum's gradient summed from the block's end, for dt and A
     if (warp == 0) {
       float g0[2], z = 0.f, acc_d = 0.f, acc_r = 0.f;
@@ -465,16 +483,17 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_grad_kernel(const SsdArgs p) 
   }
   // the scores' gradients into B and C
   __syncthreads();
+  if (!second) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      sM[(ty + 16 * i) * kPitchT + tx + 16 * j] = dG[i][j];
-      sQ[(tx + 16 * j) * kPitchT + ty + 16 * i] = dG[i][j];
-    }
+      for (int j = 0; j < 4; ++j) {
+        sM[(ty + 16 * i) * kPitchT + tx + 16 * j] = dG[i][j];
+        sQ[(tx + 16 * j) * kPitchT + ty + 16 * i] = dG[i][j];
+      }
+  }
   __syncthreads();
-  mm<4, NI, true, false>(dC, sM, kPitchT, sB, kPitchN, kT, ty, tx);
-  mm<4, NI, true, false>(dB, sQ, kPitchT, sC, kPitchN, kT, ty, tx);
+  mm<4, NI, true, false>(acc, second ? sQ : sM, kPitchT, second ? sC : sB, kPitchN, kT, ty, tx);
   const int64_t plane = static_cast<int64_t>(p.b) * p.l * p.g * N;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -483,15 +502,9 @@ __global__ void __launch_bounds__(kThreads, 1) ssd_grad_kernel(const SsdArgs p) 
     const int64_t at = ((static_cast<int64_t>(b) * p.l + t0 + t) * p.g + g) * N + tx * 4;
 #pragma unroll
     for (int q = 0; q < N / 64; ++q) {
-      const float4 vb = make_float4(dB[i][q * 4], dB[i][q * 4 + 1], dB[i][q * 4 + 2], dB[i][q * 4 + 3]);
-      const float4 vc = make_float4(dC[i][q * 4], dC[i][q * 4 + 1], dC[i][q * 4 + 2], dC[i][q * 4 + 3]);
-      if (p.n_sub == 1) {
-        st4(static_cast<T*>(p.dB) + at + q * 64, vb);
-        st4(static_cast<T*>(p.dC) + at + q * 64, vc);
-      } else {
-        st4(p.partial + sub * 2 * plane + at + q * 64, vb);
-        st4(p.partial + (sub * 2 + 1) * plane + at + q * 64, vc);
-      }
+      const float4 v = make_float4(acc[i][q * 4], acc[i][q * 4 + 1], acc[i][q * 4 + 2], acc[i][q * 4 + 3]);
+      if (p.n_sub == 1) st4(static_cast<T*>(second ? p.dB : p.dC) + at + q * 64, v);
+      else st4(p.partial + (sub * 2 + (second ? 0 : 1)) * plane + at + q * 64, v);
     }
   }
 }
@@ -545,7 +558,7 @@ bool backward(const SsdArgs& p, cudaStream_t s) {
   ssd_pass_kernel<true><<<dim3(per / kThreads, p.b * p.h), kThreads, 0, s>>>(reinterpret_cast<float4*>(p.dstates), p.decay,
                                                                              reinterpret_cast<const float4*>(p.dlast), reinterpret_cast<float4*>(p.dfirst),
                                                                              p.n_chunks, per);
-  ssd_grad_kernel<N, T><<<dim3(p.n_chunks, p.g * p.n_sub, p.b), kThreads, grad_smem<N>(), s>>>(p);
+  ssd_grad_kernel<N, T><<<dim3(p.n_chunks, p.g * p.n_sub, p.b), 2 * kThreads, grad_smem<N>(), s>>>(p);
   if (p.n_sub > 1) {
     const int64_t plane4 = static_cast<int64_t>(p.b) * p.l * p.g * N / 4;
     ssd_merge_kernel<T><<<static_cast<unsigned>((2 * plane4 + kThreads - 1) / kThreads), kThreads, 0, s>>>(
