@@ -168,6 +168,20 @@ void rope_apply(const void* x, const float* cos_sin, void* y, int s, int b, int 
 // dbias: fp32 (accumulate: added to), or of dy's type
 void bias_grad_reduce(const void* dy, void* dbias, int64_t rows, int cols, bool is_bf16, bool out_f32, bool accumulate, cudaStream_t s);
 
+// gradient of an embedding table [vocab, h], zero on entry, from that of n looked-up rows; row i lies at i / inner * st_outer + i % inner * st_inner
+struct EmbeddingGradArgs {
+  const void* dy;
+  const int64_t* ids;
+  void* dw;
+  int* order;      // n
+  float* parts;    // embedding_grad_parts(n, h)
+  int n, h, inner;
+  int64_t vocab, st_outer, st_inner;
+  bool is_bf16;
+};
+int64_t embedding_grad_parts(int n, int h);
+void embedding_grad(const EmbeddingGradArgs& a, cudaStream_t s);
+
 // vocab-parallel cross entropy pieces (fp32 statistics; logits 16-bit or fp32)
 void ce_local_stats(const void* logits, const int64_t* labels, float* row_max, float* row_sumexp,
                     float* tgt_logit, int64_t rows, int vocab_local, int vocab_start, int ldl,

@@ -513,6 +513,28 @@ Tensor rope_apply(const Tensor& x, const Tensor& cos_sin, bool interleaved, bool
   count();
   return y;
 }
+// ids: int64 [n] or [outer, inner], contiguous; dy: ids' shape x h, 16-byte rows at any strides of the leading dimensions
+Tensor embedding_grad(const Tensor& dy, const Tensor& ids, int64_t vocab) {
+  c10::cuda::CUDAGuard guard(dy.device());
+  TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous() && (ids.dim() == 1 || ids.dim() == 2) && dy.dim() == ids.dim() + 1 &&
+              ids.numel() > 0 && ids.numel() < (1 << 20) && vocab > 0 && vocab <= 0x7fffffff, "embedding_grad: ids");
+  const int64_t h = dy.size(-1);
+  TORCH_CHECK((dy.scalar_type() == at::kBFloat16 || dy.scalar_type() == at::kHalf) && h > 0 && h % 8 == 0 && h < (1 << 24) && dy.stride(-1) == 1 &&
+              reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 == 0, "embedding_grad: rows of 16 bytes");
+  for (int64_t i = 0; i < ids.dim(); ++i) TORCH_CHECK(dy.size(i) == ids.size(i) && dy.stride(i) % 8 == 0, "embedding_grad: shape of dy");
+  b200::EmbeddingGradArgs a{};
+  a.n = static_cast<int>(ids.numel()); a.h = static_cast<int>(h); a.vocab = vocab; a.is_bf16 = is_bf16(dy);
+  a.inner = static_cast<int>(ids.size(-1));
+  a.st_outer = ids.dim() == 2 ? dy.stride(0) : 0;
+  a.st_inner = dy.stride(ids.dim() - 1);
+  auto dw = torch::zeros({vocab, h}, dy.options());
+  auto order = torch::empty({a.n}, dy.options().dtype(at::kInt));
+  auto parts = torch::empty({b200::embedding_grad_parts(a.n, a.h)}, dy.options().dtype(at::kFloat));
+  a.dy = dy.data_ptr(); a.ids = ids.data_ptr<int64_t>(); a.dw = dw.data_ptr(); a.order = order.data_ptr<int>(); a.parts = parts.data_ptr<float>();
+  b200::embedding_grad(a, cur_stream());
+  count();
+  return dw;
+}
 void bias_grad(const Tensor& dy, Tensor& dbias, bool accumulate) {
   c10::cuda::CUDAGuard guard(dy.device());
   const bool f32 = dbias.scalar_type() == at::kFloat;
@@ -1085,6 +1107,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout_bwd", &dropout_bwd);
   m.def("rope_apply", &rope_apply);
   m.def("bias_grad", &bias_grad);
+  m.def("embedding_grad", &embedding_grad);
   m.def("ce_local_stats", &ce_local_stats);
   m.def("ce_rescale", &ce_rescale);
   m.def("ce_grad", &ce_grad);

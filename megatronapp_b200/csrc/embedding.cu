@@ -1,0 +1,176 @@
+// Gradient of an embedding table from the gradient of the looked-up rows, in a fixed order and without a sort over the key bits.
+//
+// A training step has some thousand tokens, each a row of one or a few KB: little to do, so what counts is the number of dependent steps.
+//   order: a token's place among all, sorted by id and then by position, is the number of tokens before it in that order, which a warp
+//     counts for four tokens at once (4096 tokens: 16.8 M compares, a few us; 32 bits suffice for ids that the lookup has accepted).
+//   sum:   a CTA takes 16 places and all columns of a slice, every row's address known from the start.  Runs of one id inside the tile are
+//     summed in fp32 and stored; what continues into a neighbouring tile is left as a partial sum.
+//   merge: a CTA whose tile holds the beginning of such a run adds the following tiles' parts to it.
+// Quadratic in the tokens, so it ends at 16384 (about 20 us); beyond that a radix sort is the better way and PyTorch's is used.
+// 4096 tokens, 50304 x 768 and 1024 x 768: the two gradients took some 40 launches and 240 us with PyTorch's sort.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include "b200_api.h"
+#include "common.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr int kOrderWarps = 8, kOrderTokens = 4;      // per warp
+constexpr int kTile = 16, kSumThreads = 128, kMergeGroups = 4;
+
+__global__ void __launch_bounds__(kOrderWarps * 32) embed_order_kernel(const int64_t* __restrict__ ids, int* __restrict__ order, int n) {
+  const int lane = threadIdx.x & 31, i0 = (blockIdx.x * kOrderWarps + (threadIdx.x >> 5)) * kOrderTokens;
+  if (i0 >= n) return;
+  int mine[kOrderTokens], count[kOrderTokens];
+#pragma unroll
+  for (int k = 0; k < kOrderTokens; ++k) {
+    mine[k] = static_cast<int>(ids[min(i0 + k, n - 1)]);
+    count[k] = 0;
+  }
+  // tokens before i0 come first at equal ids, those from i0 + kOrderTokens on do not
+#pragma unroll 8
+  for (int j = lane; j < i0; j += 32) {
+    const int v = static_cast<int>(ids[j]);
+#pragma unroll
+    for (int k = 0; k < kOrderTokens; ++k) count[k] += v <= mine[k];
+  }
+#pragma unroll 8
+  for (int j = i0 + lane; j < n; j += 32) {
+    const int v = static_cast<int>(ids[j]);
+#pragma unroll
+    for (int k = 0; k < kOrderTokens; ++k) count[k] += v < mine[k] || (v == mine[k] && j < i0 + k);
+  }
+#pragma unroll
+  for (int k = 0; k < kOrderTokens; ++k) {
+    const int c = __reduce_add_sync(0xffffffffu, count[k]);
+    if (lane == 0 && i0 + k < n) order[c] = i0 + k;
+  }
+}
+
+template <typename T> __device__ __forceinline__ float2 unpack(uint32_t u);
+template <> __device__ __forceinline__ float2 unpack<__nv_bfloat16>(uint32_t u) { return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u)); }
+template <> __device__ __forceinline__ float2 unpack<__half>(uint32_t u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
+template <typename T> __device__ __forceinline__ uint32_t pack(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack<__nv_bfloat16>(float a, float b) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t pack<__half>(float a, float b) {
+  __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+template <typename T>
+__device__ __forceinline__ void store_row(T* dst, const float (&acc)[8]) {
+  *reinterpret_cast<uint4*>(dst) = make_uint4(pack<T>(acc[0], acc[1]), pack<T>(acc[2], acc[3]), pack<T>(acc[4], acc[5]), pack<T>(acc[6], acc[7]));
+}
+__device__ __forceinline__ void store_part(float* dst, const float (&acc)[8]) {
+  reinterpret_cast<float4*>(dst)[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  reinterpret_cast<float4*>(dst)[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+}
+
+// parts[tile]: the tile's share of a run that it has in common with a neighbour: [0] began before the tile, [1] begins in it
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads) embed_sum_kernel(const T* __restrict__ dy, const int64_t* __restrict__ ids, const int* __restrict__ order,
+                                                                T* __restrict__ dw, float* __restrict__ parts, int n, int h, int64_t vocab, int inner,
+                                                                int64_t st_outer, int64_t st_inner) {
+  __shared__ int s_row[kTile];
+  __shared__ int64_t s_id[kTile + 2];                 // with the neighbours' ids at both ends, -1 outside
+  const int p0 = blockIdx.x * kTile, m = min(kTile, n - p0), t = threadIdx.x;
+  if (t < kTile + 2) {
+    const int p = p0 + t - 1;
+    const int row = p >= 0 && p < n ? order[p] : -1;
+    s_id[t] = row >= 0 ? ids[row] : -1;
+    if (t >= 1 && t <= kTile) s_row[t - 1] = max(row, 0);
+  }
+  __syncthreads();
+  const int col = (blockIdx.y * kSumThreads + t) * 8;
+  if (col >= h) return;
+  uint4 v[kTile];
+#pragma unroll
+  for (int i = 0; i < kTile; ++i) v[i] = *reinterpret_cast<const uint4*>(dy + s_row[i] / inner * st_outer + s_row[i] % inner * st_inner + col);
+  float acc[8];
+  bool before = m > 0 && s_id[0] == s_id[1];
+#pragma unroll
+  for (int i = 0; i < kTile; ++i) {
+    if (i >= m) break;
+    const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+    const bool fresh = i == 0 || s_id[i] != s_id[i + 1];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 f = unpack<T>(u[q]);
+      acc[2 * q] = fresh ? f.x : acc[2 * q] + f.x;
+      acc[2 * q + 1] = fresh ? f.y : acc[2 * q + 1] + f.y;
+    }
+    const int64_t id = s_id[i + 1];
+    if (i + 1 < m && s_id[i + 2] == id) continue;
+    // the run's end in this tile (the slot behind a last, short tile holds -1)
+    const bool after = i + 1 == m && s_id[i + 2] == id;
+    if (before || after) store_part(parts + (static_cast<int64_t>(blockIdx.x) * 2 + (before ? 0 : 1)) * h + col, acc);
+    else if (id >= 0 && id < vocab) store_row(dw + id * h + col, acc);
+    before = false;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSumThreads * kMergeGroups) embed_merge_kernel(const int64_t* __restrict__ ids, const int* __restrict__ order,
+                                                                                 T* __restrict__ dw, const float* __restrict__ parts, int n, int h, int64_t vocab) {
+  // a run that begins in this tile and goes on: its last id is the next tile's first and not the tile before's last
+  const int p0 = blockIdx.x * kTile, next = p0 + kTile;
+  if (next >= n) return;
+  const int64_t id = ids[order[next - 1]];
+  if (ids[order[next]] != id || (p0 > 0 && ids[order[p0 - 1]] == id) || id < 0 || id >= vocab) return;
+  // the last tile whose first id is still this one; ids are in order
+  int lo = blockIdx.x + 1, hi = (n + kTile - 1) / kTile;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (ids[order[mid * kTile]] == id) lo = mid;
+    else hi = mid;
+  }
+  __shared__ float s_acc[kMergeGroups - 1][kSumThreads][9];
+  const int group = threadIdx.x / kSumThreads, t = threadIdx.x % kSumThreads, col = (blockIdx.y * kSumThreads + t) * 8;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (col < h) {
+#pragma unroll 8
+    for (int tile = blockIdx.x + group; tile <= lo; tile += kMergeGroups) {
+      const float4* part = reinterpret_cast<const float4*>(parts + (static_cast<int64_t>(tile) * 2 + (tile == static_cast<int>(blockIdx.x) ? 1 : 0)) * h + col);
+      const float4 c = part[0], d = part[1];
+      acc[0] += c.x; acc[1] += c.y; acc[2] += c.z; acc[3] += c.w; acc[4] += d.x; acc[5] += d.y; acc[6] += d.z; acc[7] += d.w;
+    }
+  }
+  if (group > 0) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s_acc[group - 1][t][q] = acc[q];
+  }
+  __syncthreads();
+  if (group > 0 || col >= h) return;
+#pragma unroll
+  for (int k = 0; k < kMergeGroups - 1; ++k)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[q] += s_acc[k][t][q];
+  store_row(dw + id * h + col, acc);
+}
+
+template <typename T>
+void run(const EmbeddingGradArgs& a, cudaStream_t s) {
+  const int n = a.n, h = a.h;
+  T* dw = static_cast<T*>(a.dw);
+  const int per = kOrderWarps * kOrderTokens;
+  embed_order_kernel<<<(n + per - 1) / per, kOrderWarps * 32, 0, s>>>(a.ids, a.order, n);
+  const dim3 grid((n + kTile - 1) / kTile, (h / 8 + kSumThreads - 1) / kSumThreads);
+  embed_sum_kernel<T><<<grid, kSumThreads, 0, s>>>(static_cast<const T*>(a.dy), a.ids, a.order, dw, a.parts, n, h, a.vocab, a.inner, a.st_outer, a.st_inner);
+  if (n > kTile) embed_merge_kernel<T><<<grid, kSumThreads * kMergeGroups, 0, s>>>(a.ids, a.order, dw, a.parts, n, h, a.vocab);
+}
+
+}  // namespace
+
+int64_t embedding_grad_parts(int n, int h) { return static_cast<int64_t>((n + kTile - 1) / kTile) * 2 * h; }
+
+void embedding_grad(const EmbeddingGradArgs& a, cudaStream_t s) {
+  if (a.is_bf16) run<__nv_bfloat16>(a, s);
+  else run<__half>(a, s);
+}
+
+}  // namespace b200

@@ -16,11 +16,21 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ... import ops
 from ...parallel import state as ps
 from ...parallel.mappings import scatter_to_sequence_parallel_region
 from ...parallel.random import get_cuda_rng_tracker
 from ...parallel.tp_layers import VocabParallelEmbedding
 from ...transformer.module import MegatronModule
+
+
+class Embedding(nn.Embedding):
+    """``nn.Embedding`` whose plain lookup has the framework's gradient kernels."""
+
+    def forward(self, input):
+        if self.padding_idx is None and self.max_norm is None and not self.scale_grad_by_freq and not self.sparse:
+            return ops.embedding(input, self.weight)
+        return super().forward(input)
 
 
 class LanguageModelEmbedding(MegatronModule):
@@ -42,8 +52,8 @@ class LanguageModelEmbedding(MegatronModule):
             reduce_scatter_embeddings=self.reduce_scatter_embeddings, config=config)
         dev = "cpu" if (config.use_cpu_initialization or not torch.cuda.is_available()) else torch.cuda.current_device()
         if self.add_position_embedding:
-            self.position_embeddings = nn.Embedding(max_sequence_length, config.hidden_size,
-                                                    dtype=config.params_dtype, device=dev)
+            self.position_embeddings = Embedding(max_sequence_length, config.hidden_size,
+                                                 dtype=config.params_dtype, device=dev)
             if config.perform_initialization:
                 config.init_method(self.position_embeddings.weight)
         if num_tokentypes > 0:

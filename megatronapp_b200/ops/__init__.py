@@ -208,6 +208,40 @@ def bias_grad(dy2: torch.Tensor, dtype: Optional[torch.dtype] = None) -> torch.T
 
 
 # ---------------------------------------------------------------------------
+# embedding lookup
+# ---------------------------------------------------------------------------
+
+_EMBED_TOKENS = 16384          # the kernels' work is quadratic in the tokens; beyond, PyTorch's radix sort costs less
+
+
+class _EmbeddingFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, ids, weight):
+        ctx.save_for_backward(ids)
+        ctx.vocab = weight.shape[0]
+        return torch.nn.functional.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (ids,) = ctx.saved_tensors
+        if torch.is_grad_enabled():                     # a gradient that is differentiated again
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids, ctx.vocab, -1, False)
+        if dy.stride(-1) != 1 or any(st % 8 for st in dy.stride()[:-1]) or dy.data_ptr() % 16:
+            dy = dy.clone(memory_format=torch.contiguous_format)
+        return None, ext().embedding_grad(dy, ids.long().contiguous(), ctx.vocab)
+
+
+def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """Rows ``ids`` of ``weight``; the dense gradient of a 16-bit table comes from kernels that sum in fp32 and a fixed order."""
+    if (_native(weight) and weight.requires_grad and torch.is_grad_enabled() and ids.is_cuda and ids.dim() in (1, 2) and weight.dim() == 2
+            and 0 < ids.numel() <= _EMBED_TOKENS and weight.shape[1] % 8 == 0 and 0 < weight.shape[1] < 1 << 24 and 0 < weight.shape[0] <= 0x7fffffff
+            and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()):
+        return _EmbeddingFn.apply(ids, weight)
+    return torch.nn.functional.embedding(ids, weight)
+
+
+# ---------------------------------------------------------------------------
 # LayerNorm / RMSNorm
 # ---------------------------------------------------------------------------
 

@@ -24,7 +24,6 @@ from typing import Callable, List, Optional
 import torch
 import torch.distributed as dist
 import torch.nn as nn
-import torch.nn.functional as F
 
 from . import state as ps
 from .mappings import (
@@ -577,7 +576,7 @@ class VocabParallelEmbedding(nn.Module):
             local = (input_ - self.vocab_start_index).masked_fill(mask, 0)
         else:
             local = input_
-        out = F.embedding(local, self.weight)
+        out = ops.embedding(local, self.weight)
         if self.tp_size > 1:
             out = out.masked_fill(mask.unsqueeze(-1), 0.0)
         if self.reduce_scatter_embeddings:
