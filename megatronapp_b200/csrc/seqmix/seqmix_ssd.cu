@@ -9,11 +9,15 @@
 // gradient that enters each block's starting state, walked in reverse, then one kernel for all gradients of a block, whose CTA walks the
 // heads of a group so that the gradients of B and C add up in registers.  Exponents above the diagonal are never taken (they can overflow).
 //
-// Tiles are fp32 in shared memory, 4 x 4 or 4 x 8 results per thread: bound by fp32 multiply-adds (2.1 M per head and block backward,
-// 1.3 M forward) and the shared-memory reads that feed them.  The block-by-block PyTorch form took some 2900 launches and 14 ms of
+// fp32 inputs, and the gradients: tiles in fp32 in shared memory, 4 x 4 or 4 x 8 results per thread, bound by fp32 multiply-adds (2.1 M per
+// head and block backward, 1.3 M forward) and the shared-memory reads that feed them.  bf16 inputs: block states and outputs on the tensor
+// instructions (64 heads x 2048 steps x 64 x 128: outputs 140 -> 56 us, states 57 -> 33.5 and 59 -> 33.5; the final state's and the initial
+// state's gradient's errors are 2.3e-7 and 1.0e-7 of their size, with multiply-adds 2.4e-7 and 1.8e-7).  The block-by-block PyTorch form took some 2900 launches and 14 ms of
 // device time for 64 heads x 2048 steps.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "seq_common.cuh"
 #include "seqmix_api.h"
@@ -188,6 +192,213 @@ __global__ void __launch_bounds__(kThreads) ssd_state_kernel(const SsdArgs p) {
 #pragma unroll
     for (int q = 0; q < N / 64; ++q)
       *reinterpret_cast<float4*>(out + (ty * 4 + i) * N + q * 64 + tx * 4) = make_float4(acc[i][q * 4], acc[i][q * 4 + 1], acc[i][q * 4 + 2], acc[i][q * 4 + 3]);
+}
+
+// ---- bf16 operands on the tensor instructions.  A bf16 operand enters as it is; an fp32 one as three bf16 parts that add up to it exactly
+// (truncated, so 8 + 8 + 8 bits and no part overflows).  The products of parts are exact; the first parts' are summed by themselves, since
+// these instructions cut their sums off where a multiply-add rounds, and a third of the additions at full size leaves a third of that error.
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t shared_at(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(shared_at(p)) : "memory");
+}
+__device__ __forceinline__ void ldm4_trans(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(shared_at(p)) : "memory");
+}
+__device__ __forceinline__ void ldm2_trans(uint32_t& r0, uint32_t& r1, const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(shared_at(p)) : "memory");
+}
+__device__ __forceinline__ float high_part(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+__device__ __forceinline__ float rest_of(float v, float high) { return v == high ? 0.f : v - high; }   // an infinity has no rest
+__device__ __forceinline__ uint32_t pack_high(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&part)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    part[i] = pack_high(x, y);
+    x = rest_of(x, high_part(x));
+    y = rest_of(y, high_part(y));
+  }
+}
+constexpr int kPitchH = 72;                     // bf16 rows of 64, 16 bytes further on in each: ldmatrix without conflicts
+constexpr int kPlane = kT * kPitchH;
+// 64 rows of W columns as they are
+template <int W>
+__device__ __forceinline__ void copy_rows(__nv_bfloat16* dst, int pitch, const __nv_bfloat16* src, int64_t stride, int rows) {
+#pragma unroll
+  for (int k = 0; k < kT * (W / 4) / kThreads; ++k) {
+    const int i = threadIdx.x + k * kThreads, r = i / (W / 4), c = (i % (W / 4)) * 4;
+    *reinterpret_cast<uint2*>(dst + r * pitch + c) = r < rows ? *reinterpret_cast<const uint2*>(src + r * stride + c) : make_uint2(0u, 0u);
+  }
+}
+__device__ __forceinline__ void store_split(__nv_bfloat16* plane, float4 v) {
+  uint32_t lo[3], hi[3];
+  split3(v.x, v.y, lo);
+  split3(v.z, v.w, hi);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(plane + k * kPlane) = make_uint2(lo[k], hi[k]);
+}
+
+// ssd_state_kernel for bf16: a warp takes 16 (N = 64: 8) columns n and all 64 rows p
+template <int N, bool kGrad>
+__global__ void __launch_bounds__(kThreads) ssd_state_mma_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  using H = __nv_bfloat16;
+  constexpr int kPitchB = N + 8, NT = N / 64;
+  H *sX = reinterpret_cast<H*>(sm), *sB = sX + 3 * kPlane;
+  float *s_dt = reinterpret_cast<float*>(sB + kT * kPitchB), *s_cum = s_dt + kT;
+  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), g = h / (p.h / p.g);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if constexpr (kGrad) copy_rows<N>(sB, kPitchB, static_cast<const H*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows);
+  else copy_rows<N>(sB, kPitchB, static_cast<const H*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows);
+  const int64_t stride = kGrad ? static_cast<int64_t>(p.h) * kP : p.x_sl;
+  const H* x = kGrad ? static_cast<const H*>(p.dy) + ((static_cast<int64_t>(b) * p.l + t0) * p.h + h) * kP : static_cast<const H*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP;
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = threadIdx.x + k * kThreads, r = i / 16;
+    v[k] = r < rows ? ld4(x + r * stride + (i % 16) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  block_decay(s_dt, s_cum, p.dt + (static_cast<int64_t>(b) * p.l + t0) * p.h + h, p.h, rows, p.A[h]);
+  const float end = s_cum[kT - 1];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = threadIdx.x + k * kThreads, r = i / 16;
+    const float f = r >= rows ? 0.f : kGrad ? expf(s_cum[r]) : expf(end - s_cum[r]) * s_dt[r];
+    store_split(sX + r * kPitchH + (i % 16) * 4, make_float4(v[k].x * f, v[k].y * f, v[k].z * f, v[k].w * f));
+  }
+  if (!kGrad && threadIdx.x == 0) p.decay[(static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c] = expf(end);
+  __syncthreads();
+  const int n0 = warp * (8 * NT);
+  float acc[4][NT][4], low[4][NT][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = low[m][n][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < kT / 16; ++k) {
+    uint32_t fb[4];
+    const H* bp = sB + (k * 16 + (lane & 15)) * kPitchB + n0;
+    if constexpr (NT == 2) ldm4_trans(fb, bp + (lane >> 4) * 8);
+    else ldm2_trans(fb[0], fb[1], bp);
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        uint32_t fa[4];
+        ldm4_trans(fa, sX + q * kPlane + (k * 16 + (lane & 7) + (lane >> 4) * 8) * kPitchH + m * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma16816(q == 0 ? acc[m][n] : low[m][n], fa, fb[2 * n], fb[2 * n + 1]);
+      }
+  }
+  float* out = (kGrad ? p.dstates : p.states) + ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N);
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      float* o = out + (m * 16 + (lane >> 2)) * N + n0 + n * 8 + (lane & 3) * 2;
+      *reinterpret_cast<float2*>(o) = make_float2(acc[m][n][0] + low[m][n][0], acc[m][n][1] + low[m][n][1]);
+      *reinterpret_cast<float2*>(o + 8 * N) = make_float2(acc[m][n][2] + low[m][n][2], acc[m][n][3] + low[m][n][3]);
+    }
+}
+
+// ssd_out_kernel for bf16: a warp takes 8 columns p and all 64 rows t.  Its rows of the state come straight from memory into the operand's
+// registers: a thread's four neighbouring values stand for the k slots 2i, 2i + 1, 2i + 8, 2i + 9 in both operands.
+template <int N>
+__global__ void __launch_bounds__(kThreads, 3) ssd_out_mma_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  using H = __nv_bfloat16;
+  constexpr int kPitchC = N + 16;
+  H *sM = reinterpret_cast<H*>(sm), *sX = sM + 3 * kPlane, *sC = sX + kPlane;
+  float *s_dt = reinterpret_cast<float*>(sC + kT * kPitchC), *s_cum = s_dt + kT;
+  const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), g = h / (p.h / p.g);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, tg = lane & 3;
+  const float* S = p.states + ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N) + (warp * 8 + gr) * N + tg * 4;
+  float4 st[N / 16];
+#pragma unroll
+  for (int k = 0; k < N / 16; ++k) st[k] = *reinterpret_cast<const float4*>(S + k * 16);
+  const float* G = p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT);
+  float4 v[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] = *reinterpret_cast<const float4*>(G + (threadIdx.x + k * kThreads) * 4);
+  copy_rows<N>(sC, kPitchC, static_cast<const H*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows);
+  copy_rows<kP>(sX, kPitchH, static_cast<const H*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP, p.x_sl, rows);
+  block_decay(s_dt, s_cum, p.dt + (static_cast<int64_t>(b) * p.l + t0) * p.h + h, p.h, rows, p.A[h]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = threadIdx.x + k * kThreads, t = i / 16, u = (i % 16) * 4;
+    float e[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = u + q <= t ? e[q] * expf(s_cum[t] - s_cum[u + q]) * s_dt[u + q] : 0.f;
+    store_split(sM + t * kPitchH + u, make_float4(e[0], e[1], e[2], e[3]));
+  }
+  __syncthreads();
+  float acc[4][4], low[4][4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[m][e] = low[m][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < N / 16; ++k) {
+    uint32_t b0[3], b1[3];
+    split3(st[k].x, st[k].y, b0);
+    split3(st[k].z, st[k].w, b1);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const H* cp = sC + (m * 16 + gr) * kPitchC + k * 16 + tg * 4;
+      const uint2 r0 = *reinterpret_cast<const uint2*>(cp), r1 = *reinterpret_cast<const uint2*>(cp + 8 * kPitchC);
+      const uint32_t fa[4] = {r0.x, r1.x, r0.y, r1.y};
+#pragma unroll
+      for (int q = 0; q < 3; ++q) mma16816(q == 0 ? acc[m] : low[m], fa, b0[q], b1[q]);
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const float e0 = expf(s_cum[m * 16 + gr]), e1 = expf(s_cum[m * 16 + gr + 8]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      acc[m][e] = (acc[m][e] + low[m][e]) * (e < 2 ? e0 : e1);
+      low[m][e] = 0.f;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kT / 16; ++k) {
+    uint32_t x0, x1;
+    ldm2_trans(x0, x1, sX + (k * 16 + (lane & 15)) * kPitchH + warp * 8);
+#pragma unroll
+    for (int m = k; m < 4; ++m)                 // nothing above the diagonal
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        uint32_t fa[4];
+        ldm4(fa, sM + q * kPlane + (m * 16 + (lane & 15)) * kPitchH + k * 16 + (lane >> 4) * 8);
+        mma16816(q == 0 ? acc[m] : low[m], fa, x0, x1);
+      }
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[m][e] += low[m][e];
+  const float d = p.D[h];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int at = (m * 16 + gr + 8 * e) * kPitchH + warp * 8 + tg * 2;
+      const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sX + at));
+      *reinterpret_cast<__nv_bfloat162*>(sM + at) = __floats2bfloat162_rn(fmaf(d, xv.x, acc[m][2 * e]), fmaf(d, xv.y, acc[m][2 * e + 1]));
+    }
+  __syncthreads();
+  H* y = static_cast<H*>(p.y) + ((static_cast<int64_t>(b) * p.l + t0) * p.h + h) * kP;
+  for (int i = threadIdx.x; i < rows * (kP / 8); i += kThreads) {
+    const int t = i / (kP / 8), q = (i % (kP / 8)) * 8;
+    *reinterpret_cast<uint4*>(y + static_cast<int64_t>(t) * p.h * kP + q) = *reinterpret_cast<const uint4*>(sM + t * kPitchH + q);
+  }
 }
 
 // along the blocks, in place.  Forward: each block's contribution becomes the state it starts from.  Reverse: the gradient of each block's
@@ -526,6 +737,8 @@ __global__ void __launch_bounds__(kThreads) ssd_merge_kernel(const float4* __res
 template <int N> constexpr int scores_smem() { return 2 * kT * (N + 4) * 4; }
 template <int N> constexpr int state_smem() { return (kT * kPitchT + kT * (N + 4) + 2 * kT) * 4; }
 template <int N> constexpr int out_smem() { return (2 * kT * kPitchT + 2 * kT * (N + 4) + 2 * kT) * 4; }
+template <int N> constexpr int state_mma_smem() { return (3 * kPlane + kT * (N + 8)) * 2 + 2 * kT * 4; }
+template <int N> constexpr int out_mma_smem() { return (4 * kPlane + kT * (N + 16)) * 2 + 2 * kT * 4; }
 template <int N> constexpr int grad_smem() { return (4 * kT * (N + 4) + 5 * kT * kPitchT + 13 * kT + 16) * 4; }
 static_assert(grad_smem<128>() <= 232448, "one CTA's shared memory");
 
@@ -536,24 +749,38 @@ bool with_smem(K kern, int bytes) {
 
 template <int N, typename T>
 bool forward(const SsdArgs& p, cudaStream_t s) {
-  static const bool ok = with_smem(ssd_scores_kernel<N, T>, scores_smem<N>()) && with_smem(ssd_state_kernel<N, T, false>, state_smem<N>()) &&
-                         with_smem(ssd_out_kernel<N, T>, out_smem<N>());
+  constexpr bool mma = std::is_same<T, __nv_bfloat16>::value;
+  const dim3 grid(p.n_chunks, p.h, p.b);
+  static const bool ok = [] {
+    bool all = with_smem(ssd_scores_kernel<N, T>, scores_smem<N>());
+    if constexpr (mma) return all && with_smem(ssd_state_mma_kernel<N, false>, state_mma_smem<N>()) && with_smem(ssd_out_mma_kernel<N>, out_mma_smem<N>());
+    else return all && with_smem(ssd_state_kernel<N, T, false>, state_smem<N>()) && with_smem(ssd_out_kernel<N, T>, out_smem<N>());
+  }();
   if (!ok) return false;
   ssd_scores_kernel<N, T><<<dim3(p.n_chunks, p.g, p.b), kThreads, scores_smem<N>(), s>>>(p);
-  ssd_state_kernel<N, T, false><<<dim3(p.n_chunks, p.h, p.b), kThreads, state_smem<N>(), s>>>(p);
+  if constexpr (mma) ssd_state_mma_kernel<N, false><<<grid, kThreads, state_mma_smem<N>(), s>>>(p);
+  else ssd_state_kernel<N, T, false><<<grid, kThreads, state_smem<N>(), s>>>(p);
   constexpr int per = kP * N / 4;
   ssd_pass_kernel<false><<<dim3(per / kThreads, p.b * p.h), kThreads, 0, s>>>(reinterpret_cast<float4*>(p.states), p.decay,
                                                                               reinterpret_cast<const float4*>(p.first), reinterpret_cast<float4*>(p.last),
                                                                               p.n_chunks, per);
-  ssd_out_kernel<N, T><<<dim3(p.n_chunks, p.h, p.b), kThreads, out_smem<N>(), s>>>(p);
+  if constexpr (mma) ssd_out_mma_kernel<N><<<grid, kThreads, out_mma_smem<N>(), s>>>(p);
+  else ssd_out_kernel<N, T><<<grid, kThreads, out_smem<N>(), s>>>(p);
   return true;
 }
 
 template <int N, typename T>
 bool backward(const SsdArgs& p, cudaStream_t s) {
-  static const bool ok = with_smem(ssd_state_kernel<N, T, true>, state_smem<N>()) && with_smem(ssd_grad_kernel<N, T>, grad_smem<N>());
+  constexpr bool mma = std::is_same<T, __nv_bfloat16>::value;
+  const dim3 grid(p.n_chunks, p.h, p.b);
+  static const bool ok = [] {
+    bool all = with_smem(ssd_grad_kernel<N, T>, grad_smem<N>());
+    if constexpr (mma) return all && with_smem(ssd_state_mma_kernel<N, true>, state_mma_smem<N>());
+    else return all && with_smem(ssd_state_kernel<N, T, true>, state_smem<N>());
+  }();
   if (!ok) return false;
-  ssd_state_kernel<N, T, true><<<dim3(p.n_chunks, p.h, p.b), kThreads, state_smem<N>(), s>>>(p);
+  if constexpr (mma) ssd_state_mma_kernel<N, true><<<grid, kThreads, state_mma_smem<N>(), s>>>(p);
+  else ssd_state_kernel<N, T, true><<<grid, kThreads, state_smem<N>(), s>>>(p);
   constexpr int per = kP * N / 4;
   ssd_pass_kernel<true><<<dim3(per / kThreads, p.b * p.h), kThreads, 0, s>>>(reinterpret_cast<float4*>(p.dstates), p.decay,
                                                                              reinterpret_cast<const float4*>(p.dlast), reinterpret_cast<float4*>(p.dfirst),

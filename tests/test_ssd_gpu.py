@@ -57,6 +57,28 @@ def test_against_the_recurrence(b, l, h, g, n, dtype, init, steep):
         assert float((a.detach().double() - w.detach()).norm()) <= tol * max(float(w.norm()), 1e-6), i
 
 
+@pytest.mark.parametrize("b,l,h,g,n,steep", [(1, 1, 1, 1, 64, 1.0), (2, 65, 4, 2, 128, 1.0), (1, 191, 6, 3, 64, 1.0), (1, 300, 2, 1, 128, 30.0)])
+def test_bf16_inputs_are_no_less_exact(b, l, h, g, n, steep):
+    """The tensor instructions' three-part operands against the fp32 kernels fed with the same numbers: final state, state gradients, and y
+    up to its own rounding."""
+    from megatronapp_b200.ssm.mamba import ssd_scan
+
+    ins = _case(b, l, h, g, n, torch.bfloat16, True, steep)
+    wide, full = ([t.detach().to(d).requires_grad_() for t in ins] for d in (torch.float64, torch.float32))
+    want_y, want_last = _oracle(*wide)
+    outs = [ssd_scan(*i[:6], initial_state=i[6]) for i in (ins, full)]
+    dy, dl = torch.randn_like(outs[0][0]), torch.randn_like(want_last).float()
+    want_d = torch.autograd.grad((want_y, want_last), (wide[1], wide[6]), (dy.double(), dl.double()))
+    errors = []
+    for i, (y, last) in zip((ins, full), outs):
+        got = torch.autograd.grad((y, last), (i[1], i[6]), (dy.to(y.dtype), dl))
+        errors.append([float((a.detach().double() - w.detach()).norm() / w.detach().norm()) for a, w in zip((last, *got), (want_last, *want_d))])
+    # sums in another order: the same size of error, not the same error
+    assert all(e <= 1.5 * f + 2.0 ** -23 for e, f in zip(*errors)), errors
+    # y is off by a unit only where the exact result lies within the fp32 error of a rounding boundary: 2e-5 of its size against 2^-9 to 2^-8
+    assert float((outs[0][0] != want_y.bfloat16()).float().mean()) <= 0.02
+
+
 def test_other_ways_to_differentiate():
     """Only the final state's gradient, a second derivative, and forward-mode take the routes that they need."""
     from megatronapp_b200.ssm.mamba import ssd_scan, ssd_scan_torch
