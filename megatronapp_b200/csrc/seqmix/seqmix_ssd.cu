@@ -120,22 +120,34 @@ __device__ __forceinline__ void load_rows(float* dst, int pitch, const T* src, i
 }
 struct One { __device__ float operator()(int) const { return 1.f; } };
 
-// dt and the running sum of dt * A of one block (dt = 0 from `rows` on); all threads call it
+// dt and the running sum of dt * A of one block (dt = 0 from `rows` on); all threads call it.  The sum goes step by step: neighbours then share
+// what was rounded before them, and the exponentials of their differences keep it out (a scan over the lanes left 2^-24 of the sum in each).
 __device__ __forceinline__ void block_decay(float* s_dt, float* s_cum, const float* dt, int64_t stride, int rows, float a) {
   if (threadIdx.x < 32) {
     const int l = threadIdx.x;
-    const float d0 = 2 * l < rows ? dt[2 * l * stride] : 0.f, d1 = 2 * l + 1 < rows ? dt[(2 * l + 1) * stride] : 0.f;
-    const float v0 = d0 * a, pair = v0 + d1 * a;
-    float incl = pair;
+    const float d0 = l < rows ? dt[l * stride] : 0.f, d1 = l + 32 < rows ? dt[(l + 32) * stride] : 0.f;
+    s_dt[l] = d0;
+    s_dt[l + 32] = d1;
+    s_cum[l] = d0 * a;
+    s_cum[l + 32] = d1 * a;
+    __syncwarp();
+    if (l == 0) {
+      float run = 0.f;
+#pragma unroll 1
+      for (float4* q = reinterpret_cast<float4*>(s_cum); q < reinterpret_cast<float4*>(s_cum + kT); q += 4) {
+        float4 v[4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (l >= o) incl += v;
+        for (int i = 0; i < 4; ++i) v[i] = q[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          run += v[i].x; v[i].x = run;
+          run += v[i].y; v[i].y = run;
+          run += v[i].z; v[i].z = run;
+          run += v[i].w; v[i].w = run;
+          q[i] = v[i];
+        }
+      }
     }
-    s_dt[2 * l] = d0;
-    s_dt[2 * l + 1] = d1;
-    s_cum[2 * l] = (incl - pair) + v0;
-    s_cum[2 * l + 1] = incl;
   }
   __syncthreads();
 }

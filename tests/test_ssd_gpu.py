@@ -123,12 +123,13 @@ def test_mixer_core(s, b, hidden, g, n, dtype):
     u = (y.reshape(b, s, di) * torch.nn.functional.silu(z)).view(b, s, g, di // g)
     want = ((u * torch.rsqrt(u.pow(2).mean(-1, keepdim=True) + 1e-5)).view(b, s, di) * wide[6]).transpose(0, 1)
     plain = mixer_core_torch(*ins, g, 64, scan=ssd_scan_torch).to(dtype)
-    do = torch.randn_like(out)
+    do = rnd(*out.shape).to(dtype)
     off = lambda a, w: float((a.detach().double() - w.detach()).norm())  # noqa: E731
     got, ref, other = torch.autograd.grad(out, ins, do), torch.autograd.grad(want, wide, do.double()), torch.autograd.grad(plain, ins, do)
     for i, (a, w, o) in enumerate(zip([out, *got], [want, *ref], [plain, *other])):
         # fp32: rounding of the sums; bf16: the stored x B C, y and the gradients between the kernels each carry half a unit of 2^-8, and their
         # results' own; independent, four of them.  In sums that cancel (over all steps, for A and the steps' bias) those roundings stand against
-        # the terms and not the sum, as they do in the PyTorch form, which rounds at more places
+        # the terms and not the sum, as they do in the PyTorch form, which rounds at more places: two draws of like errors over the heads, eight
+        # or more independent ones, whose norms stay within twice one another
         limit = (5e-5 if dtype == torch.float32 else 2.0 ** -7) * max(float(w.detach().norm()), 1e-6)
-        assert off(a, w) <= (limit if dtype == torch.float32 else max(limit, off(o, w))), i
+        assert off(a, w) <= (limit if dtype == torch.float32 else max(limit, 2 * off(o, w))), i
