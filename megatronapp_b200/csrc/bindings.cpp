@@ -535,6 +535,48 @@ Tensor embedding_grad(const Tensor& dy, const Tensor& ids, int64_t vocab) {
   count();
   return dw;
 }
+static b200::RouterArgs router_args(const Tensor& x, const Tensor& w) {
+  TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.is_contiguous() && w.is_contiguous() && x.size(1) == w.size(1) &&
+              x.size(1) % 8 == 0 && x.size(0) > 0 && x.size(0) < (1 << 28) && w.size(0) > 0 && w.size(0) <= 256 && x.size(1) > 0 && x.size(1) <= (1 << 16),
+              "router_linear: shapes");
+  TORCH_CHECK((x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf) && (w.scalar_type() == at::kFloat || w.scalar_type() == x.scalar_type()) &&
+              reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0, "router_linear: types");
+  b200::RouterArgs a{};
+  a.x = x.data_ptr(); a.w = w.data_ptr();
+  a.n = static_cast<int>(x.size(0)); a.h = static_cast<int>(x.size(1)); a.experts = static_cast<int>(w.size(0));
+  a.bf16 = is_bf16(x); a.w_f32 = w.scalar_type() == at::kFloat;
+  return a;
+}
+Tensor router_linear_fwd(const Tensor& x, const Tensor& w) {
+  c10::cuda::CUDAGuard guard(x.device());
+  auto a = router_args(x, w);
+  auto out = torch::empty({x.size(0), w.size(0)}, x.options().dtype(at::kFloat));
+  a.logits = out.data_ptr<float>();
+  b200::router_linear(a, cur_stream());
+  count();
+  return out;
+}
+std::vector<Tensor> router_linear_bwd(const Tensor& dlogits, const Tensor& x, const Tensor& w, bool need_x, bool need_w) {
+  c10::cuda::CUDAGuard guard(x.device());
+  auto a = router_args(x, w);
+  TORCH_CHECK(dlogits.is_cuda() && dlogits.scalar_type() == at::kFloat && dlogits.is_contiguous() && dlogits.dim() == 2 && dlogits.size(0) == x.size(0) &&
+              dlogits.size(1) == w.size(0), "router_linear: dlogits");
+  a.dlogits = dlogits.data_ptr<float>();
+  Tensor dx, dw, part;
+  if (need_x) {
+    dx = torch::empty_like(x);
+    a.dx = dx.data_ptr();
+  }
+  if (need_w) {
+    dw = torch::empty_like(w);
+    part = torch::empty({b200::router_shares(a.n), w.size(0), w.size(1)}, dlogits.options());
+    a.dw = dw.data_ptr();
+    a.part = part.data_ptr<float>();
+  }
+  b200::router_linear(a, cur_stream());
+  count();
+  return {dx, dw};
+}
 void bias_grad(const Tensor& dy, Tensor& dbias, bool accumulate) {
   c10::cuda::CUDAGuard guard(dy.device());
   const bool f32 = dbias.scalar_type() == at::kFloat;
@@ -1107,6 +1149,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout_bwd", &dropout_bwd);
   m.def("rope_apply", &rope_apply);
   m.def("bias_grad", &bias_grad);
+  m.def("router_linear_fwd", &router_linear_fwd);
+  m.def("router_linear_bwd", &router_linear_bwd);
   m.def("embedding_grad", &embedding_grad);
   m.def("ce_local_stats", &ce_local_stats);
   m.def("ce_rescale", &ce_rescale);

@@ -58,6 +58,10 @@ class TopKRouter(MegatronModule):
     def gating(self, x):
         dt = torch.float32 if self.config.moe_router_dtype == "fp32" else (
             torch.float64 if self.config.moe_router_dtype == "fp64" else x.dtype)
+        if dt == torch.float32 and self.logit_bias is None:
+            from ..ops.moe import router_linear
+
+            return router_linear(x, self.weight)
         return torch.nn.functional.linear(x.to(dt), self.weight.to(dt), None if self.logit_bias is None else self.logit_bias.to(dt))
 
     def apply_input_jitter(self, x):
