@@ -9,10 +9,11 @@
 // gradient that enters each block's starting state, walked in reverse, then one kernel for all gradients of a block, whose CTA walks the
 // heads of a group so that the gradients of B and C add up in registers.  Exponents above the diagonal are never taken (they can overflow).
 //
-// fp32 inputs, and the gradients: tiles in fp32 in shared memory, 4 x 4 or 4 x 8 results per thread, bound by fp32 multiply-adds (2.1 M per
-// head and block backward, 1.3 M forward) and the shared-memory reads that feed them.  bf16 inputs: block states and outputs on the tensor
-// instructions (64 heads x 2048 steps x 64 x 128: outputs 140 -> 56 us, states 57 -> 33.5 and 59 -> 33.5; the final state's and the initial
-// state's gradient's errors are 2.3e-7 and 1.0e-7 of their size, with multiply-adds 2.4e-7 and 1.8e-7).  The block-by-block PyTorch form took some 2900 launches and 14 ms of
+// fp32 inputs: tiles in fp32 in shared memory, 4 x 4 or 4 x 8 results per thread, bound by fp32 multiply-adds (2.1 M per head and block
+// backward, 1.3 M forward) and the shared-memory reads that feed them.  bf16 inputs: block states, outputs and gradients on the tensor
+// instructions (64 heads x 2048 steps x 64 x 128: outputs 140 -> 56 us, states 57 -> 34 and 59 -> 34, gradients 383 -> 191; errors of the final
+// state, the gradients of dt and of the initial state 1.8e-7, 3.2e-7 and 1.2e-7 of their size at 65 steps, with multiply-adds 1.9e-7, 3.5e-7
+// and 1.9e-7).  The block-by-block PyTorch form took some 2900 launches and 14 ms of
 // device time for 64 heads x 2048 steps.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -242,7 +243,7 @@ template <int W>
 __device__ __forceinline__ void copy_rows(__nv_bfloat16* dst, int pitch, const __nv_bfloat16* src, int64_t stride, int rows) {
 #pragma unroll
   for (int k = 0; k < kT * (W / 4) / kThreads; ++k) {
-    const int i = threadIdx.x + k * kThreads, r = i / (W / 4), c = (i % (W / 4)) * 4;
+    const int i = (threadIdx.x & (kThreads - 1)) + k * kThreads, r = i / (W / 4), c = (i % (W / 4)) * 4;
     *reinterpret_cast<uint2*>(dst + r * pitch + c) = r < rows ? *reinterpret_cast<const uint2*>(src + r * stride + c) : make_uint2(0u, 0u);
   }
 }
@@ -732,6 +733,356 @@ __global__ void __launch_bounds__(2 * kThreads, 1) ssd_grad_kernel(const SsdArgs
   }
 }
 
+// ssd_grad_kernel for bf16, the same two halves.  A warp takes 16 rows and half of the columns of every product, so sums along a row come from
+// two warps.  The states and the decayed scores stand in shared memory as three bf16 planes.  Bound by the tensor instructions (about 2700 per
+// head and block, 18 cycles each in a scheduler: 90 us of the 191 at 64 heads x 2048 steps) and the phases between them.
+template <int N>
+__global__ void __launch_bounds__(2 * kThreads, 1) ssd_grad_mma_kernel(const SsdArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  using H = __nv_bfloat16;
+  constexpr int kPitchN = N + 8, kPlaneN = kT * kPitchN, NT = N / 16;    // n tiles of 8 in half of the columns
+  H* sC = reinterpret_cast<H*>(sm);            // [t][n]
+  H* sB = sC + kPlaneN;                        // [u][n]
+  H* sS = sB + kPlaneN;                        // 3 x [p][n] state at the block's start
+  H* sR = sS + 3 * kPlaneN;                    // 3 x [p][n] gradient of the state at its end
+  H* sX = sR + 3 * kPlaneN;                    // [u][p]
+  H* sY = sX + kPlane;                         // [t][p] dy
+  H* sM = sY + kPlane;                         // 3 x [t][u] decayed scores, then the group's score gradients
+  float* sG = reinterpret_cast<float*>(sM + 3 * kPlane);    // [t][u]
+  float* sQ = sG + kT * kPitchT;               // [u][p] the end state's part of dx
+  float* s_dt = sQ + kT * kPitchT;
+  float *s_cum = s_dt + kT, *s_row = s_cum + kT, *s_end = s_row + 4 * kT, *s_dir = s_end + 2 * kT, *s_col = s_dir + 2 * kT, *s_red = s_col + 4 * kT;
+  const int c = blockIdx.x, b = blockIdx.z, t0 = c * kT, rows = min(kT, p.l - t0), hpg = p.h / p.g;
+  const int g = blockIdx.y / p.n_sub, sub = blockIdx.y % p.n_sub, per = hpg / p.n_sub;
+  const bool second = threadIdx.x >= kThreads;
+  const int tid = threadIdx.x & (kThreads - 1), warp = tid >> 5, lane = tid & 31, gr = lane >> 2, tg = lane & 3;
+  const int m0 = (warp & 3) * 16, side = warp >> 2;             // this warp's rows, and which half of the columns
+  const int h0 = g * hpg + sub * per;
+  // operand addresses of this lane, see ldm4: rows x k as stored, k x rows transposed; n x k as stored, k x n transposed
+  auto a_at = [&](const H* base, int pitch, int m, int k) { return base + (m + (lane & 15)) * pitch + k + (lane >> 4) * 8; };
+  auto at_at = [&](const H* base, int pitch, int m, int k) { return base + (k + (lane & 7) + (lane >> 4) * 8) * pitch + m + ((lane >> 3) & 1) * 8; };
+  auto b_at = [&](const H* base, int pitch, int n, int k) { return base + (n + (lane & 7) + (lane >> 4) * 8) * pitch + k + ((lane >> 3) & 1) * 8; };
+  auto bt_at = [&](const H* base, int pitch, int n, int k) { return base + (k + (lane & 15)) * pitch + n + (lane >> 4) * 8; };
+  auto quad_sum = [](float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+  };
+  // the second half fetches a head's states and takes its part of their product on the way
+  auto fetch_states = [&](int h) {
+    const int64_t at = ((static_cast<int64_t>(b) * p.h + h) * p.n_chunks + c) * (kP * N);
+    float rs = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < kP * (N / 4) / kThreads; ++k) {
+      const int i = tid + k * kThreads, r = i / (N / 4), q = (i % (N / 4)) * 4;
+      const float4 s = *reinterpret_cast<const float4*>(p.states + at + r * N + q), e = *reinterpret_cast<const float4*>(p.dstates + at + r * N + q);
+      rs += s.x * e.x + s.y * e.y + s.z * e.z + s.w * e.w;
+      uint32_t lo[3], hi[3];
+      split3(s.x, s.y, lo);
+      split3(s.z, s.w, hi);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(sS + j * kPlaneN + r * kPitchN + q) = make_uint2(lo[j], hi[j]);
+      split3(e.x, e.y, lo);
+      split3(e.z, e.w, hi);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(sR + j * kPlaneN + r * kPitchN + q) = make_uint2(lo[j], hi[j]);
+    }
+    return dev::warp_sum(rs);
+  };
+  float rs = 0.f;
+  if (second) rs = fetch_states(h0);
+  else {
+    copy_rows<N>(sC, kPitchN, static_cast<const H*>(p.C) + b * p.c_sb + t0 * p.c_sl + g * N, p.c_sl, rows);
+    copy_rows<N>(sB, kPitchN, static_cast<const H*>(p.B) + b * p.b_sb + t0 * p.b_sl + g * N, p.b_sl, rows);
+    load_rows<kT>(sG, kPitchT, p.scores + ((static_cast<int64_t>(b) * p.n_chunks + c) * p.g + g) * (kT * kT), static_cast<int64_t>(kT), kT, One{});
+  }
+  float acc[NT][4], dG[4][4];                  // dC in the first half, dB in the second
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+  zero(dG);
+  for (int hi = 0; hi < per; ++hi) {
+    const int h = h0 + hi;
+    const float a = p.A[h];
+    const int64_t row0 = (static_cast<int64_t>(b) * p.l + t0) * p.h + h;
+    __syncthreads();                           // the head before is done with its tiles
+    if (second) copy_rows<kP>(sX, kPitchH, static_cast<const H*>(p.x) + b * p.x_sb + t0 * p.x_sl + h * kP, p.x_sl, rows);
+    else copy_rows<kP>(sY, kPitchH, static_cast<const H*>(p.dy) + row0 * kP, static_cast<int64_t>(p.h) * kP, rows);
+    block_decay(s_dt, s_cum, p.dt + row0, p.h, rows, a);  // and all tiles are there
+    const float end = s_cum[kT - 1];
+    const int r0 = m0 + gr, r1 = r0 + 8;       // this thread's two rows
+    const float cum0 = s_cum[r0], cum1 = s_cum[r1];
+    uint32_t fx[4][4];                         // the warp's rows of Y (first half) or X
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ldm4(fx[k], a_at(second ? sX : sY, kPitchH, m0, k * 16));
+
+    if (!second) {
+      // gradient of the scores, and through their decays of cum
+      {
+        float v[4][4];
+        zero(v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            uint32_t fb[4];
+            ldm4(fb, b_at(sX, kPitchH, side * 32 + j * 8, k * 16));
+            mma16816(v[j], fx[k], fb[0], fb[1]);
+            mma16816(v[j + 1], fx[k], fb[2], fb[3]);
+          }
+        float row[2] = {0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int u = side * 32 + j * 8 + tg * 2;
+          float col[2] = {0.f, 0.f}, wg[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int t = e < 2 ? r0 : r1, uu = u + (e & 1);
+            const float w = uu <= t ? expf((e < 2 ? cum0 : cum1) - s_cum[uu]) : 0.f;
+            wg[e] = w * sG[t * kPitchT + uu];
+            const float d = v[j][e] * s_dt[uu];
+            dG[j][e] = fmaf(d, w, dG[j][e]);
+            const float q = uu < t ? d * wg[e] : 0.f;      // on the diagonal the two ends cancel
+            row[e >> 1] += q;
+            col[e & 1] += q;
+          }
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            uint32_t part[3];
+            split3(wg[2 * e], wg[2 * e + 1], part);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) *reinterpret_cast<uint32_t*>(sM + q * kPlane + (e == 0 ? r0 : r1) * kPitchH + u) = part[q];
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) col[e] += __shfl_xor_sync(0xffffffffu, col[e], o);
+          }
+          if (gr == 0) {
+            s_col[(warp & 3) * kT + u] = col[0];
+            s_col[(warp & 3) * kT + u + 1] = col[1];
+          }
+        }
+        row[0] = quad_sum(row[0]);
+        row[1] = quad_sum(row[1]);
+        if (tg == 0) {
+          s_row[side * kT + r0] = row[0];
+          s_row[side * kT + r1] = row[1];
+        }
+      }
+    } else {
+      // the end state's part of dx
+      float v[4][4], low[4][4];
+      zero(v);
+      zero(low);
+#pragma unroll 2
+      for (int k = 0; k < N / 16; ++k) {
+        uint32_t fa[4];
+        ldm4(fa, a_at(sB, kPitchN, m0, k * 16));
+#pragma unroll
+        for (int j = 0; j < 4; j += 2)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            uint32_t fb[4];
+            ldm4(fb, b_at(sR + q * kPlaneN, kPitchN, side * 32 + j * 8, k * 16));
+            mma16816(q == 0 ? v[j] : low[j], fa, fb[0], fb[1]);
+            mma16816(q == 0 ? v[j + 1] : low[j + 1], fa, fb[2], fb[3]);
+          }
+      }
+      const float e0 = expf(end - cum0), e1 = expf(end - cum1);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float* o = sQ + r0 * kPitchT + side * 32 + j * 8 + tg * 2;
+        *reinterpret_cast<float2*>(o) = make_float2(e0 * (v[j][0] + low[j][0]), e0 * (v[j][1] + low[j][1]));
+        *reinterpret_cast<float2*>(o + 8 * kPitchT) = make_float2(e1 * (v[j][2] + low[j][2]), e1 * (v[j][3] + low[j][3]));
+      }
+    }
+    // C through the starting state (first half), B through the end state (second): 32 columns at a time
+    {
+      const float e0 = second ? expf(end - cum0) * s_dt[r0] : expf(cum0), e1 = second ? expf(end - cum1) * s_dt[r1] : expf(cum1);
+      float row[2] = {0.f, 0.f};
+#pragma unroll
+      for (int n0 = 0; n0 < NT; n0 += 4) {
+        float v[4][4], low[4][4];
+        zero(v);
+        zero(low);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int j = 0; j < 4; j += 2)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+              uint32_t fb[4];
+              ldm4_trans(fb, bt_at((second ? sR : sS) + q * kPlaneN, kPitchN, side * (N / 2) + (n0 + j) * 8, k * 16));
+              mma16816(q == 0 ? v[j] : low[j], fx[k], fb[0], fb[1]);
+              mma16816(q == 0 ? v[j + 1] : low[j + 1], fx[k], fb[2], fb[3]);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const H* other = (second ? sB : sC) + r0 * kPitchN + side * (N / 2) + (n0 + j) * 8 + tg * 2;
+          const float2 o0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(other));
+          const float2 o1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(other + 8 * kPitchN));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float w = (e < 2 ? e0 : e1) * (v[j][e] + low[j][e]);
+            acc[n0 + j][e] += w;
+            row[e >> 1] = fmaf(w, e == 0 ? o0.x : e == 1 ? o0.y : e == 2 ? o1.x : o1.y, row[e >> 1]);
+          }
+        }
+      }
+      row[0] = quad_sum(row[0]);
+      row[1] = quad_sum(row[1]);
+      float* dst = second ? s_end + side * kT : s_row + (2 + side) * kT;
+      if (tg == 0) {
+        dst[r0] = row[0];
+        dst[r1] = row[1];
+      }
+    }
+    if (second && lane == 0) s_red[8 + warp] = rs;
+    __syncthreads();
+    if (second) {
+      if (hi + 1 < per) rs = fetch_states(h + 1);
+      continue;
+    }
+    // dx, dt through x, and D; rows are steps u now
+    float dd = 0.f;
+    {
+      float v[4][4], low[4][4];
+      zero(v);
+      zero(low);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k * 16 < m0) continue;             // no later step's scores before the diagonal
+        uint32_t fa[3][4];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) ldm4_trans(fa[q], at_at(sM + q * kPlane, kPitchH, m0, k * 16));
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+          uint32_t fb[4];
+          ldm4_trans(fb, bt_at(sY, kPitchH, side * 32 + j * 8, k * 16));
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            mma16816(q == 0 ? v[j] : low[j], fa[q], fb[0], fb[1]);
+            mma16816(q == 0 ? v[j + 1] : low[j + 1], fa[q], fb[2], fb[3]);
+          }
+        }
+      }
+      const float d = p.D[h];
+      H* dx = static_cast<H*>(p.dx) + row0 * kP;
+      float dir[2] = {0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int u = e == 0 ? r0 : r1, q = side * 32 + j * 8 + tg * 2;
+          const float2 end_part = *reinterpret_cast<const float2*>(sQ + u * kPitchT + q);
+          const float2 xv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sX + u * kPitchH + q));
+          const float2 yv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sY + u * kPitchH + q));
+          const float pre0 = v[j][2 * e] + low[j][2 * e] + end_part.x, pre1 = v[j][2 * e + 1] + low[j][2 * e + 1] + end_part.y;
+          dir[e] = fmaf(xv.x, pre0, fmaf(xv.y, pre1, dir[e]));
+          dd = fmaf(xv.x, yv.x, fmaf(xv.y, yv.y, dd));
+          if (u < rows)
+            *reinterpret_cast<__nv_bfloat162*>(dx + static_cast<int64_t>(u) * p.h * kP + q) =
+                __floats2bfloat162_rn(fmaf(s_dt[u], pre0, d * yv.x), fmaf(s_dt[u], pre1, d * yv.y));
+        }
+      dir[0] = quad_sum(dir[0]);
+      dir[1] = quad_sum(dir[1]);
+      if (tg == 0) {
+        s_dir[side * kT + r0] = dir[0];
+        s_dir[side * kT + r1] = dir[1];
+      }
+      dd = dev::warp_sum(dd);
+      if (lane == 0) s_red[warp] = dd;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");                  // the first half alone
+    // cum's gradient summed from the block's end, for dt and A
+    if (warp == 0) {
+      float g0[2], z = 0.f, acc_d = 0.f, acc_r = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        acc_d += s_red[w];
+        acc_r += s_red[8 + w];
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = 2 * lane + e;
+        const float to_end = s_end[t] + s_end[kT + t];
+        float v = (s_row[t] + s_row[kT + t]) + (s_row[2 * kT + t] + s_row[3 * kT + t]) - to_end;
+        z += to_end;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) v -= s_col[w * kT + t];
+        g0[e] = v;
+      }
+      z = dev::warp_sum(z);
+      if (lane == 31) g0[1] += z + expf(end) * acc_r;
+      float incl = g0[0] + g0[1];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float v = __shfl_down_sync(0xffffffffu, incl, o);
+        if (lane + o < 32) incl += v;
+      }
+      const float dda0 = incl, dda1 = incl - g0[0];
+      const int t = 2 * lane;
+      if (t < rows) p.ddt[row0 + static_cast<int64_t>(t) * p.h] = fmaf(a, dda0, s_dir[t] + s_dir[kT + t]);
+      if (t + 1 < rows) p.ddt[row0 + static_cast<int64_t>(t + 1) * p.h] = fmaf(a, dda1, s_dir[t + 1] + s_dir[kT + t + 1]);
+      const float da = dev::warp_sum(s_dt[t] * dda0 + s_dt[t + 1] * dda1);
+      if (lane == 0) {
+        const int64_t at = (static_cast<int64_t>(b) * p.n_chunks + c) * p.h + h;
+        p.dA[at] = da;
+        p.dD[at] = acc_d;
+      }
+    }
+  }
+  // the scores' gradients into B and C
+  __syncthreads();
+  if (!second) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        uint32_t part[3];
+        split3(dG[j][2 * e], dG[j][2 * e + 1], part);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          *reinterpret_cast<uint32_t*>(sM + q * kPlane + (m0 + gr + 8 * e) * kPitchH + side * 32 + j * 8 + tg * 2) = part[q];
+      }
+  }
+  __syncthreads();
+  uint32_t fa[4][3][4];                        // rows of the score gradients, or of their transpose
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      if (second) ldm4_trans(fa[k][q], at_at(sM + q * kPlane, kPitchH, m0, k * 16));
+      else ldm4(fa[k][q], a_at(sM + q * kPlane, kPitchH, m0, k * 16));
+    }
+  const int64_t plane = static_cast<int64_t>(p.b) * p.l * p.g * N;
+#pragma unroll
+  for (int j = 0; j < NT; j += 2) {
+    float v[2][4], low[2][4];
+    zero(v);
+    zero(low);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      uint32_t fb[4];
+      ldm4_trans(fb, bt_at(second ? sC : sB, kPitchN, side * (N / 2) + j * 8, k * 16));
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        mma16816(q == 0 ? v[0] : low[0], fa[k][q], fb[0], fb[1]);
+        mma16816(q == 0 ? v[1] : low[1], fa[k][q], fb[2], fb[3]);
+      }
+    }
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int t = m0 + gr + 8 * e;
+        if (t >= rows) continue;
+        const float o0 = acc[j + jj][2 * e] + (v[jj][2 * e] + low[jj][2 * e]), o1 = acc[j + jj][2 * e + 1] + (v[jj][2 * e + 1] + low[jj][2 * e + 1]);
+        const int64_t at = ((static_cast<int64_t>(b) * p.l + t0 + t) * p.g + g) * N + side * (N / 2) + (j + jj) * 8 + tg * 2;
+        if (p.n_sub == 1) *reinterpret_cast<__nv_bfloat162*>(static_cast<H*>(second ? p.dB : p.dC) + at) = __floats2bfloat162_rn(o0, o1);
+        else *reinterpret_cast<float2*>(p.partial + (sub * 2 + (second ? 0 : 1)) * plane + at) = make_float2(o0, o1);
+      }
+  }
+}
+
 // dB and dC from the partial sums of n_sub CTAs
 template <typename T>
 __global__ void __launch_bounds__(kThreads) ssd_merge_kernel(const float4* __restrict__ part, T* __restrict__ dB, T* __restrict__ dC, int64_t plane4, int n_sub) {
@@ -752,7 +1103,8 @@ template <int N> constexpr int out_smem() { return (2 * kT * kPitchT + 2 * kT * 
 template <int N> constexpr int state_mma_smem() { return (3 * kPlane + kT * (N + 8)) * 2 + 2 * kT * 4; }
 template <int N> constexpr int out_mma_smem() { return (4 * kPlane + kT * (N + 16)) * 2 + 2 * kT * 4; }
 template <int N> constexpr int grad_smem() { return (4 * kT * (N + 4) + 5 * kT * kPitchT + 13 * kT + 16) * 4; }
-static_assert(grad_smem<128>() <= 232448, "one CTA's shared memory");
+template <int N> constexpr int grad_mma_smem() { return (8 * kT * (N + 8) + 5 * kPlane) * 2 + (2 * kT * kPitchT + 14 * kT + 16) * 4; }
+static_assert(grad_smem<128>() <= 232448 && grad_mma_smem<128>() <= 232448, "one CTA's shared memory");
 
 template <typename K>
 bool with_smem(K kern, int bytes) {
@@ -786,9 +1138,8 @@ bool backward(const SsdArgs& p, cudaStream_t s) {
   constexpr bool mma = std::is_same<T, __nv_bfloat16>::value;
   const dim3 grid(p.n_chunks, p.h, p.b);
   static const bool ok = [] {
-    bool all = with_smem(ssd_grad_kernel<N, T>, grad_smem<N>());
-    if constexpr (mma) return all && with_smem(ssd_state_mma_kernel<N, true>, state_mma_smem<N>());
-    else return all && with_smem(ssd_state_kernel<N, T, true>, state_smem<N>());
+    if constexpr (mma) return with_smem(ssd_state_mma_kernel<N, true>, state_mma_smem<N>()) && with_smem(ssd_grad_mma_kernel<N>, grad_mma_smem<N>());
+    else return with_smem(ssd_state_kernel<N, T, true>, state_smem<N>()) && with_smem(ssd_grad_kernel<N, T>, grad_smem<N>());
   }();
   if (!ok) return false;
   if constexpr (mma) ssd_state_mma_kernel<N, true><<<grid, kThreads, state_mma_smem<N>(), s>>>(p);
@@ -797,7 +1148,9 @@ bool backward(const SsdArgs& p, cudaStream_t s) {
   ssd_pass_kernel<true><<<dim3(per / kThreads, p.b * p.h), kThreads, 0, s>>>(reinterpret_cast<float4*>(p.dstates), p.decay,
                                                                              reinterpret_cast<const float4*>(p.dlast), reinterpret_cast<float4*>(p.dfirst),
                                                                              p.n_chunks, per);
-  ssd_grad_kernel<N, T><<<dim3(p.n_chunks, p.g * p.n_sub, p.b), 2 * kThreads, grad_smem<N>(), s>>>(p);
+  const dim3 grad_grid(p.n_chunks, p.g * p.n_sub, p.b);
+  if constexpr (mma) ssd_grad_mma_kernel<N><<<grad_grid, 2 * kThreads, grad_mma_smem<N>(), s>>>(p);
+  else ssd_grad_kernel<N, T><<<grad_grid, 2 * kThreads, grad_smem<N>(), s>>>(p);
   if (p.n_sub > 1) {
     const int64_t plane4 = static_cast<int64_t>(p.b) * p.l * p.g * N / 4;
     ssd_merge_kernel<T><<<static_cast<unsigned>((2 * plane4 + kThreads - 1) / kThreads), kThreads, 0, s>>>(
