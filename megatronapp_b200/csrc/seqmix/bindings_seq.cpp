@@ -1028,7 +1028,8 @@ std::vector<Tensor> mamba_before_scan_grad(const Tensor& dxs, const Tensor& dB, 
   TORCH_CHECK(dxs.numel() == rows * p.di && dB.numel() == rows * gn && dC.numel() == rows * gn && ddt.numel() == rows * p.heads && dzx.is_contiguous() &&
               dzx.sizes() == zx.sizes() && dzx.scalar_type() == zx.scalar_type(), "bad gradients");
   check_f32(ddt, "ddt");
-  Tensor part = torch::empty({static_cast<int64_t>(p.b) * b200seq::mamba_conv_parts(p.s), 5, p.conv}, dt_bias.options());
+  p.conv_run = b200seq::mamba_conv_run(p.s, p.b, p.conv, zx.scalar_type() == at::kBFloat16);
+  Tensor part = torch::empty({static_cast<int64_t>(p.b) * b200seq::mamba_conv_parts(p.s, p.conv_run), 5, p.conv}, dt_bias.options());
   p.dxs = dxs.data_ptr(); p.dB = dB.data_ptr(); p.dC = dC.data_ptr(); p.ddt = ddt.data_ptr<float>(); p.dzx = dzx.data_ptr(); p.conv_part = part.data_ptr<float>();
   b200seq::mamba_before_scan_grad(p, zx.scalar_type() == at::kBFloat16, cur_stream());
   count(2); check_last_error("mamba_before_scan_grad");

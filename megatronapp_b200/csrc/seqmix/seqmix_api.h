@@ -346,9 +346,11 @@ struct MambaArgs {
   float* conv_part;               // [b * mamba_conv_parts, 5, conv]: four taps, bias
   float* norm_part;               // [mamba_norm_parts, di]
   int s, b, width, di, conv, heads, groups;
+  int conv_run;                   // backward: mamba_conv_run
   float eps;
 };
-int mamba_conv_parts(int steps);
+int mamba_conv_run(int steps, int batch, int conv, bool bf16);
+int mamba_conv_parts(int steps, int run);
 int mamba_norm_parts(int steps, int batch);
 void mamba_before_scan(const MambaArgs& p, bool bf16, cudaStream_t s);
 void mamba_before_scan_grad(const MambaArgs& p, bool bf16, cudaStream_t s);

@@ -35,7 +35,7 @@ template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16*
 }
 
 // ---- convolution.  A thread walks `kRun` steps of four channels with the window in registers.
-constexpr int kFwdRun = 16, kBwdRun = 32;
+constexpr int kFwdRun = 16, kBwdRun = 32;        // backward: 32 or a little more, see mamba_conv_run
 
 template <typename T>
 __global__ void __launch_bounds__(128) mamba_conv_kernel(const MambaArgs p) {
@@ -77,10 +77,10 @@ __global__ void __launch_bounds__(128) mamba_conv_kernel(const MambaArgs p) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128) mamba_conv_grad_kernel(const MambaArgs p) {
+__global__ void __launch_bounds__(128, 5) mamba_conv_grad_kernel(const MambaArgs p) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= p.conv) return;
-  const int t0 = blockIdx.y * kBwdRun, b = blockIdx.z;
+  const int run = p.conv_run, t0 = blockIdx.y * run, b = blockIdx.z;
   const int64_t step = static_cast<int64_t>(p.b) * p.width, at = static_cast<int64_t>(b) * p.width + p.di + c;
   const T* x = static_cast<const T*>(p.zx) + at;
   T* dx = static_cast<T*>(p.dzx) + at;
@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(128) mamba_conv_grad_kernel(const MambaArgs p)
 #pragma unroll
   for (int k = 0; k < 3; ++k)
     if (t0 - 3 + k >= 0) load4(x + (t0 - 3 + k) * step, win[k + 1]);
-#pragma unroll 2
-  for (int i = 0; i < kBwdRun + 3; ++i) {
+#pragma unroll 1
+  for (int i = 0; i < run + 3; ++i) {
     const int t = t0 + i;
     float g[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) mamba_conv_grad_kernel(const MambaArgs p)
       for (int k = 0; k < 4; ++k) v = fmaf(w[e][k], win[k][e], v);
       const float sg = sigmoidf_(v), pre = g[e] * (sg * fmaf(v, 1.f - sg, 1.f));
       d[3][e] = t < p.s ? pre : 0.f;
-      if (i < kBwdRun) {
+      if (i < run) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) dw[k][e] = fmaf(d[3][e], win[k][e], dw[k][e]);
         db[e] += d[3][e];
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(128) mamba_norm_kernel(const MambaArgs p) {
 }
 
 // four warps of a CTA share kNormRows rows of one group; kVec: groups of four channels per lane
-constexpr int kNormRows = 32;
+constexpr int kNormRows = 16;      // four to a warp, each two dependent passes: latency, so many CTAs (2048 x 4096: 52 us with 32 rows, 33 with 16)
 template <typename T, int kVec>
 __global__ void __launch_bounds__(128) mamba_norm_grad_kernel(const MambaArgs p) {
   extern __shared__ float s_dw[];
@@ -308,7 +308,7 @@ void before_scan(const MambaArgs& p, cudaStream_t s) {
 template <typename T>
 void before_scan_grad(const MambaArgs& p, cudaStream_t s) {
   const int64_t n = static_cast<int64_t>(p.b) * p.s * p.heads;
-  mamba_conv_grad_kernel<T><<<dim3((p.conv / 4 + 127) / 128, mamba_conv_parts(p.s), p.b), 128, 0, s>>>(p);
+  mamba_conv_grad_kernel<T><<<dim3((p.conv / 4 + 127) / 128, mamba_conv_parts(p.s, p.conv_run), p.b), 128, 0, s>>>(p);
   mamba_dt_kernel<T, true><<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(p);
 }
 template <typename T>
@@ -319,7 +319,19 @@ void norm(const MambaArgs& p, cudaStream_t s) {
 
 }  // namespace
 
-int mamba_conv_parts(int steps) { return (steps + kBwdRun - 1) / kBwdRun; }
+// Steps of a backward run.  A CTA takes long for what it does (35 dependent steps), so a last wave of a few CTAs costs as much as a full one:
+// the runs are lengthened until the last full wave holds them all (2048 steps x 6144 channels: 768 CTAs on 592 places 73 us, 588 with runs
+// of 42 steps 50; 96 registers instead of 104 make it 740 places, and 732 CTAs with runs of 34 steps take 44).
+int mamba_conv_run(int steps, int batch, int conv, bool bf16) {
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bf16 ? mamba_conv_grad_kernel<__nv_bfloat16> : mamba_conv_grad_kernel<float>, 128, 0) != cudaSuccess)
+    return kBwdRun;
+  const int64_t rows = static_cast<int64_t>((conv / 4 + 127) / 128) * batch, ctas = rows * ((steps + kBwdRun - 1) / kBwdRun);
+  const int64_t places = static_cast<int64_t>(sms) * per_sm, parts = ctas / (places > 0 ? places : 1) * places / rows;
+  return parts < 1 ? kBwdRun : static_cast<int>((steps + parts - 1) / parts < kBwdRun ? kBwdRun : (steps + parts - 1) / parts);
+}
+int mamba_conv_parts(int steps, int run) { return (steps + run - 1) / run; }
 int mamba_norm_parts(int steps, int batch) { return static_cast<int>((static_cast<int64_t>(steps) * batch + kNormRows - 1) / kNormRows); }
 
 void mamba_before_scan(const MambaArgs& p, bool bf16, cudaStream_t s) { bf16 ? before_scan<__nv_bfloat16>(p, s) : before_scan<float>(p, s); }

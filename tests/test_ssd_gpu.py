@@ -105,7 +105,8 @@ def test_other_ways_to_differentiate():
     (1, 1, 128, 1, 64, torch.float32),                        # one step; the convolution sees only padding before it
     (35, 3, 128, 2, 64, torch.float32),                       # one step more than a run and its halo, batch inside the rows
     (130, 2, 256, 8, 128, torch.bfloat16),                    # groups of 64 channels: a norm of half a warp
-    (66, 1, 2048, 1, 64, torch.bfloat16)])                    # one group of 4096 channels
+    (66, 1, 2048, 1, 64, torch.bfloat16),                     # one group of 4096 channels
+    (1030, 4, 1024, 8, 64, torch.bfloat16)])                  # more than one wave of the convolution's gradient: runs longer than 32 steps
 def test_mixer_core(s, b, hidden, g, n, dtype):
     """Everything between the two projections, against the same in 64 bits."""
     from megatronapp_b200.ssm.mamba import _MixerCoreFn, mixer_core_torch, ssd_scan_torch
