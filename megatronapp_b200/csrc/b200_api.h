@@ -182,18 +182,17 @@ struct EmbeddingGradArgs {
 int64_t embedding_grad_parts(int n, int h);
 void embedding_grad(const EmbeddingGradArgs& a, cudaStream_t s);
 
-// router logits [n, experts] = x [n, h] . w [experts, h]^T and gradients, whichever of logits, dx and dw is set; rows contiguous, h % 8 == 0
+// gradients of the router logits x [n, h] . w [experts, h]^T, whichever of dx and dw is set; rows contiguous, h % 8 == 0
 struct RouterArgs {
   const void *x, *w;
   const float* dlogits;
-  float* logits;
   void *dx, *dw;       // of x's and w's type
   float* part;         // for dw: router_shares(n) x experts x h
   int n, h, experts;
   bool bf16, w_f32;    // x (and w, unless fp32): bf16, else fp16
 };
 int router_shares(int n);
-void router_linear(const RouterArgs& a, cudaStream_t s);
+void router_linear_grad(const RouterArgs& a, cudaStream_t s);
 
 // vocab-parallel cross entropy pieces (fp32 statistics; logits 16-bit or fp32)
 void ce_local_stats(const void* logits, const int64_t* labels, float* row_max, float* row_sumexp,

@@ -547,15 +547,6 @@ static b200::RouterArgs router_args(const Tensor& x, const Tensor& w) {
   a.bf16 = is_bf16(x); a.w_f32 = w.scalar_type() == at::kFloat;
   return a;
 }
-Tensor router_linear_fwd(const Tensor& x, const Tensor& w) {
-  c10::cuda::CUDAGuard guard(x.device());
-  auto a = router_args(x, w);
-  auto out = torch::empty({x.size(0), w.size(0)}, x.options().dtype(at::kFloat));
-  a.logits = out.data_ptr<float>();
-  b200::router_linear(a, cur_stream());
-  count();
-  return out;
-}
 std::vector<Tensor> router_linear_bwd(const Tensor& dlogits, const Tensor& x, const Tensor& w, bool need_x, bool need_w) {
   c10::cuda::CUDAGuard guard(x.device());
   auto a = router_args(x, w);
@@ -573,7 +564,7 @@ std::vector<Tensor> router_linear_bwd(const Tensor& dlogits, const Tensor& x, co
     a.dw = dw.data_ptr();
     a.part = part.data_ptr<float>();
   }
-  b200::router_linear(a, cur_stream());
+  b200::router_linear_grad(a, cur_stream());
   count();
   return {dx, dw};
 }
@@ -1149,7 +1140,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout_bwd", &dropout_bwd);
   m.def("rope_apply", &rope_apply);
   m.def("bias_grad", &bias_grad);
-  m.def("router_linear_fwd", &router_linear_fwd);
   m.def("router_linear_bwd", &router_linear_bwd);
   m.def("embedding_grad", &embedding_grad);
   m.def("ce_local_stats", &ce_local_stats);

@@ -1,11 +1,12 @@
-// Router logits of a mixture of experts: a product with a handful of output columns, fp32 sums of 16-bit tokens and 16-bit or fp32 weights,
-// and its two gradients.  With so few columns the tokens' bytes are the bound, so they are read once, in 16 bits, and never widened in memory.
-//   logits: a warp takes two tokens and eight experts, 256 columns of all of them at a time.
-//   dx:     a thread takes eight columns of eight tokens and walks the experts.
-//   dw:     a thread takes eight columns of eight experts and walks its CTA's share of the tokens; a second kernel adds the shares in order.
-// Forward and backward, with an fp32 copy of the tokens and library products / here: 4096 tokens x 2048, 8 experts 161 / 36 us; 16 experts
-// 141 / 48; 4096 x 4096, 32 experts 270 / 155; 16384 x 4096, 32 experts 677 / 542; 512 x 1024, 8 experts 51 / 23.  With 64 experts the
-// products are work for larger tiles (16384 tokens' would be slower here), so 32 is the most that comes this way.
+// Gradients of a mixture of experts' router logits: products with a handful of columns on one side, fp32 sums of 16-bit tokens and 16-bit or
+// fp32 weights.  With so few columns the tokens' bytes are the bound, so they are read once, in 16 bits, and never widened in memory.
+//   dx: a thread takes eight columns of eight tokens and walks the experts.
+//   dw: a thread takes eight columns of eight experts and walks its CTA's share of the tokens; a second kernel adds the shares in order.
+// The logits themselves stay the library's fp32 product of widened operands: experts of a token can lie within the rounding of a sum of each
+// other, and sums in another order then choose other ones (one token of 4096 in a layer of 8 experts, whose output changes entirely).
+// Forward and backward, us, with library products / with these gradients: 4096 tokens x 2048, 8 experts 147 / 73; 4096 x 4096, 32 experts
+// 257 / 237; 16384 x 4096, 32 experts 662 / 625; 512 x 1024, 8 experts 33 / 29.  With 64 experts the products are work for larger tiles, so 32
+// is the most that comes this way.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -17,7 +18,7 @@ namespace b200 {
 namespace {
 
 constexpr int kE = 8;             // experts of a pass
-constexpr int kTok = 2, kTokDx = 8, kSumGroups = 8;
+constexpr int kTokDx = 8, kSumGroups = 8;
 
 __device__ __forceinline__ void get8(const float* p, float (&v)[8]) {
   const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
@@ -65,35 +66,6 @@ __device__ __forceinline__ void put4(__nv_bfloat16* p, float4 v) {
 __device__ __forceinline__ void put4(__half* p, float4 v) {
   reinterpret_cast<__half2*>(p)[0] = narrow_f16(v.x, v.y);
   reinterpret_cast<__half2*>(p)[1] = narrow_f16(v.z, v.w);
-}
-
-template <typename T, typename W>
-__global__ void __launch_bounds__(128) router_logits_kernel(const T* __restrict__ x, const W* __restrict__ w, float* __restrict__ out, int n, int h, int e_all) {
-  const int lane = threadIdx.x & 31, t0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * kTok, e0 = blockIdx.y * kE;
-  if (t0 >= n) return;
-  float acc[kTok][kE] = {};
-#pragma unroll 2
-  for (int c = lane * 8; c < h; c += 256) {
-    float xv[kTok][8];
-#pragma unroll
-    for (int k = 0; k < kTok; ++k) get8(x + static_cast<int64_t>(min(t0 + k, n - 1)) * h + c, xv[k]);
-#pragma unroll
-    for (int e = 0; e < kE; ++e) {
-      float wv[8];
-      get8(w + static_cast<int64_t>(min(e0 + e, e_all - 1)) * h + c, wv);
-#pragma unroll
-      for (int k = 0; k < kTok; ++k)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) acc[k][e] = fmaf(xv[k][q], wv[q], acc[k][e]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kTok; ++k)
-#pragma unroll
-    for (int e = 0; e < kE; ++e) {
-      const float v = warp_sum(acc[k][e]);
-      if (lane == k * kE + e && t0 + k < n && e0 + e < e_all) out[static_cast<int64_t>(t0 + k) * e_all + e0 + e] = v;
-    }
 }
 
 template <typename T, typename W>
@@ -189,7 +161,6 @@ void run(const RouterArgs& a, cudaStream_t s) {
   const T* x = static_cast<const T*>(a.x);
   const W* w = static_cast<const W*>(a.w);
   const int groups = (a.experts + kE - 1) / kE, octets = (a.h / 8 + 127) / 128;
-  if (a.logits != nullptr) router_logits_kernel<T, W><<<dim3((a.n + 4 * kTok - 1) / (4 * kTok), groups), 128, 0, s>>>(x, w, a.logits, a.n, a.h, a.experts);
   if (a.dx != nullptr) router_dx_kernel<T, W><<<dim3((a.n + kTokDx - 1) / kTokDx, octets), 128, 0, s>>>(a.dlogits, w, static_cast<T*>(a.dx), a.n, a.h, a.experts);
   if (a.dw != nullptr) {
     const int shares = router_shares(a.n), per = (a.n + shares - 1) / shares;
@@ -204,7 +175,7 @@ void run(const RouterArgs& a, cudaStream_t s) {
 // 32 tokens a share until there are 128 shares
 int router_shares(int n) { return n >= 32 * 128 ? 128 : (n + 31) / 32; }
 
-void router_linear(const RouterArgs& a, cudaStream_t s) {
+void router_linear_grad(const RouterArgs& a, cudaStream_t s) {
   if (a.bf16) {
     if (a.w_f32) run<__nv_bfloat16, float>(a, s);
     else run<__nv_bfloat16, __nv_bfloat16>(a, s);

@@ -226,31 +226,35 @@ _ROUTER_EXPERTS = 32           # more output columns are a product for larger ti
 
 
 class _RouterLinear(torch.autograd.Function):
+    """The logits are the library's fp32 product: experts of a token lie within a rounding of each other often enough that sums in another
+    order choose other ones.  The gradients are this framework's kernels; the tokens are kept in 16 bits."""
+
     @staticmethod
     def forward(ctx, x, weight):
         ctx.save_for_backward(x, weight)
-        return ext().router_linear_fwd(x, weight)
+        return torch.nn.functional.linear(x.float(), weight.float())
 
     @staticmethod
     def backward(ctx, dl):
         x, weight = ctx.saved_tensors
+        need_x, need_w = ctx.needs_input_grad
         if torch.is_grad_enabled():                     # a gradient that is differentiated again
             return (dl @ weight.float()).to(x.dtype), (dl.t() @ x.float()).to(weight.dtype)
-        dx, dw = ext().router_linear_bwd(dl.contiguous(), x, weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-        return dx if ctx.needs_input_grad[0] else None, dw if ctx.needs_input_grad[1] else None
+        if not x.is_contiguous() or x.data_ptr() % 16:
+            x = x.clone(memory_format=torch.contiguous_format)
+        dx, dw = ext().router_linear_bwd(dl.contiguous(), x, weight, need_x, need_w)
+        return dx if need_x else None, dw if need_w else None
 
 
 def router_linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """fp32 ``x [..., h] . weight [experts, h]^T`` of 16-bit tokens, summed in fp32."""
     h = x.shape[-1]
-    if (_native(x) and weight.is_cuda and weight.dtype in (x.dtype, torch.float32) and 0 < weight.shape[0] <= _ROUTER_EXPERTS and h % 8 == 0
+    if (_native(x) and torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad) and weight.is_cuda
+            and weight.dtype in (x.dtype, torch.float32) and 0 < weight.shape[0] <= _ROUTER_EXPERTS and h % 8 == 0
             and 0 < h <= 1 << 16 and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and 0 < x.numel() // h < 1 << 28
             and not torch.is_autocast_enabled() and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
             and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()):
-        flat = x.reshape(-1, h)
-        if not flat.is_contiguous() or flat.data_ptr() % 16:
-            flat = flat.clone(memory_format=torch.contiguous_format)
-        return _RouterLinear.apply(flat, weight).view(*x.shape[:-1], weight.shape[0])
+        return _RouterLinear.apply(x.reshape(-1, h), weight).view(*x.shape[:-1], weight.shape[0])
     return torch.nn.functional.linear(x.float(), weight.float())
 
 

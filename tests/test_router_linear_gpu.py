@@ -34,3 +34,17 @@ def test_against_64_bits(n, h, e, dtype, wide):
     plain, = torch.autograd.grad(torch.nn.functional.linear(x.float(), w.float()), x, dl, create_graph=True)
     second, want = (torch.autograd.grad(t.float().square().sum(), w)[0] for t in (again, plain))
     assert torch.allclose(second.float(), want.float(), rtol=2.0 ** -7, atol=2.0 ** -7 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("shape,h,e", [((1,), 264, 4), ((2048, 2), 2048, 8), ((33, 3), 520, 32), ((4100,), 1024, 16)])
+def test_logits_choose_the_experts_of_the_plain_product(shape, h, e):
+    """Two experts of a token can lie closer than fp32 sums in another order leave them, so the logits are the plain product's bits."""
+    from megatronapp_b200.ops import moe
+
+    g = torch.Generator("cuda").manual_seed(h)
+    x = torch.randn(*shape, h, generator=g, device="cuda").bfloat16().requires_grad_()
+    w = (0.02 * torch.randn(e, h, generator=g, device="cuda")).bfloat16().requires_grad_()
+    for a in (x, x.detach().transpose(0, -2).contiguous().transpose(0, -2).requires_grad_()):
+        for grad in (True, False):
+            with torch.set_grad_enabled(grad):
+                assert torch.equal(moe.router_linear(a, w), torch.nn.functional.linear(a.float(), w.float()))
