@@ -165,8 +165,9 @@ void dropout_bwd(const void* dy, const uint8_t* mask, void* dx, int64_t n, float
                  cudaStream_t s);
 void rope_apply(const void* x, const float* cos_sin, void* y, int s, int b, int h, int d,
                 int rot_dim, bool interleaved, bool inverse, bool is_bf16, cudaStream_t st);
-// dbias: fp32 (accumulate: added to), or of dy's type
-void bias_grad_reduce(const void* dy, void* dbias, int64_t rows, int cols, bool is_bf16, bool out_f32, bool accumulate, cudaStream_t s);
+// dbias: fp32 or of dy's type; part: fp32 [bias_grad_parts(rows, cols), cols], nullptr where that is 0
+int bias_grad_parts(int64_t rows, int cols);
+void bias_grad_reduce(const void* dy, void* dbias, float* part, int64_t rows, int cols, bool is_bf16, bool out_f32, cudaStream_t s);
 
 // gradient of an embedding table [vocab, h], zero on entry, from that of n looked-up rows; row i lies at i / inner * st_outer + i % inner * st_inner
 struct EmbeddingGradArgs {

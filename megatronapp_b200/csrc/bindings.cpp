@@ -568,14 +568,18 @@ std::vector<Tensor> router_linear_bwd(const Tensor& dlogits, const Tensor& x, co
   count();
   return {dx, dw};
 }
-void bias_grad(const Tensor& dy, Tensor& dbias, bool accumulate) {
+void bias_grad(const Tensor& dy, Tensor& dbias) {
   c10::cuda::CUDAGuard guard(dy.device());
   const bool f32 = dbias.scalar_type() == at::kFloat;
-  TORCH_CHECK(dy.is_contiguous() && (f32 || (dbias.scalar_type() == dy.scalar_type() && !accumulate)) && dbias.is_contiguous());
+  TORCH_CHECK(dy.is_contiguous() && (f32 || dbias.scalar_type() == dy.scalar_type()) && dbias.is_contiguous());
   const int cols = static_cast<int>(dy.size(-1));
   TORCH_CHECK(cols > 0 && cols % 8 == 0 && dbias.numel() == cols);
-  b200::bias_grad_reduce(dy.data_ptr(), dbias.data_ptr(), dy.numel() / cols, cols, is_bf16(dy), f32, accumulate, cur_stream());
-  count();
+  const int64_t rows = dy.numel() / cols;
+  const int parts = b200::bias_grad_parts(rows, cols);
+  Tensor part;
+  if (parts > 0) part = torch::empty({parts, cols}, dy.options().dtype(at::kFloat));
+  b200::bias_grad_reduce(dy.data_ptr(), dbias.data_ptr(), parts > 0 ? part.data_ptr<float>() : nullptr, rows, cols, is_bf16(dy), f32, cur_stream());
+  count(parts > 0 ? 2 : 1);
 }
 
 std::vector<Tensor> ce_local_stats(const Tensor& logits, const Tensor& labels, int64_t vocab_start) {

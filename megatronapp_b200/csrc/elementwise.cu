@@ -421,6 +421,9 @@ static inline void ln_fast_shape(int cols, int& vpt, int& threads) {
   }
 }
 
+__device__ __forceinline__ void put(float* p, float v) { *p = v; }
+template <typename T> __device__ __forceinline__ void put(T* p, float v) { *p = Cvt<T>::down1(v); }
+
 // column sums of the partials, straight into the parameter's type.  blockIdx.y: gamma or beta; 32 columns x 32 partial rows at a time, all of a
 // thread's loads (10 at 296 partials) in flight together: 768 columns 7.0 -> 2.9 us, and no conversion launches behind it
 template <typename T>
@@ -440,7 +443,7 @@ __global__ void __launch_bounds__(1024) ln_bwd_finalize_kernel(const float* __re
   // warp w sums columns w: lane = partial row
   const float s = warp_sum(sm[tx][ty]);
   const int out = blockIdx.x * 32 + ty;
-  if (tx == 0 && out < cols) (blockIdx.y == 0 ? dgamma : dbeta)[out] = Cvt<T>::down1(s);
+  if (tx == 0 && out < cols) put((blockIdx.y == 0 ? dgamma : dbeta) + out, s);
 }
 
 // ------------------------------------------------------------------ activations
@@ -626,13 +629,14 @@ __global__ void rope_kernel(const T* __restrict__ x, const float* __restrict__ c
   }
 }
 
-// dbias[c] (+)= sum_r dy[r, c].  A CTA sums 64 columns over its share of the rows; where the columns alone leave SMs idle, the CTAs of a cluster
-// share them and the first adds the shares up in order: one launch, the same sums every time (before: a fill, atomic additions, a conversion)
-__device__ __forceinline__ void put(float* p, float v) { *p = v; }
-template <typename T> __device__ __forceinline__ void put(T* p, float v) { *p = Cvt<T>::down1(v); }
+// dbias[c] = sum_r dy[r, c].  A CTA sums 64 columns over its share of the rows.  Up to 512 rows a CTA, the CTAs of a cluster share the rows and the
+// first adds the shares up in order, in one launch; longer shares are cut finer, and a second launch adds them up in order.  us, cluster / two
+// launches / what stood here before both (a fill, atomic additions, a conversion), inputs from HBM where they do not fit L2 eight times:
+//   4096 x 768 4.0 / 4.4 / 8.3     4096 x 4096 9.1 / 10.7 / 9.9    16384 x 768 22 / 8.5 / 12    65536 x 512 77 / 15 / 18
+//   262144 x 256 290 / 25 / 28     4096 x 12288 25 / 18 / 20       65536 x 4096 96 / 81 / 85 (6.6 TB/s)
 template <typename T, typename O>
-__global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ dy, O* __restrict__ dbias, int64_t rows, int cols, int rows_per_cta,
-                                                        bool accumulate) {
+__global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ dy, O* __restrict__ dbias, float* __restrict__ part, int64_t rows, int cols,
+                                                        int rows_per_cta) {
   __shared__ float sm[32][65], total[64];
   const int cv = threadIdx.x & 7;        // 8 vectors of 8 columns = 64 columns per CTA
   const int rl = threadIdx.x >> 3;       // 32 row lanes
@@ -659,6 +663,10 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ dy
     total[threadIdx.x] = t;
   }
   const int c = blockIdx.x * 64 + threadIdx.x;
+  if (part != nullptr) {
+    if (threadIdx.x < 64 && c < cols) part[static_cast<int64_t>(blockIdx.y) * cols + c] = total[threadIdx.x];
+    return;
+  }
   float sum = 0.f;
   if (gridDim.y > 1) {
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -669,10 +677,16 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const T* __restrict__ dy
   } else if (threadIdx.x < 64) {
     sum = total[threadIdx.x];
   }
-  if (blockIdx.y == 0 && threadIdx.x < 64 && c < cols) {
-    if constexpr (sizeof(O) == 4) { if (accumulate) sum += dbias[c]; }
-    put(dbias + c, sum);
-  }
+  if (blockIdx.y == 0 && threadIdx.x < 64 && c < cols) put(dbias + c, sum);
+}
+template <typename O>
+__global__ void __launch_bounds__(128) bias_grad_few_parts_kernel(const float* __restrict__ part, O* __restrict__ dbias, int n, int cols) {
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (c >= cols) return;
+  float v = 0.f;
+#pragma unroll 4
+  for (int i = 0; i < n; ++i) v += part[static_cast<int64_t>(i) * cols + c];
+  put(dbias + c, v);
 }
 
 // ------------------------------------------------------------------ cross entropy
@@ -1030,11 +1044,35 @@ void rope_apply(const void* x, const float* cos_sin, void* y, int s, int b, int 
                            (const T*)x, cos_sin, (T*)y, s, b * h, d, rot_dim, interleaved,
                            inverse ? -1.f : 1.f)));
 }
+// CTAs of a cluster: at least 256 rows each
+static unsigned bias_grad_cluster(int64_t rows, int cols) {
+  unsigned split = 1;
+  while (split < 8 && (cols + 63) / 64 * split < 296 && rows >= 512 * static_cast<int64_t>(split)) split *= 2;
+  return split;
+}
+// six CTAs per SM (all that fit at once) for sums that come from HBM or whose columns alone are many, four for shorter ones: the second launch
+// has fewer parts to add
+static int bias_grad_rows_per_cta(int64_t rows, int cols) {
+  const int64_t col_blocks = (cols + 63) / 64, places = 148 * (rows * cols > int64_t{1} << 25 || col_blocks >= 148 ? 6 : 4);
+  const int64_t split = places > col_blocks ? places / col_blocks : 1, per = (rows + split - 1) / split;
+  return static_cast<int>((per + 31) / 32 * 32);
+}
+int bias_grad_parts(int64_t rows, int cols) {
+  if (rows <= 512 * static_cast<int64_t>(bias_grad_cluster(rows, cols))) return 0;
+  const int per = bias_grad_rows_per_cta(rows, cols);
+  return static_cast<int>((rows + per - 1) / per);
+}
 template <typename T, typename O>
-static void launch_bias_grad(const T* dy, O* dbias, int64_t rows, int cols, bool accumulate, cudaStream_t s) {
+static void launch_bias_grad(const T* dy, O* dbias, float* part, int64_t rows, int cols, cudaStream_t s) {
   const int col_blocks = (cols + 63) / 64;
-  unsigned split = 1;                                    // CTAs of a cluster, at least 256 rows each
-  while (split < 8 && col_blocks * split < 296 && rows >= 512 * static_cast<int64_t>(split)) split *= 2;
+  if (part != nullptr) {
+    const int n = bias_grad_parts(rows, cols);
+    bias_grad_kernel<T, O><<<dim3(col_blocks, n), 256, 0, s>>>(dy, dbias, part, rows, cols, bias_grad_rows_per_cta(rows, cols));
+    if (n <= 4) bias_grad_few_parts_kernel<O><<<(cols + 127) / 128, 128, 0, s>>>(part, dbias, n, cols);
+    else ln_bwd_finalize_kernel<O><<<(cols + 31) / 32, 1024, 0, s>>>(part, nullptr, dbias, nullptr, n, cols);
+    return;
+  }
+  const unsigned split = bias_grad_cluster(rows, cols);
   const int rows_per_cta = static_cast<int>((rows + split - 1) / split);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(col_blocks, split);
@@ -1046,12 +1084,12 @@ static void launch_bias_grad(const T* dy, O* dbias, int64_t rows, int cols, bool
   attr.val.clusterDim.y = split;
   cfg.attrs = &attr;
   cfg.numAttrs = split > 1 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, bias_grad_kernel<T, O>, dy, dbias, rows, cols, rows_per_cta, accumulate);
+  cudaLaunchKernelEx(&cfg, bias_grad_kernel<T, O>, dy, dbias, part, rows, cols, rows_per_cta);
 }
-void bias_grad_reduce(const void* dy, void* dbias, int64_t rows, int cols, bool is_bf16, bool out_f32, bool accumulate, cudaStream_t s) {
+void bias_grad_reduce(const void* dy, void* dbias, float* part, int64_t rows, int cols, bool is_bf16, bool out_f32, cudaStream_t s) {
   DISPATCH_16(is_bf16, {
-    if (out_f32) launch_bias_grad<T, float>((const T*)dy, (float*)dbias, rows, cols, accumulate, s);
-    else launch_bias_grad<T, T>((const T*)dy, (T*)dbias, rows, cols, false, s);
+    if (out_f32) launch_bias_grad<T, float>((const T*)dy, (float*)dbias, part, rows, cols, s);
+    else launch_bias_grad<T, T>((const T*)dy, (T*)dbias, part, rows, cols, s);
   });
 }
 

@@ -202,7 +202,7 @@ def bias_grad(dy2: torch.Tensor, dtype: Optional[torch.dtype] = None) -> torch.T
     if _native(dy2) and dy2.shape[-1] % 8 == 0:
         direct = dtype in (torch.float32, dy2.dtype)
         out = torch.empty(dy2.shape[-1], dtype=dtype if direct else torch.float32, device=dy2.device)
-        ext().bias_grad(dy2.contiguous(), out, False)
+        ext().bias_grad(dy2.contiguous(), out)
         return out if direct else out.to(dtype)
     return dy2.float().sum(dim=0).to(dtype)
 

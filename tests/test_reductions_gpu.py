@@ -35,3 +35,21 @@ def test_norm_parameter_gradients(rows, cols, rms):
         assert a.dtype == torch.bfloat16
         # one rounding to bf16 (7 stored bits: at most 2^-8 of the value), beside fp32 sums
         assert float((a.double() - w).abs().max()) <= 2.0 ** -8 * float(w.abs().max()) + 1e-5 * rows ** 0.5 * 8
+
+
+@pytest.mark.parametrize("rows,cols,launches", [
+    (513, 20000, 2), (4096, 64, 1), (4097, 64, 2), (4128, 72, 2), (70001, 256, 2), (200000, 8, 2), (1024, 12288, 1), (2049, 12288, 2), (5000, 16392, 2)])
+def test_long_bias_grad(rows, cols, launches):
+    """Shares of more than 512 rows are cut finer than a cluster has CTAs, so that few columns do not leave the device idle; remainders of rows
+    and columns around that line."""
+    from megatronapp_b200 import ops
+
+    dy = torch.randn(rows, cols, device="cuda", dtype=torch.bfloat16)
+    want = dy.double().sum(0)
+    for dtype in (torch.float32, torch.bfloat16):
+        before = ops.launch_count()
+        got = ops.bias_grad(dy, dtype)
+        assert ops.launch_count() == before + launches and got.dtype == dtype and torch.equal(got, ops.bias_grad(dy, dtype))
+        # fp32 as above, then one rounding to 16 bits
+        bound = 2.0 ** -24 * rows * 4 + (2.0 ** -8 * want.abs() if dtype is torch.bfloat16 else 0.0)
+        assert bool(((got.double() - want).abs() <= bound).all())
