@@ -79,11 +79,13 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 // its loop converged, on descriptors that advance by constants, and one elected lane issues.
 __device__ __forceinline__ uint64_t desc_at(uint64_t base, uint32_t bytes) { return base + (bytes >> 4); }
 
+// A wait that runs out is noted in `failed`.  At its end the CTA then leaves g_attn_error for attn_status, fills the rows that it owns with NaN
+// and waits (always within kWaitLimit) for its own copies and MMAs in flight.
 constexpr int kWaitLimit = 1 << 20;
 __device__ int g_attn_error = 0;
 // false: the wait ran out here, or another thread of the CTA gave up
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* failed) {
-  for (int i = 0; i < kWaitLimit; ++i) {
+__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatile int* failed, int limit = kWaitLimit) {
+  for (int i = 0; i < limit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255) == 255 && *failed) return false;
   }
@@ -91,8 +93,8 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   return false;
 }
 // the same for a whole warp, which leaves the wait converged
-__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* failed) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, failed));
+__device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* failed, int limit = kWaitLimit) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, failed, limit));
 }
 
 // One warpgroup copies and issues, four do the softmax arithmetic.  A CTA of 640 threads starts with 96 registers each; the math
@@ -115,6 +117,14 @@ __device__ __forceinline__ void store_row32(uint8_t* dst, const uint32_t (&v)[32
     *reinterpret_cast<uint4*>(dst + u * 16) = w;
   }
 }
+// after a wait that ran out, by the math warps: NaN (in either type) in `rows` rows of D columns
+template <int D>
+__device__ __forceinline__ void fill_nan(void* out, int64_t base, int64_t stride, int rows) {
+  constexpr int kChunks = D / 8;
+  for (int i = threadIdx.x - 128; i < rows * kChunks; i += kThreads - 128)
+    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(out) + base + i / kChunks * stride + i % kChunks * 8) =
+        make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+}
 __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
@@ -127,6 +137,7 @@ struct FwdParams {
   int b, hq, hkv, sq, sk;
   float scale_log2;      // softmax scale * log2(e)
   int causal;
+  int wait_limit;        // tries of a wait before it gives up
 };
 
 template <int D>
@@ -170,7 +181,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint64_t* s_full = bars + 9;        // 2 (per q tile); S(j + 1) complete says that PV(j), issued before it, is too
   uint64_t* p_ready = bars + 11;      // 2 (per q tile) x 2: the first and second 32 columns of both halves' P
   uint64_t* o_done = bars + 15;       // 2
-  uint64_t* drained = bars + 17;      // 1, failure path only
+  uint64_t* drained = bars + 17;      // 1, after a wait that ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* failed = reinterpret_cast<volatile int*>(bars + 19);
 
@@ -207,6 +218,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  int nk = 0, nv = 0;                         // thread 0: blocks whose copies it has started
   const uint32_t tmem_S = tmem_base;          // S[t] at col t*128
   const uint32_t tmem_O = tmem_base + 256;    // O[t] at col 256 + t*D
 
@@ -219,26 +231,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int t = 0; t < ntiles; ++t)
         for (int c = 0; c < L::kDC; ++c)
           tma_load_4d(&tmap_q, q_full, sQ + t * L::kTile + c * (kBlockQ * 128), c * 64, h, bi, t == 0 ? q0_0 : q0_1);
-      int nk = 0, nv = 0;
       while (nk < nmax) {
         const int st = nk % kS;
         const uint32_t ph = ((nk / kS) & 1) ^ 1;
-        if (!wait_bar(&k_empty[st], ph, failed)) break;
+        if (!wait_bar(&k_empty[st], ph, failed, p.wait_limit)) break;
         mbar_arrive_expect_tx(&k_full[st], L::kTile);
         for (int c = 0; c < L::kDC; ++c)
           tma_load_4d(&tmap_k, &k_full[st], sK + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, nk * kBlockKV);
         ++nk;
-        if (!wait_bar(&v_empty[st], ph, failed)) break;
+        if (!wait_bar(&v_empty[st], ph, failed, p.wait_limit)) break;
         mbar_arrive_expect_tx(&v_full[st], L::kTile);
         for (int c = 0; c < L::kDC; ++c)
           tma_load_4d(&tmap_v, &v_full[st], sV + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, nv * kBlockKV);
         ++nv;
-      }
-      if (*failed) {                                        // let the copies in flight land before the CTA ends
-        volatile int never = 0;
-        wait_bar(q_full, 0, &never);
-        for (int i = max(0, nk - kS); i < nk; ++i) wait_bar(&k_full[i % kS], (i / kS) & 1, &never);
-        for (int i = max(0, nv - kS); i < nv; ++i) wait_bar(&v_full[i % kS], (i / kS) & 1, &never);
       }
     } else if (warp_idx == 1 && nmax > 0) {
       // ============================================================ MMA issuer
@@ -270,7 +275,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
       };
       auto commit = [&](uint64_t* bar) { if (elect_one()) umma_commit(bar); };
-      bool ok = wait_bar_warp(q_full, 0, failed) && wait_bar_warp(&k_full[0], 0, failed);
+      bool ok = wait_bar_warp(q_full, 0, failed, p.wait_limit) && wait_bar_warp(&k_full[0], 0, failed, p.wait_limit);
       if (ok) {
         tc_fence_after();
         if (nkv_0 > 0) issue_S(0, 0);
@@ -279,16 +284,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       for (int j = 0; j < nmax && ok; ++j) {
         const int nx = (j + 1) % kS;
-        ok = wait_bar_warp(&v_full[j % kS], (j / kS) & 1, failed) && (j + 1 >= nmax || wait_bar_warp(&k_full[nx], ((j + 1) / kS) & 1, failed));
+        ok = wait_bar_warp(&v_full[j % kS], (j / kS) & 1, failed, p.wait_limit) && (j + 1 >= nmax || wait_bar_warp(&k_full[nx], ((j + 1) / kS) & 1, failed, p.wait_limit));
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           const int nt = t == 0 ? nkv_0 : nkv_1;
           if (j >= nt || !ok) continue;
-          ok = wait_bar_warp(&p_ready[t * 2], j & 1, failed);
+          ok = wait_bar_warp(&p_ready[t * 2], j & 1, failed, p.wait_limit);
           if (!ok) continue;
           tc_fence_after();
           issue_PV(t, j, 0);                                // while the second part's weights are made
-          ok = wait_bar_warp(&p_ready[t * 2 + 1], j & 1, failed);
+          ok = wait_bar_warp(&p_ready[t * 2 + 1], j & 1, failed, p.wait_limit);
           if (!ok) continue;
           tc_fence_after();
           issue_PV(t, j, 1);
@@ -298,11 +303,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (!ok) break;
         commit(&v_empty[j % kS]);
         if (j + 1 < nmax) commit(&k_empty[nx]);
-      }
-      if (!ok) {                                            // the MMAs in flight finish before TMEM is freed
-        volatile int never = 0;
-        commit(drained);
-        wait_bar_warp(drained, 0, &never);
       }
     }
   } else {
@@ -387,7 +387,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // a wait that runs out is noted, not acted on: the halves' warpgroups go on to their exchanges together, and every later wait ends at once
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      wait_bar(&s_full[t], j & 1, failed);
+      wait_bar(&s_full[t], j & 1, failed, p.wait_limit);
       __syncwarp();
       tc_fence_after();
       const int kbase = j * kBlockKV;
@@ -397,7 +397,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       else block(j, std::false_type{});
     }
     if (n > 0) {
-      ok = wait_bar_warp(&o_done[t], 0, failed);
+      ok = wait_bar_warp(&o_done[t], 0, failed, p.wait_limit);
       tc_fence_after();
       float la, lb;
       un2(l2, la, lb);
@@ -423,7 +423,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *failed) atomicExch(&g_attn_error, 1);
+  if (*failed) {                                  // every wait is over, so all threads read the same
+    volatile int never = 0;
+    if (threadIdx.x == 0) {
+      atomicExch(&g_attn_error, 1);
+      wait_bar(q_full, 0, &never);
+      for (int i = max(0, nk - kS); i < nk; ++i) wait_bar(&k_full[i % kS], (i / kS) & 1, &never);
+      for (int i = max(0, nv - kS); i < nv; ++i) wait_bar(&v_full[i % kS], (i / kS) & 1, &never);
+    } else if (warp_idx == 1) {
+      if (elect_one()) umma_commit(drained);
+      wait_bar_warp(drained, 0, &never);
+    } else if (warp_idx >= 4) {
+      const int rows = min(2 * kBlockQ, p.sq - q0_0);
+      fill_nan<D>(p.o, static_cast<int64_t>(q0_0) * p.o_ss + static_cast<int64_t>(bi) * p.o_sb + static_cast<int64_t>(h) * p.o_sh, p.o_ss, rows);
+      for (int i = threadIdx.x - 128; i < rows; i += kThreads - 128)
+        p.lse[(static_cast<int64_t>(bi) * p.hq + h) * p.sq + q0_0 + i] = __int_as_float(0x7fffffff);
+    }
+    __syncthreads();
+  }
   if (warp_idx == 2) tmem_dealloc<512>(tmem_base);
 }
 
@@ -485,6 +502,7 @@ struct BwdParams {
   int b, hq, hkv, sq, sk;
   float scale_log2, scale;
   int causal;
+  int wait_limit;       // tries of a wait before it gives up
 };
 
 constexpr int kBwdRows = 128;   // resident rows per CTA (keys for dK/dV, queries for dQ)
@@ -532,7 +550,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   uint64_t* t_full = bars + 1 + 2 * kS;  // 2
   uint64_t* pds_ready = t_full + 2;      // 2
   uint64_t* acc_done = pds_ready + 2;    // 1
-  uint64_t* drained = acc_done + 1;      // 1, failure path only
+  uint64_t* drained = acc_done + 1;      // 1, after a wait that ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   volatile int* failed = reinterpret_cast<volatile int*>(bars + 25);
 
@@ -575,6 +593,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  int n_loaded = 0;                            // thread 0: blocks whose copies it has started
   const uint32_t tmem_T1 = tmem_base;          // T1[buf] at col buf*64: P overwrites the first half of each 32 cols
   const uint32_t tmem_T2 = tmem_base + 128;    // T2[buf] at col 128 + buf*64: so does dS
   const uint32_t tmem_A1 = tmem_base + 256;    // dV or dQ
@@ -589,12 +608,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
         tma_load_4d(&tmap_x1, x_full, sX1 + c * (kBwdRows * 128), c * 64, out_head, bi, r0);
         tma_load_4d(&tmap_x2, x_full, sX2 + c * (kBwdRows * 128), c * 64, out_head, bi, r0);
       }
-      int it = 0;
-      for (; it < n_iter; ++it) {
-        const int ys = it % kS;
+      for (; n_loaded < n_iter; ++n_loaded) {
+        const int it = n_loaded, ys = it % kS;
         const int head = kDQ ? out_head / G : head0 + it / n_col;   // head of the streamed tiles
         const int c0 = (col_blk0 + it % n_col) * kBwdCols;
-        if (!wait_bar(&y_empty[ys], ((it / kS) & 1) ^ 1, failed)) break;
+        if (!wait_bar(&y_empty[ys], ((it / kS) & 1) ^ 1, failed, p.wait_limit)) break;
         mbar_arrive_expect_tx(&y_full[ys], 2 * L::kY + (kDQ ? 0 : 512));
         uint8_t* y1 = sY + ys * 2 * L::kY;
         uint8_t* y2 = y1 + L::kY;
@@ -607,11 +625,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
           bulk_load_1d(sStat + ys * 128, p.nlse + base, 256, &y_full[ys]);
           bulk_load_1d(sStat + ys * 128 + 64, p.ndelta + base, 256, &y_full[ys]);
         }
-      }
-      if (*failed) {                                        // let the copies in flight land before the CTA ends
-        volatile int never = 0;
-        wait_bar(x_full, 0, &never);
-        for (int i = max(0, it - kS); i < it; ++i) wait_bar(&y_full[i % kS], (i / kS) & 1, &never);
       }
     } else if (warp_idx == 1 && n_iter > 0) {
       // ============================================================ MMA issuer
@@ -636,7 +649,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
           umma_commit(&t_full[it & 1]);
         }
       };
-      bool ok = wait_bar_warp(x_full, 0, failed) && wait_bar_warp(&y_full[0], 0, failed);
+      bool ok = wait_bar_warp(x_full, 0, failed, p.wait_limit) && wait_bar_warp(&y_full[0], 0, failed, p.wait_limit);
       if (ok) {
         tc_fence_after();
         issue_T(0);
@@ -644,12 +657,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
       for (int it = 0; it < n_iter && ok; ++it) {
         const int ys = it % kS, tb = it & 1;
         if (it + 1 < n_iter) {
-          ok = wait_bar_warp(&y_full[(it + 1) % kS], ((it + 1) / kS) & 1, failed);
+          ok = wait_bar_warp(&y_full[(it + 1) % kS], ((it + 1) / kS) & 1, failed, p.wait_limit);
           if (!ok) break;
           tc_fence_after();
           issue_T(it + 1);     // overwrites T[(it+1)&1]: its P/dS were consumed by the accumulate MMAs of it-1
         }
-        ok = wait_bar_warp(&pds_ready[tb], (it >> 1) & 1, failed);
+        ok = wait_bar_warp(&pds_ready[tb], (it >> 1) & 1, failed, p.wait_limit);
         if (!ok) break;
         tc_fence_after();
         const uint64_t y1 = desc_at(yn_desc, ys * 2 * L::kY);
@@ -669,13 +682,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
           umma_commit(&y_empty[ys]);
         }
       }
-      if (ok) {
-        commit(acc_done);
-      } else {                                              // the MMAs in flight finish before TMEM is freed
-        volatile int never = 0;
-        commit(drained);
-        wait_bar_warp(drained, 0, &never);
-      }
+      if (ok) commit(acc_done);
     }
   } else {
     // ============================================================ P / dS math + epilogue
@@ -744,7 +751,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
     bool ok = true;
     for (int it = tb; it < n_iter; it += 2) {
       const int c0 = (col_blk0 + it % n_col) * kBwdCols;
-      ok = wait_bar_warp(&t_full[tb], (it >> 1) & 1, failed);
+      ok = wait_bar_warp(&t_full[tb], (it >> 1) & 1, failed, p.wait_limit);
       if (!ok) break;
       tc_fence_after();
       // masking: key index > query index is masked (causal); also ragged tails
@@ -754,7 +761,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
       if (need_mask) block(it, c0, std::true_type{});
       else block(it, c0, std::false_type{});
     }
-    if (n_iter > 0 && ok) ok = wait_bar_warp(acc_done, 0, failed);
+    if (n_iter > 0 && ok) ok = wait_bar_warp(acc_done, 0, failed, p.wait_limit);
     if (ok) {
       tc_fence_after();
       const int limit = kDQ ? p.sq : p.sk;
@@ -782,7 +789,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *failed) atomicExch(&g_attn_error, 1);
+  if (*failed) {                                  // every wait is over, so all threads read the same
+    volatile int never = 0;
+    if (threadIdx.x == 0) {
+      atomicExch(&g_attn_error, 1);
+      wait_bar(x_full, 0, &never);
+      for (int i = max(0, n_loaded - kS); i < n_loaded; ++i) wait_bar(&y_full[i % kS], (i / kS) & 1, &never);
+    } else if (warp_idx == 1) {
+      if (elect_one()) umma_commit(drained);
+      wait_bar_warp(drained, 0, &never);
+    } else if (warp_idx >= 4) {
+      const int rows = min(kBwdRows, (kDQ ? p.sq : p.sk) - r0);
+      fill_nan<D>(p.out1, static_cast<int64_t>(r0) * p.o1_ss + static_cast<int64_t>(bi) * p.o1_sb + static_cast<int64_t>(out_head) * p.o1_sh, p.o1_ss, rows);
+      if (!kDQ)
+        fill_nan<D>(p.out2, static_cast<int64_t>(r0) * p.o2_ss + static_cast<int64_t>(bi) * p.o2_sb + static_cast<int64_t>(out_head) * p.o2_sh, p.o2_ss, rows);
+    }
+    __syncthreads();
+  }
   if (warp_idx == 2) tmem_dealloc<512>(tmem_base);
 }
 
@@ -856,7 +879,7 @@ int launch_fwd(const AttnArgs& a, cudaStream_t s) {
   FwdParams p{};
   p.lse = a.lse; p.o = a.o; p.o_sb = a.o_sb; p.o_sh = a.o_sh; p.o_ss = a.o_ss;
   p.b = a.b; p.hq = a.hq; p.hkv = a.hkv; p.sq = a.sq; p.sk = a.sk;
-  p.scale_log2 = a.scale * kLog2e; p.causal = a.causal ? 1 : 0;
+  p.scale_log2 = a.scale * kLog2e; p.causal = a.causal ? 1 : 0; p.wait_limit = a.wait_limit < 0 ? kWaitLimit : a.wait_limit;
   const int64_t ctas = static_cast<int64_t>((a.sq + 2 * kBlockQ - 1) / (2 * kBlockQ)) * a.hq * a.b;
   if (ctas > 0x7fffffff) { g_attn_err = "too many query blocks"; return -12; }
   kern<<<static_cast<unsigned>(ctas), kThreads, L::kTotal, s>>>(tq, tk, tv, p);
@@ -895,7 +918,7 @@ int launch_bwd_one(const AttnArgs& a, cudaStream_t s) {
     p.out2 = a.dk; p.o2_sb = a.dk_sb; p.o2_sh = a.dk_sh; p.o2_ss = a.dk_ss;
   }
   p.b = a.b; p.hq = a.hq; p.hkv = a.hkv; p.sq = a.sq; p.sk = a.sk;
-  p.scale_log2 = a.scale * kLog2e; p.scale = a.scale; p.causal = a.causal ? 1 : 0;
+  p.scale_log2 = a.scale * kLog2e; p.scale = a.scale; p.causal = a.causal ? 1 : 0; p.wait_limit = a.wait_limit < 0 ? kWaitLimit : a.wait_limit;
   const int64_t ctas = static_cast<int64_t>(((kDQ ? a.sq : a.sk) + kBwdRows - 1) / kBwdRows) * (kDQ ? a.hq : a.hkv) * a.b;
   if (ctas > 0x7fffffff) { g_attn_err = "too many row blocks"; return -12; }
   kern<<<static_cast<unsigned>(ctas), kThreads, L::kTotal, s>>>(x1, x2, y1, y2, p);
@@ -920,6 +943,14 @@ int launch_bwd(const AttnArgs& a, cudaStream_t s) {
 }  // namespace
 
 const char* attn_last_error() { return g_attn_err.c_str(); }
+
+int attn_status(bool clear) {
+  int v = 0;
+  const int zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_attn_error, sizeof(int)) != cudaSuccess) return -1;
+  if (clear && v != 0 && cudaMemcpyToSymbol(g_attn_error, &zero, sizeof(int)) != cudaSuccess) return -1;
+  return v;
+}
 
 int attn_fwd(const AttnArgs& a, cudaStream_t s) {
   if (a.d != 64 && a.d != 128) { g_attn_err = "head dim must be 64 or 128"; return -1; }

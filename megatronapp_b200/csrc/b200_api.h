@@ -241,12 +241,14 @@ struct AttnArgs {
   bool is_bf16;
   void* probs_out;  // optional MegaScope export [b,hq,sq,sk] (fwd only)
   int64_t q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_sb, o_sh, o_ss;
+  int wait_limit = -1;  // tries of a wait inside the kernels before it gives up (tests); below 0: the kernels' own limit
   int64_t do_sb, do_sh, do_ss, dq_sb, dq_sh, dq_ss, dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
 };
 int attn_fwd(const AttnArgs& a, cudaStream_t s);
 int attn_bwd(const AttnArgs& a, cudaStream_t s);
 const char* attn_last_error();
 
+int attn_status(bool clear);   // 1: a kernel of this process gave up on a wait (its rows are NaN); synchronises
 // causal attention with logistic weights over packed prompts (tcgen05)
 struct SigAttnArgs {
   const void *q, *k, *v;   // [T, H, d], [T, G, d], [T, G, d] contiguous, padded with zeros to d = 64 or 128

@@ -726,7 +726,7 @@ void check_bhsd(const Tensor& t, const char* name) {
 }  // namespace
 // q/k/v: strided logical [b,h,s,d] views (e.g. permuted [s,b,h,d] activations).  The output is
 // allocated [s,b,h,d]-contiguous and returned as its [b,h,s,d] view.
-std::vector<Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal, bool want_probs) {
+std::vector<Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal, bool want_probs, int wait_limit) {
   c10::cuda::CUDAGuard guard(q.device());
   check_bhsd(q, "q"); check_bhsd(k, "k"); check_bhsd(v, "v");
   b200::AttnArgs a{};
@@ -743,6 +743,7 @@ std::vector<Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, 
   a.o_sb = o.stride(0); a.o_sh = o.stride(1); a.o_ss = o.stride(2);
   a.scale = static_cast<float>(scale); a.causal = causal; a.is_bf16 = is_bf16(q);
   a.probs_out = want_probs ? reinterpret_cast<void*>(1) : nullptr;
+  a.wait_limit = wait_limit;
   int rc = b200::attn_fwd(a, cur_stream());
   TORCH_CHECK(rc == 0, "b200 attn_fwd failed: ", rc, " ", b200::attn_last_error());
   count();
@@ -810,7 +811,7 @@ void window_attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 }
 std::vector<Tensor> attn_bwd(const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o,
                              const Tensor& lse, double scale, bool causal, const c10::optional<Tensor>& dq_out,
-                             const c10::optional<Tensor>& dk_out, const c10::optional<Tensor>& dv_out) {
+                             const c10::optional<Tensor>& dk_out, const c10::optional<Tensor>& dv_out, int wait_limit) {
   c10::cuda::CUDAGuard guard(q.device());
   check_bhsd(q, "q"); check_bhsd(k, "k"); check_bhsd(v, "v"); check_bhsd(o, "o");
   b200::AttnArgs a{};
@@ -836,6 +837,7 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o, const Tensor& q, const Tensor& k
   a.dk_sb = dk.stride(0); a.dk_sh = dk.stride(1); a.dk_ss = dk.stride(2);
   a.dv_sb = dv.stride(0); a.dv_sh = dv.stride(1); a.dv_ss = dv.stride(2);
   a.scale = static_cast<float>(scale); a.causal = causal; a.is_bf16 = is_bf16(q);
+  a.wait_limit = wait_limit;
   int rc = b200::attn_bwd(a, cur_stream());
   TORCH_CHECK(rc == 0, "b200 attn_bwd failed: ", rc, " ", b200::attn_last_error());
   count(3);
@@ -1156,12 +1158,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("add_into_f32", &add_into_f32);
   m.def("check_finite", &check_finite);
   m.def("chunk_mean", &chunk_mean);
-  m.def("attn_fwd", &attn_fwd);
+  m.def("attn_fwd", [](const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal, bool want_probs) {
+    return attn_fwd(q, k, v, scale, causal, want_probs, -1);
+  });
+  m.def("attn_fwd_limited", &attn_fwd);      // with the tries of a wait inside the kernel before it gives up
   m.def("sigmoid_attn_fwd", &sigmoid_attn_fwd);
   m.def("sigmoid_attn_status", []() { return b200::sigmoid_attn_status(); });
   m.def("window_attn_fwd", &window_attn_fwd);
   m.def("window_attn_status", []() { return b200::window_attn_status(); });
-  m.def("attn_bwd", &attn_bwd);
+  m.def("attn_bwd", [](const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, double scale, bool causal,
+                       const c10::optional<Tensor>& dq, const c10::optional<Tensor>& dk, const c10::optional<Tensor>& dv) {
+    return attn_bwd(d_o, q, k, v, o, lse, scale, causal, dq, dk, dv, -1);
+  });
+  m.def("attn_bwd_limited", &attn_bwd);
+  m.def("attn_status", [](bool clear) { return b200::attn_status(clear); }, py::arg("clear") = false);
   m.def("arena_alloc", &arena_alloc);
   m.def("arena_open", &arena_open);
   m.def("arena_close", &arena_close);

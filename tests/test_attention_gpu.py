@@ -5,6 +5,14 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def _no_wait_ran_out():
+    from megatronapp_b200 import ops
+
+    yield
+    assert ops.ext().attn_status() == 0
+
+
 def _oracle(q, k, v, scale, causal, do):
     rep = q.shape[1] // k.shape[1]
     q, k, v = (t.detach().double().requires_grad_() for t in (q, k, v))
@@ -65,3 +73,28 @@ def test_forward_tiles(b, hq, hkv, sq, sk, d, causal, dtype):
     k[::97] *= 6
     q, k, v = (t.to(dtype).permute(1, 2, 0, 3) for t in (q, k, v))
     _close([ops.attention(q, k, v, d ** -0.5, causal)], _oracle(q, k, v, d ** -0.5, causal, None), dtype)
+
+
+@pytest.mark.parametrize("sq,sk,d,causal", [(300, 300, 128, True), (64, 64, 64, True), (256, 640, 64, False)])
+def test_a_wait_that_runs_out_shows(sq, sk, d, causal):
+    """Waits that give up at once: the kernel ends by itself, its rows are NaN and the status says so; the next call is sound again."""
+    from megatronapp_b200 import ops
+
+    ext = ops.ext()
+    assert ext.attn_status() == 0
+    g = torch.Generator("cuda").manual_seed(3)
+    q, k, v = (torch.randn(s, 2, 4, d, generator=g, device="cuda").bfloat16().permute(1, 2, 0, 3) for s in (sq, sk, sk))
+    scale = d ** -0.5
+    o, lse, _ = ext.attn_fwd_limited(q, k, v, scale, causal, False, 0)
+    assert ext.attn_status() == 1 and ext.attn_status(True) == 1 and ext.attn_status() == 0
+    assert torch.isnan(o).all() and torch.isnan(lse).all()
+    o, lse, _ = ext.attn_fwd(q, k, v, scale, causal, False)
+    _close([o], _oracle(q, k, v, scale, causal, None), torch.bfloat16)
+    if sq % 64 == 0:
+        do = torch.randn(sq, 2, 4, d, generator=g, device="cuda").bfloat16().permute(1, 2, 0, 3)
+        for t in ext.attn_bwd_limited(do, q, k, v, o, lse, scale, causal, None, None, None, 0):
+            assert torch.isnan(t).all()
+        assert ext.attn_status(True) == 1
+        got = ext.attn_bwd(do, q, k, v, o, lse, scale, causal, None, None, None)
+        _close(got, _oracle(q, k, v, scale, causal, do)[1:], torch.bfloat16)
+    assert ext.attn_status() == 0
