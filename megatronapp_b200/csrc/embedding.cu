@@ -6,7 +6,8 @@
 //   sum:   a CTA takes 16 places and all columns of a slice, every row's address known from the start.  Runs of one id inside the tile are
 //     summed in fp32 and stored; what continues into a neighbouring tile is left as a partial sum.
 //   merge: a CTA whose tile holds the beginning of such a run adds the following tiles' parts to it.
-// Quadratic in the tokens, so it ends at 16384 (about 20 us); beyond that a radix sort is the better way and PyTorch's is used.
+// Quadratic in the tokens, so it ends at 16384 (100 us with a table of 50304 x 768, 25 of them its zeros); beyond that a radix sort is the better
+// way and PyTorch's is used, as it is for up to 2048 tokens, for which it needs no sort.
 // 4096 tokens, 50304 x 768 and 1024 x 768: the two gradients took some 40 launches and 240 us with PyTorch's sort.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

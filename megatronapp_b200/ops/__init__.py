@@ -211,7 +211,11 @@ def bias_grad(dy2: torch.Tensor, dtype: Optional[torch.dtype] = None) -> torch.T
 # embedding lookup
 # ---------------------------------------------------------------------------
 
-_EMBED_TOKENS = 16384          # the kernels' work is quadratic in the tokens; beyond, PyTorch's radix sort costs less
+# Up to 3072 tokens PyTorch takes one launch of its own and no sort, above a radix sort of some twenty launches; the kernels' work is quadratic in
+# the tokens, and three launches behind a Python node cost the host more than one.  us of a call alone here / there, tables of 50304 x 768 and
+# 1024 x 768: 64 tokens 86 / 58 and 88 / 64; 2048 86 / 114 and 86 / 68; 3072 87 / 161 and 86 / 95; 4096 86 / 210 and 87 / 156; 16384 113 / 361
+# and 94 / 177
+_EMBED_FROM, _EMBED_TO = 2049, 16384
 
 
 class _EmbeddingFn(torch.autograd.Function):
@@ -234,7 +238,7 @@ class _EmbeddingFn(torch.autograd.Function):
 def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """Rows ``ids`` of ``weight``; the dense gradient of a 16-bit table comes from kernels that sum in fp32 and a fixed order."""
     if (_native(weight) and weight.requires_grad and torch.is_grad_enabled() and ids.is_cuda and ids.dim() in (1, 2) and weight.dim() == 2
-            and 0 < ids.numel() <= _EMBED_TOKENS and weight.shape[1] % 8 == 0 and 0 < weight.shape[1] < 1 << 24 and 0 < weight.shape[0] <= 0x7fffffff
+            and _EMBED_FROM <= ids.numel() <= _EMBED_TO and weight.shape[1] % 8 == 0 and 0 < weight.shape[1] < 1 << 24 and 0 < weight.shape[0] <= 0x7fffffff
             and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
             and not torch.jit.is_tracing() and not torch.compiler.is_compiling()):
         return _EmbeddingFn.apply(ids, weight)

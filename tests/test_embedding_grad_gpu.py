@@ -5,6 +5,13 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture
+def kernels_for_all_lengths(monkeypatch):
+    from megatronapp_b200 import ops
+
+    monkeypatch.setattr(ops, "_EMBED_FROM", 1)
+
+
 def _ids(kind, n, vocab, g):
     if kind == "same":
         return torch.full((n,), vocab - 1)
@@ -16,7 +23,7 @@ def _ids(kind, n, vocab, g):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("kind", ["spread", "few", "same"])
 @pytest.mark.parametrize("n,h,vocab", [(1, 8, 1), (15, 768, 40), (16, 1032, 7), (17, 64, 5), (96, 256, 50304), (4100, 768, 1024), (16384, 264, 512)])
-def test_against_64_bits(n, h, vocab, kind, dtype):
+def test_against_64_bits(n, h, vocab, kind, dtype, kernels_for_all_lengths):
     from megatronapp_b200 import ops
 
     vocab = max(vocab, 3) if kind == "few" else vocab
@@ -36,7 +43,7 @@ def test_against_64_bits(n, h, vocab, kind, dtype):
     assert torch.equal(again, w.grad)
 
 
-def test_layouts_and_other_ways_of_differentiating():
+def test_layouts_and_other_ways_of_differentiating(kernels_for_all_lengths):
     from megatronapp_b200 import ops
 
     g = torch.Generator().manual_seed(3)
@@ -62,3 +69,13 @@ def test_layouts_and_other_ways_of_differentiating():
     assert torch.equal(dw, own)
     assert torch.equal(torch.autograd.grad(dw, v, torch.ones_like(dw))[0], torch.ones_like(v))
     assert torch.equal(torch.func.vjp(lambda t: ops.embedding(ids, t), w.detach())[1](v.detach())[0], own)
+
+
+@pytest.mark.parametrize("n,own", [(1, False), (64, False), (2048, False), (2049, True), (16384, True), (16385, False)])
+def test_lengths_that_come_this_way(n, own):
+    """Few tokens need no sort, and PyTorch's one launch beats three and a Python node."""
+    from megatronapp_b200 import ops
+
+    w = torch.zeros(64, 8, dtype=torch.bfloat16, device="cuda", requires_grad=True)
+    out = ops.embedding(torch.zeros(n, dtype=torch.long, device="cuda"), w)
+    assert out.grad_fn.name().startswith("_EmbeddingFn" if own else "EmbeddingBackward")
