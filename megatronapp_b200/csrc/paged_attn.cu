@@ -25,6 +25,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <cmath>
 #include <string>
 
 #include "b200_api.h"
@@ -96,6 +97,7 @@ struct PagedParams {
   int n_tiles;                 // chunks: tiles of this launch (its grid is n_tiles * ng * splits); decode: requests
   int splits;                  // chunks: key ranges of a tile; decode: CTAs, or 0 for one per (request, KV head)
   bool beside_chunks;          // decode: the launch before is the chunks'
+  uint32_t q_keep, q_sign;     // the kernels' running maxima want a positive scale: queries are negated for a negative one, zeros for zero
   float* ws;                   // decode: two partials of 16 rows x (d + 2) per CTA
 };
 
@@ -148,8 +150,8 @@ struct Tile {
                                                              (static_cast<int64_t>(t) * np + hk * G + (valid ? row & (G - 1) : 0)) * D) + tg;
 #pragma unroll
       for (int k = 0; k < D / 16; ++k) {
-        qf[k][i] = valid ? qp[k * 8] : 0u;
-        qf[k][i + 2] = valid ? qp[k * 8 + 4] : 0u;
+        qf[k][i] = valid ? (qp[k * 8] & p.q_keep) ^ p.q_sign : 0u;
+        qf[k][i + 2] = valid ? (qp[k * 8 + 4] & p.q_keep) ^ p.q_sign : 0u;
       }
     }
     m[0] = m[1] = -INFINITY;
@@ -213,15 +215,15 @@ struct Tile {
         for (int j = 0; j < kNT; ++j) mx = fmaxf(mx, fmaxf(s[j][2 * i], s[j][2 * i + 1]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float mn = fmaxf(m[i], mx * sc);
+        const float mn = fmaxf(m[i], mx);                            // unscaled: the largest score's weight is one whatever its size
         const float use = mn == -INFINITY ? 0.f : mn;                // nothing visible yet: keep the arithmetic finite
-        const float corr = exp2f(m[i] - use);
+        const float corr = exp2f((m[i] - use) * sc);
         m[i] = mn;
         float sum = 0.f;
 #pragma unroll
         for (int j = 0; j < kNT; ++j) {
-          s[j][2 * i] = exp2f(fmaf(s[j][2 * i], sc, -use));
-          s[j][2 * i + 1] = exp2f(fmaf(s[j][2 * i + 1], sc, -use));
+          s[j][2 * i] = exp2f((s[j][2 * i] - use) * sc);
+          s[j][2 * i + 1] = exp2f((s[j][2 * i + 1] - use) * sc);
           sum += s[j][2 * i] + s[j][2 * i + 1];
         }
         l[i] = l[i] * corr + sum;                                    // this thread's columns; the quad's are added at the end
@@ -298,10 +300,11 @@ struct Tile {
 
 // running sum of weighted partials; no keys: zeros
 struct Merge {
-  float M = -INFINITY, L = 0.f;
+  float sc, M = -INFINITY, L = 0.f;
   float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+  __device__ __forceinline__ explicit Merge(float scale_log2) : sc(scale_log2) {}
   __device__ __forceinline__ void add(float m, float l, const float4& v) {
-    const float f = exp2f(m - M);
+    const float f = exp2f((m - M) * sc);
     L = fmaf(l, f, L);
     if (l > 0.f) {
       O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
@@ -423,7 +426,7 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     float* ws = p.ws + (static_cast<int64_t>(blockIdx.x) * 2 + (st0 == 0 ? 1 : 0)) * (16 * (D + 2));
     for (int idx = tid; idx < (it.n << p.group_shift) * (D / 4); idx += 128) {
       const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
-      Merge x;
+      Merge x(a.scale_log2);
 #pragma unroll
       for (int w = 0; w < 4; ++w) x.M = fmaxf(x.M, s_m[w * 16 + row]);
       if (x.M > -INFINITY) {
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(512) paged_merge_kernel(const PagedParams p) {
     M = warp_max(M);
     const float use = M == -INFINITY ? 0.f : M;
     for (int i = lane; i < parts; i += 32) {
-      const float f = exp2f(s_f[row][i] - use), l = slot(i0 + i)[16 * D + 16 + row];
+      const float f = exp2f((s_f[row][i] - use) * a.scale_log2), l = slot(i0 + i)[16 * D + 16 + row];
       s_f[row][i] = l > 0.f ? f : 0.f;
       L = fmaf(l, f, L);
     }
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
   cluster.sync();
   for (int idx = rank * 128 + tid; idx < n_rows * (D / 4); idx += p.splits * 128) {
     const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
-    Merge x;
+    Merge x(a.scale_log2);
     for (int c = 0; c < p.splits; ++c) x.M = fmaxf(x.M, *cluster.map_shared_rank(s_m + row, c));
     if (x.M > -INFINITY) {
       for (int c = 0; c < p.splits; ++c)
@@ -719,6 +722,9 @@ void paged_write(const PagedWriteArgs& w, cudaStream_t s) {
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s) {
   PagedParams p{};
   p.a = a;
+  p.a.scale_log2 = a.scale_log2 == 0.f ? 1.f : fabsf(a.scale_log2);
+  p.q_keep = a.scale_log2 == 0.f ? 0u : 0xffffffffu;
+  p.q_sign = a.scale_log2 < 0.f ? 0x80008000u : 0u;
   p.group_shift = log2_exact(a.group);
   p.bs_shift = log2_exact(a.block_size);
   if (a.cu != nullptr && chunk_tiles > 0) {

@@ -87,3 +87,43 @@ def test_key_ranges():
         for n in (1, 255, 512, 1000, 4096, 100000):
             r = key_ranges(tiles, n)
             assert r in (1, 2, 4, 8, 16) and (r == 1 or n >= 256 * r)
+
+
+def _four_keys(dtype, scores, values, d=64):
+    """One decoding request that sees four keys; ``scores [heads][4]`` lie along the first axis (the query is one there), ``values [4, heads]``
+    in every column."""
+    heads = len(scores)
+    cx, q, k, v = _step([(3, 1)], heads, heads, d, 16, dtype)
+    q.zero_()
+    q[:, :, 0] = 1
+    kk, vv = torch.zeros(4, heads, d, device="cuda", dtype=dtype), torch.zeros(4, heads, d, device="cuda", dtype=dtype)
+    kk[:, :, 0] = torch.tensor(scores, device="cuda").t().to(dtype)
+    vv[:] = values.to(dtype).unsqueeze(-1)
+    kc, vc = cx.kv[1]
+    slots = torch.tensor(cx.seqs["0"].blocks[0] * 16) + torch.arange(4)
+    kc[slots.cuda()], vc[slots.cuda()] = kk, vv
+    return cx, q, kk[3:], vv[3:], kk[..., 0].double()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reqs", [[(500, 1)], [(5000, 1), (3, 1)], [(300, 70)], [(2000, 40)]])
+@pytest.mark.parametrize("dtype,scale", [(torch.float16, -1.0), (torch.bfloat16, -0.5), (torch.float16, 0.0), (torch.bfloat16, 0.0)])
+def test_scales_that_are_not_positive(reqs, dtype, scale):
+    cx, q, k, v = _step(reqs, 4, 2, 64, 16, dtype)
+    want, _, _ = _oracle(cx, reqs, q, k, v, scale, 16)
+    got = cx.attend(1, q, k, v, scale).double()
+    unit = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+    # scores of up to 50: their own fp32 rounding moves a weight by 2^-18
+    assert float((got - want).abs().max()) <= unit * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,size", [(torch.float16, 30000.0), (torch.bfloat16, 1e6)])
+def test_scores_beyond_the_exponent(dtype, size):
+    """Scores so large that one unit of their rounding is more than any weight can hold: the largest key has all the weight."""
+    scores = [[0.25, -0.5, 0.5, 0.125], [0.0, 0.0, -1.0, -1.0], [-0.5, -0.25, -0.25, -1.0]]
+    val = torch.arange(12, device="cuda").view(4, 3) + 1.0
+    cx, q, k, v, s = _four_keys(dtype, [[x * size for x in r] for r in scores], val)
+    q *= size
+    got = cx.attend(1, q, k, v, 64.0)[0, :, 0].double().cpu()
+    assert torch.equal(got, torch.tensor([7.0, (2 + 5) / 2, (6 + 9) / 2], dtype=torch.float64))
