@@ -8,8 +8,8 @@
 // A tile is up to 16 or 64 rows, a row being one (token, query head) of one request and one KV head: all query heads of a group share
 // every key/value row that is read, and so do the tokens of a chunk.  Keys come in stages of 64, gathered page by page into a ring of
 // shared-memory buffers by 16-byte asynchronous copies (32 KB each at d = 128), and are
-// multiplied by m16n8k16 tensor instructions from there.  The weights stay exact to about 16 bits: each enters the value product as a 16-bit
-// part and the rest of it, so the result carries fp32 sums of fp32 weights as far as its 16-bit output can show.
+// multiplied by m16n8k16 tensor instructions from there.  The weights are fp32: each enters the value product as three 16-bit parts that add
+// up to it (fp16: to 2^-40 of the largest weight where it is below 2^-16 of that).
 //   rows = 16 (decode, short chunks): the four warps take 16 keys of a stage each, bound by HBM.  The stages of all (request, KV head)
 //     pairs stand in one line that is cut evenly over three CTAs per SM, whatever the contexts' lengths; an item that a cut falls into
 //     leaves partial (max, sum, accumulator) triples, which a small second kernel merges.  64 contexts of 1k to 4k, 32 / 8 heads of 128:
@@ -106,13 +106,83 @@ struct PagedParams {
 template <int D, bool kBf16, int RW>
 struct Tile {
   static constexpr int kWarpKeys = kStageKeys / (4 / RW), kNT = kWarpKeys / 8, kChunks = D / 8;
+  // weights are at most one.  fp16 parts end at 2^-24, so there they and their sums are carried 2^15 times as large
+  static constexpr float kUnit = kBf16 ? 1.f : 32768.f;
   using L = Smem<D>;
   float m[2], l[2], o[D / 8][4];
+
+  // one stage's scores become weights; running maxima and sums follow, and where `plain` the product with V is added
+  template <bool kHalf>
+  __device__ __forceinline__ void weigh_and_add(float (&s)[kNT][4], uint32_t v_at, float sc, bool plain) {
+#pragma unroll
+    for (int i = 0; i < (kHalf ? 1 : 2); ++i) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < kNT; ++j) mx = fmaxf(mx, fmaxf(s[j][2 * i], s[j][2 * i + 1]));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float mn = fmaxf(m[i], mx);                              // unscaled: the largest score's weight is one whatever its size
+      const float use = mn == -INFINITY ? 0.f : mn;                  // nothing visible yet: keep the arithmetic finite
+      const float corr = exp2f((m[i] - use) * sc);
+      m[i] = mn;
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < kNT; ++j) {
+        s[j][2 * i] = exp2f((s[j][2 * i] - use) * sc) * kUnit;
+        s[j][2 * i + 1] = exp2f((s[j][2 * i + 1] - use) * sc) * kUnit;
+        sum += s[j][2 * i] + s[j][2 * i + 1];
+      }
+      l[i] = l[i] * corr + sum;                                      // this thread's columns; the quad's are added at the end
+      if (__any_sync(0xffffffffu, corr != 1.f)) {                    // seldom after the first stages
+#pragma unroll
+        for (int j = 0; j < D / 8; ++j) {
+          o[j][2 * i] *= corr;
+          o[j][2 * i + 1] *= corr;
+          if (kHalf) {
+            o[j][2] *= corr;
+            o[j][3] *= corr;
+          }
+        }
+      }
+    }
+    if (!plain) return;
+#pragma unroll
+    for (int k = 0; k < kWarpKeys / 16; ++k) {
+      uint32_t part[3][4];
+#pragma unroll
+      for (int e = 0; e < 4; e += kHalf ? 2 : 1) {
+        float x = s[2 * k + (e >> 1)][(e & 1) * 2], y = s[2 * k + (e >> 1)][(e & 1) * 2 + 1];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          part[q][e] = pack2<kBf16>(x, y);
+          const float2 h = unpack2<kBf16>(part[q][e]);
+          x -= h.x;
+          y -= h.y;
+        }
+      }
+      if (kHalf) {                                                   // the second parts ride in the rows that stand empty
+        part[0][1] = part[1][0];
+        part[0][3] = part[1][2];
+        part[2][1] = part[2][3] = 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < D / 8; j += 2) {
+        uint32_t b[4];
+        ldsm4_t(v_at + k * 16 * L::kPitch + j * 16, b);
+#pragma unroll
+        for (int q = 0; q < 3; q += kHalf ? 2 : 1) {
+          mma16816<kBf16>(o[j], part[q], b[0], b[1]);
+          mma16816<kBf16>(o[j + 1], part[q], b[2], b[3]);
+        }
+      }
+    }
+  }
 
   __device__ __forceinline__ void run(const PagedParams& p, uint8_t* smem, const int32_t* bt, int hk, int t0, int n, int min_vis, int k0, int k1) {
     const PagedAttnArgs& a = p.a;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tg = lane & 3;
     const int G = 1 << p.group_shift, np = a.ng << p.group_shift, n_rows = n << p.group_shift;
+    const bool half = RW == 1 && n_rows <= 8;                        // rows 8 to 15 of the tile stand empty
     const int n_stages = k1 > k0 ? (k1 - k0 + kStageKeys - 1) / kStageKeys : 0;
     // ---- gather of one stage into its ring buffer
     const uint32_t ring = smem_u32(smem);
@@ -208,55 +278,9 @@ struct Tile {
           for (int e = 0; e < 4; ++e)
             if (kb + wkey + j * 8 + tg * 2 + (e & 1) >= min(vis[e >> 1], k1)) s[j][e] = -INFINITY;
       }
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        float mx = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < kNT; ++j) mx = fmaxf(mx, fmaxf(s[j][2 * i], s[j][2 * i + 1]));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float mn = fmaxf(m[i], mx);                            // unscaled: the largest score's weight is one whatever its size
-        const float use = mn == -INFINITY ? 0.f : mn;                // nothing visible yet: keep the arithmetic finite
-        const float corr = exp2f((m[i] - use) * sc);
-        m[i] = mn;
-        float sum = 0.f;
-#pragma unroll
-        for (int j = 0; j < kNT; ++j) {
-          s[j][2 * i] = exp2f((s[j][2 * i] - use) * sc);
-          s[j][2 * i + 1] = exp2f((s[j][2 * i + 1] - use) * sc);
-          sum += s[j][2 * i] + s[j][2 * i + 1];
-        }
-        l[i] = l[i] * corr + sum;                                    // this thread's columns; the quad's are added at the end
-        if (__any_sync(0xffffffffu, corr != 1.f)) {                  // seldom after the first stages
-#pragma unroll
-          for (int j = 0; j < D / 8; ++j) {
-            o[j][2 * i] *= corr;
-            o[j][2 * i + 1] *= corr;
-          }
-        }
-      }
-      if (plain) {
-#pragma unroll
-        for (int k = 0; k < kWarpKeys / 16; ++k) {
-          uint32_t hi[4], lo[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float x = s[2 * k + (e >> 1)][(e & 1) * 2], y = s[2 * k + (e >> 1)][(e & 1) * 2 + 1];
-            hi[e] = pack2<kBf16>(x, y);
-            const float2 h = unpack2<kBf16>(hi[e]);
-            lo[e] = pack2<kBf16>(x - h.x, y - h.y);
-          }
-#pragma unroll
-          for (int j = 0; j < D / 8; j += 2) {
-            uint32_t b[4];
-            ldsm4_t(buf + v_off + k * 16 * L::kPitch + j * 16, b);
-            mma16816<kBf16>(o[j], hi, b[0], b[1]);
-            mma16816<kBf16>(o[j], lo, b[0], b[1]);
-            mma16816<kBf16>(o[j + 1], hi, b[2], b[3]);
-            mma16816<kBf16>(o[j + 1], lo, b[2], b[3]);
-          }
-        }
-      } else {
+      if (RW == 1 && half) weigh_and_add<true>(s, buf + v_off, sc, plain);
+      else weigh_and_add<false>(s, buf + v_off, sc, plain);
+      if (!plain) {
         const uint8_t* vrow = smem + (st % L::kStages) * L::kStage + (kStageKeys + wkey) * L::kPitch + tg * 4;
 #pragma unroll
         for (int j = 0; j < kNT; ++j)
@@ -275,6 +299,13 @@ struct Tile {
       }
     }
     cp_async_wait<0>();
+    if (half) {
+#pragma unroll
+      for (int j = 0; j < D / 8; ++j) {
+        o[j][0] += o[j][2];
+        o[j][1] += o[j][3];
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);

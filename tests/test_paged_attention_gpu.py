@@ -106,6 +106,37 @@ def _four_keys(dtype, scores, values, d=64):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_weights_enter_with_all_their_bits(dtype):
+    """Values that cancel but for 2^-24 of their sum: the weights' own rounding is all that is left."""
+    g = torch.Generator().manual_seed(1)
+    scores = (torch.rand(32, 4, generator=g, dtype=torch.float64) * 0.5).to(dtype)
+    scores[:, 0] = 0.625                                     # the largest: its weight is one
+    w = torch.exp2((scores.double() - 0.625) * 1.4426950408889634).cuda()
+    val = torch.zeros(4, 32, dtype=torch.float64, device="cuda")
+    val[1] = 1
+    for i in (0, 2, 3):                                      # each takes the rest away as far as its 16 bits go
+        val[i] = (-(w.t() * val).sum(0) / w[:, i]).to(dtype)
+    cx, q, k, v, _ = _four_keys(dtype, scores.tolist(), val)
+    want = (w.t() * val).sum(0) / w.sum(1)
+    got = cx.attend(1, q, k, v, 1.0)[0].double()
+    # exp2f is within 2 ulp (2^-23) and so are fp32 sums of four terms of at most one
+    assert float((got - want.unsqueeze(-1)).abs().max()) <= 2.0 ** -21
+
+
+@pytest.mark.gpu
+def test_small_weights_of_fp16():
+    """Weights below fp16's normal range, of keys whose values are large, beside one large weight whose value is zero."""
+    scores = [[0.0, -12.0 - 0.0625 * h, -13.0, -14.5] for h in range(16)]
+    val = torch.tensor([[0.0] * 16, [60000.0] * 16, [30000.0] * 16, [-50000.0] * 16], device="cuda")
+    cx, q, k, v, s = _four_keys(torch.float16, scores, val)
+    w = torch.exp(s)
+    want = (w * val.half().double()).sum(0) / w.sum(0)
+    got = cx.attend(1, q, k, v, 1.0)[0].double()
+    assert float(((got - want.unsqueeze(-1)) / want.unsqueeze(-1)).abs().max()) <= 2.0 ** -11 + 2.0 ** -18
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("reqs", [[(500, 1)], [(5000, 1), (3, 1)], [(300, 70)], [(2000, 40)]])
 @pytest.mark.parametrize("dtype,scale", [(torch.float16, -1.0), (torch.bfloat16, -0.5), (torch.float16, 0.0), (torch.bfloat16, 0.0)])
 def test_scales_that_are_not_positive(reqs, dtype, scale):
