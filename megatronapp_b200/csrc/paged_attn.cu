@@ -123,7 +123,7 @@ struct Tile {
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
       const float mn = fmaxf(m[i], mx);                              // unscaled: the largest score's weight is one whatever its size
       const float use = mn == -INFINITY ? 0.f : mn;                  // nothing visible yet: keep the arithmetic finite
-      const float corr = exp2f((m[i] - use) * sc);
+      const float corr = m[i] == mn ? 1.f : exp2f((m[i] - use) * sc);     // also of a row without a key so far: its sums are zero
       m[i] = mn;
       float sum = 0.f;
 #pragma unroll
