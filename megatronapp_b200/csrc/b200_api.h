@@ -240,15 +240,15 @@ struct AttnArgs {
   bool causal;
   bool is_bf16;
   void* probs_out;  // optional MegaScope export [b,hq,sq,sk] (fwd only)
-  int64_t q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_sb, o_sh, o_ss;
   int wait_limit = -1;  // tries of a wait inside the kernels before it gives up (tests); below 0: the kernels' own limit
+  int64_t q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_sb, o_sh, o_ss;
   int64_t do_sb, do_sh, do_ss, dq_sb, dq_sh, dq_ss, dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
 };
 int attn_fwd(const AttnArgs& a, cudaStream_t s);
 int attn_bwd(const AttnArgs& a, cudaStream_t s);
 const char* attn_last_error();
-
 int attn_status(bool clear);   // 1: a kernel of this process gave up on a wait (its rows are NaN); synchronises
+
 // causal attention with logistic weights over packed prompts (tcgen05)
 struct SigAttnArgs {
   const void *q, *k, *v;   // [T, H, d], [T, G, d], [T, G, d] contiguous, padded with zeros to d = 64 or 128
@@ -323,6 +323,8 @@ struct PagedAttnArgs {
   const int32_t* tok_len;   // [T] keys visible to the token (its position + 1)
   const int32_t* cu;        // [n_seqs + 1] tokens of one request lie side by side (nullptr: each token by itself)
   int n_seqs;
+  int decode_len, decode_mean;   // keys of the longest and of an average context beside the chunks (0: not known)
+  bool decode_single;       // with cu: each request beside the chunks has one token
   int n_tokens, ng, group, head_dim, block_size, max_blocks;
   float scale_log2;
   bool is_bf16;
@@ -337,6 +339,7 @@ struct PagedWriteArgs {
 bool paged_attention_supported(int head_dim, int group);
 void paged_write(const PagedWriteArgs& w, cudaStream_t s);
 int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
+bool paged_decode_by_rows(const PagedAttnArgs& a);        // which of the two decode kernels
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s);
 const char* paged_attention_last_error();
 

@@ -935,11 +935,13 @@ void embed_scatter(const Tensor& tokens, const Tensor& weight, std::vector<int64
 }
 // k_new / v_new [T, ng, d] are written to their cache rows `slots` first.  With cu (int32 [R + 1]) the tokens of a request share its
 // keys: chunk_tiles is the number of tiles of 64 / group tokens over the requests with more than 16 / group new tokens, cut into
-// chunk_splits key ranges each; splits <= 0 then says that there are no other requests (how theirs are cut up is the kernel's own business).
+// chunk_splits key ranges each; splits <= 0 then says that there are no other requests.  How theirs are cut up is the kernel's own business, for
+// which decode_len and decode_mean tell their longest and average context and decode_single whether each has one new token.
 Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& block_table,
                        const Tensor& tok_req, const Tensor& tok_len, int64_t block_size, double scale, int64_t splits,
                        const c10::optional<Tensor>& k_new, const c10::optional<Tensor>& v_new, const c10::optional<Tensor>& slots,
-                       const c10::optional<Tensor>& cu, int64_t chunk_tiles, int64_t chunk_splits) {
+                       const c10::optional<Tensor>& cu, int64_t chunk_tiles, int64_t chunk_splits, int64_t decode_len, int64_t decode_mean,
+                       bool decode_single) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && k_cache.dim() == 3 && k_cache.is_contiguous() && v_cache.is_contiguous());
   TORCH_CHECK(q.scalar_type() == k_cache.scalar_type() && (is_bf16(q) || q.scalar_type() == at::kHalf));
@@ -973,6 +975,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
   if (cu.has_value()) {
     TORCH_CHECK(cu->scalar_type() == at::kInt && cu->is_contiguous() && cu->numel() >= 1, "cu must be int32");
     a.cu = cu->data_ptr<int32_t>(); a.n_seqs = static_cast<int>(cu->numel()) - 1;
+    a.decode_len = static_cast<int>(decode_len); a.decode_mean = static_cast<int>(decode_mean); a.decode_single = decode_single;
   }
   if (T == 0) return out;
   const bool decode = !cu.has_value() || splits > 0;
@@ -981,7 +984,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
   const int rc = b200::paged_attention(a, decode, static_cast<int>(chunk_tiles), static_cast<int>(chunk_splits), decode ? ws.data_ptr<float>() : nullptr,
                                        cur_stream());
   TORCH_CHECK(rc == 0, "b200 paged_attention failed: ", rc, " ", b200::paged_attention_last_error());
-  count((decode ? 2 : 0) + (cu.has_value() && chunk_tiles > 0 ? 1 : 0));
+  count((decode ? (ws.numel() > 0 ? 2 : 1) : 0) + (cu.has_value() && chunk_tiles > 0 ? 1 : 0));
   return out;
 }
 bool paged_attention_supported(int64_t head_dim, int64_t group) { return b200::paged_attention_supported(static_cast<int>(head_dim), static_cast<int>(group)); }
@@ -1184,7 +1187,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embed_scatter", &embed_scatter);
   m.def("paged_attention", &paged_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"), py::arg("tok_req"),
         py::arg("tok_len"), py::arg("block_size"), py::arg("scale"), py::arg("splits"), py::arg("k_new") = py::none(), py::arg("v_new") = py::none(),
-        py::arg("slots") = py::none(), py::arg("cu") = py::none(), py::arg("chunk_tiles") = 0, py::arg("chunk_splits") = 1);
+        py::arg("slots") = py::none(), py::arg("cu") = py::none(), py::arg("chunk_tiles") = 0, py::arg("chunk_splits") = 1,
+        py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false);
+  m.def("paged_decode_by_rows", [](int64_t requests, int ng, int group, int head_dim, int longest, int mean, bool single) {
+    b200::PagedAttnArgs a{};
+    const int32_t none = 0;
+    a.cu = &none; a.n_seqs = static_cast<int>(requests); a.ng = ng; a.group = group; a.head_dim = head_dim; a.block_size = 1; a.max_blocks = longest;
+    a.decode_mean = mean; a.decode_single = single;
+    return b200::paged_decode_by_rows(a);
+  });
   m.def("paged_attention_supported", &paged_attention_supported);
   m.def("spin", &spin);
   m.def("write_flag", &write_flag);

@@ -97,7 +97,8 @@ struct PagedParams {
   int n_tiles;                 // chunks: tiles of this launch (its grid is n_tiles * ng * splits); decode: requests
   int splits;                  // chunks: key ranges of a tile; decode: CTAs, or 0 for one per (request, KV head)
   bool beside_chunks;          // decode: the launch before is the chunks'
-  uint32_t q_keep, q_sign;     // the kernels' running maxima want a positive scale: queries are negated for a negative one, zeros for zero
+  float row_scale;             // rows kernel: the scale as it was given
+  uint32_t q_keep, q_sign;     // tiles: the kernels' running maxima want a positive scale: queries are negated for a negative one, zeros for zero
   float* ws;                   // decode: two partials of 16 rows x (d + 2) per CTA
 };
 
@@ -553,6 +554,103 @@ __global__ void __launch_bounds__(512) paged_merge_kernel(const PagedParams p) {
   }
 }
 
+// ---- decode with few rows per key and many short contexts: a tile of the kernels above is mostly empty and its start and end cost more than
+// its keys.  D / 8 lanes share a key (16 bytes each), the CTA's key groups walk a token's keys side by side in fp32 multiply-adds and merge at the
+// end; small CTAs, many per SM, hide the latency that the tiles' rings hide there.
+template <bool kBf16>
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = unpack2<kBf16>(w[i]);
+    f[2 * i] = v.x;
+    f[2 * i + 1] = v.y;
+  }
+}
+template <int D, int G, bool kBf16>
+__global__ void __launch_bounds__(128, G == 1 ? 12 : G == 2 ? 7 : 4) paged_rows_kernel(const PagedParams p) {
+  constexpr int kLanes = D / 8, kWarpKeys = 32 / kLanes, kGroups = 4 * kWarpKeys;
+  __shared__ float s_m[kGroups][G], s_l[kGroups][G];
+  __shared__ float s_acc[kGroups][G][D];
+  const PagedAttnArgs& a = p.a;
+  allow_next();
+  if (!p.beside_chunks) await_previous();
+  const int r = blockIdx.x / a.ng, hk = blockIdx.x % a.ng, np = a.ng * G;
+  const Item it = decode_item(p, r);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lk = lane % kLanes, grp = warp * kWarpKeys + lane / kLanes;
+  // the key groups of a warp run different trip counts at the end of a context: shuffles name only the group's lanes
+  const unsigned gmask = ((1u << kLanes) - 1u) << (lane / kLanes * kLanes);
+  for (int t = it.t0; t < it.t0 + it.n; ++t) {
+    const int len = a.tok_len[t];
+    float q[G][8], m[G], l[G], acc[G][8];
+    const uint16_t* qp = static_cast<const uint16_t*>(a.q) + (static_cast<int64_t>(t) * np + hk * G) * D + lk * 8;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      unpack8<kBf16>(*reinterpret_cast<const uint4*>(qp + g * D), q[g]);
+      m[g] = -INFINITY;
+      l[g] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        q[g][j] *= p.row_scale;
+        acc[g][j] = 0.f;
+      }
+    }
+    const int32_t* bt = a.block_table + static_cast<int64_t>(a.tok_req[t]) * a.max_blocks;
+    for (int k = grp; k < len; k += kGroups) {
+      const int blk = p.bs_shift >= 0 ? k >> p.bs_shift : k / a.block_size;
+      const int64_t slot = static_cast<int64_t>(bt[blk]) * a.block_size + (k - blk * a.block_size);
+      const int64_t off = (slot * a.ng + hk) * D + lk * 8;
+      const uint4 kraw = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.k_cache) + off);
+      const uint4 vraw = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.v_cache) + off);
+      float kf[8], vf[8];
+      unpack8<kBf16>(kraw, kf);
+      unpack8<kBf16>(vraw, vf);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s = fmaf(q[g][j], kf[j], s);
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(gmask, s, o, kLanes);
+        const float mn = fmaxf(m[g], s);
+        const float corr = exp2f(m[g] - mn), w = exp2f(s - mn);
+        l[g] = l[g] * corr + w;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[g][j] = fmaf(acc[g][j], corr, w * vf[j]);
+        m[g] = mn;
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if (lk == 0) {
+        s_m[grp][g] = m[g];
+        s_l[grp][g] = l[g];
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s_acc[grp][g][lk * 8 + j] = acc[g][j];
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < G * D; idx += 128) {
+      const int g = idx / D, d = idx % D;
+      float M = -INFINITY, L = 0.f, O = 0.f;
+#pragma unroll
+      for (int c = 0; c < kGroups; ++c) M = fmaxf(M, s_m[c][g]);
+      if (M > -INFINITY) {
+#pragma unroll
+        for (int c = 0; c < kGroups; ++c) {
+          const float w = exp2f(s_m[c][g] - M);
+          L = fmaf(s_l[c][g], w, L);
+          O = fmaf(s_acc[c][g][d], w, O);
+        }
+      }
+      const uint32_t o16 = pack2<kBf16>(L > 0.f ? O / L : 0.f, 0.f);
+      static_cast<uint16_t*>(a.out)[(static_cast<int64_t>(t) * np + hk * G + g) * D + d] = static_cast<uint16_t>(o16);
+    }
+    __syncthreads();                                                 // the groups' shares have been read
+  }
+  if (p.beside_chunks) await_previous();
+}
+
 // ---- chunks
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p) {
@@ -712,10 +810,25 @@ int launch_decode(const PagedParams& p, cudaStream_t s) {
   return rc != 0 || p.splits == 0 ? rc : launch(paged_merge_kernel<D, kBf16>, items, 512, 0, 1, p, s);
 }
 
+template <int D, bool kBf16>
+int launch_rows(const PagedParams& p, cudaStream_t s) {
+  const unsigned items = static_cast<unsigned>(p.n_tiles * p.a.ng);
+  if (p.a.group == 1) return launch(paged_rows_kernel<D, 1, kBf16>, items, 128, 0, 1, p, s);
+  if (p.a.group == 2) return launch(paged_rows_kernel<D, 2, kBf16>, items, 128, 0, 1, p, s);
+  return launch(paged_rows_kernel<D, 4, kBf16>, items, 128, 0, 1, p, s);
+}
+
 int log2_exact(int v) {
   for (int i = 0; i < 31; ++i)
     if (v == 1 << i) return i;
   return -1;
+}
+
+int64_t decode_items(const PagedAttnArgs& a) { return static_cast<int64_t>(a.cu != nullptr ? a.n_seqs : a.n_tokens) * a.ng; }
+// keys of the longest context, as far as the caller knows
+int64_t decode_keys(const PagedAttnArgs& a) {
+  const int64_t all = static_cast<int64_t>(a.max_blocks) * a.block_size;
+  return a.decode_len > 0 && a.decode_len < all ? a.decode_len : all;
 }
 
 // the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Contexts of up to 8 stages (512
@@ -723,8 +836,7 @@ int log2_exact(int v) {
 // removes (a step of 34 requests of 64 to 153 keys x 12 heads beside two chunks of 37: 44.7 us cut, 23.2 whole; 5 requests of up to
 // 600 keys x 8 heads: 29.1 and 16.3)
 int decode_ctas(const PagedAttnArgs& a) {
-  const int64_t items = static_cast<int64_t>(a.cu != nullptr ? a.n_seqs : a.n_tokens) * a.ng;
-  const int64_t longest = (static_cast<int64_t>(a.max_blocks) * a.block_size + kStageKeys - 1) / kStageKeys;
+  const int64_t items = decode_items(a), longest = (decode_keys(a) + kStageKeys - 1) / kStageKeys;
   if (longest <= 8 || (longest <= 16 && items <= kDecodeCtas)) return 0;
   const int64_t n = items * longest / 2;
   return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
@@ -734,11 +846,31 @@ int decode_ctas(const PagedAttnArgs& a) {
 
 const char* paged_attention_last_error() { return g_paged_err.c_str(); }
 
+// Rows of a tile that stand empty (all but `group` of 16) against keys to share: from how many (request, KV head) pairs on, and up to which
+// context, a CTA per pair is the better one.  us, tiles / rows: 256 requests of 100 keys x 32 heads of 128, group 1 165 / 88, group 2 167 / 133;
+// of 600 keys 581 / 422 and 596 / 703; 512 of 600 x 32 heads of 64 947 / 519 and 949 / 676; 512 of 16 keys x 8 heads of 128, group 4 60 / 41,
+// of 63 keys 70 / 76; 64 of 300 x 8 heads of 128, group 1 35 / 45: there all pairs run at once.  Lengths that differ leave the rows' CTAs
+// uneven, which the tiles' line is not: 96 requests of 64 to 1000 keys x 12 heads of 128 96 / 111, of 64 70 / 61.
+bool paged_decode_by_rows(const PagedAttnArgs& a) {
+  if (a.cu != nullptr && !a.decode_single) return false;             // tokens of one request would each read all its keys
+  const int64_t items = decode_items(a), keys = decode_keys(a);
+  if (items <= kDecodeCtas) return false;
+  const bool many = items > 2 * kDecodeCtas, narrow = a.head_dim == 64;
+  if (a.group == 1) {
+    if (a.decode_mean > 0 && 2 * keys > 3 * a.decode_mean && keys > (narrow ? 1024 : 256)) return false;
+    return keys <= (items >= 4096 ? 2048 : many ? 1024 : narrow ? 640 : 160);
+  }
+  if (a.group == 2) return keys <= (many ? (narrow ? 640 : 160) : 32);
+  return a.group == 4 && many && keys <= 32;
+}
+
 bool paged_attention_supported(int head_dim, int group) {
   return (head_dim == 64 || head_dim == 128) && (group == 1 || group == 2 || group == 4 || group == 8);
 }
 
-int64_t paged_decode_workspace(const PagedAttnArgs& a) { return static_cast<int64_t>(decode_ctas(a)) * 2 * 16 * (a.head_dim + 2); }
+int64_t paged_decode_workspace(const PagedAttnArgs& a) {
+  return paged_decode_by_rows(a) ? 0 : static_cast<int64_t>(decode_ctas(a)) * 2 * 16 * (a.head_dim + 2);
+}
 
 void paged_write(const PagedWriteArgs& w, cudaStream_t s) {
   const int chunks = w.head_dim / 8;
@@ -753,6 +885,7 @@ void paged_write(const PagedWriteArgs& w, cudaStream_t s) {
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s) {
   PagedParams p{};
   p.a = a;
+  p.row_scale = a.scale_log2;
   p.a.scale_log2 = a.scale_log2 == 0.f ? 1.f : fabsf(a.scale_log2);
   p.q_keep = a.scale_log2 == 0.f ? 0u : 0xffffffffu;
   p.q_sign = a.scale_log2 < 0.f ? 0x80008000u : 0u;
@@ -768,9 +901,14 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
   }
   if (a.cu != nullptr && !decode) return 0;                          // every request is a chunk
   p.n_tiles = a.cu != nullptr ? a.n_seqs : a.n_tokens;
+  p.beside_chunks = a.cu != nullptr && chunk_tiles > 0;
+  if (paged_decode_by_rows(a)) {
+    if (decode_items(a) > 0x7fffffff) { g_paged_err = "paged attention: too many requests"; return -12; }
+    return a.head_dim == 128 ? (a.is_bf16 ? launch_rows<128, true>(p, s) : launch_rows<128, false>(p, s))
+                             : (a.is_bf16 ? launch_rows<64, true>(p, s) : launch_rows<64, false>(p, s));
+  }
   p.splits = decode_ctas(a);
   p.ws = ws;
-  p.beside_chunks = a.cu != nullptr && chunk_tiles > 0;
   return a.head_dim == 128 ? (a.is_bf16 ? launch_decode<128, true>(p, s) : launch_decode<128, false>(p, s))
                            : (a.is_bf16 ? launch_decode<64, true>(p, s) : launch_decode<64, false>(p, s));
 }

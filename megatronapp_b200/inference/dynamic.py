@@ -315,12 +315,16 @@ class DynamicInferenceContext:
 
     def _paged_plan(self, group: int, ng: int) -> tuple:
         """How this step's paged attention is cut up: (requests with at most 16 rows, 64-row tiles of the others, key ranges of
-        those).  The same for all layers of one head layout, made once a step."""
+        those, the former's longest and average context, whether each of them has one token).  The same for all layers of one head layout, made once a
+        step."""
         plan = self._paged_plans.get((group, ng))
         if plan is None:
-            new = [p[2] for p in self._plan]
-            chunks = [-(-n * group // 64) for n in new if n * group > 16]
-            plan = self._paged_plans[(group, ng)] = (len(new) - len(chunks), sum(chunks), key_ranges(sum(chunks) * ng, self._max_len))
+            few, chunks = ([p for p in self._plan if (p[2] * group <= 16) == f] for f in (True, False))
+            tiles = sum(-(-p[2] * group // 64) for p in chunks)
+            keys = [p[2] + p[3] for p in few]
+            plan = self._paged_plans[(group, ng)] = (
+                len(few), tiles, key_ranges(tiles * ng, self._max_len),
+                max(keys, default=0), sum(keys) // max(1, len(few)), all(p[2] == 1 for p in few))
         return plan
 
     # -- attention over the paged cache --------------------------------------------
@@ -337,7 +341,7 @@ class DynamicInferenceContext:
 
             ext = ops.ext()
             if ext.paged_attention_supported(q.shape[-1], np_ // ng):
-                decode, chunk_tiles, chunk_splits = self._paged_plan(np_ // ng, ng)
+                decode, chunk_tiles, chunk_splits, *contexts = self._paged_plan(np_ // ng, ng)
                 self.kernel_calls += 1
                 if k.dtype == v.dtype == q.dtype == kc.dtype and _rows_of_16_bytes(k) and _rows_of_16_bytes(v):
                     new = (k, v, self._write_slots)                    # written by the same call
@@ -346,7 +350,7 @@ class DynamicInferenceContext:
                     vc[self._write_slots] = v
                     new = (None, None, None)
                 return ext.paged_attention(q.contiguous(), kc, vc, self._block_table, self._tok_req, self._tok_len,
-                                           self.block_size, float(scale), decode, *new, self.packed.cu, chunk_tiles, chunk_splits)
+                                           self.block_size, float(scale), decode, *new, self.packed.cu, chunk_tiles, chunk_splits, *contexts)
         kc[self._write_slots] = k
         vc[self._write_slots] = v
         self._ensure_gather(q.device)

@@ -158,3 +158,43 @@ def test_scores_beyond_the_exponent(dtype, size):
     q *= size
     got = cx.attend(1, q, k, v, 64.0)[0, :, 0].double().cpu()
     assert torch.equal(got, torch.tensor([7.0, (2 + 5) / 2, (6 + 9) / 2], dtype=torch.float64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,longest,chunk,hq,hkv,d,block,dtype", [
+    (130, 128, 0, 4, 4, 64, 16, torch.bfloat16),              # group 1, some 500 pairs, short contexts
+    (250, 250, 0, 4, 4, 128, 24, torch.float16),              # 1000 pairs; a block size that is no power of two
+    (300, 600, 70, 8, 4, 64, 16, torch.bfloat16),             # group 2 beside a chunk of several tiles
+    (225, 128, 9, 8, 4, 128, 16, torch.float16),              # ... beside a chunk of one tile, one of more tokens than a decoding request
+    (230, 32, 0, 16, 4, 128, 32, torch.bfloat16)])            # group 4
+def test_many_requests_with_few_rows(n, longest, chunk, hq, hkv, d, block, dtype):
+    """One CTA per (request, KV head) instead of tiles, against 64 bits; contexts of one key and of the longest length among them."""
+    from megatronapp_b200 import ops
+
+    g = torch.Generator().manual_seed(n)
+    reqs = [(0, 1), (longest - 1, 1)] + [(int(a), 1) for a in torch.randint(0, longest, (n - 2,), generator=g)]
+    if chunk:
+        reqs.insert(n // 2, (33, chunk))
+    assert ops.ext().paged_decode_by_rows(len(reqs), hkv, hq // hkv, d, longest, longest // 2, True)
+    cx, q, k, v = _step(reqs, hq, hkv, d, block, dtype)
+    want, kc, vc = _oracle(cx, reqs, q, k, v, d ** -0.5, block)
+    for _ in range(2):
+        got = cx.attend(1, q, k, v, d ** -0.5)
+        assert torch.equal(cx.kv[1][0], kc) and torch.equal(cx.kv[1][1], vc)
+        unit = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+        assert float((got.double() - want).abs().max()) <= unit * max(1.0, float(want.abs().max()))
+        assert float((got.double() - want).norm()) <= 0.5 * unit * float(want.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("requests,ng,group,d,longest,mean,single,rows", [
+    (64, 8, 1, 128, 100, 100, True, True), (512, 32, 1, 64, 600, 600, True, True), (512, 32, 1, 64, 2048, 2048, True, True),
+    (512, 32, 1, 64, 2049, 2049, True, False), (256, 12, 2, 64, 600, 600, True, True), (256, 12, 2, 128, 600, 600, True, False),
+    (512, 8, 4, 128, 16, 16, True, True), (512, 8, 4, 128, 63, 63, True, False), (512, 8, 8, 128, 16, 16, True, False),
+    (64, 8, 1, 128, 600, 600, True, False), (32, 12, 1, 64, 100, 100, True, False), (512, 32, 1, 64, 100, 100, False, False),
+    (96, 12, 1, 128, 1000, 1000, True, True), (96, 12, 1, 128, 1000, 532, True, False), (96, 12, 1, 64, 1000, 532, True, True)])
+def test_which_decode_kernel(requests, ng, group, d, longest, mean, single, rows):
+    """Lengths and counts at which a CTA per (request, KV head) was measured faster than tiles, and some at which it was not."""
+    from megatronapp_b200 import ops
+
+    assert ops.ext().paged_decode_by_rows(requests, ng, group, d, longest, mean, single) == rows
