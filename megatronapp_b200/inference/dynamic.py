@@ -323,7 +323,7 @@ class DynamicInferenceContext:
             tiles = sum(-(-p[2] * group // 64) for p in chunks)
             keys = [p[2] + p[3] for p in few]
             plan = self._paged_plans[(group, ng)] = (
-                len(few), tiles, key_ranges(tiles * ng, self._max_len),
+                len(few), tiles, key_ranges(tiles * ng, max((p[2] + p[3] for p in chunks), default=0)),
                 max(keys, default=0), sum(keys) // max(1, len(few)), all(p[2] == 1 for p in few))
         return plan
 

@@ -198,3 +198,25 @@ def test_which_decode_kernel(requests, ng, group, d, longest, mean, single, rows
     from megatronapp_b200 import ops
 
     assert ops.ext().paged_decode_by_rows(requests, ng, group, d, longest, mean, single) == rows
+
+
+def test_a_plan_looks_at_the_contexts_that_it_cuts():
+    """Key ranges follow the portions' own contexts, and the decode kernels hear of the others' only."""
+    from megatronapp_b200.inference.dynamic import DynamicInferenceContext
+
+    def plan(reqs, group, ng):
+        cx = DynamicInferenceContext(1 << 16, sum(-(-(a + n) // 16) for a, n in reqs) + 1, 16, 1 << 16, len(reqs))
+        for i in range(len(reqs)):
+            cx.add_request(str(i))
+        old = [(str(i), a) for i, (a, _) in enumerate(reqs) if a]
+        if old:
+            cx.begin_step(old, "cpu")
+            cx.end_step()
+        cx.begin_step([(str(i), n) for i, (_, n) in enumerate(reqs)], "cpu")
+        return cx._paged_plan(group, ng)
+
+    # (requests of up to 16 rows, tiles, key ranges of those, longest and average context of the former, one token each)
+    assert plan([(0, 16), (4095, 1)], 4, 8) == (1, 1, 1, 4096, 4096, True)          # a fresh portion is not cut for its neighbour's context
+    assert plan([(8000, 64), (99, 1), (199, 1)], 1, 8) == (2, 1, 16, 200, 150, True)
+    assert plan([(10, 3), (20, 1)], 4, 8) == (2, 0, 1, 21, 17, False)
+    assert plan([(0, 100)], 4, 8) == (0, 7, 1, 0, 0, True)
