@@ -57,8 +57,8 @@ def ssd_scan_torch(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
     b, l, h, p = x.shape
     g, n = B.shape[2], B.shape[3]
     rep = h // g
-    Bh = B.repeat_interleave(rep, dim=2).float()
-    Ch = C.repeat_interleave(rep, dim=2).float()
+    # each group's columns for all of its heads; expanded and not repeat_interleave, which a tracer cannot follow on the GPU
+    Bh, Ch = (t.unsqueeze(3).expand(b, l, g, rep, n).reshape(b, l, h, n).float() for t in (B, C))
     xf, dtf = x.float(), dt.float()
     dA = dtf * A.float().view(1, 1, h)                               # [b, l, h] log decay per step
     state = torch.zeros(b, h, p, n, dtype=torch.float32, device=x.device) if initial_state is None else initial_state.float()
@@ -126,14 +126,19 @@ def _steps(t: torch.Tensor) -> torch.Tensor:
     return t if ok else t.clone(memory_format=torch.contiguous_format)
 
 
+def _plain_eager() -> bool:
+    """Nobody has to see the single operations: no forward-mode or functorch transform, no tracer, no compiler."""
+    return (torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 def ssd_scan(x, dt, A, B, C, D, chunk: int = 64, initial_state=None):
     """x [b, l, h, p], dt [b, l, h] (>0), A [h] (<0), B/C [b, l, g, n], D [h] -> y [b, l, h, p], final state (fp32).
     Recurrence per head: S_t = exp(dt_t A) S_{t-1} + dt_t x_t B_t^T ;  y_t = S_t C_t + D x_t.  bf16 / fp32 CUDA tensors with 64-wide heads and
-    64 or 128 states run on the block kernels (64 steps a block, whatever ``chunk`` says), others, and tensors under forward-mode or
-    functorch transforms, in the PyTorch form."""
+    64 or 128 states run on the block kernels (64 steps a block, whatever ``chunk`` says), others, and tensors that are traced, compiled or under
+    forward-mode or functorch transforms, in the PyTorch form."""
     if (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and B.dtype == C.dtype == x.dtype and x.shape[3] == 64 and B.shape[3] in (64, 128)
-            and x.shape[2] % B.shape[2] == 0 and x.numel() > 0 and x.shape[0] * x.shape[2] <= 65535
-            and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()):
+            and x.shape[2] % B.shape[2] == 0 and x.numel() > 0 and x.shape[0] * x.shape[2] <= 65535 and _plain_eager()):
         f32 = lambda t: t.float().contiguous()  # noqa: E731
         return _SSDFn.apply(_steps(x), f32(dt), f32(A), _steps(B), _steps(C), f32(D), None if initial_state is None else f32(initial_state))
     return ssd_scan_torch(x, dt, A, B, C, D, chunk, initial_state)
@@ -198,6 +203,12 @@ def _scan_views(xbc, di, gn, nh, headdim, groups):
     b, s, _ = xbc.shape
     x, B, C = torch.split(xbc, [di, gn, gn], dim=-1)
     return x.view(b, s, nh, headdim), B.view(b, s, groups, gn // groups), C.view(b, s, groups, gn // groups)
+
+
+def _only_its_weights(conv) -> bool:
+    """A convolution that can be left out of the call: nobody put a hook or a forward of their own on it."""
+    return (type(conv).forward is nn.Conv1d.forward and "forward" not in vars(conv) and not torch.nn.modules.module._has_any_global_hook()
+            and not any((conv._forward_hooks, conv._forward_pre_hooks, conv._backward_hooks, conv._backward_pre_hooks)))
 
 
 @dataclass
@@ -266,8 +277,7 @@ class MambaMixer(MegatronModule):
                 and conv.weight.dtype == conv.bias.dtype == self.norm_weight.dtype == zx.dtype and self.d_conv == 4 and self.headdim == 64
                 and self.d_state in (64, 128) and zx.shape[2] % 8 == 0 and (di // ng) % 4 == 0 and di // ng <= 4096
                 and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (conv.weight, conv.bias, self.norm_weight))
-                and zx.shape[1] * self.nheads_local <= 65535 and zx.shape[0] <= 1 << 19 and not conv._forward_hooks and not conv._forward_pre_hooks
-                and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active())
+                and zx.shape[1] * self.nheads_local <= 65535 and zx.shape[0] <= 1 << 19 and _only_its_weights(conv) and _plain_eager())
 
     def forward(self, hidden_states, inference_context=None):
         zxbcdt, _ = self.in_proj(hidden_states)                         # [s, b, local]  (s is the full sequence)

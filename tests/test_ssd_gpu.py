@@ -138,3 +138,45 @@ def test_mixer_core(s, b, hidden, g, n, dtype):
         # or more independent ones, whose norms stay within twice one another
         limit = (5e-5 if dtype == torch.float32 else 2.0 ** -7) * max(float(w.detach().norm()), 1e-6)
         assert off(a, w) <= (limit if dtype == torch.float32 else max(limit, 2 * off(o, w))), i
+
+
+def _mixer():
+    from megatronapp_b200.config.transformer_config import TransformerConfig
+    from megatronapp_b200.parallel import state as ps
+    from megatronapp_b200.ssm.mamba import MambaMixer
+
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1, 1)
+    cfg = TransformerConfig(num_layers=1, hidden_size=128, num_attention_heads=2, params_dtype=torch.bfloat16, bf16=True, mamba_state_dim=64,
+                            mamba_head_dim=64, mamba_num_groups=2)
+    return MambaMixer(cfg, layer_number=1).cuda()
+
+
+def test_tracing_sees_the_operations():
+    from megatronapp_b200.ssm.mamba import ssd_scan
+
+    ins = [t.detach() for t in _case(1, 70, 2, 1, 64, torch.float32, False)[:6]]
+    want = ssd_scan(*ins)[0]
+    traced = torch.jit.trace(lambda *a: ssd_scan(*a)[0], ins, check_trace=False)
+    assert "PythonOp" not in str(traced.graph) and torch.allclose(traced(*ins), want, rtol=1e-3, atol=1e-3 * float(want.abs().max()))
+    mix, x = _mixer().requires_grad_(False), torch.randn(20, 1, 128, device="cuda").bfloat16()
+    want = mix(x)[0]
+    graph = str(torch.jit.trace(lambda t: mix(t)[0], (x,), check_trace=False).graph)
+    assert "_MixerCoreFn" not in graph and "_SSDFn" not in graph
+    assert float((mix(x)[0] - want).norm()) == 0.0
+
+
+@pytest.mark.parametrize("kind", ["forward", "forward_pre", "full_backward", "full_backward_pre", "own forward"])
+def test_hooks_of_the_convolution_fire(kind):
+    mix = _mixer()
+    x = torch.randn(20, 1, 128, device="cuda").bfloat16().requires_grad_()
+    want, = torch.autograd.grad(mix(x)[0].float().square().sum(), x)
+    calls = []
+    if kind == "own forward":
+        plain = mix.conv1d.forward
+        mix.conv1d.forward = lambda t: calls.append(1) or plain(t)
+    else:
+        getattr(mix.conv1d, f"register_{kind}_hook")(lambda *a: calls.append(1))
+    got, = torch.autograd.grad(mix(x)[0].float().square().sum(), x)
+    assert calls
+    assert float((got - want).float().norm()) <= 0.05 * float(want.float().norm())       # a few roundings to 16 bits in other places
