@@ -180,3 +180,43 @@ def test_hooks_of_the_convolution_fire(kind):
     got, = torch.autograd.grad(mix(x)[0].float().square().sum(), x)
     assert calls
     assert float((got - want).float().norm()) <= 0.05 * float(want.float().norm())       # a few roundings to 16 bits in other places
+
+
+def _oracle_by_blocks(x, dt, A, B, C, D):
+    """The recurrence in blocks of 64 steps, for lengths that the step-by-step form has no memory for."""
+    b, l, h, p = x.shape
+    rep = h // B.shape[2]
+    B, C = (t.repeat_interleave(rep, dim=2) for t in (B, C))
+    S, ys = x.new_zeros(b, h, p, B.shape[3]), []
+    for i in range(0, l, 64):
+        X, Bc, Cc = (t[:, i:i + 64].transpose(1, 2) for t in (x * dt.unsqueeze(-1), B, C))
+        cum = (dt * A)[:, i:i + 64].cumsum(1).transpose(1, 2)
+        low = torch.ones(cum.shape[-1], cum.shape[-1], dtype=torch.bool, device=x.device).tril()
+        decay = (cum.unsqueeze(-1) - cum.unsqueeze(-2)).masked_fill(~low, float("-inf")).exp()
+        ys.append(((Cc @ Bc.transpose(-1, -2) * decay) @ X + cum.exp().unsqueeze(-1) * (Cc @ S.transpose(-1, -2))).transpose(1, 2))
+        S = S * cum[..., -1:, None].exp() + (X * (cum[..., -1:] - cum).exp().unsqueeze(-1)).transpose(-1, -2) @ Bc
+    return torch.cat(ys, 1) + D.view(1, 1, h, 1) * x, S
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.bfloat16, 128), (torch.bfloat16, 64), (torch.float32, 128), (torch.float32, 64)])
+@pytest.mark.parametrize("l,h,launches", [
+    (3589, 12, 3),              # 57 blocks x 8: a CTA walks all three heads of a group
+    (1762, 16, 4)])             # 28 blocks x 8 x 2: two CTAs share a group's four heads, two each, and their parts are merged
+def test_heads_of_a_group_in_one_block(l, h, launches, dtype, n):
+    from megatronapp_b200.ops import seqmix
+    from megatronapp_b200.ssm.mamba import ssd_scan
+
+    ins = _case(2, l, h, 4, n, dtype, False)[:6]
+    y, last = ssd_scan(*ins)
+    wide = [t.detach().double().requires_grad_() for t in ins]
+    want_y, want_last = _oracle_by_blocks(*wide)
+    dy, dl = torch.randn_like(y), torch.randn_like(last)
+    before = seqmix.ext().launch_count()
+    got = torch.autograd.grad((y, last), ins, (dy, dl))
+    assert seqmix.ext().launch_count() == before + launches
+    want = torch.autograd.grad((want_y, want_last), wide, (dy.double(), dl.double()))
+    c = float((wide[1] * -wide[2]).detach().sum(1).max()) * 64 / l
+    for i, (a, w) in enumerate(zip([y, last, *got], [want_y, want_last, *want])):
+        # as against the recurrence; the sums over all steps (of A and D) are of terms of either sign, whose rounding grows as they do
+        tol = 2e-5 + 2.0 ** -23 * c if a.dtype == torch.float32 else 2.0 ** -8
+        assert float((a.detach().double() - w.detach()).norm()) <= tol * float(w.norm()), i
