@@ -183,7 +183,8 @@ struct EmbeddingGradArgs {
 int64_t embedding_grad_parts(int n, int h);
 void embedding_grad(const EmbeddingGradArgs& a, cudaStream_t s);
 
-// gradients of the router logits x [n, h] . w [experts, h]^T, whichever of dx and dw is set; rows contiguous, h % 8 == 0
+// gradients of the router logits x [n, h] . w [experts, h]^T, whichever of dx and dw is set; rows contiguous, h % 8 == 0, experts <= kRouterExperts
+constexpr int kRouterExperts = 32;
 struct RouterArgs {
   const void *x, *w;
   const float* dlogits;

@@ -537,7 +537,7 @@ Tensor embedding_grad(const Tensor& dy, const Tensor& ids, int64_t vocab) {
 }
 static b200::RouterArgs router_args(const Tensor& x, const Tensor& w) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.dim() == 2 && w.dim() == 2 && x.is_contiguous() && w.is_contiguous() && x.size(1) == w.size(1) &&
-              x.size(1) % 8 == 0 && x.size(0) > 0 && x.size(0) < (1 << 28) && w.size(0) > 0 && w.size(0) <= 256 && x.size(1) > 0 && x.size(1) <= (1 << 16),
+              x.size(1) % 8 == 0 && x.size(0) > 0 && x.size(0) < (1 << 28) && w.size(0) > 0 && w.size(0) <= b200::kRouterExperts && x.size(1) > 0 && x.size(1) <= (1 << 16),
               "router_linear: shapes");
   TORCH_CHECK((x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kHalf) && (w.scalar_type() == at::kFloat || w.scalar_type() == x.scalar_type()) &&
               reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0, "router_linear: types");

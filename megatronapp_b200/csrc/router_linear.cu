@@ -70,30 +70,24 @@ __device__ __forceinline__ void put4(__half* p, float4 v) {
 
 template <typename T, typename W>
 __global__ void __launch_bounds__(128) router_dx_kernel(const float* __restrict__ dl, const W* __restrict__ w, T* __restrict__ dx, int n, int h, int e_all) {
-  __shared__ float s_dl[32][kTokDx];           // 32 experts of a pass
+  __shared__ float s_dl[kRouterExperts][kTokDx];
   const int c = (blockIdx.y * 128 + threadIdx.x) * 8, t0 = blockIdx.x * kTokDx;
-  float acc[kTokDx][8] = {};
-  for (int e0 = 0; e0 < e_all; e0 += 32) {
-    const int m = min(32, e_all - e0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < m * kTokDx; i += 128) {
-      const int k = i / m, e = i % m;
-      s_dl[e][k] = t0 + k < n ? dl[static_cast<int64_t>(t0 + k) * e_all + e0 + e] : 0.f;
-    }
-    __syncthreads();
-    if (c < h) {
-#pragma unroll 8
-      for (int e = 0; e < m; ++e) {
-        float wv[8];
-        get8(w + static_cast<int64_t>(e0 + e) * h + c, wv);
-#pragma unroll
-        for (int k = 0; k < kTokDx; ++k)
-#pragma unroll
-          for (int q = 0; q < 8; ++q) acc[k][q] = fmaf(s_dl[e][k], wv[q], acc[k][q]);
-      }
-    }
+  for (int i = threadIdx.x; i < e_all * kTokDx; i += 128) {
+    const int k = i / e_all, e = i % e_all;
+    s_dl[e][k] = t0 + k < n ? dl[static_cast<int64_t>(t0 + k) * e_all + e] : 0.f;
   }
+  __syncthreads();
   if (c >= h) return;
+  float acc[kTokDx][8] = {};
+#pragma unroll 8
+  for (int e = 0; e < e_all; ++e) {
+    float wv[8];
+    get8(w + static_cast<int64_t>(e) * h + c, wv);
+#pragma unroll
+    for (int k = 0; k < kTokDx; ++k)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[k][q] = fmaf(s_dl[e][k], wv[q], acc[k][q]);
+  }
 #pragma unroll
   for (int k = 0; k < kTokDx; ++k)
     if (t0 + k < n) put8(dx + static_cast<int64_t>(t0 + k) * h + c, acc[k]);
