@@ -164,7 +164,7 @@ def test_moe_layer_fused_matches_sequential():
     _assert_small(gc.check_moe_layer(), 5e-2)
 
 
-def test_loss_curve_matches_unmodified_reference():
+def test_loss_curve_matches_unmodified_reference(tmp_path):
     """Same weights + same data through baseline/_ref (the reference's own train_step) and through this framework:
     per-step training loss within 1e-2 for 20 optimizer steps (tools/ref_parity.py)."""
     import json
@@ -174,7 +174,7 @@ def test_loss_curve_matches_unmodified_reference():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     if not os.path.isdir(os.path.join(root, "baseline", "_ref", "megatron")):
         pytest.skip("baseline/_ref not installed")
-    out = os.path.join(root, "gpurun_out", "ref_parity_pytest.json")
+    out = str(tmp_path / "ref_parity.json")
     p = subprocess.run([sys.executable, os.path.join(root, "tools", "ref_parity.py"), "--steps", "20", "--out", out],
                        capture_output=True, text=True, timeout=600, cwd=root)
     line = [l for l in p.stdout.splitlines() if l.startswith("REF_PARITY ")]

@@ -13,8 +13,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.skipif(not torch.cuda.is_available() or torch.cuda.device_count() < 2, reason="needs 2 GPUs")
-def test_fused_collective_kernels_two_gpus():
-    out = os.path.join(ROOT, "gpurun_out", "multi_pytest.json")
+def test_fused_collective_kernels_two_gpus(tmp_path):
+    out = str(tmp_path / "multi.json")
     cmd = [sys.executable, "-m", "torch.distributed.run", "--nproc-per-node", "2", "--master-addr", "127.0.0.1",
            "--master-port", "29547", os.path.join(ROOT, "tools", "multi_gpu_checks.py"), "--out", out, "--skip-model"]
     p = subprocess.run(cmd, capture_output=True, text=True, timeout=900, cwd=ROOT)

@@ -3,7 +3,7 @@
 Each check runs in its own subprocess with a timeout so a hung / faulting kernel cannot take
 the whole session (or the GPU lease) down; results are merged into one JSON file.
 
-    python tools/gpu_checks.py --out gpurun_out/checks.json [--only gemm_nt,ln] [--perf]
+    python tools/gpu_checks.py --out build/checks.json [--only gemm_nt,ln] [--perf]
 """
 from __future__ import annotations
 
@@ -978,7 +978,7 @@ PERF = {"paged_attention_perf": check_paged_attention_perf, "mxfp8_perf": check_
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "checks.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "checks.json"))
     ap.add_argument("--only", default=None)
     ap.add_argument("--perf", action="store_true")
     ap.add_argument("--one", default=None)

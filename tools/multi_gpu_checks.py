@@ -1,7 +1,7 @@
 """Multi-GPU checks of the fused compute+collective kernels (run under torchrun, N >= 2):
 
     python -m torch.distributed.run --nproc-per-node 2 --master-addr 127.0.0.1 --master-port 29533 \
-        tools/multi_gpu_checks.py --out gpurun_out/multi.json
+        tools/multi_gpu_checks.py --out build/multi.json
 
 Numerics: fused kernel vs (NCCL collective + fp32 matmul); timing: device events, max over
 ranks, against the unfused cuBLAS + NCCL sequence on the same tensors.
@@ -116,7 +116,7 @@ def dp_and_embed_checks(arena, fc, group, rank, world, dt, log, ops):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "multi.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "multi.json"))
     ap.add_argument("--skip-model", action="store_true")
     ap.add_argument("--skip-moe", action="store_true")
     ap.add_argument("--skip-kernels", action="store_true")

@@ -1,7 +1,7 @@
 """Turn ncu output into the markdown summaries kept under profiles/.
 
-    python tools/ncu_summary.py rep gpurun_out/kernels_r1.ncu-rep > profiles/r1_ncu_kernels.md
-    python tools/ncu_summary.py launches gpurun_out/launches_r1b.csv > profiles/r1_launch_breakdown.md
+    python tools/ncu_summary.py rep build/kernels.ncu-rep > profiles/ncu_kernels.md
+    python tools/ncu_summary.py launches build/launches.csv > profiles/launch_breakdown.md
 """
 import collections
 import csv

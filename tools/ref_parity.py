@@ -1,6 +1,6 @@
 """Loss-trajectory parity against the UNMODIFIED reference (baseline/_ref), same weights, same data.
 
-    python tools/ref_parity.py --steps 20 [--out gpurun_out/ref_parity.json]                 # 1 GPU
+    python tools/ref_parity.py --steps 20 [--out build/ref_parity.json]                 # 1 GPU
     python -m torch.distributed.run --nproc-per-node 2 --master-addr 127.0.0.1 --master-port 29541 \
         tools/ref_parity.py --tp 2                                                            # TP2 (+SP on our side)
 
@@ -36,7 +36,7 @@ def main():
     ap.add_argument("--vocab", type=int, default=8192)
     ap.add_argument("--micro-batch", type=int, default=4)
     ap.add_argument("--n-mb", type=int, default=2)
-    ap.add_argument("--out", default=os.path.join(ROOT, "gpurun_out", "ref_parity.json"))
+    ap.add_argument("--out", default=os.path.join(ROOT, "build", "ref_parity.json"))
     a = ap.parse_args()
     import torch
 

@@ -1,7 +1,7 @@
 """Small-shape exercise of the flag-protocol / peer-memory kernels, meant to run under compute-sanitizer:
 
     python -m torch.distributed.run --no-python --nproc-per-node 2 --master-addr 127.0.0.1 --master-port 29599 \\
-        compute-sanitizer --tool synccheck --log-file gpurun_out/synccheck_%p.log python tools/sanitize_comm.py
+        compute-sanitizer --tool synccheck --log-file build/synccheck_%p.log python tools/sanitize_comm.py
 
 (fused AG->GEMM, GEMM->RS, bucket reduce-scatter, embedding scatter, device barrier; with WORLD_SIZE=1 the single-GPU
 shared-memory kernels instead: paged attention, MX quantiser, norms, MoE layout / gather kernels).  Prints OK lines so the
