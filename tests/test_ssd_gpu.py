@@ -147,7 +147,7 @@ def _mixer():
 
     if not ps.model_parallel_is_initialized():
         ps.initialize_model_parallel(1, 1)
-    cfg = TransformerConfig(num_layers=1, hidden_size=128, num_attention_heads=2, params_dtype=torch.bfloat16, bf16=True, mamba_state_dim=64,
+    cfg = TransformerConfig(num_layers=1, hidden_size=256, num_attention_heads=2, params_dtype=torch.bfloat16, bf16=True, mamba_state_dim=64,
                             mamba_head_dim=64, mamba_num_groups=2)
     return MambaMixer(cfg, layer_number=1).cuda()
 
@@ -159,7 +159,8 @@ def test_tracing_sees_the_operations():
     want = ssd_scan(*ins)[0]
     traced = torch.jit.trace(lambda *a: ssd_scan(*a)[0], ins, check_trace=False)
     assert "PythonOp" not in str(traced.graph) and torch.allclose(traced(*ins), want, rtol=1e-3, atol=1e-3 * float(want.abs().max()))
-    mix, x = _mixer().requires_grad_(False), torch.randn(20, 1, 128, device="cuda").bfloat16()
+    mix, x = _mixer().requires_grad_(False), torch.randn(20, 1, 256, device="cuda").bfloat16()
+    assert mix._fused_core_ok(mix.in_proj(x)[0])
     want = mix(x)[0]
     graph = str(torch.jit.trace(lambda t: mix(t)[0], (x,), check_trace=False).graph)
     assert "_MixerCoreFn" not in graph and "_SSDFn" not in graph
@@ -169,7 +170,8 @@ def test_tracing_sees_the_operations():
 @pytest.mark.parametrize("kind", ["forward", "forward_pre", "full_backward", "full_backward_pre", "own forward"])
 def test_hooks_of_the_convolution_fire(kind):
     mix = _mixer()
-    x = torch.randn(20, 1, 128, device="cuda").bfloat16().requires_grad_()
+    x = torch.randn(20, 1, 256, device="cuda").bfloat16().requires_grad_()
+    assert mix._fused_core_ok(mix.in_proj(x)[0])
     want, = torch.autograd.grad(mix(x)[0].float().square().sum(), x)
     calls = []
     if kind == "own forward":
