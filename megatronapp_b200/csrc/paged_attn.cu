@@ -13,11 +13,12 @@
 //   rows = 16 (decode, short chunks): the four warps take 16 keys of a stage each, bound by HBM.  The stages of all (request, KV head)
 //     pairs stand in one line that is cut evenly over three CTAs per SM, whatever the contexts' lengths; an item that a cut falls into
 //     leaves partial (max, sum, accumulator) triples, which a small second kernel merges.  64 contexts of 1k to 4k, 32 / 8 heads of 128:
-//     117 us, 5.7 TB/s, the rest latency of one stage's dependent steps (138 with three stages and two CTAs per SM; 456 with a key per 16
-//     lanes and no load in flight behind it).
+//     120 us, 5.6 TB/s, the rest latency of one stage's dependent steps (138 with three stages and two CTAs per SM; 456 with a key per 16
+//     lanes and no load in flight behind it).  Many short contexts with few heads a group go by rows instead, see paged_rows_kernel.
 //   rows = 64 (chunks): a warp takes 16 rows and all keys of a stage, longest tiles first, bound by the tensor instructions.  Where the
 //     tiles are few and the context is long, the CTAs of a cluster take key ranges and merge through distributed shared memory.  Two
-//     chunks of 500 tokens beside 24 decoding requests: 865 us before, every token reading all its keys, 57 + 39 us now.
+//     chunks of 500 tokens beside 24 decoding requests: 865 us before, every token reading all its keys, 67 + 40 us now (57 + 39 when the
+//     weights' third parts were left out).
 //
 // Replaces the reference's dynamic-context attention (core/inference/contexts/dynamic_context.py + flash_attn_with_kvcache
 // in attention.py:590-603) and this repo's earlier gather + einsum path (inference/dynamic.py).
