@@ -92,9 +92,21 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, volatil
   *failed = 1;
   return false;
 }
-// the same for a whole warp, which leaves the wait converged
+// the same for a whole warp, which votes after every try and so stays converged: 65 cycles for a barrier that is ready (123 where the lanes
+// loop on their own and vote at the end)
 __device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, volatile int* failed, int limit = kWaitLimit) {
-  return __all_sync(0xffffffffu, wait_bar(bar, parity, failed, limit));
+  for (int i = 0; i < limit; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 255) == 255 && __any_sync(0xffffffffu, *failed != 0)) return false;
+  }
+  *failed = 1;
+  return false;
+}
+
+// One arrival for a warp: 32 of them on one word are carried out one after another
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
 }
 
 // One warpgroup copies and issues, four do the softmax arithmetic.  A CTA of 640 threads starts with 96 registers each; the math
@@ -154,12 +166,14 @@ struct FwdSmem {
 };
 
 // ------------------------------------------------------------------------------------ forward
-// P (16-bit) overwrites S columns in TMEM and feeds the PV product as the TMEM A operand.  Two query tiles alternate between the tensor
-// core (1024 cycles a key block at D = 128) and the softmax (1024 cycles of exponentials at one block's rate), so what counts is the time
-// from S to P of one tile.  Two warpgroups share it, 64 columns of each row apiece: S is read once into registers, the halves
-// exchange their row maxima through shared memory, and each packs its P into its own half of the S columns.  The product with V
-// starts on the first 32 columns of both halves while the others' exponentials are still taken.
-// 32 / 8 heads x 4096 x 128 causal: 201 us with one warpgroup a tile, 158 with two, 151 with P in two parts; 32 heads x 8192: 630, 524, 503.
+// P (16-bit) goes to TMEM columns of its own and feeds the PV product as the TMEM A operand.  Two query tiles alternate between the tensor
+// core (1024 cycles a key block at D = 128) and the softmax (1024 cycles of exponentials at one block's rate).  Two warpgroups share a
+// tile, 64 columns of each row apiece: S is read once into registers, the halves exchange their row maxima through shared memory, and
+// each packs its P into its own 32 columns.  S's columns are free again as soon as they are in registers, so the next S (the other
+// tile's where there is one buffer, this tile's where there are two) is made under this one's exponentials: a warpgroup that has handed
+// over its P finds its next S waiting.  Two warps issue: a wait that is already over costs 65 to 120 cycles, the tensor core's queue holds four
+// MMAs (256 cycles), and one warp that goes through all waits in turn leaves it empty (174 us where two take 139).
+// 32 / 8 heads x 4096 x 128 causal: 145 us with P over S and S after its PV, 131 so; 32 heads x 8192: 479 -> 435 us.
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -178,12 +192,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint64_t* k_empty = bars + 3;       // 2
   uint64_t* v_full = bars + 5;        // 2
   uint64_t* v_empty = bars + 7;       // 2
-  uint64_t* s_full = bars + 9;        // 2 (per q tile); S(j + 1) complete says that PV(j), issued before it, is too
-  uint64_t* p_ready = bars + 11;      // 2 (per q tile) x 2: the first and second 32 columns of both halves' P
-  uint64_t* o_done = bars + 15;       // 2
+  uint64_t* s_full = bars + 9;        // 2 (per q tile)
+  uint64_t* s_read = bars + 11;       // 2 (per q tile): S is in registers
+  uint64_t* p_ready = bars + 13;      // 2 (per q tile)
+  uint64_t* pv_done = bars + 15;      // 2 (per q tile): P's columns are free and O is up to date
   uint64_t* drained = bars + 17;      // 1, after a wait that ran out
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
-  volatile int* failed = reinterpret_cast<volatile int*>(bars + 19);
+  uint64_t* s_issued = bars + 18;     // 4: the CTA's S number i (of both tiles) is in the tensor core's queue, at i % 4
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+  volatile int* failed = reinterpret_cast<volatile int*>(bars + 23);
 
   const int warp_idx = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);   // known to be uniform: see desc_at
   const int lane = threadIdx.x & 31;
@@ -206,9 +222,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 256); mbar_init(&p_ready[2 + i], 256); mbar_init(&o_done[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&s_read[i], 8);
+      mbar_init(&p_ready[i], 8); mbar_init(&pv_done[i], 1);
     }
-    mbar_init(drained, 1);
+    mbar_init(drained, 2);
+    for (int i = 0; i < 4; ++i) mbar_init(&s_issued[i], 1);
     *failed = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
@@ -218,9 +236,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  int nk = 0, nv = 0;                         // thread 0: blocks whose copies it has started
-  const uint32_t tmem_S = tmem_base;          // S[t] at col t*128
-  const uint32_t tmem_O = tmem_base + 256;    // O[t] at col 256 + t*D
+  int n_loaded = 0;                           // blocks whose copies this thread (lane 0 of warps 0 and 3) has started
+  const uint32_t tmem_O = tmem_base;                                 // O[t] at col t*D
+  const uint32_t tmem_P = tmem_base + 2 * D;                         // P[t] at col 2*D + t*64
+  const uint32_t tmem_S = tmem_base + 2 * D + 128;                   // S[t] at t*128 of the remaining 256, or one S for both in 128
+  constexpr int kSBufs = D == 64 ? 2 : 1;
+  static_assert(2 * D + 128 + kSBufs * 128 <= 512, "TMEM columns");
 
   if (warp_idx < 4) {
     regs_give<kIssueRegs>();
@@ -231,78 +252,86 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int t = 0; t < ntiles; ++t)
         for (int c = 0; c < L::kDC; ++c)
           tma_load_4d(&tmap_q, q_full, sQ + t * L::kTile + c * (kBlockQ * 128), c * 64, h, bi, t == 0 ? q0_0 : q0_1);
-      while (nk < nmax) {
-        const int st = nk % kS;
-        const uint32_t ph = ((nk / kS) & 1) ^ 1;
-        if (!wait_bar(&k_empty[st], ph, failed, p.wait_limit)) break;
+      for (; n_loaded < nmax; ++n_loaded) {
+        const int st = n_loaded % kS;
+        if (!wait_bar(&k_empty[st], ((n_loaded / kS) & 1) ^ 1, failed, p.wait_limit)) break;
         mbar_arrive_expect_tx(&k_full[st], L::kTile);
         for (int c = 0; c < L::kDC; ++c)
-          tma_load_4d(&tmap_k, &k_full[st], sK + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, nk * kBlockKV);
-        ++nk;
-        if (!wait_bar(&v_empty[st], ph, failed, p.wait_limit)) break;
+          tma_load_4d(&tmap_k, &k_full[st], sK + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, n_loaded * kBlockKV);
+      }
+    } else if (warp_idx == 3 && lane == 0) {
+      // K runs up to two blocks ahead of V: a producer each
+      for (; n_loaded < nmax; ++n_loaded) {
+        const int st = n_loaded % kS;
+        if (!wait_bar(&v_empty[st], ((n_loaded / kS) & 1) ^ 1, failed, p.wait_limit)) break;
         mbar_arrive_expect_tx(&v_full[st], L::kTile);
         for (int c = 0; c < L::kDC; ++c)
-          tma_load_4d(&tmap_v, &v_full[st], sV + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, nv * kBlockKV);
-        ++nv;
+          tma_load_4d(&tmap_v, &v_full[st], sV + st * L::kTile + c * (kBlockKV * 128), c * 64, hk, bi, n_loaded * kBlockKV);
       }
-    } else if (warp_idx == 1 && nmax > 0) {
-      // ============================================================ MMA issuer
+    } else if (warp_idx == 1) {
+      // ============================================================ issuer of S = Q K^T
       constexpr uint32_t idesc_s = make_idesc_f16(kBf16, kBlockQ, kBlockKV, false, false);
-      constexpr uint32_t idesc_o = make_idesc_f16(kBf16, kBlockQ, D, false, true);
       const uint64_t q_desc = make_smem_desc_sw128(smem_u32(sQ), 1024, 0), k_desc = make_smem_desc_sw128(smem_u32(sK), 1024, 0);
-      // V is MN-major for its product (N = d contiguous): 16 key rows per k-step, LBO = next 64-wide d chunk
-      const uint64_t v_desc = make_smem_desc_sw128(smem_u32(sV), 1024, kBlockKV * 128);
-      auto issue_S = [&](int t, int j) {
-        const uint64_t a0 = desc_at(q_desc, t * L::kTile), b0 = desc_at(k_desc, (j % kS) * L::kTile);
-        if (elect_one()) {
-#pragma unroll
-          for (int k = 0; k < D / 16; ++k) {
-            const uint32_t off = (k >> 2) * (kBlockQ * 128) + (k & 3) * 32;
-            umma_f16_ss(tmem_S + t * 128, desc_at(a0, off), desc_at(b0, off), idesc_s, k != 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[t]);
-        }
-      };
-      auto issue_PV = [&](int t, int j, int part) {
-        const uint64_t b0 = desc_at(v_desc, (j % kS) * L::kTile + part * (2 * 16 * 128));
-        const uint32_t tP = tmem_S + t * 128 + part * 16, first = (j | part) != 0 ? 1u : 0u;
-        if (elect_one()) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            // A = P from TMEM: row = lane, 16 keys = 8 packed 32-bit columns per k-step, 64 keys per half of the S columns; `part` is
-            // the first or second 32 keys of both halves
-            umma_f16_ts(tmem_O + t * D, tP + (k >> 1) * 64 + (k & 1) * 8, desc_at(b0, ((k >> 1) * 4 + (k & 1)) * 16 * 128), idesc_o, k != 0 ? 1u : first);
-        }
-      };
-      auto commit = [&](uint64_t* bar) { if (elect_one()) umma_commit(bar); };
-      bool ok = wait_bar_warp(q_full, 0, failed, p.wait_limit) && wait_bar_warp(&k_full[0], 0, failed, p.wait_limit);
-      if (ok) {
-        tc_fence_after();
-        if (nkv_0 > 0) issue_S(0, 0);
-        if (nkv_1 > 0) issue_S(1, 0);
-        commit(&k_empty[0]);
-      }
+      bool ok = nmax > 0 && wait_bar_warp(q_full, 0, failed, p.wait_limit);
+      int item = 0;
       for (int j = 0; j < nmax && ok; ++j) {
-        const int nx = (j + 1) % kS;
-        ok = wait_bar_warp(&v_full[j % kS], (j / kS) & 1, failed, p.wait_limit) && (j + 1 >= nmax || wait_bar_warp(&k_full[nx], ((j + 1) / kS) & 1, failed, p.wait_limit));
+        const int st = j % kS;
+        ok = wait_bar_warp(&k_full[st], (j / kS) & 1, failed, p.wait_limit);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          const int nt = t == 0 ? nkv_0 : nkv_1;
-          if (j >= nt || !ok) continue;
-          ok = wait_bar_warp(&p_ready[t * 2], j & 1, failed, p.wait_limit);
+          if (j >= (t == 0 ? nkv_0 : nkv_1) || !ok) continue;
+          // the S before it in its buffer is in registers: this tile's where each has its own, else the other's, if that has such a block
+          const bool other = kSBufs == 1 && (t == 1 ? j < nkv_0 : j <= nkv_1);
+          const int rt = other ? 1 - t : t, rj = other && t == 1 ? j : j - 1;
+          ok = rj < 0 || wait_bar_warp(&s_read[rt], rj & 1, failed, p.wait_limit);
           if (!ok) continue;
           tc_fence_after();
-          issue_PV(t, j, 0);                                // while the second part's weights are made
-          ok = wait_bar_warp(&p_ready[t * 2 + 1], j & 1, failed, p.wait_limit);
-          if (!ok) continue;
-          tc_fence_after();
-          issue_PV(t, j, 1);
-          if (j + 1 < nt) issue_S(t, j + 1);
-          else commit(&o_done[t]);
+          const uint64_t a0 = desc_at(q_desc, t * L::kTile), b0 = desc_at(k_desc, st * L::kTile);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < D / 16; ++k) {
+              const uint32_t off = (k >> 2) * (kBlockQ * 128) + (k & 3) * 32;
+              umma_f16_ss(tmem_S + (kSBufs == 2 ? t * 128 : 0), desc_at(a0, off), desc_at(b0, off), idesc_s, k != 0 ? 1u : 0u);
+            }
+            umma_commit(&s_full[t]);
+            if (t == 1 || j >= nkv_1) umma_commit(&k_empty[st]);
+            if (kSBufs == 1) mbar_arrive(&s_issued[item & 3]);
+          }
+          ++item;
         }
-        if (!ok) break;
-        commit(&v_empty[j % kS]);
-        if (j + 1 < nmax) commit(&k_empty[nx]);
+      }
+    } else if (warp_idx == 2) {
+      // ============================================================ issuer of O += P V
+      // a warp of its own: a wait and the steps around it take a few hundred cycles beside the math, and the tensor core's queue is short
+      constexpr uint32_t idesc_o = make_idesc_f16(kBf16, kBlockQ, D, false, true);
+      // V is MN-major for its product (N = d contiguous): 16 key rows per k-step, LBO = next 64-wide d chunk
+      const uint64_t v_desc = make_smem_desc_sw128(smem_u32(sV), 1024, kBlockKV * 128);
+      bool ok = true;
+      // With one S buffer its next S is what everything waits for: 512 cycles of MMAs, and as long again for the steps from S to registers to
+      // the next S.  A product goes into that gap, behind the S two blocks on, and never beside one.
+      const int n_items = nkv_0 + nkv_1;
+      int item = 2;
+      for (int j = 0; j < nmax && ok; ++j) {
+        const int st = j % kS;
+        ok = wait_bar_warp(&v_full[st], (j / kS) & 1, failed, p.wait_limit);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (j >= (t == 0 ? nkv_0 : nkv_1)) continue;
+          if (kSBufs == 1 && item < n_items) ok = ok && wait_bar_warp(&s_issued[item & 3], (item >> 2) & 1, failed, p.wait_limit);
+          ++item;
+          ok = ok && wait_bar_warp(&p_ready[t], j & 1, failed, p.wait_limit);
+          if (!ok) continue;
+          tc_fence_after();
+          const uint64_t b0 = desc_at(v_desc, st * L::kTile);
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < kBlockKV / 16; ++k)
+              // A = P from TMEM: row = lane, 16 keys = 8 packed 32-bit columns per k-step
+              umma_f16_ts(tmem_O + t * D, tmem_P + t * 64 + k * 8, desc_at(b0, k * 16 * 128), idesc_o, k != 0 || j != 0 ? 1u : 0u);
+            umma_commit(&pv_done[t]);
+            if (t == 1 || j >= nkv_1) umma_commit(&v_empty[st]);
+          }
+        }
       }
     }
   } else {
@@ -315,7 +344,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int q0 = t == 0 ? q0_0 : q0_1;
     const int qrow = q0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tS = tmem_S + t * 128 + half * 64 + lane_addr;
+    const uint32_t tS = tmem_S + (kSBufs == 2 ? t * 128 : 0) + half * 64 + lane_addr;
+    const uint32_t tP = tmem_P + t * 64 + half * 32 + lane_addr;
     const uint32_t tO = tmem_O + t * D + half * (D / 2) + lane_addr;
     float* ex = sEx + t * (2 * kBlockQ);          // + parity * 4 kBlockQ + half * kBlockQ + row
     float m = -INFINITY;                          // running max (exp2 domain, already scaled)
@@ -331,6 +361,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       tmem_ld_32x32(tS, v[0]);
       tmem_ld_32x32(tS + 32, v[1]);
       tmem_ld_wait();
+      tc_fence_before();
+      warp_arrive(&s_read[t]);
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int c = 0; c < 2; ++c)
@@ -342,7 +374,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       float* slot = ex + (j & 1) * (4 * kBlockQ);
       slot[half * kBlockQ + r] = mine;
-      named_bar_sync(1 + t, 256);
+      named_bar_sync(1 + t * 4 + quad, 64);          // the two warps of these rows
       float m_new = fmaxf(m, fmaxf(mine, slot[(half ^ 1) * kBlockQ + r]) * sc);   // softmax scale is positive
       if (m_new == -INFINITY) m_new = 0.f;         // fully masked so far: keep everything finite
       const bool grow = (m_new - m) > kRescaleThreshold;   // also true on the first block (m = -inf)
@@ -352,6 +384,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         m = m_cur;
         l2 = mul2(l2, f2(alpha, alpha));
         if (j > 0) {
+          wait_bar_warp(&pv_done[t], (j - 1) & 1, failed, p.wait_limit);
+          tc_fence_after();
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {     // in small pieces: the scores are in registers
             uint32_t o[16];
@@ -376,19 +410,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           l2 = add2(l2, f2(p0, p1));
           pk[i >> 1] = pack16<kBf16>(p0, p1);
         }
-        // packed chunk c -> columns [16c, 16c+16) of this half, whose scores are in registers
-        tmem_st_32x16(tS + c * 16, pk);
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(&p_ready[t * 2 + c]);
+        if (c == 0 && j > 0) {                     // P's columns are free, after the product before
+          wait_bar_warp(&pv_done[t], (j - 1) & 1, failed, p.wait_limit);
+          tc_fence_after();
+        }
+        tmem_st_32x16(tP + c * 16, pk);
       }
+      tmem_st_wait();
+      tc_fence_before();
+      warp_arrive(&p_ready[t]);
     };
 
     // a wait that runs out is noted, not acted on: the halves' warpgroups go on to their exchanges together, and every later wait ends at once
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      wait_bar(&s_full[t], j & 1, failed, p.wait_limit);
-      __syncwarp();
+      wait_bar_warp(&s_full[t], j & 1, failed, p.wait_limit);
       tc_fence_after();
       const int kbase = j * kBlockKV;
       // diagonal block of a causal tile, or the ragged tail of the key sequence
@@ -397,13 +433,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       else block(j, std::false_type{});
     }
     if (n > 0) {
-      ok = wait_bar_warp(&o_done[t], 0, failed, p.wait_limit);
+      ok = wait_bar_warp(&pv_done[t], (n - 1) & 1, failed, p.wait_limit);
       tc_fence_after();
       float la, lb;
       un2(l2, la, lb);
       float* slot = ex + (n & 1) * (4 * kBlockQ);
       slot[half * kBlockQ + r] = la + lb;
-      named_bar_sync(1 + t, 256);
+      named_bar_sync(1 + t * 4 + quad, 64);          // the two warps of these rows
       const float l = slot[r] + slot[kBlockQ + r];
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       const bool valid = qrow < p.sq && ok;
@@ -428,9 +464,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (threadIdx.x == 0) {
       atomicExch(&g_attn_error, 1);
       wait_bar(q_full, 0, &never);
-      for (int i = max(0, nk - kS); i < nk; ++i) wait_bar(&k_full[i % kS], (i / kS) & 1, &never);
-      for (int i = max(0, nv - kS); i < nv; ++i) wait_bar(&v_full[i % kS], (i / kS) & 1, &never);
-    } else if (warp_idx == 1) {
+      for (int i = max(0, n_loaded - kS); i < n_loaded; ++i) wait_bar(&k_full[i % kS], (i / kS) & 1, &never);
+    } else if (warp_idx == 3 && lane == 0) {
+      for (int i = max(0, n_loaded - kS); i < n_loaded; ++i) wait_bar(&v_full[i % kS], (i / kS) & 1, &never);
+    } else if (warp_idx == 1 || warp_idx == 2) {
       if (elect_one()) umma_commit(drained);
       wait_bar_warp(drained, 0, &never);
     } else if (warp_idx >= 4) {
@@ -524,12 +561,14 @@ struct BwdSmem {
 
 // kDQ = false: rows are keys   (X1 = K, X2 = V, Y1 = Q_i, Y2 = dO_i): acc1 = dV, acc2 = dK
 // kDQ = true : rows are queries (X1 = Q, X2 = dO, Y1 = K_j, Y2 = V_j): acc1 = dQ
-// P / dS (16-bit) overwrite the T1 / T2 accumulator columns in TMEM and feed the accumulate MMAs as
-// the TMEM A operand, so the only shared-memory traffic is the operand tiles themselves.
+// P / dS (16-bit) go to TMEM columns of their own and feed the accumulate MMAs as the TMEM A operand, so the only shared-memory
+// traffic is the operand tiles themselves.
 // A block's MMAs take about 1300 cycles (T at N = 64 is bound by its shared-memory reads), its exponentials and products about 2500
 // in one warpgroup: a warp per scheduler that waits on its own results.  So the blocks alternate between two T buffers, the
-// tensor core working on one while the other's P / dS are made, and two warpgroups share a buffer, 32 columns each.
-// CTAs start with the longest rows of a causal problem.  32 / 8 heads x 4096 x 128: dK / dV 405 -> 281 us, dQ 278 -> 231 us.
+// tensor core working on one while the other's P / dS are made, and two warpgroups share a buffer, 32 columns each.  T is in registers
+// 150 cycles after it is complete; its columns then take the next T, so that the math finds it made.  One warp issues T, one the products
+// with P / dS: the waits of either take long enough to empty the tensor core's queue.
+// CTAs start with the longest rows of a causal problem.  32 / 8 heads x 4096 x 128, both kernels: 513 us with P / dS over T, 441 so.
 template <int D, bool kDQ, bool kBf16>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_constant__ CUtensorMap tmap_x2,
@@ -548,9 +587,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   uint64_t* y_full = bars + 1;           // kS
   uint64_t* y_empty = bars + 1 + kS;     // kS
   uint64_t* t_full = bars + 1 + 2 * kS;  // 2
-  uint64_t* pds_ready = t_full + 2;      // 2
-  uint64_t* acc_done = pds_ready + 2;    // 1
-  uint64_t* drained = acc_done + 1;      // 1, after a wait that ran out
+  uint64_t* t_read = t_full + 2;         // 2: T1 and T2 are in registers
+  uint64_t* pds_ready = t_read + 2;      // 2
+  uint64_t* acc_done = pds_ready + 2;    // 2: the P / dS columns are free, the accumulators up to date
+  uint64_t* drained = acc_done + 2;      // 1, after a wait that ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
   volatile int* failed = reinterpret_cast<volatile int*>(bars + 25);
 
@@ -581,9 +621,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   if (threadIdx.x == 0) {
     mbar_init(x_full, 1);
     for (int i = 0; i < kS; ++i) { mbar_init(&y_full[i], 1); mbar_init(&y_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&pds_ready[i], 256); }
-    mbar_init(acc_done, 1);
-    mbar_init(drained, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_read[i], 8); mbar_init(&pds_ready[i], 8); mbar_init(&acc_done[i], 1); }
+    mbar_init(drained, 2);
     *failed = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_x1); tma_prefetch_desc(&tmap_x2); tma_prefetch_desc(&tmap_y1); tma_prefetch_desc(&tmap_y2);
@@ -594,10 +633,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   int n_loaded = 0;                            // thread 0: blocks whose copies it has started
-  const uint32_t tmem_T1 = tmem_base;          // T1[buf] at col buf*64: P overwrites the first half of each 32 cols
-  const uint32_t tmem_T2 = tmem_base + 128;    // T2[buf] at col 128 + buf*64: so does dS
-  const uint32_t tmem_A1 = tmem_base + 256;    // dV or dQ
-  const uint32_t tmem_A2 = tmem_base + 256 + D;  // dK
+  constexpr int kTBufs = kDQ || D == 64 ? 2 : 1;   // T1 and T2 of dK / dV at D = 128 have room for one block
+  const uint32_t tmem_A1 = tmem_base;              // dV or dQ
+  const uint32_t tmem_A2 = tmem_base + D;          // dK
+  const uint32_t tmem_P = tmem_base + (kDQ ? D : 2 * D);   // [buf] at buf*64: 32 columns of P, 32 of dS
+  const uint32_t tmem_T = tmem_P + 128;            // [buf] at buf*128: T1 in 64 columns, T2 in 64
+  static_assert((kDQ ? D : 2 * D) + 128 + kTBufs * 128 <= 512, "TMEM columns");
 
   if (warp_idx < 4) {
     regs_give<kIssueRegs>();
@@ -627,16 +668,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
         }
       }
     } else if (warp_idx == 1 && n_iter > 0) {
-      // ============================================================ MMA issuer
+      // ============================================================ issuer of T1 and T2
       constexpr uint32_t idesc_t = make_idesc_f16(kBf16, kBwdRows, kBwdCols, false, false);
-      constexpr uint32_t idesc_a = make_idesc_f16(kBf16, kBwdRows, D, false, true);
       const uint64_t x_desc = make_smem_desc_sw128(smem_u32(sX1), 1024, 0), y_desc = make_smem_desc_sw128(smem_u32(sY), 1024, 0);
-      // streamed tile as MN-major B (N = d contiguous, K = its 64 rows)
-      const uint64_t yn_desc = make_smem_desc_sw128(smem_u32(sY), 1024, kBwdCols * 128);
-      auto commit = [&](uint64_t* bar) { if (elect_one()) umma_commit(bar); };
-      auto issue_T = [&](int it) {
-        const uint32_t tb = (it & 1) * 64;
-        const uint64_t y1 = desc_at(y_desc, (it % kS) * 2 * L::kY);
+      bool ok = wait_bar_warp(x_full, 0, failed, p.wait_limit);
+      for (int it = 0; it < n_iter && ok; ++it) {
+        const int ys = it % kS, before = it - kTBufs;          // the block before it in its buffer is in registers
+        ok = wait_bar_warp(&y_full[ys], (it / kS) & 1, failed, p.wait_limit) &&
+             (before < 0 || wait_bar_warp(&t_read[before & 1], (before >> 1) & 1, failed, p.wait_limit));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t tT = tmem_T + (kTBufs == 2 ? (it & 1) * 128 : 0);
+        const uint64_t y1 = desc_at(y_desc, ys * 2 * L::kY);
         if (elect_one()) {
 #pragma unroll
           for (int x = 0; x < 2; ++x)
@@ -644,26 +687,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
             for (int k = 0; k < D / 16; ++k) {
               const uint32_t xo = x * (L::kX2Off - L::kX1Off) + (k >> 2) * (kBwdRows * 128) + (k & 3) * 32;
               const uint32_t yo = x * L::kY + (k >> 2) * (kBwdCols * 128) + (k & 3) * 32;
-              umma_f16_ss((x == 0 ? tmem_T1 : tmem_T2) + tb, desc_at(x_desc, xo), desc_at(y1, yo), idesc_t, k != 0 ? 1u : 0u);
+              umma_f16_ss(tT + x * 64, desc_at(x_desc, xo), desc_at(y1, yo), idesc_t, k != 0 ? 1u : 0u);
             }
           umma_commit(&t_full[it & 1]);
         }
-      };
-      bool ok = wait_bar_warp(x_full, 0, failed, p.wait_limit) && wait_bar_warp(&y_full[0], 0, failed, p.wait_limit);
-      if (ok) {
-        tc_fence_after();
-        issue_T(0);
       }
-      for (int it = 0; it < n_iter && ok; ++it) {
+    } else if (warp_idx == 2) {
+      // ============================================================ issuer of the products with P and dS
+      constexpr uint32_t idesc_a = make_idesc_f16(kBf16, kBwdRows, D, false, true);
+      // streamed tile as MN-major B (N = d contiguous, K = its 64 rows)
+      const uint64_t yn_desc = make_smem_desc_sw128(smem_u32(sY), 1024, kBwdCols * 128);
+      for (int it = 0; it < n_iter; ++it) {
         const int ys = it % kS, tb = it & 1;
-        if (it + 1 < n_iter) {
-          ok = wait_bar_warp(&y_full[(it + 1) % kS], ((it + 1) / kS) & 1, failed, p.wait_limit);
-          if (!ok) break;
-          tc_fence_after();
-          issue_T(it + 1);     // overwrites T[(it+1)&1]: its P/dS were consumed by the accumulate MMAs of it-1
-        }
-        ok = wait_bar_warp(&pds_ready[tb], (it >> 1) & 1, failed, p.wait_limit);
-        if (!ok) break;
+        if (!wait_bar_warp(&y_full[ys], (it / kS) & 1, failed, p.wait_limit) ||
+            !wait_bar_warp(&pds_ready[tb], (it >> 1) & 1, failed, p.wait_limit)) break;
         tc_fence_after();
         const uint64_t y1 = desc_at(yn_desc, ys * 2 * L::kY);
         const uint32_t first = it != 0 ? 1u : 0u;
@@ -671,18 +708,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
 #pragma unroll
           for (int k = 0; k < kBwdCols / 16; ++k) {
             // A = P / dS from TMEM (row = lane, 16 k-values = 8 packed 32-bit columns per step)
-            const uint32_t acol = tb * 64 + (k >> 1) * 32 + (k & 1) * 8, acc = k != 0 ? 1u : first;
+            const uint32_t tP = tmem_P + tb * 64 + k * 8, acc = k != 0 ? 1u : first;
             if (kDQ) {
-              umma_f16_ts(tmem_A1, tmem_T2 + acol, desc_at(y1, k * 16 * 128), idesc_a, acc);
+              umma_f16_ts(tmem_A1, tP + 32, desc_at(y1, k * 16 * 128), idesc_a, acc);
             } else {
-              umma_f16_ts(tmem_A1, tmem_T1 + acol, desc_at(y1, L::kY + k * 16 * 128), idesc_a, acc);
-              umma_f16_ts(tmem_A2, tmem_T2 + acol, desc_at(y1, k * 16 * 128), idesc_a, acc);
+              umma_f16_ts(tmem_A1, tP, desc_at(y1, L::kY + k * 16 * 128), idesc_a, acc);
+              umma_f16_ts(tmem_A2, tP + 32, desc_at(y1, k * 16 * 128), idesc_a, acc);
             }
           }
+          umma_commit(&acc_done[tb]);
           umma_commit(&y_empty[ys]);
         }
       }
-      if (ok) commit(acc_done);
     }
   } else {
     // ============================================================ P / dS math + epilogue
@@ -700,7 +737,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
       row_nlse = f2(p.nlse[idx], p.nlse[idx]);     // already in the exp2 domain (-inf for fully masked rows)
       row_ndelta = f2(p.ndelta[idx], p.ndelta[idx]);
     }
-    const uint32_t a1 = tmem_T1 + tb * 64 + half * 32 + lane_addr, a2 = tmem_T2 + tb * 64 + half * 32 + lane_addr;
+    const uint32_t a1 = tmem_T + (kTBufs == 2 ? tb * 128 : 0) + half * 32 + lane_addr, a2 = a1 + 64;
+    const uint32_t tP = tmem_P + tb * 64 + half * 16 + lane_addr;
     // one streamed block: P = exp2(T1 * scale - lse2), dS = P * (T2 - delta), written back to TMEM
     auto block = [&](int it, int c0, auto masked_tag) {
       constexpr bool kMasked = decltype(masked_tag)::value;
@@ -712,6 +750,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
       tmem_ld_32x16(a1 + 16, t1[1]);
       tmem_ld_32x16(a2 + 16, t2[1]);
       tmem_ld_wait();
+      tc_fence_before();
+      warp_arrive(&t_read[tb]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t pk[8], dk[8];
@@ -740,13 +780,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
             dk[i >> 1] = pack16<kBf16>(d0, d1);
           }
         }
-        // packed chunk c -> columns [8c, 8c+8) of this half, whose fp32 values are in registers
-        tmem_st_32x8(a2 + c * 8, dk);
-        if (!kDQ) tmem_st_32x8(a1 + c * 8, pk);
+        if (c == 0 && it >= 2) {                           // this buffer's P / dS have been multiplied
+          wait_bar_warp(&acc_done[tb], ((it >> 1) - 1) & 1, failed, p.wait_limit);
+          tc_fence_after();
+        }
+        tmem_st_32x8(tP + 32 + c * 8, dk);
+        if (!kDQ) tmem_st_32x8(tP + c * 8, pk);
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&pds_ready[tb]);
+      warp_arrive(&pds_ready[tb]);
     };
     bool ok = true;
     for (int it = tb; it < n_iter; it += 2) {
@@ -761,7 +804,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
       if (need_mask) block(it, c0, std::true_type{});
       else block(it, c0, std::false_type{});
     }
-    if (n_iter > 0 && ok) ok = wait_bar_warp(acc_done, 0, failed, p.wait_limit);
+    // the products of this buffer's last block, then of the last one: a barrier is never more than one phase ahead of a wait
+    for (int it = max(0, n_iter - 2); it < n_iter; ++it)
+      if (ok && (it == n_iter - 1 || (it & 1) == tb)) ok = wait_bar_warp(&acc_done[it & 1], (it >> 1) & 1, failed, p.wait_limit);
     if (ok) {
       tc_fence_after();
       const int limit = kDQ ? p.sq : p.sk;
@@ -795,7 +840,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
       atomicExch(&g_attn_error, 1);
       wait_bar(x_full, 0, &never);
       for (int i = max(0, n_loaded - kS); i < n_loaded; ++i) wait_bar(&y_full[i % kS], (i / kS) & 1, &never);
-    } else if (warp_idx == 1) {
+    } else if (warp_idx == 1 || warp_idx == 2) {
       if (elect_one()) umma_commit(drained);
       wait_bar_warp(drained, 0, &never);
     } else if (warp_idx >= 4) {
