@@ -126,6 +126,10 @@ __device__ __forceinline__ void tma_reduce_add_2d(const void* tmap, const void* 
       ::"l"(tmap), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
       : "memory");
 }
+// 16 bytes to a shared-memory address
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // 1-D bulk copies (TMA engine, no tensor map): gmem -> smem with mbarrier completion, smem -> gmem
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   asm volatile(

@@ -36,6 +36,7 @@
 //                 offsets array; fp32 TMA reduce-add into main_grad.
 #include "b200_api.h"
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 
 #include <mutex>
 #include <string>
@@ -156,10 +157,6 @@ __device__ __forceinline__ void tmem_alloc2(uint32_t* smem_dst) {
 template <uint32_t kCols>
 __device__ __forceinline__ void tmem_dealloc2(uint32_t taddr) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kCols) : "memory");
-}
-
-__device__ __forceinline__ float gelu2(float x) {
-  return 0.5f * x * (1.f + tanhf(0.79788456f * x * (1.f + 0.044715f * x * x)));
 }
 
 // One unit of work of a CTA pair.  Every role (producer / MMA / epilogue) of both CTAs derives it from the tile index
@@ -367,10 +364,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     }
     mbar_fence_init();
   }
-  cluster_sync_all();                    // peer barriers are initialised before any remote arrive
   if (warp_idx == 2) tmem_alloc2<2 * BN>(tmem_ptr_smem);
   tc_fence_before();
-  __syncthreads();
+  cluster_sync_all();                    // peer barriers are initialised before any remote arrive, the accumulators allocated
   tc_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
   constexpr uint32_t kPairStageBytes = 2 * (L::kA + L::kB);
@@ -499,7 +495,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     const int row_in_tile = ew * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
-    int cbuf = 0;
+    [[maybe_unused]] int cbuf = 0;
+    [[maybe_unused]] Slabs slabs(lane);
     uint32_t* pending_flag = nullptr;   // RS: flag of the previous pushed tile, not yet published
     for (int tile = cluster_id; tile < num_tiles; tile += n_clusters) {
       const Tile2 t = tile_info<kMode>(p, tile);
@@ -534,10 +531,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           named_bar_sync(3, kEpiThreads);
         }
       }
-      if (!empty) {
-        mbar_wait(&tmem_full_bar[acc], acc_phase);
-        tc_fence_after();
-      }
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + acc * BN;
       float rscale = 1.f;
       if constexpr (kMode == kModeGroupM) {
@@ -547,56 +540,91 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       if constexpr (kMode == kModeGroupM) {
         if (bias_base != nullptr) bias_base += static_cast<size_t>(t.group) * p.N;
       }
-#pragma unroll 1
-      for (int c = 0; c < BN / 64; ++c) {
-        uint32_t v0[32], v1[32];
+      if constexpr (kMode != kModeRS) {
+        const int n0 = n_blk * BN, n_chunks = min(BN, p.N - n0 + 63) / 64;
+        slabs.at(smem_c + ew * (kCBufs * kSlabBytes), (kMode == kModeGroupK ? t.group * p.group_stride : 0) + m0 + ew * 32, m0 + ew * 32 < p.M);
+        const uint16_t* bias = kEpi == kEpiStore16 ? bias_base : nullptr;
+        uint32_t bias_next = bias_pair(bias, n0, p.N, lane);   // loaded a slab ahead
         if (!empty) {
+          mbar_wait(&tmem_full_bar[acc], acc_phase);
+          __syncwarp();
+          tc_fence_after();
+        }
+#pragma unroll 1
+        for (int c = 0; c < n_chunks; ++c) {
+          uint32_t v0[32], v1[32];
+          if (!empty) {
+            tmem_ld_32x32(taddr + c * 64, v0);
+            tmem_ld_32x32(taddr + c * 64 + 32, v1);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v0[i] = v1[i] = 0u;
+          }
+          if (c == n_chunks - 1 && !empty) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if (leader) mbar_arrive(&tmem_empty_bar[acc]);
+              else mbar_arrive_remote(&tmem_empty_bar[acc], 0);
+            }
+          }
+          const int gcol0 = n0 + c * 64;
+          if constexpr (kEpi == kEpiStore16) {
+            const uint32_t bias2 = bias_next;
+            if (c + 1 < n_chunks) bias_next = bias_pair(bias, gcol0 + 64, p.N, lane);
+            if (p.D_pre != nullptr) slabs.store16<false>(&tmap_d_pre, gcol0, p.is_bf16 != 0, false, bias != nullptr, v0, v1, bias2, 1.f);
+            slabs.store16<kMode == kModeGroupM>(&tmap_d, gcol0, p.is_bf16 != 0, p.act == 1, bias != nullptr, v0, v1, bias2, rscale);
+          } else {
+            slabs.store32<kEpi == kEpiAccumF32>(&tmap_d, gcol0, v0);
+            slabs.store32<kEpi == kEpiAccumF32>(&tmap_d, gcol0 + 32, v1);
+          }
+        }
+      } else {
+        mbar_wait(&tmem_full_bar[acc], acc_phase);
+        tc_fence_after();
+#pragma unroll 1
+        for (int c = 0; c < BN / 64; ++c) {
+          uint32_t v0[32], v1[32];
           tmem_ld_32x32(taddr + c * 64, v0);
           tmem_ld_32x32(taddr + c * 64 + 32, v1);
           tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v0[i] = v1[i] = 0u;
-        }
-        if (c == BN / 64 - 1 && !empty) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (leader) mbar_arrive(&tmem_empty_bar[acc]);
-            else mbar_arrive_remote(&tmem_empty_bar[acc], 0);
+          if (c == BN / 64 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if (leader) mbar_arrive(&tmem_empty_bar[acc]);
+              else mbar_arrive_remote(&tmem_empty_bar[acc], 0);
+            }
           }
-        }
-        const int gcol0 = n_blk * BN + c * 64;
-        if constexpr (kEpi == kEpiStore16 || kEpi == kEpiReduceScatter) {
+          const int gcol0 = n_blk * BN + c * 64;
           float f[64];
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             f[i] = __uint_as_float(v0[i]);
             f[32 + i] = __uint_as_float(v1[i]);
           }
-          if constexpr (kMode == kModeRS) {
-            if (own) {
-              // fold the reduction in: partials of the tp-1 peers for this row, bf16 in this rank's staging
-              const uint16_t* stage_base = reinterpret_cast<const uint16_t*>(p.peer_buf[p.tp_rank]);
-              for (int s = 0; s < p.tp_size; ++s) {
-                if (s == p.tp_rank) continue;
-                const uint16_t* src = stage_base +
-                                      (static_cast<size_t>(s) * p.rows_per_rank + lrow0 + row_in_tile) * p.N + gcol0;
-                int4 raw[8];
+          if (own) {
+            // fold the reduction in: partials of the tp-1 peers for this row, bf16 in this rank's staging
+            const uint16_t* stage_base = reinterpret_cast<const uint16_t*>(p.peer_buf[p.tp_rank]);
+            for (int s = 0; s < p.tp_size; ++s) {
+              if (s == p.tp_rank) continue;
+              const uint16_t* src = stage_base +
+                                    (static_cast<size_t>(s) * p.rows_per_rank + lrow0 + row_in_tile) * p.N + gcol0;
+              int4 raw[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  if (gcol0 + j * 8 < p.N) raw[j] = ld_cg_v4(reinterpret_cast<const int4*>(src + j * 8));
-                  else raw[j] = make_int4(0, 0, 0, 0);
-                }
+              for (int j = 0; j < 8; ++j) {
+                if (gcol0 + j * 8 < p.N) raw[j] = ld_cg_v4(reinterpret_cast<const int4*>(src + j * 8));
+                else raw[j] = make_int4(0, 0, 0, 0);
+              }
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  const uint32_t* uu = reinterpret_cast<const uint32_t*>(&raw[j]);
+              for (int j = 0; j < 8; ++j) {
+                const uint32_t* uu = reinterpret_cast<const uint32_t*>(&raw[j]);
 #pragma unroll
-                  for (int q = 0; q < 4; ++q) {
-                    float2 f2 = p.is_bf16 ? unpack_bf16x2(uu[q]) : __half22float2(*reinterpret_cast<const __half2*>(&uu[q]));
-                    f[j * 8 + 2 * q] += f2.x;
-                    f[j * 8 + 2 * q + 1] += f2.y;
-                  }
+                for (int q = 0; q < 4; ++q) {
+                  float2 f2 = p.is_bf16 ? unpack_bf16x2(uu[q]) : __half22float2(*reinterpret_cast<const __half2*>(&uu[q]));
+                  f[j * 8 + 2 * q] += f2.x;
+                  f[j * 8 + 2 * q + 1] += f2.y;
                 }
               }
             }
@@ -613,62 +641,32 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
               }
             }
           }
-          const int n_out = (kMode != kModeRS && p.D_pre != nullptr) ? 2 : 1;
-          for (int o = 0; o < n_out; ++o) {
-            const bool pre = (n_out == 2 && o == 0);
-            if (epi_tid == 0) tma_store_wait_read<kCBufs - 1>();
-            named_bar_sync(1, kEpiThreads);
-            uint8_t* sc = smem_c + cbuf * L::kC + row_in_tile * 128;
+          if (epi_tid == 0) tma_store_wait_read<kCBufs - 1>();
+          named_bar_sync(1, kEpiThreads);
+          uint8_t* sc = smem_c + cbuf * L::kC + row_in_tile * 128;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              uint32_t pk[4];
+          for (int j = 0; j < 8; ++j) {
+            uint32_t pk[4];
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                float a = f[j * 8 + 2 * q], b = f[j * 8 + 2 * q + 1];
-                if (!pre && p.act == 1) { a = gelu2(a); b = gelu2(b); }
-                if constexpr (kMode == kModeGroupM) { if (!pre) { a *= rscale; b *= rscale; } }
-                if (p.is_bf16) pk[q] = pack_bf16x2(a, b);
-                else {
-                  __half2 h = __floats2half2_rn(a, b);
-                  pk[q] = *reinterpret_cast<uint32_t*>(&h);
-                }
+            for (int q = 0; q < 4; ++q) {
+              float a = f[j * 8 + 2 * q], b = f[j * 8 + 2 * q + 1];
+              if (p.act == 1) { a = gelu_tanh(a); b = gelu_tanh(b); }
+              if (p.is_bf16) pk[q] = pack_bf16x2(a, b);
+              else {
+                __half2 h = __floats2half2_rn(a, b);
+                pk[q] = *reinterpret_cast<uint32_t*>(&h);
               }
-              *reinterpret_cast<uint4*>(sc + ((j ^ (row_in_tile & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             }
-            fence_proxy_async_smem();
-            named_bar_sync(2, kEpiThreads);
-            if (epi_tid == 0) {
-              if constexpr (kMode == kModeRS) {
-                if (own) tma_store_2d(&tmap_d, smem_c + cbuf * L::kC, gcol0, lrow0);
-                else tma_store_2d(&peer_maps.m[owner], smem_c + cbuf * L::kC, gcol0, p.tp_rank * p.rows_per_rank + lrow0);
-              } else {
-                tma_store_2d(pre ? &tmap_d_pre : &tmap_d, smem_c + cbuf * L::kC, gcol0, m0);
-              }
-              tma_store_commit();
-            }
-            if (++cbuf == kCBufs) cbuf = 0;
+            *reinterpret_cast<uint4*>(sc + ((j ^ (row_in_tile & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
           }
-        } else {
-          const int drow0 = (kMode == kModeGroupK) ? t.group * p.group_stride + m0 : m0;
-#pragma unroll
-          for (int hseg = 0; hseg < 2; ++hseg) {
-            const uint32_t* v = hseg == 0 ? v0 : v1;
-            if (epi_tid == 0) tma_store_wait_read<kCBufs - 1>();
-            named_bar_sync(1, kEpiThreads);
-            uint8_t* sc = smem_c + cbuf * L::kC + row_in_tile * 128;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<uint4*>(sc + ((j ^ (row_in_tile & 7)) << 4)) =
-                  make_uint4(v[j * 4], v[j * 4 + 1], v[j * 4 + 2], v[j * 4 + 3]);
-            fence_proxy_async_smem();
-            named_bar_sync(2, kEpiThreads);
-            if (epi_tid == 0) {
-              if constexpr (kEpi == kEpiAccumF32) tma_reduce_add_2d(&tmap_d, smem_c + cbuf * L::kC, gcol0 + hseg * 32, drow0);
-              else tma_store_2d(&tmap_d, smem_c + cbuf * L::kC, gcol0 + hseg * 32, drow0);
-              tma_store_commit();
-            }
-            if (++cbuf == kCBufs) cbuf = 0;
+          fence_proxy_async_smem();
+          named_bar_sync(2, kEpiThreads);
+          if (epi_tid == 0) {
+            if (own) tma_store_2d(&tmap_d, smem_c + cbuf * L::kC, gcol0, lrow0);
+            else tma_store_2d(&peer_maps.m[owner], smem_c + cbuf * L::kC, gcol0, p.tp_rank * p.rows_per_rank + lrow0);
+            tma_store_commit();
           }
+          if (++cbuf == kCBufs) cbuf = 0;
         }
       }
       if constexpr (kMode == kModeRS) {
@@ -690,7 +688,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       }
       if (!empty && ++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
-    if (epi_tid == 0) {
+    if (kMode == kModeRS ? epi_tid == 0 : lane == 0) {
       tma_store_wait_all<0>();
       if constexpr (kMode == kModeRS) {
         if (pending_flag != nullptr) {
@@ -702,7 +700,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   }
 
   tc_fence_before();
-  __syncthreads();
   cluster_sync_all();        // both CTAs are done with TMEM and with each other's barriers
   if (warp_idx == 2) {
     tc_fence_after();
@@ -895,15 +892,15 @@ int gemm2_bf16(const GemmArgs& a) {
   if (!a.b_mn_major) ok = ok && tmap2(&tb, a.B, dt, a.K, static_cast<uint64_t>(a.N) * b_groups, a.ldb, BK, BN / 2);
   else ok = ok && tmap2(&tb, a.B, dt, a.N, static_cast<uint64_t>(a.K) * b_groups, a.ldb, 64, BK);
   if (a.epilogue == kEpiStore16) {
-    ok = ok && tmap2(&td, a.D, dt, a.N, a.M, a.ldd, 64, BM);
-    if (a.D_pre) ok = ok && tmap2(&tdp, a.D_pre, dt, a.N, a.M, a.ldd, 64, BM);
+    ok = ok && tmap2(&td, a.D, dt, a.N, a.M, a.ldd, 64, kSlabRows);
+    if (a.D_pre) ok = ok && tmap2(&tdp, a.D_pre, dt, a.N, a.M, a.ldd, 64, kSlabRows);
     else tdp = td;
   } else if (a.epilogue == kEpiReduceScatter) {
     ok = ok && tmap2(&td, a.D, dt, a.N, p.rows_per_rank, a.ldd, 64, BM);
     tdp = td;
   } else {
     const uint64_t d_rows = (mode == kModeGroupK) ? static_cast<uint64_t>(a.n_groups) * a.group_stride : a.M;
-    ok = ok && tmap2(&td, a.D, 2, a.N, d_rows, a.ldd, 32, BM);
+    ok = ok && tmap2(&td, a.D, 2, a.N, d_rows, a.ldd, 32, kSlabRows);
     tdp = td;
   }
   if (!ok) return -5;

@@ -22,6 +22,7 @@
 //                       reducer for the rows this rank owns (fixed src order => deterministic).
 #include "b200_api.h"
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 
 #include <mutex>
 #include <string>
@@ -66,12 +67,6 @@ struct DevParams {
 struct PeerMaps {
   CUtensorMap m[kMaxPeers];
 };
-
-__device__ __forceinline__ float gelu_tanh(float x) {
-  const float k0 = 0.79788456f, k1 = 0.044715f;
-  float inner = k0 * x * (1.f + k1 * x * x);
-  return 0.5f * x * (1.f + tanhf(inner));
-}
 
 template <int BLOCK_N, int kStages>
 struct SmemLayout {
@@ -364,22 +359,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     const int row_in_tile = ew * 32 + lane;
     int acc = 0;
     uint32_t acc_phase = 0;
-    int cbuf = 0;
+    [[maybe_unused]] int cbuf = 0;
+    [[maybe_unused]] Slabs slabs(lane);
     uint32_t* pending_flag = nullptr;   // reduce-scatter: flag of the previous tile, not yet published
     for (int tile = cta; tile < num_tiles; tile += n_ctas) {
       int m_blk, n_blk;
       tile_coords(p, tile, m_blk, n_blk);
+      const int n0 = n_blk * BLOCK_N, n_chunks = kEpi == kEpiReduceScatter ? BLOCK_N / 64 : min(BLOCK_N, p.N - n0 + 63) / 64;
+      slabs.at(smem_c + ew * (2 * kSlabBytes), m_blk * BLOCK_M + ew * 32, m_blk * BLOCK_M + ew * 32 < p.M);
+      const uint16_t* bias = kEpi == kEpiStore16 ? reinterpret_cast<const uint16_t*>(p.bias) : nullptr;
+      uint32_t bias_next = bias_pair(bias, n0, p.N, lane);       // loaded a slab ahead
       mbar_wait(&tmem_full_bar[acc], acc_phase);
+      __syncwarp();
       tc_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + acc * BLOCK_N;
-      const int grow = m_blk * BLOCK_M + row_in_tile;
 #pragma unroll 1
-      for (int c = 0; c < BLOCK_N / 64; ++c) {
+      for (int c = 0; c < n_chunks; ++c) {
         uint32_t v0[32], v1[32];
         tmem_ld_32x32(taddr + c * 64, v0);
         tmem_ld_32x32(taddr + c * 64 + 32, v1);
         tmem_ld_wait();
-        if (c == BLOCK_N / 64 - 1) {
+        if (c == n_chunks - 1) {
           // accumulator fully drained into registers: hand TMEM back to the MMA warp
           tc_fence_before();
           __syncwarp();
@@ -387,86 +387,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
         const int gcol0 = n_blk * BLOCK_N + c * 64;
         if constexpr (kEpi == kEpiStore16) {
-          float f[64];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            f[i] = __uint_as_float(v0[i]);
-            f[32 + i] = __uint_as_float(v1[i]);
-          }
-          if (p.bias != nullptr) {
-            const uint32_t* b32 = reinterpret_cast<const uint32_t*>(
-                reinterpret_cast<const uint16_t*>(p.bias) + gcol0);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (gcol0 + 2 * i < p.N) {
-                uint32_t bb = __ldg(b32 + i);
-                float2 bf;
-                if (p.is_bf16) bf = unpack_bf16x2(bb);
-                else bf = __half22float2(*reinterpret_cast<__half2*>(&bb));
-                f[2 * i] += bf.x;
-                f[2 * i + 1] += bf.y;
-              }
-            }
-          }
-          const int n_out = (p.D_pre != nullptr) ? 2 : 1;
-          for (int o = 0; o < n_out; ++o) {
-            const bool pre = (n_out == 2 && o == 0);
-            // staging buffer cbuf was last read by the TMA store issued two chunks ago
-            if (epi_tid == 0) tma_store_wait_read<1>();
-            named_bar_sync(1, kNumEpiThreads);
-            uint8_t* sc = smem_c + cbuf * L::kCBytes + row_in_tile * 128;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              uint32_t pk[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                float a = f[j * 8 + 2 * q], b = f[j * 8 + 2 * q + 1];
-                if (!pre && p.act == 1) { a = gelu_tanh(a); b = gelu_tanh(b); }
-                if (p.is_bf16) pk[q] = pack_bf16x2(a, b);
-                else {
-                  __half2 h = __floats2half2_rn(a, b);
-                  pk[q] = *reinterpret_cast<uint32_t*>(&h);
-                }
-              }
-              // 128B swizzle: 16-byte chunk j of row r lives at chunk (j ^ (r & 7))
-              *reinterpret_cast<uint4*>(sc + ((j ^ (row_in_tile & 7)) << 4)) =
-                  make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            }
-            fence_proxy_async_smem();
-            named_bar_sync(2, kNumEpiThreads);
-            if (epi_tid == 0) {
-              tma_store_2d(pre ? &tmap_d_pre : &tmap_d, smem_c + cbuf * L::kCBytes, gcol0,
-                           m_blk * BLOCK_M);
-              tma_store_commit();
-            }
-            cbuf ^= 1;
-          }
+          const uint32_t bias2 = bias_next;
+          if (c + 1 < n_chunks) bias_next = bias_pair(bias, gcol0 + 64, p.N, lane);
+          if (p.D_pre != nullptr) slabs.store16<false>(&tmap_d_pre, gcol0, p.is_bf16 != 0, false, bias != nullptr, v0, v1, bias2, 1.f);
+          slabs.store16<false>(&tmap_d, gcol0, p.is_bf16 != 0, p.act == 1, bias != nullptr, v0, v1, bias2, 1.f);
         } else if constexpr (kEpi == kEpiAccumF32 || kEpi == kEpiStoreF32) {
-          // fp32 tile -> smem (two 32-column halves, 128B-swizzled) -> TMA store / TMA reduce-add.
-          // The "+=" happens in L2 (cp.reduce.async.bulk.tensor .add), so no main_grad read
-          // round trip stalls the epilogue warps.
-#pragma unroll
-          for (int hseg = 0; hseg < 2; ++hseg) {
-            const uint32_t* v = hseg == 0 ? v0 : v1;
-            if (epi_tid == 0) tma_store_wait_read<1>();
-            named_bar_sync(1, kNumEpiThreads);
-            uint8_t* sc = smem_c + cbuf * L::kCBytes + row_in_tile * 128;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              *reinterpret_cast<uint4*>(sc + ((j ^ (row_in_tile & 7)) << 4)) =
-                  make_uint4(v[j * 4], v[j * 4 + 1], v[j * 4 + 2], v[j * 4 + 3]);
-            }
-            fence_proxy_async_smem();
-            named_bar_sync(2, kNumEpiThreads);
-            if (epi_tid == 0) {
-              if constexpr (kEpi == kEpiAccumF32)
-                tma_reduce_add_2d(&tmap_d, smem_c + cbuf * L::kCBytes, gcol0 + hseg * 32, m_blk * BLOCK_M);
-              else
-                tma_store_2d(&tmap_d, smem_c + cbuf * L::kCBytes, gcol0 + hseg * 32, m_blk * BLOCK_M);
-              tma_store_commit();
-            }
-            cbuf ^= 1;
-          }
+          // The "+=" happens in L2 (cp.reduce.async.bulk.tensor .add), so no main_grad read round trip stalls the epilogue warps.
+          slabs.store32<kEpi == kEpiAccumF32>(&tmap_d, gcol0, v0);
+          slabs.store32<kEpi == kEpiAccumF32>(&tmap_d, gcol0 + 32, v1);
         } else {  // kEpiReduceScatter: partial tile -> owner's staging buffer [src][rows_per_rank][N]
           // Same swizzled-smem staging as the plain store epilogue, but the TMA store targets the
           // owner's arena over NVLink: the epilogue warps never wait on a remote write.
@@ -519,7 +447,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
     if constexpr (kEpi == kEpiStore16 || kEpi == kEpiAccumF32 || kEpi == kEpiStoreF32) {
-      if (epi_tid == 0) tma_store_wait_all<0>();
+      if (lane == 0) tma_store_wait_all<0>();
     }
     if constexpr (kEpi == kEpiReduceScatter) {
       if (epi_tid == 0) {
@@ -820,11 +748,11 @@ int gemm_bf16(const GemmArgs& a) {
   if (!a.b_mn_major) ok = ok && make_tmap_2d(&tb, a.B, a.is_bf16, a.K, a.N, a.ldb, BLOCK_K, block_n);
   else ok = ok && make_tmap_2d(&tb, a.B, a.is_bf16, a.N, a.K, a.ldb, 64, BLOCK_K);
   if (a.epilogue == kEpiStore16) {
-    ok = ok && make_tmap_2d(&td, a.D, a.is_bf16, a.N, a.M, a.ldd, 64, BLOCK_M);
-    if (a.D_pre) ok = ok && make_tmap_2d(&tdp, a.D_pre, a.is_bf16, a.N, a.M, a.ldd, 64, BLOCK_M);
+    ok = ok && make_tmap_2d(&td, a.D, a.is_bf16, a.N, a.M, a.ldd, 64, kSlabRows);
+    if (a.D_pre) ok = ok && make_tmap_2d(&tdp, a.D_pre, a.is_bf16, a.N, a.M, a.ldd, 64, kSlabRows);
     else tdp = td;
   } else if (a.epilogue == kEpiAccumF32 || a.epilogue == kEpiStoreF32) {
-    ok = ok && make_tmap_2d(&td, a.D, a.is_bf16, a.N, a.M, a.ldd, 32, BLOCK_M, /*is_f32=*/true);
+    ok = ok && make_tmap_2d(&td, a.D, a.is_bf16, a.N, a.M, a.ldd, 32, kSlabRows, /*is_f32=*/true);
     tdp = td;
   } else { td = ta; tdp = ta; }
   if (!ok) return -5;
