@@ -338,10 +338,10 @@ struct PagedWriteArgs {
   int n_tokens, ng, head_dim;
 };
 bool paged_attention_supported(int head_dim, int group);
-void paged_write(const PagedWriteArgs& w, cudaStream_t s);
+void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cudaStream_t s);
 int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
 bool paged_decode_by_rows(const PagedAttnArgs& a);        // which of the two decode kernels
-int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s);
+int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s);
 const char* paged_attention_last_error();
 
 // ---------------------------------------------------------------- MoE (moe.cu)

@@ -953,18 +953,6 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
   TORCH_CHECK(tok_req.numel() >= T && tok_len.numel() >= T, "tok_req / tok_len must cover every token");
   TORCH_CHECK(np % ng == 0 && k_cache.size(2) == d && b200::paged_attention_supported(d, np / ng), "unsupported paged attention shape");
   for (const Tensor* t : {&q, &k_cache, &v_cache}) TORCH_CHECK(reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "operands must be 16-byte aligned");
-  if (k_new.has_value() && T > 0) {
-    TORCH_CHECK(v_new.has_value() && slots.has_value() && slots->scalar_type() == at::kLong && slots->is_contiguous() && slots->numel() == T);
-    b200::PagedWriteArgs w{};
-    for (const Tensor* t : {&*k_new, &*v_new})
-      TORCH_CHECK(t->dim() == 3 && t->size(0) == T && t->size(1) == ng && t->size(2) == d && t->scalar_type() == q.scalar_type() && t->stride(2) == 1 &&
-                  t->stride(0) % 8 == 0 && t->stride(1) % 8 == 0 && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "bad new keys or values");
-    w.k = k_new->data_ptr(); w.v = v_new->data_ptr(); w.k_cache = k_cache.data_ptr(); w.v_cache = v_cache.data_ptr();
-    w.slots = slots->data_ptr<int64_t>(); w.k_st = k_new->stride(0); w.k_sh = k_new->stride(1); w.v_st = v_new->stride(0); w.v_sh = v_new->stride(1);
-    w.n_tokens = T; w.ng = ng; w.head_dim = d;
-    b200::paged_write(w, cur_stream());
-    count();
-  }
   auto out = at::empty_like(q);
   b200::PagedAttnArgs a{};
   a.q = q.data_ptr(); a.k_cache = k_cache.data_ptr(); a.v_cache = v_cache.data_ptr(); a.out = out.data_ptr();
@@ -978,13 +966,25 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
     a.decode_len = static_cast<int>(decode_len); a.decode_mean = static_cast<int>(decode_mean); a.decode_single = decode_single;
   }
   if (T == 0) return out;
-  const bool decode = !cu.has_value() || splits > 0;
+  const bool decode = !cu.has_value() || splits > 0, written = k_new.has_value();
   Tensor ws;
   if (decode) ws = at::empty({b200::paged_decode_workspace(a)}, q.options().dtype(at::kFloat));
-  const int rc = b200::paged_attention(a, decode, static_cast<int>(chunk_tiles), static_cast<int>(chunk_splits), decode ? ws.data_ptr<float>() : nullptr,
-                                       cur_stream());
+  float* ws_ptr = decode && ws.numel() > 0 ? ws.data_ptr<float>() : nullptr;
+  if (written) {
+    TORCH_CHECK(v_new.has_value() && slots.has_value() && slots->scalar_type() == at::kLong && slots->is_contiguous() && slots->numel() == T);
+    b200::PagedWriteArgs w{};
+    for (const Tensor* t : {&*k_new, &*v_new})
+      TORCH_CHECK(t->dim() == 3 && t->size(0) == T && t->size(1) == ng && t->size(2) == d && t->scalar_type() == q.scalar_type() && t->stride(2) == 1 &&
+                  t->stride(0) % 8 == 0 && t->stride(1) % 8 == 0 && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "bad new keys or values");
+    w.k = k_new->data_ptr(); w.v = v_new->data_ptr(); w.k_cache = k_cache.data_ptr(); w.v_cache = v_cache.data_ptr();
+    w.slots = slots->data_ptr<int64_t>(); w.k_st = k_new->stride(0); w.k_sh = k_new->stride(1); w.v_st = v_new->stride(0); w.v_sh = v_new->stride(1);
+    w.n_tokens = T; w.ng = ng; w.head_dim = d;
+    b200::paged_write(w, a, ws_ptr, cur_stream());
+    count();
+  }
+  const int rc = b200::paged_attention(a, decode, static_cast<int>(chunk_tiles), static_cast<int>(chunk_splits), ws_ptr, written, cur_stream());
   TORCH_CHECK(rc == 0, "b200 paged_attention failed: ", rc, " ", b200::paged_attention_last_error());
-  count((decode ? (ws.numel() > 0 ? 2 : 1) : 0) + (cu.has_value() && chunk_tiles > 0 ? 1 : 0));
+  count((decode ? 1 : 0) + (cu.has_value() && chunk_tiles > 0 ? 1 : 0));
   return out;
 }
 bool paged_attention_supported(int64_t head_dim, int64_t group) { return b200::paged_attention_supported(static_cast<int>(head_dim), static_cast<int>(group)); }

@@ -12,9 +12,10 @@
 // up to it (fp16: to 2^-40 of the largest weight where it is below 2^-16 of that).
 //   rows = 16 (decode, short chunks): the four warps take 16 keys of a stage each, bound by HBM.  The stages of all (request, KV head)
 //     pairs stand in one line that is cut evenly over three CTAs per SM, whatever the contexts' lengths; an item that a cut falls into
-//     leaves partial (max, sum, accumulator) triples, which a small second kernel merges.  64 contexts of 1k to 4k, 32 / 8 heads of 128:
-//     120 us, 5.6 TB/s, the rest latency of one stage's dependent steps (138 with three stages and two CTAs per SM; 456 with a key per 16
-//     lanes and no load in flight behind it).  Many short contexts with few heads a group go by rows instead, see paged_rows_kernel.
+//     leaves partial (max, sum, accumulator) triples, and the CTA that counts the last of them puts them together.  What a CTA needs to know before its
+//     first key (a request per thread) is read while the new keys are still being written.  64 contexts of 1k to 4k, 32 / 8 heads of 128:
+//     128 us with the write, 134 with a kernel of its own for the parts; one of 12000: 24 and 29, of 500: 17 and 22 (138 for the former's
+//     decode alone with three stages and two CTAs per SM; 456 with a key per 16 lanes and no load in flight behind it).  Many short contexts with few heads a group go by rows instead, see paged_rows_kernel.
 //   rows = 64 (chunks): a warp takes 16 rows and all keys of a stage, longest tiles first, bound by the tensor instructions.  Where the
 //     tiles are few and the context is long, the CTAs of a cluster take key ranges and merge through distributed shared memory.  Two
 //     chunks of 500 tokens beside 24 decoding requests: 865 us before, every token reading all its keys, 67 + 40 us now (57 + 39 when the
@@ -74,7 +75,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 // Launches of a step overlap: every kernel lets the next one start once all its own CTAs run, and waits for the one before where it reads
-// what that wrote: the write kernel's rows (the first of the others), the decode parts (merge).  The decode kernel beside chunks reads
+// what that wrote: the write kernel's rows and zeroed counters (the first of the others).  The decode kernel beside chunks reads
 // nothing of theirs, and what both read was complete before the first began: it waits before its end, which keeps the stream's order
 // for what follows.
 __device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -100,7 +101,9 @@ struct PagedParams {
   bool beside_chunks;          // decode: the launch before is the chunks'
   float row_scale;             // rows kernel: the scale as it was given
   uint32_t q_keep, q_sign;     // tiles: the kernels' running maxima want a positive scale: queries are negated for a negative one, zeros for zero
+  bool behind_write;           // the launch before is the write of this call's keys, before which all else that is read was complete
   float* ws;                   // decode: two partials of 16 rows x (d + 2) per CTA
+  int* arrived;                // decode: parts of each (request, KV head) that are in ws, zero at the start
 };
 
 // One tile's keys k0 .. k1 - 1 (stages aligned to k0): running maximum, sum and accumulator of this warp's rows g and g + 8.  RW row
@@ -366,21 +369,6 @@ __device__ __forceinline__ Item decode_item(const PagedParams& p, int r) {
   it.stages = it.n > 0 ? max(1, (it.max_vis + kStageKeys - 1) / kStageKeys) : 0;      // a request without keys still gets its zeros written
   return it;
 }
-// one warp: the stages of all requests, and of those before request `upto`
-__device__ __forceinline__ void count_stages(const PagedParams& p, int upto, int& total, int& before) {
-  const int lane = threadIdx.x & 31;
-  total = before = 0;
-  for (int r = lane; r < p.n_tiles; r += 32) {
-    const int s = decode_item(p, r).stages;
-    total += s;
-    if (r < upto) before += s;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    total += __shfl_xor_sync(0xffffffffu, total, o);
-    before += __shfl_xor_sync(0xffffffffu, before, o);
-  }
-}
 // where the line is cut: its first `rem` parts have q + 1 stages, the others q
 struct Cuts {
   int q, rem;
@@ -389,63 +377,140 @@ struct Cuts {
   __device__ __forceinline__ int part_of(int x) const { return x < rem * (q + 1) ? x / (q + 1) : rem + (x - rem * (q + 1)) / max(q, 1); }
 };
 
+// An item that cuts fell into: parts i0 .. i1 of it are in ws, the CTA that came last puts them together.  slot(i): part i
+template <int D, bool kBf16, typename Slot, typename Out>
+__device__ __forceinline__ void merge_parts(float scale_log2, uint8_t* smem, int rows, int i0, int i1, Slot slot, Out out_row) {
+  float* s_inv = reinterpret_cast<float*>(smem);                     // [16]
+  float4* s_o = reinterpret_cast<float4*>(smem + 64);                // [128]
+  float* s_f = reinterpret_cast<float*>(smem + 64 + 2048);           // [16][parts]: the parts' weights
+  static_assert(64 + 2048 + 16 * kDecodeCtas * 4 <= Smem<D>::kStatOff, "over the ring");
+  const int parts = i1 - i0 + 1, lane = threadIdx.x & 31;
+  for (int row = threadIdx.x >> 5; row < rows; row += 4) {
+    float M = -INFINITY, L = 0.f;
+    float* f_row = s_f + row * parts;
+    for (int i = lane; i < parts; i += 32) {
+      f_row[i] = __ldcg(slot(i0 + i) + 16 * D + row);
+      M = fmaxf(M, f_row[i]);
+    }
+    M = warp_max(M);
+    const float use = M == -INFINITY ? 0.f : M;
+    for (int i = lane; i < parts; i += 32) {
+      const float f = exp2f((f_row[i] - use) * scale_log2), l = __ldcg(slot(i0 + i) + 16 * D + 16 + row);
+      f_row[i] = l > 0.f ? f : 0.f;
+      L = fmaf(l, f, L);
+    }
+    L = warp_sum(L);
+    if (lane == 0) s_inv[row] = L > 0.f ? 1.f / L : L;               // 0 without keys; NaN stays NaN
+  }
+  __syncthreads();
+  // where the rows leave threads over, these take every second or fourth part
+  const int quads = rows * (D / 4), share = quads <= 32 ? 4 : (quads <= 64 ? 2 : 1), step = 128 / share;
+  const int mine = static_cast<int>(threadIdx.x) / step, thread = static_cast<int>(threadIdx.x) % step;
+  for (int idx0 = 0; idx0 < quads; idx0 += step) {
+    const int idx = idx0 + thread, row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+    const bool valid = idx < quads;
+    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid) {
+#pragma unroll 8
+      for (int i = mine; i < parts; i += share) {
+        const float f = s_f[row * parts + i];
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(slot(i0 + i) + row * D + col));
+        O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
+      }
+    }
+    if (share > 1) {                                                 // then idx0 is 0: one trip
+      s_o[threadIdx.x] = O;
+      __syncthreads();
+      if (mine == 0) {
+        for (int k = 1; k < share; ++k) {
+          const float4 v = s_o[k * step + thread];
+          O.x += v.x; O.y += v.y; O.z += v.z; O.w += v.w;
+        }
+      }
+    }
+    if (mine == 0 && valid) {
+      const float inv = s_inv[row];
+      *reinterpret_cast<uint2*>(out_row(row) + col) = make_uint2(pack2<kBf16>(O.x * inv, O.y * inv), pack2<kBf16>(O.z * inv, O.w * inv));
+    }
+  }
+}
+
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams p) {
   using L = Smem<D>;
   extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ int s_find[2];
+  __shared__ int s_inside, s_r, s_last, s_sum[2][4];
+  __shared__ Item s_item;
   const PagedAttnArgs& a = p.a;
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
   allow_next();
-  if (!p.beside_chunks) await_previous();
-  int at, end;
+  if (!p.beside_chunks && !p.behind_write) await_previous();
+  int at, end, parts_of_line = 0, line = 0;
   if (p.splits == 0) {                                               // one item, whole
-    const int stages = decode_item(p, blockIdx.x / a.ng).stages;
+    const int r0 = blockIdx.x / a.ng;
+    const Item mine = decode_item(p, r0);
     at = 0;
-    end = stages;
+    end = mine.stages;
     if (tid == 0) {
-      s_find[0] = blockIdx.x / a.ng;
-      s_find[1] = static_cast<int>(blockIdx.x % a.ng) * stages;
+      s_r = r0;
+      s_item = mine;
+      s_inside = static_cast<int>(blockIdx.x % a.ng) * mine.stages;
     }
   } else {
-    int total, before;
-    count_stages(p, 0, total, before);
-    const Cuts cuts(total * a.ng, p.splits);
+    // a request per thread; the first 128 stay in registers for the search
+    Item mine = decode_item(p, tid);
+    int total = mine.stages;
+    for (int r0 = tid + 128; r0 < p.n_tiles; r0 += 128) total += decode_item(p, r0).stages;
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (lane == 0) s_sum[1][warp] = total;
+    __syncthreads();
+    total = s_sum[1][0] + s_sum[1][1] + s_sum[1][2] + s_sum[1][3];
+    line = total * a.ng;
+    parts_of_line = p.splits;
+    const Cuts cuts(line, p.splits);
     at = cuts.at(blockIdx.x);
     end = cuts.at(blockIdx.x + 1);
-  }
-  if (at >= end) {
-    if (p.beside_chunks) await_previous();
-    return;
-  }
-  // the request that this CTA's part of the line starts in
-  if (p.splits != 0 && tid < 32) {
+    // the request that this CTA's part of the line starts in
     int seen = 0;
-    for (int r0 = 0; r0 < p.n_tiles; r0 += 32) {
-      const int s = decode_item(p, r0 + lane).stages;
-      int incl = s;
+    for (int r0 = 0, turn = 0; r0 < p.n_tiles && at < end; r0 += 128, turn ^= 1) {
+      if (r0 > 0) mine = decode_item(p, r0 + tid);
+      int incl = mine.stages;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
-      const int first = (seen + incl - s) * a.ng;
-      if (s > 0 && at >= first && at < first + s * a.ng) {
-        s_find[0] = r0 + lane;
-        s_find[1] = at - first;
+      if (lane == 31) s_sum[turn][warp] = incl;
+      __syncthreads();
+      int before = seen;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        if (w < warp) before += s_sum[turn][w];
+        seen += s_sum[turn][w];
       }
-      seen += __shfl_sync(0xffffffffu, incl, 31);
+      const int first = (before + incl - mine.stages) * a.ng;
+      if (mine.stages > 0 && at >= first && at < first + mine.stages * a.ng) {
+        s_r = r0 + tid;
+        s_item = mine;
+        s_inside = at - first;
+      }
       if (seen * a.ng > at) break;
     }
   }
+  if (at >= end) {
+    if (p.beside_chunks || p.behind_write) await_previous();
+    return;
+  }
   __syncthreads();
-  int r = s_find[0], inside = s_find[1];
-  Item it = decode_item(p, r);
+  int r = s_r, inside = s_inside;
+  Item it = s_item;
   float* part = reinterpret_cast<float*>(smem);                      // [4 warps][16][D] over the ring
   float* s_m = reinterpret_cast<float*>(smem + L::kStatOff);
   float* s_l = s_m + 64;
   Tile<D, kBf16, 1> tile;
+  const Cuts cuts(line, max(parts_of_line, 1));
+  if (p.behind_write) await_previous();                              // the new keys are in their pages, the counters zero
   while (true) {
     const int hk = inside / it.stages, st0 = inside % it.stages;
     const int n_st = min(it.stages - st0, end - at);
@@ -455,6 +520,9 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     tile.spill(part, s_m, s_l);
     __syncthreads();
     const bool whole = n_st == it.stages;
+    auto out_row = [&](int row) {
+      return static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
+    };
     // slot 0: a part that starts inside its item; slot 1: one that starts with it
     float* ws = p.ws + (static_cast<int64_t>(blockIdx.x) * 2 + (st0 == 0 ? 1 : 0)) * (16 * (D + 2));
     for (int idx = tid; idx < (it.n << p.group_shift) * (D / 4); idx += 128) {
@@ -467,14 +535,25 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
         for (int w = 0; w < 4; ++w) x.add(s_m[w * 16 + row], s_l[w * 16 + row], *reinterpret_cast<const float4*>(part + (w * 16 + row) * D + col));
       }
       if (whole) {
-        uint16_t* out = static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
-        *reinterpret_cast<uint2*>(out + col) = x.result<kBf16>();
+        *reinterpret_cast<uint2*>(out_row(row) + col) = x.result<kBf16>();
       } else {
         *reinterpret_cast<float4*>(ws + row * D + col) = x.O;
         if (col == 0) {
           ws[16 * D + row] = x.M;
           ws[16 * D + 16 + row] = x.L;
         }
+      }
+    }
+    if (!whole) {
+      const int first = at - st0, i0 = cuts.part_of(first), i1 = cuts.part_of(first + it.stages - 1);
+      __threadfence();
+      __syncthreads();                                               // this part is in ws for whoever counts it
+      if (tid == 0) s_last = atomicAdd(p.arrived + r * a.ng + hk, 1) == i1 - i0;
+      __syncthreads();
+      if (s_last) {
+        __threadfence();
+        merge_parts<D, kBf16>(a.scale_log2, smem, it.n << p.group_shift, i0, i1,
+                              [&](int i) { return p.ws + (static_cast<int64_t>(i) * 2 + (i > i0 || cuts.at(i) > first ? 0 : 1)) * (16 * (D + 2)); }, out_row);
       }
     }
     at += n_st;
@@ -488,71 +567,6 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     __syncthreads();                                                 // the partials have been read; the ring fills again
   }
   if (p.beside_chunks) await_previous();
-}
-
-// items that a cut fell into: their CTAs' partials, one CTA per (request, KV head)
-template <int D, bool kBf16>
-__global__ void __launch_bounds__(512) paged_merge_kernel(const PagedParams p) {
-  await_previous();
-  const PagedAttnArgs& a = p.a;
-  const int r = blockIdx.x / a.ng, hk = blockIdx.x % a.ng, G = 1 << p.group_shift, np = a.ng << p.group_shift;
-  const Item it = decode_item(p, r);
-  if (it.stages == 0) return;
-  int total, before;
-  count_stages(p, r, total, before);
-  const Cuts cuts(total * a.ng, p.splits);
-  const int first = before * a.ng + hk * it.stages, i0 = cuts.part_of(first), i1 = cuts.part_of(first + it.stages - 1);
-  if (i0 == i1) return;                                              // one CTA had all of it
-  auto slot = [&](int i) { return p.ws + (static_cast<int64_t>(i) * 2 + (i > i0 || cuts.at(i) > first ? 0 : 1)) * (16 * (D + 2)); };
-  // the parts' weights first, then the accumulators: every load of a pass stands by itself
-  __shared__ float s_f[16][kDecodeCtas + 1], s_inv[16];
-  const int rows = it.n << p.group_shift, parts = i1 - i0 + 1, lane = threadIdx.x & 31;
-  for (int row = threadIdx.x >> 5; row < rows; row += 16) {
-    float M = -INFINITY, L = 0.f;
-    for (int i = lane; i < parts; i += 32) {
-      s_f[row][i] = slot(i0 + i)[16 * D + row];
-      M = fmaxf(M, s_f[row][i]);
-    }
-    M = warp_max(M);
-    const float use = M == -INFINITY ? 0.f : M;
-    for (int i = lane; i < parts; i += 32) {
-      const float f = exp2f((s_f[row][i] - use) * a.scale_log2), l = slot(i0 + i)[16 * D + 16 + row];
-      s_f[row][i] = l > 0.f ? f : 0.f;
-      L = fmaf(l, f, L);
-    }
-    L = warp_sum(L);
-    if (lane == 0) s_inv[row] = L > 0.f ? 1.f / L : L;               // 0 without keys; NaN stays NaN
-  }
-  __syncthreads();
-  // four groups of threads take every fourth part of 128 column quads at a time
-  __shared__ float4 s_o[3][128];
-  const int group = threadIdx.x >> 7, thread = threadIdx.x & 127;
-  for (int idx0 = 0; idx0 < rows * (D / 4); idx0 += 128) {
-    const int idx = idx0 + thread, row = idx / (D / 4), col = (idx % (D / 4)) * 4;
-    const bool valid = idx < rows * (D / 4);
-    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) {
-#pragma unroll 8
-      for (int i = group; i < parts; i += 4) {
-        const float f = s_f[row][i];
-        const float4 v = *reinterpret_cast<const float4*>(slot(i0 + i) + row * D + col);
-        O.x = fmaf(v.x, f, O.x); O.y = fmaf(v.y, f, O.y); O.z = fmaf(v.z, f, O.z); O.w = fmaf(v.w, f, O.w);
-      }
-    }
-    if (group > 0) s_o[group - 1][thread] = O;
-    __syncthreads();
-    if (group == 0 && valid) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float4 v = s_o[k][thread];
-        O.x += v.x; O.y += v.y; O.z += v.z; O.w += v.w;
-      }
-      const float inv = s_inv[row];
-      uint16_t* out = static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(it.t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
-      *reinterpret_cast<uint2*>(out + col) = make_uint2(pack2<kBf16>(O.x * inv, O.y * inv), pack2<kBf16>(O.z * inv, O.w * inv));
-    }
-    __syncthreads();
-  }
 }
 
 // ---- decode with few rows per key and many short contexts: a tile of the kernels above is mostly empty and its start and end cost more than
@@ -751,9 +765,11 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
 // new keys and values [T, ng, d] (any token and head strides) into their cache rows, 16 bytes per thread
 __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* __restrict__ kc,
                                                           uint4* __restrict__ vc, const int64_t* __restrict__ slots, int n_tok, int ng, int chunks,
-                                                          int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh) {
+                                                          int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh, int* __restrict__ arrived,
+                                                          int64_t n_arrived) {
   allow_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, row = static_cast<int64_t>(ng) * chunks;
+  for (int64_t i = idx; i < n_arrived; i += static_cast<int64_t>(gridDim.x) * 256) arrived[i] = 0;
   if (idx >= n_tok * row) return;
   const int64_t t = idx / row;
   const int c = static_cast<int>(idx % row), h = c / chunks, u = c % chunks;
@@ -807,8 +823,7 @@ int launch_decode(const PagedParams& p, cudaStream_t s) {
     return -12;
   }
   const unsigned items = static_cast<unsigned>(p.n_tiles * p.a.ng);
-  const int rc = launch(kern, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, p, s);
-  return rc != 0 || p.splits == 0 ? rc : launch(paged_merge_kernel<D, kBf16>, items, 512, 0, 1, p, s);
+  return launch(kern, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, p, s);
 }
 
 template <int D, bool kBf16>
@@ -832,16 +847,20 @@ int64_t decode_keys(const PagedAttnArgs& a) {
   return a.decode_len > 0 && a.decode_len < all ? a.decode_len : all;
 }
 
-// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Contexts of up to 8 stages (512
-// keys), or 16 where all items run at once, are not cut at all (0): the merge kernel then costs as much as the imbalance that it
-// removes (a step of 34 requests of 64 to 153 keys x 12 heads beside two chunks of 37: 44.7 us cut, 23.2 whole; 5 requests of up to
-// 600 keys x 8 heads: 29.1 and 16.3)
+// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Contexts of up to 4 stages (256
+// keys), or 8 where not all items run at once, are not cut at all (0): putting parts together then costs as much as the imbalance
+// that it removes.  us, whole / cut: 90 requests of up to 300 keys x 8 heads of 128 35.8 / 42.0; 16 of up to 1000 x 8 heads 37.9 / 27.6, 8 of up to 700
+// 27.6 / 21.5, 1 of 500 21.5 / 17.4
 int decode_ctas(const PagedAttnArgs& a) {
   const int64_t items = decode_items(a), longest = (decode_keys(a) + kStageKeys - 1) / kStageKeys;
-  if (longest <= 8 || (longest <= 16 && items <= kDecodeCtas)) return 0;
+  if (longest <= 4 || (longest <= 8 && items > kDecodeCtas)) return 0;
   const int64_t n = items * longest / 2;
   return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
 }
+
+// a workspace holds the CTAs' partials and, behind them, a counter for each (request, KV head)
+int64_t decode_parts(const PagedAttnArgs& a) { return static_cast<int64_t>(decode_ctas(a)) * 2 * 16 * (a.head_dim + 2); }
+int* arrived_in(const PagedAttnArgs& a, float* ws) { return reinterpret_cast<int*>(ws + decode_parts(a)); }
 
 }  // namespace
 
@@ -870,20 +889,25 @@ bool paged_attention_supported(int head_dim, int group) {
 }
 
 int64_t paged_decode_workspace(const PagedAttnArgs& a) {
-  return paged_decode_by_rows(a) ? 0 : static_cast<int64_t>(decode_ctas(a)) * 2 * 16 * (a.head_dim + 2);
+  if (paged_decode_by_rows(a)) return 0;
+  const int64_t parts = decode_parts(a);
+  return parts > 0 ? parts + decode_items(a) : 0;
 }
 
-void paged_write(const PagedWriteArgs& w, cudaStream_t s) {
+// zeroes the decode kernel's counters (`ws`, where that call will have a workspace) too
+void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cudaStream_t s) {
   const int chunks = w.head_dim / 8;
   const int64_t n = static_cast<int64_t>(w.n_tokens) * w.ng * chunks;
   if (n == 0) return;
   paged_write_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
       static_cast<const uint4*>(w.k), static_cast<const uint4*>(w.v), static_cast<uint4*>(w.k_cache), static_cast<uint4*>(w.v_cache), w.slots,
-      w.n_tokens, w.ng, chunks, w.k_st / 8, w.k_sh / 8, w.v_st / 8, w.v_sh / 8);
+      w.n_tokens, w.ng, chunks, w.k_st / 8, w.k_sh / 8, w.v_st / 8, w.v_sh / 8, ws != nullptr ? arrived_in(a, ws) : nullptr,
+      ws != nullptr ? decode_items(a) : 0);
 }
 
 // with cu: chunk_tiles tiles of 64 rows over the requests with more than 16, in chunk_splits key ranges; decode: whether there are others
-int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, cudaStream_t s) {
+// `written`: paged_write went before it with the same workspace
+int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s) {
   PagedParams p{};
   p.a = a;
   p.row_scale = a.scale_log2;
@@ -909,7 +933,15 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
                              : (a.is_bf16 ? launch_rows<64, true>(p, s) : launch_rows<64, false>(p, s));
   }
   p.splits = decode_ctas(a);
+  p.behind_write = written && !p.beside_chunks;
   p.ws = ws;
+  if (p.splits > 0) {
+    p.arrived = arrived_in(a, ws);
+    if (!written) {
+      const cudaError_t e = cudaMemsetAsync(p.arrived, 0, sizeof(int) * static_cast<size_t>(decode_items(a)), s);
+      if (e != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(e); return -13; }
+    }
+  }
   return a.head_dim == 128 ? (a.is_bf16 ? launch_decode<128, true>(p, s) : launch_decode<128, false>(p, s))
                            : (a.is_bf16 ? launch_decode<64, true>(p, s) : launch_decode<64, false>(p, s));
 }
