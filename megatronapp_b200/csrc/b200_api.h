@@ -326,6 +326,7 @@ struct PagedAttnArgs {
   int n_seqs;
   int decode_len, decode_mean;   // keys of the longest and of an average context beside the chunks (0: not known)
   bool decode_single;       // with cu: each request beside the chunks has one token
+  bool beside_chunks;       // with cu: there are chunks
   int n_tokens, ng, group, head_dim, block_size, max_blocks;
   float scale_log2;
   bool is_bf16;

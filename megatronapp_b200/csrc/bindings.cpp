@@ -964,6 +964,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
     TORCH_CHECK(cu->scalar_type() == at::kInt && cu->is_contiguous() && cu->numel() >= 1, "cu must be int32");
     a.cu = cu->data_ptr<int32_t>(); a.n_seqs = static_cast<int>(cu->numel()) - 1;
     a.decode_len = static_cast<int>(decode_len); a.decode_mean = static_cast<int>(decode_mean); a.decode_single = decode_single;
+    a.beside_chunks = chunk_tiles > 0;
   }
   if (T == 0) return out;
   const bool decode = !cu.has_value() || splits > 0, written = k_new.has_value();

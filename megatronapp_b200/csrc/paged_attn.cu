@@ -435,7 +435,8 @@ __device__ __forceinline__ void merge_parts(float scale_log2, uint8_t* smem, int
   }
 }
 
-template <int D, bool kBf16>
+// kCut: a part of the line per CTA, else one item
+template <int D, bool kBf16, bool kCut>
 __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams p) {
   using L = Smem<D>;
   extern __shared__ __align__(16) uint8_t smem[];
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
   allow_next();
   if (!p.beside_chunks && !p.behind_write) await_previous();
   int at, end, parts_of_line = 0, line = 0;
-  if (p.splits == 0) {                                               // one item, whole
+  if constexpr (!kCut) {
     const int r0 = blockIdx.x / a.ng;
     const Item mine = decode_item(p, r0);
     at = 0;
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
         }
       }
     }
-    if (!whole) {
+    if (kCut && !whole) {
       const int first = at - st0, i0 = cuts.part_of(first), i1 = cuts.part_of(first + it.stages - 1);
       __threadfence();
       __syncthreads();                                               // this part is in ws for whoever counts it
@@ -763,13 +764,16 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
 }
 
 // new keys and values [T, ng, d] (any token and head strides) into their cache rows, 16 bytes per thread
+// kCount: counters of the decode kernel are set to zero too.  Kernels of their own: with the few instructions more, steps that need no counters took 1.2 to
+// 1.8 us longer (81 requests of up to 182 keys x 12 heads of 128: 21.7 -> 23.5)
+template <bool kCount>
 __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* __restrict__ kc,
                                                           uint4* __restrict__ vc, const int64_t* __restrict__ slots, int n_tok, int ng, int chunks,
                                                           int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh, int* __restrict__ arrived,
                                                           int64_t n_arrived) {
   allow_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, row = static_cast<int64_t>(ng) * chunks;
-  for (int64_t i = idx; i < n_arrived; i += static_cast<int64_t>(gridDim.x) * 256) arrived[i] = 0;
+  if (kCount && idx < n_arrived) arrived[idx] = 0;
   if (idx >= n_tok * row) return;
   const int64_t t = idx / row;
   const int c = static_cast<int>(idx % row), h = c / chunks, u = c % chunks;
@@ -814,8 +818,11 @@ int launch_chunks(const PagedParams& p, cudaStream_t s) {
 
 template <int D, bool kBf16>
 int launch_decode(const PagedParams& p, cudaStream_t s) {
-  auto kern = paged_decode_kernel<D, kBf16>;
-  static const cudaError_t ready = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
+  auto cut = paged_decode_kernel<D, kBf16, true>, whole = paged_decode_kernel<D, kBf16, false>;
+  static const cudaError_t ready = [&] {
+    const cudaError_t e = cudaFuncSetAttribute(cut, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(whole, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
+  }();
   if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
   // the line of stages is counted in 32 bits
   if (static_cast<int64_t>(p.n_tiles) * p.a.ng * ((static_cast<int64_t>(p.a.max_blocks) * p.a.block_size + kStageKeys - 1) / kStageKeys + 1) > 0x7fffffff) {
@@ -823,7 +830,7 @@ int launch_decode(const PagedParams& p, cudaStream_t s) {
     return -12;
   }
   const unsigned items = static_cast<unsigned>(p.n_tiles * p.a.ng);
-  return launch(kern, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, p, s);
+  return launch(p.splits > 0 ? cut : whole, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, p, s);
 }
 
 template <int D, bool kBf16>
@@ -847,13 +854,15 @@ int64_t decode_keys(const PagedAttnArgs& a) {
   return a.decode_len > 0 && a.decode_len < all ? a.decode_len : all;
 }
 
-// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Contexts of up to 4 stages (256
-// keys), or 8 where not all items run at once, are not cut at all (0): putting parts together then costs as much as the imbalance
-// that it removes.  us, whole / cut: 90 requests of up to 300 keys x 8 heads of 128 35.8 / 42.0; 16 of up to 1000 x 8 heads 37.9 / 27.6, 8 of up to 700
-// 27.6 / 21.5, 1 of 500 21.5 / 17.4
+// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Short contexts are not cut at all
+// (0): putting parts together then costs as much as the imbalance that it removes.  us, whole / cut, heads of 128: 90 requests of up to 300 keys x 8
+// heads 35.8 / 42.0, 40 of up to 429 x 4 beside chunks 29.1 / 40.9, 2 of up to 430 x 8 beside one 26.5 /
+// 30.7, but 1 of 500 x 8 21.5 / 17.4, 8 of up to 700 27.6 / 21.5; a stage of heads of 64 takes
+// half as long: 10 of up to 824 x 12 beside chunks 21.9 / 29.3, 1 of 522 x 8 10.3 / 12.4
 int decode_ctas(const PagedAttnArgs& a) {
   const int64_t items = decode_items(a), longest = (decode_keys(a) + kStageKeys - 1) / kStageKeys;
-  if (longest <= 4 || (longest <= 8 && items > kDecodeCtas)) return 0;
+  const bool whole = a.head_dim == 64 ? longest <= (items <= kDecodeCtas ? 16 : 8) : longest <= (items <= 64 && !a.beside_chunks ? 4 : 8);
+  if (whole) return 0;
   const int64_t n = items * longest / 2;
   return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
 }
@@ -899,10 +908,11 @@ void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cud
   const int chunks = w.head_dim / 8;
   const int64_t n = static_cast<int64_t>(w.n_tokens) * w.ng * chunks;
   if (n == 0) return;
-  paged_write_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(
+  const int64_t n_arrived = ws != nullptr ? decode_items(a) : 0;
+  auto kern = n_arrived > 0 ? paged_write_kernel<true> : paged_write_kernel<false>;
+  kern<<<static_cast<unsigned>(((n > n_arrived ? n : n_arrived) + 255) / 256), 256, 0, s>>>(
       static_cast<const uint4*>(w.k), static_cast<const uint4*>(w.v), static_cast<uint4*>(w.k_cache), static_cast<uint4*>(w.v_cache), w.slots,
-      w.n_tokens, w.ng, chunks, w.k_st / 8, w.k_sh / 8, w.v_st / 8, w.v_sh / 8, ws != nullptr ? arrived_in(a, ws) : nullptr,
-      ws != nullptr ? decode_items(a) : 0);
+      w.n_tokens, w.ng, chunks, w.k_st / 8, w.k_sh / 8, w.v_st / 8, w.v_sh / 8, n_arrived > 0 ? arrived_in(a, ws) : nullptr, n_arrived);
 }
 
 // with cu: chunk_tiles tiles of 64 rows over the requests with more than 16, in chunk_splits key ranges; decode: whether there are others
@@ -926,7 +936,7 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
   }
   if (a.cu != nullptr && !decode) return 0;                          // every request is a chunk
   p.n_tiles = a.cu != nullptr ? a.n_seqs : a.n_tokens;
-  p.beside_chunks = a.cu != nullptr && chunk_tiles > 0;
+  p.beside_chunks = a.beside_chunks;
   if (paged_decode_by_rows(a)) {
     if (decode_items(a) > 0x7fffffff) { g_paged_err = "paged attention: too many requests"; return -12; }
     return a.head_dim == 128 ? (a.is_bf16 ? launch_rows<128, true>(p, s) : launch_rows<128, false>(p, s))
