@@ -126,6 +126,10 @@ __device__ __forceinline__ void tma_reduce_add_2d(const void* tmap, const void* 
       ::"l"(tmap), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
       : "memory");
 }
+// Launches of a stream overlap: a kernel that allows it lets the next one's CTAs start where SMs are free, and that one waits, before it touches
+// memory, until everything before it is complete and visible.
+__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // 16 bytes to a shared-memory address
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");

@@ -368,6 +368,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   tc_fence_before();
   cluster_sync_all();                    // peer barriers are initialised before any remote arrive, the accumulators allocated
   tc_fence_after();
+  if constexpr (kMode == kModePlain || kMode == kModeGroupM || kMode == kModeGroupK) {
+    pdl_allow_next();
+    pdl_await_previous();
+  }
   const uint32_t tmem_base = *tmem_ptr_smem;
   constexpr uint32_t kPairStageBytes = 2 * (L::kA + L::kB);
 
@@ -755,8 +759,17 @@ int launch2(const GemmArgs& a, const P2& p, const CUtensorMap& ta, const CUtenso
     }
     set = true;
   }
-  kern<<<grid, kThreads, Smem2T<BN>::kTotal, a.stream>>>(ta, tal, tb, td, tdp, pm, p);
-  cudaError_t e = cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Smem2T<BN>::kTotal;
+  cfg.stream = a.stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = MODE == kModePlain || MODE == kModeGroupM || MODE == kModeGroupK ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tal, tb, td, tdp, pm, p);
   if (e != cudaSuccess) { g_err2 = std::string("launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
 }

@@ -36,3 +36,41 @@ def test_store_bias_gelu(M, N, K, dtype):
         assert bool(((acc.double() - d.double() - want).abs() <= fp32 + 2.0 ** -23 * (want.abs() + d.double().abs())).all())
         ops.gemm(A, B, out=d, epilogue=2)
         assert bool(((d.double() - want).abs() <= fp32).all())
+
+
+def test_launches_that_overlap():
+    """A product's kernel starts while the one before it still runs: chains of them, results that the next reads or overwrites, in order and in a graph."""
+    from megatronapp_b200 import ops
+
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn(2048, 512, generator=g).bfloat16().cuda()
+    w = [(torch.randn(512, 512, generator=g) * 512 ** -0.5).bfloat16().cuda() for _ in range(4)]
+    acc, bufs = torch.zeros(512, 512, device="cuda"), [torch.empty_like(x) for _ in range(2)]
+
+    def chain(pause):
+        acc.zero_()
+        a = x
+        for i in range(24):
+            out = bufs[i & 1]                                # read by the product before this one's predecessor
+            ops.gemm(a, w[i & 3], out=out)
+            pause()
+            if i % 5 == 4:
+                out.mul_(1.0)                                # a kernel of another kind between them
+            ops.gemm(out, a, out=acc, a_mn=True, b_mn=True, epilogue=1)
+            pause()
+            a = out
+        return a.clone(), acc.clone()
+
+    want = chain(torch.cuda.synchronize)
+    for _ in range(5):
+        for got, ref in zip(chain(lambda: None), want):
+            assert torch.equal(got, ref)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = chain(lambda: None)
+    for _ in range(3):
+        for o in outs:
+            o.zero_()
+        graph.replay()
+        for got, ref in zip(outs, want):
+            assert torch.equal(got, ref)
