@@ -66,6 +66,13 @@ def reset_launch_count() -> None:
         ext().reset_launch_count()
 
 
+def _eager() -> bool:
+    """Whether nothing watches the operators themselves (forward-mode, functorch transforms, tracing): the nodes of the native module do for autograd
+    then, the ``torch.autograd.Function`` classes below for everything else."""
+    return (torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+            and not torch._C._is_tracing() and not torch.compiler.is_compiling())
+
+
 def _native(t: torch.Tensor) -> bool:
     return t.is_cuda and t.dtype in (torch.bfloat16, torch.float16)
 
@@ -85,26 +92,16 @@ def gemm_ref(a, b, a_mn=False, b_mn=False, bias=None, act=0, out_dtype=None):
     return d.to(out_dtype or a.dtype)
 
 
-def _gemm_ok(a, b, d) -> bool:
-    if not (_native(a) and a.dtype == b.dtype):
-        return False
-    for t in (a, b, d):
-        if t.dim() != 2 or t.stride(1) != 1 or t.stride(0) % 8 != 0 or t.data_ptr() % 16 != 0:
-            return False
-    return True
-
-
 def gemm(a, b, out=None, *, a_mn=False, b_mn=False, epilogue=EPI_STORE16, bias=None, act=0,
          out_pre=None, block_n=0):
     """tcgen05 GEMM.  ``epilogue``: 0 store 16-bit, 1 ``out += acc`` (fp32), 2 ``out = acc`` (fp32)."""
-    M = a.shape[1] if a_mn else a.shape[0]
-    N = b.shape[1] if b_mn else b.shape[0]
+    if _native(a):
+        taken = ext().gemm_if_taken(a, b, out, a_mn, b_mn, epilogue, bias, act, out_pre, block_n)
+        if taken is not None:
+            return taken
     if out is None:
-        out = torch.empty(M, N, dtype=a.dtype if epilogue == EPI_STORE16 else torch.float32,
-                          device=a.device)
-    if a.is_cuda and _gemm_ok(a, b, out) and (epilogue == EPI_STORE16 or out.shape[1] % 4 == 0):
-        ext().gemm(a, b, out, a_mn, b_mn, epilogue, bias, act, out_pre, block_n)
-        return out
+        out = torch.empty(a.shape[1] if a_mn else a.shape[0], b.shape[1] if b_mn else b.shape[0],
+                          dtype=a.dtype if epilogue == EPI_STORE16 else torch.float32, device=a.device)
     if a.is_cuda:
         fallback_counts["gemm"] += 1
     # reference / library path (CPU, fp32 params, odd shapes)
@@ -239,8 +236,7 @@ def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """Rows ``ids`` of ``weight``; the dense gradient of a 16-bit table comes from kernels that sum in fp32 and a fixed order."""
     if (_native(weight) and weight.requires_grad and torch.is_grad_enabled() and ids.is_cuda and ids.dim() in (1, 2) and weight.dim() == 2
             and _EMBED_FROM <= ids.numel() <= _EMBED_TO and weight.shape[1] % 8 == 0 and 0 < weight.shape[1] < 1 << 24 and 0 < weight.shape[0] <= 0x7fffffff
-            and torch.autograd.forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling()):
+            and _eager()):
         return _EmbeddingFn.apply(ids, weight)
     return torch.nn.functional.embedding(ids, weight)
 
@@ -282,6 +278,8 @@ class _NormFn(torch.autograd.Function):
 
 def layer_norm(x, gamma, beta=None, eps=1e-5, rms=False, zero_centered=False):
     if _native(x) and gamma.dtype == x.dtype and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
+        if _eager():
+            return ext().norm(x, gamma, beta, eps, rms, zero_centered)
         return _NormFn.apply(x, gamma, beta, eps, rms, zero_centered)
     if x.is_cuda:
         fallback_counts["norm"] += 1
@@ -387,6 +385,8 @@ def bias_dropout_add(x, bias, residual, p: float, training: bool):
             seed = int(torch.cuda.initial_seed() & 0x7FFFFFFFFFFFFFFF)
             _BDA_OFFSET[0] += 1
             return _BdaFn.apply(x, bias, residual, p_eff, seed, _BDA_OFFSET[0])
+        if _eager():
+            return ext().bias_add(x, bias, residual)
         return _BdaFn.apply(x, bias, residual, 0.0, 0, 0)
     return bias_dropout_add_ref(x, bias, residual, p, training)
 
@@ -523,6 +523,8 @@ def attention_packed_qkv(mixed, scale=None, causal=True):
             and mixed.shape[0] % 64 == 0 and native_attention_available()):
         return None
     scale = scale if scale is not None else 1.0 / math.sqrt(hn)
+    if _eager():
+        return ext().attention_packed(mixed, scale, causal)
     return _PackedQKVAttnFn.apply(mixed, scale, causal)
 
 
@@ -568,6 +570,8 @@ def attention(q, k, v, scale=None, causal=True, dropout_p=0.0, training=True, ma
               and q.shape[1] % k.shape[1] == 0 and (not needs_grad or (sq % 64 == 0 and sk % 64 == 0)))
     if impl in ("auto", "native") and usable and native_attention_available():
         q, k, v = (t if _attn_view_ok(t) else t.contiguous() for t in (q, k, v))
+        if _eager():
+            return ext().attention(q, k, v, scale, causal)
         return _AttnFn.apply(q, k, v, scale, causal)
     if impl == "native":
         raise RuntimeError("native attention requested but not usable for this problem")
