@@ -447,17 +447,14 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
   const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
   allow_next();
   if (!p.beside_chunks && !p.behind_write) await_previous();
-  int at, end, parts_of_line = 0, line = 0;
+  int at, end, parts_of_line = 0, line = 0, r = 0, inside = 0;
+  Item it;
   if constexpr (!kCut) {
-    const int r0 = blockIdx.x / a.ng;
-    const Item mine = decode_item(p, r0);
+    r = blockIdx.x / a.ng;
+    it = decode_item(p, r);
     at = 0;
-    end = mine.stages;
-    if (tid == 0) {
-      s_r = r0;
-      s_item = mine;
-      s_inside = static_cast<int>(blockIdx.x % a.ng) * mine.stages;
-    }
+    end = it.stages;
+    inside = static_cast<int>(blockIdx.x % a.ng) * it.stages;
   } else {
     // a request per thread; the first 128 stay in registers for the search
     Item mine = decode_item(p, tid);
@@ -503,14 +500,17 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     if (p.beside_chunks || p.behind_write) await_previous();
     return;
   }
-  __syncthreads();
-  int r = s_r, inside = s_inside;
-  Item it = s_item;
+  if constexpr (kCut) {
+    __syncthreads();
+    r = s_r;
+    inside = s_inside;
+    it = s_item;
+  }
   float* part = reinterpret_cast<float*>(smem);                      // [4 warps][16][D] over the ring
   float* s_m = reinterpret_cast<float*>(smem + L::kStatOff);
   float* s_l = s_m + 64;
   Tile<D, kBf16, 1> tile;
-  const Cuts cuts(line, max(parts_of_line, 1));
+  const Cuts cuts(kCut ? line : 0, kCut ? parts_of_line : 1);
   if (p.behind_write) await_previous();                              // the new keys are in their pages, the counters zero
   while (true) {
     const int hk = inside / it.stages, st0 = inside % it.stages;
