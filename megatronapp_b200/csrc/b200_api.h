@@ -327,6 +327,8 @@ struct PagedAttnArgs {
   int decode_len, decode_mean;   // keys of the longest and of an average context beside the chunks (0: not known)
   bool decode_single;       // with cu: each request beside the chunks has one token
   bool beside_chunks;       // with cu: there are chunks
+  int wide_tiles, wide_splits;   // with cu: tiles of 128 rows over the chunks, in key ranges each (0: not to be used)
+  int64_t n_slots;          // of the caches
   int n_tokens, ng, group, head_dim, block_size, max_blocks;
   float scale_log2;
   bool is_bf16;
@@ -342,6 +344,8 @@ bool paged_attention_supported(int head_dim, int group);
 void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cudaStream_t s);
 int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
 bool paged_decode_by_rows(const PagedAttnArgs& a);        // which of the two decode kernels
+bool paged_wide_tiles(const PagedAttnArgs& a);            // which of the two chunk kernels
+int paged_status();          // 1: a kernel of this process gave up on a wait (its rows are NaN)
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s);
 const char* paged_attention_last_error();
 

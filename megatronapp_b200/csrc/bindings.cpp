@@ -1043,7 +1043,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
                        const Tensor& tok_req, const Tensor& tok_len, int64_t block_size, double scale, int64_t splits,
                        const c10::optional<Tensor>& k_new, const c10::optional<Tensor>& v_new, const c10::optional<Tensor>& slots,
                        const c10::optional<Tensor>& cu, int64_t chunk_tiles, int64_t chunk_splits, int64_t decode_len, int64_t decode_mean,
-                       bool decode_single) {
+                       bool decode_single, int64_t wide_tiles, int64_t wide_splits) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && k_cache.dim() == 3 && k_cache.is_contiguous() && v_cache.is_contiguous());
   TORCH_CHECK(q.scalar_type() == k_cache.scalar_type() && (is_bf16(q) || q.scalar_type() == at::kHalf));
@@ -1067,6 +1067,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
     a.cu = cu->data_ptr<int32_t>(); a.n_seqs = static_cast<int>(cu->numel()) - 1;
     a.decode_len = static_cast<int>(decode_len); a.decode_mean = static_cast<int>(decode_mean); a.decode_single = decode_single;
     a.beside_chunks = chunk_tiles > 0;
+    a.wide_tiles = static_cast<int>(wide_tiles); a.wide_splits = static_cast<int>(wide_splits); a.n_slots = k_cache.size(0);
   }
   if (T == 0) return out;
   const bool decode = !cu.has_value() || splits > 0, written = k_new.has_value();
@@ -1300,7 +1301,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("paged_attention", &paged_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"), py::arg("tok_req"),
         py::arg("tok_len"), py::arg("block_size"), py::arg("scale"), py::arg("splits"), py::arg("k_new") = py::none(), py::arg("v_new") = py::none(),
         py::arg("slots") = py::none(), py::arg("cu") = py::none(), py::arg("chunk_tiles") = 0, py::arg("chunk_splits") = 1,
-        py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false);
+        py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false, py::arg("wide_tiles") = 0, py::arg("wide_splits") = 1);
+  m.def("paged_status", []() { return b200::paged_status(); });
   m.def("paged_decode_by_rows", [](int64_t requests, int ng, int group, int head_dim, int longest, int mean, bool single) {
     b200::PagedAttnArgs a{};
     const int32_t none = 0;

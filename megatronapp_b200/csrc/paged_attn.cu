@@ -24,6 +24,7 @@
 // Replaces the reference's dynamic-context attention (core/inference/contexts/dynamic_context.py + flash_attn_with_kvcache
 // in attention.py:590-603) and this repo's earlier gather + einsum path (inference/dynamic.py).
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -763,6 +764,471 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
   cluster.sync();                                                    // no CTA leaves while another reads its partials
 }
 
+// ---- chunks on tcgen05: pages of 8 to 64 slots, or whole multiples of 64, which a TMA box can fetch.  A tile is 128 rows.  Its stages of 64
+// keys go through a ring of three; scores and weights have two TMEM buffers each, so that a stage's scores are made under the one before's
+// exponentials.  The weights' three parts (see weigh_and_add) lie side by side in TMEM as A operands of three products with the same V.  Two threads
+// share a row, 32 keys each.  Where only some rows see a stage's keys, its V is looked at in shared memory first: keys that nobody sees
+// become zeros, and values that are not finite are taken out and added by hand to the rows that see them.
+// Bound by the chain of a stage and by the products (8 + 24 MMAs a stage at d = 128).  Two portions of 500 tokens x 32 / 8 heads of 128 beside 24 decoding
+// requests: 87 us the step, 110 with the 64-row tiles; four of 512 and one request 83 and 160.  Registers and ring are kept so small that a decode CTA
+// fits beside one of these.
+template <int D>
+struct WideSmem {
+  static constexpr int kDC = D / 64, kRows = 128, kStages = 3;
+  static constexpr int kQ = kRows * 128 * kDC, kKV = kStageKeys * 128 * kDC;
+  static constexpr int kKOff = kQ, kVOff = kKOff + kStages * kKV;
+  static constexpr int kExOff = kVOff + kStages * kKV;               // [parity][half][row]: partial maxima, then sums
+  static constexpr int kStatOff = kExOff + 2 * 2 * kRows * 4;        // max and sum of a row, for the cluster
+  static constexpr int kBarOff = kStatOff + 2 * kRows * 4;
+  static constexpr int kTotal = kBarOff + 256 + 1024;                // + alignment slack
+  static_assert(kRows * D * 4 <= 2 * kStages * kKV, "after the last stage, partial accumulators reuse the ring");
+};
+constexpr int kWideThreads = 384, kWideTries = 1 << 20;
+__device__ int g_paged_error = 0;
+
+// bounded: a wait that runs out is noted, and every later one ends at once
+__device__ __forceinline__ void wide_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
+  for (int i = 0; i < kWideTries; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return;
+    if ((i & 255) == 255 && __any_sync(0xffffffffu, *failed != 0)) return;
+  }
+  *failed = 1;
+}
+__device__ __forceinline__ void wide_arrive(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+// whether any of the 256 softmax threads says so; they meet here
+__device__ __forceinline__ bool wide_any(bool mine) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred P, Q;\n\t"
+      "setp.ne.u32 P, %1, 0;\n\t"
+      "barrier.cta.red.or.pred Q, 2, 256, P;\n\t"
+      "selp.u32 %0, 1, 0, Q;\n\t}\n"
+      : "=r"(r) : "r"(mine ? 1u : 0u) : "memory");
+  return r != 0;
+}
+
+// at most 96 registers (a bound of 576 threads): with 384 threads, room for a decode CTA's
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(576, 1)
+paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PagedParams p) {
+  using L = WideSmem<D>;
+  constexpr int kS = L::kStages;
+  constexpr float kUnit = kBf16 ? 1.f : 32768.f;                     // see Tile
+  constexpr float kSlack = kBf16 ? 8.f : 0.f;                        // accumulators are rescaled when a maximum has grown by 2^8; fp16 weights stay below one
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ int s_tile[2];
+  float* s_ex = reinterpret_cast<float*>(smem + L::kExOff);
+  uint64_t* k_full = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
+  uint64_t* k_empty = k_full + kS;
+  uint64_t* v_full = k_empty + kS;
+  uint64_t* v_empty = v_full + kS;
+  uint64_t* s_full = v_empty + kS;     // 2
+  uint64_t* s_read = s_full + 2;       // 2: scores are in registers
+  uint64_t* p_ready = s_read + 2;      // 2
+  uint64_t* pv_done = p_ready + 2;     // 2: the weights' columns are free, the accumulator is up to date
+  uint64_t* drained = pv_done + 2;     // 1, after a wait that ran out
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
+  volatile int* failed = reinterpret_cast<volatile int*>(drained + 2);
+  const PagedAttnArgs& a = p.a;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(blockIdx.x) % p.splits, item = static_cast<int>(blockIdx.x) / p.splits;
+  const int hk = item % a.ng, tile_at = p.n_tiles - 1 - item / a.ng;
+  const int G = 1 << p.group_shift, np = a.ng << p.group_shift, per_tile = L::kRows >> p.group_shift;
+  if (warp == 1 && lane == 0) {
+    for (int i = 0; i < kS; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_read[i], 8); mbar_init(&p_ready[i], 8); mbar_init(&pv_done[i], 1); }
+    mbar_init(drained, 2);
+    *failed = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+  }
+  if (warp == 2) tmem_alloc<512>(tmem_slot);
+  await_previous();
+  allow_next();
+  if (warp == 0) {                                                   // as in paged_chunk_kernel, in tiles of 128 rows
+    int before = 0;
+    for (int r0 = 0; r0 < a.n_seqs; r0 += 32) {
+      const int r = r0 + lane;
+      const int c0 = r < a.n_seqs ? a.cu[r] : 0, c1 = r < a.n_seqs ? a.cu[r + 1] : 0, len = c1 - c0;
+      const int tiles = (len << p.group_shift) > 16 ? (len + per_tile - 1) / per_tile : 0;
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const int first = before + incl - tiles;
+      if (tiles > 0 && tile_at >= first && tile_at < first + tiles) {
+        const int off = (tile_at - first) * per_tile;
+        s_tile[0] = c0 + off;
+        s_tile[1] = min(per_tile, len - off);
+      }
+      before += __shfl_sync(0xffffffffu, incl, 31);
+      if (before > tile_at) break;
+    }
+    if (lane == 0 && before <= tile_at) s_tile[1] = 0;               // more tiles launched than there are
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem_O = tmem, tmem_S = tmem + 128, tmem_P = tmem + 256;      // S: 2 x 64 columns; P: 2 x 3 x 32
+  const int t0 = s_tile[0], n = s_tile[1];
+  if (n == 0) {
+    if (warp == 2) tmem_dealloc<512>(tmem);
+    return;
+  }
+  const int n_rows = n << p.group_shift;
+  int max_vis = 0, min_vis = 0x7fffffff;
+  for (int i = lane; i < n; i += 32) {
+    const int v = a.tok_len[t0 + i];
+    max_vis = max(max_vis, v);
+    min_vis = min(min_vis, v);
+  }
+  max_vis = __reduce_max_sync(0xffffffffu, max_vis);
+  min_vis = __reduce_min_sync(0xffffffffu, min_vis);
+  const int per = ((max_vis + p.splits - 1) / p.splits + kStageKeys - 1) / kStageKeys * kStageKeys;
+  const int k0 = rank * per, k1 = min(max_vis, k0 + per), n_st = k1 > k0 ? (k1 - k0 + kStageKeys - 1) / kStageKeys : 0;
+  const int32_t* bt = a.block_table + static_cast<int64_t>(a.tok_req[t0]) * a.max_blocks;
+  uint8_t *sQ = smem, *sK = smem + L::kKOff, *sV = smem + L::kVOff;
+  int n_loaded = 0;                                                  // warp 0: stages whose copies it has started
+  auto out_row = [&](int row) {
+    return static_cast<uint16_t*>(a.out) + (static_cast<int64_t>(t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D;
+  };
+  float m = -INFINITY, l = 0.f;                                      // softmax threads: the row's
+
+  if (warp == 0) {
+    // ---- copies: a lane per page
+    const int box = min(a.block_size, kStageKeys);
+    fence_proxy_async_all();                                         // the new keys were written by plain stores
+    for (; n_loaded < n_st; ++n_loaded) {
+      const int st = n_loaded % kS, key = k0 + n_loaded * kStageKeys + lane * box;
+      const bool mine = lane * box < kStageKeys && key < k1;
+      const int pages = __popc(__ballot_sync(0xffffffffu, mine));
+      int slot = 0;
+      if (mine) {
+        const int blk = p.bs_shift >= 0 ? key >> p.bs_shift : key / a.block_size;
+        slot = bt[blk] * a.block_size + (key - blk * a.block_size);
+      }
+      wide_wait(&k_empty[st], ((n_loaded / kS) & 1) ^ 1, failed);
+      wide_wait(&v_empty[st], ((n_loaded / kS) & 1) ^ 1, failed);
+      if (__any_sync(0xffffffffu, *failed != 0)) break;
+      for (int kv = 0; kv < 2; ++kv) {
+        uint64_t* full = kv == 0 ? &k_full[st] : &v_full[st];
+        if (lane == 0) mbar_arrive_expect_tx(full, pages * box * D * 2);
+        __syncwarp();
+        if (mine) {
+          uint8_t* dst = (kv == 0 ? sK : sV) + st * L::kKV + lane * box * 128;
+          for (int c = 0; c < L::kDC; ++c) tma_load_3d(kv == 0 ? &map_k : &map_v, full, dst + c * (kStageKeys * 128), c * 64, hk, slot);
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp == 1) {
+    // ---- S = Q K^T
+    constexpr uint32_t idesc = make_idesc_f16(kBf16, L::kRows, kStageKeys, false, false);
+    const uint64_t q_desc = make_smem_desc_sw128(smem_u32(sQ), 1024, 0), k_desc = make_smem_desc_sw128(smem_u32(sK), 1024, 0);
+    named_bar_sync(3, 288);                                          // the queries are in place
+    for (int j = 0; j < n_st; ++j) {
+      const int st = j % kS, b = j & 1;
+      wide_wait(&k_full[st], (j / kS) & 1, failed);
+      if (j >= 2) wide_wait(&s_read[b], ((j >> 1) - 1) & 1, failed);
+      if (__any_sync(0xffffffffu, *failed != 0)) break;
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k)
+          umma_f16_ss(tmem_S + b * kStageKeys, q_desc + (((k >> 2) * (L::kRows * 128) + (k & 3) * 32) >> 4),
+                      k_desc + ((st * L::kKV + (k >> 2) * (kStageKeys * 128) + (k & 3) * 32) >> 4), idesc, k != 0 ? 1u : 0u);
+        umma_commit(&s_full[b]);
+        umma_commit(&k_empty[st]);
+      }
+      __syncwarp();
+    }
+  } else if (warp == 2) {
+    // ---- O += P V, part by part
+    constexpr uint32_t idesc = make_idesc_f16(kBf16, L::kRows, D, false, true);
+    const uint64_t v_desc = make_smem_desc_sw128(smem_u32(sV), 1024, kStageKeys * 128);
+    for (int j = 0; j < n_st; ++j) {
+      const int st = j % kS, b = j & 1;
+      wide_wait(&v_full[st], (j / kS) & 1, failed);
+      wide_wait(&p_ready[b], (j >> 1) & 1, failed);
+      if (__any_sync(0xffffffffu, *failed != 0)) break;
+      tc_fence_after();
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < kStageKeys / 16; ++k)
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            umma_f16_ts(tmem_O, tmem_P + b * 96 + q * 32 + k * 8, v_desc + ((st * L::kKV + k * 16 * 128) >> 4), idesc, j != 0 || k != 0 || q != 0 ? 1u : 0u);
+        umma_commit(&pv_done[b]);
+        umma_commit(&v_empty[st]);
+      }
+      __syncwarp();
+    }
+  } else if (warp >= 4) {
+    // ---- softmax: half of a stage's keys of a row
+    const int tid = threadIdx.x - 128, half = tid >> 7, quad = warp & 3, r = quad * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
+    for (int i = tid; i < L::kRows * (D / 8); i += 256) {            // queries, 16 bytes at a time, 128B-swizzled
+      const int row = i / (D / 8), ch = i % (D / 8);
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      if (row < n_rows) {
+        w = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(a.q) +
+                                            (static_cast<int64_t>(t0 + (row >> p.group_shift)) * np + hk * G + (row & (G - 1))) * D + ch * 8);
+        w.x = (w.x & p.q_keep) ^ p.q_sign; w.y = (w.y & p.q_keep) ^ p.q_sign; w.z = (w.z & p.q_keep) ^ p.q_sign; w.w = (w.w & p.q_keep) ^ p.q_sign;
+      }
+      st_shared_v4(smem_u32(sQ) + (ch >> 3) * (L::kRows * 128) + row * 128 + (((ch & 7) ^ (row & 7)) << 4), w.x, w.y, w.z, w.w);
+    }
+    fence_proxy_async_smem();
+    named_bar_sync(3, 288);
+    const int vis = r < n_rows ? a.tok_len[t0 + (r >> p.group_shift)] : 0;
+    const float sc = a.scale_log2;
+    const uint32_t tO = tmem_O + half * (D / 2) + lanes;
+    for (int j = 0; j < n_st; ++j) {
+      const int b = j & 1, kb = k0 + j * kStageKeys;
+      uint32_t v[32];
+      float s[32];
+      wide_wait(&s_full[b], (j >> 1) & 1, failed);
+      tc_fence_after();
+      tmem_ld_32x32(tmem_S + b * kStageKeys + half * 32 + lanes, v);
+      tmem_ld_wait();
+      tc_fence_before();
+      wide_arrive(&s_read[b]);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) s[i] = __uint_as_float(v[i]);
+      bool odd = false;
+      if (kb + kStageKeys > min_vis || kb + kStageKeys > k1) {
+        const int lim = min(vis, k1) - kb - half * 32;
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (i >= lim) s[i] = -INFINITY;
+        // V of keys that nobody sees, and values that only some rows see and that are not finite: not as zero times infinity
+        wide_wait(&v_full[j % kS], (j / kS) & 1, failed);
+        const int from = max(0, min(min_vis, k1) - kb), none = k1 - kb;
+        uint8_t* tile = sV + (j % kS) * L::kKV;
+        bool found = false;
+        for (int i = tid; i < (kStageKeys - from) * (D / 8); i += 256) {
+          const int row = from + i / (D / 8), ch = i % (D / 8);
+          uint4* at = reinterpret_cast<uint4*>(tile + (ch >> 3) * (kStageKeys * 128) + row * 128 + (((ch & 7) ^ (row & 7)) << 4));
+          if (row >= none) {
+            *at = make_uint4(0u, 0u, 0u, 0u);
+          } else if (n > 1) {
+            const uint32_t e = kBf16 ? 0x7f80u : 0x7c00u;
+            uint4 w4 = *at;
+            uint32_t ws[4] = {w4.x, w4.y, w4.z, w4.w};
+            bool here = false;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              if ((ws[q] & e) == e) { ws[q] &= 0xffff0000u; here = true; }
+              if (((ws[q] >> 16) & e) == e) { ws[q] &= 0x0000ffffu; here = true; }
+            }
+            if (here) {
+              *at = make_uint4(ws[0], ws[1], ws[2], ws[3]);
+              found = true;
+            }
+          }
+        }
+        fence_proxy_async_smem();
+        odd = wide_any(found);
+      }
+      float mx = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
+      float* slot = s_ex + (j & 1) * (2 * L::kRows);
+      slot[half * L::kRows + r] = mx;
+      named_bar_sync(4 + quad, 64);                                  // the two warps of these rows
+      const float mn = fmaxf(m, fmaxf(mx, slot[(half ^ 1) * L::kRows + r]));
+      const bool grow = mn > m && !((mn - m) * sc <= kSlack);        // from nothing at the first visible key: the difference is infinite
+      if (__any_sync(0xffffffffu, grow)) {
+        const float corr = grow ? exp2f((m - mn) * sc) : 1.f;        // also of a row without a key so far: its sums are zero
+        if (grow) m = mn;
+        l *= corr;
+        if (j > 0) {
+          wide_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, failed);
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) {
+            uint32_t o[16];
+            tmem_ld_32x16(tO + c * 16, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+            tmem_st_32x16(tO + c * 16, o);
+          }
+        }
+      }
+      const float use = m == -INFINITY ? 0.f : m;                    // nothing visible yet: keep the arithmetic finite
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        s[i] = exp2f((s[i] - use) * sc) * kUnit;
+        sum += s[i];
+      }
+      l += sum;
+      if (j >= 2) {
+        wide_wait(&pv_done[b], ((j >> 1) - 1) & 1, failed);
+        tc_fence_after();
+      }
+      const uint32_t tP = tmem_P + b * 96 + half * 16 + lanes;
+      {
+        float x[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = s[i];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          uint32_t part[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            part[i] = pack2<kBf16>(x[2 * i], x[2 * i + 1]);
+            const float2 h = unpack2<kBf16>(part[i]);
+            x[2 * i] -= h.x;
+            x[2 * i + 1] -= h.y;
+          }
+          tmem_st_32x16(tP + q * 32, part);
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      wide_arrive(&p_ready[b]);
+      if (odd) {                                                     // what was taken out of V, by hand: one half's keys, then the other's
+        wide_wait(&pv_done[b], (j >> 1) & 1, failed);
+        tc_fence_after();
+        for (int turn = 0; turn < 2; ++turn) {
+          if (turn == half) {
+            for (int c = 0; c < D / 16; ++c) {
+              uint32_t o[16];
+              tmem_ld_32x16(tmem_O + c * 16 + lanes, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const int key = kb + half * 32 + i;
+                if (key >= min(vis, k1) || key < min_vis) continue;
+                const int blk = key / a.block_size;
+                const uint16_t* src = static_cast<const uint16_t*>(a.v_cache) +
+                                      ((static_cast<int64_t>(bt[blk]) * a.block_size + (key - blk * a.block_size)) * a.ng + hk) * D + c * 16;
+#pragma unroll
+                for (int d = 0; d < 16; ++d) {
+                  const uint16_t raw = src[d], e = kBf16 ? 0x7f80 : 0x7c00;
+                  if ((raw & e) == e) o[d] = __float_as_uint(fmaf(s[i], unpack2<kBf16>(raw).x, __uint_as_float(o[d])));
+                }
+              }
+              __syncwarp();
+              tmem_st_32x16(tmem_O + c * 16 + lanes, o);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+          }
+          named_bar_sync(2, 256);
+          tc_fence_after();
+        }
+      }
+    }
+    if (n_st > 0) {
+      wide_wait(&pv_done[(n_st - 1) & 1], ((n_st - 1) >> 1) & 1, failed);
+      tc_fence_after();
+    }
+    float* slot = s_ex + (n_st & 1) * (2 * L::kRows);
+    slot[half * L::kRows + r] = l;
+    named_bar_sync(4 + quad, 64);
+    l = slot[r] + slot[L::kRows + r];
+    if (p.splits == 1) {
+      const float inv = l > 0.f ? 1.f / l : l;                       // 0 without keys; NaN stays NaN
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) {
+        uint32_t o[32];
+        if (n_st > 0) {
+          tmem_ld_32x32(tO + c * 32, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+        }
+        if (r < n_rows) {
+          uint4* dst = reinterpret_cast<uint4*>(out_row(r) + half * (D / 2) + c * 32);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              w[i] = pack2<kBf16>(__uint_as_float(o[u * 8 + 2 * i]) * inv, __uint_as_float(o[u * 8 + 2 * i + 1]) * inv);
+            dst[u] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+    } else {
+      // the cluster's partials, over the ring: every product has been made
+      named_bar_sync(2, 256);
+      float* part = reinterpret_cast<float*>(smem + L::kKOff) + r * D + half * (D / 2);
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) {
+        uint32_t o[32];
+        if (n_st > 0) {
+          tmem_ld_32x32(tO + c * 32, o);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) reinterpret_cast<uint4*>(part + c * 32)[i] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+      }
+      if (half == 0) {
+        reinterpret_cast<float*>(smem + L::kStatOff)[r] = m;
+        reinterpret_cast<float*>(smem + L::kStatOff)[L::kRows + r] = l;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*failed) {                                                     // every wait is over, so all threads read the same
+    volatile int never = 0;
+    if (threadIdx.x == 0) atomicExch(&g_paged_error, 1);
+    if (warp == 0) {
+      for (int i = max(0, n_loaded - kS); i < n_loaded; ++i) {
+        wide_wait(&k_full[i % kS], (i / kS) & 1, &never);
+        wide_wait(&v_full[i % kS], (i / kS) & 1, &never);
+      }
+    } else if (warp == 1 || warp == 2) {
+      if (elect_one()) umma_commit(drained);
+      wide_wait(drained, 0, &never);
+    } else if (warp >= 4) {
+      const float nan = __int_as_float(0x7fffffff);
+      for (int i = threadIdx.x - 128; i < n_rows * (D / 8); i += 256)
+        *reinterpret_cast<uint4*>(out_row(i / (D / 8)) + i % (D / 8) * 8) = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+      if (threadIdx.x - 128 < L::kRows) {                            // for the cluster: a sum that is not a number
+        reinterpret_cast<float*>(smem + L::kStatOff)[threadIdx.x - 128] = 0.f;
+        reinterpret_cast<float*>(smem + L::kStatOff)[L::kRows + threadIdx.x - 128] = nan;
+      }
+    }
+    __syncthreads();
+  }
+  if (warp == 2) tmem_dealloc<512>(tmem);
+  if (p.splits == 1) return;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  const float* part = reinterpret_cast<const float*>(smem + L::kKOff);
+  const float* s_m = reinterpret_cast<const float*>(smem + L::kStatOff);
+  const float* s_l = s_m + L::kRows;
+  for (int idx = rank * kWideThreads + threadIdx.x; idx < n_rows * (D / 4); idx += p.splits * kWideThreads) {
+    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+    Merge x(a.scale_log2);
+    for (int c = 0; c < p.splits; ++c) x.M = fmaxf(x.M, *cluster.map_shared_rank(s_m + row, c));
+    if (x.M > -INFINITY) {
+      for (int c = 0; c < p.splits; ++c)
+        x.add(*cluster.map_shared_rank(s_m + row, c), *cluster.map_shared_rank(s_l + row, c),
+              *cluster.map_shared_rank(reinterpret_cast<const float4*>(part + row * D + col), c));
+    }
+    *reinterpret_cast<uint2*>(out_row(row) + col) = x.result<kBf16>();
+  }
+  cluster.sync();                                                    // no CTA leaves while another reads its partials
+}
+
 // new keys and values [T, ng, d] (any token and head strides) into their cache rows, 16 bytes per thread
 // kCount: counters of the decode kernel are set to zero too.  Kernels of their own: with the few instructions more, steps that need no counters took 1.2 to
 // 1.8 us longer (81 requests of up to 182 keys x 12 heads of 128: 21.7 -> 23.5)
@@ -783,8 +1249,8 @@ __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restric
 }
 
 // in the stream's order, but for what the kernels' own waits leave open (await_previous)
-template <typename K>
-int launch(K kern, unsigned ctas, int threads, int smem, int cluster, const PagedParams& p, cudaStream_t s) {
+template <typename K, typename... Args>
+int launch(K kern, unsigned ctas, int threads, int smem, int cluster, cudaStream_t s, const Args&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
@@ -798,7 +1264,7 @@ int launch(K kern, unsigned ctas, int threads, int smem, int cluster, const Page
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
   if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
 }
@@ -813,7 +1279,39 @@ int launch_chunks(const PagedParams& p, cudaStream_t s) {
   if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
   const int64_t ctas = static_cast<int64_t>(p.n_tiles) * p.a.ng * p.splits;
   if (ctas > 0x7fffffff) { g_paged_err = "paged attention: too many tiles"; return -12; }
-  return launch(kern, static_cast<unsigned>(ctas), 128, Smem<D>::kTotal, p.splits, p, s);
+  return launch(kern, static_cast<unsigned>(ctas), 128, Smem<D>::kTotal, p.splits, s, p);
+}
+
+// the pages of a cache as boxes of up to 64 slots x 64 values of one head
+bool page_map(CUtensorMap* map, const void* cache, const PagedAttnArgs& a) {
+  typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                               const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const EncodeFn fn = [] {
+    void* ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<EncodeFn>(ptr) : nullptr;
+  }();
+  if (fn == nullptr) return false;
+  ensure_cuda_context();
+  const cuuint64_t d = a.head_dim, ng = a.ng;
+  const cuuint64_t dims[3] = {d, ng, static_cast<cuuint64_t>(a.n_slots)}, strides[2] = {d * 2, d * ng * 2};
+  const cuuint32_t box[3] = {64, 1, static_cast<cuuint32_t>(a.block_size < kStageKeys ? a.block_size : kStageKeys)}, step[3] = {1, 1, 1};
+  return fn(map, a.is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(cache), dims, strides, box, step,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int D, bool kBf16>
+int launch_wide(const PagedParams& p, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t s) {
+  auto kern = paged_wide_kernel<D, kBf16>;
+  static const cudaError_t ready = [&] {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WideSmem<D>::kTotal);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  }();
+  if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
+  const int64_t ctas = static_cast<int64_t>(p.n_tiles) * p.a.ng * p.splits;
+  if (ctas > 0x7fffffff) { g_paged_err = "paged attention: too many tiles"; return -12; }
+  return launch(kern, static_cast<unsigned>(ctas), kWideThreads, WideSmem<D>::kTotal, p.splits, s, mk, mv, p);
 }
 
 template <int D, bool kBf16>
@@ -830,15 +1328,15 @@ int launch_decode(const PagedParams& p, cudaStream_t s) {
     return -12;
   }
   const unsigned items = static_cast<unsigned>(p.n_tiles * p.a.ng);
-  return launch(p.splits > 0 ? cut : whole, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, p, s);
+  return launch(p.splits > 0 ? cut : whole, p.splits > 0 ? p.splits : items, 128, Smem<D>::kTotal, 1, s, p);
 }
 
 template <int D, bool kBf16>
 int launch_rows(const PagedParams& p, cudaStream_t s) {
   const unsigned items = static_cast<unsigned>(p.n_tiles * p.a.ng);
-  if (p.a.group == 1) return launch(paged_rows_kernel<D, 1, kBf16>, items, 128, 0, 1, p, s);
-  if (p.a.group == 2) return launch(paged_rows_kernel<D, 2, kBf16>, items, 128, 0, 1, p, s);
-  return launch(paged_rows_kernel<D, 4, kBf16>, items, 128, 0, 1, p, s);
+  if (p.a.group == 1) return launch(paged_rows_kernel<D, 1, kBf16>, items, 128, 0, 1, s, p);
+  if (p.a.group == 2) return launch(paged_rows_kernel<D, 2, kBf16>, items, 128, 0, 1, s, p);
+  return launch(paged_rows_kernel<D, 4, kBf16>, items, 128, 0, 1, s, p);
 }
 
 int log2_exact(int v) {
@@ -857,11 +1355,11 @@ int64_t decode_keys(const PagedAttnArgs& a) {
 // the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Short contexts are not cut at all
 // (0): putting parts together then costs as much as the imbalance that it removes.  us, whole / cut, heads of 128: 90 requests of up to 300 keys x 8
 // heads 35.8 / 42.0, 40 of up to 429 x 4 beside chunks 29.1 / 40.9, 2 of up to 430 x 8 beside one 26.5 /
-// 30.7, but 1 of 500 x 8 21.5 / 17.4, 8 of up to 700 27.6 / 21.5; a stage of heads of 64 takes
+// 30.7, 9 of up to 373 x 4 14.4 / 16.5, but 1 of 500 x 8 21.5 / 17.4, 8 of up to 700 27.6 / 21.5; a stage of heads of 64 takes
 // half as long: 10 of up to 824 x 12 beside chunks 21.9 / 29.3, 1 of 522 x 8 10.3 / 12.4
 int decode_ctas(const PagedAttnArgs& a) {
   const int64_t items = decode_items(a), longest = (decode_keys(a) + kStageKeys - 1) / kStageKeys;
-  const bool whole = a.head_dim == 64 ? longest <= (items <= kDecodeCtas ? 16 : 8) : longest <= (items <= 64 && !a.beside_chunks ? 4 : 8);
+  const bool whole = a.head_dim == 64 ? longest <= (items <= kDecodeCtas ? 16 : 8) : longest <= (items <= 16 && !a.beside_chunks ? 4 : 8);
   if (whole) return 0;
   const int64_t n = items * longest / 2;
   return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
@@ -891,6 +1389,17 @@ bool paged_decode_by_rows(const PagedAttnArgs& a) {
   }
   if (a.group == 2) return keys <= (many ? (narrow ? 640 : 160) : 32);
   return a.group == 4 && many && keys <= 32;
+}
+
+// Whether chunks go by tiles of 128 rows on tcgen05: where a stage of 64 keys is whole pages, or a piece of one, on 8-row boundaries of the swizzle
+bool paged_wide_tiles(const PagedAttnArgs& a) {
+  return a.wide_tiles > 0 && a.n_slots > 0 && a.n_slots <= 0x7fffffff && a.block_size % 8 == 0 &&
+         (kStageKeys % a.block_size == 0 || a.block_size % kStageKeys == 0);
+}
+
+int paged_status() {
+  int v = 0;
+  return cudaMemcpyFromSymbol(&v, g_paged_error, sizeof(int)) == cudaSuccess ? v : -1;
 }
 
 bool paged_attention_supported(int head_dim, int group) {
@@ -926,7 +1435,15 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
   p.q_sign = a.scale_log2 < 0.f ? 0x80008000u : 0u;
   p.group_shift = log2_exact(a.group);
   p.bs_shift = log2_exact(a.block_size);
-  if (a.cu != nullptr && chunk_tiles > 0) {
+  CUtensorMap mk, mv;
+  if (a.cu != nullptr && chunk_tiles > 0 && paged_wide_tiles(a) && page_map(&mk, a.k_cache, a) && page_map(&mv, a.v_cache, a)) {
+    p.n_tiles = a.wide_tiles;
+    p.splits = 1;
+    while (2 * p.splits <= a.wide_splits && p.splits < 16) p.splits *= 2;
+    const int rc = a.head_dim == 128 ? (a.is_bf16 ? launch_wide<128, true>(p, mk, mv, s) : launch_wide<128, false>(p, mk, mv, s))
+                                     : (a.is_bf16 ? launch_wide<64, true>(p, mk, mv, s) : launch_wide<64, false>(p, mk, mv, s));
+    if (rc != 0) return rc;
+  } else if (a.cu != nullptr && chunk_tiles > 0) {
     p.n_tiles = chunk_tiles;
     p.splits = 1;
     while (2 * p.splits <= chunk_splits && p.splits < 16) p.splits *= 2;

@@ -327,6 +327,18 @@ class DynamicInferenceContext:
                 max(keys, default=0), sum(keys) // max(1, len(few)), all(p[2] == 1 for p in few))
         return plan
 
+    def _wide_plan(self, group: int, ng: int, d: int) -> tuple:
+        """The portions' tiles of 128 rows and key ranges of those, for the kernel that has one such tile on an SM; no tiles where the contexts
+        are so short that its start (12.4 us a step against 8.3 to 10.4) costs more than its stages give.  us, 64-row / 128-row tiles, 32 / 8 heads of 128:
+        one portion of 100 13.6 / 14.4, of 150 16.5 / 14.5; 12 heads of 64: one of 220 14.4 / 16.5, four with up to 300 keys 20.0 / 18.5."""
+        plan = self._paged_plans.get((group, ng, d, "wide"))
+        if plan is None:
+            chunks = [p for p in self._plan if p[2] * group > 16]
+            longest = max((p[2] + p[3] for p in chunks), default=0)
+            tiles = sum(-(-p[2] * group // 128) for p in chunks) if longest >= (160 if d == 128 else 256) else 0
+            plan = self._paged_plans[(group, ng, d, "wide")] = (tiles, key_ranges(2 * tiles * ng, longest))
+        return plan
+
     # -- attention over the paged cache --------------------------------------------
     def attend(self, layer: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
         """``q [T, np, hn]``, new ``k / v [T, ng, hn(v)]`` -> ``[T, np, hn_v]``; writes k / v into their pages first."""
@@ -350,7 +362,8 @@ class DynamicInferenceContext:
                     vc[self._write_slots] = v
                     new = (None, None, None)
                 return ext.paged_attention(q.contiguous(), kc, vc, self._block_table, self._tok_req, self._tok_len,
-                                           self.block_size, float(scale), decode, *new, self.packed.cu, chunk_tiles, chunk_splits, *contexts)
+                                           self.block_size, float(scale), decode, *new, self.packed.cu, chunk_tiles, chunk_splits, *contexts,
+                                           *self._wide_plan(np_ // ng, ng, q.shape[-1]))
         kc[self._write_slots] = k
         vc[self._write_slots] = v
         self._ensure_gather(q.device)

@@ -1,0 +1,45 @@
+"""Chunks in tiles of 128 rows: page sizes around a stage of 64 keys, rows around a tile, key ranges, and cache rows that no token may see."""
+import pytest
+import torch
+
+from test_paged_attention_gpu import _oracle, _step
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reqs,hq,hkv,d,block,dtype", [
+    ([(0, 127), (64, 128), (165, 129)], 2, 2, 64, 8, torch.bfloat16),            # a row less and more than a tile, the smallest pages
+    ([(63, 200), (0, 70)], 4, 4, 128, 64, torch.float16),                        # a page is a stage
+    ([(300, 90), (1, 80)], 8, 2, 128, 128, torch.bfloat16),                      # a page is two
+    ([(191, 33), (192, 64), (1000, 1)], 8, 1, 64, 32, torch.float16),            # 16 tokens a tile, stages that end with the context
+    ([(5000, 150)], 4, 1, 128, 16, torch.bfloat16),                              # key ranges in a cluster
+    ([(1500, 300), (2, 300)], 2, 1, 64, 16, torch.bfloat16)])                    # a tile whose later ranges are empty
+def test_wide_tiles(reqs, hq, hkv, d, block, dtype):
+    from megatronapp_b200 import ops
+
+    cx, q, k, v = _step(reqs, hq, hkv, d, block, dtype)
+    kc, vc = cx.kv[1]
+    seen = torch.zeros(kc.shape[0], dtype=torch.bool, device="cuda")
+    for i, (a, n) in enumerate(reqs):
+        seen[(torch.tensor(cx.seqs[str(i)].blocks).unsqueeze(1) * block + torch.arange(block)).view(-1)[:a + n].cuda()] = True
+    kc[~seen], vc[~seen] = float("nan"), float("inf")              # pages of nobody, and what lies behind the last token
+    want, _, _ = _oracle(cx, reqs, q, k, v, d ** -0.5, block)
+    got = cx.attend(1, q, k, v, d ** -0.5)
+    unit = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11    # the result's own rounding, as in the tests of the other tiles
+    assert float((got.double() - want).abs().max()) <= unit * max(1.0, float(want.abs().max()))
+    assert float((got.double() - want).norm()) <= 0.5 * unit * float(want.norm())
+    assert ops.ext().paged_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_values_of_later_tokens_stay_out_of_wide_tiles(dtype):
+    """Values that are not finite, in both halves of a stage and in its first and last key."""
+    reqs = [(60, 260)]
+    cx, q, k, v = _step(reqs, 8, 2, 128, 16, dtype)
+    v[4, 0, 5], v[67, 0, 127], v[68, 1, 64], v[140, 1, 63] = float("inf"), float("-inf"), float("nan"), float("inf")
+    want, _, _ = _oracle(cx, reqs, q, k, v, 0.1, 16)
+    got = cx.attend(1, q, k, v, 0.1).double()
+    assert torch.equal(torch.isfinite(got), torch.isfinite(want))
+    ok = torch.isfinite(want)
+    assert ok[:4].all() and not ok[4:, :4, 5].any() and ok[:68, 4:].all()
+    assert float((got[ok] - want[ok]).abs().max()) <= 2.0 ** -7
