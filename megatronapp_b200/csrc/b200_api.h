@@ -349,6 +349,10 @@ int paged_status();          // 1: a kernel of this process gave up on a wait (i
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s);
 const char* paged_attention_last_error();
 
+// ranges [n][3]: first byte, byte behind the last (even ones), blocks of kZeroBlockBytes before it (counted from 16-byte boundaries)
+constexpr int64_t kZeroBlockBytes = 65536;
+void zero_ranges(void* base, const int64_t* ranges, int n, int64_t blocks, cudaStream_t s);
+
 // ---------------------------------------------------------------- MoE (moe.cu)
 void moe_router_topk_fwd(const float* logits, float* probs, uint8_t* map, int32_t* tokens_per_expert, int n, int E, int k,
                          bool pre_softmax, float scaling, cudaStream_t s);

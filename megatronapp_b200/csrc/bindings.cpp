@@ -1262,6 +1262,28 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout_bwd", &dropout_bwd);
   m.def("rope_apply", &rope_apply);
   m.def("bias_grad", &bias_grad);
+  m.def("zero_ranges_plan", [](int64_t element_size, const std::vector<std::pair<int64_t, int64_t>>& ranges) {
+    // rows of zero_ranges' table, and the blocks that it takes
+    TORCH_CHECK(element_size % 2 == 0, "zero_ranges: elements of two or more bytes");
+    Tensor t = at::empty({static_cast<int64_t>(ranges.size()), 3}, at::kLong);
+    int64_t blocks = 0, *row = t.data_ptr<int64_t>();
+    for (const auto& [from, to] : ranges) {
+      TORCH_CHECK(0 <= from && from < to, "zero_ranges: empty range");
+      *row++ = from * element_size;
+      *row++ = to * element_size;
+      *row++ = blocks;
+      blocks += (to * element_size - from * element_size / 16 * 16 + b200::kZeroBlockBytes - 1) / b200::kZeroBlockBytes;
+    }
+    TORCH_CHECK(blocks <= 0x7fffffff, "zero_ranges: too large");
+    return std::make_pair(t, blocks);
+  });
+  m.def("zero_ranges", [](Tensor& data, const Tensor& ranges, int64_t blocks) {
+    c10::cuda::CUDAGuard guard(data.device());
+    TORCH_CHECK(data.is_cuda() && data.is_contiguous() && ranges.device() == data.device() && ranges.is_contiguous() && ranges.scalar_type() == at::kLong &&
+                ranges.dim() == 2 && ranges.size(1) == 3 && reinterpret_cast<uintptr_t>(data.data_ptr()) % 16 == 0, "zero_ranges: bad arguments");
+    b200::zero_ranges(data.data_ptr(), ranges.data_ptr<int64_t>(), static_cast<int>(ranges.size(0)), blocks, cur_stream());
+    count();
+  });
   m.def("router_linear_bwd", &router_linear_bwd);
   m.def("embedding_grad", &embedding_grad);
   m.def("ce_local_stats", &ce_local_stats);

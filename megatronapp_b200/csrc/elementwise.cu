@@ -1157,4 +1157,29 @@ void chunk_mean(const void* x, float* out, int64_t rows, int cols, int pixels, b
                            (const T*)x, out, rows, cols, pixels)));
 }
 
+namespace {
+// ranges [n][3]: first byte, byte behind the last (even ones), number of the first block.  A block of 256 threads takes 64 KB.  Bound by its stores: 159 MB
+// of a 50304 x 768 table's fp32 gradient among 17 ranges.
+__global__ void __launch_bounds__(256) zero_ranges_kernel(uint8_t* __restrict__ base, const int64_t* __restrict__ ranges, int n) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (ranges[3 * mid + 2] <= static_cast<int64_t>(blockIdx.x)) lo = mid;
+    else hi = mid - 1;
+  }
+  const int64_t from = ranges[3 * lo], to = ranges[3 * lo + 1];
+  const int64_t first = (from & ~int64_t(15)) + (blockIdx.x - ranges[3 * lo + 2]) * kZeroBlockBytes;
+  const int64_t last = first + kZeroBlockBytes < to ? first + kZeroBlockBytes : to;
+  for (int64_t at = first + threadIdx.x * 16; at < last; at += 256 * 16) {
+    if (at >= from && at + 16 <= to) *reinterpret_cast<uint4*>(base + at) = make_uint4(0u, 0u, 0u, 0u);
+    else
+      for (int64_t b = at < from ? from : at; b < at + 16 && b < to; b += 2) *reinterpret_cast<uint16_t*>(base + b) = 0;
+  }
+}
+}  // namespace
+
+void zero_ranges(void* base, const int64_t* ranges, int n, int64_t blocks, cudaStream_t s) {
+  if (blocks > 0) zero_ranges_kernel<<<static_cast<unsigned>(blocks), 256, 0, s>>>(static_cast<uint8_t*>(base), ranges, n);
+}
+
 }  // namespace b200
