@@ -331,13 +331,10 @@ class DynamicInferenceContext:
         """The portions' tiles of 128 rows and key ranges of those, for the kernel that has one such tile on an SM; no tiles where the contexts
         are so short that its start (12.4 us a step against 8.3 to 10.4) costs more than its stages give.  us, 64-row / 128-row tiles, 32 / 8 heads of 128:
         one portion of 100 13.6 / 14.4, of 150 16.5 / 14.5; 12 heads of 64: one of 220 14.4 / 16.5, four with up to 300 keys 20.0 / 18.5."""
-        plan = self._paged_plans.get((group, ng, d, "wide"))
-        if plan is None:
-            chunks = [p for p in self._plan if p[2] * group > 16]
-            longest = max((p[2] + p[3] for p in chunks), default=0)
-            tiles = sum(-(-p[2] * group // 128) for p in chunks) if longest >= (160 if d == 128 else 256) else 0
-            plan = self._paged_plans[(group, ng, d, "wide")] = (tiles, key_ranges(2 * tiles * ng, longest))
-        return plan
+        chunks = [p for p in self._plan if p[2] * group > 16]
+        longest = max((p[2] + p[3] for p in chunks), default=0)
+        tiles = sum(-(-p[2] * group // 128) for p in chunks) if longest >= (160 if d == 128 else 256) else 0
+        return tiles, key_ranges(2 * tiles * ng, longest)
 
     # -- attention over the paged cache --------------------------------------------
     def attend(self, layer: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
@@ -347,13 +344,21 @@ class DynamicInferenceContext:
             self.kv[layer] = (torch.zeros(n_slots, *k.shape[1:], dtype=k.dtype, device=k.device),
                               torch.zeros(n_slots, *v.shape[1:], dtype=v.dtype, device=v.device))
         kc, vc = self.kv[layer]
-        np_, ng = q.shape[1], k.shape[1]
-        if q.is_cuda and self.use_paged_kernel and k.shape[-1] == v.shape[-1] == q.shape[-1] and q.dtype in (torch.bfloat16, torch.float16):
+        (_, np_, d), ng = q.shape, k.shape[1]
+        if q.is_cuda and self.use_paged_kernel and k.shape[-1] == v.shape[-1] == d and q.dtype in (torch.bfloat16, torch.float16):
             from .. import ops
 
             ext = ops.ext()
-            if ext.paged_attention_supported(q.shape[-1], np_ // ng):
-                decode, chunk_tiles, chunk_splits, *contexts = self._paged_plan(np_ // ng, ng)
+            heads = (np_ // ng, ng, d)
+            plan = self._paged_plans.get(heads)                        # made once a step: () where the kernels do not take the heads
+            if plan is None:
+                plan = ()
+                if ext.paged_attention_supported(d, np_ // ng):
+                    decode, *cuts = self._paged_plan(np_ // ng, ng)
+                    plan = (decode, (*cuts, *self._wide_plan(*heads)))
+                self._paged_plans[heads] = plan
+            if plan:
+                decode, cuts = plan
                 self.kernel_calls += 1
                 if k.dtype == v.dtype == q.dtype == kc.dtype and _rows_of_16_bytes(k) and _rows_of_16_bytes(v):
                     new = (k, v, self._write_slots)                    # written by the same call
@@ -362,8 +367,7 @@ class DynamicInferenceContext:
                     vc[self._write_slots] = v
                     new = (None, None, None)
                 return ext.paged_attention(q.contiguous(), kc, vc, self._block_table, self._tok_req, self._tok_len,
-                                           self.block_size, float(scale), decode, *new, self.packed.cu, chunk_tiles, chunk_splits, *contexts,
-                                           *self._wide_plan(np_ // ng, ng, q.shape[-1]))
+                                           self.block_size, float(scale), decode, *new, self.packed.cu, *cuts)
         kc[self._write_slots] = k
         vc[self._write_slots] = v
         self._ensure_gather(q.device)
