@@ -325,9 +325,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const uint64_t b0 = desc_at(v_desc, st * L::kTile);
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < kBlockKV / 16; ++k)
-              // A = P from TMEM: row = lane, 16 keys = 8 packed 32-bit columns per k-step
-              umma_f16_ts(tmem_O + t * D, tmem_P + t * 64 + k * 8, desc_at(b0, k * 16 * 128), idesc_o, k != 0 || j != 0 ? 1u : 0u);
+            for (int i = 0; i < kBlockKV / 16; ++i) {
+              // A = P from TMEM: row = lane, 16 keys = 8 packed 32-bit columns per k-step.  The first 32 keys of both halves go before the other 32: fp32
+              // sums depend on the order, and results stay what they are only while it does
+              const int k = (i >> 2) * 2 + ((i >> 1) & 1) * 4 + (i & 1);
+              umma_f16_ts(tmem_O + t * D, tmem_P + t * 64 + k * 8, desc_at(b0, k * 16 * 128), idesc_o, i != 0 || j != 0 ? 1u : 0u);
+            }
             umma_commit(&pv_done[t]);
             if (t == 1 || j >= nkv_1) umma_commit(&v_empty[st]);
           }
