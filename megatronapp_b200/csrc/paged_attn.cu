@@ -1435,6 +1435,13 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
   p.q_sign = a.scale_log2 < 0.f ? 0x80008000u : 0u;
   p.group_shift = log2_exact(a.group);
   p.bs_shift = log2_exact(a.block_size);
+  // Counters that no write kernel of this call has zeroed are zeroed in front of all launches: the first one waits for that, and the decode kernel
+  // beside chunks, which counts without a wait of its own, starts when all of theirs have
+  const int decode_cut = decode && !paged_decode_by_rows(a) ? decode_ctas(a) : 0;
+  if (decode_cut > 0 && !written) {
+    const cudaError_t e = cudaMemsetAsync(arrived_in(a, ws), 0, sizeof(int) * static_cast<size_t>(decode_items(a)), s);
+    if (e != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(e); return -13; }
+  }
   CUtensorMap mk, mv;
   if (a.cu != nullptr && chunk_tiles > 0 && paged_wide_tiles(a) && page_map(&mk, a.k_cache, a) && page_map(&mv, a.v_cache, a)) {
     p.n_tiles = a.wide_tiles;
@@ -1459,16 +1466,10 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
     return a.head_dim == 128 ? (a.is_bf16 ? launch_rows<128, true>(p, s) : launch_rows<128, false>(p, s))
                              : (a.is_bf16 ? launch_rows<64, true>(p, s) : launch_rows<64, false>(p, s));
   }
-  p.splits = decode_ctas(a);
+  p.splits = decode_cut;
   p.behind_write = written && !p.beside_chunks;
   p.ws = ws;
-  if (p.splits > 0) {
-    p.arrived = arrived_in(a, ws);
-    if (!written) {
-      const cudaError_t e = cudaMemsetAsync(p.arrived, 0, sizeof(int) * static_cast<size_t>(decode_items(a)), s);
-      if (e != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(e); return -13; }
-    }
-  }
+  if (p.splits > 0) p.arrived = arrived_in(a, ws);
   return a.head_dim == 128 ? (a.is_bf16 ? launch_decode<128, true>(p, s) : launch_decode<128, false>(p, s))
                            : (a.is_bf16 ? launch_decode<64, true>(p, s) : launch_decode<64, false>(p, s));
 }
