@@ -130,6 +130,23 @@ __device__ __forceinline__ void tma_reduce_add_2d(const void* tmap, const void* 
 // memory, until everything before it is complete and visible.
 __device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of what the kernel before may still have been writing when this one started: they stay behind the wait, and do not go by the read-only path, which
+// takes memory to be as it was when the kernel started
+__device__ __forceinline__ int32_t ld_awaited(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_awaited(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_awaited(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.b16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+  return v;
+}
 // 16 bytes to a shared-memory address
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");

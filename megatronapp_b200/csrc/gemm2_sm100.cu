@@ -178,7 +178,7 @@ __device__ __forceinline__ Tile2 tile_info(const P2& p, int tile) {
     const int r = tile - t.group * per_group;
     t.m_blk = r / p.num_n_blocks;
     t.n_blk = r - t.m_blk * p.num_n_blocks;
-    const int r0 = __ldg(p.group_offsets + t.group), r1 = __ldg(p.group_offsets + t.group + 1);
+    const int r0 = ld_awaited(p.group_offsets + t.group), r1 = ld_awaited(p.group_offsets + t.group + 1);
     t.kb0 = r0 / BK; t.kb1 = r1 / BK;
     t.valid = t.kb1 > t.kb0;
     return t;
@@ -198,11 +198,11 @@ __device__ __forceinline__ Tile2 tile_info(const P2& p, int tile) {
   t.valid = t.m_blk < p.num_m_blocks;          // the last L2 band may be partial
   if constexpr (kMode == kModeGroupM) {
     const int row0 = t.m_blk * 256;
-    const int total = __ldg(p.group_offsets + p.n_groups);
+    const int total = ld_awaited(p.group_offsets + p.n_groups);
     t.valid = t.valid && row0 < total;
     int e = 0;
     if (t.valid) {
-      while (e + 1 < p.n_groups && __ldg(p.group_offsets + e + 1) <= row0) ++e;
+      while (e + 1 < p.n_groups && ld_awaited(p.group_offsets + e + 1) <= row0) ++e;
     }
     t.group = e;
   }
@@ -538,7 +538,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + acc * BN;
       float rscale = 1.f;
       if constexpr (kMode == kModeGroupM) {
-        if (p.row_scale != nullptr) rscale = __ldg(p.row_scale + m0 + row_in_tile);
+        if (p.row_scale != nullptr) rscale = ld_awaited(p.row_scale + m0 + row_in_tile);
       }
       const uint16_t* bias_base = reinterpret_cast<const uint16_t*>(p.bias);
       if constexpr (kMode == kModeGroupM) {

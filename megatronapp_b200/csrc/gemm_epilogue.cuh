@@ -56,7 +56,7 @@ __device__ __forceinline__ void stage_row16(uint32_t row, int swz, const uint32_
 __device__ __forceinline__ uint32_t bias_pair(const uint16_t* bias, int col, int n, int lane) {
   col += 2 * lane;
   if (bias == nullptr || col >= n) return 0u;
-  return __ldg(bias + col) | (col + 1 < n ? static_cast<uint32_t>(__ldg(bias + col + 1)) << 16 : 0u);
+  return ld_awaited(bias + col) | (col + 1 < n ? ld_awaited(bias + col + 1) << 16 : 0u);
 }
 
 // one warp's two slabs and where they go: rows `row0` on of a matrix, nothing where these lie below it

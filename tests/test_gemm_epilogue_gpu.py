@@ -74,3 +74,38 @@ def test_launches_that_overlap():
         graph.replay()
         for got, ref in zip(outs, want):
             assert torch.equal(got, ref)
+
+
+def test_bias_scales_and_groups_that_the_launch_before_writes():
+    """What a product's epilogue reads beside its operands may be the result of the launch that it overlaps: other values each time, in the same buffers."""
+    from megatronapp_b200 import ops
+
+    g = torch.Generator().manual_seed(2)
+    cap, G, N, K = 1024, 3, 512, 256
+    a = [(torch.randn(256, K, generator=g) * (i + 1)).bfloat16().cuda() for i in range(4)]
+    b = torch.randn(max(N, cap), K, generator=g).bfloat16().cuda()
+    x, w = torch.randn(cap, K, generator=g).bfloat16().cuda(), torch.randn(G * N, K, generator=g).bfloat16().cuda()
+    offsets = torch.tensor([0, 256, 256, 1024], dtype=torch.int32, device="cuda")
+    y16, y32 = torch.empty(256, N, dtype=torch.bfloat16, device="cuda"), torch.empty(256, cap, device="cuda")
+
+    def chain(pause):
+        outs = []
+        for i in range(24):
+            z, zg = torch.empty(cap, N, dtype=torch.bfloat16, device="cuda"), torch.empty(cap, N, dtype=torch.bfloat16, device="cuda")
+            ops.gemm(a[i & 3], b[:N], out=y16)
+            pause()
+            ops.gemm(x, w[:N], out=z, bias=y16[i & 7])
+            pause()
+            ops.gemm(a[i & 3], b[:cap], out=y32, epilogue=2)
+            pause()
+            ops.ext().gemm_grouped(x, w, zg, offsets, 1, False, y16[:G], 0, None, y32[i & 7], G, N)
+            pause()
+            outs += [z, zg]
+        return outs
+
+    want = chain(torch.cuda.synchronize)
+    assert not torch.equal(want[0], want[2]) and not torch.equal(want[1], want[3])
+    z = x.double() @ w[:N].double().t() + (a[0].double() @ b[:N].double().t()).bfloat16()[0].double()
+    assert float((want[0].double() - z).abs().max()) <= 2.0 ** -7 * float(z.abs().max())
+    for _ in range(5):
+        assert all(torch.equal(p, q) for p, q in zip(chain(lambda: None), want))
