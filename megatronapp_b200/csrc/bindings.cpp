@@ -1325,6 +1325,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("slots") = py::none(), py::arg("cu") = py::none(), py::arg("chunk_tiles") = 0, py::arg("chunk_splits") = 1,
         py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false, py::arg("wide_tiles") = 0, py::arg("wide_splits") = 1);
   m.def("paged_status", []() { return b200::paged_status(); });
+  m.def("paged_wide_ranges", [](int tiles, int ranges, int ng, int head_dim, bool bf16) {
+    b200::PagedAttnArgs a{};
+    a.wide_tiles = tiles; a.wide_splits = ranges; a.ng = ng; a.head_dim = head_dim; a.is_bf16 = bf16;
+    int resident = 0;
+    const int taken = b200::paged_wide_ranges(a, &resident);
+    return std::make_pair(taken, resident);
+  });
   m.def("paged_decode_by_rows", [](int64_t requests, int ng, int group, int head_dim, int longest, int mean, bool single) {
     b200::PagedAttnArgs a{};
     const int32_t none = 0;

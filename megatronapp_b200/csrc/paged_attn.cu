@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
 #include <cmath>
 #include <string>
 
@@ -1249,22 +1250,28 @@ __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restric
 }
 
 // in the stream's order, but for what the kernels' own waits leave open (await_previous)
+struct Launch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2]{};
+  Launch(unsigned ctas, int threads, int smem, int cluster, cudaStream_t s) {
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+  }
+  Launch(const Launch&) = delete;
+};
 template <typename K, typename... Args>
 int launch(K kern, unsigned ctas, int threads, int smem, int cluster, cudaStream_t s, const Args&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[2]{};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  const Launch l(ctas, threads, smem, cluster, s);
+  const cudaError_t e = cudaLaunchKernelEx(&l.cfg, kern, args...);
   if (e != cudaSuccess) { g_paged_err = std::string("paged attention launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
 }
@@ -1302,16 +1309,53 @@ bool page_map(CUtensorMap* map, const void* cache, const PagedAttnArgs& a) {
 }
 
 template <int D, bool kBf16>
-int launch_wide(const PagedParams& p, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t s) {
-  auto kern = paged_wide_kernel<D, kBf16>;
-  static const cudaError_t ready = [&] {
+cudaError_t wide_ready() {
+  static const cudaError_t ready = [] {
+    auto kern = paged_wide_kernel<D, kBf16>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WideSmem<D>::kTotal);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   }();
-  if (ready != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(ready); return -10; }
+  return ready;
+}
+
+// how many clusters of 2^log CTAs of this kernel the device has room for at once (0: none, or it cannot say); asked once a device
+template <int D, bool kBf16>
+int wide_clusters(int log) {
+  constexpr int kDevices = 16;
+  static std::atomic<int> known[kDevices][5];                        // + 1
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
+  if (const int v = known[dev][log].load(std::memory_order_relaxed); v > 0) return v - 1;
+  if (wide_ready<D, kBf16>() != cudaSuccess) return 0;
+  const Launch l(1u << log, kWideThreads, WideSmem<D>::kTotal, 1 << log, nullptr);
+  if (cudaOccupancyMaxActiveClusters(&n, paged_wide_kernel<D, kBf16>, &l.cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  known[dev][log].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+int wide_clusters(const PagedAttnArgs& a, int log) {
+  return a.head_dim == 128 ? (a.is_bf16 ? wide_clusters<128, true>(log) : wide_clusters<128, false>(log))
+                           : (a.is_bf16 ? wide_clusters<64, true>(log) : wide_clusters<64, false>(log));
+}
+
+// A tile's key ranges are the CTAs of a cluster, which start together or not at all.  One CTA takes an SM, and a cluster's SMs lie side by side: of the 148, ones of 16
+// find room for fewer than nine.  So there are only as many ranges as let all clusters run at once.
+int wide_ranges(const PagedAttnArgs& a) {
+  const int64_t clusters = static_cast<int64_t>(a.wide_tiles) * a.ng;
+  int log = 0;
+  while (log < 4 && (2 << log) <= a.wide_splits) ++log;
+  while (log > 0 && wide_clusters(a, log) < clusters) --log;
+  return 1 << log;
+}
+
+template <int D, bool kBf16>
+int launch_wide(const PagedParams& p, const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t s) {
+  if (const cudaError_t e = wide_ready<D, kBf16>(); e != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(e); return -10; }
   const int64_t ctas = static_cast<int64_t>(p.n_tiles) * p.a.ng * p.splits;
   if (ctas > 0x7fffffff) { g_paged_err = "paged attention: too many tiles"; return -12; }
-  return launch(kern, static_cast<unsigned>(ctas), kWideThreads, WideSmem<D>::kTotal, p.splits, s, mk, mv, p);
+  return launch(paged_wide_kernel<D, kBf16>, static_cast<unsigned>(ctas), kWideThreads, WideSmem<D>::kTotal, p.splits, s, mk, mv, p);
 }
 
 template <int D, bool kBf16>
@@ -1397,6 +1441,14 @@ bool paged_wide_tiles(const PagedAttnArgs& a) {
          (kStageKeys % a.block_size == 0 || a.block_size % kStageKeys == 0);
 }
 
+int paged_wide_ranges(const PagedAttnArgs& a, int* resident) {
+  const int ranges = wide_ranges(a);
+  int log = 0;
+  while ((1 << log) < ranges) ++log;
+  *resident = wide_clusters(a, log);
+  return ranges;
+}
+
 int paged_status() {
   int v = 0;
   return cudaMemcpyFromSymbol(&v, g_paged_error, sizeof(int)) == cudaSuccess ? v : -1;
@@ -1445,8 +1497,7 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
   CUtensorMap mk, mv;
   if (a.cu != nullptr && chunk_tiles > 0 && paged_wide_tiles(a) && page_map(&mk, a.k_cache, a) && page_map(&mv, a.v_cache, a)) {
     p.n_tiles = a.wide_tiles;
-    p.splits = 1;
-    while (2 * p.splits <= a.wide_splits && p.splits < 16) p.splits *= 2;
+    p.splits = wide_ranges(a);
     const int rc = a.head_dim == 128 ? (a.is_bf16 ? launch_wide<128, true>(p, mk, mv, s) : launch_wide<128, false>(p, mk, mv, s))
                                      : (a.is_bf16 ? launch_wide<64, true>(p, mk, mv, s) : launch_wide<64, false>(p, mk, mv, s));
     if (rc != 0) return rc;

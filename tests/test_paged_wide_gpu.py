@@ -43,3 +43,22 @@ def test_values_of_later_tokens_stay_out_of_wide_tiles(dtype):
     ok = torch.isfinite(want)
     assert ok[:4].all() and not ok[4:, :4, 5].any() and ok[:68, 4:].all()
     assert float((got[ok] - want[ok]).abs().max()) <= 2.0 ** -7
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [64, 128])
+def test_all_clusters_find_room(d):
+    """No more key ranges than let the clusters of all (tile, head) pairs run at once, and no fewer."""
+    from megatronapp_b200 import ops
+
+    plan = ops.ext().paged_wide_ranges
+    for pairs in (1, 2, 5, 8, 9, 12, 18, 37, 74, 500):
+        for asked in (1, 3, 16):
+            ranges, resident = plan(pairs, asked, 1, d, True)
+            assert ranges in (1, 2, 4, 8, 16) and ranges <= asked and (ranges == 1 or resident >= pairs)
+            assert 2 * ranges > asked or plan(1, 2 * ranges, 1, d, True)[1] < pairs
+    reqs = [(9000, 32)]                                            # nine clusters of 16 have no room on 148 SMs
+    cx, q, k, v = _step(reqs, 9, 9, d, 16, torch.bfloat16)
+    want, _, _ = _oracle(cx, reqs, q, k, v, d ** -0.5, 16)
+    got = cx.attend(1, q, k, v, d ** -0.5)
+    assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
