@@ -329,6 +329,7 @@ struct PagedAttnArgs {
   bool beside_chunks;       // with cu: there are chunks
   int wide_tiles, wide_splits;   // with cu: tiles of 128 rows over the chunks, in key ranges each (0: not to be used)
   int64_t n_slots;          // of the caches
+  int wait_limit;           // of the 128-row tiles: tries of a wait before it gives up (negative: the usual number)
   int n_tokens, ng, group, head_dim, block_size, max_blocks;
   float scale_log2;
   bool is_bf16;
@@ -346,7 +347,7 @@ int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
 bool paged_decode_by_rows(const PagedAttnArgs& a);        // which of the two decode kernels
 bool paged_wide_tiles(const PagedAttnArgs& a);            // which of the two chunk kernels
 int paged_wide_ranges(const PagedAttnArgs& a, int* resident);   // key ranges that this one takes, and how many such clusters have room at once
-int paged_status();          // 1: a kernel of this process gave up on a wait (its rows are NaN)
+int paged_status(bool clear);   // 1: a kernel of this process gave up on a wait (its rows are NaN)
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s);
 const char* paged_attention_last_error();
 

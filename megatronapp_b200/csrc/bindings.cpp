@@ -1043,7 +1043,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
                        const Tensor& tok_req, const Tensor& tok_len, int64_t block_size, double scale, int64_t splits,
                        const c10::optional<Tensor>& k_new, const c10::optional<Tensor>& v_new, const c10::optional<Tensor>& slots,
                        const c10::optional<Tensor>& cu, int64_t chunk_tiles, int64_t chunk_splits, int64_t decode_len, int64_t decode_mean,
-                       bool decode_single, int64_t wide_tiles, int64_t wide_splits) {
+                       bool decode_single, int64_t wide_tiles, int64_t wide_splits, int64_t wait_limit) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(q.dim() == 3 && q.is_contiguous() && k_cache.dim() == 3 && k_cache.is_contiguous() && v_cache.is_contiguous());
   TORCH_CHECK(q.scalar_type() == k_cache.scalar_type() && (is_bf16(q) || q.scalar_type() == at::kHalf));
@@ -1068,6 +1068,7 @@ Tensor paged_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
     a.decode_len = static_cast<int>(decode_len); a.decode_mean = static_cast<int>(decode_mean); a.decode_single = decode_single;
     a.beside_chunks = chunk_tiles > 0;
     a.wide_tiles = static_cast<int>(wide_tiles); a.wide_splits = static_cast<int>(wide_splits); a.n_slots = k_cache.size(0);
+    a.wait_limit = static_cast<int>(wait_limit);
   }
   if (T == 0) return out;
   const bool decode = !cu.has_value() || splits > 0, written = k_new.has_value();
@@ -1323,8 +1324,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("paged_attention", &paged_attention, py::arg("q"), py::arg("k_cache"), py::arg("v_cache"), py::arg("block_table"), py::arg("tok_req"),
         py::arg("tok_len"), py::arg("block_size"), py::arg("scale"), py::arg("splits"), py::arg("k_new") = py::none(), py::arg("v_new") = py::none(),
         py::arg("slots") = py::none(), py::arg("cu") = py::none(), py::arg("chunk_tiles") = 0, py::arg("chunk_splits") = 1,
-        py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false, py::arg("wide_tiles") = 0, py::arg("wide_splits") = 1);
-  m.def("paged_status", []() { return b200::paged_status(); });
+        py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false, py::arg("wide_tiles") = 0, py::arg("wide_splits") = 1,
+        py::arg("wait_limit") = -1);
+  m.def("paged_status", [](bool clear) { return b200::paged_status(clear); }, py::arg("clear") = false);
   m.def("paged_wide_ranges", [](int tiles, int ranges, int ng, int head_dim, bool bf16) {
     b200::PagedAttnArgs a{};
     a.wide_tiles = tiles; a.wide_splits = ranges; a.ng = ng; a.head_dim = head_dim; a.is_bf16 = bf16;

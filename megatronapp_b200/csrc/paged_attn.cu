@@ -787,11 +787,12 @@ struct WideSmem {
 constexpr int kWideThreads = 384, kWideTries = 1 << 20;
 __device__ int g_paged_error = 0;
 
-// bounded: a wait that runs out is noted, and every later one ends at once
-__device__ __forceinline__ void wide_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
-  for (int i = 0; i < kWideTries; ++i) {
+// bounded: a wait that runs out is noted, and every later one ends at once.  At its end the CTA then leaves g_paged_error for paged_status, fills its rows with
+// NaN and waits (always within kWideTries) for its own copies and MMAs in flight.
+__device__ __forceinline__ void wide_wait(uint64_t* bar, uint32_t parity, volatile int* failed, int limit = kWideTries) {
+  for (int left = limit; left > 0; --left) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return;
-    if ((i & 255) == 255 && __any_sync(0xffffffffu, *failed != 0)) return;
+    if ((left & 255) == 0 && __any_sync(0xffffffffu, *failed != 0)) return;
   }
   *failed = 1;
 }
@@ -916,8 +917,8 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
         const int blk = p.bs_shift >= 0 ? key >> p.bs_shift : key / a.block_size;
         slot = bt[blk] * a.block_size + (key - blk * a.block_size);
       }
-      wide_wait(&k_empty[st], ((n_loaded / kS) & 1) ^ 1, failed);
-      wide_wait(&v_empty[st], ((n_loaded / kS) & 1) ^ 1, failed);
+      wide_wait(&k_empty[st], ((n_loaded / kS) & 1) ^ 1, failed, a.wait_limit);
+      wide_wait(&v_empty[st], ((n_loaded / kS) & 1) ^ 1, failed, a.wait_limit);
       if (__any_sync(0xffffffffu, *failed != 0)) break;
       for (int kv = 0; kv < 2; ++kv) {
         uint64_t* full = kv == 0 ? &k_full[st] : &v_full[st];
@@ -937,8 +938,8 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
     named_bar_sync(3, 288);                                          // the queries are in place
     for (int j = 0; j < n_st; ++j) {
       const int st = j % kS, b = j & 1;
-      wide_wait(&k_full[st], (j / kS) & 1, failed);
-      if (j >= 2) wide_wait(&s_read[b], ((j >> 1) - 1) & 1, failed);
+      wide_wait(&k_full[st], (j / kS) & 1, failed, a.wait_limit);
+      if (j >= 2) wide_wait(&s_read[b], ((j >> 1) - 1) & 1, failed, a.wait_limit);
       if (__any_sync(0xffffffffu, *failed != 0)) break;
       tc_fence_after();
       if (elect_one()) {
@@ -957,8 +958,8 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
     const uint64_t v_desc = make_smem_desc_sw128(smem_u32(sV), 1024, kStageKeys * 128);
     for (int j = 0; j < n_st; ++j) {
       const int st = j % kS, b = j & 1;
-      wide_wait(&v_full[st], (j / kS) & 1, failed);
-      wide_wait(&p_ready[b], (j >> 1) & 1, failed);
+      wide_wait(&v_full[st], (j / kS) & 1, failed, a.wait_limit);
+      wide_wait(&p_ready[b], (j >> 1) & 1, failed, a.wait_limit);
       if (__any_sync(0xffffffffu, *failed != 0)) break;
       tc_fence_after();
       if (elect_one()) {
@@ -995,7 +996,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       const int b = j & 1, kb = k0 + j * kStageKeys;
       uint32_t v[32];
       float s[32];
-      wide_wait(&s_full[b], (j >> 1) & 1, failed);
+      wide_wait(&s_full[b], (j >> 1) & 1, failed, a.wait_limit);
       tc_fence_after();
       tmem_ld_32x32(tmem_S + b * kStageKeys + half * 32 + lanes, v);
       tmem_ld_wait();
@@ -1010,7 +1011,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
         for (int i = 0; i < 32; ++i)
           if (i >= lim) s[i] = -INFINITY;
         // V of keys that nobody sees, and values that only some rows see and that are not finite: not as zero times infinity
-        wide_wait(&v_full[j % kS], (j / kS) & 1, failed);
+        wide_wait(&v_full[j % kS], (j / kS) & 1, failed, a.wait_limit);
         const int from = max(0, min(min_vis, k1) - kb), none = k1 - kb;
         uint8_t* tile = sV + (j % kS) * L::kKV;
         bool found = false;
@@ -1051,7 +1052,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
         if (grow) m = mn;
         l *= corr;
         if (j > 0) {
-          wide_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, failed);
+          wide_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, failed, a.wait_limit);
           tc_fence_after();
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {
@@ -1073,7 +1074,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       }
       l += sum;
       if (j >= 2) {
-        wide_wait(&pv_done[b], ((j >> 1) - 1) & 1, failed);
+        wide_wait(&pv_done[b], ((j >> 1) - 1) & 1, failed, a.wait_limit);
         tc_fence_after();
       }
       const uint32_t tP = tmem_P + b * 96 + half * 16 + lanes;
@@ -1098,7 +1099,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       tc_fence_before();
       wide_arrive(&p_ready[b]);
       if (odd) {                                                     // what was taken out of V, by hand: one half's keys, then the other's
-        wide_wait(&pv_done[b], (j >> 1) & 1, failed);
+        wide_wait(&pv_done[b], (j >> 1) & 1, failed, a.wait_limit);
         tc_fence_after();
         for (int turn = 0; turn < 2; ++turn) {
           if (turn == half) {
@@ -1131,7 +1132,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
       }
     }
     if (n_st > 0) {
-      wide_wait(&pv_done[(n_st - 1) & 1], ((n_st - 1) >> 1) & 1, failed);
+      wide_wait(&pv_done[(n_st - 1) & 1], ((n_st - 1) >> 1) & 1, failed, a.wait_limit);
       tc_fence_after();
     }
     float* slot = s_ex + (n_st & 1) * (2 * L::kRows);
@@ -1449,9 +1450,12 @@ int paged_wide_ranges(const PagedAttnArgs& a, int* resident) {
   return ranges;
 }
 
-int paged_status() {
+int paged_status(bool clear) {
   int v = 0;
-  return cudaMemcpyFromSymbol(&v, g_paged_error, sizeof(int)) == cudaSuccess ? v : -1;
+  const int zero = 0;
+  if (cudaMemcpyFromSymbol(&v, g_paged_error, sizeof(int)) != cudaSuccess) return -1;
+  if (clear && v != 0 && cudaMemcpyToSymbol(g_paged_error, &zero, sizeof(int)) != cudaSuccess) return -1;
+  return v;
 }
 
 bool paged_attention_supported(int head_dim, int group) {
@@ -1481,6 +1485,7 @@ void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cud
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s) {
   PagedParams p{};
   p.a = a;
+  p.a.wait_limit = a.wait_limit < 0 ? kWideTries : a.wait_limit;
   p.row_scale = a.scale_log2;
   p.a.scale_log2 = a.scale_log2 == 0.f ? 1.f : fabsf(a.scale_log2);
   p.q_keep = a.scale_log2 == 0.f ? 0u : 0xffffffffu;

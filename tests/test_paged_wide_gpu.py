@@ -62,3 +62,31 @@ def test_all_clusters_find_room(d):
     want, _, _ = _oracle(cx, reqs, q, k, v, d ** -0.5, 16)
     got = cx.attend(1, q, k, v, d ** -0.5)
     assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reqs,hq,hkv,d,ranges", [
+    ([(300, 100), (50, 1), (0, 70)], 4, 2, 64, 1),
+    ([(5000, 150)], 4, 1, 128, 8),                                 # a cluster
+    ([(1100, 40), (1, 1), (0, 30)], 2, 1, 64, 2)])                 # ... one of whose CTAs has no keys of the second portion
+def test_a_wait_that_runs_out_shows(reqs, hq, hkv, d, ranges):
+    """Waits that give up at once: the kernel ends by itself, the portions' rows are NaN and the status says so; the next call is sound again."""
+    from megatronapp_b200 import ops
+
+    ext, scale = ops.ext(), d ** -0.5
+    cx, q, k, v = _step(reqs, hq, hkv, d, 16, torch.bfloat16)
+    want, kc, vc = _oracle(cx, reqs, q, k, v, scale, 16)
+    tiles = sum(-(-n * (hq // hkv) // 128) for _, n in reqs if n > 1)
+
+    def call(**limit):
+        return ext.paged_attention(q, kc, vc, cx._block_table, cx._tok_req, cx._tok_len, 16, scale, sum(n == 1 for _, n in reqs), None, None, None,
+                                   cx.packed.cu, 1, 1, 0, 0, False, tiles, ranges, **limit)
+
+    portion = torch.tensor([n > 1 for _, n in reqs for _ in range(n)], device="cuda")
+    assert ext.paged_status() == 0
+    got = call(wait_limit=0)
+    assert ext.paged_status() == 1 and ext.paged_status(True) == 1 and ext.paged_status() == 0
+    assert torch.isnan(got[portion]).all() and torch.isfinite(got[~portion]).all()
+    got = call()
+    assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
+    assert ext.paged_status() == 0
