@@ -336,6 +336,11 @@ class DynamicInferenceContext:
         tiles = sum(-(-p[2] * group // 128) for p in chunks) if longest >= (160 if d == 128 else 256) else 0
         return tiles, key_ranges(2 * tiles * ng, longest)
 
+    def _kernel_plan(self, group: int, ng: int, d: int) -> tuple:
+        """(Requests with at most 16 rows, the kernels' other numbers); a step without portions has no tiles to choose between."""
+        decode, *cuts = self._paged_plan(group, ng)
+        return decode, (*cuts, *(self._wide_plan(group, ng, d) if cuts[0] else (0, 1)))
+
     # -- attention over the paged cache --------------------------------------------
     def attend(self, layer: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
         """``q [T, np, hn]``, new ``k / v [T, ng, hn(v)]`` -> ``[T, np, hn_v]``; writes k / v into their pages first."""
@@ -354,8 +359,7 @@ class DynamicInferenceContext:
             if plan is None:
                 plan = ()
                 if ext.paged_attention_supported(d, np_ // ng):
-                    decode, *cuts = self._paged_plan(np_ // ng, ng)
-                    plan = (decode, (*cuts, *self._wide_plan(*heads)))
+                    plan = self._kernel_plan(*heads)
                 self._paged_plans[heads] = plan
             if plan:
                 decode, cuts = plan
