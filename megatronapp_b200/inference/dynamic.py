@@ -63,7 +63,8 @@ class _Seq:
 
 def key_ranges(tiles: int, max_len: int) -> int:
     """Into how many key ranges (CTAs of a cluster) a (64-row tile, KV head) of a prompt portion is cut: only where the tiles leave
-    most of the 296 CTA places empty and the context is long enough to pay for the merge."""
+    most of the 296 CTA places empty and the context is long enough to pay for the merge.  A 128-row tile counts as two: it has an SM to itself, one of 148
+    places (the launch takes fewer ranges where the clusters would not all run at once)."""
     n = 1
     while n < 16 and tiles * n <= 148 and max_len >= 512 * n:
         n *= 2
@@ -327,19 +328,26 @@ class DynamicInferenceContext:
                 max(keys, default=0), sum(keys) // max(1, len(few)), all(p[2] == 1 for p in few))
         return plan
 
-    def _wide_plan(self, group: int, ng: int, d: int) -> tuple:
-        """The portions' tiles of 128 rows and key ranges of those, for the kernel that has one such tile on an SM; no tiles where the contexts
-        are so short that its start (12.4 us a step against 8.3 to 10.4) costs more than its stages give.  us, 64-row / 128-row tiles, 32 / 8 heads of 128:
-        one portion of 100 13.6 / 14.4, of 150 16.5 / 14.5; 12 heads of 64: one of 220 14.4 / 16.5, four with up to 300 keys 20.0 / 18.5."""
+    def _wide_plan(self, group: int, ng: int, d: int, ranges64: int) -> tuple:
+        """The portions' tiles of 128 rows and key ranges of those, for the kernel that has one such tile on an SM; no tiles where the 64-row ones, in
+        ``ranges64`` key ranges, are the better ones.  Its start costs 3 to 4 us more; a stage of 64 keys takes 1.4 us for 3.4 at heads of 128, 1.2 for 2.1 at
+        64, but nothing runs beside the start of a later wave.  128-row / 64-row times of 1420 drawn steps, geometric means: heads of 128 from three stages
+        0.92, from six 0.80, from twelve 0.56; heads of 64 below six stages a CTA 1.05, from six 0.95, from nine 0.67, more than two waves below twelve
+        stages 1.06, from there 0.77, fewer key ranges than the 64-row tiles take 1.1 to 1.4."""
         chunks = [p for p in self._plan if p[2] * group > 16]
-        longest = max((p[2] + p[3] for p in chunks), default=0)
-        tiles = sum(-(-p[2] * group // 128) for p in chunks) if longest >= (160 if d == 128 else 256) else 0
-        return tiles, key_ranges(2 * tiles * ng, longest)
+        longest = max(p[2] + p[3] for p in chunks)
+        tiles = sum(-(-p[2] * group // 128) for p in chunks)
+        ranges = key_ranges(2 * tiles * ng, longest)
+        if d == 128:
+            better = longest >= 160
+        else:
+            better = longest > 64 * ranges64 * (11 if tiles * ng > 2 * 148 else 5) and ranges >= ranges64
+        return (tiles, ranges) if better else (0, 1)
 
     def _kernel_plan(self, group: int, ng: int, d: int) -> tuple:
         """(Requests with at most 16 rows, the kernels' other numbers); a step without portions has no tiles to choose between."""
         decode, *cuts = self._paged_plan(group, ng)
-        return decode, (*cuts, *(self._wide_plan(group, ng, d) if cuts[0] else (0, 1)))
+        return decode, (*cuts, *(self._wide_plan(group, ng, d, cuts[1]) if cuts[0] else (0, 1)))
 
     # -- attention over the paged cache --------------------------------------------
     def attend(self, layer: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float) -> torch.Tensor:
