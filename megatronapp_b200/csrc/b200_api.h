@@ -345,7 +345,8 @@ bool paged_attention_supported(int head_dim, int group);
 void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cudaStream_t s);
 int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
 bool paged_decode_by_rows(const PagedAttnArgs& a);        // which of the two decode kernels
-bool paged_wide_tiles(const PagedAttnArgs& a);            // which of the two chunk kernels
+bool paged_wide_tiles(const PagedAttnArgs& a);            // whether the 128-row tiles take the chunks' pages
+int paged_chunk_rows(const PagedAttnArgs& a);             // rows of a tile of the chunk kernel that a call takes: 64 or 128
 int paged_wide_ranges(const PagedAttnArgs& a, int* resident);   // key ranges that this one takes, and how many such clusters have room at once
 int paged_status(bool clear);   // 1: a kernel of this process gave up on a wait (its rows are NaN)
 int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int chunk_splits, float* ws, bool written, cudaStream_t s);

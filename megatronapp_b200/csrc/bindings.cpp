@@ -1327,6 +1327,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("decode_len") = 0, py::arg("decode_mean") = 0, py::arg("decode_single") = false, py::arg("wide_tiles") = 0, py::arg("wide_splits") = 1,
         py::arg("wait_limit") = -1);
   m.def("paged_status", [](bool clear) { return b200::paged_status(clear); }, py::arg("clear") = false);
+  m.def("paged_chunk_rows", [](const Tensor& k_cache, const Tensor& v_cache, int block_size, int wide_tiles) {
+    b200::PagedAttnArgs a{};
+    a.k_cache = k_cache.data_ptr(); a.v_cache = v_cache.data_ptr(); a.n_slots = k_cache.size(0);
+    a.ng = static_cast<int>(k_cache.size(1)); a.head_dim = static_cast<int>(k_cache.size(2)); a.is_bf16 = is_bf16(k_cache);
+    a.block_size = block_size; a.wide_tiles = wide_tiles;
+    return b200::paged_chunk_rows(a);
+  });
   m.def("paged_wide_ranges", [](int tiles, int ranges, int ng, int head_dim, bool bf16) {
     b200::PagedAttnArgs a{};
     a.wide_tiles = tiles; a.wide_splits = ranges; a.ng = ng; a.head_dim = head_dim; a.is_bf16 = bf16;

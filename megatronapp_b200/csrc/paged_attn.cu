@@ -1442,6 +1442,15 @@ bool paged_wide_tiles(const PagedAttnArgs& a) {
          (kStageKeys % a.block_size == 0 || a.block_size % kStageKeys == 0);
 }
 
+namespace {
+bool wide_maps(const PagedAttnArgs& a, CUtensorMap* mk, CUtensorMap* mv) { return paged_wide_tiles(a) && page_map(mk, a.k_cache, a) && page_map(mv, a.v_cache, a); }
+}  // namespace
+
+int paged_chunk_rows(const PagedAttnArgs& a) {
+  CUtensorMap mk, mv;
+  return wide_maps(a, &mk, &mv) ? 128 : 64;
+}
+
 int paged_wide_ranges(const PagedAttnArgs& a, int* resident) {
   const int ranges = wide_ranges(a);
   int log = 0;
@@ -1500,7 +1509,7 @@ int paged_attention(const PagedAttnArgs& a, bool decode, int chunk_tiles, int ch
     if (e != cudaSuccess) { g_paged_err = std::string("paged attention: ") + cudaGetErrorString(e); return -13; }
   }
   CUtensorMap mk, mv;
-  if (a.cu != nullptr && chunk_tiles > 0 && paged_wide_tiles(a) && page_map(&mk, a.k_cache, a) && page_map(&mv, a.v_cache, a)) {
+  if (a.cu != nullptr && chunk_tiles > 0 && wide_maps(a, &mk, &mv)) {
     p.n_tiles = a.wide_tiles;
     p.splits = wide_ranges(a);
     const int rc = a.head_dim == 128 ? (a.is_bf16 ? launch_wide<128, true>(p, mk, mv, s) : launch_wide<128, false>(p, mk, mv, s))

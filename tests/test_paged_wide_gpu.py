@@ -5,6 +5,19 @@ import torch
 from test_paged_attention_gpu import _oracle, _step
 
 
+def _by_wide_tiles(cx, hq, hkv, d, block):
+    """The step's portions go by tiles of 128 rows, whatever the rule says of them; whether they do is looked at."""
+    from megatronapp_b200 import ops
+    from megatronapp_b200.inference.dynamic import key_ranges
+
+    group = hq // hkv
+    portions = [p for p in cx._plan if p[2] * group > 16]
+    tiles, longest = sum(-(-p[2] * group // 128) for p in portions), max(p[2] + p[3] for p in portions)
+    decode, cuts = cx._kernel_plan(group, hkv, d)
+    cx._paged_plans[group, hkv, d] = decode, (*cuts[:-2], tiles, key_ranges(2 * tiles * hkv, longest))
+    assert ops.ext().paged_chunk_rows(*cx.kv[1], block, tiles) == 128
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("reqs,hq,hkv,d,block,dtype", [
     ([(0, 127), (64, 128), (165, 129)], 2, 2, 64, 8, torch.bfloat16),            # a row less and more than a tile, the smallest pages
@@ -23,6 +36,7 @@ def test_wide_tiles(reqs, hq, hkv, d, block, dtype):
         seen[(torch.tensor(cx.seqs[str(i)].blocks).unsqueeze(1) * block + torch.arange(block)).view(-1)[:a + n].cuda()] = True
     kc[~seen], vc[~seen] = float("nan"), float("inf")              # pages of nobody, and what lies behind the last token
     want, _, _ = _oracle(cx, reqs, q, k, v, d ** -0.5, block)
+    _by_wide_tiles(cx, hq, hkv, d, block)
     got = cx.attend(1, q, k, v, d ** -0.5)
     unit = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11    # the result's own rounding, as in the tests of the other tiles
     assert float((got.double() - want).abs().max()) <= unit * max(1.0, float(want.abs().max()))
@@ -38,6 +52,7 @@ def test_values_of_later_tokens_stay_out_of_wide_tiles(dtype):
     cx, q, k, v = _step(reqs, 8, 2, 128, 16, dtype)
     v[4, 0, 5], v[67, 0, 127], v[68, 1, 64], v[140, 1, 63] = float("inf"), float("-inf"), float("nan"), float("inf")
     want, _, _ = _oracle(cx, reqs, q, k, v, 0.1, 16)
+    _by_wide_tiles(cx, 8, 2, 128, 16)
     got = cx.attend(1, q, k, v, 0.1).double()
     assert torch.equal(torch.isfinite(got), torch.isfinite(want))
     ok = torch.isfinite(want)
@@ -60,6 +75,7 @@ def test_all_clusters_find_room(d):
     reqs = [(9000, 32)]                                            # nine clusters of 16 have no room on 148 SMs
     cx, q, k, v = _step(reqs, 9, 9, d, 16, torch.bfloat16)
     want, _, _ = _oracle(cx, reqs, q, k, v, d ** -0.5, 16)
+    _by_wide_tiles(cx, 9, 9, d, 16)
     got = cx.attend(1, q, k, v, d ** -0.5)
     assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
 
@@ -90,3 +106,33 @@ def test_a_wait_that_runs_out_shows(reqs, hq, hkv, d, ranges):
     got = call()
     assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * max(1.0, float(want.abs().max()))
     assert ext.paged_status() == 0
+
+
+@pytest.mark.gpu
+def test_which_pages_go_by_which_tiles():
+    """Whole pages to a stage of 64 keys, or whole stages to a page, of a multiple of eight slots: 128 rows where the plan has such tiles, 64 rows elsewhere."""
+    from megatronapp_b200 import ops
+
+    for d in (64, 128):
+        cache = torch.empty(768, 2, d, dtype=torch.bfloat16, device="cuda")
+        assert [ops.ext().paged_chunk_rows(cache, cache, b, 1) for b in (8, 16, 32, 64, 128, 192, 4, 12, 24, 48, 96)] == [128] * 6 + [64] * 5
+        assert ops.ext().paged_chunk_rows(cache, cache, 16, 0) == 64
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [0.1, -0.5, 0.0])
+@pytest.mark.parametrize("reqs,hq,hkv,d,ranges,dtype", [
+    ([(9000, 30)], 8, 2, 128, 16, torch.bfloat16),
+    ([(5000, 30), (3, 1)], 4, 4, 64, 16, torch.float16),
+    ([(1100, 40), (0, 20)], 4, 1, 64, 4, torch.float16)])           # a tile whose later ranges are empty
+def test_key_ranges_of_64_row_tiles(reqs, hq, hkv, d, ranges, dtype, scale):
+    """Pages that only the 64-row tiles take: their clusters' merge."""
+    from megatronapp_b200 import ops
+
+    cx, q, k, v = _step(reqs, hq, hkv, d, 24, dtype)
+    want, _, _ = _oracle(cx, reqs, q, k, v, scale, 24)
+    assert cx._kernel_plan(hq // hkv, hkv, d)[1][1] == ranges and ops.ext().paged_chunk_rows(*cx.kv[1], 24, 1) == 64
+    got = cx.attend(1, q, k, v, scale)
+    unit = 2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11
+    # scores of up to 50: their own fp32 rounding moves a weight by 2^-18
+    assert float((got.double() - want).abs().max()) <= unit * max(1.0, float(want.abs().max()))
