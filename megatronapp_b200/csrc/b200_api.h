@@ -345,6 +345,7 @@ bool paged_attention_supported(int head_dim, int group);
 void paged_write(const PagedWriteArgs& w, const PagedAttnArgs& a, float* ws, cudaStream_t s);
 int64_t paged_decode_workspace(const PagedAttnArgs& a);   // floats
 bool paged_decode_by_rows(const PagedAttnArgs& a);        // which of the two decode kernels
+int paged_decode_cut(const PagedAttnArgs& a);             // CTAs that the decode stages are cut for, 0 where items stay whole
 bool paged_wide_tiles(const PagedAttnArgs& a);            // whether the 128-row tiles take the chunks' pages
 int paged_chunk_rows(const PagedAttnArgs& a);             // rows of a tile of the chunk kernel that a call takes: 64 or 128
 int paged_wide_ranges(const PagedAttnArgs& a, int* resident);   // key ranges that this one takes, and how many such clusters have room at once

@@ -1348,6 +1348,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     a.decode_mean = mean; a.decode_single = single;
     return b200::paged_decode_by_rows(a);
   });
+  m.def("paged_decode_cut", [](int64_t requests, int ng, int group, int head_dim, int longest, int mean, bool beside_chunks) {
+    b200::PagedAttnArgs a{};
+    const int32_t none = 0;
+    a.cu = &none; a.n_seqs = static_cast<int>(requests); a.ng = ng; a.group = group; a.head_dim = head_dim; a.block_size = 1; a.max_blocks = longest;
+    a.decode_mean = mean; a.beside_chunks = beside_chunks;
+    return b200::paged_decode_cut(a);
+  });
   m.def("paged_attention_supported", &paged_attention_supported);
   m.def("spin", &spin);
   m.def("write_flag", &write_flag);

@@ -1397,17 +1397,22 @@ int64_t decode_keys(const PagedAttnArgs& a) {
   return a.decode_len > 0 && a.decode_len < all ? a.decode_len : all;
 }
 
-// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Short contexts are not cut at all
-// (0): putting parts together then costs as much as the imbalance that it removes.  us, whole / cut, heads of 128: 90 requests of up to 300 keys x 8
-// heads 35.8 / 42.0, 40 of up to 429 x 4 beside chunks 29.1 / 40.9, 2 of up to 430 x 8 beside one 26.5 /
-// 30.7, 9 of up to 373 x 4 14.4 / 16.5, but 1 of 500 x 8 21.5 / 17.4, 8 of up to 700 27.6 / 21.5; a stage of heads of 64 takes
-// half as long: 10 of up to 824 x 12 beside chunks 21.9 / 29.3, 1 of 522 x 8 10.3 / 12.4
+// the line of decode stages is cut for three CTAs per SM, but for no more than there can be pairs of stages.  Where that gains little the items stay whole (0):
+// putting parts together costs as much as the imbalance that it removes.  A stage of heads of 64 takes half as long: us, whole / cut, 10 requests of up to 824 keys x 12
+// beside chunks 21.9 / 29.3, 1 of 522 x 8 10.3 / 12.4.  Heads of 128, geometric means of cut / whole over 513 drawn steps: alone, up to 24 (request, head) pairs of 5
+// stages 1.20, of 8 0.87, of 10 0.74; 100 to 300 of 9 1.00, of 12 0.92, of 14 0.85; above 444 of 9 to 13 1.06, of 16 0.93: what counts is by how much the longest
+// exceeds a CTA's share.  Beside chunks, behind whose CTAs the many short parts start: up to 96 of 9 0.92, of 12 0.79; 100 to 300 of 9 1.13, of 13 1.06, of 15 0.88
 int decode_ctas(const PagedAttnArgs& a) {
   const int64_t items = decode_items(a), longest = (decode_keys(a) + kStageKeys - 1) / kStageKeys;
-  const bool whole = a.head_dim == 64 ? longest <= (items <= kDecodeCtas ? 16 : 8) : longest <= (items <= 16 && !a.beside_chunks ? 4 : 8);
-  if (whole) return 0;
-  const int64_t n = items * longest / 2;
-  return static_cast<int>(n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n));
+  const int64_t n = items * longest / 2, ctas = n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n);
+  bool whole;
+  if (a.head_dim == 64) whole = longest <= (items <= kDecodeCtas ? 16 : 8);
+  else if (a.beside_chunks) whole = longest <= (items <= 96 ? 8 : 13);
+  else {
+    const double mean = a.decode_mean > 0 ? a.decode_mean / static_cast<double>(kStageKeys) : static_cast<double>(longest), share = items * mean / ctas;
+    whole = (longest <= 8 && items > 16) || longest - (share > 1. ? share : 1.) < 6.;
+  }
+  return whole ? 0 : static_cast<int>(ctas);
 }
 
 // a workspace holds the CTAs' partials and, behind them, a counter for each (request, KV head)
@@ -1470,6 +1475,8 @@ int paged_status(bool clear) {
 bool paged_attention_supported(int head_dim, int group) {
   return (head_dim == 64 || head_dim == 128) && (group == 1 || group == 2 || group == 4 || group == 8);
 }
+
+int paged_decode_cut(const PagedAttnArgs& a) { return paged_decode_by_rows(a) ? 0 : decode_ctas(a); }
 
 int64_t paged_decode_workspace(const PagedAttnArgs& a) {
   if (paged_decode_by_rows(a)) return 0;
