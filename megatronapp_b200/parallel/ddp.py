@@ -144,7 +144,12 @@ class ParamAndGradBuffer:
         self._zero_plan = None
         if self._zero_ranges and self.grad_data.is_cuda:
             table, blocks = ops.ext().zero_ranges_plan(self.grad_data.element_size(), self._zero_ranges)
-            self._zero_plan = (table.to(self.grad_data.device), blocks)
+            self._zero_plan = (self._buffer(), table.to(self.grad_data.device), blocks)
+
+    def _buffer(self) -> tuple:
+        """What a table of byte ranges into ``grad_data`` holds for."""
+        g = self.grad_data
+        return g.device, g.dtype, g.numel(), g.is_contiguous() and g.data_ptr() % 16 == 0
 
     # ---- gradient sync ---------------------------------------------------------
     def reset(self):
@@ -156,8 +161,8 @@ class ParamAndGradBuffer:
     def zero(self):
         if self._zero_ranges is None:
             self.grad_data.zero_()
-        elif self._zero_plan is not None and self.grad_data.device == self._zero_plan[0].device:
-            ops.ext().zero_ranges(self.grad_data, *self._zero_plan)
+        elif self._zero_plan is not None and self._zero_plan[0] == self._buffer():
+            ops.ext().zero_ranges(self.grad_data, *self._zero_plan[1:])
         else:
             for a, b in self._zero_ranges:
                 self.grad_data[a:b].zero_()

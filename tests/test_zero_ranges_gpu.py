@@ -20,3 +20,22 @@ def test_only_the_ranges(ranges, dtype):
     assert torch.equal(data, want)
     with pytest.raises(RuntimeError):
         ops.ext().zero_ranges_plan(data.element_size(), [(5, 5)])
+
+
+@pytest.mark.parametrize("change", [lambda g: g, lambda g: g.bfloat16(), lambda g: torch.cat([g, g])[1:g.numel() + 1], lambda g: g[:1000].clone(),
+                                    lambda g: torch.stack([g, g], 1)[:, 0]])
+def test_a_buffer_that_was_put_in_place_of_the_first(change):
+    """A gradient buffer of another type, size, alignment or stride: its ranges become zeros, and nothing else does."""
+    from megatronapp_b200.parallel.ddp import DistributedDataParallelConfig, ParamAndGradBuffer
+
+    params = [torch.nn.Parameter(torch.zeros(n, device="cuda")) for n in (640, 1000, 64)]
+    params[1].b200_wgrad_store_first = True
+    buf = ParamAndGradBuffer(DistributedDataParallelConfig(), torch.float32, torch.float32, params, None, 1, None, 1.0, "cuda")
+    s, e, _ = buf.param_index[params[1]]
+    buf.grad_data = change(torch.full_like(buf.grad_data, 3.0))
+    want = buf.grad_data.clone()
+    want[:s], want[e:] = 0, 0
+    around = buf.grad_data._base if buf.grad_data._base is not None else buf.grad_data
+    rest = int((around == 3).sum()) - int((buf.grad_data == 3).sum())
+    buf.zero()
+    assert torch.equal(buf.grad_data, want) and int((around == 3).sum()) - int((buf.grad_data == 3).sum()) == rest
