@@ -1401,13 +1401,13 @@ int64_t decode_keys(const PagedAttnArgs& a) {
 // putting parts together costs as much as the imbalance that it removes.  A stage of heads of 64 takes half as long: us, whole / cut, 10 requests of up to 824 keys x 12
 // beside chunks 21.9 / 29.3, 1 of 522 x 8 10.3 / 12.4.  Heads of 128, geometric means of cut / whole over 513 drawn steps: alone, up to 24 (request, head) pairs of 5
 // stages 1.20, of 8 0.87, of 10 0.74; 100 to 300 of 9 1.00, of 12 0.92, of 14 0.85; above 444 of 9 to 13 1.06, of 16 0.93: what counts is by how much the longest
-// exceeds a CTA's share.  Beside chunks, behind whose CTAs the many short parts start: up to 96 of 9 0.92, of 12 0.79; 100 to 300 of 9 1.13, of 13 1.06, of 15 0.88
+// exceeds a CTA's share.  Beside chunks, behind whose CTAs the many short parts start: up to 96 of 9 0.92, of 12 0.79; 100 to 300 of 9 1.13, of 13 1.06, of 14 0.97 (up to 1.24), of 15 0.88
 int decode_ctas(const PagedAttnArgs& a) {
   const int64_t items = decode_items(a), longest = (decode_keys(a) + kStageKeys - 1) / kStageKeys;
   const int64_t n = items * longest / 2, ctas = n < 1 ? 1 : (n > kDecodeCtas ? kDecodeCtas : n);
   bool whole;
   if (a.head_dim == 64) whole = longest <= (items <= kDecodeCtas ? 16 : 8);
-  else if (a.beside_chunks) whole = longest <= (items <= 96 ? 8 : 13);
+  else if (a.beside_chunks) whole = longest <= (items <= 96 ? 8 : 14);
   else {
     const double mean = a.decode_mean > 0 ? a.decode_mean / static_cast<double>(kStageKeys) : static_cast<double>(longest), share = items * mean / ctas;
     whole = (longest <= 8 && items > 16) || longest - (share > 1. ? share : 1.) < 6.;

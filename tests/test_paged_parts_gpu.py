@@ -33,7 +33,7 @@ def test_parts(reqs, hq, hkv, d):
     (1, 8, 1, 128, 448, 448, False, 0), (1, 8, 1, 128, 449, 449, False, 32),                     # few (request, head) pairs: eight stages
     (8, 4, 4, 128, 512, 300, False, 0), (8, 4, 4, 128, 513, 300, False, 144),                    # more than 16: nine
     (47, 8, 4, 128, 529, 299, False, 0), (47, 8, 4, 128, 640, 299, False, 444),                  # six stages more than a CTA's share
-    (24, 4, 4, 128, 513, 300, True, 432), (25, 4, 4, 128, 832, 400, True, 0), (25, 4, 4, 128, 833, 400, True, 444),       # beside chunks
+    (24, 4, 4, 128, 513, 300, True, 432), (25, 4, 4, 128, 896, 400, True, 0), (25, 4, 4, 128, 897, 400, True, 444),       # beside chunks
     (30, 12, 1, 64, 1024, 600, True, 0), (30, 12, 1, 64, 1025, 600, False, 444), (64, 8, 4, 64, 512, 300, False, 0), (64, 8, 4, 64, 513, 300, False, 444)])
 def test_which_contexts_are_cut(requests, ng, group, d, longest, mean, beside, ctas):
     """Either side of the lengths and counts at which cut contexts were measured faster than whole ones."""
