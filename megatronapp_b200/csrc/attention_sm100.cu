@@ -2,7 +2,7 @@
 // two 128-row query tiles per CTA processed ping-pong by two pairs of softmax warpgroups.
 //
 // Forward  (attn_fwd_kernel):  S = Q K^T -> online softmax (exp2 domain, lazy rescale) ->
-//                              P (16-bit, over S in TMEM) -> O += P V (O stays in TMEM).
+//                              P (16-bit, TMEM columns of its own) -> O += P V (O stays in TMEM).
 // Backward (two kernels, deterministic, no atomics):
 //   attn_bwd_kernel<dK, dV> : CTA per 128-key block, loops over 64-query blocks
 //                             S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q

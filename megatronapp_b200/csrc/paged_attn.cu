@@ -5,21 +5,21 @@
 // tok_len[t] keys of that request; keys live in fixed-size pages of a shared pool, found through the request's block
 // table.
 //
-// A tile is up to 16 or 64 rows, a row being one (token, query head) of one request and one KV head: all query heads of a group share
+// A tile is up to 16, 64 or 128 rows, a row being one (token, query head) of one request and one KV head: all query heads of a group share
 // every key/value row that is read, and so do the tokens of a chunk.  Keys come in stages of 64, gathered page by page into a ring of
-// shared-memory buffers by 16-byte asynchronous copies (32 KB each at d = 128), and are
-// multiplied by m16n8k16 tensor instructions from there.  The weights are fp32: each enters the value product as three 16-bit parts that add
-// up to it (fp16: to 2^-40 of the largest weight where it is below 2^-16 of that).
+// shared-memory buffers, for 16 and 64 rows by 16-byte asynchronous copies (32 KB each at d = 128) and
+// multiplied by m16n8k16 tensor instructions from there, for 128 by TMA and multiplied on tcgen05.  The weights are fp32: each enters the value product as three 16-bit
+// parts that add up to it (fp16: to 2^-40 of the largest weight where it is below 2^-16 of that).
 //   rows = 16 (decode, short chunks): the four warps take 16 keys of a stage each, bound by HBM.  The stages of all (request, KV head)
 //     pairs stand in one line that is cut evenly over three CTAs per SM, whatever the contexts' lengths; an item that a cut falls into
 //     leaves partial (max, sum, accumulator) triples, and the CTA that counts the last of them puts them together.  What a CTA needs to know before its
 //     first key (a request per thread) is read while the new keys are still being written.  64 contexts of 1k to 4k, 32 / 8 heads of 128:
 //     128 us with the write, 134 with a kernel of its own for the parts; one of 12000: 24 and 29, of 500: 17 and 22 (138 for the former's
 //     decode alone with three stages and two CTAs per SM; 456 with a key per 16 lanes and no load in flight behind it).  Many short contexts with few heads a group go by rows instead, see paged_rows_kernel.
-//   rows = 64 (chunks): a warp takes 16 rows and all keys of a stage, longest tiles first, bound by the tensor instructions.  Where the
-//     tiles are few and the context is long, the CTAs of a cluster take key ranges and merge through distributed shared memory.  Two
-//     chunks of 500 tokens beside 24 decoding requests: 865 us before, every token reading all its keys, 67 + 40 us now (57 + 39 when the
-//     weights' third parts were left out).
+//   rows = 64 (chunks of short contexts, or in pages that a TMA box does not fit): a warp takes 16 rows and all keys of a stage, longest tiles first, bound by the
+//     tensor instructions.  Where the tiles are few and the context is long, the CTAs of a cluster take key ranges and merge through distributed shared memory.  Two
+//     chunks of 500 tokens beside 24 decoding requests, a step: 865 us when every token read all its keys, 110 by these tiles.
+//   rows = 128 (chunks otherwise, the plan says which): see paged_wide_kernel, 87 us for the same step.
 //
 // Replaces the reference's dynamic-context attention (core/inference/contexts/dynamic_context.py + flash_attn_with_kvcache
 // in attention.py:590-603) and this repo's earlier gather + einsum path (inference/dynamic.py).
@@ -79,9 +79,8 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
 // Launches of a step overlap: every kernel lets the next one start once all its own CTAs run, and waits for the one before where it reads
 // what that wrote: the write kernel's rows and zeroed counters (the first of the others).  The decode kernel beside chunks reads
 // nothing of theirs, and what both read was complete before the first began: it waits before its end, which keeps the stream's order
-// for what follows.
-__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// for what follows (pdl_allow_next, pdl_await_previous).
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -447,8 +446,8 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
   const PagedAttnArgs& a = p.a;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
-  allow_next();
-  if (!p.beside_chunks && !p.behind_write) await_previous();
+  pdl_allow_next();
+  if (!p.beside_chunks && !p.behind_write) pdl_await_previous();
   int at, end, parts_of_line = 0, line = 0, r = 0, inside = 0;
   Item it;
   if constexpr (!kCut) {
@@ -499,7 +498,7 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     }
   }
   if (at >= end) {
-    if (p.beside_chunks || p.behind_write) await_previous();
+    if (p.beside_chunks || p.behind_write) pdl_await_previous();
     return;
   }
   if constexpr (kCut) {
@@ -513,7 +512,7 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
   float* s_l = s_m + 64;
   Tile<D, kBf16, 1> tile;
   const Cuts cuts(kCut ? line : 0, kCut ? parts_of_line : 1);
-  if (p.behind_write) await_previous();                              // the new keys are in their pages, the counters zero
+  if (p.behind_write) pdl_await_previous();                          // the new keys are in their pages, the counters zero
   while (true) {
     const int hk = inside / it.stages, st0 = inside % it.stages;
     const int n_st = min(it.stages - st0, end - at);
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(128, 3) paged_decode_kernel(const PagedParams 
     }
     __syncthreads();                                                 // the partials have been read; the ring fills again
   }
-  if (p.beside_chunks) await_previous();
+  if (p.beside_chunks) pdl_await_previous();
 }
 
 // ---- decode with few rows per key and many short contexts: a tile of the kernels above is mostly empty and its start and end cost more than
@@ -591,8 +590,8 @@ __global__ void __launch_bounds__(128, G == 1 ? 12 : G == 2 ? 7 : 4) paged_rows_
   __shared__ float s_m[kGroups][G], s_l[kGroups][G];
   __shared__ float s_acc[kGroups][G][D];
   const PagedAttnArgs& a = p.a;
-  allow_next();
-  if (!p.beside_chunks) await_previous();
+  pdl_allow_next();
+  if (!p.beside_chunks) pdl_await_previous();
   const int r = blockIdx.x / a.ng, hk = blockIdx.x % a.ng, np = a.ng * G;
   const Item it = decode_item(p, r);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lk = lane % kLanes, grp = warp * kWarpKeys + lane / kLanes;
@@ -666,10 +665,53 @@ __global__ void __launch_bounds__(128, G == 1 ? 12 : G == 2 ? 7 : 4) paged_rows_
     }
     __syncthreads();                                                 // the groups' shares have been read
   }
-  if (p.beside_chunks) await_previous();
+  if (p.beside_chunks) pdl_await_previous();
 }
 
 // ---- chunks
+// one warp: that run of `per_tile` tokens among the requests with more than 16 rows: its first token, and how many it has
+__device__ __forceinline__ void find_tile(const PagedParams& p, int per_tile, int tile_at, int* s_tile) {
+  const PagedAttnArgs& a = p.a;
+  const int lane = threadIdx.x & 31;
+  int before = 0;
+  for (int r0 = 0; r0 < a.n_seqs; r0 += 32) {
+    const int r = r0 + lane;
+    const int c0 = r < a.n_seqs ? a.cu[r] : 0, c1 = r < a.n_seqs ? a.cu[r + 1] : 0, len = c1 - c0;
+    const int tiles = (len << p.group_shift) > 16 ? (len + per_tile - 1) / per_tile : 0;
+    int incl = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const int first = before + incl - tiles;
+    if (tiles > 0 && tile_at >= first && tile_at < first + tiles) {
+      const int off = (tile_at - first) * per_tile;
+      s_tile[0] = c0 + off;
+      s_tile[1] = min(per_tile, len - off);
+    }
+    before += __shfl_sync(0xffffffffu, incl, 31);
+    if (before > tile_at) break;
+  }
+  if (lane == 0 && before <= tile_at) s_tile[1] = 0;                 // more tiles launched than there are
+}
+// the partials of a cluster's CTAs, behind its barrier: thread `first` of all of them
+template <int D, bool kBf16, typename Out>
+__device__ __forceinline__ void merge_cluster(const PagedParams& p, int first, int threads, int n_rows, const float* part, const float* s_m, const float* s_l, Out out_row) {
+  cg::cluster_group cluster = cg::this_cluster();
+  for (int idx = first; idx < n_rows * (D / 4); idx += p.splits * threads) {
+    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
+    Merge x(p.a.scale_log2);
+    for (int c = 0; c < p.splits; ++c) x.M = fmaxf(x.M, *cluster.map_shared_rank(s_m + row, c));
+    if (x.M > -INFINITY) {
+      for (int c = 0; c < p.splits; ++c)
+        x.add(*cluster.map_shared_rank(s_m + row, c), *cluster.map_shared_rank(s_l + row, c),
+              *cluster.map_shared_rank(reinterpret_cast<const float4*>(part + row * D + col), c));
+    }
+    *reinterpret_cast<uint2*>(out_row(row) + col) = x.result<kBf16>();
+  }
+}
+
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p) {
   using L = Smem<D>;
@@ -681,33 +723,9 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
   const int rank = static_cast<int>(blockIdx.x) % p.splits, item = static_cast<int>(blockIdx.x) / p.splits;
   const int hk = item % a.ng, tile_at = p.n_tiles - 1 - item / a.ng; // later tiles of a chunk see more keys: they go first
   const int G = 1 << p.group_shift, np = a.ng << p.group_shift;
-  await_previous();
-  allow_next();
-  // that run of 64 / G tokens among the requests with more than 16 rows
-  const int per_tile = kRows >> p.group_shift;
-  if (warp == 0) {
-    int before = 0;
-    for (int r0 = 0; r0 < a.n_seqs; r0 += 32) {
-      const int r = r0 + lane;
-      const int c0 = r < a.n_seqs ? a.cu[r] : 0, c1 = r < a.n_seqs ? a.cu[r + 1] : 0, len = c1 - c0;
-      const int tiles = (len << p.group_shift) > 16 ? (len + per_tile - 1) / per_tile : 0;
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int first = before + incl - tiles;
-      if (tiles > 0 && tile_at >= first && tile_at < first + tiles) {
-        const int off = (tile_at - first) * per_tile;
-        s_tile[0] = c0 + off;
-        s_tile[1] = min(per_tile, len - off);
-      }
-      before += __shfl_sync(0xffffffffu, incl, 31);
-      if (before > tile_at) break;
-    }
-    if (lane == 0 && before <= tile_at) s_tile[1] = 0;               // more tiles launched than there are
-  }
+  pdl_await_previous();
+  pdl_allow_next();
+  if (warp == 0) find_tile(p, kRows >> p.group_shift, tile_at, s_tile);
   __syncthreads();
   const int t0 = s_tile[0], n = s_tile[1];
   if (n == 0) return;
@@ -751,17 +769,7 @@ __global__ void __launch_bounds__(128, 2) paged_chunk_kernel(const PagedParams p
   tile.spill(part, s_m, s_l);
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
-  for (int idx = rank * 128 + tid; idx < n_rows * (D / 4); idx += p.splits * 128) {
-    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
-    Merge x(a.scale_log2);
-    for (int c = 0; c < p.splits; ++c) x.M = fmaxf(x.M, *cluster.map_shared_rank(s_m + row, c));
-    if (x.M > -INFINITY) {
-      for (int c = 0; c < p.splits; ++c)
-        x.add(*cluster.map_shared_rank(s_m + row, c), *cluster.map_shared_rank(s_l + row, c),
-              *cluster.map_shared_rank(reinterpret_cast<const float4*>(part + row * D + col), c));
-    }
-    *reinterpret_cast<uint2*>(out_row(row) + col) = x.result<kBf16>();
-  }
+  merge_cluster<D, kBf16>(p, rank * 128 + tid, 128, n_rows, part, s_m, s_l, out_row);
   cluster.sync();                                                    // no CTA leaves while another reads its partials
 }
 
@@ -850,31 +858,9 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
     tma_prefetch_desc(&map_v);
   }
   if (warp == 2) tmem_alloc<512>(tmem_slot);
-  await_previous();
-  allow_next();
-  if (warp == 0) {                                                   // as in paged_chunk_kernel, in tiles of 128 rows
-    int before = 0;
-    for (int r0 = 0; r0 < a.n_seqs; r0 += 32) {
-      const int r = r0 + lane;
-      const int c0 = r < a.n_seqs ? a.cu[r] : 0, c1 = r < a.n_seqs ? a.cu[r + 1] : 0, len = c1 - c0;
-      const int tiles = (len << p.group_shift) > 16 ? (len + per_tile - 1) / per_tile : 0;
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int first = before + incl - tiles;
-      if (tiles > 0 && tile_at >= first && tile_at < first + tiles) {
-        const int off = (tile_at - first) * per_tile;
-        s_tile[0] = c0 + off;
-        s_tile[1] = min(per_tile, len - off);
-      }
-      before += __shfl_sync(0xffffffffu, incl, 31);
-      if (before > tile_at) break;
-    }
-    if (lane == 0 && before <= tile_at) s_tile[1] = 0;               // more tiles launched than there are
-  }
+  pdl_await_previous();
+  pdl_allow_next();
+  if (warp == 0) find_tile(p, per_tile, tile_at, s_tile);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1217,17 +1203,7 @@ paged_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_consta
   const float* part = reinterpret_cast<const float*>(smem + L::kKOff);
   const float* s_m = reinterpret_cast<const float*>(smem + L::kStatOff);
   const float* s_l = s_m + L::kRows;
-  for (int idx = rank * kWideThreads + threadIdx.x; idx < n_rows * (D / 4); idx += p.splits * kWideThreads) {
-    const int row = idx / (D / 4), col = (idx % (D / 4)) * 4;
-    Merge x(a.scale_log2);
-    for (int c = 0; c < p.splits; ++c) x.M = fmaxf(x.M, *cluster.map_shared_rank(s_m + row, c));
-    if (x.M > -INFINITY) {
-      for (int c = 0; c < p.splits; ++c)
-        x.add(*cluster.map_shared_rank(s_m + row, c), *cluster.map_shared_rank(s_l + row, c),
-              *cluster.map_shared_rank(reinterpret_cast<const float4*>(part + row * D + col), c));
-    }
-    *reinterpret_cast<uint2*>(out_row(row) + col) = x.result<kBf16>();
-  }
+  merge_cluster<D, kBf16>(p, rank * kWideThreads + threadIdx.x, kWideThreads, n_rows, part, s_m, s_l, out_row);
   cluster.sync();                                                    // no CTA leaves while another reads its partials
 }
 
@@ -1239,7 +1215,7 @@ __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restric
                                                           uint4* __restrict__ vc, const int64_t* __restrict__ slots, int n_tok, int ng, int chunks,
                                                           int64_t k_st, int64_t k_sh, int64_t v_st, int64_t v_sh, int* __restrict__ arrived,
                                                           int64_t n_arrived) {
-  allow_next();
+  pdl_allow_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, row = static_cast<int64_t>(ng) * chunks;
   if (kCount && idx < n_arrived) arrived[idx] = 0;
   if (idx >= n_tok * row) return;
@@ -1250,7 +1226,7 @@ __global__ void __launch_bounds__(256) paged_write_kernel(const uint4* __restric
   vc[dst] = v[t * v_st + h * v_sh + u];
 }
 
-// in the stream's order, but for what the kernels' own waits leave open (await_previous)
+// in the stream's order, but for what the kernels' own waits leave open (pdl_await_previous)
 struct Launch {
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2]{};
