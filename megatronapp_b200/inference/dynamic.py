@@ -341,7 +341,7 @@ class DynamicInferenceContext:
         if d == 128:
             better = longest >= 160
         else:
-            better = longest > 64 * ranges64 * (11 if tiles * ng > 2 * 148 else 5) and ranges >= ranges64
+            better = -(-longest // 64) >= (12 if tiles * ng > 2 * 148 else 6) * ranges64 and ranges >= ranges64
         return (tiles, ranges) if better else (0, 1)
 
     def _kernel_plan(self, group: int, ng: int, d: int) -> tuple:

@@ -28,9 +28,10 @@ def test_a_step_without_portions_plans_no_tiles():
     ([(0, 320)], 1, 4, 64, (0, 1)), ([(0, 321)], 1, 4, 64, (3, 1)),                      # heads of 64: more than five stages
     ([(113, 113)] * 4, 8, 12, 64, (0, 1)), ([(240, 113)] * 4, 8, 12, 64, (0, 1)),        # more than two waves
     ([(600, 113)] * 4, 8, 12, 64, (32, 1)),                                              # ... of more than eleven stages
+    ([(0, 214), (214, 214), (428, 214), (0, 214)], 1, 8, 64, (0, 1)),                    # in two ranges five and a half stages
     ([(2159, 122)], 1, 8, 64, (0, 1)),                                                   # in eight ranges five stages
     ([(2584, 22), (223, 219), (304, 22), (48, 22)], 1, 8, 64, (0, 1)),                   # two ranges where the 64-row tiles take four
-    ([(4000, 100)], 1, 4, 64, (0, 1)), ([(9000, 100)], 1, 4, 64, (1, 16))])                # in sixteen ranges five stages, nine
+    ([(4000, 100)], 1, 4, 64, (0, 1)), ([(9000, 100)], 1, 4, 64, (1, 16))])                # in sixteen ranges four stages, nine
 def test_tiles_that_have_the_better_kernel(reqs, group, ng, d, want):
     cuts = _context(reqs)._kernel_plan(group, ng, d)[1]
     assert cuts[-2:] == want
