@@ -331,9 +331,9 @@ class DynamicInferenceContext:
     def _wide_plan(self, group: int, ng: int, d: int, ranges64: int) -> tuple:
         """The portions' tiles of 128 rows and key ranges of those, for the kernel that has one such tile on an SM; no tiles where the 64-row ones, in
         ``ranges64`` key ranges, are the better ones.  Its start costs 3 to 4 us more; a stage of 64 keys takes 1.4 us for 3.4 at heads of 128, 1.2 for 2.1 at
-        64, but nothing runs beside the start of a later wave.  128-row / 64-row times of 1420 drawn steps, geometric means: heads of 128 from three stages
-        0.92, from six 0.80, from twelve 0.56; heads of 64 below six stages a CTA 1.05, from six 0.95, from nine 0.67, more than two waves below twelve
-        stages 1.06, from there 0.77, fewer key ranges than the 64-row tiles take 1.1 to 1.4."""
+        64, but nothing runs beside the start of a later wave.  128-row / 64-row times of 1415 drawn steps, geometric means by a CTA's
+        stages: heads of 128 below 160 keys 1.02, from there 0.87, from six stages 0.75, from twelve 0.56; heads of 64 below six 1.07, from there 0.91, from nine
+        0.77, from twelve 0.64; more than two waves of those below twelve 1.05, from there 0.77; fewer key ranges than the 64-row tiles take 1.06, up to 1.3."""
         chunks = [p for p in self._plan if p[2] * group > 16]
         longest = max(p[2] + p[3] for p in chunks)
         tiles = sum(-(-p[2] * group // 128) for p in chunks)
