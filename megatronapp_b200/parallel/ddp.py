@@ -142,7 +142,7 @@ class ParamAndGradBuffer:
             self._zero_ranges = rng
         # one launch for all ranges: 17 fills took the host 107 us of a training pass of four layers
         self._zero_plan = None
-        if self._zero_ranges and self.grad_data.is_cuda:
+        if self._zero_ranges and self.grad_data.is_cuda and self.grad_data.element_size() % 2 == 0:
             table, blocks = ops.ext().zero_ranges_plan(self.grad_data.element_size(), self._zero_ranges)
             self._zero_plan = (self._buffer(), table.to(self.grad_data.device), blocks)
 

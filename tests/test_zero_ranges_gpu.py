@@ -39,3 +39,19 @@ def test_a_buffer_that_was_put_in_place_of_the_first(change):
     rest = int((around == 3).sum()) - int((buf.grad_data == 3).sum())
     buf.zero()
     assert torch.equal(buf.grad_data, want) and int((around == 3).sum()) - int((buf.grad_data == 3).sum()) == rest
+
+
+@pytest.mark.parametrize("dtype", [torch.float8_e4m3fn, torch.bfloat16, torch.float64])
+def test_buffers_of_any_type(dtype):
+    """One-byte gradients, whose ranges may start off the kernel's two bytes, are filled range by range."""
+    from megatronapp_b200.parallel.ddp import DistributedDataParallelConfig, ParamAndGradBuffer
+
+    params = [torch.nn.Parameter(torch.zeros(n, device="cuda")) for n in (640, 1001, 64)]
+    params[1].b200_wgrad_store_first = True
+    buf = ParamAndGradBuffer(DistributedDataParallelConfig(), torch.float32, dtype, params, None, 1, None, 1.0, "cuda")
+    s, e, _ = buf.param_index[params[1]]
+    buf.grad_data.view(torch.uint8).fill_(1)
+    buf.zero()
+    size = buf.grad_data.element_size()
+    got = buf.grad_data.view(torch.uint8)
+    assert bool((got[s * size:e * size] == 1).all()) and not got[:s * size].any() and not got[e * size:].any()
