@@ -40,3 +40,19 @@ def test_which_contexts_are_cut(requests, ng, group, d, longest, mean, beside, c
     from megatronapp_b200 import ops
 
     assert ops.ext().paged_decode_cut(requests, ng, group, d, longest, mean, beside) == ctas
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,group,n", [(128, 4, 3), (64, 1, 3), (128, 1, 90), (64, 2, 200)])      # few CTAs, and more than run at once
+def test_what_follows_waits_for_portions_too(d, group, n):
+    """Decoding requests that are done long before the portion beside them: the next launch of the stream sees the portion's rows."""
+    reqs = [(6000, 500)] + [(5, 1)] * n
+    cx, q, k, v = _step(reqs, 8 * group, 8, d, 16, torch.bfloat16)
+    want = cx.attend(1, q, k, v, d ** -0.5)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        out = cx.attend(1, q, k, v, d ** -0.5)
+        copy = out.clone()
+        out.zero_()
+        torch.cuda.synchronize()
+        assert torch.equal(copy, want) and not out.any()
