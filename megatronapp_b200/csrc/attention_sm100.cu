@@ -3,10 +3,10 @@
 //
 // Forward  (attn_fwd_kernel):  S = Q K^T -> online softmax (exp2 domain, lazy rescale) ->
 //                              P (16-bit, TMEM columns of its own) -> O += P V (O stays in TMEM).
-// Backward (two kernels, deterministic, no atomics):
-//   attn_bwd_kernel<dK, dV> : CTA per 128-key block, loops over 64-query blocks
+// Backward (one launch of two parts, deterministic, no atomics):
+//   bwd_part<dK, dV> : CTA per 128-key block, loops over 64-query blocks
 //                             S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q
-//   attn_bwd_kernel<dQ>     : CTA per 128-query block, loops over 64-key blocks
+//   bwd_part<dQ>     : CTA per 128-query block, loops over 64-key blocks
 //                             S = Q K^T, dP = dO V^T, dQ += dS K
 // Operands are strided [b, h, s, d] views (last dim contiguous) so the Megatron [s, b, h, d]
 // activations are consumed in place (4-D tensor maps); outputs are written in [s, b, h, d].
@@ -498,6 +498,7 @@ attn_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ d
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = (lane % kLanes) * 8;
   const int hi = blockIdx.y, bi = blockIdx.z;
   const int s0 = (blockIdx.x * 8 + warp) * (kRows * kSteps) + lane / kLanes;
+  pdl_allow_next();
   const uint16_t* po = o + bi * o_sb + hi * o_sh + col;
   const uint16_t* pd = d_o + bi * do_sb + hi * do_sh + col;
   uint4 a[kSteps], c[kSteps];
@@ -536,19 +537,19 @@ attn_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ d
 struct BwdParams {
   const float* nlse;    // [b, hq, sq] -LSE in the exp2 domain (-lse * log2e)
   const float* ndelta;  // [b, hq, sq] -delta
-  void* out1;           // dq (kDQ) or dv
-  void* out2;           // unused (kDQ) or dk
-  int64_t o1_sb, o1_sh, o1_ss, o2_sb, o2_sh, o2_ss;
+  void *dq, *dk, *dv;
+  int64_t dq_sb, dq_sh, dq_ss, dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
   int b, hq, hkv, sq, sk;
   float scale_log2, scale;
   int causal;
   int wait_limit;       // tries of a wait before it gives up
+  int n_kv;             // CTAs for dK and dV; those behind them are for dQ
 };
 
 constexpr int kBwdRows = 128;   // resident rows per CTA (keys for dK/dV, queries for dQ)
 constexpr int kBwdCols = 64;    // streamed rows per iteration (queries for dK/dV, keys for dQ)
 
-template <int D, bool kDQ>
+template <int D>
 struct BwdSmem {
   static constexpr int kDC = D / 64;
   static constexpr int kStages = 4;                     // streamed-tile ring depth (hides TMA latency)
@@ -571,13 +572,12 @@ struct BwdSmem {
 // tensor core working on one while the other's P / dS are made, and two warpgroups share a buffer, 32 columns each.  T is in registers
 // 150 cycles after it is complete; its columns then take the next T, so that the math finds it made.  One warp issues T, one the products
 // with P / dS: the waits of either take long enough to empty the tensor core's queue.
-// CTAs start with the longest rows of a causal problem.  32 / 8 heads x 4096 x 128, both kernels: 513 us with P / dS over T, 441 so.
+// CTAs start with the longest rows of a causal problem.  32 / 8 heads x 4096 x 128, both parts: 513 us with P / dS over T, 441 so.
+// The maps' boxes are 64 rows high.  bid: this CTA's place among those of its part.
 template <int D, bool kDQ, bool kBf16>
-__global__ void __launch_bounds__(kThreads, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_constant__ CUtensorMap tmap_x2,
-                const __grid_constant__ CUtensorMap tmap_y1, const __grid_constant__ CUtensorMap tmap_y2,
-                const BwdParams p) {
-  using L = BwdSmem<D, kDQ>;
+__device__ __forceinline__ void bwd_part(const CUtensorMap& tmap_x1, const CUtensorMap& tmap_x2, const CUtensorMap& tmap_y1, const CUtensorMap& tmap_y2,
+                                         const BwdParams& p, int bid) {
+  using L = BwdSmem<D>;
   constexpr int kS = L::kStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -602,9 +602,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   const int G = p.hq / p.hkv;
   // (row block, head, batch) from one grid dimension: every head's longest row block comes before any shorter one
   const int n_out = kDQ ? p.hq : p.hkv;
-  const int blk = static_cast<int>(blockIdx.x) / (n_out * p.b), hb = static_cast<int>(blockIdx.x) % (n_out * p.b);
+  const int blk = bid / (n_out * p.b), hb = bid % (n_out * p.b);
   const int out_head = hb % n_out, bi = hb / n_out;
-  const int n_blk = static_cast<int>(gridDim.x) / (n_out * p.b);
+  const int n_blk = ((kDQ ? p.sq : p.sk) + kBwdRows - 1) / kBwdRows;
   const int r0 = (kDQ ? n_blk - 1 - blk : blk) * kBwdRows;
   // iteration space
   int col_blk0, n_col, n_heads, head0;
@@ -635,7 +635,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  int n_loaded = 0;                            // thread 0: blocks whose copies it has started
+  pdl_await_previous();                        // the statistics of the launch before
+  volatile int* s_loaded = failed + 2;         // blocks whose copies were started, for the end of a CTA in which a wait ran out
   constexpr int kTBufs = kDQ || D == 64 ? 2 : 1;   // T1 and T2 of dK / dV at D = 128 have room for one block
   const uint32_t tmem_A1 = tmem_base;              // dV or dQ
   const uint32_t tmem_A2 = tmem_base + D;          // dK
@@ -648,10 +649,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
     if (warp_idx == 0 && lane == 0 && n_iter > 0) {
       // ============================================================ TMA producer
       mbar_arrive_expect_tx(x_full, 2 * L::kX);
-      for (int c = 0; c < L::kDC; ++c) {
-        tma_load_4d(&tmap_x1, x_full, sX1 + c * (kBwdRows * 128), c * 64, out_head, bi, r0);
-        tma_load_4d(&tmap_x2, x_full, sX2 + c * (kBwdRows * 128), c * 64, out_head, bi, r0);
+      for (int c = 0; c < 2 * L::kDC; ++c) {
+        const int off = (c >> 1) * (kBwdRows * 128) + (c & 1) * (64 * 128), row = r0 + (c & 1) * 64;
+        tma_load_4d(&tmap_x1, x_full, sX1 + off, (c >> 1) * 64, out_head, bi, row);
+        tma_load_4d(&tmap_x2, x_full, sX2 + off, (c >> 1) * 64, out_head, bi, row);
       }
+      int n_loaded = 0;
       for (; n_loaded < n_iter; ++n_loaded) {
         const int it = n_loaded, ys = it % kS;
         const int head = kDQ ? out_head / G : head0 + it / n_col;   // head of the streamed tiles
@@ -670,6 +673,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
           bulk_load_1d(sStat + ys * 128 + 64, p.ndelta + base, 256, &y_full[ys]);
         }
       }
+      *s_loaded = n_loaded;
     } else if (warp_idx == 1 && n_iter > 0) {
       // ============================================================ issuer of T1 and T2
       constexpr uint32_t idesc_t = make_idesc_f16(kBf16, kBwdRows, kBwdCols, false, false);
@@ -830,9 +834,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
         }
       };
       // the warpgroups share the epilogue: 32 columns of dQ each, or half of dV's or dK's
-      if (kDQ) store_acc(tmem_A1, p.out1, p.o1_sb, p.o1_sh, p.o1_ss, p.scale, min(wg, D / 32), min(wg + 1, D / 32));
-      else if (tb == 0) store_acc(tmem_A1, p.out1, p.o1_sb, p.o1_sh, p.o1_ss, 1.f, half * (D / 64), (half + 1) * (D / 64));
-      else store_acc(tmem_A2, p.out2, p.o2_sb, p.o2_sh, p.o2_ss, p.scale, half * (D / 64), (half + 1) * (D / 64));
+      if (kDQ) store_acc(tmem_A1, p.dq, p.dq_sb, p.dq_sh, p.dq_ss, p.scale, min(wg, D / 32), min(wg + 1, D / 32));
+      else if (tb == 0) store_acc(tmem_A1, p.dv, p.dv_sb, p.dv_sh, p.dv_ss, 1.f, half * (D / 64), (half + 1) * (D / 64));
+      else store_acc(tmem_A2, p.dk, p.dk_sb, p.dk_sh, p.dk_ss, p.scale, half * (D / 64), (half + 1) * (D / 64));
     }
   }
   tc_fence_before();
@@ -842,19 +846,38 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_x1, const __grid_consta
     if (threadIdx.x == 0) {
       atomicExch(&g_attn_error, 1);
       wait_bar(x_full, 0, &never);
+      const int n_loaded = *s_loaded;
       for (int i = max(0, n_loaded - kS); i < n_loaded; ++i) wait_bar(&y_full[i % kS], (i / kS) & 1, &never);
     } else if (warp_idx == 1 || warp_idx == 2) {
       if (elect_one()) umma_commit(drained);
       wait_bar_warp(drained, 0, &never);
     } else if (warp_idx >= 4) {
       const int rows = min(kBwdRows, (kDQ ? p.sq : p.sk) - r0);
-      fill_nan<D>(p.out1, static_cast<int64_t>(r0) * p.o1_ss + static_cast<int64_t>(bi) * p.o1_sb + static_cast<int64_t>(out_head) * p.o1_sh, p.o1_ss, rows);
-      if (!kDQ)
-        fill_nan<D>(p.out2, static_cast<int64_t>(r0) * p.o2_ss + static_cast<int64_t>(bi) * p.o2_sb + static_cast<int64_t>(out_head) * p.o2_sh, p.o2_ss, rows);
+      auto fill = [&](void* out, int64_t sb, int64_t sh, int64_t ss) {
+        fill_nan<D>(out, static_cast<int64_t>(r0) * ss + static_cast<int64_t>(bi) * sb + static_cast<int64_t>(out_head) * sh, ss, rows);
+      };
+      if (kDQ) {
+        fill(p.dq, p.dq_sb, p.dq_sh, p.dq_ss);
+      } else {
+        fill(p.dv, p.dv_sb, p.dv_sh, p.dv_ss);
+        fill(p.dk, p.dk_sb, p.dk_sh, p.dk_ss);
+      }
     }
     __syncthreads();
   }
   if (warp_idx == 2) tmem_dealloc<512>(tmem_base);
+}
+
+// dK and dV first, then dQ, each with its longest rows first: neither waits for the other, and the short rows of the former end under the long ones of
+// the latter.  us of a backward call, a launch each / one: 1 x 32 / 8 heads x 4096 x 128 457 / 439, x 512 54 / 41; 4 x 12 x 1024 x 64 73 / 64, 2 x 16 x 256
+// x 64 23 / 12.5 (neither part fills the SMs).
+template <int D, bool kBf16>
+__global__ void __launch_bounds__(kThreads, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                const __grid_constant__ CUtensorMap tmap_do, const BwdParams p) {
+  const int bid = static_cast<int>(blockIdx.x);
+  if (bid < p.n_kv) bwd_part<D, false, kBf16>(tmap_k, tmap_v, tmap_q, tmap_do, p, bid);
+  else bwd_part<D, true, kBf16>(tmap_q, tmap_do, tmap_k, tmap_v, p, bid - p.n_kv);
 }
 
 // ------------------------------------------------------------------------------------ host side
@@ -937,40 +960,40 @@ int launch_fwd(const AttnArgs& a, cudaStream_t s) {
 }
 
 
-template <int D, bool kDQ, bool kBf16>
-int launch_bwd_one(const AttnArgs& a, cudaStream_t s) {
-  using L = BwdSmem<D, kDQ>;
-  CUtensorMap x1{}, x2{}, y1{}, y2{};
-  bool ok = true;
-  if (kDQ) {
-    ok = ok && make_tmap_bhsd(&x1, a.q, a.is_bf16, D, a.hq, a.b, a.sq, a.q_sh, a.q_sb, a.q_ss, kBwdRows);
-    ok = ok && make_tmap_bhsd(&x2, a.d_o, a.is_bf16, D, a.hq, a.b, a.sq, a.do_sh, a.do_sb, a.do_ss, kBwdRows);
-    ok = ok && make_tmap_bhsd(&y1, a.k, a.is_bf16, D, a.hkv, a.b, a.sk, a.k_sh, a.k_sb, a.k_ss, kBwdCols);
-    ok = ok && make_tmap_bhsd(&y2, a.v, a.is_bf16, D, a.hkv, a.b, a.sk, a.v_sh, a.v_sb, a.v_ss, kBwdCols);
-  } else {
-    ok = ok && make_tmap_bhsd(&x1, a.k, a.is_bf16, D, a.hkv, a.b, a.sk, a.k_sh, a.k_sb, a.k_ss, kBwdRows);
-    ok = ok && make_tmap_bhsd(&x2, a.v, a.is_bf16, D, a.hkv, a.b, a.sk, a.v_sh, a.v_sb, a.v_ss, kBwdRows);
-    ok = ok && make_tmap_bhsd(&y1, a.q, a.is_bf16, D, a.hq, a.b, a.sq, a.q_sh, a.q_sb, a.q_ss, kBwdCols);
-    ok = ok && make_tmap_bhsd(&y2, a.d_o, a.is_bf16, D, a.hq, a.b, a.sq, a.do_sh, a.do_sb, a.do_ss, kBwdCols);
-  }
-  if (!ok) return -5;
-  auto kern = attn_bwd_kernel<D, kDQ, kBf16>;
+template <int D, bool kBf16>
+int launch_bwd_parts(const AttnArgs& a, cudaStream_t s) {
+  using L = BwdSmem<D>;
+  CUtensorMap tq{}, tk{}, tv{}, tdo{};
+  if (!make_tmap_bhsd(&tq, a.q, a.is_bf16, D, a.hq, a.b, a.sq, a.q_sh, a.q_sb, a.q_ss, kBwdCols) ||
+      !make_tmap_bhsd(&tk, a.k, a.is_bf16, D, a.hkv, a.b, a.sk, a.k_sh, a.k_sb, a.k_ss, kBwdCols) ||
+      !make_tmap_bhsd(&tv, a.v, a.is_bf16, D, a.hkv, a.b, a.sk, a.v_sh, a.v_sb, a.v_ss, kBwdCols) ||
+      !make_tmap_bhsd(&tdo, a.d_o, a.is_bf16, D, a.hq, a.b, a.sq, a.do_sh, a.do_sb, a.do_ss, kBwdCols))
+    return -5;
+  auto kern = attn_bwd_kernel<D, kBf16>;
   static const bool ready = prepare_kernel(kern, L::kTotal, "attn_bwd");
   if (!ready) return -10;
   BwdParams p{};
   p.nlse = a.delta + static_cast<int64_t>(a.b) * a.hq * a.sq;   // written by attn_delta_kernel
   p.ndelta = a.delta;
-  if (kDQ) { p.out1 = a.dq; p.o1_sb = a.dq_sb; p.o1_sh = a.dq_sh; p.o1_ss = a.dq_ss; }
-  else {
-    p.out1 = a.dv; p.o1_sb = a.dv_sb; p.o1_sh = a.dv_sh; p.o1_ss = a.dv_ss;
-    p.out2 = a.dk; p.o2_sb = a.dk_sb; p.o2_sh = a.dk_sh; p.o2_ss = a.dk_ss;
-  }
+  p.dq = a.dq; p.dq_sb = a.dq_sb; p.dq_sh = a.dq_sh; p.dq_ss = a.dq_ss;
+  p.dk = a.dk; p.dk_sb = a.dk_sb; p.dk_sh = a.dk_sh; p.dk_ss = a.dk_ss;
+  p.dv = a.dv; p.dv_sb = a.dv_sb; p.dv_sh = a.dv_sh; p.dv_ss = a.dv_ss;
   p.b = a.b; p.hq = a.hq; p.hkv = a.hkv; p.sq = a.sq; p.sk = a.sk;
   p.scale_log2 = a.scale * kLog2e; p.scale = a.scale; p.causal = a.causal ? 1 : 0; p.wait_limit = a.wait_limit < 0 ? kWaitLimit : a.wait_limit;
-  const int64_t ctas = static_cast<int64_t>(((kDQ ? a.sq : a.sk) + kBwdRows - 1) / kBwdRows) * (kDQ ? a.hq : a.hkv) * a.b;
-  if (ctas > 0x7fffffff) { g_attn_err = "too many row blocks"; return -12; }
-  kern<<<static_cast<unsigned>(ctas), kThreads, L::kTotal, s>>>(x1, x2, y1, y2, p);
-  cudaError_t e = cudaGetLastError();
+  const int64_t n_kv = static_cast<int64_t>((a.sk + kBwdRows - 1) / kBwdRows) * a.hkv * a.b, n_q = static_cast<int64_t>((a.sq + kBwdRows - 1) / kBwdRows) * a.hq * a.b;
+  if (n_kv + n_q > 0x7fffffff) { g_attn_err = "too many row blocks"; return -12; }
+  p.n_kv = static_cast<int>(n_kv);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(n_kv + n_q));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};                    // CTAs may start under the statistics' kernel, and wait for its end
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, p);
   if (e != cudaSuccess) { g_attn_err = std::string("attn_bwd launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
 }
@@ -983,9 +1006,9 @@ int launch_bwd(const AttnArgs& a, cudaStream_t s) {
   attn_delta_kernel<D><<<dim3((a.sq + kPerBlock - 1) / kPerBlock, a.hq, a.b), 256, 0, s>>>(
       static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.d_o), a.delta, a.lse, a.delta + rows, a.hq, a.sq, a.o_sb, a.o_sh, a.o_ss,
       a.do_sb, a.do_sh, a.do_ss, a.is_bf16 ? 1 : 0);
-  int rc = a.is_bf16 ? launch_bwd_one<D, false, true>(a, s) : launch_bwd_one<D, false, false>(a, s);
-  if (rc != 0) return rc;
-  return a.is_bf16 ? launch_bwd_one<D, true, true>(a, s) : launch_bwd_one<D, true, false>(a, s);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { g_attn_err = std::string("attn_delta launch: ") + cudaGetErrorString(e); return -11; }
+  return a.is_bf16 ? launch_bwd_parts<D, true>(a, s) : launch_bwd_parts<D, false>(a, s);
 }
 
 }  // namespace

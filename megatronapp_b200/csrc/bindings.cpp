@@ -856,7 +856,7 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o, const Tensor& q, const Tensor& k
   a.wait_limit = wait_limit;
   int rc = b200::attn_bwd(a, cur_stream());
   TORCH_CHECK(rc == 0, "b200 attn_bwd failed: ", rc, " ", b200::attn_last_error());
-  count(3);
+  count(2);
   return {dq, dk, dv};
 }
 
