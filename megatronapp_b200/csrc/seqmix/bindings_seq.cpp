@@ -932,9 +932,9 @@ std::vector<Tensor> ssd_forward(const Tensor& x, const Tensor& dt, const Tensor&
   count(4); check_last_error("ssd_forward");
   return {y, last, scores, states, decay};
 }
-// -> dx, ddt, dA, dB, dC, dD, d(initial state)
+// -> dx, ddt, dA, dB, dC, dD, d(initial state); without `sums` dA and dD are those of each block, [b, blocks, heads]
 std::vector<Tensor> ssd_backward(const Tensor& dy, c10::optional<Tensor> dlast, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B,
-                                 const Tensor& C, const Tensor& D, const Tensor& scores, const Tensor& states, const Tensor& decay, bool want_first) {
+                                 const Tensor& C, const Tensor& D, const Tensor& scores, const Tensor& states, const Tensor& decay, bool want_first, bool sums) {
   c10::cuda::CUDAGuard g(x.device());
   b200seq::SsdArgs p = ssd_args(x, dt, A, B, C, D);
   const int64_t n = B.size(3);
@@ -959,6 +959,7 @@ std::vector<Tensor> ssd_backward(const Tensor& dy, c10::optional<Tensor> dlast, 
   p.partial = sub > 1 ? partial.data_ptr<float>() : nullptr;
   TORCH_CHECK(b200seq::ssd_backward(p, static_cast<int>(n), x.scalar_type() == at::kBFloat16, cur_stream()), "ssd_backward: shared memory");
   count(sub > 1 ? 4 : 3); check_last_error("ssd_backward");
+  if (!sums) return {dx, ddt, dA, dB, dC, dD, dfirst};
   return {dx, ddt, dA.sum(at::IntArrayRef{0, 1}), dB, dC, dD.sum(at::IntArrayRef{0, 1}), dfirst};
 }
 
@@ -1004,7 +1005,7 @@ std::vector<Tensor> mamba_gated_norm(const Tensor& y, const Tensor& zx, const Te
   count(); check_last_error("mamba_gated_norm");
   return {out, rstd};
 }
-// the norm's half of the backward -> dy [b, s, di], dzx [s, b, width] with its z columns filled, d(norm weight) fp32 [di]
+// the norm's half of the backward -> dy [b, s, di], dzx [s, b, width] with its z columns filled, d(norm weight) [di]
 std::vector<Tensor> mamba_gated_norm_grad(const Tensor& dout, const Tensor& rstd, const Tensor& y, const Tensor& zx, const Tensor& conv_w, const Tensor& conv_b,
                                           const Tensor& dt_bias, const Tensor& norm_w, int64_t groups) {
   c10::cuda::CUDAGuard g(zx.device());
@@ -1012,14 +1013,18 @@ std::vector<Tensor> mamba_gated_norm_grad(const Tensor& dout, const Tensor& rstd
   TORCH_CHECK(y.is_contiguous() && y.scalar_type() == zx.scalar_type() && y.numel() == static_cast<int64_t>(p.s) * p.b * p.di, "bad y");
   TORCH_CHECK(dout.is_contiguous() && dout.scalar_type() == zx.scalar_type() && dout.numel() == y.numel() && reinterpret_cast<uintptr_t>(dout.data_ptr()) % 16 == 0, "bad dout");
   check_f32(rstd, "rstd");
-  Tensor dy = torch::empty_like(y), dzx = torch::empty_like(zx), part = torch::empty({b200seq::mamba_norm_parts(p.s, p.b), p.di}, dt_bias.options());
+  Tensor dy = torch::empty_like(y), dzx = torch::empty_like(zx), part;
+  p.norm_rows = b200seq::mamba_norm_rows(p.s, p.b, p.groups);
+  part = torch::empty({b200seq::mamba_norm_parts(p.s, p.b, p.norm_rows), p.di}, dt_bias.options());
   p.y = y.data_ptr(); p.dout = dout.data_ptr(); p.rstd = rstd.data_ptr<float>(); p.dy = dy.data_ptr(); p.dzx = dzx.data_ptr(); p.norm_part = part.data_ptr<float>();
+  Tensor dnorm = torch::empty_like(norm_w);
+  p.dnorm_w = dnorm.data_ptr();
   b200seq::mamba_gated_norm_grad(p, zx.scalar_type() == at::kBFloat16, cur_stream());
-  count(); check_last_error("mamba_gated_norm_grad");
-  return {dy, dzx, part.sum(0)};
+  count(2); check_last_error("mamba_gated_norm_grad");
+  return {dy, dzx, dnorm};
 }
-// the other half: fills dzx's columns x B C and dt -> d(taps and bias) fp32 [5, conv], d(dt_bias) fp32 [heads].  ddt is overwritten.
-std::vector<Tensor> mamba_before_scan_grad(const Tensor& dxs, const Tensor& dB, const Tensor& dC, Tensor ddt, Tensor dzx, const Tensor& zx, const Tensor& conv_w,
+// the other half: fills dzx's columns x B C and dt -> d(taps), d(bias), d(dt_bias), dA and dD (fp32 [heads]) from those of each block.  ddt is overwritten.
+std::vector<Tensor> mamba_before_scan_grad(const Tensor& dxs, const Tensor& dB, const Tensor& dC, Tensor ddt, const Tensor& dA, const Tensor& dD, Tensor dzx, const Tensor& zx, const Tensor& conv_w,
                                            const Tensor& conv_b, const Tensor& dt_bias, const Tensor& norm_w, int64_t groups) {
   c10::cuda::CUDAGuard g(zx.device());
   b200seq::MambaArgs p = mamba_args(zx, conv_w, conv_b, dt_bias, norm_w, groups, 0.0);
@@ -1027,13 +1032,19 @@ std::vector<Tensor> mamba_before_scan_grad(const Tensor& dxs, const Tensor& dB, 
   for (const Tensor* t : {&dxs, &dB, &dC}) TORCH_CHECK(t->is_contiguous() && t->scalar_type() == zx.scalar_type() && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 == 0, "bad gradients");
   TORCH_CHECK(dxs.numel() == rows * p.di && dB.numel() == rows * gn && dC.numel() == rows * gn && ddt.numel() == rows * p.heads && dzx.is_contiguous() &&
               dzx.sizes() == zx.sizes() && dzx.scalar_type() == zx.scalar_type(), "bad gradients");
-  check_f32(ddt, "ddt");
+  check_f32(ddt, "ddt"); check_f32(dA, "dA"); check_f32(dD, "dD");
+  TORCH_CHECK(dA.dim() == 3 && dA.size(0) == p.b && dA.size(2) == p.heads && dA.sizes() == dD.sizes(), "dA and dD must be [b, blocks, heads]");
+  p.n_chunks = static_cast<int>(dA.size(1)); p.dA_part = dA.data_ptr<float>(); p.dD_part = dD.data_ptr<float>();
   p.conv_run = b200seq::mamba_conv_run(p.s, p.b, p.conv, zx.scalar_type() == at::kBFloat16);
   Tensor part = torch::empty({static_cast<int64_t>(p.b) * b200seq::mamba_conv_parts(p.s, p.conv_run), 5, p.conv}, dt_bias.options());
   p.dxs = dxs.data_ptr(); p.dB = dB.data_ptr(); p.dC = dC.data_ptr(); p.ddt = ddt.data_ptr<float>(); p.dzx = dzx.data_ptr(); p.conv_part = part.data_ptr<float>();
+  Tensor dconv_w = torch::empty_like(conv_w), dconv_b = torch::empty_like(conv_b), ddt_bias = torch::empty_like(dt_bias);
+  Tensor sum_a = torch::empty_like(ddt_bias), sum_d = torch::empty_like(ddt_bias);
+  p.dA = sum_a.data_ptr<float>(); p.dD = sum_d.data_ptr<float>();
+  p.dconv_w = dconv_w.data_ptr(); p.dconv_b = dconv_b.data_ptr(); p.ddt_bias = ddt_bias.data_ptr<float>();
   b200seq::mamba_before_scan_grad(p, zx.scalar_type() == at::kBFloat16, cur_stream());
-  count(2); check_last_error("mamba_before_scan_grad");
-  return {part.sum(0), ddt.view({rows, p.heads}).sum(0)};
+  count(3); check_last_error("mamba_before_scan_grad");
+  return {dconv_w, dconv_b, ddt_bias, sum_a, sum_d};
 }
 
 }  // namespace
@@ -1074,7 +1085,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mamba_gated_norm_grad", &mamba_gated_norm_grad);
   m.def("mamba_before_scan_grad", &mamba_before_scan_grad);
   m.def("ssd_forward", &ssd_forward);
-  m.def("ssd_backward", &ssd_backward);
+  m.def("ssd_backward", &ssd_backward, py::arg("dy"), py::arg("dlast"), py::arg("x"), py::arg("dt"), py::arg("A"), py::arg("B"), py::arg("C"), py::arg("D"),
+        py::arg("scores"), py::arg("states"), py::arg("decay"), py::arg("want_first"), py::arg("sums") = true);
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("reset_launch_count", []() { g_launches.store(0); });
 }

@@ -345,13 +345,19 @@ struct MambaArgs {
   void* dzx;                      // [s, b, width]
   float* conv_part;               // [b * mamba_conv_parts, 5, conv]: four taps, bias
   float* norm_part;               // [mamba_norm_parts, di]
+  void *dconv_w, *dconv_b, *dnorm_w;   // as conv_w, conv_b, norm_w
+  float *ddt_bias, *dA, *dD;      // [heads]
+  const float *dA_part, *dD_part; // [b, n_chunks, heads]
   int s, b, width, di, conv, heads, groups;
-  int conv_run;                   // backward: mamba_conv_run
+  int n_chunks;                   // of the scan
+  int conv_run, norm_rows;        // backward: mamba_conv_run, mamba_norm_rows
+  int fwd_run;                    // steps of a CTA of the convolution
   float eps;
 };
 int mamba_conv_run(int steps, int batch, int conv, bool bf16);
 int mamba_conv_parts(int steps, int run);
-int mamba_norm_parts(int steps, int batch);
+int mamba_norm_rows(int steps, int batch, int groups);
+int mamba_norm_parts(int steps, int batch, int norm_rows);
 void mamba_before_scan(const MambaArgs& p, bool bf16, cudaStream_t s);
 void mamba_before_scan_grad(const MambaArgs& p, bool bf16, cudaStream_t s);
 void mamba_gated_norm(const MambaArgs& p, bool bf16, cudaStream_t s);

@@ -2,8 +2,12 @@
 // SiLU, the step sizes' softplus, and the RMS norm of the result gated by SiLU(z), one statistic per group of channels.
 //
 // All of it reads the input projection's columns [z | x B C | dt] where they lie ([steps, batch, width]) and writes the gradients into one
-// tensor of that shape, so nothing is split, transposed, copied or concatenated.  Intermediates stay in fp32 registers; the kernels are
-// bound by HBM.  Mixer of width 2048, 2048 steps, training pass: the PyTorch form of these parts took 1.2 ms in 60 launches.
+// tensor of that shape, so nothing is split, transposed, copied or concatenated.  Intermediates stay in fp32 registers.  Mixer of width 2048,
+// 2048 steps, training pass: the PyTorch form of these parts took 1.2 ms in 60 launches.
+//
+// Bound by the sigmoids' chains of instructions and by the latency of dependent loads, at a third to two thirds of the copy bandwidth.  us at that size (50, 76, 50
+// and 84 MB), with 8-byte loads that wait for the step or row before and quotients that branch, and now: convolution 25.4 and 17.1 (21.8 with the branches),
+// its gradient 43.8 and 28.2, norm 24.5 and 13.6, its gradient 33.2 and 22.2; the column sums behind them 36 in five launches and 8 in two.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -34,50 +38,118 @@ template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16*
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
 }
 
-// ---- convolution.  A thread walks `kRun` steps of four channels with the window in registers.
-constexpr int kFwdRun = 16, kBwdRun = 32;        // backward: 32 or a little more, see mamba_conv_run
+// 1 / (1 + e^-x) without a branch: a division's check for its slow path ends every element's chain of instructions before the next one's can start.  A quick
+// quotient and one step of Newton's method for 1 / d, after which it is off by less than a unit in the last place, as a division; d beyond 2^126 has the
+// quotient 0 and takes no step.
+__device__ __forceinline__ float gate_sigmoid(float x) {
+  const float d = 1.f + expf(-x), q = __fdividef(1.f, d);
+  return d < 8.5e37f ? fmaf(q, fmaf(-d, q, 1.f), q) : q;
+}
 
-template <typename T>
-__global__ void __launch_bounds__(128) mamba_conv_kernel(const MambaArgs p) {
-  const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
+// V channels as they lie in memory (8 or 16 bytes), to be fetched ahead of their use
+template <typename T, int V> struct Raw;
+template <> struct Raw<float, 4> { float4 u; __device__ __forceinline__ void get(float (&v)[4]) const { v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; } };
+template <> struct Raw<__nv_bfloat16, 4> {
+  uint2 u;
+  __device__ __forceinline__ void get(float (&v)[4]) const {
+    v[0] = __uint_as_float(u.x << 16); v[1] = __uint_as_float(u.x & 0xffff0000u);
+    v[2] = __uint_as_float(u.y << 16); v[3] = __uint_as_float(u.y & 0xffff0000u);
+  }
+};
+template <> struct Raw<__nv_bfloat16, 8> {
+  uint4 u;
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+};
+template <typename T, int V> __device__ __forceinline__ Raw<T, V> fetch(const T* p, bool valid = true) {
+  Raw<T, V> r{};
+  if (valid) r = *reinterpret_cast<const Raw<T, V>*>(p);
+  return r;
+}
+__device__ __forceinline__ void put_vec(float* p, const float (&v)[4]) { store4(p, v); }
+__device__ __forceinline__ void put_vec(__nv_bfloat16* p, const float (&v)[4]) { store4(p, v); }
+__device__ __forceinline__ void put_vec(__nv_bfloat16* p, const float (&v)[8]) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    w[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// ---- convolution.  A thread walks `kRun` steps of V channels with the window in registers, four steps at a time; the next four are on their way
+// meanwhile.
+constexpr int kBwdRun = 32;        // backward: 32 or a little more, see mamba_conv_run
+// CTAs of the kernels below that an SM holds
+constexpr int kPlaces = 4, kSms = 148;
+// How many of `units` a CTA takes, a multiple of `step` up to `most`, when `rows` CTAs stand beside each other: a last wave of a few CTAs costs as much as a full
+// one, and every CTA costs `start` units more than those it takes
+// (2048 steps x 6144 channels, 768 CTAs of 16 steps on 592 places 26 us, 516 of 24 steps 22)
+int run_length(int64_t units, int64_t rows, int step, int most, int start) {
+  int best = step;
+  int64_t least = 0;
+  for (int run = step; run <= most; run += step) {
+    const int64_t ctas = (units + run - 1) / run * rows, cost = (ctas + kPlaces * kSms - 1) / (kPlaces * kSms) * (run + start);
+    if (least == 0 || cost <= least) { least = cost; best = run; }
+  }
+  return best;
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(128, kPlaces) mamba_conv_kernel(const MambaArgs p) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) * V;
   if (c >= p.conv) return;
-  const int t0 = blockIdx.y * kFwdRun, b = blockIdx.z;
+  const int t0 = blockIdx.y * p.fwd_run, b = blockIdx.z;
   const T* x = static_cast<const T*>(p.zx) + static_cast<int64_t>(b) * p.width + p.di + c;
   const int64_t step = static_cast<int64_t>(p.b) * p.width;
   T* out = static_cast<T*>(p.xbc) + (static_cast<int64_t>(b) * p.s) * p.conv + c;
-  float w[4][4], bias[4], win[4][4];               // w[channel][tap]
+  Raw<T, V> next[4];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) load4(static_cast<const T*>(p.conv_w) + (c + e) * 4, w[e]);
-  load4(static_cast<const T*>(p.conv_b) + c, bias);
+  for (int k = 0; k < 4; ++k) next[k] = fetch<T, V>(x + (t0 + k) * step, t0 + k < p.s);
+  float w[V][4], bias[V], win[4][V];               // w[channel][tap]
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
+  for (int e = 0; e < V; ++e) load4(static_cast<const T*>(p.conv_w) + (c + e) * 4, w[e]);
+  fetch<T, V>(static_cast<const T*>(p.conv_b) + c).get(bias);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) win[k + 1][e] = 0.f;
-    if (t0 - 3 + k >= 0) load4(x + (t0 - 3 + k) * step, win[k + 1]);
-  }
-#pragma unroll 4
-  for (int i = 0; i < kFwdRun; ++i) {
-    const int t = t0 + i;
-    if (t >= p.s) break;
+  for (int k = 0; k < 3; ++k) fetch<T, V>(x + (t0 - 3 + k) * step, t0 - 3 + k >= 0).get(win[k + 1]);
+#pragma unroll 1
+  for (int i0 = 0; i0 < p.fwd_run && t0 + i0 < p.s; i0 += 4) {
+    Raw<T, V> now[4];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) win[k][e] = win[k + 1][e];
-    load4(x + t * step, win[3]);
-    float o[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float v = bias[e];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) v = fmaf(w[e][k], win[k][e], v);
-      o[e] = v * sigmoidf_(v);
+    for (int k = 0; k < 4; ++k) {
+      now[k] = next[k];
+      next[k] = fetch<T, V>(x + (t0 + i0 + 4 + k) * step, i0 + 4 < p.fwd_run && t0 + i0 + 4 + k < p.s);
     }
-    store4(out + static_cast<int64_t>(t) * p.conv, o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = t0 + i0 + i;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int e = 0; e < V; ++e) win[k][e] = win[k + 1][e];
+      now[i].get(win[3]);
+      float o[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        float v = bias[e];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v = fmaf(w[e][k], win[k][e], v);
+        o[e] = v * gate_sigmoid(v);
+      }
+      if (t < p.s) put_vec(out + static_cast<int64_t>(t) * p.conv, o);
+    }
   }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(128, 5) mamba_conv_grad_kernel(const MambaArgs p) {
+__global__ void __launch_bounds__(128, sizeof(T) == 2 ? 4 : 3) mamba_conv_grad_kernel(const MambaArgs p) {
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= p.conv) return;
   const int run = p.conv_run, t0 = blockIdx.y * run, b = blockIdx.z;
@@ -104,42 +176,58 @@ __global__ void __launch_bounds__(128, 5) mamba_conv_grad_kernel(const MambaArgs
       db[e] = 0.f;
     }
 #pragma unroll
-  for (int k = 0; k < 3; ++k)
-    if (t0 - 3 + k >= 0) load4(x + (t0 - 3 + k) * step, win[k + 1]);
-#pragma unroll 1
-  for (int i = 0; i < run + 3; ++i) {
-    const int t = t0 + i;
-    float g[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int k = 0; k < 3; ++k) fetch<T, 4>(x + (t0 - 3 + k) * step, t0 - 3 + k >= 0).get(win[k + 1]);
+  const int steps = min(run + 3, p.s + 3 - t0);    // behind the sequence's end there is nothing but the last three steps' gradients
+  Raw<T, 4> nx[4], ng[4];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+  for (int k = 0; k < 4; ++k) {
+    nx[k] = fetch<T, 4>(x + (t0 + k) * step, t0 + k < p.s);
+    ng[k] = fetch<T, 4>(dout + (t0 + k) * dstep, t0 + k < p.s);
+  }
+#pragma unroll 1
+  for (int i0 = 0; i0 < steps; i0 += 4) {
+    Raw<T, 4> cx[4], cg[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int t = t0 + i0 + 4 + k;
+      cx[k] = nx[k];
+      cg[k] = ng[k];
+      nx[k] = fetch<T, 4>(x + t * step, i0 + 4 + k < run + 3 && t < p.s);
+      ng[k] = fetch<T, 4>(dout + t * dstep, i0 + 4 + k < run + 3 && t < p.s);
+    }
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+      const int i = i0 + k4, t = t0 + i;
+      float g[4];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          win[k][e] = win[k + 1][e];
+          d[k][e] = d[k + 1][e];
+        }
+      cx[k4].get(win[3]);
+      cg[k4].get(g);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        win[k][e] = win[k + 1][e];
-        d[k][e] = d[k + 1][e];
+        float v = bias[e];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v = fmaf(w[e][k], win[k][e], v);
+        const float sg = gate_sigmoid(v), pre = g[e] * (sg * fmaf(v, 1.f - sg, 1.f));
+        d[3][e] = t < p.s ? pre : 0.f;
+        if (i < run) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) dw[k][e] = fmaf(d[3][e], win[k][e], dw[k][e]);
+          db[e] += d[3][e];
+        }
       }
-    if (t < p.s) {
-      load4(x + t * step, win[3]);
-      load4(dout + t * dstep, g);
-    }
+      // step t - 3 has now seen the four outputs that it enters
+      if (i >= 3 && i < run + 3 && t - 3 < p.s) {
+        float o[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float v = bias[e];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) v = fmaf(w[e][k], win[k][e], v);
-      const float sg = sigmoidf_(v), pre = g[e] * (sg * fmaf(v, 1.f - sg, 1.f));
-      d[3][e] = t < p.s ? pre : 0.f;
-      if (i < run) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) dw[k][e] = fmaf(d[3][e], win[k][e], dw[k][e]);
-        db[e] += d[3][e];
+        for (int e = 0; e < 4; ++e) o[e] = fmaf(w[e][3], d[0][e], fmaf(w[e][2], d[1][e], fmaf(w[e][1], d[2][e], w[e][0] * d[3][e])));
+        store4(dx + (t - 3) * step, o);
       }
-    }
-    // step t - 3 has now seen the four outputs that it enters
-    if (i >= 3 && t - 3 < p.s) {
-      float o[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) o[e] = fmaf(w[e][3], d[0][e], fmaf(w[e][2], d[1][e], fmaf(w[e][1], d[2][e], w[e][0] * d[3][e])));
-      store4(dx + (t - 3) * step, o);
     }
   }
   float* part = p.conv_part + (static_cast<int64_t>(b) * gridDim.y + blockIdx.y) * 5 * p.conv + c;
@@ -161,124 +249,177 @@ __global__ void __launch_bounds__(256) mamba_dt_kernel(const MambaArgs p) {
   if (!kGrad) {
     p.dt[i] = v > 20.f ? v : log1pf(expf(v));
   } else {
-    const float d = p.ddt[i] * (v > 20.f ? 1.f : sigmoidf_(v));
+    const float d = p.ddt[i] * (v > 20.f ? 1.f : gate_sigmoid(v));
     p.ddt[i] = d;
     st(static_cast<T*>(p.dzx) + at, d);
   }
 }
 
-// ---- gated norm: u = y silu(z), out = u / sqrt(mean_group(u^2) + eps) * w.  One warp per (step, batch, group).
-template <typename T>
+// ---- gated norm: u = y silu(z), out = u / sqrt(mean_group(u^2) + eps) * w.  kWarps warps (one, or the CTA's four) share a (step, batch, group), each lane
+// kVec vectors of V channels, which stay in registers between the sum and the result.
+template <int kWarps>
+__device__ __forceinline__ float item_sum(float v, float* s_sum) {
+  v = warp_sum(v);
+  if constexpr (kWarps > 1) {
+    __syncthreads();                               // the sums before these have been read
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
+  }
+  return v;
+}
+
+template <typename T, int V, int kWarps, int kVec>
 __global__ void __launch_bounds__(128) mamba_norm_kernel(const MambaArgs p) {
-  const int64_t item = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5), n = static_cast<int64_t>(p.s) * p.b * p.groups;
+  __shared__ float s_sum[4];
+  const int64_t item = kWarps == 1 ? static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5) : blockIdx.x, n = static_cast<int64_t>(p.s) * p.b * p.groups;
   if (item >= n) return;
-  const int lane = threadIdx.x & 31, W = p.di / p.groups, g = static_cast<int>(item % p.groups);
+  const int lane = kWarps == 1 ? threadIdx.x & 31 : threadIdx.x, W = p.di / p.groups, g = static_cast<int>(item % p.groups);
   const int64_t row = item / p.groups;             // t * b + batch
   const int t = static_cast<int>(row / p.b), b = static_cast<int>(row % p.b);
   const T* y = static_cast<const T*>(p.y) + (static_cast<int64_t>(b) * p.s + t) * p.di + g * W;
   const T* z = static_cast<const T*>(p.zx) + row * p.width + g * W;
-  float s = 0.f;
-#pragma unroll 4
-  for (int c = lane * 4; c < W; c += 128) {
-    float yv[4], zv[4];
-    load4(y + c, yv);
-    load4(z + c, zv);
+  const T* w = static_cast<const T*>(p.norm_w) + g * W;
+  Raw<T, V> ry[kVec], rz[kVec], rw[kVec];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float u = yv[e] * zv[e] * sigmoidf_(zv[e]);
-      s = fmaf(u, u, s);
+  for (int i = 0; i < kVec; ++i) {
+    const int c = (i * 32 * kWarps + lane) * V;
+    ry[i] = fetch<T, V>(y + c, c < W);
+    rz[i] = fetch<T, V>(z + c, c < W);
+    rw[i] = fetch<T, V>(w + c, c < W);
+  }
+  float u[kVec][V], s = 0.f;
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    float zv[V];
+    ry[i].get(u[i]);
+    rz[i].get(zv);
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      u[i][e] = u[i][e] * zv[e] * gate_sigmoid(zv[e]);
+      s = fmaf(u[i][e], u[i][e], s);
     }
   }
-  s = warp_sum(s);
+  s = item_sum<kWarps>(s, s_sum);
   const float r = rsqrtf(s / W + p.eps);
   if (lane == 0) p.rstd[item] = r;
-  const T* w = static_cast<const T*>(p.norm_w) + g * W;
   T* out = static_cast<T*>(p.out) + row * p.di + g * W;
-#pragma unroll 4
-  for (int c = lane * 4; c < W; c += 128) {
-    float yv[4], zv[4], wv[4], o[4];
-    load4(y + c, yv);
-    load4(z + c, zv);
-    load4(w + c, wv);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = yv[e] * zv[e] * sigmoidf_(zv[e]) * r * wv[e];
-    store4(out + c, o);
+  for (int i = 0; i < kVec; ++i) {
+    const int c = (i * 32 * kWarps + lane) * V;
+    float wv[V], o[V];
+    rw[i].get(wv);
+#pragma unroll
+    for (int e = 0; e < V; ++e) o[e] = u[i][e] * r * wv[e];
+    if (c < W) put_vec(out + c, o);
   }
 }
 
-// four warps of a CTA share kNormRows rows of one group; kVec: groups of four channels per lane
-constexpr int kNormRows = 16;      // four to a warp, each two dependent passes: latency, so many CTAs (2048 x 4096: 52 us with 32 rows, 33 with 16)
-template <typename T, int kVec>
-__global__ void __launch_bounds__(128) mamba_norm_grad_kernel(const MambaArgs p) {
+// A CTA takes p.norm_rows rows of one group (see mamba_norm_rows), a row to each of its warps or to all four; the next row is fetched under this one
+template <typename T, int V, int kWarps, int kVec>
+__global__ void __launch_bounds__(128, V * kVec <= 16 ? kPlaces : 1) mamba_norm_grad_kernel(const MambaArgs p) {
   extern __shared__ float s_dw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = p.di / p.groups, g = blockIdx.y;
-  const int64_t n_rows = static_cast<int64_t>(p.s) * p.b;
-  const T* w = static_cast<const T*>(p.norm_w) + g * W;
-  float dw[kVec][4];
-#pragma unroll
-  for (int i = 0; i < kVec; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) dw[i][e] = 0.f;
-  for (int k = warp; k < kNormRows; k += 4) {
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * kNormRows + k;
-    if (row >= n_rows) break;
+  __shared__ float s_sum[4];
+  const int lane = kWarps == 1 ? threadIdx.x & 31 : threadIdx.x, warp = threadIdx.x >> 5, W = p.di / p.groups, g = blockIdx.y;
+  const int64_t n_rows = static_cast<int64_t>(p.s) * p.b, row_0 = static_cast<int64_t>(blockIdx.x) * p.norm_rows;
+  const int end = static_cast<int>(n_rows - row_0 < p.norm_rows ? n_rows - row_0 : p.norm_rows), first = kWarps == 1 ? warp : 0;
+  constexpr int kStep = 4 / kWarps;
+  float dw[kVec][V];
+  Raw<T, V> rw[kVec], ny[kVec], nz[kVec], ng[kVec];
+  float nr = 0.f;
+  auto ahead = [&](int k) {                        // row k of the CTA's; nothing behind its last
+    const bool valid = k < end;
+    const int64_t row = row_0 + (valid ? k : 0);
     const int t = static_cast<int>(row / p.b), b = static_cast<int>(row % p.b);
     const int64_t at_y = (static_cast<int64_t>(b) * p.s + t) * p.di + g * W, at_z = row * p.width + g * W, at_o = row * p.di + g * W;
-    const float r = p.rstd[row * p.groups + g];
-    float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int c = (i * 32 + lane) * 4;
-      if (c < W) {
-        float yv[4], zv[4], wv[4], gv[4];
-        load4(static_cast<const T*>(p.y) + at_y + c, yv);
-        load4(static_cast<const T*>(p.zx) + at_z + c, zv);
-        load4(w + c, wv);
-        load4(static_cast<const T*>(p.dout) + at_o + c, gv);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float u = yv[e] * zv[e] * sigmoidf_(zv[e]);
-          dot = fmaf(gv[e] * wv[e], u, dot);
-          dw[i][e] = fmaf(gv[e], u * r, dw[i][e]);
-        }
-      }
+      const int c = (i * 32 * kWarps + lane) * V;
+      ny[i] = fetch<T, V>(static_cast<const T*>(p.y) + at_y + c, valid && c < W);
+      nz[i] = fetch<T, V>(static_cast<const T*>(p.zx) + at_z + c, valid && c < W);
+      ng[i] = fetch<T, V>(static_cast<const T*>(p.dout) + at_o + c, valid && c < W);
     }
-    dot = warp_sum(dot) * r * r / W;
+    nr = valid ? p.rstd[row * p.groups + g] : 0.f;
+  };
+  constexpr bool kAhead = V * kVec <= 16;          // more does not fit into the registers
+  if (kAhead) ahead(first);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const int c = (i * 32 * kWarps + lane) * V;
+    rw[i] = fetch<T, V>(static_cast<const T*>(p.norm_w) + g * W + c, c < W);
+#pragma unroll
+    for (int e = 0; e < V; ++e) dw[i][e] = 0.f;
+  }
+#pragma unroll 1
+  for (int k = first; k < end; k += kStep) {
+    const int64_t row = row_0 + k;
+    const int t = static_cast<int>(row / p.b), b = static_cast<int>(row % p.b);
+    const int64_t at_y = (static_cast<int64_t>(b) * p.s + t) * p.di + g * W, at_z = row * p.width + g * W;
+    if (!kAhead) ahead(k);
+    Raw<T, V> ry[kVec], rz[kVec], rg[kVec];
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) { ry[i] = ny[i]; rz[i] = nz[i]; rg[i] = ng[i]; }
+    const float r = nr;
+    if (kAhead) ahead(k + kStep);
+    float sg[kVec][V], dot = 0.f;
 #pragma unroll
     for (int i = 0; i < kVec; ++i) {
-      const int c = (i * 32 + lane) * 4;
-      if (c < W) {
-        float yv[4], zv[4], wv[4], gv[4], dy[4], dz[4];
-        load4(static_cast<const T*>(p.y) + at_y + c, yv);
-        load4(static_cast<const T*>(p.zx) + at_z + c, zv);
-        load4(w + c, wv);
-        load4(static_cast<const T*>(p.dout) + at_o + c, gv);
+      float yv[V], zv[V], wv[V], gv[V];
+      ry[i].get(yv); rz[i].get(zv); rw[i].get(wv); rg[i].get(gv);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float sg = sigmoidf_(zv[e]), a = zv[e] * sg, du = r * fmaf(-yv[e] * a, dot, gv[e] * wv[e]);
-          dy[e] = du * a;
-          dz[e] = du * yv[e] * sg * fmaf(zv[e], 1.f - sg, 1.f);
-        }
-        store4(static_cast<T*>(p.dy) + at_y + c, dy);
-        store4(static_cast<T*>(p.dzx) + at_z + c, dz);
+      for (int e = 0; e < V; ++e) {
+        sg[i][e] = gate_sigmoid(zv[e]);
+        const float u = yv[e] * zv[e] * sg[i][e];
+        dot = fmaf(gv[e] * wv[e], u, dot);
+        dw[i][e] = fmaf(gv[e], u * r, dw[i][e]);
       }
     }
+    dot = item_sum<kWarps>(dot, s_sum) * r * r / W;
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      const int c = (i * 32 * kWarps + lane) * V;
+      float yv[V], zv[V], wv[V], gv[V], dy[V], dz[V];
+      ry[i].get(yv); rz[i].get(zv); rw[i].get(wv); rg[i].get(gv);
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const float a = zv[e] * sg[i][e], du = r * fmaf(-yv[e] * a, dot, gv[e] * wv[e]);
+        dy[e] = du * a;
+        dz[e] = du * yv[e] * sg[i][e] * fmaf(zv[e], 1.f - sg[i][e], 1.f);
+      }
+      if (c < W) {
+        put_vec(static_cast<T*>(p.dy) + at_y + c, dy);
+        put_vec(static_cast<T*>(p.dzx) + at_z + c, dz);
+      }
+    }
+  }
+  float* part = p.norm_part + (static_cast<int64_t>(blockIdx.x) * p.groups + g) * W;
+  if constexpr (kWarps > 1) {
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      const int c = (i * 32 * kWarps + lane) * V;
+#pragma unroll
+      for (int e = 0; e < V; e += 4)
+        if (c < W) *reinterpret_cast<float4*>(part + c + e) = make_float4(dw[i][e], dw[i][e + 1], dw[i][e + 2], dw[i][e + 3]);
+    }
+    return;
   }
   // the warps add up in turn
   for (int k = 0; k < 4; ++k) {
     if (warp == k) {
 #pragma unroll
       for (int i = 0; i < kVec; ++i) {
-        const int c = (i * 32 + lane) * 4;
-        if (c < W) {
-          float v[4] = {dw[i][0], dw[i][1], dw[i][2], dw[i][3]};
+        const int c = (i * 32 + lane) * V;
+#pragma unroll
+        for (int e = 0; e < V; e += 4) {
+          if (c >= W) continue;
+          float v[4] = {dw[i][e], dw[i][e + 1], dw[i][e + 2], dw[i][e + 3]};
           if (k > 0) {
             float o[4];
-            load4(s_dw + c, o);
+            load4(s_dw + c + e, o);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] += o[e];
+            for (int q = 0; q < 4; ++q) v[q] += o[q];
           }
-          store4(k < 3 ? s_dw + c : p.norm_part + (static_cast<int64_t>(blockIdx.x) * p.groups + g) * W + c, v);
+          store4(k < 3 ? s_dw + c + e : part + c + e, v);
         }
       }
     }
@@ -286,23 +427,136 @@ __global__ void __launch_bounds__(128) mamba_norm_grad_kernel(const MambaArgs p)
   }
 }
 
-template <typename T>
-void norm_grad(const MambaArgs& p, cudaStream_t s) {
-  const int W = p.di / p.groups, vec = (W / 4 + 31) / 32;
-  const dim3 grid(mamba_norm_parts(p.s, p.b), p.groups);
-  const int smem = W * 4;
-  if (vec <= 1) mamba_norm_grad_kernel<T, 1><<<grid, 128, smem, s>>>(p);
-  else if (vec <= 2) mamba_norm_grad_kernel<T, 2><<<grid, 128, smem, s>>>(p);
-  else if (vec <= 4) mamba_norm_grad_kernel<T, 4><<<grid, 128, smem, s>>>(p);
-  else if (vec <= 8) mamba_norm_grad_kernel<T, 8><<<grid, 128, smem, s>>>(p);
-  else if (vec <= 16) mamba_norm_grad_kernel<T, 16><<<grid, 128, smem, s>>>(p);
-  else mamba_norm_grad_kernel<T, 32><<<grid, 128, smem, s>>>(p);
+// ---- sums over the rows of up to four [rows, cols], in one launch.  A warp takes whole rows of 128 columns, or, where the rows are many, 16 rows of eight
+struct ColSum {
+  const float* in;
+  int rows, cols, per_cta, ctas;
+  void* out;
+  bool out_bf16;
+  int taps;            // > 0: cols are four taps of so many channels, which go to out[channel][tap], and their biases, which go to bias[channel]
+  void* bias;
+};
+struct ColSums { ColSum job[4]; int n; };
+constexpr int kSumThreads = 512;
+__device__ __forceinline__ void put_sum(void* out, bool bf16, int64_t at, float v) {
+  if (bf16) static_cast<__nv_bfloat16*>(out)[at] = __float2bfloat16_rn(v);
+  else static_cast<float*>(out)[at] = v;
+}
+__global__ void __launch_bounds__(kSumThreads) col_sums_kernel(const ColSums all) {
+  __shared__ float4 sm[kSumThreads / 32][32];
+  int at = static_cast<int>(blockIdx.x), which = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (which == i && i + 1 < all.n && at >= all.job[i].ctas) {
+      at -= all.job[i].ctas;
+      which = i + 1;
+    }
+  const ColSum& j = all.job[which];
+  const int lanes = j.per_cta / 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = at * j.per_cta + (threadIdx.x % lanes) * 4, step = kSumThreads / lanes;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (j.cols % 4 == 0 && c < j.cols) {
+    float4 part[4];                                // sums in turn, added up in pairs
+#pragma unroll
+    for (int k = 0; k < 4; ++k) part[k] = v;
+#pragma unroll 2
+    for (int r = threadIdx.x / lanes; r < j.rows; r += 4 * step) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (r + k * step >= j.rows) continue;
+        const float4 x = *reinterpret_cast<const float4*>(j.in + static_cast<int64_t>(r + k * step) * j.cols + c);
+        part[k].x += x.x; part[k].y += x.y; part[k].z += x.z; part[k].w += x.w;
+      }
+    }
+    v = make_float4((part[0].x + part[1].x) + (part[2].x + part[3].x), (part[0].y + part[1].y) + (part[2].y + part[3].y),
+                    (part[0].z + part[1].z) + (part[2].z + part[3].z), (part[0].w + part[1].w) + (part[2].w + part[3].w));
+  } else if (c < j.cols) {
+    for (int r = threadIdx.x / lanes; r < j.rows; r += step) {
+      const float* x = j.in + static_cast<int64_t>(r) * j.cols + c;
+      v.x += x[0];
+      if (c + 1 < j.cols) v.y += x[1];
+      if (c + 2 < j.cols) v.z += x[2];
+    }
+  }
+  for (int o = lanes; o < 32; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o); v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    v.z += __shfl_xor_sync(0xffffffffu, v.z, o); v.w += __shfl_xor_sync(0xffffffffu, v.w, o);
+  }
+  sm[warp][lane] = v;
+  __syncthreads();
+  const int i = threadIdx.x, col = at * j.per_cta + i;
+  if (i >= j.per_cta || col >= j.cols) return;
+  float of[kSumThreads / 32];
+#pragma unroll
+  for (int w = 0; w < kSumThreads / 32; ++w) of[w] = reinterpret_cast<const float*>(sm[w])[i];
+#pragma unroll
+  for (int o = kSumThreads / 64; o > 0; o >>= 1)
+#pragma unroll
+    for (int w = 0; w < o; ++w) of[w] += of[w + o];
+  const float t = of[0];
+  if (j.taps == 0) put_sum(j.out, j.out_bf16, col, t);
+  else if (col < 4 * j.taps) put_sum(j.out, j.out_bf16, static_cast<int64_t>(col % j.taps) * 4 + col / j.taps, t);
+  else put_sum(j.bias, j.out_bf16, col - 4 * j.taps, t);
+}
+ColSum col_sum(const float* in, int64_t rows, int cols, void* out, bool out_bf16 = false) {
+  ColSum j{in, static_cast<int>(rows), cols, rows > 512 ? 8 : 128, 0, out, out_bf16, 0, nullptr};
+  j.ctas = (cols + j.per_cta - 1) / j.per_cta;
+  return j;
+}
+void col_sums(const ColSums& all, cudaStream_t s) {
+  int ctas = 0;
+  for (int i = 0; i < all.n; ++i) ctas += all.job[i].ctas;
+  col_sums_kernel<<<ctas, kSumThreads, 0, s>>>(all);
+}
+
+// vectors of 16 bytes where all rows allow them, a warp to a row up to four vectors a lane
+template <typename T> bool whole_vectors(const MambaArgs& p) {
+  auto at_16 = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+  return (p.di / p.groups) % 8 == 0 && p.width % 8 == 0 && at_16(p.y) && at_16(p.zx) && at_16(p.out) && at_16(p.dout) && at_16(p.dy) && at_16(p.dzx);
+}
+template <bool kGrad, typename T, int V, int kWarps, int kVec>
+void launch_norm(const MambaArgs& p, cudaStream_t s) {
+  if constexpr (kGrad) {
+    const dim3 grid(mamba_norm_parts(p.s, p.b, p.norm_rows), p.groups);
+    mamba_norm_grad_kernel<T, V, kWarps, kVec><<<grid, 128, kWarps == 1 ? p.di / p.groups * 4 : 0, s>>>(p);
+  } else {
+    const int64_t n = static_cast<int64_t>(p.s) * p.b * p.groups;
+    mamba_norm_kernel<T, V, kWarps, kVec><<<static_cast<unsigned>(kWarps == 1 ? (n + 3) / 4 : n), 128, 0, s>>>(p);
+  }
+}
+template <bool kGrad, typename T, int V>
+void norm_of(const MambaArgs& p, cudaStream_t s) {
+  const int W = p.di / p.groups, lanes = (W + V - 1) / V;          // W is at most 4096
+  if (lanes <= 32) launch_norm<kGrad, T, V, 1, 1>(p, s);
+  else if (lanes <= 64) launch_norm<kGrad, T, V, 1, 2>(p, s);
+  else if (lanes <= 128) launch_norm<kGrad, T, V, 4, 1>(p, s);
+  else if (lanes <= 256) launch_norm<kGrad, T, V, 4, 2>(p, s);
+  else if (lanes <= 512) launch_norm<kGrad, T, V, 4, 4>(p, s);
+  else if constexpr (V == 4) launch_norm<kGrad, T, V, 4, 8>(p, s);
+}
+template <bool kGrad, typename T>
+void norm(const MambaArgs& p, cudaStream_t s) {
+  if constexpr (sizeof(T) == 2) {
+    if (whole_vectors<T>(p)) return norm_of<kGrad, T, 8>(p, s);
+  }
+  norm_of<kGrad, T, 4>(p, s);
 }
 
 template <typename T>
 void before_scan(const MambaArgs& p, cudaStream_t s) {
   const int64_t n = static_cast<int64_t>(p.b) * p.s * p.heads;
-  mamba_conv_kernel<T><<<dim3((p.conv / 4 + 127) / 128, (p.s + kFwdRun - 1) / kFwdRun, p.b), 128, 0, s>>>(p);
+  auto conv = [&](auto kern, int v) {
+    const int cols = (p.conv / v + 127) / 128;
+    MambaArgs q = p;
+    q.fwd_run = run_length(p.s, static_cast<int64_t>(cols) * p.b, 4, 64, 7);
+    kern<<<dim3(cols, (p.s + q.fwd_run - 1) / q.fwd_run, p.b), 128, 0, s>>>(q);
+  };
+  bool wide = false;                               // 16 bytes a thread where the rows allow it; p.conv is a multiple of eight
+  if constexpr (sizeof(T) == 2) {
+    wide = p.di % 8 == 0 && p.width % 8 == 0;
+    if (wide) conv(mamba_conv_kernel<T, 8>, 8);
+  }
+  if (!wide) conv(mamba_conv_kernel<T, 4>, 4);
   mamba_dt_kernel<T, false><<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(p);
 }
 template <typename T>
@@ -311,12 +565,6 @@ void before_scan_grad(const MambaArgs& p, cudaStream_t s) {
   mamba_conv_grad_kernel<T><<<dim3((p.conv / 4 + 127) / 128, mamba_conv_parts(p.s, p.conv_run), p.b), 128, 0, s>>>(p);
   mamba_dt_kernel<T, true><<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(p);
 }
-template <typename T>
-void norm(const MambaArgs& p, cudaStream_t s) {
-  const int64_t n = static_cast<int64_t>(p.s) * p.b * p.groups;
-  mamba_norm_kernel<T><<<static_cast<unsigned>((n + 3) / 4), 128, 0, s>>>(p);
-}
-
 }  // namespace
 
 // Steps of a backward run.  A CTA takes long for what it does (35 dependent steps), so a last wave of a few CTAs costs as much as a full one:
@@ -332,11 +580,30 @@ int mamba_conv_run(int steps, int batch, int conv, bool bf16) {
   return parts < 1 ? kBwdRun : static_cast<int>((steps + parts - 1) / parts < kBwdRun ? kBwdRun : (steps + parts - 1) / parts);
 }
 int mamba_conv_parts(int steps, int run) { return (steps + run - 1) / run; }
-int mamba_norm_parts(int steps, int batch) { return static_cast<int>((static_cast<int64_t>(steps) * batch + kNormRows - 1) / kNormRows); }
+// Rows of a CTA of the norm's gradient: they follow one another, four at a time where a warp takes a row
+int mamba_norm_rows(int steps, int batch, int groups) { return run_length(static_cast<int64_t>(steps) * batch, groups, 4, 64, 8); }
+int mamba_norm_parts(int steps, int batch, int norm_rows) { return static_cast<int>((static_cast<int64_t>(steps) * batch + norm_rows - 1) / norm_rows); }
 
 void mamba_before_scan(const MambaArgs& p, bool bf16, cudaStream_t s) { bf16 ? before_scan<__nv_bfloat16>(p, s) : before_scan<float>(p, s); }
-void mamba_before_scan_grad(const MambaArgs& p, bool bf16, cudaStream_t s) { bf16 ? before_scan_grad<__nv_bfloat16>(p, s) : before_scan_grad<float>(p, s); }
-void mamba_gated_norm(const MambaArgs& p, bool bf16, cudaStream_t s) { bf16 ? norm<__nv_bfloat16>(p, s) : norm<float>(p, s); }
-void mamba_gated_norm_grad(const MambaArgs& p, bool bf16, cudaStream_t s) { bf16 ? norm_grad<__nv_bfloat16>(p, s) : norm_grad<float>(p, s); }
+void mamba_before_scan_grad(const MambaArgs& p, bool bf16, cudaStream_t s) {
+  bf16 ? before_scan_grad<__nv_bfloat16>(p, s) : before_scan_grad<float>(p, s);
+  ColSums all{};
+  all.job[0] = col_sum(p.conv_part, static_cast<int64_t>(p.b) * mamba_conv_parts(p.s, p.conv_run), 5 * p.conv, p.dconv_w, bf16);
+  all.job[0].taps = p.conv;
+  all.job[0].bias = p.dconv_b;
+  all.job[1] = col_sum(p.ddt, static_cast<int64_t>(p.s) * p.b, p.heads, p.ddt_bias);
+  all.job[2] = col_sum(p.dA_part, static_cast<int64_t>(p.b) * p.n_chunks, p.heads, p.dA);
+  all.job[3] = col_sum(p.dD_part, static_cast<int64_t>(p.b) * p.n_chunks, p.heads, p.dD);
+  all.n = 4;
+  col_sums(all, s);
+}
+void mamba_gated_norm(const MambaArgs& p, bool bf16, cudaStream_t s) { bf16 ? norm<false, __nv_bfloat16>(p, s) : norm<false, float>(p, s); }
+void mamba_gated_norm_grad(const MambaArgs& p, bool bf16, cudaStream_t s) {
+  bf16 ? norm<true, __nv_bfloat16>(p, s) : norm<true, float>(p, s);
+  ColSums all{};
+  all.job[0] = col_sum(p.norm_part, mamba_norm_parts(p.s, p.b, p.norm_rows), p.di, p.dnorm_w, bf16);
+  all.n = 1;
+  col_sums(all, s);
+}
 
 }  // namespace b200seq

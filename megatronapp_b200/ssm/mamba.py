@@ -194,9 +194,9 @@ class _MixerCoreFn(torch.autograd.Function):
         gn = (conv_b.numel() - di) // 2
         x, B, C = _scan_views(xbc, di, gn, nh, ctx.headdim, groups)
         dy, dzx, dnorm = ext.mamba_gated_norm_grad(dout.contiguous(), rstd, y, zx, conv_w, conv_b, dt_bias, norm_w, groups)
-        dx, ddt, dA, dB, dC, dD, _ = ext.ssd_backward(dy, None, x, dt, A, B, C, D, scores, states, decay, False)
-        dconv, dbias = ext.mamba_before_scan_grad(dx, dB, dC, ddt, dzx, zx, conv_w, conv_b, dt_bias, norm_w, groups)
-        return (dzx, dconv[:4].t().reshape(conv_w.shape).to(conv_w.dtype), dconv[4].to(conv_b.dtype), dbias, dA, dD, dnorm.to(norm_w.dtype), None, None)
+        dx, ddt, dA, dB, dC, dD, _ = ext.ssd_backward(dy, None, x, dt, A, B, C, D, scores, states, decay, False, sums=False)
+        dconv_w, dconv_b, dbias, dA, dD = ext.mamba_before_scan_grad(dx, dB, dC, ddt, dA, dD, dzx, zx, conv_w, conv_b, dt_bias, norm_w, groups)
+        return dzx, dconv_w, dconv_b, dbias, dA, dD, dnorm, None, None
 
 
 def _scan_views(xbc, di, gn, nh, headdim, groups):

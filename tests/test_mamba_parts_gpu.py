@@ -1,0 +1,66 @@
+"""What stands around the Mamba-2 scan: vectors of 16 and of 8 bytes, widths of one warp and of four, runs and rows that do not fill a CTA, against 64 bits."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(got, want, dtype, terms=1):
+    # a unit of the result's type; fp32: sums of `terms` terms of either sign
+    tol = 2.0 ** -8 if dtype is torch.bfloat16 else 1e-6 + 2.0 ** -23 * terms ** 0.5
+    assert got.dtype == dtype and torch.isfinite(got).all()
+    assert float((got.double() - want).norm()) <= tol * max(float(want.norm()), 1e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("s,b,groups,w", [
+    (1, 1, 1, 64), (37, 3, 2, 256), (65, 1, 3, 264), (5, 2, 1, 512), (33, 1, 2, 520), (19, 1, 1, 1024), (7, 1, 1, 2048), (9, 1, 1, 2056), (3, 1, 2, 4096),
+    (50, 1, 2, 20), (11, 1, 2, 516), (6, 1, 2, 1028), (6, 1, 2, 2052), (700, 2, 8, 64)])
+def test_gated_norm(s, b, groups, w, dtype):
+    from megatronapp_b200.ops import seqmix
+
+    g, di, nh = torch.Generator("cuda").manual_seed(0), groups * w, 8
+    rnd = lambda *n: torch.randn(*n, generator=g, device="cuda").to(dtype)  # noqa: E731
+    conv = di + 8
+    zx, y, dout, nw, cw, cb = rnd(s, b, di + conv + nh), rnd(b, s, di), rnd(s, b, di), rnd(di), rnd(conv, 1, 4), rnd(conv)
+    args = (zx, cw, cb, torch.zeros(nh, device="cuda"), nw, groups)
+    out, rstd = seqmix.ext().mamba_gated_norm(y, *args, 1e-5)
+    dy, dzx, dw = seqmix.ext().mamba_gated_norm_grad(dout, rstd, y, *args)
+    y64, z64, w64 = (t.detach().double().requires_grad_() for t in (y, zx[..., :di], nw))
+    u = (y64.transpose(0, 1) * F.silu(z64)).reshape(s, b, groups, w)
+    want = (u * torch.rsqrt(u.pow(2).mean(-1, keepdim=True) + 1e-5)).reshape(s, b, di) * w64
+    grads = torch.autograd.grad(want, (y64, z64, w64), dout.double())
+    for got, ref, n in ((out, want.detach(), w), (dy, grads[0], w), (dzx[..., :di], grads[1], w), (dw, grads[2], s * b)):
+        _close(got, ref, dtype, n)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("s,b,di,gn,nh", [
+    (1, 1, 64, 64, 8), (3, 2, 128, 64, 8), (67, 1, 512, 128, 8), (300, 3, 64, 64, 16), (1500, 1, 1024, 512, 16),
+    (4, 1, 256, 64, 4), (40, 2, 64, 12, 4)])                       # rows of 8 bytes
+def test_convolution_and_step_sizes(s, b, di, gn, nh, dtype):
+    from megatronapp_b200.ops import seqmix
+
+    g, conv = torch.Generator("cuda").manual_seed(0), di + 2 * gn
+    rnd = lambda *n: torch.randn(*n, generator=g, device="cuda")  # noqa: E731
+    zx, cw, cb, nw, bias = rnd(s, b, di + conv + nh).to(dtype), rnd(conv, 1, 4).to(dtype), rnd(conv).to(dtype), rnd(di).to(dtype), rnd(nh)
+    ext, args = seqmix.ext(), (zx, cw, cb, bias, nw, 1)
+    xbc, dt = ext.mamba_before_scan(*args)
+    z64, w64, c64, b64 = (t.detach().double().requires_grad_() for t in (zx, cw, cb, bias))
+    x64 = z64[..., di:di + conv].permute(1, 2, 0)
+    want = F.silu(F.conv1d(x64, w64, c64, padding=3, groups=conv)[..., :s].transpose(1, 2))
+    want_dt = F.softplus(z64[..., di + conv:].transpose(0, 1) + b64)
+    _close(xbc, want.detach(), dtype, 4)
+    _close(dt, want_dt.detach(), torch.float32, 4)
+    dx, dB, dC = (rnd(b, s, n).to(dtype) for n in (di, gn, gn))
+    ddt, parts = rnd(b, s, nh), [rnd(b, 3, nh) for _ in range(2)]
+    ref = torch.autograd.grad((want, want_dt), (z64, w64, c64, b64), (torch.cat([dx, dB, dC], -1).double(), ddt.double()))
+    dzx = torch.zeros_like(zx)
+    dw, dcb, dbias, dA, dD = ext.mamba_before_scan_grad(dx, dB, dC, ddt.clone(), *parts, dzx, *args)
+    _close(dzx[..., di:], ref[0][..., di:], dtype, 4)
+    _close(dw, ref[1], dtype, s * b)
+    _close(dcb, ref[2], dtype, s * b)
+    _close(dbias, ref[3], torch.float32, s * b * 16)
+    for got, part in zip((dA, dD), parts):
+        _close(got, part.double().sum((0, 1)), torch.float32, 16 * b)
