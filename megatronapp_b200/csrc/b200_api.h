@@ -226,7 +226,7 @@ void scale_inplace(void* x, int64_t n, int dtype, float scale, const float* scal
                    cudaStream_t s);
 void cast_copy(const void* src, int src_dtype, void* dst, int dst_dtype, int64_t n, float scale,
                cudaStream_t s);
-void add_into_f32(float* dst, const void* src, int src_dtype, int64_t n, cudaStream_t s);
+void add_into_f32(float* const* dst, const void* const* src, const int64_t* n, int count, int src_dtype, cudaStream_t s);
 void check_finite(const void* x, int64_t n, int dtype, float* found_inf, cudaStream_t s);
 void chunk_mean(const void* x, float* out, int64_t rows, int cols, int pixels, bool is_bf16,
                 cudaStream_t s);

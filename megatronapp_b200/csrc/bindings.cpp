@@ -1,4 +1,5 @@
 // PyTorch bindings for the sm_100a kernels (pybind11 module megatronapp_b200._C).
+#include <torch/csrc/autograd/engine.h>
 #include <torch/extension.h>
 #include <mutex>
 #include <vector>
@@ -662,12 +663,91 @@ void cast_copy(const Tensor& src, Tensor& dst, double scale) {
   b200::cast_copy(src.data_ptr(), dtype_code(src), dst.data_ptr(), dtype_code(dst), src.numel(), static_cast<float>(scale), cur_stream());
   count();
 }
-void add_into_f32(Tensor& dst, const Tensor& src) {
-  c10::cuda::CUDAGuard guard(src.device());
-  TORCH_CHECK(src.is_contiguous() && dst.is_contiguous() && dst.scalar_type() == at::kFloat && src.numel() == dst.numel());
-  b200::add_into_f32(dst.data_ptr<float>(), src.data_ptr(), dtype_code(src), src.numel(), cur_stream());
-  count();
+// dst[i] += src[i], all on one device, no dst twice: a launch for every type of src
+void add_many_into_f32(const std::vector<Tensor>& dst, const std::vector<Tensor>& src) {
+  TORCH_CHECK(dst.size() == src.size());
+  if (src.empty()) return;
+  c10::cuda::CUDAGuard guard(src[0].device());
+  std::vector<float*> to[3];
+  std::vector<const void*> from[3];
+  std::vector<int64_t> n[3];
+  for (size_t i = 0; i < src.size(); ++i) {
+    TORCH_CHECK(src[i].is_contiguous() && dst[i].is_contiguous() && dst[i].scalar_type() == at::kFloat && src[i].numel() == dst[i].numel() &&
+                src[i].device() == src[0].device() && dst[i].device() == src[0].device());
+    const int k = dtype_code(src[i]);
+    to[k].push_back(dst[i].data_ptr<float>());
+    from[k].push_back(src[i].data_ptr());
+    n[k].push_back(src[i].numel());
+  }
+  for (int k = 0; k < 3; ++k) {
+    if (to[k].empty()) continue;
+    b200::add_into_f32(to[k].data(), from[k].data(), n[k].data(), static_cast<int>(to[k].size()), k, cur_stream());
+    count();
+  }
 }
+void add_into_f32(Tensor& dst, const Tensor& src) { add_many_into_f32({dst}, {src}); }
+
+// Gradients of biases and norms on their way into fp32 buffers: a launch for all of a backward pass instead of one for each (36 gradients of a GPT model of
+// four layers: 140 us on the device, 4.2 each with the gaps between them, and 10).
+//
+// They are added on the stream that their hooks ran on, or, at the pass's end, on the one of who called it, which by then waits for that.  Nothing outlives
+// its pass: what a pass that failed left behind is added before the next one's first, as it was when every gradient was added at once.
+struct SmallGrads : std::enable_shared_from_this<SmallGrads> {
+  static constexpr int64_t kLargest = 1 << 17;                       // elements; larger ones are no matter of launches, and are given back sooner
+  std::mutex mu;
+  std::vector<Tensor> dst, src;
+  int task = -1;
+  c10::optional<c10::cuda::CUDAStream> stream;
+
+  // false: outside of a pass, or nothing for a shared launch
+  bool take(const Tensor& to, const Tensor& grad) {
+    const int now = torch::autograd::get_current_graph_task_id();
+    if (now < 0 || grad.numel() > kLargest || !grad.is_cuda() || !grad.is_contiguous() || !to.is_contiguous() || to.scalar_type() != at::kFloat ||
+        to.numel() != grad.numel() || to.device() != grad.device())
+      return false;
+    const auto s = c10::cuda::getCurrentCUDAStream(grad.device().index());
+    std::lock_guard<std::mutex> lock(mu);
+    bool other = !src.empty() && (now != task || s != *stream);
+    for (const Tensor& t : dst) other = other || t.data_ptr() == to.data_ptr();
+    if (other) launch(*stream);
+    if (src.empty()) {
+      task = now;
+      stream = s;
+      torch::autograd::Engine::get_default_engine().queue_callback([self = shared_from_this()] { self->end_of_pass(); });
+    }
+    dst.push_back(to);
+    src.push_back(grad);
+    return true;
+  }
+  // the engine has made the caller's stream wait for those of the hooks
+  void end_of_pass() {
+    std::lock_guard<std::mutex> lock(mu);
+    if (src.empty()) return;
+    const auto s = c10::cuda::getCurrentCUDAStream(stream->device_index());
+    if (s != *stream)
+      for (const Tensor& t : src) t.record_stream(s);
+    launch(s);
+  }
+  // what is there, now, on the stream of its hooks
+  void add() {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!src.empty()) launch(*stream);
+  }
+  void forget() {
+    std::lock_guard<std::mutex> lock(mu);
+    dst.clear();
+    src.clear();
+  }
+
+ private:
+  void launch(const c10::cuda::CUDAStream& s) {
+    std::vector<Tensor> d, g;
+    d.swap(dst);
+    g.swap(src);
+    c10::cuda::CUDAStreamGuard guard(s);
+    add_many_into_f32(d, g);
+  }
+};
 void check_finite(const Tensor& x, Tensor& found) {
   c10::cuda::CUDAGuard guard(x.device());
   b200::check_finite(x.data_ptr(), x.numel(), dtype_code(x), found.data_ptr<float>(), cur_stream());
@@ -1295,6 +1375,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("scale_", &scale_);
   m.def("cast_copy", &cast_copy);
   m.def("add_into_f32", &add_into_f32);
+  m.def("add_many_into_f32", &add_many_into_f32);
+  py::class_<SmallGrads, std::shared_ptr<SmallGrads>>(m, "SmallGrads")
+      .def(py::init<>())
+      .def("take", &SmallGrads::take)
+      .def("add", &SmallGrads::add)
+      .def("forget", &SmallGrads::forget);
   m.def("check_finite", &check_finite);
   m.def("chunk_mean", &chunk_mean);
   m.def("attn_fwd", [](const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal, bool want_probs) {

@@ -315,6 +315,7 @@ class DistributedDataParallel(nn.Module):
             for p in buf.params:
                 self.param_to_buffer[p] = buf
         self._hooks = []
+        self._small = ops.ext().SmallGrads() if device.type == "cuda" else None    # see csrc/bindings.cpp
         for p, buf in self.param_to_buffer.items():
             self._hooks.append(p.register_post_accumulate_grad_hook(self._make_hook(buf)))
             p.grad_ready_hook = self._make_fused_ready(p, buf)
@@ -337,7 +338,9 @@ class DistributedDataParallel(nn.Module):
                 if getattr(param, "b200_wgrad_store_first", False) and not param.grad_added_to_main_grad:
                     param.main_grad.copy_(param.grad)      # not zeroed: see ParamAndGradBuffer.zero
                 elif param.main_grad.dtype == torch.float32 and param.grad.is_cuda and param.grad.is_contiguous():
-                    ops.ext().add_into_f32(param.main_grad, param.grad)
+                    # a bucket that may be reduced as soon as it is complete takes no gradients late
+                    if self._small is None or self.ddp_config.overlap_grad_reduce or not self._small.take(param.main_grad, param.grad):
+                        ops.ext().add_into_f32(param.main_grad, param.grad)
                 else:
                     param.main_grad.add_(param.grad.to(param.main_grad.dtype))
                 param.grad_added_to_main_grad = True
@@ -364,18 +367,26 @@ class DistributedDataParallel(nn.Module):
             self.is_last_microbatch = True
 
     def start_grad_sync(self, *unused):
+        if self._small is not None:
+            self._small.add()
         for buf in self.buffers + self.expert_parallel_buffers:
             buf.start_grad_sync(async_op=self.ddp_config.overlap_grad_reduce)
 
     def finish_grad_sync(self):
+        if self._small is not None:
+            self._small.add()
         for buf in self.buffers + self.expert_parallel_buffers:
             buf.finish_grad_sync()
 
     def scale_gradients(self, scaling_factor: float):
+        if self._small is not None:
+            self._small.add()
         for buf in self.buffers + self.expert_parallel_buffers:
             ops.scale_(buf.grad_data, scaling_factor)
 
     def zero_grad_buffer(self):
+        if self._small is not None:
+            self._small.forget()
         for buf in self.buffers + self.expert_parallel_buffers:
             buf.zero()
 

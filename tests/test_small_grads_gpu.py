@@ -1,0 +1,109 @@
+"""Gradients that a backward pass adds to the fp32 buffers in one launch: sizes around a vector and a CTA, streams, passes that fail, passes inside passes."""
+import pytest
+import torch
+import torch.nn as nn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_many_at_once(dtype):
+    from megatronapp_b200 import ops
+
+    g = torch.Generator("cuda").manual_seed(0)
+    sizes = [1, 7, 8, 9, 16383, 16384, 16385, 40000, 0] + [64 * i for i in range(1, 60)]      # more than one launch's
+    pool = torch.randn(sum(sizes) + 64 * len(sizes), generator=g, device="cuda")
+    dst, src, at = [], [], 0
+    for i, n in enumerate(sizes):
+        off = at + (i % 3 == 2)                                    # every third 4 bytes off
+        dst.append(pool[off:off + n])
+        src.append(torch.randn(n + 1, generator=g, device="cuda").to(dtype)[i % 2:i % 2 + n])
+        at += (n + 64) // 64 * 64
+    want = [d + s.float() for d, s in zip(dst, src)]
+    rest = pool.clone()
+    ops.ext().add_many_into_f32(dst, src)
+    assert all(torch.equal(d, w) for d, w in zip(dst, want))
+    for d, w in zip(dst, want):
+        d.copy_(torch.zeros_like(w))
+    mask = pool != 0
+    assert torch.equal(pool[mask], rest[mask])                     # nothing beside them
+
+
+class _Net(nn.Module):
+    def __init__(self):
+        super().__init__()
+        self.a, self.b = nn.Linear(64, 64), nn.Linear(64, 64)
+
+    def forward(self, x, fail=False, inside=False):
+        y = self.a(x).relu()
+        if fail:
+            y.register_hook(_fail)
+        if inside:
+            y = torch.utils.checkpoint.checkpoint(self.b, y, use_reentrant=True)
+        return self.b(y).square().mean()
+
+
+def _fail(_):
+    raise RuntimeError("on purpose")
+
+
+def _nets():
+    from megatronapp_b200.config.transformer_config import TransformerConfig
+    from megatronapp_b200.parallel import state as ps
+    from megatronapp_b200.parallel.ddp import DistributedDataParallel, DistributedDataParallelConfig
+
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1, 1)
+    torch.manual_seed(0)
+    net = _Net().cuda().bfloat16()
+    plain = _Net().cuda().bfloat16()
+    plain.load_state_dict(net.state_dict())
+    cfg = TransformerConfig(num_layers=1, hidden_size=64, num_attention_heads=1, params_dtype=torch.bfloat16, bf16=True)
+    return DistributedDataParallel(cfg, DistributedDataParallelConfig(grad_reduce_in_fp32=True), net), plain
+
+
+def _check(ddp, plain, times=1):
+    for (n, p), q in zip(ddp.module.named_parameters(), plain.parameters()):
+        assert p.grad is None and torch.equal(p.main_grad, times * q.grad.float()), n
+
+
+@pytest.mark.parametrize("side", [False, True])
+@pytest.mark.parametrize("inside", [False, True])
+def test_passes(side, inside):
+    ddp, plain = _nets()
+    x = torch.randn(32, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    plain(x, inside=False).backward() if not inside else plain(x, inside=True).backward()
+    ddp.zero_grad_buffer()
+    stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        loss = ddp(x, inside=inside)
+    torch.cuda.current_stream().wait_stream(stream)
+    loss.backward()
+    if inside:                                                     # the inner pass's sums were rounded apart from the outer's
+        for (n, p), q in zip(ddp.module.named_parameters(), plain.parameters()):
+            assert p.grad is None and float((p.main_grad - q.grad.float()).norm()) <= 2.0 ** -8 * float(q.grad.float().norm()), n
+    else:
+        _check(ddp, plain)
+        ddp(x).backward()                                          # the next micro-batch
+        _check(ddp, plain, 2)
+    ddp.finish_grad_sync()
+
+
+def test_a_pass_that_fails():
+    ddp, plain = _nets()
+    x = torch.randn(32, 64, device="cuda", dtype=torch.bfloat16)
+    ddp.zero_grad_buffer()
+    with pytest.raises(RuntimeError, match="on purpose"):
+        ddp(x, fail=True).backward()
+    ddp(x).backward()                                              # what came before the failure stays, as it did
+    plain(x).backward()
+    for n, p in ddp.module.named_parameters():
+        q = dict(plain.named_parameters())[n].grad.float()
+        assert torch.equal(p.main_grad, q * (2 if n.startswith("b") else 1)), n
+    ddp.zero_grad_buffer()
+    with pytest.raises(RuntimeError, match="on purpose"):
+        ddp(x, fail=True).backward()
+    ddp.zero_grad_buffer()
+    ddp(x).backward()
+    _check(ddp, plain)
