@@ -121,6 +121,14 @@ def _fp8_recipe_from_config(config, is_expert: bool = False):
                      wgrad=bool(getattr(config, "fp8_wgrad", True)))
 
 
+def _plain_linear(x, weight, bias, act, fuse_wgrad):
+    """Y = X W^T + b through the native module's node, where there is no tensor parallelism and nothing watches the operators; None elsewhere, and where the
+    kernels do not take the operands: the classes below then."""
+    if ps.get_tensor_model_parallel_world_size() > 1 or not ops._native(x) or not ops._eager():
+        return None
+    return ops.ext().linear(x, weight, bias, act, fuse_wgrad and weight.requires_grad)
+
+
 # ---------------------------------------------------------------------------
 # column parallel
 # ---------------------------------------------------------------------------
@@ -344,6 +352,9 @@ class ColumnParallelLinear(nn.Module):
                 out = gather_from_tensor_model_parallel_region(out)
             return out, (self.bias if self.skip_bias_add else None)
         bias = self.bias if not self.skip_bias_add else None
+        out = _plain_linear(input_, weight, self.bias if fused_gelu else bias, 1 if fused_gelu else 0, self.gradient_accumulation_fusion)
+        if out is not None:
+            return out, (self.bias if self.skip_bias_add and not fused_gelu else None)     # alone there is nothing to gather
         if fused_gelu:
             out = _ColumnParallelFn.apply(input_, weight, self.bias, self.sequence_parallel,
                                           self.gradient_accumulation_fusion and weight.requires_grad,
@@ -487,8 +498,10 @@ class RowParallelLinear(nn.Module):
             if not self.skip_bias_add:
                 return (out + self.bias if self.bias is not None else out), None
             return out, self.bias
-        out = _RowParallelFn.apply(input_, self.weight, self.sequence_parallel and do_reduce,
-                                   self.gradient_accumulation_fusion and self.weight.requires_grad, do_reduce)
+        out = _plain_linear(input_.contiguous(), self.weight, None, 0, self.gradient_accumulation_fusion)
+        if out is None:
+            out = _RowParallelFn.apply(input_, self.weight, self.sequence_parallel and do_reduce,
+                                       self.gradient_accumulation_fusion and self.weight.requires_grad, do_reduce)
         if not self.skip_bias_add:
             out = out + self.bias if self.bias is not None else out
             return out, None

@@ -79,3 +79,99 @@ def test_products_that_the_kernels_do_not_take():
     a, b, out = t(64, 128), t(32, 128), t(64, 32)
     before = ops.fallback_counts["gemm"]
     assert ops.gemm(a, b, out=out) is out and ops.fallback_counts["gemm"] == before
+
+
+def _linears():
+    """name -> (x, weight, bias, act)"""
+    from megatronapp_b200.parallel import state as ps
+
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1, 1)
+    g = torch.Generator("cuda").manual_seed(4)
+
+    def t(*shape, grad=True):
+        return (torch.randn(*shape, generator=g, device="cuda") * 0.1).bfloat16().requires_grad_(grad)
+
+    return {
+        "bias": (t(40, 2, 256), t(136, 256), t(136), 0), "plain": (t(300, 64), t(64, 64), None, 0), "one_row": (t(1, 128), t(8, 128), t(8), 0),
+        "gelu": (t(40, 2, 256), t(128, 256), t(128), 1), "frozen_weight": (t(40, 256), t(72, 256, grad=False), t(72), 0),
+        "frozen_input": (t(40, 256, grad=False), t(72, 256), None, 0), "frozen_bias": (t(40, 256), t(72, 256), t(72, grad=False), 0)}
+
+
+@pytest.mark.parametrize("fuse", [None, "add", "store", "unowned", "bf16"])
+@pytest.mark.parametrize("name", ["bias", "plain", "one_row", "gelu", "frozen_weight", "frozen_input", "frozen_bias"])
+def test_linear_node(name, fuse):
+    """Outputs, gradients, buffers, marks and calls of the hook: the node and the class."""
+    from megatronapp_b200 import ops
+    from megatronapp_b200.parallel import tp_layers
+
+    x, w, b, act = _linears()[name]
+    results = []
+    for native in (True, False):
+        calls = []
+        if fuse:
+            dtype = torch.bfloat16 if fuse == "bf16" else torch.float32
+            w.main_grad = torch.full(w.shape, 2.0, dtype=dtype, device="cuda")
+            w.grad_added_to_main_grad, w.b200_wgrad_store_first = fuse == "add", fuse != "unowned"
+            w.grad_ready_hook = lambda: calls.append(bool(w.grad_added_to_main_grad))
+        seen = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: (seen.append(t.shape), t)[1], lambda t: t):
+            y = ops.ext().linear(x, w, b, act, bool(fuse) and w.requires_grad) if native else \
+                tp_layers._ColumnParallelFn.apply(x, w, b, False, bool(fuse) and w.requires_grad, False, act)
+        dy = torch.randn(y.shape, generator=torch.Generator("cuda").manual_seed(5), device="cuda").to(y.dtype)
+        want = [i for i in (x, w, b) if i is not None and i.requires_grad]
+        got = [y]
+        got += torch.autograd.grad(y, want, dy, retain_graph=True, allow_unused=True)
+        got += torch.autograd.grad(y, want, dy.unsqueeze(-1).expand(*dy.shape, 2).contiguous()[..., 0], allow_unused=True)      # a strided gradient
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(y, want, dy, allow_unused=True)
+        results.append((got, seen, calls, w.main_grad.clone() if fuse else None, getattr(w, "grad_added_to_main_grad", None)))
+    (a, *ra), (c, *rc) = results
+    assert len(a) == len(c) and all((p is None and q is None) or (p.dtype == q.dtype and p.stride() == q.stride() and torch.equal(p, q)) for p, q in zip(a, c))
+    assert ra[:2] == rc[:2] and ra[3] == rc[3] and (ra[2] is None or torch.equal(ra[2], rc[2]))
+    with torch.no_grad():
+        assert ops.ext().linear(x, w, b, act, False).grad_fn is None
+
+
+def test_linear_node_leaves_the_rest_to_the_class():
+    from megatronapp_b200 import ops
+
+    t = lambda *s, **k: torch.zeros(*s, device="cuda", dtype=torch.bfloat16, **k)  # noqa: E731
+    linear = ops.ext().linear
+    assert linear(t(4, 12), t(8, 12), None, 0, False) is None and linear(t(4, 16), t(12, 16), None, 0, False) is None      # rows of no 16 bytes
+    assert linear(t(16, 4).t(), t(8, 16), None, 0, False) is None and linear(t(4, 16), t(16, 8).t(), None, 0, False) is None
+    assert linear(t(0, 16), t(8, 16), None, 0, False) is None and linear(t(4, 16).half(), t(8, 16), None, 0, False) is None
+    assert linear(t(65)[1:].view(4, 16), t(8, 16), None, 0, False) is None and linear(t(4, 16), t(8, 16), t(8).float(), 0, False) is None
+
+
+def test_what_a_hook_raises():
+    from megatronapp_b200 import ops
+
+    class Odd(Exception):
+        pass
+
+    def hook():
+        raise Odd("hook")
+
+    x, w, b, _ = _linears()["bias"]
+    w.main_grad, w.b200_wgrad_store_first, w.grad_ready_hook = torch.zeros(w.shape, device="cuda"), True, hook
+    with pytest.raises(Odd, match="hook"):
+        ops.ext().linear(x, w, b, 0, True).sum().backward()
+
+
+def test_layers_take_the_node():
+    from megatronapp_b200.config.transformer_config import TransformerConfig
+    from megatronapp_b200.parallel import state as ps
+    from megatronapp_b200.parallel.tp_layers import ColumnParallelLinear, RowParallelLinear
+
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1, 1)
+    cfg = TransformerConfig(num_layers=1, hidden_size=64, num_attention_heads=1, params_dtype=torch.bfloat16, bf16=True)
+    init = torch.nn.init.normal_
+    x = torch.randn(5, 2, 64, device="cuda").bfloat16().requires_grad_()
+    for layer in (ColumnParallelLinear(64, 128, config=cfg, init_method=init, bias=True, gather_output=False, skip_bias_add=False),
+                  RowParallelLinear(64, 128, config=cfg, init_method=init, bias=True, input_is_parallel=True, skip_bias_add=True)):
+        layer = layer.cuda()
+        assert "Fn" not in layer(x)[0].grad_fn.name()
+        with torch.autograd.forward_ad.dual_level():
+            assert layer(x)[0].grad_fn.name().endswith("FnBackward")
