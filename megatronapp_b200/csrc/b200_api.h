@@ -148,7 +148,7 @@ void layernorm_bwd(const void* dy, const void* x, const void* gamma, const float
                    cudaStream_t s);
 void layernorm_bwd_finalize(const float* dgamma_partial, const float* dbeta_partial, void* dgamma, void* dbeta, int n_partial, int cols,
                             bool is_bf16, cudaStream_t s);
-int layernorm_bwd_partials(int rows);
+int layernorm_bwd_partials(int rows, int cols);
 
 void bias_gelu_fwd(const void* x, const void* bias, void* y, int64_t rows, int cols, bool is_bf16,
                    cudaStream_t s);

@@ -441,7 +441,7 @@ std::vector<Tensor> layernorm_bwd(const Tensor& dy, const Tensor& x, const Tenso
   const int rows = static_cast<int>(x.numel() / cols);
   TORCH_CHECK(cols <= 8192, "layernorm_bwd supports cols <= 8192");
   auto dx = torch::empty_like(x);
-  const int np = b200::layernorm_bwd_partials(rows);
+  const int np = b200::layernorm_bwd_partials(rows, cols);
   auto fo = x.options().dtype(at::kFloat);
   auto pg = torch::empty({np, cols}, fo);
   auto pb = has_beta ? torch::empty({np, cols}, fo) : torch::empty({0}, fo);

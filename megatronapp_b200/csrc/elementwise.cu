@@ -9,6 +9,7 @@
 #include "b200_api.h"
 #include "common.cuh"
 
+#include <type_traits>
 #include <cooperative_groups.h>
 #include <curand_kernel.h>
 
@@ -163,260 +164,317 @@ __global__ void __launch_bounds__(kLnThreads) ln_fwd_kernel(const T* __restrict_
   }
 }
 
-// dx plus per-CTA partial column sums of dgamma/dbeta (finalised by a second tiny kernel)
-template <typename T, bool kRms>
-__global__ void __launch_bounds__(kLnThreads) ln_bwd_kernel(
-    const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
-    const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx,
-    float* __restrict__ dgamma_partial, float* __restrict__ dbeta_partial, int rows, int cols,
-    bool zero_centered) {
-  __shared__ float red[32];
-  const int nvec = cols / 8;
-  float dg_acc[kLnMaxVec][8], db_acc[kLnMaxVec][8];
-#pragma unroll
-  for (int i = 0; i < kLnMaxVec; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { dg_acc[i][j] = 0.f; db_acc[i][j] = 0.f; }
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const T* xr = x + static_cast<size_t>(row) * cols;
-    const T* dyr = dy + static_cast<size_t>(row) * cols;
-    const float mu = kRms ? 0.f : mean[row];
-    const float rs = rstd[row];
-    float xh[kLnMaxVec][8], gd[kLnMaxVec][8];
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < kLnMaxVec; ++i) {
-      const int v = threadIdx.x + i * kLnThreads;
-      if (v < nvec) {
-        float xv[8], dv[8], g[8];
-        load8(xr + v * 8, xv);
-        load8(dyr + v * 8, dv);
-        load8(gamma + v * 8, g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float gg = zero_centered ? g[j] + 1.f : g[j];
-          xh[i][j] = (xv[j] - mu) * rs;
-          gd[i][j] = gg * dv[j];
-          s1 += gd[i][j];
-          s2 += gd[i][j] * xh[i][j];
-          dg_acc[i][j] += dv[j] * xh[i][j];
-          db_acc[i][j] += dv[j];
-        }
-      }
-    }
-    if (!kRms) s1 = block_sum(s1, red);
-    s2 = block_sum(s2, red);
-    const float m1 = kRms ? 0.f : s1 / cols, m2 = s2 / cols;
-    T* dxr = dx + static_cast<size_t>(row) * cols;
-#pragma unroll
-    for (int i = 0; i < kLnMaxVec; ++i) {
-      const int v = threadIdx.x + i * kLnThreads;
-      if (v < nvec) {
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * (gd[i][j] - m1 - xh[i][j] * m2);
-        store8(dxr + v * 8, o);
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < kLnMaxVec; ++i) {
-    const int v = threadIdx.x + i * kLnThreads;
-    if (v < nvec) {
-      float* pg = dgamma_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
-      *reinterpret_cast<float4*>(pg) = make_float4(dg_acc[i][0], dg_acc[i][1], dg_acc[i][2], dg_acc[i][3]);
-      *reinterpret_cast<float4*>(pg + 4) = make_float4(dg_acc[i][4], dg_acc[i][5], dg_acc[i][6], dg_acc[i][7]);
-      if (dbeta_partial) {
-        float* pb = dbeta_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
-        *reinterpret_cast<float4*>(pb) = make_float4(db_acc[i][0], db_acc[i][1], db_acc[i][2], db_acc[i][3]);
-        *reinterpret_cast<float4*>(pb + 4) = make_float4(db_acc[i][4], db_acc[i][5], db_acc[i][6], db_acc[i][7]);
-      }
-    }
-  }
-}
-
-// ---- fast path: cols == 8 * VPT * blockDim.x; every thread owns VPT 8-element vectors of a row,
-// gamma/beta live in registers across the persistent row loop and the next row's loads are issued
-// before the reductions of the current row (more bytes in flight per SM -> closer to HBM peak)
-__device__ __forceinline__ float2 block_sum2(float a, float b, float2* red) {
+// ---- rows of up to 8192 columns, a multiple of eight, which stay in registers between their sums and the result.  Narrow rows go one to a warp, without a
+// barrier, wide ones one to a CTA of as many threads as they have vectors of eight columns (or half as many); what a lane has no column for reads as zeros.
+// us forward / backward (the backward call's second kernel and the launches included; at the copy bandwidth), with the kernels before, which had 256 threads for every
+// row whose vectors are not a multiple of 32, two barriers a sum, and three warps for a row of 768:
+//   16384 x 264    56 /  90 ->   8.5 /  19  (2.6 / 4.0)      2048 x 4096  12.5 /  21 ->  10.5 /  21  (5.1 / 7.7)
+//    4096 x 768   8.5 /  17 ->   6.2 /  15  (1.9 / 2.9)      8192 x 5120    41 /  76 ->    37 /  76  (26 / 38)
+//   16384 x 2040   80 / 159 ->    33 /  54  (20 / 31)       16384 x 8192   138 / 164 ->   108 / 163  (82 / 123)
+//    8192 x 3000   45 / 123 ->    26 /  48  (15 / 23)       16384 x 8184   131 / 432 ->   110 / 166
+// 120 drawn sizes of 16 to 16384 rows and 256 to 8192 columns, forward and backward: 0.66 of the time (geometric mean), none more than 1 us longer.
+// the CTA's sums of a and b (a warp's where kOne).  `red` is another one than the last call's: its readers are behind the barrier of the call between
+template <bool kOne>
+__device__ __forceinline__ float2 row_sum(float a, float b, float2* red) {
   a = warp_sum(a);
   b = warp_sum(b);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (l == 0) red[w] = make_float2(a, b);
-  __syncthreads();
-  float2 t = (l < nw) ? red[l] : make_float2(0.f, 0.f);
-  t.x = warp_sum(t.x);
-  t.y = warp_sum(t.y);
-  return t;
+  if constexpr (!kOne) {
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    if (lane == 0) red[threadIdx.x >> 5] = make_float2(a, b);
+    __syncthreads();
+    const float2 t = lane < warps ? red[lane] : make_float2(0.f, 0.f);
+    a = t.x;
+    b = t.y;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {              // at most 16 warps
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    a = __shfl_sync(0xffffffffu, a, 0);
+    b = __shfl_sync(0xffffffffu, b, 0);
+  }
+  return make_float2(a, b);
+}
+template <typename T>
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const float2 p0 = Cvt<T>::up(u.x), p1 = Cvt<T>::up(u.y), p2 = Cvt<T>::up(u.z), p3 = Cvt<T>::up(u.w);
+  f[0] = p0.x; f[1] = p0.y; f[2] = p1.x; f[3] = p1.y; f[4] = p2.x; f[5] = p2.y; f[6] = p3.x; f[7] = p3.y;
+}
+__device__ __forceinline__ uint4 load_vec(const void* p, int v, bool valid) { return valid ? reinterpret_cast<const uint4*>(p)[v] : make_uint4(0u, 0u, 0u, 0u); }
+
+template <typename T, bool kRms, int kWarps, int kVec>
+__global__ void __launch_bounds__(128) ln_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
+                                                                                     const T* __restrict__ beta, T* __restrict__ y, float* __restrict__ mean_out,
+                                                                                     float* __restrict__ rstd_out, int rows, int cols, float eps, bool zero_centered) {
+  __shared__ float2 red[2][4];
+  const int64_t row = kWarps == 1 ? blockIdx.x * 4ll + (threadIdx.x >> 5) : blockIdx.x;
+  if (row >= rows) return;
+  const int lane = kWarps == 1 ? threadIdx.x & 31 : threadIdx.x, nvec = cols / 8;
+  const T* xr = x + row * cols;
+  uint4 rx[kVec], rg[kVec], rb[kVec];
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) rx[i] = load_vec(xr, lane + i * 32 * kWarps, lane + i * 32 * kWarps < nvec);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const int v = lane + i * 32 * kWarps;
+    rg[i] = load_vec(gamma, v, v < nvec);
+    rb[i] = load_vec(beta, v, beta != nullptr && v < nvec);
+  }
+  float c[kVec][8], s = 0.f, mean = 0.f;
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    unpack8<T>(rx[i], c[i]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += kRms ? c[i][j] * c[i][j] : c[i][j];
+  }
+  s = row_sum<kWarps == 1>(s, 0.f, red[0]).x;
+  if (!kRms) {                                     // two passes over the registers: no E[x^2] - mean^2 cancellation
+    mean = s / cols;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < kVec; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float d = c[i][j] - mean;
+        q += lane + i * 32 * kWarps < nvec ? d * d : 0.f;
+      }
+    s = row_sum<kWarps == 1>(q, 0.f, red[1]).x;
+  }
+  const float rstd = rsqrtf(s / cols + eps);
+  if (lane == 0) {
+    if (mean_out) mean_out[row] = mean;
+    rstd_out[row] = rstd;
+  }
+  T* yr = y + row * cols;
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    const int v = lane + i * 32 * kWarps;
+    float g[8], b[8], o[8];
+    unpack8<T>(rg[i], g);
+    unpack8<T>(rb[i], b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = (c[i][j] - mean) * rstd * (zero_centered ? g[j] + 1.f : g[j]) + b[j];
+    if (v < nvec) store8(yr + v * 8, o);
+  }
 }
 
+// a CTA goes from row to row with gamma and beta in registers and the next row on its way
 template <typename T, bool kRms, int VPT>
-__global__ void __launch_bounds__(512) ln_fwd_fast_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
-                                                          const T* __restrict__ beta, T* __restrict__ y,
-                                                          float* __restrict__ mean_out, float* __restrict__ rstd_out,
-                                                          int rows, int cols, float eps, bool zero_centered) {
-  __shared__ float2 red[32];
+__global__ void __launch_bounds__(512) ln_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
+                                                          float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int cols, float eps,
+                                                          bool zero_centered) {
+  __shared__ float2 red[2][16];
+  const int nvec = cols / 8;
   float g[VPT][8], b[VPT][8];
+  uint4 next[VPT];
+  int64_t row = blockIdx.x;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * blockDim.x;
-    load8(gamma + v * 8, g[i]);
-    if (beta) load8(beta + v * 8, b[i]);
+    next[i] = load_vec(x + row * cols, v, v < nvec);
+    unpack8<T>(load_vec(gamma, v, v < nvec), g[i]);
+    unpack8<T>(load_vec(beta, v, beta != nullptr && v < nvec), b[i]);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 8; ++j)
       if (zero_centered) g[i][j] += 1.f;
-      if (!beta) b[i][j] = 0.f;
-    }
-  }
-  uint4 nxt[VPT];
-  int row = blockIdx.x;
-  if (row < rows) {
-#pragma unroll
-    for (int i = 0; i < VPT; ++i)
-      nxt[i] = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * cols + (threadIdx.x + i * blockDim.x) * 8);
   }
   const float inv_cols = 1.f / cols;
+  int odd = 0;
   for (; row < rows; row += gridDim.x) {
     float c[VPT][8];
+    const int64_t after = row + gridDim.x;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const uint4 u = nxt[i];
-      float2 p0 = Cvt<T>::up(u.x), p1 = Cvt<T>::up(u.y), p2 = Cvt<T>::up(u.z), p3 = Cvt<T>::up(u.w);
-      c[i][0] = p0.x; c[i][1] = p0.y; c[i][2] = p1.x; c[i][3] = p1.y;
-      c[i][4] = p2.x; c[i][5] = p2.y; c[i][6] = p3.x; c[i][7] = p3.y;
+      const int v = threadIdx.x + i * blockDim.x;
+      unpack8<T>(next[i], c[i]);
+      next[i] = load_vec(x + after * cols, v, after < rows && v < nvec);
     }
-    const int nrow = row + gridDim.x;
-    if (nrow < rows) {
-#pragma unroll
-      for (int i = 0; i < VPT; ++i)
-        nxt[i] = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(nrow) * cols + (threadIdx.x + i * blockDim.x) * 8);
-    }
-    float s = 0.f, q = 0.f;
+    float s = 0.f, mean = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { s += c[i][j]; q += c[i][j] * c[i][j]; }
-    float mean = 0.f, rstd;
-    if (kRms) {
-      const float2 t = block_sum2(q, 0.f, red);
-      rstd = rsqrtf(t.x * inv_cols + eps);
-    } else {
-      // two-pass variance on register-resident values (exact, no E[x^2]-mean^2 cancellation)
-      const float2 t = block_sum2(s, 0.f, red);
-      mean = t.x * inv_cols;
-      float d2 = 0.f;
+      for (int j = 0; j < 8; ++j) s += kRms ? c[i][j] * c[i][j] : c[i][j];
+    s = row_sum<false>(s, 0.f, red[odd]).x;
+    odd ^= 1;
+    if (!kRms) {                                   // two passes over the registers: no E[x^2] - mean^2 cancellation
+      mean = s * inv_cols;
+      float q = 0.f;
 #pragma unroll
       for (int i = 0; i < VPT; ++i)
+        if (threadIdx.x + i * blockDim.x < nvec) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { const float d = c[i][j] - mean; d2 += d * d; }
-      const float2 t2 = block_sum2(d2, 0.f, red);
-      rstd = rsqrtf(t2.x * inv_cols + eps);
+          for (int j = 0; j < 8; ++j) { const float d = c[i][j] - mean; q += d * d; }
+        }
+      s = row_sum<false>(q, 0.f, red[odd]).x;
+      odd ^= 1;
     }
+    const float rstd = rsqrtf(s * inv_cols + eps);
     if (threadIdx.x == 0) {
       if (mean_out) mean_out[row] = mean;
       rstd_out[row] = rstd;
     }
-    T* yr = y + static_cast<size_t>(row) * cols;
+    T* yr = y + row * cols;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
       float o[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = (c[i][j] - mean) * rstd * g[i][j] + b[i][j];
-      store8(yr + (threadIdx.x + i * blockDim.x) * 8, o);
+      if (v < nvec) store8(yr + v * 8, o);
     }
+  }
+}
+
+// ---- backward: dx, and each CTA's column sums for gamma and beta.  The next row is fetched under this one.
+template <typename T, bool kRms, int kVec>
+__global__ void __launch_bounds__(128, 4) ln_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma, const float* __restrict__ mean,
+                                                             const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dgamma_partial,
+                                                             float* __restrict__ dbeta_partial, int rows, int cols, bool zero_centered) {
+  __shared__ float s_cols[2][4][kVec * 256];       // each warp's sums for gamma, for beta
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nvec = cols / 8;
+  uint4 rg[kVec], nx[kVec], nd[kVec];
+  float dg[kVec][8], db[kVec][8], nmu = 0.f, nrs = 0.f;
+  int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + warp;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * 4;
+  auto ahead = [&](int64_t r) {
+    const bool valid = r < rows;
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      const int v = lane + i * 32;
+      nx[i] = load_vec(x + r * cols, v, valid && v < nvec);
+      nd[i] = load_vec(dy + r * cols, v, valid && v < nvec);
+    }
+    nmu = kRms || !valid ? 0.f : mean[r];
+    nrs = valid ? rstd[r] : 0.f;
+  };
+  ahead(row);
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    rg[i] = load_vec(gamma, lane + i * 32, lane + i * 32 < nvec);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dg[i][j] = db[i][j] = 0.f;
+  }
+  const float inv_cols = 1.f / cols;
+  for (; row < rows; row += stride) {
+    float xh[kVec][8], gd[kVec][8], s1 = 0.f, s2 = 0.f;
+    const float mu = nmu, rs = nrs;
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      float dv[8], g[8];
+      unpack8<T>(nx[i], xh[i]); unpack8<T>(nd[i], dv); unpack8<T>(rg[i], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {                // columns that are not there have dy = 0
+        xh[i][j] = (xh[i][j] - mu) * rs;
+        gd[i][j] = (zero_centered ? g[j] + 1.f : g[j]) * dv[j];
+        s1 += gd[i][j];
+        s2 += gd[i][j] * xh[i][j];
+        dg[i][j] += dv[j] * xh[i][j];
+        db[i][j] += dv[j];
+      }
+    }
+    ahead(row + stride);
+    const float2 t = row_sum<true>(s1, s2, nullptr);
+    const float m1 = kRms ? 0.f : t.x * inv_cols, m2 = t.y * inv_cols;
+    T* dxr = dx + row * cols;
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) {
+      const int v = lane + i * 32;
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = rs * (gd[i][j] - m1 - xh[i][j] * m2);
+      if (v < nvec) store8(dxr + v * 8, o);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kVec; ++i) {
+    float4* a = reinterpret_cast<float4*>(&s_cols[0][warp][(lane + i * 32) * 8]);
+    float4* b = reinterpret_cast<float4*>(&s_cols[1][warp][(lane + i * 32) * 8]);
+    a[0] = make_float4(dg[i][0], dg[i][1], dg[i][2], dg[i][3]);
+    a[1] = make_float4(dg[i][4], dg[i][5], dg[i][6], dg[i][7]);
+    b[0] = make_float4(db[i][0], db[i][1], db[i][2], db[i][3]);
+    b[1] = make_float4(db[i][4], db[i][5], db[i][6], db[i][7]);
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < cols; c += 128) {
+    dgamma_partial[static_cast<size_t>(blockIdx.x) * cols + c] = (s_cols[0][0][c] + s_cols[0][1][c]) + (s_cols[0][2][c] + s_cols[0][3][c]);
+    if (dbeta_partial) dbeta_partial[static_cast<size_t>(blockIdx.x) * cols + c] = (s_cols[1][0][c] + s_cols[1][1][c]) + (s_cols[1][2][c] + s_cols[1][3][c]);
   }
 }
 
 template <typename T, bool kRms, int VPT>
-__global__ void __launch_bounds__(512) ln_bwd_fast_kernel(
-    const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma, const float* __restrict__ mean,
-    const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dgamma_partial,
-    float* __restrict__ dbeta_partial, int rows, int cols, bool zero_centered) {
-  __shared__ float2 red[32];
-  float g[VPT][8], dg_acc[VPT][8], db_acc[VPT][8];
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    load8(gamma + (threadIdx.x + i * blockDim.x) * 8, g[i]);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (zero_centered) g[i][j] += 1.f;
-      dg_acc[i][j] = 0.f;
-      db_acc[i][j] = 0.f;
-    }
-  }
+__global__ void __launch_bounds__(512) ln_bwd_wide_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma, const float* __restrict__ mean,
+                                                          const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dgamma_partial,
+                                                          float* __restrict__ dbeta_partial, int rows, int cols, bool zero_centered) {
+  __shared__ float2 red[2][16];
+  const int nvec = cols / 8;
+  float g[VPT][8], dg[VPT][8], db[VPT][8], nmu = 0.f, nrs = 0.f;
   uint4 nx[VPT], nd[VPT];
-  float nmu = 0.f, nrs = 0.f;
-  int row = blockIdx.x;
-  auto prefetch = [&](int r) {
+  int64_t row = blockIdx.x;
+  auto ahead = [&](int64_t r) {
+    const bool valid = r < rows;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const size_t off = static_cast<size_t>(r) * cols + (threadIdx.x + i * blockDim.x) * 8;
-      nx[i] = *reinterpret_cast<const uint4*>(x + off);
-      nd[i] = *reinterpret_cast<const uint4*>(dy + off);
+      const int v = threadIdx.x + i * blockDim.x;
+      nx[i] = load_vec(x + r * cols, v, valid && v < nvec);
+      nd[i] = load_vec(dy + r * cols, v, valid && v < nvec);
     }
-    nmu = kRms ? 0.f : mean[r];
-    nrs = rstd[r];
+    nmu = kRms || !valid ? 0.f : mean[r];
+    nrs = valid ? rstd[r] : 0.f;
   };
-  if (row < rows) prefetch(row);
-  const float inv_cols = 1.f / cols;
-  for (; row < rows; row += gridDim.x) {
-    float xh[VPT][8], gd[VPT][8];
-    const float mu = nmu, rs = nrs;
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const uint4 ux = nx[i], ud = nd[i];
-      const float2 x0 = Cvt<T>::up(ux.x), x1 = Cvt<T>::up(ux.y), x2 = Cvt<T>::up(ux.z), x3 = Cvt<T>::up(ux.w);
-      const float2 d0 = Cvt<T>::up(ud.x), d1 = Cvt<T>::up(ud.y), d2 = Cvt<T>::up(ud.z), d3 = Cvt<T>::up(ud.w);
-      const float xv[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
-      const float dv[8] = {d0.x, d0.y, d1.x, d1.y, d2.x, d2.y, d3.x, d3.y};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        xh[i][j] = (xv[j] - mu) * rs;
-        gd[i][j] = g[i][j] * dv[j];
-        s1 += gd[i][j];
-        s2 += gd[i][j] * xh[i][j];
-        dg_acc[i][j] += dv[j] * xh[i][j];
-        db_acc[i][j] += dv[j];
-      }
-    }
-    const int nrow = row + gridDim.x;
-    if (nrow < rows) prefetch(nrow);
-    const float2 t = block_sum2(s1, s2, red);
-    const float m1 = kRms ? 0.f : t.x * inv_cols, m2 = t.y * inv_cols;
-    T* dxr = dx + static_cast<size_t>(row) * cols;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      float o[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = rs * (gd[i][j] - m1 - xh[i][j] * m2);
-      store8(dxr + (threadIdx.x + i * blockDim.x) * 8, o);
-    }
-  }
+  ahead(row);
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int v = threadIdx.x + i * blockDim.x;
-    float* pg = dgamma_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
-    *reinterpret_cast<float4*>(pg) = make_float4(dg_acc[i][0], dg_acc[i][1], dg_acc[i][2], dg_acc[i][3]);
-    *reinterpret_cast<float4*>(pg + 4) = make_float4(dg_acc[i][4], dg_acc[i][5], dg_acc[i][6], dg_acc[i][7]);
-    if (dbeta_partial) {
-      float* pb = dbeta_partial + static_cast<size_t>(blockIdx.x) * cols + v * 8;
-      *reinterpret_cast<float4*>(pb) = make_float4(db_acc[i][0], db_acc[i][1], db_acc[i][2], db_acc[i][3]);
-      *reinterpret_cast<float4*>(pb + 4) = make_float4(db_acc[i][4], db_acc[i][5], db_acc[i][6], db_acc[i][7]);
+    unpack8<T>(load_vec(gamma, v, v < nvec), g[i]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (zero_centered) g[i][j] += 1.f;
+      dg[i][j] = db[i][j] = 0.f;
     }
   }
-}
-
-// vectors-per-thread / block size for the fast path; vpt = 0 -> generic kernels
-static inline void ln_fast_shape(int cols, int& vpt, int& threads) {
-  vpt = 0; threads = 0;
-  if (cols % 8) return;
-  const int nvec = cols / 8;
-  for (int v : {1, 2, 4}) {
-    if (nvec % v == 0) {
-      const int t = nvec / v;
-      if (t <= 512 && t % 32 == 0) { vpt = v; threads = t; return; }
+  const float inv_cols = 1.f / cols;
+  int odd = 0;
+  for (; row < rows; row += gridDim.x, odd ^= 1) {
+    float xh[VPT][8], gd[VPT][8], s1 = 0.f, s2 = 0.f;
+    const float mu = nmu, rs = nrs;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      float dv[8];
+      unpack8<T>(nx[i], xh[i]); unpack8<T>(nd[i], dv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {                // columns that are not there have dy = 0
+        xh[i][j] = (xh[i][j] - mu) * rs;
+        gd[i][j] = g[i][j] * dv[j];
+        s1 += gd[i][j];
+        s2 += gd[i][j] * xh[i][j];
+        dg[i][j] += dv[j] * xh[i][j];
+        db[i][j] += dv[j];
+      }
+    }
+    ahead(row + gridDim.x);
+    const float2 t = row_sum<false>(s1, s2, red[odd]);
+    const float m1 = kRms ? 0.f : t.x * inv_cols, m2 = t.y * inv_cols;
+    T* dxr = dx + row * cols;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int v = threadIdx.x + i * blockDim.x;
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = rs * (gd[i][j] - m1 - xh[i][j] * m2);
+      if (v < nvec) store8(dxr + v * 8, o);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = (threadIdx.x + i * blockDim.x) * 8;
+    if (c >= cols) continue;
+    float* pg = dgamma_partial + static_cast<size_t>(blockIdx.x) * cols + c;
+    *reinterpret_cast<float4*>(pg) = make_float4(dg[i][0], dg[i][1], dg[i][2], dg[i][3]);
+    *reinterpret_cast<float4*>(pg + 4) = make_float4(dg[i][4], dg[i][5], dg[i][6], dg[i][7]);
+    if (dbeta_partial) {
+      float* pb = dbeta_partial + static_cast<size_t>(blockIdx.x) * cols + c;
+      *reinterpret_cast<float4*>(pb) = make_float4(db[i][0], db[i][1], db[i][2], db[i][3]);
+      *reinterpret_cast<float4*>(pb + 4) = make_float4(db[i][4], db[i][5], db[i][6], db[i][7]);
     }
   }
 }
@@ -965,26 +1023,50 @@ inline int grid_for(int64_t work_items, int threads, int max_ctas = 148 * 8) {
 
 }  // namespace
 
-int layernorm_bwd_partials(int rows) { return rows < 296 ? rows : 296; }
+template <typename F> struct first_arg;
+template <typename R, typename A, typename... B> struct first_arg<R (*)(A, B...)> { using type = std::remove_const_t<A>; };
+constexpr int kNarrowBwd = 512, kBwdPerSm = 4;
+// threads of a CTA that takes wide rows, and vectors of each thread: one up to 4096 columns
+static void wide_shape(int cols, int& vpt, int& threads) {
+  const int nvec = (cols + 7) / 8;
+  vpt = nvec <= 512 ? 1 : 2;
+  threads = (nvec + vpt * 32 - 1) / (vpt * 32) * 32;
+}
+static bool narrow_bwd(int cols) { return cols <= kNarrowBwd; }
+// CTAs of the backward kernel, each with a row of partial sums: as many as SMs hold, up to four each
+int layernorm_bwd_partials(int rows, int cols) {
+  if (narrow_bwd(cols)) return (rows + 3) / 4 < 4 * 148 ? (rows + 3) / 4 : 4 * 148;
+  int vpt, threads;
+  wide_shape(cols, vpt, threads);
+  const int fit = (vpt == 1 ? 1024 : 512) / threads, per_sm = fit < 1 ? 1 : (fit > kBwdPerSm ? kBwdPerSm : fit);
+  return rows < 148 * per_sm ? rows : 148 * per_sm;
+}
 
 void layernorm_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean,
                    float* rstd, int rows, int cols, float eps, bool rms, bool zero_centered,
                    bool is_bf16, cudaStream_t s) {
-  int vpt, threads;
-  ln_fast_shape(cols, vpt, threads);
-  if (vpt) {
-    // enough CTAs to fill every SM to its register/thread limit; rows are grid-strided
-    const int per_sm = 2048 / threads > 4 ? 4 : (2048 / threads < 1 ? 1 : 2048 / threads);
-    const int grid = rows < 148 * per_sm ? rows : 148 * per_sm;
-#define LN_FWD_FAST(V)                                                                                     \
-    DISPATCH_16(is_bf16, {                                                                                 \
-      if (rms) ln_fwd_fast_kernel<T, true, V><<<grid, threads, 0, s>>>((const T*)x, (const T*)gamma,      \
-               (const T*)beta, (T*)y, mean, rstd, rows, cols, eps, zero_centered);                        \
-      else ln_fwd_fast_kernel<T, false, V><<<grid, threads, 0, s>>>((const T*)x, (const T*)gamma,         \
-               (const T*)beta, (T*)y, mean, rstd, rows, cols, eps, zero_centered);                        \
-    })
-    if (vpt == 1) { LN_FWD_FAST(1); } else if (vpt == 2) { LN_FWD_FAST(2); } else { LN_FWD_FAST(4); }
-#undef LN_FWD_FAST
+  auto launch = [&](auto kern, unsigned grid, int threads) {
+    using P = typename first_arg<decltype(kern)>::type;
+    kern<<<grid, threads, 0, s>>>((P)x, (P)gamma, (P)beta, (std::remove_const_t<std::remove_pointer_t<P>>*)y, mean, rstd, rows, cols, eps, zero_centered);
+  };
+  if (cols % 8 == 0 && cols <= 8192) {
+    const int nvec = cols / 8;
+#define LN_ROWS(W, V) launch(rms ? ln_fwd_rows_kernel<T, true, W, V> : ln_fwd_rows_kernel<T, false, W, V>, W == 1 ? (rows + 3) / 4 : rows, 128)
+#define LN_WIDE(V) launch(rms ? ln_fwd_wide_kernel<T, true, V> : ln_fwd_wide_kernel<T, false, V>, grid, threads)
+    int vpt, threads;
+    wide_shape(cols, vpt, threads);
+    const int fit = (vpt == 1 ? 1344 : 1024) / threads, grid = rows < 148 * fit ? rows : 148 * fit;      // by their registers, 48 and 64 a thread
+    DISPATCH_16(is_bf16, {
+      if (nvec <= 32) LN_ROWS(1, 1);
+      else if (nvec <= 64) LN_ROWS(1, 2);
+      else if (nvec <= 96) LN_ROWS(1, 3);
+      else if (nvec <= 128) LN_ROWS(1, 4);
+      else if (nvec <= 256) LN_ROWS(4, 2);
+      else if (vpt == 1) LN_WIDE(1);
+      else LN_WIDE(2);
+    });
+#undef LN_ROWS
+#undef LN_WIDE
     return;
   }
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
@@ -1002,31 +1084,18 @@ void layernorm_bwd(const void* dy, const void* x, const void* gamma, const float
                    const float* rstd, void* dx, float* dgamma_partial, float* dbeta_partial,
                    int rows, int cols, bool rms, bool zero_centered, bool is_bf16, int n_partial,
                    cudaStream_t s) {
+  auto launch = [&](auto kern, int threads) {
+    using P = typename first_arg<decltype(kern)>::type;
+    kern<<<n_partial, threads, 0, s>>>((P)dy, (P)x, (P)gamma, mean, rstd, (std::remove_const_t<std::remove_pointer_t<P>>*)dx, dgamma_partial, dbeta_partial, rows,
+                                       cols, zero_centered);
+  };
   int vpt, threads;
-  ln_fast_shape(cols, vpt, threads);
-  if (vpt == 1 || vpt == 2) {   // 4 vectors per thread would spill under the 512-thread register cap
-#define LN_BWD_FAST(V)                                                                                     \
-    DISPATCH_16(is_bf16, {                                                                                 \
-      if (rms) ln_bwd_fast_kernel<T, true, V><<<n_partial, threads, 0, s>>>((const T*)dy, (const T*)x,    \
-               (const T*)gamma, mean, rstd, (T*)dx, dgamma_partial, dbeta_partial, rows, cols,            \
-               zero_centered);                                                                            \
-      else ln_bwd_fast_kernel<T, false, V><<<n_partial, threads, 0, s>>>((const T*)dy, (const T*)x,       \
-               (const T*)gamma, mean, rstd, (T*)dx, dgamma_partial, dbeta_partial, rows, cols,            \
-               zero_centered);                                                                            \
-    })
-    if (vpt == 1) { LN_BWD_FAST(1); } else { LN_BWD_FAST(2); }
-#undef LN_BWD_FAST
-    return;
-  }
+  wide_shape(cols, vpt, threads);
   DISPATCH_16(is_bf16, {
-    if (rms)
-      ln_bwd_kernel<T, true><<<n_partial, kLnThreads, 0, s>>>((const T*)dy, (const T*)x, (const T*)gamma,
-                                                              mean, rstd, (T*)dx, dgamma_partial,
-                                                              dbeta_partial, rows, cols, zero_centered);
-    else
-      ln_bwd_kernel<T, false><<<n_partial, kLnThreads, 0, s>>>((const T*)dy, (const T*)x, (const T*)gamma,
-                                                               mean, rstd, (T*)dx, dgamma_partial,
-                                                               dbeta_partial, rows, cols, zero_centered);
+    if (narrow_bwd(cols) && cols <= 256) launch(rms ? ln_bwd_rows_kernel<T, true, 1> : ln_bwd_rows_kernel<T, false, 1>, 128);
+    else if (narrow_bwd(cols)) launch(rms ? ln_bwd_rows_kernel<T, true, 2> : ln_bwd_rows_kernel<T, false, 2>, 128);
+    else if (vpt == 1) launch(rms ? ln_bwd_wide_kernel<T, true, 1> : ln_bwd_wide_kernel<T, false, 1>, threads);
+    else launch(rms ? ln_bwd_wide_kernel<T, true, 2> : ln_bwd_wide_kernel<T, false, 2>, threads);
   });
 }
 
