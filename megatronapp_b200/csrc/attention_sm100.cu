@@ -1,5 +1,5 @@
 // Flash attention for sm_100a: tcgen05 MMAs with S / O accumulators in TMEM, TMA-fed K/V ring,
-// two 128-row query tiles per CTA processed ping-pong by two pairs of softmax warpgroups.
+// two 128-row query tiles per CTA processed ping-pong by two softmax warpgroups.
 //
 // Forward  (attn_fwd_kernel):  S = Q K^T -> online softmax (exp2 domain, lazy rescale) ->
 //                              P (16-bit, TMEM columns of its own) -> O += P V (O stays in TMEM).
@@ -103,6 +103,22 @@ __device__ __forceinline__ bool wait_bar_warp(uint64_t* bar, uint32_t parity, vo
   return false;
 }
 
+// A look ahead at a barrier, whose answer is wanted some instructions later
+__device__ __forceinline__ uint32_t mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // One arrival for a warp: 32 of them on one word are carried out one after another
 __device__ __forceinline__ void warp_arrive(uint64_t* bar) {
   __syncwarp();
@@ -113,6 +129,9 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar) {
 // warpgroups take 104 and leave 64 to the first.
 constexpr int kThreads = 640, kMathRegs = 104, kIssueRegs = 64;
 static_assert(512 * kMathRegs + 128 * kIssueRegs <= kThreads * 96, "the shares come out of what the CTA was launched with");
+// The forward's two math warpgroups have a thread to a row of scores: 384 threads start with 168 registers each.
+constexpr int kFwdThreads = 384, kFwdMathRegs = 208, kFwdIssueRegs = 80;
+static_assert(256 * kFwdMathRegs + 128 * kFwdIssueRegs <= kFwdThreads * 168, "the shares come out of what the CTA was launched with");
 template <int N> __device__ __forceinline__ void regs_take() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_give() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
@@ -130,10 +149,10 @@ __device__ __forceinline__ void store_row32(uint8_t* dst, const uint32_t (&v)[32
   }
 }
 // after a wait that ran out, by the math warps: NaN (in either type) in `rows` rows of D columns
-template <int D>
+template <int D, int kN = kThreads>
 __device__ __forceinline__ void fill_nan(void* out, int64_t base, int64_t stride, int rows) {
   constexpr int kChunks = D / 8;
-  for (int i = threadIdx.x - 128; i < rows * kChunks; i += kThreads - 128)
+  for (int i = threadIdx.x - 128; i < rows * kChunks; i += kN - 128)
     *reinterpret_cast<uint4*>(static_cast<uint16_t*>(out) + base + i / kChunks * stride + i % kChunks * 8) =
         make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
 }
@@ -160,22 +179,24 @@ struct FwdSmem {
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + 2 * kTile;
   static constexpr int kVOff = kKOff + kStages * kTile;
-  static constexpr int kExOff = kVOff + kStages * kTile;          // [parity][tile][half][row] partial maxima, then sums
-  static constexpr int kBarOff = kExOff + 2 * 2 * 2 * kBlockQ * 4;
+  static constexpr int kBarOff = kVOff + kStages * kTile;
   static constexpr int kTotal = kBarOff + 256 + 1024;   // + barriers + alignment slack
 };
 
 // ------------------------------------------------------------------------------------ forward
 // P (16-bit) goes to TMEM columns of its own and feeds the PV product as the TMEM A operand.  Two query tiles alternate between the tensor
-// core (1024 cycles a key block at D = 128) and the softmax (1024 cycles of exponentials at one block's rate).  Two warpgroups share a
-// tile, 64 columns of each row apiece: S is read once into registers, the halves exchange their row maxima through shared memory, and
-// each packs its P into its own 32 columns.  S's columns are free again as soon as they are in registers, so the next S (the other
-// tile's where there is one buffer, this tile's where there are two) is made under this one's exponentials: a warpgroup that has handed
-// over its P finds its next S waiting.  Two warps issue: a wait that is already over costs 65 to 120 cycles, the tensor core's queue holds four
+// core (1024 cycles a key block at D = 128) and the softmax (1024 cycles of exponentials at one block's rate).  A thread has a row of 128 scores, read once
+// into registers: with 208 of them its exponentials follow one another at the unit's rate for two warps, where two threads to a row with 104 each took twice as long
+// for theirs and had maxima and sums to exchange (cycles from scores to weights, 2900 there and 2300 here).  S's columns are free again as soon as they are in
+// registers, so the next S (the other tile's where there is one buffer, this tile's where there are two) is made under this one's exponentials.
+// A look at a barrier takes 130 cycles with the steps around it even if it is open, so the answer is fetched ahead of its use where it is most likely yes
+// (D = 64: the next S, the product that frees P's columns; at D = 128 there the scores of the other tile come first, and it cost 1 to 10 %).
+// Two warps issue: a wait that is already over costs 65 to 120 cycles, the tensor core's queue holds four
 // MMAs (256 cycles), and one warp that goes through all waits in turn leaves it empty (174 us where two take 139).
-// 32 / 8 heads x 4096 x 128 causal: 145 us with P over S and S after its PV, 131 so; 32 heads x 8192: 479 -> 435 us.
+// us, two threads to a row / one: 32 heads x 8192 x 64 causal 404 / 367, 32 x 3 x 1337 x 64 65 / 61, 32 / 8 x 4096 x 128 130 / 126, x 512 16.5 / 14.5.
+// CTAs that go on to further blocks of the grid (clusterlaunchcontrol), and tiles that take turns at the exponentials, gave nothing or cost time.
 template <int D, bool kBf16>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
   using L = FwdSmem<D>;
@@ -185,7 +206,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint8_t* sQ = smem + L::kQOff;
   uint8_t* sK = smem + L::kKOff;
   uint8_t* sV = smem + L::kVOff;
-  float* sEx = reinterpret_cast<float*>(smem + L::kExOff);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
   uint64_t* q_full = bars;            // 1
   uint64_t* k_full = bars + 1;        // 2
@@ -222,8 +242,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&s_read[i], 8);
-      mbar_init(&p_ready[i], 8); mbar_init(&pv_done[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&s_read[i], 4);
+      mbar_init(&p_ready[i], 4); mbar_init(&pv_done[i], 1);
     }
     mbar_init(drained, 2);
     for (int i = 0; i < 4; ++i) mbar_init(&s_issued[i], 1);
@@ -244,7 +264,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   static_assert(2 * D + 128 + kSBufs * 128 <= 512, "TMEM columns");
 
   if (warp_idx < 4) {
-    regs_give<kIssueRegs>();
+    regs_give<kFwdIssueRegs>();
     if (warp_idx == 0 && lane == 0) {
       // ============================================================ TMA producer
       const int ntiles = (nkv_1 > 0) ? 2 : 1;
@@ -339,58 +359,60 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
   } else {
     // ============================================================ softmax / correction / epilogue
-    regs_take<kMathRegs>();
-    const int t = (warp_idx - 4) >> 3;            // q tile of this warpgroup
-    const int half = ((warp_idx - 4) >> 2) & 1;   // its columns of S: 64 half .. 64 half + 63, and of O: D / 2 likewise
+    regs_take<kFwdMathRegs>();
+    const int t = (warp_idx - 4) >> 2;            // q tile of this warpgroup
     const int quad = warp_idx & 3;                // TMEM lane quadrant
     const int r = quad * 32 + lane;               // row inside the tile
     const int q0 = t == 0 ? q0_0 : q0_1;
     const int qrow = q0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tS = tmem_S + (kSBufs == 2 ? t * 128 : 0) + half * 64 + lane_addr;
-    const uint32_t tP = tmem_P + t * 64 + half * 32 + lane_addr;
-    const uint32_t tO = tmem_O + t * D + half * (D / 2) + lane_addr;
-    float* ex = sEx + t * (2 * kBlockQ);          // + parity * 4 kBlockQ + half * kBlockQ + row
+    const uint32_t tS = tmem_S + (kSBufs == 2 ? t * 128 : 0) + lane_addr;
+    const uint32_t tP = tmem_P + t * 64 + lane_addr;
+    const uint32_t tO = tmem_O + t * D + lane_addr;
     float m = -INFINITY;                          // running max (exp2 domain, already scaled)
-    uint64_t l2 = 0;                              // running sum of this half's even and odd columns
+    uint64_t l2[2] = {0, 0};                      // running sums of the even and odd columns of both halves
     const int n = t == 0 ? nkv_0 : nkv_1;
     const float sc = p.scale_log2;
     const uint64_t sc2 = f2(sc, sc);
 
+    uint32_t next_there = 0;                      // the next block's scores have been made
     auto block = [&](int j, auto masked_tag) {
       constexpr bool kMasked = decltype(masked_tag)::value;
-      const int limit = (kMasked ? min(p.sk, p.causal ? qrow + 1 : p.sk) : 0) - j * kBlockKV - half * 64;   // valid: col < limit
-      uint32_t v[2][32];
-      tmem_ld_32x32(tS, v[0]);
-      tmem_ld_32x32(tS + 32, v[1]);
+      const int limit = (kMasked ? min(p.sk, p.causal ? qrow + 1 : p.sk) : 0) - j * kBlockKV;   // valid: col < limit
+      uint32_t v[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(tS + c * 32, v[c]);
       tmem_ld_wait();
       tc_fence_before();
       warp_arrive(&s_read[t]);
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      float mx[8];
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+      for (int i = 0; i < 8; ++i) mx[i] = -INFINITY;
+      // the product before, after which P's columns are free: most likely over by now
+      const uint32_t free_now = j == 0 ? 1u : kSBufs == 1 ? 0u : mbar_test(&pv_done[t], (j - 1) & 1);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
           if (kMasked && c * 32 + i >= limit) v[c][i] = 0xff800000u;   // -inf
-          mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[c][i]));
+          if (kMasked && c * 32 + i + 1 >= limit) v[c][i + 1] = 0xff800000u;
+          mx[(i >> 1) & 7] = max3(mx[(i >> 1) & 7], __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
         }
-      const float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-      float* slot = ex + (j & 1) * (4 * kBlockQ);
-      slot[half * kBlockQ + r] = mine;
-      named_bar_sync(1 + t * 4 + quad, 64);          // the two warps of these rows
-      float m_new = fmaxf(m, fmaxf(mine, slot[(half ^ 1) * kBlockQ + r]) * sc);   // softmax scale is positive
+      const float mine = max3(max3(mx[0], mx[1], mx[2]), max3(mx[3], mx[4], mx[5]), fmaxf(mx[6], mx[7]));
+      float m_new = fmaxf(m, mine * sc);           // softmax scale is positive
       if (m_new == -INFINITY) m_new = 0.f;         // fully masked so far: keep everything finite
       const bool grow = (m_new - m) > kRescaleThreshold;   // also true on the first block (m = -inf)
       if (__any_sync(0xffffffffu, grow)) {
         const float m_cur = grow ? m_new : m;
         const float alpha = grow ? fast_exp2(m - m_cur) : 1.f;
         m = m_cur;
-        l2 = mul2(l2, f2(alpha, alpha));
+        l2[0] = mul2(l2[0], f2(alpha, alpha));
+        l2[1] = mul2(l2[1], f2(alpha, alpha));
         if (j > 0) {
           wait_bar_warp(&pv_done[t], (j - 1) & 1, failed, p.wait_limit);
           tc_fence_after();
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {     // in small pieces: the scores are in registers
+          for (int c = 0; c < D / 16; ++c) {     // in small pieces: the scores are in registers
             uint32_t o[16];
             tmem_ld_32x16(tO + c * 16, o);
             tmem_ld_wait();
@@ -402,7 +424,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       const uint64_t nm2 = f2(-m, -m);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t pk[16];
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
@@ -410,24 +432,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           un2(fma2(f2(__uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1])), sc2, nm2), p0, p1);
           p0 = fast_exp2(p0);
           p1 = fast_exp2(p1);
-          l2 = add2(l2, f2(p0, p1));
+          l2[c >> 1] = add2(l2[c >> 1], f2(p0, p1));
           pk[i >> 1] = pack16<kBf16>(p0, p1);
         }
         if (c == 0 && j > 0) {                     // P's columns are free, after the product before
-          wait_bar_warp(&pv_done[t], (j - 1) & 1, failed, p.wait_limit);
+          if (!__all_sync(0xffffffffu, free_now)) wait_bar_warp(&pv_done[t], (j - 1) & 1, failed, p.wait_limit);
           tc_fence_after();
         }
         tmem_st_32x16(tP + c * 16, pk);
       }
+      if (kSBufs == 2) next_there = mbar_test(&s_full[t], (j + 1) & 1);
       tmem_st_wait();
       tc_fence_before();
       warp_arrive(&p_ready[t]);
     };
 
-    // a wait that runs out is noted, not acted on: the halves' warpgroups go on to their exchanges together, and every later wait ends at once
+    // a wait that runs out is noted, not acted on: every later wait ends at once
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      wait_bar_warp(&s_full[t], j & 1, failed, p.wait_limit);
+      if (!__all_sync(0xffffffffu, next_there)) wait_bar_warp(&s_full[t], j & 1, failed, p.wait_limit);
       tc_fence_after();
       const int kbase = j * kBlockKV;
       // diagonal block of a causal tile, or the ragged tail of the key sequence
@@ -438,25 +461,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (n > 0) {
       ok = wait_bar_warp(&pv_done[t], (n - 1) & 1, failed, p.wait_limit);
       tc_fence_after();
-      float la, lb;
-      un2(l2, la, lb);
-      float* slot = ex + (n & 1) * (4 * kBlockQ);
-      slot[half * kBlockQ + r] = la + lb;
-      named_bar_sync(1 + t * 4 + quad, 64);          // the two warps of these rows
-      const float l = slot[r] + slot[kBlockQ + r];
+      float la, lb, lc, ld;
+      un2(l2[0], la, lb);
+      un2(l2[1], lc, ld);
+      const float l = (la + lb) + (lc + ld);
       const float inv_l = l > 0.f ? 1.f / l : 0.f;
       const bool valid = qrow < p.sq && ok;
       uint8_t* orow = reinterpret_cast<uint8_t*>(p.o) +
                       (static_cast<int64_t>(qrow) * p.o_ss + static_cast<int64_t>(bi) * p.o_sb +
-                       static_cast<int64_t>(h) * p.o_sh + half * (D / 2)) * 2;
+                       static_cast<int64_t>(h) * p.o_sh) * 2;
 #pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
+      for (int c = 0; c < D / 32; ++c) {
         uint32_t v[32];
         tmem_ld_32x32(tO + c * 32, v);
         tmem_ld_wait();
         if (valid) store_row32<kBf16>(orow + c * 64, v, inv_l);
       }
-      if (valid && half == 0)
+      if (valid)
         p.lse[(static_cast<int64_t>(bi) * p.hq + h) * p.sq + qrow] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
     }
   }
@@ -475,8 +496,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       wait_bar_warp(drained, 0, &never);
     } else if (warp_idx >= 4) {
       const int rows = min(2 * kBlockQ, p.sq - q0_0);
-      fill_nan<D>(p.o, static_cast<int64_t>(q0_0) * p.o_ss + static_cast<int64_t>(bi) * p.o_sb + static_cast<int64_t>(h) * p.o_sh, p.o_ss, rows);
-      for (int i = threadIdx.x - 128; i < rows; i += kThreads - 128)
+      fill_nan<D, kFwdThreads>(p.o, static_cast<int64_t>(q0_0) * p.o_ss + static_cast<int64_t>(bi) * p.o_sb + static_cast<int64_t>(h) * p.o_sh, p.o_ss, rows);
+      for (int i = threadIdx.x - 128; i < rows; i += kFwdThreads - 128)
         p.lse[(static_cast<int64_t>(bi) * p.hq + h) * p.sq + q0_0 + i] = __int_as_float(0x7fffffff);
     }
     __syncthreads();
@@ -922,11 +943,11 @@ bool make_tmap_bhsd(CUtensorMap* map, const void* base, bool is_bf16, int d, int
 
 // once per kernel: its shared memory, and that its register shares (regs_take / regs_give) fit what it is launched with
 template <typename K>
-bool prepare_kernel(K kern, int smem, const char* name) {
+bool prepare_kernel(K kern, int smem, const char* name, int threads, int shares) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) { g_attn_err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return false; }
   cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs * kThreads < 512 * kMathRegs + 128 * kIssueRegs) {
+  if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess || fa.numRegs * threads < shares) {
     g_attn_err = std::string(name) + ": built with too few registers for its warpgroups' shares";
     return false;
   }
@@ -945,7 +966,7 @@ int launch_fwd(const AttnArgs& a, cudaStream_t s) {
   if (!make_tmap_bhsd(&tk, a.k, a.is_bf16, D, a.hkv, a.b, a.sk, a.k_sh, a.k_sb, a.k_ss, kBlockKV)) return -5;
   if (!make_tmap_bhsd(&tv, a.v, a.is_bf16, D, a.hkv, a.b, a.sk, a.v_sh, a.v_sb, a.v_ss, kBlockKV)) return -5;
   auto kern = attn_fwd_kernel<D, kBf16>;
-  static const bool ready = prepare_kernel(kern, L::kTotal, "attn_fwd");
+  static const bool ready = prepare_kernel(kern, L::kTotal, "attn_fwd", kFwdThreads, 256 * kFwdMathRegs + 128 * kFwdIssueRegs);
   if (!ready) return -10;
   FwdParams p{};
   p.lse = a.lse; p.o = a.o; p.o_sb = a.o_sb; p.o_sh = a.o_sh; p.o_ss = a.o_ss;
@@ -953,7 +974,7 @@ int launch_fwd(const AttnArgs& a, cudaStream_t s) {
   p.scale_log2 = a.scale * kLog2e; p.causal = a.causal ? 1 : 0; p.wait_limit = a.wait_limit < 0 ? kWaitLimit : a.wait_limit;
   const int64_t ctas = static_cast<int64_t>((a.sq + 2 * kBlockQ - 1) / (2 * kBlockQ)) * a.hq * a.b;
   if (ctas > 0x7fffffff) { g_attn_err = "too many query blocks"; return -12; }
-  kern<<<static_cast<unsigned>(ctas), kThreads, L::kTotal, s>>>(tq, tk, tv, p);
+  kern<<<static_cast<unsigned>(ctas), kFwdThreads, L::kTotal, s>>>(tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_attn_err = std::string("attn_fwd launch: ") + cudaGetErrorString(e); return -11; }
   return 0;
@@ -970,7 +991,7 @@ int launch_bwd_parts(const AttnArgs& a, cudaStream_t s) {
       !make_tmap_bhsd(&tdo, a.d_o, a.is_bf16, D, a.hq, a.b, a.sq, a.do_sh, a.do_sb, a.do_ss, kBwdCols))
     return -5;
   auto kern = attn_bwd_kernel<D, kBf16>;
-  static const bool ready = prepare_kernel(kern, L::kTotal, "attn_bwd");
+  static const bool ready = prepare_kernel(kern, L::kTotal, "attn_bwd", kThreads, 512 * kMathRegs + 128 * kIssueRegs);
   if (!ready) return -10;
   BwdParams p{};
   p.nlse = a.delta + static_cast<int64_t>(a.b) * a.hq * a.sq;   // written by attn_delta_kernel
