@@ -176,6 +176,7 @@ struct EmbeddingGradArgs {
   void* dw;
   int* order;      // n
   float* parts;    // embedding_grad_parts(n, h)
+  bool add;        // dw is fp32 and is added to
   int n, h, inner;
   int64_t vocab, st_outer, st_inner;
   bool is_bf16;

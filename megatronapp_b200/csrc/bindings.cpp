@@ -531,8 +531,9 @@ Tensor rope_apply(const Tensor& x, const Tensor& cos_sin, bool interleaved, bool
   count();
   return y;
 }
-// ids: int64 [n] or [outer, inner], contiguous; dy: ids' shape x h, 16-byte rows at any strides of the leading dimensions
-Tensor embedding_grad(const Tensor& dy, const Tensor& ids, int64_t vocab) {
+// ids: int64 [n] or [outer, inner], contiguous; dy: ids' shape x h, 16-byte rows at any strides of the leading dimensions.  With `into`, fp32 [vocab, h], the
+// gradient is added to that.
+Tensor embedding_grad(const Tensor& dy, const Tensor& ids, int64_t vocab, const c10::optional<Tensor>& into) {
   c10::cuda::CUDAGuard guard(dy.device());
   TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kLong && ids.is_contiguous() && (ids.dim() == 1 || ids.dim() == 2) && dy.dim() == ids.dim() + 1 &&
               ids.numel() > 0 && ids.numel() < (1 << 20) && vocab > 0 && vocab <= 0x7fffffff, "embedding_grad: ids");
@@ -545,7 +546,11 @@ Tensor embedding_grad(const Tensor& dy, const Tensor& ids, int64_t vocab) {
   a.inner = static_cast<int>(ids.size(-1));
   a.st_outer = ids.dim() == 2 ? dy.stride(0) : 0;
   a.st_inner = dy.stride(ids.dim() - 1);
-  auto dw = torch::zeros({vocab, h}, dy.options());
+  a.add = into.has_value() && into->defined();
+  if (a.add)
+    TORCH_CHECK(into->scalar_type() == at::kFloat && into->is_contiguous() && into->dim() == 2 && into->size(0) == vocab && into->size(1) == h &&
+                into->device() == dy.device() && reinterpret_cast<uintptr_t>(into->data_ptr()) % 16 == 0, "embedding_grad: buffer");
+  Tensor dw = a.add ? *into : torch::zeros({vocab, h}, dy.options());
   auto order = torch::empty({a.n}, dy.options().dtype(at::kInt));
   auto parts = torch::empty({b200::embedding_grad_parts(a.n, a.h)}, dy.options().dtype(at::kFloat));
   a.dy = dy.data_ptr(); a.ids = ids.data_ptr<int64_t>(); a.dw = dw.data_ptr(); a.order = order.data_ptr<int>(); a.parts = parts.data_ptr<float>();
@@ -1457,7 +1462,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     count();
   });
   m.def("router_linear_bwd", &router_linear_bwd);
-  m.def("embedding_grad", &embedding_grad);
+  m.def("embedding_grad", &embedding_grad, py::arg("dy"), py::arg("ids"), py::arg("vocab"), py::arg("into") = c10::optional<Tensor>());
   m.def("ce_local_stats", &ce_local_stats);
   m.def("ce_rescale", &ce_rescale);
   m.def("ce_grad", &ce_grad);

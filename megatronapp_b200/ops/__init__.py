@@ -212,7 +212,37 @@ def bias_grad(dy2: torch.Tensor, dtype: Optional[torch.dtype] = None) -> torch.T
 # the tokens, and three launches behind a Python node cost the host more than one.  us of a call alone here / there, tables of 50304 x 768 and
 # 1024 x 768: 64 tokens 86 / 58 and 88 / 64; 2048 86 / 114 and 86 / 68; 3072 87 / 161 and 86 / 95; 4096 86 / 210 and 87 / 156; 16384 113 / 361
 # and 94 / 177
+# Where the gradient goes straight into an fp32 buffer there is nothing of the table's size, and the kernels are the better way from the first token on.
 _EMBED_FROM, _EMBED_TO = 2049, 16384
+
+
+def _lookup_buffer(node):
+    """The fp32 buffer that the gradient of a looked-up table can be added to now, or None: where nobody but the owner of that buffer (``lookup_adds``, see
+    parallel/ddp.py) would see the gradient itself, and it would end there anyway."""
+    leaf = node.next_functions[1][0]
+    weight = getattr(leaf, "variable", None)
+    if weight is None or not getattr(weight, "lookup_adds", False) or weight.grad is not None or weight._backward_hooks \
+            or len(weight._post_accumulate_grad_hooks or ()) != 1 or getattr(weight, "b200_wgrad_store_first", False):
+        return None
+    main_grad = getattr(weight, "main_grad", None)
+    if main_grad is None or main_grad.dtype != torch.float32 or not main_grad.is_contiguous() or main_grad.shape != weight.shape or main_grad.data_ptr() % 16 \
+            or main_grad.device != weight.device:
+        return None
+    try:                                                # an error where gradients are asked for (autograd.grad) and do not go to the parameters
+        if not torch._C._will_engine_execute_node(leaf):
+            return None
+    except RuntimeError:
+        return None
+    # several lookups may run on streams of their own, one behind the other here; who called the pass waits for the last
+    stream = torch.cuda.current_stream(weight.device)
+    before = getattr(weight, "lookup_stream", None)
+    if before is not None and before != stream:
+        stream.wait_stream(before)
+    weight.lookup_stream = stream
+    torch.autograd.Variable._execution_engine.queue_callback(lambda: torch.cuda.current_stream(weight.device).wait_stream(stream)
+                                                             if torch.cuda.current_stream(weight.device) != stream else None)
+    weight.grad_added_to_main_grad = True
+    return main_grad
 
 
 class _EmbeddingFn(torch.autograd.Function):
@@ -229,13 +259,15 @@ class _EmbeddingFn(torch.autograd.Function):
             return None, torch.ops.aten.embedding_dense_backward(dy, ids, ctx.vocab, -1, False)
         if dy.stride(-1) != 1 or any(st % 8 for st in dy.stride()[:-1]) or dy.data_ptr() % 16:
             dy = dy.clone(memory_format=torch.contiguous_format)
-        return None, ext().embedding_grad(dy, ids.long().contiguous(), ctx.vocab)
+        into = _lookup_buffer(ctx)
+        dw = ext().embedding_grad(dy, ids.long().contiguous(), ctx.vocab, into)
+        return None, None if into is not None else dw
 
 
 def embedding(ids: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """Rows ``ids`` of ``weight``; the dense gradient of a 16-bit table comes from kernels that sum in fp32 and a fixed order."""
     if (_native(weight) and weight.requires_grad and torch.is_grad_enabled() and ids.is_cuda and ids.dim() in (1, 2) and weight.dim() == 2
-            and _EMBED_FROM <= ids.numel() <= _EMBED_TO and weight.shape[1] % 8 == 0 and 0 < weight.shape[1] < 1 << 24 and 0 < weight.shape[0] <= 0x7fffffff
+            and (1 if getattr(weight, "lookup_adds", False) else _EMBED_FROM) <= ids.numel() <= _EMBED_TO and weight.shape[1] % 8 == 0 and 0 < weight.shape[1] < 1 << 24 and 0 < weight.shape[0] <= 0x7fffffff
             and _eager()):
         return _EmbeddingFn.apply(ids, weight)
     return torch.nn.functional.embedding(ids, weight)

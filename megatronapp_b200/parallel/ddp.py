@@ -319,6 +319,8 @@ class DistributedDataParallel(nn.Module):
         for p, buf in self.param_to_buffer.items():
             self._hooks.append(p.register_post_accumulate_grad_hook(self._make_hook(buf)))
             p.grad_ready_hook = self._make_fused_ready(p, buf)
+            # the gradient of a lookup may be added to main_grad by its own kernels: no bucket waits to hear of it from the hook
+            p.lookup_adds = not ddp_config.overlap_grad_reduce and p.main_grad.dtype == torch.float32
         self.is_last_microbatch = True
 
     def _make_buffers(self, params, group, group_size, scale, device, out, kind):

@@ -1,0 +1,108 @@
+"""The gradient of a lookup, added to the fp32 buffer by its own kernels: against the dense way, and where that way is kept."""
+import pytest
+import torch
+import torch.nn as nn
+
+pytestmark = pytest.mark.gpu
+
+
+class _Net(nn.Module):
+    def __init__(self, vocab, h, dtype):
+        super().__init__()
+        self.weight = nn.Parameter((torch.randn(vocab, h, generator=torch.Generator().manual_seed(1)) * 0.5).to(dtype))
+
+    def forward(self, *ids):
+        from megatronapp_b200 import ops
+
+        return sum(ops.embedding(i, self.weight).float().square().sum() for i in ids)
+
+
+def _ddp(vocab, h, dtype, **kw):
+    from megatronapp_b200.config.transformer_config import TransformerConfig
+    from megatronapp_b200.parallel import state as ps
+    from megatronapp_b200.parallel.ddp import DistributedDataParallel, DistributedDataParallelConfig
+
+    if not ps.model_parallel_is_initialized():
+        ps.initialize_model_parallel(1, 1)
+    cfg = TransformerConfig(num_layers=1, hidden_size=64, num_attention_heads=1, params_dtype=dtype, bf16=dtype is torch.bfloat16, fp16=dtype is torch.float16)
+    return DistributedDataParallel(cfg, DistributedDataParallelConfig(grad_reduce_in_fp32=True, **kw), _Net(vocab, h, dtype).cuda())
+
+
+def _want(w, *ids):
+    """The looked-up rows' gradients 2 w, summed in 64 bits, and the size of the sums' terms."""
+    rows = torch.cat([i.reshape(-1) for i in ids])
+    dy = (2 * w.detach().float()[rows]).to(w.dtype).double()
+    return (torch.zeros(w.shape, dtype=torch.float64, device="cuda").index_add_(0, rows, t) for t in (dy, dy.abs()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,vocab,h", [((1,), 1, 8), ((16,), 3, 72), ((17,), 2, 1032), ((4, 33), 50, 256), ((4096,), 50304, 64), ((2, 5000), 7, 768)])
+def test_added_rows(shape, vocab, h, dtype):
+    ddp = _ddp(vocab, h, dtype)
+    w = ddp.module.weight
+    ids = torch.randint(0, vocab, shape, generator=torch.Generator().manual_seed(2)).cuda()
+    ddp.zero_grad_buffer()
+    w.main_grad.fill_(0.25)
+    ddp(ids).backward()
+    want, size = _want(w, ids)
+    # fp32 sums of as many terms, and one to the buffer's 0.25
+    assert bool(((w.main_grad.double() - 0.25 - want).abs() <= ids.numel() * 2.0 ** -24 * size + 2.0 ** -24 * (want.abs() + 0.25)).all())
+    assert w.grad is None and w.grad_added_to_main_grad
+    first = w.main_grad.clone()
+    ddp.zero_grad_buffer()
+    w.main_grad.fill_(0.25)
+    ddp(ids).backward()
+    assert torch.equal(w.main_grad, first)
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_two_lookups(side):
+    """Of one table, the second on a stream of its own."""
+    ddp = _ddp(300, 64, torch.bfloat16)
+    w = ddp.module.weight
+    a, b = (torch.randint(0, 300, (3000,), generator=torch.Generator().manual_seed(k)).cuda() for k in (3, 4))
+    ddp.zero_grad_buffer()
+    stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    first = ddp(a)
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        second = ddp(b)
+    torch.cuda.current_stream().wait_stream(stream)
+    (first + second).backward()
+    got = w.main_grad.clone()
+    want, size = _want(w, a, b)
+    assert bool(((got.double() - want).abs() <= 6000 * 2.0 ** -24 * size + 2.0 ** -24).all())
+
+
+def test_the_dense_way_is_kept():
+    """autograd.grad, hooks of others, a gradient that is there already, buffers reduced while the pass runs, no buffers at all."""
+    from megatronapp_b200 import ops
+
+    ids = torch.randint(0, 100, (2100,), generator=torch.Generator().manual_seed(5)).cuda()
+
+    def dense(ddp, prepare=lambda w: None):
+        w, seen = ddp.module.weight, []
+        ddp.zero_grad_buffer()
+        prepare(w)
+        handle = w.register_hook(lambda g: seen.append(g.clone()))
+        ddp(ids).backward()
+        handle.remove()
+        assert len(seen) == 1 and seen[0].shape == w.shape and torch.equal(w.main_grad, seen[0].float()) and w.grad is None
+        return seen[0]
+
+    ddp = _ddp(100, 64, torch.bfloat16)
+    g = dense(ddp)
+    w = ddp.module.weight
+    ddp.zero_grad_buffer()
+    got = torch.autograd.grad(ddp(ids), w)[0]
+    assert torch.equal(got, g) and not w.main_grad.any()
+    w.grad = torch.ones_like(w)
+    ddp(ids).backward()
+    assert torch.equal(w.main_grad, (g + 1).float()) and w.grad is None
+    over = _ddp(100, 64, torch.bfloat16, overlap_grad_reduce=True)
+    assert not over.module.weight.lookup_adds
+    dense(over)
+    plain = _Net(100, 64, torch.bfloat16).cuda()
+    plain(ids).backward()
+    assert torch.equal(plain.weight.grad, g)
+    assert ops.embedding(ids[:5], plain.weight).grad_fn.name().startswith("Embedding")
