@@ -687,6 +687,63 @@ __global__ void rope_kernel(const T* __restrict__ x, const float* __restrict__ c
   }
 }
 
+// The same with 16-byte accesses: a thread takes eight pairs of a rotated head (four, side by side, where they are interleaved), or eight values of the tail.
+// Bound by HBM.  us with a pair a thread / here (at the copy bandwidth), bf16: 8192 rows of 32 heads of 128 83 / 22 (20), interleaved 84 / 26, half of
+// each head 74 / 31; 2048 x 32 x 128 23 / 8.5 (5.1), 4096 x 12 x 64 10.5 / 5.2 (1.9).
+template <typename T, bool kInterleaved>
+__global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, const float* __restrict__ cos_sin, T* __restrict__ y, uint32_t rows, uint32_t bh,
+                                                       int d, int rot_dim, float sign) {
+  const int half = rot_dim / 2, rotated = kInterleaved ? rot_dim / 8 : rot_dim / 16;
+  const uint32_t per_row = rotated + (d - rot_dim) / 8, step = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t row = first / per_row, at = first % per_row;
+  const uint32_t row_step = step / per_row, at_step = step % per_row;
+  while (row < rows) {
+    const T* xr = x + static_cast<size_t>(row) * d;
+    T* yr = y + static_cast<size_t>(row) * d;
+    if (static_cast<int>(at) < rotated) {
+      const float* cs = cos_sin + static_cast<size_t>(row / bh) * rot_dim;
+      if constexpr (kInterleaved) {
+        float v[8], o[8];
+        load8(xr + at * 8, v);
+        const float4 c = reinterpret_cast<const float4*>(cs)[at], t = reinterpret_cast<const float4*>(cs + half)[at];
+        const float cc[4] = {c.x, c.y, c.z, c.w}, ss[4] = {sign * t.x, sign * t.y, sign * t.z, sign * t.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          o[2 * j] = v[2 * j] * cc[j] - v[2 * j + 1] * ss[j];
+          o[2 * j + 1] = v[2 * j + 1] * cc[j] + v[2 * j] * ss[j];
+        }
+        store8(yr + at * 8, o);
+      } else {
+        float a[8], b[8], c[8], t[8], o[8], q[8];
+        load8(xr + at * 8, a);
+        load8(xr + half + at * 8, b);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const float4 cv = reinterpret_cast<const float4*>(cs)[at * 2 + k], tv = reinterpret_cast<const float4*>(cs + half)[at * 2 + k];
+          c[4 * k] = cv.x; c[4 * k + 1] = cv.y; c[4 * k + 2] = cv.z; c[4 * k + 3] = cv.w;
+          t[4 * k] = sign * tv.x; t[4 * k + 1] = sign * tv.y; t[4 * k + 2] = sign * tv.z; t[4 * k + 3] = sign * tv.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          o[j] = a[j] * c[j] - b[j] * t[j];
+          q[j] = b[j] * c[j] + a[j] * t[j];
+        }
+        store8(yr + at * 8, o);
+        store8(yr + half + at * 8, q);
+      }
+    } else {
+      const int e = rot_dim + (static_cast<int>(at) - rotated) * 8;
+      *reinterpret_cast<uint4*>(yr + e) = *reinterpret_cast<const uint4*>(xr + e);
+    }
+    row += row_step;
+    at += at_step;
+    if (at >= per_row) {
+      at -= per_row;
+      ++row;
+    }
+  }
+}
+
 // dbias[c] = sum_r dy[r, c].  A CTA sums 64 columns over its share of the rows.  Up to 512 rows a CTA, the CTAs of a cluster share the rows and the
 // first adds the shares up in order, in one launch; longer shares are cut finer, and a second launch adds them up in order.  us, cluster / two
 // launches / what stood here before both (a fill, atomic additions, a conversion), inputs from HBM where they do not fit L2 eight times:
@@ -1144,7 +1201,19 @@ void dropout_bwd(const void* dy, const uint8_t* mask, void* dx, int64_t n, float
 }
 void rope_apply(const void* x, const float* cos_sin, void* y, int s, int b, int h, int d,
                 int rot_dim, bool interleaved, bool inverse, bool is_bf16, cudaStream_t st) {
-  const int64_t total = static_cast<int64_t>(s) * b * h * (d / 2);
+  const int64_t rows = static_cast<int64_t>(s) * b * h;
+  auto at_16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  if (rot_dim > 0 && rot_dim % (interleaved ? 8 : 16) == 0 && d % 8 == 0 && rot_dim <= d && rows > 0 && rows < (int64_t{1} << 30) && at_16(x) && at_16(y) &&
+      at_16(cos_sin)) {
+    const int64_t items = rows * ((interleaved ? rot_dim / 8 : rot_dim / 16) + (d - rot_dim) / 8);
+    const float sign = inverse ? -1.f : 1.f;
+    DISPATCH_16(is_bf16, {
+      auto kern = interleaved ? rope_vec_kernel<T, true> : rope_vec_kernel<T, false>;
+      kern<<<grid_for(items, 256), 256, 0, st>>>((const T*)x, cos_sin, (T*)y, static_cast<uint32_t>(rows), static_cast<uint32_t>(b * h), d, rot_dim, sign);
+    });
+    return;
+  }
+  const int64_t total = rows * (d / 2);
   DISPATCH_16(is_bf16, (rope_kernel<T><<<grid_for(total, 256), 256, 0, st>>>(
                            (const T*)x, cos_sin, (T*)y, s, b * h, d, rot_dim, interleaved,
                            inverse ? -1.f : 1.f)));

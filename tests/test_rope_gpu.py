@@ -1,0 +1,27 @@
+"""Rotary embedding in vectors of 16 bytes, and a pair a thread where rows or sizes do not allow them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("s,b,h,d,rot", [
+    (1, 1, 1, 16, 16), (3, 2, 5, 64, 64), (700, 1, 3, 128, 128), (65, 2, 4, 128, 64), (5, 1, 2, 96, 48), (2000, 2, 8, 128, 128),
+    (7, 1, 3, 64, 8), (7, 2, 3, 64, 12), (9, 1, 1, 20, 16), (33, 1, 2, 64, 24)])            # a pair a thread, for one of the two orders at least
+def test_rope(s, b, h, d, rot, interleaved, dtype):
+    from megatronapp_b200 import ops
+
+    g = torch.Generator("cuda").manual_seed(s + d)
+    ang = torch.rand(s + 2, rot // 2, generator=g, device="cuda") * 6.2
+    cs = torch.cat([ang.cos(), ang.sin()], -1)
+    wide = torch.randn(s * b * h * d + 8, generator=g, device="cuda").to(dtype)
+    for x in (wide[:-8].view(s, b, h, d), wide[1:-7].view(s, b, h, d)):                       # the second begins 2 bytes further on
+        for inverse in (False, True):
+            got = ops.ext().rope_apply(x, cs, interleaved, inverse)
+            want = ops.rope_ref(x.double(), cs, interleaved, inverse).double()
+            # two products of values up to one and their sum in fp32, then the result's rounding
+            tol = (2.0 ** -8 if dtype is torch.bfloat16 else 2.0 ** -11) * want.abs() + 2.0 ** -22 * float(x.abs().max())
+            assert bool(((got.double() - want).abs() <= tol + 2.0 ** -24).all())
+        assert torch.equal(ops.ext().rope_apply(x, cs, interleaved, False)[..., rot:], x[..., rot:])
