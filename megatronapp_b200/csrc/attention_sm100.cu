@@ -507,13 +507,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
 
 // ------------------------------------------------------------------------------------ backward
-// -delta[b, h, s] = -sum_d O * dO and -lse * log2e, the addends of the backward kernels' packed multiply-adds.  D / 8 lanes share a row
+// -delta[b, h, s] = -sum_d O * dO and -lse * log2e, the addends of the backward kernels' packed multiply-adds, in rows of whole blocks of 64: behind the last query
+// stand zeros and -infinity, of which come weights of zero.  D / 8 lanes share a row
 // (16 bytes each), a warp takes four groups of rows with all its loads in flight: 12.5 us for 32 heads x 4096 x 128 (a warp per row and
 // 4 bytes a lane took 35).
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ d_o, float* __restrict__ ndelta, const float* __restrict__ lse,
-                  float* __restrict__ nlse2, int h, int s, int64_t o_sb, int64_t o_sh, int64_t o_ss, int64_t do_sb, int64_t do_sh, int64_t do_ss,
+                  float* __restrict__ nlse2, int h, int s, int pitch, int64_t o_sb, int64_t o_sh, int64_t o_ss, int64_t do_sb, int64_t do_sh, int64_t do_ss,
                   int is_bf16) {
   constexpr int kLanes = D / 8, kRows = 32 / kLanes, kSteps = 4;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = (lane % kLanes) * 8;
@@ -546,18 +547,19 @@ attn_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ d
     }
 #pragma unroll
     for (int k = kLanes / 2; k > 0; k >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, k);
-    if (si < s && lane % kLanes == 0) {
-      const int64_t row = (static_cast<int64_t>(bi) * h + hi) * s + si;
+    if (si < pitch && lane % kLanes == 0) {
+      const int64_t head = static_cast<int64_t>(bi) * h + hi, row = head * pitch + si;
+      const float lv = si < s ? lse[head * s + si] : -INFINITY;
       ndelta[row] = -acc;
-      const float lv = lse[row];
       nlse2[row] = lv == -INFINITY ? -INFINITY : -lv * kLog2e;   // fully masked rows give P = 0
     }
   }
 }
 
 struct BwdParams {
-  const float* nlse;    // [b, hq, sq] -LSE in the exp2 domain (-lse * log2e)
-  const float* ndelta;  // [b, hq, sq] -delta
+  const float* nlse;    // [b, hq, pitch] -LSE in the exp2 domain (-lse * log2e)
+  const float* ndelta;  // [b, hq, pitch] -delta
+  int pitch;            // sq in whole blocks of 64
   void *dq, *dk, *dv;
   int64_t dq_sb, dq_sh, dq_ss, dk_sb, dk_sh, dk_ss, dv_sb, dv_sh, dv_ss;
   int b, hq, hkv, sq, sk;
@@ -689,7 +691,7 @@ __device__ __forceinline__ void bwd_part(const CUtensorMap& tmap_x1, const CUten
           tma_load_4d(&tmap_y2, &y_full[ys], y2 + c * (kBwdCols * 128), c * 64, head, bi, c0);
         }
         if (!kDQ) {
-          const int64_t base = (static_cast<int64_t>(bi) * p.hq + head) * p.sq + c0;
+          const int64_t base = (static_cast<int64_t>(bi) * p.hq + head) * p.pitch + c0;
           bulk_load_1d(sStat + ys * 128, p.nlse + base, 256, &y_full[ys]);
           bulk_load_1d(sStat + ys * 128 + 64, p.ndelta + base, 256, &y_full[ys]);
         }
@@ -761,7 +763,7 @@ __device__ __forceinline__ void bwd_part(const CUtensorMap& tmap_x1, const CUten
     const uint64_t sc2 = f2(p.scale_log2, p.scale_log2);
     uint64_t row_nlse = 0, row_ndelta = 0;         // dQ mode: statistics of this thread's query row
     if (kDQ) {
-      const int64_t idx = (static_cast<int64_t>(bi) * p.hq + out_head) * p.sq + min(grow, p.sq - 1);
+      const int64_t idx = (static_cast<int64_t>(bi) * p.hq + out_head) * p.pitch + min(grow, p.sq - 1);
       row_nlse = f2(p.nlse[idx], p.nlse[idx]);     // already in the exp2 domain (-inf for fully masked rows)
       row_ndelta = f2(p.ndelta[idx], p.ndelta[idx]);
     }
@@ -994,7 +996,8 @@ int launch_bwd_parts(const AttnArgs& a, cudaStream_t s) {
   static const bool ready = prepare_kernel(kern, L::kTotal, "attn_bwd", kThreads, 512 * kMathRegs + 128 * kIssueRegs);
   if (!ready) return -10;
   BwdParams p{};
-  p.nlse = a.delta + static_cast<int64_t>(a.b) * a.hq * a.sq;   // written by attn_delta_kernel
+  p.pitch = attn_stat_pitch(a.sq);
+  p.nlse = a.delta + static_cast<int64_t>(a.b) * a.hq * p.pitch;   // written by attn_delta_kernel
   p.ndelta = a.delta;
   p.dq = a.dq; p.dq_sb = a.dq_sb; p.dq_sh = a.dq_sh; p.dq_ss = a.dq_ss;
   p.dk = a.dk; p.dk_sb = a.dk_sb; p.dk_sh = a.dk_sh; p.dk_ss = a.dk_ss;
@@ -1021,11 +1024,12 @@ int launch_bwd_parts(const AttnArgs& a, cudaStream_t s) {
 
 template <int D>
 int launch_bwd(const AttnArgs& a, cudaStream_t s) {
-  const int64_t rows = static_cast<int64_t>(a.b) * a.hq * a.sq;
+  const int pitch = attn_stat_pitch(a.sq);
+  const int64_t rows = static_cast<int64_t>(a.b) * a.hq * pitch;
   constexpr int kPerBlock = 8 * 4 * (256 / D);   // warps x row groups x rows
   if (a.hq > 65535 || a.b > 65535) { g_attn_err = "too many heads or sequences"; return -12; }
-  attn_delta_kernel<D><<<dim3((a.sq + kPerBlock - 1) / kPerBlock, a.hq, a.b), 256, 0, s>>>(
-      static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.d_o), a.delta, a.lse, a.delta + rows, a.hq, a.sq, a.o_sb, a.o_sh, a.o_ss,
+  attn_delta_kernel<D><<<dim3((pitch + kPerBlock - 1) / kPerBlock, a.hq, a.b), 256, 0, s>>>(
+      static_cast<const uint16_t*>(a.o), static_cast<const uint16_t*>(a.d_o), a.delta, a.lse, a.delta + rows, a.hq, a.sq, pitch, a.o_sb, a.o_sh, a.o_ss,
       a.do_sb, a.do_sh, a.do_ss, a.is_bf16 ? 1 : 0);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { g_attn_err = std::string("attn_delta launch: ") + cudaGetErrorString(e); return -11; }
@@ -1035,6 +1039,8 @@ int launch_bwd(const AttnArgs& a, cudaStream_t s) {
 }  // namespace
 
 const char* attn_last_error() { return g_attn_err.c_str(); }
+
+int attn_stat_pitch(int sq) { return (sq + kBwdCols - 1) / kBwdCols * kBwdCols; }
 
 int attn_status(bool clear) {
   int v = 0;
@@ -1062,7 +1068,7 @@ int attn_bwd(const AttnArgs& a, cudaStream_t s) {
   if (a.d != 64 && a.d != 128) { g_attn_err = "head dim must be 64 or 128"; return -1; }
   if (a.hq % a.hkv != 0) { g_attn_err = "hq must be a multiple of hkv"; return -1; }
   if (a.causal && a.sq != a.sk) { g_attn_err = "causal attention needs sq == sk"; return -2; }
-  if (a.sq % kBwdCols != 0 || a.sk % kBwdCols != 0) { g_attn_err = "backward needs sq, sk multiples of 64"; return -3; }
+  if (!a.causal && (a.sq % kBwdCols != 0 || a.sk % kBwdCols != 0)) { g_attn_err = "backward that is not causal needs sq, sk multiples of 64"; return -3; }
   if (!strides_ok(a.q_sb, a.q_sh, a.q_ss, a.q) || !strides_ok(a.k_sb, a.k_sh, a.k_ss, a.k) ||
       !strides_ok(a.v_sb, a.v_sh, a.v_ss, a.v) || !strides_ok(a.o_sb, a.o_sh, a.o_ss, a.o) ||
       !strides_ok(a.do_sb, a.do_sh, a.do_ss, a.d_o) || !strides_ok(a.dq_sb, a.dq_sh, a.dq_ss, a.dq) ||

@@ -249,6 +249,7 @@ struct AttnArgs {
 int attn_fwd(const AttnArgs& a, cudaStream_t s);
 int attn_bwd(const AttnArgs& a, cudaStream_t s);
 const char* attn_last_error();
+int attn_stat_pitch(int sq);   // AttnArgs::delta is [2, b, hq, attn_stat_pitch(sq)]
 int attn_status(bool clear);   // 1: a kernel of this process gave up on a wait (its rows are NaN); synchronises
 
 // causal attention with logistic weights over packed prompts (tcgen05)

@@ -926,7 +926,7 @@ std::vector<Tensor> attn_bwd(const Tensor& d_o, const Tensor& q, const Tensor& k
   Tensor dk = dk_out.has_value() ? dk_out.value() : torch::empty({a.sk, a.b, a.hkv, a.d}, q.options()).permute({1, 2, 0, 3});
   Tensor dv = dv_out.has_value() ? dv_out.value() : torch::empty({a.sk, a.b, a.hkv, a.d}, q.options()).permute({1, 2, 0, 3});
   check_bhsd(dq, "dq"); check_bhsd(dk, "dk"); check_bhsd(dv, "dv");
-  auto delta = torch::empty({2, a.b, a.hq, a.sq}, q.options().dtype(at::kFloat));   // [delta ; lse * log2e]
+  auto delta = torch::empty({2, a.b, a.hq, b200::attn_stat_pitch(a.sq)}, q.options().dtype(at::kFloat));   // [delta ; lse * log2e]
   a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = const_cast<void*>(o.data_ptr()); a.lse = lse.data_ptr<float>();
   a.d_o = doc.data_ptr(); a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr();
   a.delta = delta.data_ptr<float>(); a.dq_accum = nullptr;

@@ -547,15 +547,29 @@ class _PackedQKVAttnFn(torch.autograd.Function):
         return dmixed, None, None
 
 
+def _short_odd_training(b, hq, hkv, sq, sk, causal):
+    """Whether a call with gradients whose lengths are no whole blocks of 64 is better here than in the library's attention. Device time of forward and
+    backward in us, library / here: grouped heads [32, 8 of 2, 459, 128] 196 / 169, [8, 8 of 2, 330, 64] 51 / 39, [1, 8 of 4, 70, 128] 38 / 21 - the
+    library writes a gradient of K and V for each query head and adds them up in a pass of its own; as many heads [8, 8, 459, 64] 49 / 48,
+    [8, 8, 129, 64] 35 / 27, [1, 8, 510, 128] 45 / 33, [32, 8, 97, 64] 49 / 39, but [32, 8, 129, 64] 60 / 62, [32, 8, 459, 64] 132 / 159. From 512 rows on
+    the padding to whole blocks is small beside the work and the library's backward is the faster: [32, 8, 600, 128] 251 / 296, [1, 16 of 4, 979, 64]
+    60 / 74. Not causal it is no better either: [6, 8, 700, 64] 56 / 72."""
+    return causal and sq == sk and 0 < sq < 512 and (hq > hkv or b * hq * sq <= 1 << 15)
+
+
 def attention_packed_qkv(mixed, scale=None, causal=True):
     """``mixed``: ``[s, b, np, 3*hn]`` (q | k | v per head).  Returns ``[b, np, s, hn]`` or ``None`` when the
     native packed path does not apply (caller falls back to split + ``attention``)."""
     hn = mixed.shape[-1] // 3
     if not (_native(mixed) and _ATTN_IMPL in ("auto", "native") and hn in (64, 128) and mixed.is_contiguous()
-            and mixed.shape[0] % 64 == 0 and native_attention_available()):
+            and native_attention_available()):
+        return None
+    sq, b, h, _ = mixed.shape
+    eager = _eager()
+    if sq % 64 != 0 and not (eager and _short_odd_training(b, h, h, sq, sq, causal)):
         return None
     scale = scale if scale is not None else 1.0 / math.sqrt(hn)
-    if _eager():
+    if eager:
         return ext().attention_packed(mixed, scale, causal)
     return _PackedQKVAttnFn.apply(mixed, scale, causal)
 
@@ -599,7 +613,8 @@ def attention(q, k, v, scale=None, causal=True, dropout_p=0.0, training=True, ma
     sq, sk = q.shape[2], k.shape[2]
     needs_grad = torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)
     usable = (_native(q) and p == 0.0 and mask is None and d in (64, 128) and (not causal or sq == sk)
-              and q.shape[1] % k.shape[1] == 0 and (not needs_grad or (sq % 64 == 0 and sk % 64 == 0)))
+              and q.shape[1] % k.shape[1] == 0 and (not needs_grad or (sq % 64 == 0 and sk % 64 == 0)
+                   or (_short_odd_training(q.shape[0], q.shape[1], k.shape[1], sq, sk, causal) and _eager())))
     if impl in ("auto", "native") and usable and native_attention_available():
         q, k, v = (t if _attn_view_ok(t) else t.contiguous() for t in (q, k, v))
         if _eager():
