@@ -233,12 +233,13 @@ def _lookup_buffer(node):
             return None
     except RuntimeError:
         return None
-    # several lookups may run on streams of their own, one behind the other here; who called the pass waits for the last
-    stream = torch.cuda.current_stream(weight.device)
+    # several lookups of a pass may run on streams of their own, one behind the other here; who called the pass waits for the last.  (An earlier pass's stream is
+    # no concern of this one's, and may not be waited for while this one is captured.)
+    stream, task = torch.cuda.current_stream(weight.device), torch._C._current_graph_task_id()
     before = getattr(weight, "lookup_stream", None)
-    if before is not None and before != stream:
-        stream.wait_stream(before)
-    weight.lookup_stream = stream
+    if before is not None and before[0] == task and before[1] != stream:
+        stream.wait_stream(before[1])
+    weight.lookup_stream = (task, stream)
     torch.autograd.Variable._execution_engine.queue_callback(lambda: torch.cuda.current_stream(weight.device).wait_stream(stream)
                                                              if torch.cuda.current_stream(weight.device) != stream else None)
     weight.grad_added_to_main_grad = True

@@ -74,6 +74,27 @@ def test_two_lookups(side):
     assert bool(((got.double() - want).abs() <= 6000 * 2.0 ** -24 * size + 2.0 ** -24).all())
 
 
+def test_captured_after_a_pass_on_another_stream():
+    """The capture must not wait for the stream of a pass that it does not hold."""
+    ids = torch.randint(0, 50, (300,), generator=torch.Generator().manual_seed(6)).cuda()
+    warm, hold = torch.cuda.Stream(), torch.cuda.Stream()
+    warm.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(warm):
+        ddp = _ddp(50, 64, torch.bfloat16)
+        w = ddp.module.weight
+        ddp.zero_grad_buffer()
+        ddp(ids).backward()
+    torch.cuda.synchronize()
+    want = w.main_grad.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=hold):
+        ddp(ids).backward()
+    assert torch.equal(w.main_grad, want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(w.main_grad, 2 * want)
+
+
 def test_the_dense_way_is_kept():
     """autograd.grad, hooks of others, a gradient that is there already, buffers reduced while the pass runs, no buffers at all."""
     from megatronapp_b200 import ops
