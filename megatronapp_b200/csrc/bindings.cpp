@@ -972,6 +972,15 @@ struct NormNode : torch::autograd::Function<NormNode> {
   }
 };
 
+// A gradient that can be read but not differentiated again: at lengths that are no whole blocks that was always an error
+struct LastGrad : torch::autograd::Function<LastGrad> {
+  static Tensor forward(AutogradContext*, const Tensor& grad, const Tensor&, const Tensor&, const Tensor&, const Tensor&) { return grad.alias(); }
+  static variable_list backward(AutogradContext*, variable_list) { TORCH_CHECK(false, "derivative of the attention's backward is not implemented"); }
+  static Tensor of(const Tensor& grad, int64_t sq, const Tensor& d_o, const Tensor& q, const Tensor& k, const Tensor& v) {
+    return at::GradMode::is_enabled() && sq % 64 != 0 ? apply(grad, d_o, q, k, v) : grad;
+  }
+};
+
 struct AttnNode : torch::autograd::Function<AttnNode> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale, bool causal) {
     auto r = attn_fwd(q, k, v, scale, causal, false, -1);
@@ -984,6 +993,7 @@ struct AttnNode : torch::autograd::Function<AttnNode> {
     const auto s = ctx->get_saved_variables();
     auto r = attn_bwd(grads[0], s[0], s[1], s[2], s[3], s[4], ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool(), c10::nullopt,
                       c10::nullopt, c10::nullopt, -1);
+    for (int i = 0; i < 3; ++i) r[i] = LastGrad::of(r[i], s[0].size(2), grads[0], s[0], s[1], s[2]);
     return {r[0], r[1], r[2], Tensor(), Tensor()};
   }
 };
@@ -1006,7 +1016,7 @@ struct PackedAttnNode : torch::autograd::Function<PackedAttnNode> {
     Tensor d = at::empty_like(s[0]);
     attn_bwd(grads[0], part(s[0], 0), part(s[0], 1), part(s[0], 2), s[1], s[2], ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool(),
              part(d, 0), part(d, 1), part(d, 2), -1);
-    return {d, Tensor(), Tensor()};
+    return {LastGrad::of(d, s[0].size(0), grads[0], s[0], s[0], s[0]), Tensor(), Tensor()};
   }
 };
 

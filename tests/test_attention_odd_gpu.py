@@ -59,3 +59,16 @@ def test_who_watches_the_operators_keeps_the_library():
         ops.attention(q, k, v, 0.125)
         assert ops.attention_packed_qkv(torch.randn(100, 1, 2, 192, device="cuda").bfloat16()) is None
     assert ops.fallback_counts["attention_sdpa"] == before + 1
+
+
+def test_second_derivatives_are_refused():
+    from megatronapp_b200 import ops
+
+    q, k, v = (torch.randn(1, 2, 100, 64, device="cuda").bfloat16().requires_grad_() for _ in range(3))
+    mixed = torch.randn(100, 1, 2, 192, device="cuda").bfloat16().requires_grad_()
+    for o, leaf in ((ops.attention(q, k, v, 0.125), q), (ops.attention_packed_qkv(mixed), mixed)):
+        plain, = torch.autograd.grad(o.float().sum(), leaf, retain_graph=True)
+        again, = torch.autograd.grad(o.float().sum(), leaf, create_graph=True)
+        assert torch.equal(plain, again)
+        with pytest.raises(RuntimeError, match="not implemented"):
+            torch.autograd.grad(again.float().square().sum() + leaf.float().sum(), leaf)
